@@ -19,8 +19,9 @@ namespace {
 constexpr int kMaxDevices = 64;
 constexpr int kCounterCapacity = 8192;
 constexpr size_t kSamplingScratchBytes = 4u << 20;  // rows * chunks * 16 B
-constexpr size_t kGemmPartialBytes = 96u << 20;     // K-split partials of the prefill GEMM
-constexpr int64_t kSliceRowsMax = 128;             // up to here M > 32 runs as 32-row slices of the decode kernel
+// 33 .. 128 rows on few weights run as 32-row slices of the decode kernel: a problem this small is all pipeline fill, and
+// the decode kernel spreads it over more CTAs.
+constexpr int64_t kSliceRowsMax = 128, kSliceWeightsMax = 4 << 20;
 
 struct DeviceCtx {
     bool ready = false;
@@ -87,10 +88,10 @@ int run_linear(xinfer_stream_t s, const void* x, xb::ActType in, bool out_f32, c
     int rc = get_ctx(&c);
     if (rc != XINFER_OK) return rc;
     cudaStream_t stream = static_cast<cudaStream_t>(s);
-    if (c->forced_path != 2 && c->forced_path != 3 && in == xb::ActType::F16 && m > 32 && m <= kSliceRowsMax &&
+    int64_t weights = 0;
+    for (int i = 0; i < (swiglu ? 2 : num); ++i) weights += proj[i].n * k;
+    if (c->forced_path != 2 && c->forced_path != 3 && in == xb::ActType::F16 && m > 32 && m <= kSliceRowsMax && weights <= kSliceWeightsMax &&
         xb::tc_eligible(x, proj, num, swiglu, 32, k, group_size)) {
-        // 33 .. 128 rows: slices of 32 rows through the decode kernel (the reference's association, and cheaper than a
-        // 256-row GEMM tile that would be mostly padding: gate-sized projection 18 us per slice against 88 us)
         const int cnt = swiglu ? 2 : num;
         const size_t ybytes = out_f32 ? 4 : 2;
         for (int64_t r0 = 0; r0 < m; r0 += 32) {
@@ -118,14 +119,14 @@ int run_linear(xinfer_stream_t s, const void* x, xb::ActType in, bool out_f32, c
             cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
             if (cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
                 void* ptr = nullptr;
-                if (cudaMalloc(&ptr, kGemmPartialBytes) == cudaSuccess) c->gemm_partials = static_cast<float*>(ptr);
+                if (cudaMalloc(&ptr, xb::gemm_partial_bytes(c->num_sms)) == cudaSuccess) c->gemm_partials = static_cast<float*>(ptr);
                 else cudaGetLastError();
             } else {
                 c->gemm_partials_tried = false;  // try again on a call that is not being captured
             }
         }
         const int r = xb::gemm_launch(stream, x, proj, num, swiglu, out_f32, m, k, c->status, xb::tc_wait_limit(), xb::tc_x_stage_limit(), c->num_sms,
-                                      c->gemm_partials, c->gemm_partials ? kGemmPartialBytes : 0);
+                                      c->gemm_partials, c->counters);
         if (r == 0) { g_last_path = 3; return XINFER_OK; }
         if (r == -1) return fail_cuda(cudaGetLastError());
     }

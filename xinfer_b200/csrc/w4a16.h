@@ -37,11 +37,13 @@ long long tc_wait_limit();  // clocks after which a device-side wait gives up (t
 int tc_x_stage_limit();     // test hook of tc_set_wait_hooks: first activation stage that is never requested (-1: off)
 
 // Dense GEMM for more than 32 activation rows (prefill chunks) on tcgen05, both operands from shared memory
-// (w4a16_gemm.cu).  One launch per projection; gate and up of the fused MLP share one.
+// (w4a16_gemm.cu).  One launch for all projections that share X; gate and up of the fused MLP are one pair.
 bool gemm_eligible(const void* x, const TcProj* proj, int num, bool swiglu, long long m, long long k, int group_size);
-// `partials` / `partial_bytes`: scratch for the fp32 partial sums of a K split (null: never split).
+// `partials` (gemm_partial_bytes) and `counters` (one zeroed int per SM, left zeroed): scratch for tiles whose K range
+// is cut between CTAs (partials null: tiles are not cut).
+size_t gemm_partial_bytes(int num_sms);
 int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num, bool swiglu, bool out_f32, long long m,
-                long long k, int* status, long long wait_limit, int x_stage_limit, int num_sms, float* partials, size_t partial_bytes);
+                long long k, int* status, long long wait_limit, int x_stage_limit, int num_sms, float* partials, int* counters);
 // Records a message for xinfer_last_cuda_error() on the calling thread (c_api.cu).
 void set_last_error(const char* msg);
 // Programmatic dependent launch (on unless XINFER_PDL=0): kernels are launched with the stream-serialization

@@ -1,29 +1,26 @@
-// INT4-G128 W4A16 GEMM for many activation rows (prefill chunks): Y[M,N] = X[M,K] * W^T (+ bias), M > 32.
+// INT4-G128 W4A16 GEMM for many activation rows (prompts, prefill chunks): Y[M,N] = X[M,K] * W^T (+ bias), M > 32.
 //
 // Replaces, for M = hundreds of rows, what the reference runs its prefill through: the same ops::linear_int4 /
 // linear_int4_fused / mlp_gate_up_swiglu_int4 entry points (src/ops/linear.h:30-139), called with
 // M = chunk length from forward_prefill_chunk (src/targets/qwen3_8/forward.cpp:402-554), where the reference
 // repeats its GEMV row by row.  At M = 512 the contraction is compute-bound (2*M*N*K flops against N*K/2 bytes:
-// ~2000 flop per weight byte), so this kernel is built around the tensor pipe, not around the weight stream:
+// ~2000 flop per weight byte), so this kernel is built around the tensor pipe:
 //
-//   * one CTA per 256 weight rows x 256 activation rows: two tcgen05.mma M = 128 x N = 256 accumulators, 2 x 256
-//     columns = all of tensor memory, accumulated over the whole K (one read-out per tile);
-//   * both operands from shared memory: the activations land by TMA in the canonical 128-byte-swizzled K-major
-//     layout; the packed weights land raw (32 bytes per row and 64-k stage), eight warps - one thread per weight
-//     row - unpack them (lop3 + one subtraction per pair, as in the decode kernel), multiply by the row's group
-//     scale and write the fp16 tiles in the same swizzled layout, so every weight is unpacked once per 256
-//     activation rows;
-//   * three two-slot rings (raw weights, unpacked weights hi + lo, activations) and mbarriers both ways; one elected
-//     thread issues the MMAs (16 per stage) and commits the stage's barriers.
-//
-// Numerics: the accumulators of 256 activation rows live in tensor memory for the whole K, so the group scale
-// cannot be applied to a per-group dot product in registers as the decode kernels do.  Instead scale * weight
-// goes into the MMA as TWO fp16 operands, hi = rn(q * s) and lo = q * s - hi, whose sum is the exact product
-// (an 11-bit by 4-bit product has 15 significant bits; fp16 subnormals aside): two MMAs per k step, products and
-// sums in fp32 in the tensor core.  The result differs from the reference's association only by the order of the
-// fp32 sums, which the tensor core truncates over the whole K (measured against the fp64 oracle, worst element over
-// rms: 3.7e-5 at K = 5120, 1.3e-4 at K = 17408), at twice the tensor work of a single rounded operand, which
-// would be 3e-4 off (1.7e-3 worst element at K = 512) and outside the reference's own 1e-4 absolute test bound.
+//   * a pair of CTAs (tcgen05 cta_group::2) owns 256 weight rows (the MMA's M, 128 per CTA) x up to 256 activation rows
+//     (its N, of which each CTA loads half: one CTA alone would have to pull 64 KB of activations through L2 per 128-k
+//     group, 18 TB/s over the chip at full tensor rate);
+//   * the int4 values go into the MMA as exact fp16 integers.  One 128-k group accumulates into one of two tensor-memory
+//     tiles (2 x 256 columns), and while the tensor core works on the next group eight warps read the finished one back
+//     and fold it into fp32 registers with the group's scale: acc += d * scale, the reference's own association
+//     (src/ops/linear.cpp:239-287).  So every product is exact and every weight costs one MMA (the form before this one
+//     put scale * weight into the MMA as a high and a low fp16 operand, two MMAs per k step, because it kept one
+//     accumulator over all of K: 113 us at M = 512, K = 5120, N = 17408);
+//   * both operands from shared memory: the activations land by TMA in the canonical 128-byte-swizzled K-major layout,
+//     the packed weights land raw (64 bytes per row and group) and four warps, one thread per weight row, unpack them
+//     into the same layout;
+//   * the work of one launch - all tiles of all its projections x K / 128 groups - is dealt to one pair per two SMs, whole
+//     tiles or, where that leaves the last wave too empty, cut evenly.  A tile that straddles a cut is finished by the CTA
+//     that arrives last, which adds the others' fp32 partials in pair order (the result does not depend on who is last).
 //
 // Every wait is bounded (WaitState); a wait that runs out sets the device status word and the CTA leaves through
 // its normal exit, releasing its tensor memory.
@@ -43,356 +40,537 @@
 namespace xb {
 namespace {
 
-constexpr int kGemmUnpackThreads = 256;             // one per weight row of the tile
-constexpr int kGemmThreads = kGemmUnpackThreads + 64;  // + TMA producer warp + MMA warp
-constexpr int kGemmProducerWarp = 8, kGemmMmaWarp = 9;
-constexpr int kGemmTileN = 256;   // weight rows per CTA (two halves of 128)
-constexpr int kGemmTileM = 256;   // activation rows per CTA (the MMA's N)
-constexpr int kGemmStageK = 64;   // k per stage: one 128-byte swizzle row of fp16
-constexpr int kWSlots = 2, kASlots = 2, kXSlots = 2;
-constexpr int kWSlotBytes = kGemmTileN * (kGemmStageK / 2);   // 8 KB of packed weights
-constexpr int kAPartBytes = kGemmTileN * kGemmStageK * 2;     // 32 KB of fp16 weights ...
-constexpr int kASlotBytes = 2 * kAPartBytes;                  // ... twice: the high and the low part of scale * weight
-constexpr int kXSlotBytes = kGemmTileM * kGemmStageK * 2;     // 32 KB of activations
+constexpr int kGemmFoldThreads = 256;    // two per weight row: each folds half of the tile's activation columns
+constexpr int kGemmUnpackThreads = 128;  // one per weight row
+constexpr int kGemmThreads = kGemmFoldThreads + kGemmUnpackThreads + 128;  // + a warpgroup with the two TMA warps and the MMA warp
+constexpr int kGemmUnpackWarp0 = 8, kGemmXWarp = 12, kGemmMmaWarp = 13, kGemmWWarp = 14;
+constexpr int kGemmTileN = 128;   // weight rows of one CTA of a pair (gate/up: 64 of each)
+constexpr int kGemmTileM = 256;   // most activation rows per tile (the MMA's N)
+constexpr int kGemmStageK = 64;   // k per operand slot: one 128-byte swizzle row of fp16
+constexpr int kOpSlots = 5;       // operand ring: a slot holds 64 k of unpacked weights and of activations
+// The packed weights come from HBM, a microsecond and more away: their ring takes what the activations leave of shared
+// memory (6 slots at 256 activation rows), and further groups are pulled into L2 ahead of it.
+constexpr int kWSlotsMax = 10, kWPrefetch = 8;
+constexpr int kWSlotBytes = kGemmTileN * 64;                // 8 KB of packed weights: one 128-k group
+constexpr int kASlotBytes = kGemmTileN * kGemmStageK * 2;   // 16 KB of fp16 weights
 constexpr int kGemmTmemCols = 512;
+constexpr int kGemmParkPitch = 9;
+constexpr int kGemmParkBytes = 2 * 256 * kGemmParkPitch * 4;  // gate/up exchange: [2][fold thread][8 columns]
+constexpr int kGemmMaxProj = 4;
+// Register split of the launch's 512 x 128: the fold keeps 128 sums per thread.
+constexpr int kFoldRegs = 184, kUnpackRegs = 88, kCtrlRegs = 48;
+static_assert(kFoldRegs * 256 + kUnpackRegs * 128 + kCtrlRegs * 128 <= 65536, "register split");
 
 struct GemmCtrl {
-    uint64_t w_full[kWSlots], w_empty[kWSlots];
-    uint64_t a_ready[kASlots], a_empty[kASlots];
-    uint64_t x_full[kXSlots], x_empty[kXSlots];
-    uint64_t d_full;
+    uint64_t w_full[kWSlotsMax], w_empty[kWSlotsMax];
+    uint64_t a_ready[kOpSlots], x_full[kOpSlots], op_empty[kOpSlots];
+    uint64_t d_full[2], d_empty[2];
     uint32_t tmem_base;
+    int last_arrival;
     WaitState ws;
 };
 
-constexpr size_t kGemmSmemBytes = 1024 /* alignment slack */ + kASlots * kASlotBytes + kXSlots * kXSlotBytes +
-                                  kWSlots * kWSlotBytes + sizeof(GemmCtrl);
+// [alignment slack] [A ring] [X ring: kOpSlots x tile_m / 2 x 128 bytes] [W ring] [park] [control]
+constexpr int kGemmSmemBytes = 227 * 1024;
+constexpr int kGemmSmemFixed = 1024 + kOpSlots * kASlotBytes + kGemmParkBytes + static_cast<int>(sizeof(GemmCtrl));
+constexpr int gemm_w_slots(int tile_m) {
+    const int n = (kGemmSmemBytes - kGemmSmemFixed - kOpSlots * tile_m * kGemmStageK) / kWSlotBytes;
+    return n < kWSlotsMax ? n : kWSlotsMax;
+}
+static_assert(gemm_w_slots(kGemmTileM) >= 4, "shared memory");
 
-struct GemmParams {
-    CUtensorMap w_map[2];   // packed weights of the two 128-row halves (the same tensor unless gate/up are paired)
-    CUtensorMap x_map;
-    const __half* scales[2];
+struct GemmProj {
+    const __half* scales[2];  // gate/up: of both
     const float* bias;
     void* y;
     long long ldy;
-    int n;          // output features
-    int m;          // activation rows
-    int groups;     // k / 128
-    int stages;     // k / 64
-    int swiglu;     // half 0 = gate rows, half 1 = up rows of the same 128 features; y = silu(gate) * up
-    int out_f32;
-    long long wait_limit;
-    int* status;
-    int x_stage_limit;  // test hook: activation stages from this index on are never requested (-1: off)
-    float* partials;  // K split over gridDim.z: fp32 partial sums [split][m][n] (summed by a second kernel); else null
+    int n;           // output features
+    int tile0;       // index of its first tile in the launch
 };
 
-// D[tmem] (+)= A[smem descriptor] * B[smem descriptor], kind::f16, one CTA.  Issued by one thread.
-__device__ __forceinline__ void umma_ss_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
+struct GemmParams {
+    CUtensorMap w_map[kGemmMaxProj];  // packed weights of each projection (gate/up: 0 = gate, 1 = up)
+    CUtensorMap x_map;
+    GemmProj proj[kGemmMaxProj];
+    int num_proj;
+    int m;           // activation rows
+    int tile_m;      // activation rows per tile, a multiple of 32
+    int w_slots;     // slots of the packed-weight ring
+    int m_tiles;
+    int groups;      // k / 128
+    long long units;     // tiles * groups
+    int pairs;           // CTA pairs of the launch
+    int whole_tiles;     // cut between tiles only
+    int swiglu;      // rows 0-63 of a CTA = gate, 64-127 = up of the same 64 features; y = silu(gate) * up
+    long long wait_limit;
+    int* status;
+    int x_stage_limit;  // test hook: activation stages (of a CTA) from this index on are never requested (-1: off)
+    float* partials;    // [CTA][2][column][fold thread]: fp32 sums of the tiles a CTA holds a part of
+    int* counters;      // [CTA]: groups of the tile that starts in that pair's range and ends behind it, added up so far
+};
+
+// D[tmem] (+)= A[smem descriptor] * B[smem descriptor], kind::f16, on a CTA pair: A and D rows 0-127 in the even CTA,
+// 128-255 in the odd one; B rows half and half, each CTA's at the descriptor's offset.  Issued by one thread of the even CTA.
+__device__ __forceinline__ void umma_ss_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                 uint32_t accumulate) {
     asm volatile(
         "{\n\t"
         ".reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
         "}"
         :
         : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// Arrives on the mbarrier at this offset in both CTAs of the pair when every MMA issued so far has completed.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+                 "h"(static_cast<uint16_t>(3))
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+}
+// A tiled load into this CTA whose bytes are counted on a barrier of either CTA of the pair (a shared::cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* map, uint32_t cluster_bar, int x, int y, uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
+        " [%0], [%1, {%3, %4}], [%2], %5;"
+        :
+        : "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(cluster_bar), "r"(x), "r"(y), "l"(policy)
+        : "memory");
+}
+// (Release at CTA scope, and the waits acquire at CTA scope: what the arriving warps publish is their own SM's shared and
+// tensor memory, fenced for that SM's tensor core; a release at cluster scope costs the arriving warp half a microsecond.)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+// Barrier of the fold threads that also tells all of them whether any of them has given up: they leave together.
+__device__ __forceinline__ bool fold_barrier_or(bool pred) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, 1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}"
+        : "=r"(r)
+        : "r"(pred ? 1u : 0u), "n"(kGemmFoldThreads)
+        : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ void fold_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kGemmFoldThreads) : "memory"); }
 
-__device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
+__device__ __forceinline__ void store_out(float* y, float v) { *y = v; }
+__device__ __forceinline__ void store_out(__half* y, float v) { *y = __float2half_rn(v); }
+
+// Scales of the groups g .. g + 7 of one weight row (g a multiple of 8; zero behind the last), and on to the next one.
+__device__ __forceinline__ uint4 load_scales(const unsigned short* sp, int g, int groups) {
+    uint4 q = make_uint4(0, 0, 0, 0);
+    if (g >= groups) return q;
+    if ((groups & 7) == 0) return __ldg(reinterpret_cast<const uint4*>(sp + g));
+    uint32_t h[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) h[j] = g + j < groups ? __ldg(sp + g + j) : 0u;
+    return make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, h[6] | h[7] << 16);
 }
-__device__ __forceinline__ uint32_t hfma2_u32(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
+__device__ __forceinline__ void shift_scales(uint4& q) {
+    q.x = __funnelshift_r(q.x, q.y, 16);
+    q.y = __funnelshift_r(q.y, q.z, 16);
+    q.z = __funnelshift_r(q.z, q.w, 16);
+    q.w >>= 16;
 }
-// scale * weight as two fp16 values whose sum is the exact product: hi = rn(q * s), lo = q * s - hi (the fused
-// multiply-add rounds once, and the residual of an 11-bit by 4-bit product fits fp16 exactly, subnormals aside)
-__device__ __forceinline__ void scale_split(uint32_t q2, uint32_t s2, uint32_t& hi, uint32_t& lo) {
-    hi = hmul2_u32(q2, s2);
-    lo = hfma2_u32(q2, s2, hi ^ 0x80008000u);
+
+// First unit of pair c: units cut evenly, or whole tiles only.
+__device__ __forceinline__ long long unit_begin(const GemmParams& p, long long c) {
+    if (p.whole_tiles) {
+        const long long tiles = p.units / p.groups;
+        return c * tiles / p.pairs * p.groups;
+    }
+    return c * p.units / p.pairs;
+}
+// The pair whose range holds unit u.
+__device__ __forceinline__ int unit_owner(const GemmParams& p, long long u) {
+    int c = static_cast<int>(u * p.pairs / p.units);
+    while (c + 1 < p.pairs && unit_begin(p, c + 1) <= u) ++c;
+    while (c > 0 && unit_begin(p, c) > u) --c;
+    return c;
+}
+__device__ __forceinline__ int proj_of_tile(const GemmParams& p, int tile) {
+    int i = 0;
+    while (i + 1 < p.num_proj && tile >= p.proj[i + 1].tile0) ++i;
+    return i;
 }
 
 template <typename OutT>
-__device__ __forceinline__ void store_out(void* y, long long off, float v) {
-    if constexpr (sizeof(OutT) == 4) static_cast<float*>(y)[off] = v;
-    else static_cast<__half*>(y)[off] = __float2half_rn(v);
-}
-
-template <typename OutT>
-__global__ void __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __grid_constant__ GemmParams p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __grid_constant__ GemmParams p) {
     extern __shared__ uint8_t gemm_smem_raw[];
     // the swizzled operand tiles want 1024-byte alignment
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint8_t* a_ring = smem;
-    uint8_t* x_ring = a_ring + kASlots * kASlotBytes;
-    uint8_t* w_ring = x_ring + kXSlots * kXSlotBytes;
-    GemmCtrl* ctrl = reinterpret_cast<GemmCtrl*>(w_ring + kWSlots * kWSlotBytes);
+    uint8_t* x_ring = a_ring + kOpSlots * kASlotBytes;
+    const uint32_t x_slot_bytes = static_cast<uint32_t>(p.tile_m) * kGemmStageK;  // this CTA's half of the rows
+    uint8_t* w_ring = x_ring + kOpSlots * x_slot_bytes;
+    const int w_slots = p.w_slots;
+    float* park = reinterpret_cast<float*>(w_ring + w_slots * kWSlotBytes);
+    GemmCtrl* ctrl = reinterpret_cast<GemmCtrl*>(w_ring + w_slots * kWSlotBytes + kGemmParkBytes);
 
     const int tid = threadIdx.x;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int lane = tid & 31;
+    const uint32_t rank = cluster_ctarank();  // the even CTA issues the pair's MMAs
     volatile WaitState* ws = &ctrl->ws;
     griddep_launch_dependents();
 
     if (tid == 0) {
-        for (int i = 0; i < kWSlots; ++i) { mbar_init(smem_u32(&ctrl->w_full[i]), 1); mbar_init(smem_u32(&ctrl->w_empty[i]), kGemmUnpackThreads / 32); }
-        for (int i = 0; i < kASlots; ++i) { mbar_init(smem_u32(&ctrl->a_ready[i]), kGemmUnpackThreads / 32); mbar_init(smem_u32(&ctrl->a_empty[i]), 1); }
-        for (int i = 0; i < kXSlots; ++i) { mbar_init(smem_u32(&ctrl->x_full[i]), 1); mbar_init(smem_u32(&ctrl->x_empty[i]), 1); }
-        mbar_init(smem_u32(&ctrl->d_full), 1);
+        for (int i = 0; i < w_slots; ++i) { mbar_init(smem_u32(&ctrl->w_full[i]), 1); mbar_init(smem_u32(&ctrl->w_empty[i]), kGemmUnpackThreads / 32); }
+        for (int i = 0; i < kOpSlots; ++i) {
+            mbar_init(smem_u32(&ctrl->a_ready[i]), 2 * kGemmUnpackThreads / 32);
+            mbar_init(smem_u32(&ctrl->x_full[i]), 1);
+            mbar_init(smem_u32(&ctrl->op_empty[i]), 1);
+        }
+        for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&ctrl->d_full[i]), 1); mbar_init(smem_u32(&ctrl->d_empty[i]), 2 * kGemmFoldThreads / 32); }
         ctrl->ws.abort_flag = 0;
         ctrl->ws.dep_ready = 0;
         ctrl->ws.limit = p.wait_limit;
         mbar_fence_init();
     }
-    if (warp == kGemmMmaWarp) {
-        tmem_alloc(smem_u32(&ctrl->tmem_base), kGemmTmemCols);
-        tmem_relinquish();
-    }
+    if (warp == kGemmMmaWarp) tmem_alloc_pair(smem_u32(&ctrl->tmem_base), kGemmTmemCols);
     tc_fence_before_sync();
     __syncthreads();
+    cluster_sync_all();  // the other CTA's barriers are initialised too
     tc_fence_after_sync();
     const uint32_t tmem_base = ctrl->tmem_base;
 
-    // this CTA's stages: all of K, or its share when K is split over gridDim.z
-    const int s_begin = static_cast<int>(static_cast<long long>(blockIdx.z) * p.stages / gridDim.z);
-    const int s_end = static_cast<int>(static_cast<long long>(blockIdx.z + 1) * p.stages / gridDim.z);
-    const int S = s_end - s_begin;  // ring slots and phases count from the CTA's first stage
-    const int tile_n = blockIdx.x, m0 = blockIdx.y * kGemmTileM;
-    // first weight row of each half
-    const int row_base0 = p.swiglu ? tile_n * 128 : tile_n * kGemmTileN;
-    const int row_base1 = p.swiglu ? tile_n * 128 : tile_n * kGemmTileN + 128;
+    // this pair's units (tile, 128-k group), tile-major; ring slots and phases count from its first unit
+    const int pair = static_cast<int>(blockIdx.x >> 1);
+    const long long u0 = unit_begin(p, pair), u1 = unit_begin(p, static_cast<long long>(pair) + 1);
+    const int U = static_cast<int>(u1 - u0);
+    const int first_tile = static_cast<int>(u0 / p.groups), first_group = static_cast<int>(u0 - static_cast<long long>(first_tile) * p.groups);
 
-    if (warp == kGemmProducerWarp) {
-        // ------------------------------------------------------------------ TMA producer (whole warp waits, one lane issues)
-        const bool leader = elect_one_sync();
-        if (leader) {
-            tma_prefetch_desc(&p.w_map[0]);
-            tma_prefetch_desc(&p.w_map[1]);
-            tma_prefetch_desc(&p.x_map);
-        }
-        const uint64_t pol_w = l2_policy_evict_first();
-        const uint64_t pol_x = l2_policy_evict_last();
-        auto issue_w = [&](int s) {
-            const uint32_t slot = static_cast<uint32_t>(s % kWSlots);
-            const uint32_t full = smem_u32(&ctrl->w_full[slot]);
-            const uint32_t dst = smem_u32(w_ring) + slot * kWSlotBytes;
-            if (leader) {
-                mbar_arrive_expect_tx(full, kWSlotBytes);
-                tma_load_2d(dst, &p.w_map[0], full, (s_begin + s) * (kGemmStageK / 2), row_base0, pol_w);
-                tma_load_2d(dst + kWSlotBytes / 2, &p.w_map[1], full, (s_begin + s) * (kGemmStageK / 2), row_base1, pol_w);
-            }
-        };
-        auto issue_x = [&](int s) {
-            const uint32_t slot = static_cast<uint32_t>(s % kXSlots);
-            const uint32_t full = smem_u32(&ctrl->x_full[slot]);
-            if (leader) {
-                mbar_arrive_expect_tx(full, kXSlotBytes);
-                tma_load_2d(smem_u32(x_ring) + slot * kXSlotBytes, &p.x_map, full, (s_begin + s) * kGemmStageK, m0, pol_x);
-            }
-        };
-        // the weights do not depend on the kernel in front of this one, the activations do
-        // (test hook: with x_stage_limit >= 0 the activation stages from that index on are never requested, so the
-        // waits for them run out and the kernel leaves through its abort path)
-        const int SX = (p.x_stage_limit >= 0 && p.x_stage_limit < S) ? p.x_stage_limit : S;
-        int nw = 0, nx = 0;
-        for (; nw < kWSlots && nw < S; ++nw) issue_w(nw);
-        griddep_wait();
-        if (leader) ws->dep_ready = 1;
-        for (; nx < kXSlots && nx < SX; ++nx) issue_x(nx);
-        bool ok = true;
-        while (ok && (nw < S || nx < SX)) {
-            if (nw < S) {
-                ok = mbar_wait_parked(smem_u32(&ctrl->w_empty[nw % kWSlots]), ((nw / kWSlots) & 1u) ^ 1u, ws);
-                if (ok) issue_w(nw++);
-            }
-            if (ok && nx < SX) {
-                ok = mbar_wait_parked(smem_u32(&ctrl->x_empty[nx % kXSlots]), ((nx / kXSlots) & 1u) ^ 1u, ws);
-                if (ok) issue_x(nx++);
-            }
-        }
-        if (ws->abort_flag) {
-            // give the copies still in flight a bounded chance to land before the CTA exits
-            const long long t0 = clock64();
-            for (int i = 0; i < kWSlots && i < nw; ++i) {
-                const int k = nw - 1 - i;
-                while (!mbar_try_wait(smem_u32(&ctrl->w_full[k % kWSlots]), (k / kWSlots) & 1u) && clock64() - t0 < p.wait_limit / 8) {
-                }
-            }
-            for (int i = 0; i < kXSlots && i < nx; ++i) {
-                const int k = nx - 1 - i;
-                while (!mbar_try_wait(smem_u32(&ctrl->x_full[k % kXSlots]), (k / kXSlots) & 1u) && clock64() - t0 < p.wait_limit / 8) {
-                }
-            }
-        }
-        __syncwarp();
-    } else if (warp == kGemmMmaWarp) {
-        // ------------------------------------------------------------------ MMA issuer
-        const bool leader = elect_one_sync();
-        constexpr uint32_t idesc = umma_idesc_f16_f32(128, kGemmTileM);
-        // K-major, 128-byte swizzle: rows of 64 k, 8-row groups 1024 bytes apart; descriptor version 1
-        constexpr uint32_t desc_hi = ((1024u >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);
-        constexpr uint32_t desc_lo_const = 1u << 16;
-        const uint32_t a_lo0 = (smem_u32(a_ring) >> 4) & 0x3FFFu;
-        const uint32_t x_lo0 = (smem_u32(x_ring) >> 4) & 0x3FFFu;
-        bool ok = true;
-        for (int s = 0; s < S && ok; ++s) {
-            const uint32_t as = static_cast<uint32_t>(s % kASlots), xs = static_cast<uint32_t>(s % kXSlots);
-            if (!mbar_wait_parked(smem_u32(&ctrl->a_ready[as]), (s / kASlots) & 1u, ws)) break;
-            if (!mbar_wait_parked(smem_u32(&ctrl->x_full[xs]), (s / kXSlots) & 1u, ws)) break;
-            tc_fence_after_sync();
-            if (leader) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const uint32_t ahi = desc_lo_const | (a_lo0 + ((as * kASlotBytes + h * (kAPartBytes / 2) + i * 32) >> 4));
-                        const uint32_t alo = ahi + (kAPartBytes >> 4);
-                        const uint32_t xlo = desc_lo_const | (x_lo0 + ((xs * kXSlotBytes + i * 32) >> 4));
-                        const uint64_t bdesc = (static_cast<uint64_t>(desc_hi) << 32) | xlo;
-                        umma_ss_f16(tmem_base + h * 256, (static_cast<uint64_t>(desc_hi) << 32) | ahi, bdesc, idesc, (s > 0 || i > 0) ? 1u : 0u);
-                        umma_ss_f16(tmem_base + h * 256, (static_cast<uint64_t>(desc_hi) << 32) | alo, bdesc, idesc, 1u);
+    if (warp >= kGemmXWarp) {
+        setmaxnreg_dec<kCtrlRegs>();
+        if (warp == kGemmWWarp) {
+            // -------------------------------------------------------------- TMA: packed weights (whole warp waits, one lane issues)
+            // They do not depend on the kernel in front of this one.
+            const bool leader = elect_one_sync();
+            if (leader)
+                for (int i = 0; i < (p.swiglu ? 2 : p.num_proj); ++i) tma_prefetch_desc(&p.w_map[i]);
+            const uint64_t pol_w = l2_policy_evict_first();
+            // two cursors into the unit list: the one that loads, and one that pulls into L2 ahead of it
+            struct Cursor { int tile, group; } at = {first_tile, first_group}, ahead = at;
+            auto visit = [&](Cursor& c, bool load, uint32_t dst, uint32_t full) {
+                const int pr = proj_of_tile(p, c.tile);
+                const int rel = c.tile - p.proj[pr].tile0, nt2 = rel / p.m_tiles, nt = nt2 * 2 + static_cast<int>(rank);
+                if (leader) {
+                    if (load) {
+                        if (p.swiglu) {
+                            tma_load_2d(dst, &p.w_map[0], full, c.group * 64, nt * 64, pol_w);
+                            tma_load_2d(dst + kWSlotBytes / 2, &p.w_map[1], full, c.group * 64, nt * 64, pol_w);
+                        } else {
+                            tma_load_2d(dst, &p.w_map[pr], full, c.group * 64, nt * kGemmTileN, pol_w);
+                        }
+                    } else if (rel == nt2 * p.m_tiles) {  // the tiles over further activation rows find them there
+                        if (p.swiglu) {
+                            tma_prefetch_l2_2d(&p.w_map[0], c.group * 64, nt * 64);
+                            tma_prefetch_l2_2d(&p.w_map[1], c.group * 64, nt * 64);
+                        } else {
+                            tma_prefetch_l2_2d(&p.w_map[pr], c.group * 64, nt * kGemmTileN);
+                        }
                     }
                 }
-                umma_commit(smem_u32(&ctrl->a_empty[as]));
-                umma_commit(smem_u32(&ctrl->x_empty[xs]));
-                if (s == S - 1) umma_commit(smem_u32(&ctrl->d_full));
+                if (++c.group == p.groups) { c.group = 0; ++c.tile; }
+            };
+            int slot = 0, n = 0, na = 0;
+            uint32_t phase = 1;  // parity under which a slot's first use passes at once
+            for (; n < U; ++n) {
+                const uint32_t full = smem_u32(&ctrl->w_full[slot]);
+                if (!mbar_wait_parked(smem_u32(&ctrl->w_empty[slot]), phase, ws)) break;
+                if (leader) mbar_arrive_expect_tx(full, kWSlotBytes);
+                visit(at, true, smem_u32(w_ring) + slot * kWSlotBytes, full);
+                if (++slot == w_slots) { slot = 0; phase ^= 1u; }
+                if (n + 1 >= w_slots) {
+                    if (na <= n) { na = n + 1; ahead = at; }
+                    for (; na < U && na <= n + kWPrefetch; ++na) visit(ahead, false, 0, 0);
+                }
+            }
+            if (ws->abort_flag) {
+                // give the copies still in flight a bounded chance to land before the CTA exits
+                const long long t0 = clock64();
+                for (int i = 0; i < w_slots && i < n; ++i) {
+                    const int k = n - 1 - i;
+                    while (!mbar_try_wait(smem_u32(&ctrl->w_full[k % w_slots]), (k / w_slots) & 1u) && clock64() - t0 < p.wait_limit / 8) {
+                    }
+                }
             }
             __syncwarp();
+        } else if (warp == kGemmXWarp) {
+            // -------------------------------------------------------------- TMA: activations
+            const bool leader = elect_one_sync();
+            if (leader) tma_prefetch_desc(&p.x_map);
+            const uint64_t pol_x = l2_policy_evict_last();
+            int tile = first_tile, group = first_group;
+            const int S = 2 * U;  // 64-k stages, two per unit
+            const int SX = (p.x_stage_limit >= 0 && p.x_stage_limit < S) ? p.x_stage_limit : S;
+            griddep_wait();
+            if (leader) ws->dep_ready = 1;
+            int nx = 0, slot = 0;
+            uint32_t phase = 1;
+            for (; nx < SX; ++nx) {
+                if (!mbar_wait_parked(smem_u32(&ctrl->op_empty[slot]), phase, ws)) break;
+                const uint32_t full = smem_u32(&ctrl->x_full[slot]);
+                const int pr = proj_of_tile(p, tile);
+                const int m0 = ((tile - p.proj[pr].tile0) % p.m_tiles) * p.tile_m + static_cast<int>(rank) * (p.tile_m >> 1);
+                if (leader) {
+                    // both halves of the rows are counted on the even CTA's barrier, where the MMAs are issued
+                    if (rank == 0) mbar_arrive_expect_tx(full, 2 * x_slot_bytes);
+                    tma_load_2d_pair(smem_u32(x_ring) + slot * x_slot_bytes, &p.x_map, mapa_shared_cluster(full, 0),
+                                     group * 128 + (nx & 1) * kGemmStageK, m0, pol_x);
+                }
+                if ((nx & 1) && ++group == p.groups) { group = 0; ++tile; }
+                if (++slot == kOpSlots) { slot = 0; phase ^= 1u; }
+            }
+            if (ws->abort_flag) {
+                const long long t0 = clock64();
+                for (int i = 0; i < kOpSlots && i < nx; ++i) {
+                    const int k = nx - 1 - i;
+                    while (!mbar_try_wait(smem_u32(&ctrl->x_full[k % kOpSlots]), (k / kOpSlots) & 1u) && clock64() - t0 < p.wait_limit / 8) {
+                    }
+                }
+            }
+            __syncwarp();
+        } else if (warp == kGemmMmaWarp && rank == 0) {
+            // -------------------------------------------------------------- MMA issuer of the pair
+            const bool leader = elect_one_sync();
+            const uint32_t idesc = umma_idesc_f16_f32(256, 0) | (static_cast<uint32_t>(p.tile_m >> 3) << 17);
+            // K-major, 128-byte swizzle: rows of 64 k, 8-row groups 1024 bytes apart; descriptor version 1
+            constexpr uint32_t desc_hi = ((1024u >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);
+            constexpr uint32_t desc_lo_const = 1u << 16;
+            const uint32_t a_lo0 = (smem_u32(a_ring) >> 4) & 0x3FFFu;
+            const uint32_t x_lo0 = (smem_u32(x_ring) >> 4) & 0x3FFFu;
+            bool ok = true;
+            uint32_t slot = 0, phase = 0;
+            for (int i = 0; i < U && ok; ++i) {
+                const uint32_t buf = static_cast<uint32_t>(i & 1);
+                if (i >= 2 && !mbar_wait_parked(smem_u32(&ctrl->d_empty[buf]), ((i >> 1) & 1u) ^ 1u, ws)) break;
+#pragma unroll 1
+                for (int half = 0; half < 2; ++half) {
+                    ok = mbar_wait_parked(smem_u32(&ctrl->x_full[slot]), phase, ws) &&
+                         mbar_wait_parked(smem_u32(&ctrl->a_ready[slot]), phase, ws);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    if (leader) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const uint32_t alo = desc_lo_const | (a_lo0 + ((slot * kASlotBytes + k * 32) >> 4));
+                            const uint32_t xlo = desc_lo_const | (x_lo0 + ((slot * x_slot_bytes + k * 32) >> 4));
+                            umma_ss_f16_pair(tmem_base + buf * 256, (static_cast<uint64_t>(desc_hi) << 32) | alo,
+                                             (static_cast<uint64_t>(desc_hi) << 32) | xlo, idesc, (half > 0 || k > 0) ? 1u : 0u);
+                        }
+                        umma_commit_pair(smem_u32(&ctrl->op_empty[slot]));
+                        if (half) umma_commit_pair(smem_u32(&ctrl->d_full[buf]));
+                    }
+                    __syncwarp();
+                    if (++slot == kOpSlots) { slot = 0; phase ^= 1u; }
+                }
+            }
+        }
+    } else if (warp >= kGemmUnpackWarp0) {
+        // ------------------------------------------------------------------ unpack: one thread per weight row of the tile
+        setmaxnreg_dec<kUnpackRegs>();
+        const int r = tid - kGemmFoldThreads;
+        // raw rows of 64 bytes under the 64-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ ((r >> 1) & 3)
+        const uint32_t w_row = static_cast<uint32_t>(r) * 64, w_sw = static_cast<uint32_t>((r >> 1) & 3);
+        const uint32_t a_row = static_cast<uint32_t>((r >> 3) * 1024 + (r & 7) * 128), a_sw = static_cast<uint32_t>(r & 7);
+        bool ok = true;
+        int wslot = 0, aslot = 0;
+        uint32_t w_phase = 0, a_phase = 1;
+        for (int i = 0; i < U && ok; ++i) {
+            if (!mbar_wait(smem_u32(&ctrl->w_full[wslot]), w_phase, ws)) break;
+            const uint32_t wsrc = smem_u32(w_ring) + wslot * kWSlotBytes + w_row;
+            uint4 v[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) v[c] = lds128(wsrc + ((static_cast<uint32_t>(c) ^ w_sw) << 4));
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                if (!mbar_wait(smem_u32(&ctrl->op_empty[aslot]), a_phase, ws)) { ok = false; break; }
+                const uint32_t adst = smem_u32(a_ring) + aslot * kASlotBytes + a_row;
+                const uint32_t words[8] = {v[2 * half].x, v[2 * half].y, v[2 * half].z, v[2 * half].w,
+                                           v[2 * half + 1].x, v[2 * half + 1].y, v[2 * half + 1].z, v[2 * half + 1].w};
+#pragma unroll
+                for (int w = 0; w < 8; ++w) {
+                    uint32_t q[4];
+                    dequant_word(words[w], q);  // (k0,k4) (k1,k5) (k2,k6) (k3,k7)
+                    uint4 o;
+                    o.x = prmt(q[0], q[1], 0x5410u);  // (k0,k1)
+                    o.y = prmt(q[2], q[3], 0x5410u);  // (k2,k3)
+                    o.z = prmt(q[0], q[1], 0x7632u);  // (k4,k5)
+                    o.w = prmt(q[2], q[3], 0x7632u);  // (k6,k7)
+                    sts128(adst + ((static_cast<uint32_t>(w) ^ a_sw) << 4), o);
+                }
+                fence_proxy_async_smem();  // the tensor core reads this tile through the async proxy
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive_cluster(mapa_shared_cluster(smem_u32(&ctrl->a_ready[aslot]), 0));
+                    if (half) mbar_arrive(smem_u32(&ctrl->w_empty[wslot]));
+                }
+                if (++aslot == kOpSlots) { aslot = 0; a_phase ^= 1u; }
+            }
+            if (++wslot == w_slots) { wslot = 0; w_phase ^= 1u; }
         }
     } else {
-        // ------------------------------------------------------------------ unpack (then epilogue): one thread per weight row
-        const int h = tid >> 7, r = tid & 127;
-        const int row = (h ? row_base1 : row_base0) + r;
-        const bool valid = row < p.n;
-        const unsigned short* sp = reinterpret_cast<const unsigned short*>(p.scales[h]) + static_cast<long long>(valid ? row : 0) * p.groups;
-        const uint32_t w_off = static_cast<uint32_t>((h * 128 + r) * (kGemmStageK / 2));
-        const uint32_t a_off = static_cast<uint32_t>(h * (kAPartBytes / 2) + (r >> 3) * 1024 + (r & 7) * 128);
-        const uint32_t sw = static_cast<uint32_t>(r & 7);
-        bool ok = true;
-        // the scale of the stage's 128-k group (two stages per group), fetched one stage ahead
-        uint32_t q_next = (valid && S > 0) ? static_cast<uint32_t>(__ldg(sp + (s_begin >> 1))) : 0u;
-        for (int s = 0; s < S; ++s) {
-            const uint32_t sc2 = q_next | (q_next << 16);
-            if (s + 1 < S) q_next = valid ? static_cast<uint32_t>(__ldg(sp + ((s_begin + s + 1) >> 1))) : 0u;
-            const uint32_t wslot = static_cast<uint32_t>(s % kWSlots), aslot = static_cast<uint32_t>(s % kASlots);
-            if (!mbar_wait(smem_u32(&ctrl->w_full[wslot]), (s / kWSlots) & 1u, ws)) { ok = false; break; }
-            const uint32_t wsrc = smem_u32(w_ring) + wslot * kWSlotBytes + w_off;
-            const uint4 v0 = lds128(wsrc), v1 = lds128(wsrc + 16);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&ctrl->w_empty[wslot]));
-            if (s >= kASlots) {
-                if (!mbar_wait(smem_u32(&ctrl->a_empty[aslot]), ((s / kASlots) & 1u) ^ 1u, ws)) { ok = false; break; }
-            }
-            const uint32_t adst = smem_u32(a_ring) + aslot * kASlotBytes + a_off;
-            const uint32_t words[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        // ------------------------------------------------------------------ fold, then write: two threads per weight row
+        setmaxnreg_inc<kFoldRegs>();
+        const int r = tid & 127, ch = tid >> 7;          // tile row, column half
+        const int half_cols = p.tile_m >> 1;             // a multiple of 16
+        const uint32_t d_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(ch * half_cols);
+        const bool up_row = p.swiglu && r >= 64;
+        float acc[kGemmTileM / 2];
+        int i = 0, tile = first_tile, group = first_group;
+        bool dead = false;
+        while (i < U) {
+            // one tile, or the part of it that lies in this pair's range
+            const int pr = proj_of_tile(p, tile);
+            const GemmProj& pj = p.proj[pr];
+            const int rel = tile - pj.tile0, nt = rel / p.m_tiles * 2 + static_cast<int>(rank), m0 = (rel % p.m_tiles) * p.tile_m;
+            const int row = p.swiglu ? nt * 64 + (r & 63) : nt * kGemmTileN + r;
+            const bool valid = row < pj.n;
+            const unsigned short* sp = reinterpret_cast<const unsigned short*>(pj.scales[up_row ? 1 : 0]) +
+                                       static_cast<long long>(valid ? row : 0) * p.groups;
+            const int seg_begin = group, seg_end = (U - i < p.groups - group) ? group + (U - i) : p.groups;
 #pragma unroll
-            for (int w = 0; w < 8; ++w) {
-                uint32_t q[4];
-                dequant_word(words[w], q);  // (k0,k4) (k1,k5) (k2,k6) (k3,k7)
-                uint4 hi, lo;
-                scale_split(prmt(q[0], q[1], 0x5410u), sc2, hi.x, lo.x);  // (k0,k1)
-                scale_split(prmt(q[2], q[3], 0x5410u), sc2, hi.y, lo.y);  // (k2,k3)
-                scale_split(prmt(q[0], q[1], 0x7632u), sc2, hi.z, lo.z);  // (k4,k5)
-                scale_split(prmt(q[2], q[3], 0x7632u), sc2, hi.w, lo.w);  // (k6,k7)
-                const uint32_t at = adst + ((static_cast<uint32_t>(w) ^ sw) << 4);
-                sts128(at, hi);
-                sts128(at + kAPartBytes, lo);
+            for (int j = 0; j < kGemmTileM / 2; ++j) acc[j] = 0.f;
+            // scales eight groups at a time, a block of eight ahead of its use (one group ahead, their latency is the loop's)
+            uint4 q_cur = load_scales(sp, seg_begin & ~7, p.groups), q_next = load_scales(sp, (seg_begin & ~7) + 8, p.groups);
+            for (int j = 0; j < (seg_begin & 7); ++j) shift_scales(q_cur);
+            for (; group < seg_end; ++group, ++i) {
+                const float sc = __half2float(__ushort_as_half(static_cast<unsigned short>(q_cur.x & 0xFFFFu)));
+                shift_scales(q_cur);
+                if ((group & 7) == 7) {
+                    q_cur = q_next;
+                    q_next = load_scales(sp, group + 9, p.groups);
+                }
+                const uint32_t buf = static_cast<uint32_t>(i & 1);
+                if (dead || !mbar_wait_parked(smem_u32(&ctrl->d_full[buf]), (i >> 1) & 1u, ws)) { dead = true; continue; }
+                tc_fence_after_sync();
+                const uint32_t src = d_addr + buf * 256;
+                // 32 columns a read (one tcgen05.ld; with two of 16 the whole kernel is 20 % slower at M = 512).  A tile of
+                // fewer columns reads on into columns that are allocated and not used.
+#pragma unroll
+                for (int c = 0; c < kGemmTileM / 64; ++c) {
+                    if (c * 32 < half_cols) {
+                        uint32_t d[32];
+                        tmem_ld32(src + c * 32, d);
+                        tmem_wait_ld();
+                        if (c * 32 + 32 >= half_cols) {  // the last read of this group: the MMA warp may have the columns
+                            tc_fence_before_sync();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_cluster(mapa_shared_cluster(smem_u32(&ctrl->d_empty[buf]), 0));
+                        }
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) acc[c * 32 + j] = fmaf(__uint_as_float(d[j]), sc, acc[c * 32 + j]);
+                    }
+                }
             }
-            fence_proxy_async_smem();  // the tensor core reads this tile through the async proxy
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&ctrl->a_ready[aslot]));
-        }
+            if (fold_barrier_or(dead || ws->abort_flag != 0)) break;
 
-        // ---------------------------------------------------------------- epilogue: this row's 256 sums
-        if (ok) ok = mbar_wait(smem_u32(&ctrl->d_full), 0u, ws);
-        // The read-out is taken by all 256 threads or by none (its gate/up exchange has barriers of its own): a wait
-        // that gave up anywhere has set the abort flag before returning, and every thread arrives here.
-        asm volatile("bar.sync 1, %0;" ::"n"(kGemmUnpackThreads) : "memory");
-        if (!ws->abort_flag) {
-            tc_fence_after_sync();
-            const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
-            const float bias = (valid && p.bias && !p.swiglu) ? p.bias[row] : 0.f;
-            if (!p.swiglu) {
-#pragma unroll 1
-                for (int c = 0; c < kGemmTileM / 16; ++c) {
-                    uint32_t d[16];
-                    tmem_ld16(tmem_base + lane_sel + h * 256 + c * 16, d);
-                    tmem_wait_ld();
-                    if (valid) {
-                        if (p.partials) {
-                            float* ws_out = p.partials + static_cast<long long>(blockIdx.z) * p.m * p.n;
+            // ------------------------------------------------------------ a straddling tile: the last CTA to arrive finishes it
+            int c_first = 0, c_last = 0;
+            const bool split = seg_begin > 0 || seg_end < p.groups;
+            if (split) {
+                const long long tu = static_cast<long long>(tile) * p.groups;
+                c_first = unit_owner(p, tu);
+                c_last = unit_owner(p, tu + p.groups - 1);
+                const size_t slot_floats = static_cast<size_t>(kGemmTileN) * kGemmTileM;
+                float* mine = p.partials + (static_cast<size_t>(blockIdx.x) * 2 + (seg_begin > 0 ? 0 : 1)) * slot_floats + tid;
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                const int m = m0 + c * 16 + j;
-                                if (m < p.m) ws_out[static_cast<long long>(m) * p.n + row] = __uint_as_float(d[j]);
+                for (int j = 0; j < kGemmTileM / 2; ++j)
+                    if (j < half_cols) __stcg(mine + j * kGemmFoldThreads, acc[j]);
+                __threadfence();
+                fold_barrier();
+                if (tid == 0) {
+                    const int n = seg_end - seg_begin, old = atomicAdd(p.counters + c_first * 2 + rank, n);
+                    const bool last = old + n == p.groups;
+                    if (last) p.counters[c_first * 2 + rank] = 0;  // as the next launch expects it
+                    ctrl->last_arrival = last ? 1 : 0;
+                    __threadfence();
+                }
+                fold_barrier();
+            }
+            if (!split || ctrl->last_arrival) {
+                const float bias = (valid && pj.bias && !p.swiglu) ? pj.bias[row] : 0.f;
+                if (split) __threadfence();
+#pragma unroll
+                for (int c = 0; c < kGemmTileM / 32; ++c) {
+                    if (c * 16 < half_cols) {
+                        if (split) {
+                            float sum[16];
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) sum[j] = 0.f;
+                            for (int o = c_first; o <= c_last; ++o) {
+                                if (o == pair) {
+#pragma unroll
+                                    for (int j = 0; j < 16; ++j) sum[j] += acc[c * 16 + j];
+                                } else {
+                                    // a contributor's part of this tile: slot 1 if the tile starts in its range, else slot 0
+                                    const float* src = p.partials +
+                                                       ((static_cast<size_t>(o) * 2 + rank) * 2 + (o == c_first ? 1 : 0)) * kGemmTileN * kGemmTileM +
+                                                       static_cast<size_t>(c) * 16 * kGemmFoldThreads + tid;
+#pragma unroll
+                                    for (int j = 0; j < 16; ++j) sum[j] += __ldcg(src + j * kGemmFoldThreads);
+                                }
+                            }
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) acc[c * 16 + j] = sum[j];
+                        }
+                        const int mc = m0 + ch * half_cols + c * 16;
+                        OutT* out = static_cast<OutT*>(pj.y) + static_cast<long long>(mc) * pj.ldy + row;
+                        if (!p.swiglu) {
+                            if (valid) {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j, out += pj.ldy)
+                                    if (mc + j < p.m) store_out(out, acc[c * 16 + j] + bias);
                             }
                         } else {
+                            // Gate and up of one feature sit in different warps, which trade halves of the 16 columns: the
+                            // gate thread finishes columns 0-7, the up thread 8-15.  Two buffers, one barrier a chunk.
+                            float* buf = park + (c & 1) * (kGemmParkBytes / 8);
+                            float* mine = buf + (ch * 128 + r) * kGemmParkPitch;
+                            const float* theirs = buf + (ch * 128 + (r ^ 64)) * kGemmParkPitch;
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                const int m = m0 + c * 16 + j;
-                                if (m < p.m) store_out<OutT>(p.y, static_cast<long long>(m) * p.ldy + row, __uint_as_float(d[j]) + bias);
+                            for (int j = 0; j < 8; ++j) mine[j] = up_row ? acc[c * 16 + j] : acc[c * 16 + 8 + j];
+                            fold_barrier();
+                            if (up_row) out += 8 * pj.ldy;
+                            if (valid) {
+#pragma unroll
+                                for (int j = 0; j < 8; ++j, out += pj.ldy) {
+                                    const float g = up_row ? theirs[j] : acc[c * 16 + j], u = up_row ? acc[c * 16 + 8 + j] : theirs[j];
+                                    if (mc + j + (up_row ? 8 : 0) < p.m) store_out(out, (g / (1.0f + expf(-g))) * u);
+                                }
                             }
                         }
                     }
                 }
-            } else {
-                // gate (half 0) and up (half 1) of one feature sit in different warps: the up half parks its values in
-                // shared memory (the activation ring, idle by now), 16 columns at a time
-                float* park = reinterpret_cast<float*>(x_ring);  // [128 rows][17]
-#pragma unroll 1
-                for (int c = 0; c < kGemmTileM / 16; ++c) {
-                    uint32_t d[16];
-                    tmem_ld16(tmem_base + lane_sel + h * 256 + c * 16, d);
-                    tmem_wait_ld();
-                    if (h == 1) {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) park[r * 17 + j] = __uint_as_float(d[j]);
-                    }
-                    asm volatile("bar.sync 1, %0;" ::"n"(kGemmUnpackThreads) : "memory");
-                    if (h == 0 && valid) {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const int m = m0 + c * 16 + j;
-                            const float g = __uint_as_float(d[j]), u = park[r * 17 + j];
-                            if (m < p.m) store_out<OutT>(p.y, static_cast<long long>(m) * p.ldy + row, (g / (1.0f + expf(-g))) * u);
-                        }
-                    }
-                    asm volatile("bar.sync 1, %0;" ::"n"(kGemmUnpackThreads) : "memory");
-                }
             }
+            if (group == p.groups) { group = 0; ++tile; }
         }
     }
 
     // ---------------------------------------------------------------------- teardown
     tc_fence_before_sync();
     __syncthreads();
+    cluster_sync_all();  // the pair's MMAs read both CTAs' shared memory, and each arrives on the other's barriers
     if (tid == 0 && ctrl->ws.abort_flag && p.status) atomicExch(p.status, kStatusWaitTimeout);
     if (warp == kGemmMmaWarp) {
         __syncwarp();
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, kGemmTmemCols);
-    }
-}
-
-// Sums the K splits in split order (deterministic), adds the bias and converts.
-template <typename OutT>
-__global__ void __launch_bounds__(256) gemm_splitk_reduce_kernel(void* y, long long ldy, const float* partials, int splits,
-                                                                 int m, int n, const float* bias) {
-    griddep_prologue();
-    const long long total = static_cast<long long>(m) * n;
-    for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        float sum = 0.f;
-        for (int z = 0; z < splits; ++z) sum += __ldcg(partials + z * total + i);
-        const int row = static_cast<int>(i / n), col = static_cast<int>(i - static_cast<long long>(row) * n);
-        if (bias) sum += bias[col];
-        store_out<OutT>(y, static_cast<long long>(row) * ldy + col, sum);
+        tmem_dealloc_pair(tmem_base, kGemmTmemCols);
     }
 }
 
@@ -412,23 +590,25 @@ EncodeTiledFn gemm_encode_fn() {
     return fn;
 }
 
-// packed weights [n rows][k/2 bytes]: boxes of 128 rows x 32 bytes (64 k), dense in shared memory
-bool encode_gemm_w(CUtensorMap* map, const uint8_t* w, long long n, long long k) {
+// packed weights [n rows][k/2 bytes]: boxes of `rows` rows x 64 bytes (one 128-k group), 64-byte swizzled so that the
+// unpacking threads - one per row - read their 16-byte chunks without bank conflicts
+bool encode_gemm_w(CUtensorMap* map, const uint8_t* w, long long n, long long k, int rows) {
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k / 2), static_cast<cuuint64_t>(n)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k / 2)};
-    const cuuint32_t box[2] = {kGemmStageK / 2, 128};
+    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(rows)};
     const cuuint32_t estr[2] = {1, 1};
     return gemm_encode_fn() &&
            gemm_encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(w), dims, strides, box, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// activations [m rows][k] fp16: boxes of 256 rows x 64 k, 128-byte swizzled (the MMA's K-major operand layout)
-bool encode_gemm_x(CUtensorMap* map, const __half* x, long long m, long long k) {
+// activations [m rows][k] fp16: boxes of tile_m / 2 rows (each CTA of a pair loads half) x 64 k, 128-byte swizzled (the
+// MMA's K-major operand layout)
+bool encode_gemm_x(CUtensorMap* map, const __half* x, long long m, long long k, int tile_m) {
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(m)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k) * 2};
-    const cuuint32_t box[2] = {kGemmStageK, kGemmTileM};
+    const cuuint32_t box[2] = {kGemmStageK, static_cast<cuuint32_t>(tile_m / 2)};
     const cuuint32_t estr[2] = {1, 1};
     return gemm_encode_fn() &&
            gemm_encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(x), dims, strides, box, estr,
@@ -447,8 +627,13 @@ cudaError_t gemm_configure_and_launch(const GemmParams& p, dim3 grid, cudaStream
     {
         std::lock_guard<std::mutex> lock(mu);
         if (!configured[dev]) {
-            e = cudaFuncSetAttribute(w4a16_gemm_kernel<OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(kGemmSmemBytes));
+            // the register re-split draws on what the block was launched with: a request above that would wait forever
+            cudaFuncAttributes a;
+            e = cudaFuncGetAttributes(&a, w4a16_gemm_kernel<OutT>);
+            if (e != cudaSuccess) return e;
+            if (a.numRegs * kGemmThreads < kFoldRegs * kGemmFoldThreads + kUnpackRegs * kGemmUnpackThreads + kCtrlRegs * 128)
+                return cudaErrorLaunchOutOfResources;
+            e = cudaFuncSetAttribute(w4a16_gemm_kernel<OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemBytes);
             if (e != cudaSuccess) return e;
             configured[dev] = true;
         }
@@ -469,61 +654,63 @@ bool gemm_eligible(const void* x, const TcProj* proj, int num, bool swiglu, long
     return true;
 }
 
-// One launch per projection (gate and up of the fused MLP share one).  Returns 0, -1 on a launch error, -2 when
-// the problem cannot be described to the kernel.
+size_t gemm_partial_bytes(int num_sms) {
+    return static_cast<size_t>(num_sms) * 2 * kGemmTileN * kGemmTileM * sizeof(float);
+}
+
+// One launch for all projections that share X.  Returns 0, -1 on a launch error, -2 when the problem cannot be
+// described to the kernel.
 int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num, bool swiglu, bool out_f32, long long m,
-                long long k, int* status, long long wait_limit, int x_stage_limit, int num_sms, float* partials, size_t partial_bytes) {
-    const int launches = swiglu ? 1 : num;
-    for (int i = 0; i < launches; ++i) {
-        GemmParams p;
-        memset(&p, 0, sizeof(p));
-        const TcProj& a = proj[i];
-        const TcProj& b = swiglu ? proj[1] : proj[i];
-        if (!encode_gemm_w(&p.w_map[0], a.w, a.n, k) || !encode_gemm_w(&p.w_map[1], b.w, b.n, k)) return -2;
-        if (!encode_gemm_x(&p.x_map, static_cast<const __half*>(x), m, k)) return -2;
-        p.scales[0] = static_cast<const __half*>(a.scales);
-        p.scales[1] = static_cast<const __half*>(b.scales);
-        p.bias = a.bias;
-        p.y = a.y;
-        p.ldy = a.ldy > 0 ? a.ldy : a.n;
-        p.n = static_cast<int>(a.n);
-        p.m = static_cast<int>(m);
-        p.groups = static_cast<int>(k / 128);
-        p.stages = static_cast<int>(k / kGemmStageK);
-        p.swiglu = swiglu ? 1 : 0;
-        p.out_f32 = out_f32 ? 1 : 0;
-        p.wait_limit = wait_limit;
-        p.x_stage_limit = x_stage_limit;
-        p.status = status;
-        const int rows_per_cta = swiglu ? 128 : kGemmTileN;
-        dim3 grid(static_cast<unsigned>((a.n + rows_per_cta - 1) / rows_per_cta), static_cast<unsigned>((m + kGemmTileM - 1) / kGemmTileM));
-        // Few tiles (N = 5120 at M = 512 is 40): K is split over gridDim.z so that about two CTAs per SM's worth of
-        // work exists, the fp32 partials go through a scratch buffer and a second kernel adds them in split order.
-        int splits = 1;
-        const long long tiles = static_cast<long long>(grid.x) * grid.y;
-        if (!swiglu && partials && tiles * 2 <= num_sms) {
-            splits = static_cast<int>((2LL * num_sms) / tiles);
-            if (splits > 8) splits = 8;
-            if (splits > p.stages / 8) splits = p.stages / 8;
-            const long long per_split = static_cast<long long>(m) * a.n * 4;
-            if (per_split * splits > static_cast<long long>(partial_bytes)) splits = static_cast<int>(partial_bytes / per_split);
-            if (splits < 2) splits = 1;
-        }
-        grid.z = static_cast<unsigned>(splits);
-        p.partials = splits > 1 ? partials : nullptr;
-        cudaError_t e = out_f32 ? gemm_configure_and_launch<float>(p, grid, stream) : gemm_configure_and_launch<__half>(p, grid, stream);
-        if (e != cudaSuccess) return -1;
-        if (splits > 1) {
-            const long long total = m * a.n;
-            const unsigned blocks = static_cast<unsigned>(total / 1024 + 1 < 4096 ? total / 1024 + 1 : 4096);
-            e = out_f32 ? launch_pdl(gemm_splitk_reduce_kernel<float>, dim3(blocks), dim3(256), 0, stream, p.y, p.ldy,
-                                     static_cast<const float*>(partials), splits, p.m, p.n, p.bias)
-                        : launch_pdl(gemm_splitk_reduce_kernel<__half>, dim3(blocks), dim3(256), 0, stream, p.y, p.ldy,
-                                     static_cast<const float*>(partials), splits, p.m, p.n, p.bias);
-            if (e != cudaSuccess) return -1;
-        }
+                long long k, int* status, long long wait_limit, int x_stage_limit, int num_sms, float* partials, int* counters) {
+    GemmParams p;
+    memset(&p, 0, sizeof(p));
+    // rows per tile: as few tiles as 256 rows allow, evenly filled, in steps of 32 (a fold thread reads 16 columns at a time)
+    p.m_tiles = static_cast<int>((m + kGemmTileM - 1) / kGemmTileM);
+    p.tile_m = static_cast<int>(((m + p.m_tiles - 1) / p.m_tiles + 31) / 32 * 32);
+    p.w_slots = gemm_w_slots(p.tile_m);
+    p.groups = static_cast<int>(k / 128);
+    long long tiles = 0;
+    if (swiglu) {
+        if (!encode_gemm_w(&p.w_map[0], proj[0].w, proj[0].n, k, 64) || !encode_gemm_w(&p.w_map[1], proj[1].w, proj[1].n, k, 64)) return -2;
+        p.proj[0].scales[1] = static_cast<const __half*>(proj[1].scales);
     }
-    return 0;
+    p.num_proj = swiglu ? 1 : num;
+    for (int i = 0; i < p.num_proj; ++i) {
+        const TcProj& a = proj[i];
+        if (!swiglu && !encode_gemm_w(&p.w_map[i], a.w, a.n, k, kGemmTileN)) return -2;
+        p.proj[i].scales[0] = static_cast<const __half*>(a.scales);
+        p.proj[i].bias = a.bias;
+        p.proj[i].y = a.y;
+        p.proj[i].ldy = a.ldy > 0 ? a.ldy : a.n;
+        p.proj[i].n = static_cast<int>(a.n);
+        p.proj[i].tile0 = static_cast<int>(tiles);
+        const int rows = swiglu ? kGemmTileN : 2 * kGemmTileN;  // of a pair
+        tiles += (a.n + rows - 1) / rows * p.m_tiles;
+    }
+    if (tiles > (1 << 30)) return -2;
+    if (!encode_gemm_x(&p.x_map, static_cast<const __half*>(x), m, k, p.tile_m)) return -2;
+    p.m = static_cast<int>(m);
+    p.units = tiles * p.groups;
+    p.swiglu = swiglu ? 1 : 0;
+    p.wait_limit = wait_limit;
+    p.x_stage_limit = x_stage_limit;
+    p.status = status;
+    p.partials = partials;
+    p.counters = counters;
+    // One pair per two SMs.  Cutting tiles evens the pairs' work out and costs the exchange of partial sums, about as
+    // much as kCutCost groups; a small problem takes fewer pairs (below eight groups each, the pipeline's fill dominates).
+    constexpr long long kCutCost = 10;
+    const long long max_pairs = num_sms / 2;
+    const long long whole = (tiles + max_pairs - 1) / max_pairs * p.groups;
+    long long cut_pairs = p.units / 8;
+    if (cut_pairs < 1) cut_pairs = 1;
+    if (cut_pairs > max_pairs) cut_pairs = max_pairs;
+    p.whole_tiles = (!partials || whole <= (p.units + cut_pairs - 1) / cut_pairs + kCutCost) ? 1 : 0;
+    const long long pairs = p.whole_tiles ? (tiles < max_pairs ? tiles : max_pairs) : cut_pairs;
+    p.pairs = static_cast<int>(pairs);
+    const dim3 grid(static_cast<unsigned>(2 * pairs));
+    const cudaError_t e = out_f32 ? gemm_configure_and_launch<float>(p, grid, stream) : gemm_configure_and_launch<__half>(p, grid, stream);
+    return e == cudaSuccess ? 0 : -1;
 }
 
 }  // namespace xb
