@@ -1,0 +1,90 @@
+"""The delta rule over longer calls (blocks of 16 tokens on the tensor cores) and the vectorised convolution, at the
+sizes where they can go wrong: around the change of kernel, around block edges, strong decay, repeated keys, and a state
+carried from call to call.  Against the fp32 restatement of the reference in oracle/."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cuda():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    import xinfer_b200.ops as ops
+    return ops
+
+
+def dev(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def delta_rule_f64(qkv, z, b, a, A_log, dt_bias, norm_w, S, hv, hk):
+    T = qkv.shape[0]
+    f = lambda x: np.asarray(x, np.float64)  # noqa: E731
+    q, k = f(qkv[:, :hk * 128]).reshape(T, hk, 128), f(qkv[:, hk * 128:2 * hk * 128]).reshape(T, hk, 128)
+    v, zz = f(qkv[:, 2 * hk * 128:]).reshape(T, hv, 128), f(z).reshape(T, hv, 128)
+    unit = lambda x: x / np.sqrt((x * x).sum(-1, keepdims=True) + 1e-6)  # noqa: E731
+    q, k = np.repeat(unit(q) * 0.08838834764, hv // hk, 1), np.repeat(unit(k), hv // hk, 1)
+    beta = 1 / (1 + np.exp(-f(b)))
+    g = np.exp(-np.exp(f(A_log)) * np.logaddexp(0, f(a) + f(dt_bias)))
+    S, out = f(S).copy(), np.empty((T, hv, 128))
+    for t in range(T):
+        S *= g[t][:, None, None]
+        d = (v[t] - np.einsum("hkd,hk->hd", S, k[t])) * beta[t][:, None]
+        S += k[t][:, :, None] * d[:, None, :]
+        out[t] = np.einsum("hkd,hk->hd", S, q[t])
+    out = out / np.sqrt((out * out).mean(-1, keepdims=True) + 1e-6) * f(norm_w) * zz / (1 + np.exp(-zz))
+    return out.reshape(T, hv * 128), S
+
+
+@pytest.mark.parametrize("T", [1, 16, 17, 31, 32, 33, 77])
+@pytest.mark.parametrize("kind", ["plain", "slow decay", "one key"])
+def test_delta_rule_blocks(cuda, T, kind):
+    import torch
+    hv, hk = 6, 2
+    rng = np.random.default_rng(T)
+    qkv = rng.normal(0, 1, (2 * T, 2 * hk * 128 + hv * 128)).astype(np.float16)
+    z, b, a = (rng.normal(0, 1, (2 * T, n)).astype(np.float16) for n in (hv * 128, hv, hv))
+    if kind == "slow decay":
+        a = (a - 6).astype(np.float16)
+    if kind == "one key":
+        qkv[:, hk * 128:2 * hk * 128] = qkv[0, hk * 128:2 * hk * 128]
+    A_log, dt_bias = (rng.normal(0, 0.5, hv).astype(np.float32) for _ in range(2))
+    norm_w = rng.normal(1, 0.02, 128).astype(np.float32)
+    S = rng.normal(0, 0.05, (hv, 128, 128)).astype(np.float32)
+    want, S_want = delta_rule_f64(qkv, z, b, a, A_log, dt_bias, norm_w, S, hv, hk)
+    out, S_d = torch.full((2 * T, hv * 128), float("nan"), dtype=torch.float16, device="cuda"), dev(S)
+    args = [dev(x) for x in (qkv, z, b, a)]
+    for c in range(2):  # two calls: the second starts from the first one's state
+        part = [x[c * T:(c + 1) * T] for x in args]
+        assert cuda.recurrent_gated_delta_net(out[c * T:(c + 1) * T], *part, dev(A_log), dev(dt_bias), dev(norm_w), S_d, T, False, hv, hk) == 0
+    torch.cuda.synchronize()
+    rel = lambda x, y: np.linalg.norm(np.asarray(x, np.float64) - y) / np.linalg.norm(y)  # noqa: E731
+    # the output is rounded to fp16 once: 2^-11 at most, a third of that in the 2-norm.  The state: fp32 rounding of some
+    # 128-term sums per token, 6e-8 each, which decay forgets after a few tokens (slow decay: adds up over the call).
+    assert rel(out.float().cpu().numpy(), want) <= 5e-4
+    assert rel(S_d.cpu().numpy(), S_want) <= 6e-8 * 128 ** 0.5 * (T if kind == "slow decay" else 8) ** 0.5
+
+
+@pytest.mark.parametrize("T,C", [(1, 4), (2, 10), (3, 516), (8, 513), (9, 512), (40, 1028)])
+def test_conv1d_spans(cuda, T, C):
+    """One and several spans of positions, channel counts with and without vector access, in place, with and without state."""
+    import torch
+    rng = np.random.default_rng(T + C)
+    x, w, st = rng.normal(0, 1, (T, C)).astype(np.float16), rng.normal(0, 0.5, (C, 4)).astype(np.float32), rng.normal(0, 1, (3, C)).astype(np.float32)
+    for state in (st, None):
+        ref = None if state is None else state.copy()
+        want = np.asarray(oracle.conv1d_silu(x, w, ref), np.float32)
+        for in_place in (False, True):
+            x_d, st_d = dev(x), None if state is None else dev(state)
+            y = x_d if in_place else torch.full_like(x_d, float("nan"))
+            assert cuda.causal_conv1d_silu(y, x_d, dev(w), T, st_d, C) == 0
+            # one fp16 rounding on either side
+            assert np.all(np.abs(y.float().cpu().numpy() - want) <= 2 ** -10 * np.maximum(np.abs(want), 2 ** -14))
+            if state is not None:
+                assert np.array_equal(st_d.cpu().numpy(), ref)

@@ -30,6 +30,7 @@
 
 #include "launch.cuh"
 #include "mixers.h"
+#include "ptx_sm100.cuh"
 
 namespace xb {
 
@@ -768,183 +769,704 @@ __global__ void __launch_bounds__(512, 2) gdn_spec_kernel(__half* out, const __h
 }
 
 // ------------------------------------------------------------------------------- the same two mixers over a prompt chunk
-// Prefill keeps every row, so there is nothing to replay or to hold back: the delta rule walks all `rc` positions of a
-// chunk in one launch with the state in registers and writes the state back once (the step kernels above would need
-// rc / 4 launches, each re-reading and re-writing the state).  Rows are found through chunk_row (the chunk's group-by-group row
-// order).  Per token the arithmetic is the step kernels', operation by operation, so the results are bit-identical.
-// The convolution has no recurrence on its outputs (y_p needs the inputs p-3 .. p only), so every (position, channel)
-// is a thread of its own; inputs in front of the chunk come from the state.  A second, tiny launch then moves the
-// chunk's last three inputs into the state (it must not run while the first one still reads the old state).
-__global__ void conv1d_chunk_kernel(__half* out, const __half* in, const float* conv_w, const float* state, int rc, int channels) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int b = blockIdx.y, batch = gridDim.y, p = blockIdx.z;
+// Prefill keeps every row, so there is nothing to replay or to hold back.  Rows are found through chunk_row (the chunk's
+// group-by-group row order; with one sequence simply the positions).
+//
+// The convolution has no recurrence on its outputs (y_p needs the inputs p-3 .. p only): a thread takes V channels and
+// `span` consecutive positions with the window in registers.  The threads of the first positions are the only readers of
+// the state and also the ones that replace it by the chunk's last three inputs, so one launch does both.  (span = rc when
+// the output overwrites the input.)  Bound by its memory traffic; 512 x 10240 in 8 us against 35 with a thread per element
+// and a second launch for the state.
+template <int V>
+__global__ void __launch_bounds__(128) conv1d_chunk_kernel(__half* out, const __half* in, const float* conv_w, float* state, int rc,
+                                                           int channels, int span) {
+    griddep_prologue();
+    const int c = (blockIdx.z * 128 + threadIdx.x) * V;
+    const int b = blockIdx.y, batch = gridDim.y, p0 = blockIdx.x * span;
     if (c >= channels) return;
-    const float* st = state + static_cast<long long>(b) * 3 * channels;
-    float x[4];
+    float* st = state ? state + static_cast<long long>(b) * 3 * channels : nullptr;
+    struct alignas(2 * V) Vec { __half h[V]; };
+    auto load = [&](int p, float (&x)[V]) {  // the input at position p; negative: the state's slot 3 + p
+        if (p >= 0) {
+            const Vec v = *reinterpret_cast<const Vec*>(in + chunk_row(p, b, batch, rc) * channels + c);
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-        const int q = p - 3 + t;   // input position; negative: the state's slot 3 + q
-        x[t] = q >= 0 ? __half2float(in[chunk_row(q, b, batch, rc) * channels + c]) : st[(3 + q) * channels + c];
-    }
-    const float w0 = conv_w[c * 4], w1 = conv_w[c * 4 + 1], w2 = conv_w[c * 4 + 2], w3 = conv_w[c * 4 + 3];
-    const float sum = w0 * x[0] + w1 * x[1] + w2 * x[2] + w3 * x[3];
-    out[chunk_row(p, b, batch, rc) * channels + c] = __float2half_rn(sum / (1.0f + expf(-sum)));
-}
-__global__ void conv1d_chunk_state_kernel(const __half* in, float* state, int rc, int channels) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int b = blockIdx.y, batch = gridDim.y;
-    if (c >= channels) return;
-    float* st = state + static_cast<long long>(b) * 3 * channels;
-    float s[3];
+            for (int e = 0; e < V; ++e) x[e] = __half2float(v.h[e]);
+        } else {
 #pragma unroll
-    for (int t = 0; t < 3; ++t) {
-        const int q = rc - 3 + t;   // the new slot t holds the input at position rc - 3 + t
-        s[t] = q >= 0 ? __half2float(in[chunk_row(q, b, batch, rc) * channels + c]) : st[(3 + q) * channels + c];
-    }
-#pragma unroll
-    for (int t = 0; t < 3; ++t) st[t * channels + c] = s[t];
-}
-
-__global__ void __launch_bounds__(512, 2) gdn_chunk_kernel(__half* out, const __half* qkv, const __half* z,
-                                                           const __half* bb, const __half* aa, const float* A_log,
-                                                           const float* dt_bias, const float* norm_w, float* state, int rc,
-                                                           int hv, int hk) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    __shared__ __align__(16) float sh_q[8][128], sh_k[8][128];
-    __shared__ float sh_v[8][128], sh_z[8][128];
-    __shared__ float sh_beta[8], sh_eg[8], red[2][8][4];
-    __shared__ float part_sum[2][4][128], attn_all[8][4][128];
-    const int h = blockIdx.x, b = blockIdx.y, batch = gridDim.y;
-    const int j = threadIdx.x & 127, part = threadIdx.x >> 7;
-    const int lane = threadIdx.x & 31, wig = (threadIdx.x >> 5) & 3;
-    const int i0 = part * 32;
-    const int h_k = h / (hv / hk);
-    const int channels = 2 * hk * 128 + hv * 128;
-    const int value_dim = hv * 128;
-    float* S = state + (static_cast<long long>(b) * hv + h) * (128 * 128);
-    float col[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) col[i] = S[(i0 + i) * 128 + j];
-    const float exp_a_log = expf(A_log[h]);
-    const float dtb = dt_bias[h];
-    const float nw = norm_w[j];
-
-    // Blocks of eight positions.  With one sequence per GPU a chunk is 512 sequential tokens on 48 SMs, so what counts
-    // is the latency of a token: every global load of a block (q, k, v, z of its eight tokens; thread group `part`
-    // takes tokens part and part + 4) is issued at the top of the block and staged in shared memory, and the norms of
-    // all eight tokens share one barrier, so that the recurrence itself touches registers and shared memory only.
-    for (int p0 = 0; p0 < rc; p0 += 8) {
-        const int nb = rc - p0 < 8 ? rc - p0 : 8;
-        // ---- phase 0: per-token quantities that do not depend on the state
-        float raw_q[2] = {0.f, 0.f}, raw_k[2] = {0.f, 0.f};
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int tt = part + 4 * u;
-            if (tt < nb) {
-                const long long row = chunk_row(p0 + tt, b, batch, rc);
-                const __half* cur = qkv + row * channels;
-                raw_q[u] = __half2float(cur[h_k * 128 + j]);
-                raw_k[u] = __half2float(cur[hk * 128 + h_k * 128 + j]);
-                sh_v[tt][j] = __half2float(cur[2 * hk * 128 + h * 128 + j]);
-                sh_z[tt][j] = __half2float(z[row * value_dim + h * 128 + j]);
-            }
+            for (int e = 0; e < V; ++e) x[e] = st ? st[(3 + p) * static_cast<long long>(channels) + c + e] : 0.f;
         }
+    };
+    float w[V][4], x0[V], x1[V], x2[V], tail[3][V];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int tt = part + 4 * u;
-            const float wq = warp_sum(raw_q[u] * raw_q[u]), wk = warp_sum(raw_k[u] * raw_k[u]);
-            if (lane == 0) { red[0][tt][wig] = wq; red[1][tt][wig] = wk; }
+    for (int e = 0; e < V; ++e) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) w[e][t] = conv_w[(c + e) * 4 + t];
+    }
+    load(p0 - 3, x0);
+    load(p0 - 2, x1);
+    load(p0 - 1, x2);
+    if (p0 == 0 && st) {
+#pragma unroll
+        for (int t = 0; t < 3; ++t) load(rc - 3 + t, tail[t]);
+    }
+    const int p1 = p0 + span < rc ? p0 + span : rc;
+#pragma unroll 4
+    for (int p = p0; p < p1; ++p) {
+        float x[V];
+        load(p, x);
+        Vec o;
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            const float sum = w[e][0] * x0[e] + w[e][1] * x1[e] + w[e][2] * x2[e] + w[e][3] * x[e];
+            o.h[e] = __float2half_rn(sum / (1.0f + expf(-sum)));
+            x0[e] = x1[e];
+            x1[e] = x2[e];
+            x2[e] = x[e];
+        }
+        *reinterpret_cast<Vec*>(out + chunk_row(p, b, batch, rc) * channels + c) = o;
+    }
+    if (p0 == 0 && st) {
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+#pragma unroll
+            for (int e = 0; e < V; ++e) st[t * static_cast<long long>(channels) + c + e] = tail[t][e];
+        }
+    }
+}
+
+// The delta rule over a chunk: rc sequential tokens, so what counts is the latency of a token and how few instructions it
+// takes.  The columns of a head's 128 x 128 state do not interact, so a head is eight CTAs of 16 columns (one cluster; with
+// one sequence 48 heads alone would be 48 SMs), and inside a CTA a warp owns four columns by itself - eight lanes per
+// column, 16 rows each, in registers - and runs its tokens without any barrier:
+//   both dot products of a token are taken on the old state S, together:    ks = k.S, qs = q.S   (three shuffles each)
+//   delta = (v - g ks) beta;    out = g qs + (q.k) delta = q.(g S + k delta);    S = g S + k delta
+// Tokens come in blocks of 16: while one is walked, the next one's q, k, v and gates are in flight, and its norms are
+// taken once per block.  The gated RMSNorm of the outputs spans the head's 128 columns: every CTA sends its sums of
+// squares of a block to the other seven through distributed shared memory, and finishes the block one block later, so
+// that the cluster barrier in between has a block's time to complete.
+// For short chunks (kGdnWalkRows); a token costs 0.6 us.
+// Up to here the token-by-token kernel is the faster one (16 rows: 13 us against 15 for the two launches of the blocked form).
+constexpr int kGdnWalkRows = 16;
+constexpr int kGdnCols = 16, kGdnBlock = 16, kGdnSlices = 128 / kGdnCols, kGdnThreads = kGdnCols * 8;
+
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float sum_f32x2(uint64_t a) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));
+    return lo + hi;
+}
+
+__global__ void __cluster_dims__(kGdnSlices, 1, 1) __launch_bounds__(kGdnThreads) gdn_walk_kernel(
+    __half* out, const __half* qkv, const __half* z, const __half* bb, const __half* aa, const float* A_log, const float* dt_bias,
+    const float* norm_w, float* state, int rc, int hv, int hk, int zero_state) {
+    griddep_prologue();
+    __shared__ __align__(16) float sh_q[2][kGdnBlock][128], sh_k[2][kGdnBlock][128];
+    __shared__ float sh_v[2][kGdnBlock][kGdnCols], sh_out[kGdnBlock][kGdnCols + 1];
+    __shared__ float4 sh_gate[2][kGdnBlock];                 // decay, beta, q.k
+    __shared__ float sh_sq[2][kGdnSlices][kGdnBlock];        // sums of squares of the outputs, by column slice
+    __shared__ float sh_s[128][kGdnCols + 1];
+    const int slice = blockIdx.x % kGdnSlices, h = blockIdx.x / kGdnSlices, b = blockIdx.y, batch = gridDim.y;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int cl = lane >> 3, rg = lane & 7, col = warp * 4 + cl;  // rows of a lane: 4 (rg + 8 m) + e, m, e = 0..3
+    const int h_k = h / (hv / hk), channels = 2 * hk * 128 + hv * 128, value_dim = hv * 128;
+    const int col0 = slice * kGdnCols;
+
+    // ---- the state slice, through shared memory so that global accesses are whole 64-byte rows
+    float* S = state + (static_cast<long long>(b) * hv + h) * (128 * 128) + col0;
+    uint64_t s2[8];
+    if (zero_state) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s2[i] = 0;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 128 * kGdnCols / (4 * kGdnThreads); ++i) {
+            const int idx = i * kGdnThreads + tid, row = idx >> 2, c4 = (idx & 3) * 4;
+            const float4 v = *reinterpret_cast<const float4*>(S + row * 128 + c4);
+            sh_s[row][c4] = v.x; sh_s[row][c4 + 1] = v.y; sh_s[row][c4 + 2] = v.z; sh_s[row][c4 + 3] = v.w;
         }
         __syncthreads();
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int tt = part + 4 * u;
-            if (tt < nb) {
-                const float q_sq = ((red[0][tt][0] + red[0][tt][1]) + red[0][tt][2]) + red[0][tt][3];
-                const float k_sq = ((red[1][tt][0] + red[1][tt][1]) + red[1][tt][2]) + red[1][tt][3];
-                sh_q[tt][j] = (raw_q[u] * (1.0f / sqrtf(q_sq + 1e-6f))) * 0.08838834764f;
-                sh_k[tt][j] = raw_k[u] * (1.0f / sqrtf(k_sq + 1e-6f));
-                if (j == 0) {
-                    const long long row = chunk_row(p0 + tt, b, batch, rc);
-                    const float b_val = __half2float(bb[row * hv + h]);
-                    sh_beta[tt] = 1.0f / (1.0f + expf(-b_val));
-                    const float a_val = __half2float(aa[row * hv + h]) + dtb;
-                    const float softplus = (a_val > 20.0f) ? a_val : logf(1.0f + expf(a_val));
-                    sh_eg[tt] = expf(-exp_a_log * softplus);
-                }
+        for (int i = 0; i < 8; ++i) {
+            const int row = 4 * (rg + 8 * (i >> 1)) + 2 * (i & 1);
+            s2[i] = pack_f32x2(sh_s[row][col], sh_s[row + 1][col]);
+        }
+    }
+    const float exp_a_log = expf(A_log[h]), dtb = dt_bias[h];
+    // the output columns of this thread: token tid / 8 of a block, columns 2 (tid % 8) and the next
+    const int ot = tid >> 3, oc = (tid & 7) * 2;
+    const float nw0 = norm_w[col0 + oc], nw1 = norm_w[col0 + oc + 1];
+
+    // ---- a block's inputs: each warp fetches q and k of four tokens, the CTA its 16 values per token, 16 threads the gates
+    uint2 rq[kGdnBlock / 4], rk[kGdnBlock / 4];
+    __half2 rv;
+    __half ra, rb;
+    auto fetch = [&](int p0) {
+#pragma unroll
+        for (int u = 0; u < kGdnBlock / 4; ++u) {
+            const int p = p0 + warp + 4 * u;
+            if (p < rc) {
+                const __half* cur = qkv + chunk_row(p, b, batch, rc) * channels + h_k * 128 + lane * 4;
+                rq[u] = *reinterpret_cast<const uint2*>(cur);
+                rk[u] = *reinterpret_cast<const uint2*>(cur + hk * 128);
             }
         }
-        __syncthreads();
+        if (p0 + ot < rc) {
+            const long long row = chunk_row(p0 + ot, b, batch, rc);
+            rv = *reinterpret_cast<const __half2*>(qkv + row * channels + 2 * hk * 128 + h * 128 + col0 + oc);
+            if ((tid & 7) == 0) { ra = aa[row * hv + h]; rb = bb[row * hv + h]; }
+        }
+    };
+    auto stage = [&](int p0, int buf) {
+        float4* gate = sh_gate[buf];
+#pragma unroll
+        for (int u = 0; u < kGdnBlock / 4; ++u) {
+            const int t = warp + 4 * u;
+            if (p0 + t < rc) {
+                const float2 qa = __half22float2(*reinterpret_cast<const __half2*>(&rq[u].x)), qb = __half22float2(*reinterpret_cast<const __half2*>(&rq[u].y));
+                const float2 ka = __half22float2(*reinterpret_cast<const __half2*>(&rk[u].x)), kb = __half22float2(*reinterpret_cast<const __half2*>(&rk[u].y));
+                const float q_sq = warp_sum(qa.x * qa.x + qa.y * qa.y + qb.x * qb.x + qb.y * qb.y);
+                const float k_sq = warp_sum(ka.x * ka.x + ka.y * ka.y + kb.x * kb.x + kb.y * kb.y);
+                const float iq = 1.0f / sqrtf(q_sq + 1e-6f), ik = 1.0f / sqrtf(k_sq + 1e-6f);
+                const float4 qn = make_float4((qa.x * iq) * 0.08838834764f, (qa.y * iq) * 0.08838834764f, (qb.x * iq) * 0.08838834764f,
+                                              (qb.y * iq) * 0.08838834764f);
+                const float4 kn = make_float4(ka.x * ik, ka.y * ik, kb.x * ik, kb.y * ik);
+                const float qk = warp_sum(qn.x * kn.x + qn.y * kn.y + qn.z * kn.z + qn.w * kn.w);
+                *reinterpret_cast<float4*>(&sh_q[buf][t][lane * 4]) = qn;
+                *reinterpret_cast<float4*>(&sh_k[buf][t][lane * 4]) = kn;
+                if (lane == 0) gate[t].z = qk;
+            }
+        }
+        if (p0 + ot < rc) {
+            const float2 v = __half22float2(rv);
+            sh_v[buf][ot][oc] = v.x;
+            sh_v[buf][ot][oc + 1] = v.y;
+            if ((tid & 7) == 0) {
+                const float a_val = __half2float(ra) + dtb;
+                const float softplus = (a_val > 20.0f) ? a_val : logf(1.0f + expf(a_val));
+                gate[ot].x = expf(-exp_a_log * softplus);
+                gate[ot].y = 1.0f / (1.0f + expf(-__half2float(rb)));
+            }
+        }
+    };
 
-        // ---- phase 1: the recurrence
+    float o0 = 0.f, o1 = 0.f;  // this thread's outputs of the block whose norm is still under way
+    auto finish = [&](int p0, int buf) {
+        cluster_wait();
+        if (p0 + ot < rc) {
+            float sq = 0.f;
+#pragma unroll
+            for (int r = 0; r < kGdnSlices; ++r) sq += sh_sq[buf][r][ot];
+            const float inv_std = 1.0f / sqrtf(sq / 128.0f + 1e-6f);
+            const long long at = chunk_row(p0 + ot, b, batch, rc) * value_dim + h * 128 + col0 + oc;
+            const float2 zv = __half22float2(*reinterpret_cast<const __half2*>(z + at));
+            const float y0 = o0 * inv_std * nw0 * (zv.x / (1.0f + expf(-zv.x))), y1 = o1 * inv_std * nw1 * (zv.y / (1.0f + expf(-zv.y)));
+            *reinterpret_cast<__half2*>(out + at) = __floats2half2_rn(y0, y1);
+        }
+    };
+
+    fetch(0);
+    stage(0, 0);
+    int n = 0;
+    for (int p0 = 0; p0 < rc; p0 += kGdnBlock, ++n) {
+        const int buf = n & 1, nb = rc - p0 < kGdnBlock ? rc - p0 : kGdnBlock;
+        __syncthreads();
+        if (p0 + kGdnBlock < rc) fetch(p0 + kGdnBlock);
+#pragma unroll 2
         for (int t = 0; t < nb; ++t) {
-            const float v = sh_v[t][j];
-            const float eg = sh_eg[t];
-            float kv_mem = 0.f;
-            const float4* k4 = reinterpret_cast<const float4*>(&sh_k[t][i0]);
-            const float4* q4 = reinterpret_cast<const float4*>(&sh_q[t][i0]);
+            const float4 gate = sh_gate[buf][t];
+            const float v = sh_v[buf][t][col];
+            uint64_t k2[8], ks0 = 0, ks1 = 0, qs0 = 0, qs1 = 0;
 #pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                const float4 kk = k4[m];
-                const float kv[4] = {kk.x, kk.y, kk.z, kk.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float sv = col[m * 4 + e] * eg;
-                    col[m * 4 + e] = sv;
-                    kv_mem += sv * kv[e];
-                }
+            for (int m = 0; m < 4; ++m) {
+                const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(&sh_k[buf][t][4 * (rg + 8 * m)]);
+                const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(&sh_q[buf][t][4 * (rg + 8 * m)]);
+                k2[2 * m] = kk.x;
+                k2[2 * m + 1] = kk.y;
+                ks0 = fma_f32x2(s2[2 * m], kk.x, ks0);
+                ks1 = fma_f32x2(s2[2 * m + 1], kk.y, ks1);
+                qs0 = fma_f32x2(s2[2 * m], qq.x, qs0);
+                qs1 = fma_f32x2(s2[2 * m + 1], qq.y, qs1);
             }
-            part_sum[t & 1][part][j] = kv_mem;
-            __syncthreads();
-            const float* ps = &part_sum[t & 1][0][j];
-            const float delta = (v - (((ps[0] + ps[128]) + ps[256]) + ps[384])) * sh_beta[t];
-            float attn = 0.f;
+            float ks = sum_f32x2(ks0) + sum_f32x2(ks1), qs = sum_f32x2(qs0) + sum_f32x2(qs1);
 #pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                const float4 kk = k4[m], qq = q4[m];
-                const float kv[4] = {kk.x, kk.y, kk.z, kk.w}, qv[4] = {qq.x, qq.y, qq.z, qq.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float ns = col[m * 4 + e] + kv[e] * delta;
-                    col[m * 4 + e] = ns;
-                    attn += ns * qv[e];
-                }
+            for (int off = 1; off < 8; off <<= 1) {
+                ks += __shfl_xor_sync(0xffffffffu, ks, off);
+                qs += __shfl_xor_sync(0xffffffffu, qs, off);
             }
-            attn_all[t][part][j] = attn;
+            const float delta = (v - gate.x * ks) * gate.y;
+            const uint64_t d2 = pack_f32x2(delta, delta), g2 = pack_f32x2(gate.x, gate.x);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s2[i] = fma_f32x2(k2[i], d2, mul_f32x2(s2[i], g2));
+            if (rg == 0) sh_out[t][col] = gate.x * qs + gate.z * delta;
         }
         __syncthreads();
+        if (n > 0) finish(p0 - kGdnBlock, buf ^ 1);
+        // this block's sums of squares: eight threads per token, the r-th of them sends to CTA r of the cluster
+        o0 = ot < nb ? sh_out[ot][oc] : 0.f;
+        o1 = ot < nb ? sh_out[ot][oc + 1] : 0.f;
+        float sq = o0 * o0 + o1 * o1;
+#pragma unroll
+        for (int off = 1; off < 8; off <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+        st_shared_cluster_f32(mapa_shared_cluster(smem_u32(&sh_sq[buf][slice][ot]), tid & 7), sq);
+        cluster_arrive();
+        if (p0 + kGdnBlock < rc) stage(p0 + kGdnBlock, buf ^ 1);
+    }
+    finish((n - 1) * kGdnBlock, (n - 1) & 1);
 
-        // ---- phase 2: gated RMSNorm of every token's output
-        float attn2[2];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int tt = part + 4 * u;
-            attn2[u] = tt < nb ? ((attn_all[tt][0][j] + attn_all[tt][1][j]) + attn_all[tt][2][j]) + attn_all[tt][3][j] : 0.f;
-            const float wsq = warp_sum(attn2[u] * attn2[u]);
-            if (lane == 0) red[0][tt][wig] = wsq;
-        }
-        __syncthreads();
+    for (int i = 0; i < 8; ++i) {
+        const int row = 4 * (rg + 8 * (i >> 1)) + 2 * (i & 1);
+        float lo, hi;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(s2[i]));
+        sh_s[row][col] = lo;
+        sh_s[row + 1][col] = hi;
+    }
+    __syncthreads();
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int tt = part + 4 * u;
-            if (tt < nb) {
-                const float sq = ((red[0][tt][0] + red[0][tt][1]) + red[0][tt][2]) + red[0][tt][3];
-                const float inv_std = 1.0f / sqrtf(sq / 128.0f + 1e-6f);
-                const long long row = chunk_row(p0 + tt, b, batch, rc);
-                const float zv = sh_z[tt][j];
-                const float silu_z = zv / (1.0f + expf(-zv));
-                out[row * value_dim + h * 128 + j] = __float2half_rn(attn2[u] * inv_std * nw * silu_z);
-            }
+    for (int i = 0; i < 128 * kGdnCols / (4 * kGdnThreads); ++i) {
+        const int idx = i * kGdnThreads + tid, row = idx >> 2, c4 = (idx & 3) * 4;
+        *reinterpret_cast<float4*>(S + row * 128 + c4) = make_float4(sh_s[row][c4], sh_s[row][c4 + 1], sh_s[row][c4 + 2], sh_s[row][c4 + 3]);
+    }
+}
+
+// ------------------------------------------------------------------------------- the delta rule over longer chunks
+// Blocks of 16 tokens on the tensor cores.  With G_i the product of the decay factors of a block's tokens 0 .. i (kept as
+// sums of logarithms, so only ratios <= 1 are ever formed) and S0 the state in front of the block, the recurrence unrolls to
+//   delta = (I + L)^-1 diag(beta) (V - diag(G) K S0),     L_ij = beta_i G_i / G_j (k_i.k_j)   for j < i
+//   O = diag(G) Q S0 + P delta,                           P_ij = G_i / G_j (q_i.k_j)          for j <= i
+//   S = G_15 S0 + K^T diag(G_15 / G_j) delta
+// which is the same arithmetic, token for token, in another order (the blocked form of the delta rule published as
+// "Parallelizing Linear Transformers with the Delta Rule over Sequence Length", Yang et al. 2024).  What does not involve the
+// state - (I + L)^-1 diag(beta), P, the norms and the decays - is computed for all blocks of all heads at once by
+// gdn_block_kernel, a warp per block; gdn_scan_kernel then walks the blocks.
+//
+// Everything keeps fp32's precision: k and q enter as their raw fp16 values (their norms are row factors), every other
+// operand x as two fp16 values, hi = rn(2^-4 x) and mid = rn(2^11 (2^-4 x - hi)), 22 significant bits and the sign of mid,
+// which is fp32 to its last bit, in the range of +-2^20; the products with mid are summed apart and scaled back.  (With
+// tf32 operands the same kernel ran at a quarter of the rate: mma.sync of that type does 90 multiply-adds per clock and SM.)
+// Transposed products (state S^T, with the value columns as the MMA's rows) let a warp keep its 16 x 128 slice of the state
+// in accumulators that are A operands as they stand.
+// 512 tokens, one sequence, 48 heads: 160 us, 1.5 ms through the step's kernel eight tokens a launch, 300 us with
+// gdn_walk_kernel; bound by the latency of a block (1800 instructions per warp at 0.2 per clock, one warp per scheduler).
+constexpr int kScanBlock = 16, kScanWarps = 2, kScanCols = 16 * kScanWarps, kScanSlices = 128 / kScanCols, kScanPitch = 136;
+constexpr float kSplitDown = 0.0625f, kSplitUp = 16.0f, kMidUp = 2048.0f, kMidDown = 1.0f / 2048.0f;
+struct GdnBlock {                         // one block of one head, written by gdn_block_kernel
+    __half t[2][kScanBlock][kScanBlock];  // (I + L)^-1 diag(beta): rn(x), rn(2^11 (x - hi))
+    __half p[2][kScanBlock][kScanBlock];
+    float4 coef[kScanBlock];              // per token: 16 G_i / |k_i|, 16 G_i / (|q_i| sqrt(128)), G_15 / G_i / |k_i|, G_15
+};
+
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Two already scaled values as fp16 pairs hi and mid.
+__device__ __forceinline__ void split_f16x2(float x, float y, uint32_t& hi, uint32_t& mid) {
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(h);
+    const __half2 m = __floats2half2_rn((x - f.x) * kMidUp, (y - f.y) * kMidUp);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    mid = *reinterpret_cast<const uint32_t*>(&m);
+}
+// Two adjacent C fragments (16 x 8 each) as the A fragment of the 16 x 16 tile.
+__device__ __forceinline__ void split_frag(const float (&c0)[4], const float (&c1)[4], uint32_t (&hi)[4], uint32_t (&mid)[4]) {
+    split_f16x2(c0[0], c0[1], hi[0], mid[0]);
+    split_f16x2(c0[2], c0[3], hi[1], mid[1]);
+    split_f16x2(c1[0], c1[1], hi[2], mid[2]);
+    split_f16x2(c1[2], c1[3], hi[3], mid[3]);
+}
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4_trans(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+
+// One warp per (block, value head, sequence).
+__global__ void __launch_bounds__(128) gdn_block_kernel(GdnBlock* blocks, const __half* qkv, const __half* bb, const __half* aa,
+                                                        const float* A_log, const float* dt_bias, int rc, int hv, int hk) {
+    griddep_prologue();
+    __shared__ float sh_l[4][kScanBlock][kScanBlock + 1];
+    __shared__ float sh_lg[4][kScanBlock], sh_ik[4][kScanBlock], sh_iq[4][kScanBlock], sh_beta[4][kScanBlock];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int nblocks = (rc + kScanBlock - 1) / kScanBlock;
+    const int blk = blockIdx.x * 4 + warp, h = blockIdx.y, b = blockIdx.z, batch = gridDim.z;
+    if (blk >= nblocks) return;  // (no barrier below spans warps)
+    const int p0 = blk * kScanBlock, h_k = h / (hv / hk), channels = 2 * hk * 128 + hv * 128;
+    GdnBlock& out = blocks[(static_cast<long long>(b) * hv + h) * nblocks + blk];
+
+    // rows g and g + 8 of K and Q as A fragments; the same registers are the B fragments of K^T
+    const __half *k_row[2], *q_row[2];
+    bool live[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int p = p0 + g + 8 * r;
+        live[r] = p < rc;
+        q_row[r] = qkv + chunk_row(live[r] ? p : p0, b, batch, rc) * channels + h_k * 128;
+        k_row[r] = q_row[r] + hk * 128;
+    }
+    float kk[2][4] = {}, qk[2][4] = {}, k_sq[2] = {0.f, 0.f}, q_sq[2] = {0.f, 0.f};
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+        uint32_t ka[4], qa[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = i & 1, col = ks * 16 + (i >> 1) * 8 + 2 * t;
+            ka[i] = live[r] ? *reinterpret_cast<const uint32_t*>(k_row[r] + col) : 0u;
+            qa[i] = live[r] ? *reinterpret_cast<const uint32_t*>(q_row[r] + col) : 0u;
+            const float2 kf = __half22float2(*reinterpret_cast<const __half2*>(&ka[i])), qf = __half22float2(*reinterpret_cast<const __half2*>(&qa[i]));
+            k_sq[r] += kf.x * kf.x + kf.y * kf.y;
+            q_sq[r] += qf.x * qf.x + qf.y * qf.y;
         }
-        __syncthreads();
+        mma_f16(kk[0], ka, ka[0], ka[2]);
+        mma_f16(kk[1], ka, ka[1], ka[3]);
+        mma_f16(qk[0], qa, ka[0], ka[2]);
+        mma_f16(qk[1], qa, ka[1], ka[3]);
     }
 #pragma unroll
-    for (int i = 0; i < 32; ++i) S[(i0 + i) * 128 + j] = col[i];
+    for (int r = 0; r < 2; ++r) {
+#pragma unroll
+        for (int off = 1; off < 4; off <<= 1) {
+            k_sq[r] += __shfl_xor_sync(0xffffffffu, k_sq[r], off);
+            q_sq[r] += __shfl_xor_sync(0xffffffffu, q_sq[r], off);
+        }
+        if (t == 0) {
+            sh_ik[warp][g + 8 * r] = 1.0f / sqrtf(k_sq[r] + 1e-6f);
+            sh_iq[warp][g + 8 * r] = (1.0f / sqrtf(q_sq[r] + 1e-6f)) * 0.08838834764f;
+        }
+    }
+    // log of the cumulative decay and beta; positions behind the end decay nothing and write nothing
+    float lg = 0.f, beta = 0.f;
+    if (lane < kScanBlock && p0 + lane < rc) {
+        const long long row = chunk_row(p0 + lane, b, batch, rc);
+        const float a_val = __half2float(aa[row * hv + h]) + dt_bias[h];
+        const float softplus = (a_val > 20.0f) ? a_val : logf(1.0f + expf(a_val));
+        lg = -expf(A_log[h]) * softplus;
+        beta = 1.0f / (1.0f + expf(-__half2float(bb[row * hv + h])));
+    }
+    if (lane < kScanBlock) { sh_lg[warp][lane] = lg; sh_beta[warp][lane] = beta; }
+    __syncwarp();
+    // logarithms of G_i / G_j, summed from j + 1 on (a difference of prefix sums would lose what they have in common)
+    const int j = lane & (kScanBlock - 1);
+    float prefix = 0.f, suffix = 0.f;
+    for (int i = 0; i <= j; ++i) prefix += sh_lg[warp][i];
+    if (lane < kScanBlock) {
+        for (int i = j + 1; i < kScanBlock; ++i) {
+            suffix += sh_lg[warp][i];
+            sh_l[warp][i][j] = suffix;
+        }
+        sh_l[warp][j][j] = 0.f;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+        float ratio[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int i = g + 8 * (e >> 1), jj = nt * 8 + 2 * t + (e & 1);
+            ratio[e] = jj <= i ? expf(sh_l[warp][i][jj]) : 0.f;
+        }
+        float pv[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int i = g + 8 * (e >> 1), jj = nt * 8 + 2 * t + (e & 1);
+            const float ikj = sh_ik[warp][jj];
+            sh_l[warp][i][jj] = jj < i ? sh_beta[warp][i] * ratio[e] * (kk[nt][e] * sh_ik[warp][i] * ikj) : 0.f;
+            pv[e] = ratio[e] * (qk[nt][e] * sh_iq[warp][i] * ikj);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            uint32_t hi, mid;
+            split_f16x2(pv[2 * r], pv[2 * r + 1], hi, mid);
+            *reinterpret_cast<uint32_t*>(&out.p[0][g + 8 * r][nt * 8 + 2 * t]) = hi;
+            *reinterpret_cast<uint32_t*>(&out.p[1][g + 8 * r][nt * 8 + 2 * t]) = mid;
+        }
+    }
+    __syncwarp();
+    // column j of the inverse by forward substitution, a lane per column
+    float x[kScanBlock];
+#pragma unroll
+    for (int i = 0; i < kScanBlock; ++i) {
+        float s0 = i == j ? 1.f : 0.f, s1 = 0.f;
+#pragma unroll
+        for (int m = 0; m < i; ++m) {
+            if (m & 1) s1 = fmaf(-sh_l[warp][i][m], x[m], s1);
+            else s0 = fmaf(-sh_l[warp][i][m], x[m], s0);
+        }
+        x[i] = s0 + s1;
+    }
+    if (lane < kScanBlock) {
+        const float bj = sh_beta[warp][j];
+#pragma unroll
+        for (int i = 0; i < kScanBlock; ++i) {
+            const float v = x[i] * bj;
+            const __half hi = __float2half_rn(v);
+            out.t[0][i][j] = hi;
+            out.t[1][i][j] = __float2half_rn((v - __half2float(hi)) * kMidUp);
+        }
+        const float gj = expf(prefix);
+        out.coef[j] = make_float4(kSplitUp * gj * sh_ik[warp][j], kSplitUp * gj * sh_iq[warp][j], expf(suffix) * sh_ik[warp][j],
+                                  expf(prefix + suffix));
+    }
+}
+
+__global__ void __cluster_dims__(kScanSlices, 1, 1) __launch_bounds__(32 * kScanWarps) gdn_scan_kernel(
+    __half* out, const __half* qkv, const __half* z, const GdnBlock* blocks, const float* norm_w, float* state, int rc, int hv, int hk,
+    int zero_state) {
+    griddep_prologue();
+    __shared__ __align__(16) __half sh_q[2][kScanBlock][kScanPitch], sh_k[2][kScanBlock][kScanPitch];
+    __shared__ float sh_sq[2][kScanSlices * kScanWarps][kScanBlock];  // sums of squares of the outputs, by warp of the cluster
+    const int slice = blockIdx.x % kScanSlices, h = blockIdx.x / kScanSlices, b = blockIdx.y, batch = gridDim.y;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int nblocks = (rc + kScanBlock - 1) / kScanBlock;
+    const int h_k = h / (hv / hk), channels = 2 * hk * 128 + hv * 128, value_dim = hv * 128;
+    const int c0 = slice * kScanCols + warp * 16 + g;  // value columns of this thread: c0 and c0 + 8
+    const GdnBlock* blk = blocks + (static_cast<long long>(b) * hv + h) * nblocks;
+    float* S = state + (static_cast<long long>(b) * hv + h) * (128 * 128);
+
+    // a block's q and k: 16-byte pieces straight into shared memory, zeros behind the end
+    auto stage = [&](int n) {
+        const int buf = n & 1;
+#pragma unroll
+        for (int u = 0; u < kScanBlock * 16 / (32 * kScanWarps); ++u) {
+            const int idx = u * 32 * kScanWarps + tid, row = idx >> 4, c = (idx & 15) * 8, p = n * kScanBlock + row;
+            const __half* cur = qkv + chunk_row(p < rc ? p : n * kScanBlock, b, batch, rc) * channels + h_k * 128 + c;
+            const int bytes = p < rc ? 16 : 0;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(&sh_q[buf][row][c])), "l"(cur), "r"(bytes) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(&sh_k[buf][row][c])), "l"(cur + hk * 128), "r"(bytes) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // its small operands: v of the thread's two columns and four tokens 8 (i / 2) + 2t + i % 2, the block's matrices and factors
+    __half rv[2][4];
+    uint32_t rt[2][2][2], rp[2][2][2];  // [hi, mid][i tile][j half]
+    float4 rcoef[4];
+    auto fetch = [&](int n) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int j = 8 * (i >> 1) + 2 * t + (i & 1), p = n * kScanBlock + j;
+            const __half* cur = qkv + chunk_row(p < rc ? p : n * kScanBlock, b, batch, rc) * channels + 2 * hk * 128 + h * 128 + c0;
+            rv[0][i] = p < rc ? cur[0] : __half(0.f);
+            rv[1][i] = p < rc ? cur[8] : __half(0.f);
+            rcoef[i] = __ldg(&blk[n].coef[j]);
+        }
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+#pragma unroll
+            for (int it = 0; it < 2; ++it) {
+#pragma unroll
+                for (int jh = 0; jh < 2; ++jh) {
+                    rt[w][it][jh] = __ldg(reinterpret_cast<const uint32_t*>(&blk[n].t[w][it * 8 + g][jh * 8 + 2 * t]));
+                    rp[w][it][jh] = __ldg(reinterpret_cast<const uint32_t*>(&blk[n].p[w][it * 8 + g][jh * 8 + 2 * t]));
+                }
+            }
+        }
+    };
+    stage(0);
+    fetch(0);
+
+    float s[16][4];  // 2^-4 S^T: s[n][e] = 2^-4 S[8n + 2t + (e & 1)][c0 + 8 (e >> 1)]
+#pragma unroll
+    for (int n = 0; n < 16; ++n) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[n][e] = zero_state ? 0.f : kSplitDown * S[(8 * n + 2 * t + (e & 1)) * 128 + c0 + 8 * (e >> 1)];
+    }
+    const float nw[2] = {norm_w[c0], norm_w[c0 + 8]};
+
+    // The block whose norm is under way: its outputs [token tile][fragment], gates and rows.  Its stores are issued behind
+    // the next cluster barrier's arrive, which is a release and would wait for them.
+    float o[2][4];
+    __half zv[2][4];
+    auto out_row = [&](int n, int i) -> long long {
+        const int p = n * kScanBlock + 8 * (i >> 1) + 2 * t + (i & 1);
+        return p < rc ? chunk_row(p, b, batch, rc) * value_dim + h * 128 + c0 : -1;
+    };
+    auto fetch_z = [&](int n) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const long long at = out_row(n, i);
+            zv[0][i] = at >= 0 ? z[at] : __half(0.f);
+            zv[1][i] = at >= 0 ? z[at + 8] : __half(0.f);
+        }
+    };
+    __half y[2][4];
+    auto norm = [&](int n) {
+        cluster_wait();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float sq = 0.f;
+#pragma unroll
+            for (int r = 0; r < kScanSlices * kScanWarps; ++r) sq += sh_sq[n & 1][r][8 * (i >> 1) + 2 * t + (i & 1)];
+            const float inv_std = 1.0f / sqrtf(sq / 128.0f + 1e-6f);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float zf = __half2float(zv[c][i]);
+                y[c][i] = __float2half_rn(o[i >> 1][2 * c + (i & 1)] * inv_std * nw[c] * (zf / (1.0f + expf(-zf))));
+            }
+        }
+    };
+    auto store = [&](int n) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const long long at = out_row(n, i);
+            if (at >= 0) {
+                out[at] = y[0][i];
+                out[at + 8] = y[1][i];
+            }
+        }
+    };
+    // ldmatrix addresses: [token][state row] tiles, (token halves) x (row halves), plain and transposed
+    const uint32_t lm_row = static_cast<uint32_t>(((lane >> 4) & 1) * 8 + (lane & 7)), lm_col = static_cast<uint32_t>(((lane >> 3) & 1) * 8);
+    const uint32_t lt_row = static_cast<uint32_t>(((lane >> 3) & 1) * 8 + (lane & 7)), lt_col = static_cast<uint32_t>(((lane >> 4) & 1) * 8);
+
+    for (int n = 0; n < nblocks; ++n) {
+        const int buf = n & 1;
+        // this block's small operands, before the next block's take their registers
+        float v[2][4];
+        float4 coef[4];
+        uint32_t tm[2][2][2], pm[2][2][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[0][i] = __half2float(rv[0][i]);
+            v[1][i] = __half2float(rv[1][i]);
+            coef[i] = rcoef[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            tm[i >> 2][(i >> 1) & 1][i & 1] = rt[i >> 2][(i >> 1) & 1][i & 1];
+            pm[i >> 2][(i >> 1) & 1][i & 1] = rp[i >> 2][(i >> 1) & 1][i & 1];
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (n > 0) fetch_z(n - 1);
+        if (n + 1 < nblocks) {
+            stage(n + 1);
+            fetch(n + 1);
+        }
+
+        // (K S0)^T and (Q S0)^T: 16 value columns x 16 tokens, contraction over the 128 state rows
+        float ks[2][2][4] = {}, qs[2][2][4] = {};  // [hi, mid][token tile]
+        const uint32_t k_base = smem_u32(&sh_k[buf][lm_row][lm_col]), q_base = smem_u32(&sh_q[buf][lm_row][lm_col]);
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            uint32_t hi[4], mid[4], kb[4], qb[4];
+            ldsm4(k_base + m * 32, kb);
+            ldsm4(q_base + m * 32, qb);
+            split_frag(s[2 * m], s[2 * m + 1], hi, mid);
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+                mma_f16(ks[0][nt], hi, kb[2 * nt], kb[2 * nt + 1]);
+                mma_f16(qs[0][nt], hi, qb[2 * nt], qb[2 * nt + 1]);
+                mma_f16(ks[1][nt], mid, kb[2 * nt], kb[2 * nt + 1]);
+                mma_f16(qs[1][nt], mid, qb[2 * nt], qb[2 * nt + 1]);
+            }
+        }
+        // 2^-4 delta^T = (2^-4 (V - diag(G / |k|) K S0))^T T^T
+        float delta[2][4] = {}, acc[2][4] = {}, u[2][4];
+        uint32_t ahi[4], amid[4];
+        {
+            float r[2][4];
+#pragma unroll
+            for (int jt = 0; jt < 2; ++jt) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    r[jt][e] = kSplitDown * (v[e >> 1][jt * 2 + (e & 1)] - coef[jt * 2 + (e & 1)].x * (ks[0][jt][e] + kMidDown * ks[1][jt][e]));
+            }
+            split_frag(r[0], r[1], ahi, amid);
+        }
+#pragma unroll
+        for (int it = 0; it < 2; ++it) {
+            mma_f16(delta[it], ahi, tm[0][it][0], tm[0][it][1]);
+            mma_f16(acc[it], ahi, tm[1][it][0], tm[1][it][1]);
+            mma_f16(acc[it], amid, tm[0][it][0], tm[0][it][1]);
+        }
+#pragma unroll
+        for (int jt = 0; jt < 2; ++jt) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                delta[jt][e] += kMidDown * acc[jt][e];
+                u[jt][e] = delta[jt][e] * coef[jt * 2 + (e & 1)].z;
+                acc[jt][e] = 0.f;
+            }
+        }
+        // O^T = diag(G / |q|) (Q S0)^T + delta^T P^T
+        float od[2][4] = {};
+        split_frag(delta[0], delta[1], ahi, amid);
+#pragma unroll
+        for (int it = 0; it < 2; ++it) {
+            mma_f16(od[it], ahi, pm[0][it][0], pm[0][it][1]);
+            mma_f16(acc[it], ahi, pm[1][it][0], pm[1][it][1]);
+            mma_f16(acc[it], amid, pm[0][it][0], pm[0][it][1]);
+        }
+        // S^T = G_15 S^T + (diag(G_15 / G_j / |k_j|) delta)^T K
+        const float ge = coef[0].w;
+        const uint32_t kt_base = smem_u32(&sh_k[buf][lt_row][lt_col]);
+        split_frag(u[0], u[1], ahi, amid);
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            uint32_t kb[4];
+            ldsm4_trans(kt_base + m * 32, kb);
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+                float (&sn)[4] = s[2 * m + nt];
+                float low[4] = {};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sn[e] *= ge;
+                mma_f16(sn, ahi, kb[2 * nt], kb[2 * nt + 1]);
+                mma_f16(low, amid, kb[2 * nt], kb[2 * nt + 1]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sn[e] = fmaf(low[e], kMidDown, sn[e]);
+            }
+        }
+        if (n > 0) norm(n - 1);
+        // sums of squares over this warp's 16 columns, to every CTA of the cluster
+        float sq[4];
+#pragma unroll
+        for (int jt = 0; jt < 2; ++jt) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                o[jt][e] = coef[jt * 2 + (e & 1)].y * (qs[0][jt][e] + kMidDown * qs[1][jt][e]) + kSplitUp * (od[jt][e] + kMidDown * acc[jt][e]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float a = o[i >> 1][i & 1], c = o[i >> 1][2 + (i & 1)];
+            sq[i] = a * a + c * c;
+#pragma unroll
+            for (int off = 4; off < 32; off <<= 1) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], off);
+        }
+        if (g < kScanSlices) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                st_shared_cluster_f32(mapa_shared_cluster(smem_u32(&sh_sq[buf][slice * kScanWarps + warp][8 * (i >> 1) + 2 * t + (i & 1)]), g), sq[i]);
+        }
+        cluster_arrive();
+        if (n > 0) store(n - 1);
+    }
+    fetch_z(nblocks - 1);
+    norm(nblocks - 1);
+    store(nblocks - 1);
+#pragma unroll
+    for (int n = 0; n < 16; ++n) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[(8 * n + 2 * t + (e & 1)) * 128 + c0 + 8 * (e >> 1)] = kSplitUp * s[n][e];
+    }
 }
 
 // ------------------------------------------------------------------------------- speculative bookkeeping
@@ -1100,17 +1622,39 @@ int gdn_spec(cudaStream_t s, __half* out, const __half* qkv, const __half* z, co
 int conv1d_chunk(cudaStream_t s, __half* out, const __half* in, const float* conv_w, float* state, int batch, int rc,
                  int channels) {
     if (rc <= 0) return 0;
-    dim3 grid((channels + 255) / 256, batch, rc);
-    launch_pdl(conv1d_chunk_kernel, dim3(grid), dim3(256), 0, s, out, in, conv_w, static_cast<const float*>(state), rc, channels);
-    dim3 grid2((channels + 255) / 256, batch);
-    launch_pdl(conv1d_chunk_state_kernel, dim3(grid2), dim3(256), 0, s, in, state, rc, channels);
+    // Eight positions per thread; all of them when the output lies over the input (a position's inputs are its neighbours').
+    const size_t bytes = static_cast<size_t>(batch) * rc * channels * sizeof(__half);
+    const char *o = reinterpret_cast<const char*>(out), *i = reinterpret_cast<const char*>(in);
+    const int span = (o < i + bytes && i < o + bytes) ? rc : 8;
+    const bool vec = channels % 4 == 0 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in)) & 7) == 0;
+    const int per_block = 128 * (vec ? 4 : 1);
+    dim3 grid((rc + span - 1) / span, batch, (channels + per_block - 1) / per_block);
+    launch_pdl(vec ? conv1d_chunk_kernel<4> : conv1d_chunk_kernel<1>, grid, dim3(128), 0, s, out, in, conv_w, state, rc, channels, span);
     return XB_LAUNCH_OK();
 }
 
+bool gdn_chunk_aligned(const void* out, const void* qkv, const void* z, const void* state) {
+    return ((reinterpret_cast<uintptr_t>(qkv) & 15) | (reinterpret_cast<uintptr_t>(state) & 15) |
+            ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(z)) & 3)) == 0;
+}
+
+size_t gdn_chunk_scratch_bytes(int batch, int rc, int hv) {
+    return static_cast<size_t>(batch) * hv * ((rc + kScanBlock - 1) / kScanBlock) * sizeof(GdnBlock);
+}
+
 int gdn_chunk(cudaStream_t s, __half* out, const __half* qkv, const __half* z, const __half* b, const __half* a,
-              const float* A_log, const float* dt_bias, const float* norm_w, float* state, int batch, int rc, int hv, int hk) {
-    dim3 grid(hv, batch);
-    launch_pdl(gdn_chunk_kernel, dim3(grid), dim3(512), 0, s, out, qkv, z, b, a, A_log, dt_bias, norm_w, state, rc, hv, hk);
+              const float* A_log, const float* dt_bias, const float* norm_w, float* state, int batch, int rc, int hv, int hk,
+              void* scratch, int zero_state) {
+    if (rc <= kGdnWalkRows) {
+        launch_pdl(gdn_walk_kernel, dim3(hv * kGdnSlices, batch), dim3(kGdnThreads), 0, s, out, qkv, z, b, a, A_log, dt_bias, norm_w,
+                   state, rc, hv, hk, zero_state);
+        return XB_LAUNCH_OK();
+    }
+    GdnBlock* blocks = static_cast<GdnBlock*>(scratch);
+    const int nblocks = (rc + kScanBlock - 1) / kScanBlock;
+    launch_pdl(gdn_block_kernel, dim3((nblocks + 3) / 4, hv, batch), dim3(128), 0, s, blocks, qkv, b, a, A_log, dt_bias, rc, hv, hk);
+    launch_pdl(gdn_scan_kernel, dim3(hv * kScanSlices, batch), dim3(32 * kScanWarps), 0, s, out, qkv, z, static_cast<const GdnBlock*>(blocks),
+               norm_w, state, rc, hv, hk, zero_state);
     return XB_LAUNCH_OK();
 }
 

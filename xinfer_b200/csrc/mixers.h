@@ -66,11 +66,16 @@ __host__ __device__ inline long long chunk_row(int p, int b, int batch, int rc) 
     return static_cast<long long>(j) * batch * 4 + static_cast<long long>(b) * rj + i;
 }
 // The convolution and the gated delta rule over all rc positions of a prefill chunk in one launch each (rows in
-// chunk_row order, every row kept, the state read once and written back once; nothing pending afterwards).
+// chunk_row order, every row kept, the state read once and written back once; nothing pending afterwards).  A null
+// convolution state means zeros; zero_state starts the recurrence from zeros.
 int conv1d_chunk(cudaStream_t s, __half* out, const __half* in, const float* conv_w, float* state, int batch, int rc,
                  int channels);
 int gdn_chunk(cudaStream_t s, __half* out, const __half* qkv, const __half* z, const __half* b, const __half* a,
-              const float* A_log, const float* dt_bias, const float* norm_w, float* state, int batch, int rc, int hv, int hk);
+              const float* A_log, const float* dt_bias, const float* norm_w, float* state, int batch, int rc, int hv, int hk,
+              void* scratch, int zero_state = 0);
+size_t gdn_chunk_scratch_bytes(int batch, int rc, int hv);  // of `scratch`, 16-byte aligned
+// Whether the vector accesses of gdn_chunk fit these pointers.
+bool gdn_chunk_aligned(const void* out, const void* qkv, const void* z, const void* state);
 
 int spec_commit(cudaStream_t s, const void* accept_records, const long long* draft_tokens, int batch, int k,
                 int rows_per_seq, int* ctx, int* n_commit, long long* cur_tok, long long* emitted, int* emitted_n,

@@ -7,9 +7,8 @@
 //   sdpa_causal_cached              src/ops/attention.h:89-113
 //   causal_conv1d_silu              src/targets/qwen3_8/linear_attn.h:15-21
 //   recurrent_gated_delta_net       src/targets/qwen3_8/linear_attn.h:41-58
-// They run the product kernels (the ones the speculative step launches), not separate test kernels: the
-// stateful ops go through the same pending-update / commit mechanism as the step, with the commit applied
-// before the call returns to the stream, which gives the reference's "state is updated by the call" contract.
+// They run the product kernels (the ones the speculative step and the chunked prefill launch), not separate test
+// kernels; the stateful ops update their state in the call, as the reference's do.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -152,28 +151,9 @@ int xinfer_causal_conv1d_silu_f16(xinfer_stream_t s, void* out_qkv, const void* 
     if (num_channels <= 0 || num_channels > INT32_MAX) return XINFER_ERR_INVALID_ARGUMENT;
     if (seq_len <= 0) return XINFER_NOOP_INVALID_SHAPE;
     if (!out_qkv || !in_qkv || !conv_w) return XINFER_ERR_INVALID_ARGUMENT;
-    const int ch = static_cast<int>(num_channels);
-    // pending inputs [8][ch], and a zero state [3][ch] for callers without one ("assumes zeros for past")
-    float* scr = nullptr;
-    int rc = scratch(static_cast<size_t>(11) * ch * sizeof(float), &scr);
-    if (rc != XINFER_OK) return rc;
-    cudaStream_t st = static_cast<cudaStream_t>(s);
-    float* state = conv_state;
-    if (!state) {
-        state = scr + static_cast<size_t>(8) * ch;
-        if (cudaMemsetAsync(state, 0, static_cast<size_t>(3) * ch * sizeof(float), st) != cudaSuccess) return ok_or_cuda(-1);
-    }
-    const __half* in = static_cast<const __half*>(in_qkv);
-    __half* out = static_cast<__half*>(out_qkv);
-    int prev = 0;
-    for (int64_t t0 = 0; t0 < seq_len; t0 += 8) {
-        const int rows = static_cast<int>(seq_len - t0 < 8 ? seq_len - t0 : 8);
-        rc = xb::conv1d_spec(st, out + t0 * ch, in + t0 * ch, conv_w, state, scr, nullptr, 1, rows, prev, ch, prev);
-        if (rc != 0) return ok_or_cuda(rc);
-        prev = rows;
-    }
-    // commit the last chunk's inputs to the state
-    return ok_or_cuda(xb::conv1d_spec(st, out, in, conv_w, state, scr, nullptr, 1, 0, prev, ch, prev));
+    if (seq_len > INT32_MAX) return XINFER_ERR_INVALID_ARGUMENT;
+    return ok_or_cuda(xb::conv1d_chunk(static_cast<cudaStream_t>(s), static_cast<__half*>(out_qkv), static_cast<const __half*>(in_qkv),
+                                       conv_w, conv_state, 1, static_cast<int>(seq_len), static_cast<int>(num_channels)));
 }
 
 int xinfer_recurrent_gated_delta_net_f16(xinfer_stream_t s, void* out, const void* qkv, const void* z, const void* b,
@@ -187,6 +167,24 @@ int xinfer_recurrent_gated_delta_net_f16(xinfer_stream_t s, void* out, const voi
     if (num_v_heads <= 0 || num_k_heads <= 0 || num_v_heads % num_k_heads) return XINFER_ERR_INVALID_ARGUMENT;
     if (!out || !qkv || !z || !b || !a || !A_log || !dt_bias || !norm_weight || !state_buffer) return XINFER_ERR_INVALID_ARGUMENT;
     const int hv = static_cast<int>(num_v_heads), hk = static_cast<int>(num_k_heads);
+    if (xb::gdn_chunk_aligned(out, qkv, z, state_buffer)) {
+        // pieces of 4096 rows bound the scratch (29 MB at 48 heads)
+        const int64_t piece = 4096, ch = 2 * static_cast<int64_t>(hk) * 128 + static_cast<int64_t>(hv) * 128, vd = static_cast<int64_t>(hv) * 128;
+        float* blocks = nullptr;
+        const int most = static_cast<int>(seq_len < piece ? seq_len : piece);
+        const int rc = scratch(xb::gdn_chunk_scratch_bytes(1, most, hv), &blocks);
+        if (rc != XINFER_OK) return rc;
+        for (int64_t t0 = 0; t0 < seq_len; t0 += piece) {
+            const int rows = static_cast<int>(seq_len - t0 < piece ? seq_len - t0 : piece);
+            const int r = xb::gdn_chunk(static_cast<cudaStream_t>(s), static_cast<__half*>(out) + t0 * vd, static_cast<const __half*>(qkv) + t0 * ch,
+                                        static_cast<const __half*>(z) + t0 * vd, static_cast<const __half*>(b) + t0 * hv,
+                                        static_cast<const __half*>(a) + t0 * hv, A_log, dt_bias, norm_weight, state_buffer, 1, rows, hv, hk,
+                                        blocks, zero_state && t0 == 0);
+            if (r != 0) return ok_or_cuda(r);
+        }
+        return XINFER_OK;
+    }
+    // pointers that the vector accesses of the chunk kernel do not fit: eight tokens a launch through the step's kernel
     const size_t pk = static_cast<size_t>(hv) * 8 * 128;
     float* scr = nullptr;
     int rc = scratch((2 * pk + static_cast<size_t>(hv) * 8) * sizeof(float), &scr);

@@ -191,6 +191,7 @@ struct xinfer_spec_decoder {
                *abuf = nullptr, *cat = nullptr, *hprev = nullptr;
         long long* tokens = nullptr;
         int* entry_ctx = nullptr;        // context length in front of every (group, sequence) entry of a chunk
+        void* gdn_scratch = nullptr;     // per-block operands of the delta rule
         float* attn_scratch = nullptr;   // split partials of one attention launch over all entries
         int attn_splits = 1;
     } chunk;
@@ -676,7 +677,7 @@ int ensure_chunk_bufs(Dec* d, int rows) {
     const size_t wide = mx(hq * 512, ch), mix = mx(mx(hq * 256, hv * 128), H);
     const size_t per_row = 3 * H + F + wide + ch + hq * 256 + 2 * hkv * 256 + mix + hv * 128 + 2 * hv + 2 * H + H;
     const size_t halves = (per_row + 64) * static_cast<size_t>(rows);
-    if (cb.x) { cudaFree(cb.x); cudaFree(cb.attn_scratch); cb = Dec::ChunkBufs(); }
+    if (cb.x) { cudaFree(cb.x); cudaFree(cb.attn_scratch); cudaFree(cb.gdn_scratch); cb = Dec::ChunkBufs(); }
     __half* base = nullptr;
     if (cudaMalloc(&base, halves * sizeof(__half) + static_cast<size_t>(rows) * (sizeof(long long) + sizeof(int)) + 256) != cudaSuccess) {
         cudaGetLastError();
@@ -704,6 +705,14 @@ int ensure_chunk_bufs(Dec* d, int rows) {
     if (cudaMalloc(&cb.attn_scratch, xb::attn_scratch_bytes(entries, static_cast<int>(hkv), ns)) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(base);
+        cb = Dec::ChunkBufs();
+        return XINFER_ERR_OUT_OF_MEMORY;
+    }
+    // (`rows` is a whole number of positions for every sequence, and no chunk holds more than that)
+    if (cudaMalloc(&cb.gdn_scratch, xb::gdn_chunk_scratch_bytes(d->batch, (rows + d->batch - 1) / d->batch, static_cast<int>(hv))) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(base);
+        cudaFree(cb.attn_scratch);
         cb = Dec::ChunkBufs();
         return XINFER_ERR_OUT_OF_MEMORY;
     }
@@ -771,7 +780,7 @@ int prefill_chunk(Dec* d, cudaStream_t s, const long long* prompt, int64_t T, in
             const xinfer_fused_desc fd[4] = {desc(cb.wide, L.in_qkv), desc(cb.zbuf, L.in_z), desc(cb.bbuf, L.in_b), desc(cb.abuf, L.in_a)};
             LIN(xinfer_linear_int4_fused_f16(st, cb.normed, fd, 4, M, H, 128));
             NL(xb::conv1d_chunk(s, cb.wide2, cb.wide, L.conv_w, L.conv_state, B, Rc, ch));
-            NL(xb::gdn_chunk(s, cb.mix_out, cb.wide2, cb.zbuf, cb.bbuf, cb.abuf, L.A_log, L.dt_bias, L.gdn_norm, L.S, B, Rc, hv, hk));
+            NL(xb::gdn_chunk(s, cb.mix_out, cb.wide2, cb.zbuf, cb.bbuf, cb.abuf, L.A_log, L.dt_bias, L.gdn_norm, L.S, B, Rc, hv, hk, cb.gdn_scratch));
             LIN(xinfer_linear_int4_f16f16(st, cb.proj_out, cb.mix_out, L.out_proj.w, L.out_proj.s, nullptr, M, L.out_proj.n,
                                           L.out_proj.k, 128));
         }
@@ -954,7 +963,7 @@ void xinfer_spec_decoder_destroy(xinfer_spec_decoder* d) {
     if (d->graph) cudaGraphDestroy(d->graph);
     if (d->plan) xb::tc_plan_delete(d->plan);  // the recorded plan points into this decoder's weights
     if (d->arena) xinfer_arena_destroy(d->arena);
-    if (d->chunk.x) { cudaFree(d->chunk.x); cudaFree(d->chunk.attn_scratch); }
+    if (d->chunk.x) { cudaFree(d->chunk.x); cudaFree(d->chunk.attn_scratch); cudaFree(d->chunk.gdn_scratch); }
     if (d->h_emitted) cudaFreeHost(d->h_emitted);
     if (d->h_emitted_n) cudaFreeHost(d->h_emitted_n);
     delete d;
