@@ -200,6 +200,15 @@ uint64_t crc_update(uint64_t crc, const void* data, size_t n) {
 namespace xb {
 void set_last_error(const char* msg) { g_last_error = msg ? msg : ""; }
 
+int device_facts(int** status, int* num_sms) {
+    DeviceCtx* c = nullptr;
+    const int rc = get_ctx(&c);
+    if (rc != XINFER_OK) return rc;
+    *status = c->status;
+    *num_sms = c->num_sms;
+    return XINFER_OK;
+}
+
 int run_tc_linear(cudaStream_t s, const void* x, const TcProj* proj, int num, bool swiglu, bool out_f32, long long m,
                   long long k, int group_size, const TpLink* tp, int layout_flags) {
     DeviceCtx* c = nullptr;

@@ -189,8 +189,7 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(__half* q_out, __half* k
                                                         const float* q_norm_w, const float* k_norm_w, const int* ctx,
                                                         int rows_per_seq, int hq, int hkv, long long max_seq,
                                                         float eps, float log_theta, int rope_dim, int q_head_stride,
-                                                        const long long* positions, int ctx_base, __half* k_out,
-                                                        int cache_batch) {
+                                                        const long long* positions, int ctx_base, __half* k_out) {
     griddep_prologue();
     __shared__ float red[32];
     __shared__ float vals[256];
@@ -198,13 +197,12 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(__half* q_out, __half* k
     const int slot = blockIdx.y;
     const int d = threadIdx.x;
     const int b = row / rows_per_seq, i = row % rows_per_seq;
-    const int bc = cache_batch > 0 ? b % cache_batch : b;  // the sequence whose cache this entry writes (see attn_decode_ex)
     const long long pos = positions ? positions[row] : static_cast<long long>(ctx ? ctx[b] : ctx_base) + i;
     const bool in_cache = pos >= 0 && pos < max_seq;
     if (slot >= hq + hkv) {  // value head: plain copy into the cache
         const int h = slot - hq - hkv;
         if (in_cache && v_cache && v_in)
-            v_cache[((static_cast<long long>(bc) * max_seq + pos) * hkv + h) * 256 + d] =
+            v_cache[((static_cast<long long>(b) * max_seq + pos) * hkv + h) * 256 + d] =
                 v_in[(static_cast<long long>(row) * hkv + h) * 256 + d];
         return;
     }
@@ -237,341 +235,10 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(__half* q_out, __half* k
     if (is_q) {
         q_out[(static_cast<long long>(row) * hq + h) * 256 + d] = o;
     } else if (k_cache) {
-        if (in_cache) k_cache[((static_cast<long long>(bc) * max_seq + pos) * hkv + h) * 256 + d] = o;
+        if (in_cache) k_cache[((static_cast<long long>(b) * max_seq + pos) * hkv + h) * 256 + d] = o;
     } else if (k_out) {
         k_out[(static_cast<long long>(row) * hkv + h) * 256 + d] = o;
     }
-}
-
-// ------------------------------------------------------------------------------- split-KV GQA attention
-// Grid (splits, Hkv, B), 256 threads, two CTAs per SM.  Keys stream through shared memory in chunks of 32 via
-// cp.async, double buffered, and both products are computed transposed so that the G * R query rows that share
-// one KV head (G = Hq / Hkv, at most 32 rows) sit on the N side of mma.sync m16n8k16, eight rows per tile, and
-// nothing is padded to 16:
-//   S^T = K Q^T   warp (kq, kt) owns the keys [16 kt, 16 kt + 16) of the chunk and the head dims
-//                 [64 kq, 64 kq + 64); its slice of Q stays in registers as B fragments for the whole kernel,
-//                 so a chunk costs one read of K from shared memory and no read of Q; the four partial sums
-//                 over kq meet in shared memory, where the softmax threads add them;
-//   O^T += V^T P^T  warp w owns the output dims [32 w, 32 w + 32); V is read once per chunk (ldmatrix.trans).
-// The kernel is bound by shared-memory bandwidth (two CTAs per SM share it): per 32 KB chunk this layout moves
-// about 100 KB through shared memory where the untransposed one moved 165 KB.
-// Each CTA writes an unnormalised partial (max, sum, O) per row.
-constexpr int kAttnChunk = 32;
-constexpr int kAttnStages = 2;  // the loop below is written for exactly two slots
-constexpr int kAttnThreads = 256;
-constexpr int kAttnLd = 264;  // padded row of 256 halves (528 B): conflict-free ldmatrix
-constexpr int kAttnRows = 32;
-constexpr int kAttnSpLd = 36;  // row pitch (floats) of the score planes: 2 * 36 = 8 mod 32 makes the MMA threads' stores
-                               // conflict-free, 144-byte rows let a softmax thread fetch its four keys with one 16-byte load
-
-struct AttnSmem {
-    __half q[kAttnRows][kAttnLd];
-    __half k[kAttnStages][kAttnChunk][kAttnLd];
-    __half v[kAttnStages][kAttnChunk][kAttnLd];
-    float sp[4][kAttnRows][kAttnSpLd];  // score partial sums over the four dim quarters, [query row][key]
-    __half p[kAttnRows][kAttnChunk + 8];
-    float row_max[kAttnRows];   // running maximum of scale * log2(e) * score (the softmax runs in base 2)
-    float row_sum[kAttnRows];
-    float row_alpha[kAttnRows];
-};
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-__device__ __forceinline__ void ldmatrix_x4(uint32_t* r, const void* p) {
-    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
-}
-__device__ __forceinline__ void ldmatrix_x2(uint32_t* r, const void* p) {
-    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(a));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t* r, const void* p) {
-    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
-}
-__device__ __forceinline__ void ldmatrix_x2_trans(uint32_t* r, const void* p) {
-    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(a));
-}
-__device__ __forceinline__ void mma16816(float* c, const uint32_t* a, const uint32_t* b) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-        "{%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
-// NT = number of 8-row tiles that hold query rows (1..4): arrays and loops are sized for it at compile time.
-template <int NT>
-__global__ void __launch_bounds__(kAttnThreads, 2) attn_split_kernel(float* part_o, float* part_ml, const __half* q,
-                                                         const __half* k_cache, const __half* v_cache, const int* ctx,
-                                                         int rows_per_seq, int hq, int hkv, long long max_seq,
-                                                         float scale, int ctx_base, int cache_batch) {
-    griddep_prologue();
-    extern __shared__ __align__(16) uint8_t attn_smem_raw[];
-    AttnSmem& sm = *reinterpret_cast<AttnSmem*>(attn_smem_raw);
-    const int split = blockIdx.x, nsplit = gridDim.x, kvh = blockIdx.y, b = blockIdx.z;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int kq = warp >> 1, kt = warp & 1;  // S^T role: dim quarter, 16-key tile
-    const int G = hq / hkv;
-    const int nrows = G * rows_per_seq;  // valid query rows, row = g * R + i
-    const int ctx_b = ctx ? ctx[b] : ctx_base;  // (null: the stand-alone entry point's host-side start position)
-    const int bc = cache_batch > 0 ? b % cache_batch : b;
-    const float scale2 = scale * 1.4426950408889634f;  // exp(x) = exp2(x * log2 e)
-    long long total_keys = static_cast<long long>(ctx_b) + rows_per_seq;
-    if (total_keys > max_seq) total_keys = max_seq;
-    const int nchunks = static_cast<int>((total_keys + kAttnChunk - 1) / kAttnChunk);
-    const int c_begin = static_cast<int>(static_cast<long long>(split) * nchunks / nsplit);
-    const int c_end = static_cast<int>(static_cast<long long>(split + 1) * nchunks / nsplit);
-
-    // stage the query rows (zero padded to 32)
-    for (int idx = tid; idx < kAttnRows * 32; idx += kAttnThreads) {
-        const int r = idx >> 5, seg = idx & 31;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (r < nrows) {
-            const int g = r / rows_per_seq, i = r % rows_per_seq;
-            const long long row = static_cast<long long>(b) * rows_per_seq + i;
-            v = *reinterpret_cast<const uint4*>(q + (row * hq + kvh * G + g) * 256 + seg * 8);
-        }
-        *reinterpret_cast<uint4*>(&sm.q[r][seg * 8]) = v;
-    }
-    if (tid < kAttnRows) {
-        sm.row_max[tid] = -INFINITY;
-        sm.row_sum[tid] = 0.f;
-    }
-
-    // one cp.async group per chunk (an empty one past the split's end)
-    auto load_chunk = [&](int c, int buf) {
-        const long long key0 = static_cast<long long>(c) * kAttnChunk;
-        if (c < c_end)
-        for (int idx = tid; idx < kAttnChunk * 32; idx += kAttnThreads) {
-            const int r = idx >> 5, seg = idx & 31;
-            long long key = key0 + r;
-            if (key >= total_keys) key = total_keys - 1;  // clamped rows are masked out below
-            const long long off = ((static_cast<long long>(bc) * max_seq + key) * hkv + kvh) * 256 + seg * 8;
-            cp_async16(&sm.k[buf][r][seg * 8], k_cache + off);
-            cp_async16(&sm.v[buf][r][seg * 8], v_cache + off);
-        }
-        cp_async_commit();
-    };
-
-    // O^T accumulators: [16-dim tile][8-row tile]; element e of a tile is (dim g4 + 8 (e >> 1), row 2 t4 + (e & 1))
-    float o_acc[2][NT][4];
-#pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) o_acc[mi][nt][e] = 0.f;
-
-    for (int i = 0; i < kAttnStages - 1; ++i) load_chunk(c_begin + i, i);
-
-    // this warp's slice of Q (all rows, dims [64 kq, 64 kq + 64)) as B fragments, read once
-    __syncthreads();
-    uint32_t qf[4][NT][2];
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-            ldmatrix_x2(qf[ks][nt], &sm.q[nt * 8 + (lane & 7)][kq * 64 + ks * 16 + ((lane >> 3) & 1) * 8]);
-
-    for (int c = c_begin; c < c_end; ++c) {
-        const int buf = (c - c_begin) % kAttnStages;
-        // Chunk c has landed for every thread after this barrier, and every warp has finished the previous
-        // chunk's P V: the other slot may be refilled.  (Three barriers per chunk; requesting the next chunk
-        // before the wait instead would need a fourth one at the end of the iteration.)
-        cp_async_wait<0>();
-        __syncthreads();
-        load_chunk(c + 1, (c - c_begin + 1) % kAttnStages);
-
-        // S^T = K Q^T for this warp's 16 keys, summed over its 64 dims
-        {
-            float s_acc[NT][4];
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) s_acc[nt][e] = 0.f;
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-                uint32_t afr[4];
-                ldmatrix_x4(afr, &sm.k[buf][kt * 16 + (lane & 15)][kq * 64 + ks * 16 + (lane >> 4) * 8]);
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt)
-                    mma16816(s_acc[nt], afr, qf[ks][nt]);
-            }
-            const int g4 = lane >> 2, t4 = lane & 3;
-            float* sp0 = &sm.sp[kq][t4 * 2][kt * 16 + g4];
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
-                {
-                    // fragment element e: key g4 + 8 (e >> 1), query row 8 nt + 2 t4 + (e & 1)
-                    sp0[(nt * 8) * kAttnSpLd] = s_acc[nt][0];
-                    sp0[(nt * 8 + 1) * kAttnSpLd] = s_acc[nt][1];
-                    sp0[(nt * 8) * kAttnSpLd + 8] = s_acc[nt][2];
-                    sp0[(nt * 8 + 1) * kAttnSpLd + 8] = s_acc[nt][3];
-                }
-        }
-        __syncthreads();
-
-        // online softmax: 8 threads per row, 4 keys each
-        {
-            const int r = tid >> 3, part = tid & 7;
-            const int i = r % rows_per_seq;
-            const long long limit = static_cast<long long>(ctx_b) + i + 1;  // keys visible to this row
-            const long long key0 = static_cast<long long>(c) * kAttnChunk + part * 4;
-            float sc[4];
-            float mx = -INFINITY;
-            {
-                // this thread's four keys of its row, one 16-byte load per dim quarter
-                const float4 q0 = *reinterpret_cast<const float4*>(&sm.sp[0][r][part * 4]);
-                const float4 q1 = *reinterpret_cast<const float4*>(&sm.sp[1][r][part * 4]);
-                const float4 q2 = *reinterpret_cast<const float4*>(&sm.sp[2][r][part * 4]);
-                const float4 q3 = *reinterpret_cast<const float4*>(&sm.sp[3][r][part * 4]);
-                sc[0] = (q0.x + q1.x) + (q2.x + q3.x);
-                sc[1] = (q0.y + q1.y) + (q2.y + q3.y);
-                sc[2] = (q0.z + q1.z) + (q2.z + q3.z);
-                sc[3] = (q0.w + q1.w) + (q2.w + q3.w);
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const bool vis = (r < nrows) && (key0 + j < limit) && (key0 + j < total_keys);
-                sc[j] = vis ? sc[j] * scale2 : -INFINITY;
-                mx = fmaxf(mx, sc[j]);
-            }
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-            const float old_max = sm.row_max[r];
-            const float new_max = fmaxf(old_max, mx);
-            float sum = 0.f;
-            float pv[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                pv[j] = (sc[j] == -INFINITY) ? 0.f : exp2f(sc[j] - new_max);
-                sum += pv[j];
-            }
-            {
-                const __half2 p01 = __floats2half2_rn(pv[0], pv[1]), p23 = __floats2half2_rn(pv[2], pv[3]);
-                uint2 packed;
-                packed.x = *reinterpret_cast<const uint32_t*>(&p01);
-                packed.y = *reinterpret_cast<const uint32_t*>(&p23);
-                *reinterpret_cast<uint2*>(&sm.p[r][part * 4]) = packed;
-            }
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-            __syncwarp();
-            if (part == 0) {
-                const float alpha = (old_max == -INFINITY) ? 0.f : exp2f(old_max - new_max);
-                sm.row_alpha[r] = alpha;
-                sm.row_sum[r] = sm.row_sum[r] * alpha + sum;
-                sm.row_max[r] = new_max;
-            }
-        }
-        __syncthreads();
-
-        // O^T = alpha * O^T + V^T P^T for this warp's 32 output dims
-        {
-            const int t4 = lane & 3;
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                const float a0 = sm.row_alpha[nt * 8 + t4 * 2], a1 = sm.row_alpha[nt * 8 + t4 * 2 + 1];
-#pragma unroll
-                for (int mi = 0; mi < 2; ++mi) {
-                    o_acc[mi][nt][0] *= a0;
-                    o_acc[mi][nt][1] *= a1;
-                    o_acc[mi][nt][2] *= a0;
-                    o_acc[mi][nt][3] *= a1;
-                }
-            }
-            // P^T as B fragments: one ldmatrix.x4 per 8-row tile fetches the chunk's 32 keys (both 16-key steps)
-            uint32_t pall[NT][4];
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) ldmatrix_x4(pall[nt], &sm.p[nt * 8 + (lane & 7)][(lane >> 3) * 8]);
-#pragma unroll
-            for (int ks = 0; ks < kAttnChunk / 16; ++ks) {
-                uint32_t pfr[NT][2];
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    pfr[nt][0] = pall[nt][2 * ks];
-                    pfr[nt][1] = pall[nt][2 * ks + 1];
-                }
-#pragma unroll
-                for (int mi = 0; mi < 2; ++mi) {
-                    // A = V^T: matrix j = lane >> 3 of the four 8x8 blocks is (dims + 8 (j & 1), keys + 8 (j >> 1)),
-                    // stored key-major, hence the transposing load
-                    uint32_t afr[4];
-                    const int j = lane >> 3;
-                    ldmatrix_x4_trans(afr, &sm.v[buf][ks * 16 + (j >> 1) * 8 + (lane & 7)][warp * 32 + mi * 16 + (j & 1) * 8]);
-#pragma unroll
-                    for (int nt = 0; nt < NT; ++nt)
-                        mma16816(o_acc[mi][nt], afr, pfr[nt]);
-                }
-            }
-        }
-    }
-    cp_async_wait<0>();
-
-    // write the partial: O [rows][256] fp32, (max in base-2 units, sum) per row
-    const long long pbase = (static_cast<long long>(b) * hkv + kvh) * nsplit + split;
-    float* po = part_o + pbase * (kAttnRows * 256);
-    const int g4 = lane >> 2, t4 = lane & 3;
-#pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int r = nt * 8 + t4 * 2 + (e & 1);
-                const int col = warp * 32 + mi * 16 + g4 + (e >> 1) * 8;
-                if (r < nrows) po[r * 256 + col] = o_acc[mi][nt][e];
-            }
-    if (tid < nrows) {
-        part_ml[pbase * (kAttnRows * 2) + tid * 2] = sm.row_max[tid];
-        part_ml[pbase * (kAttnRows * 2) + tid * 2 + 1] = sm.row_sum[tid];
-    }
-}
-
-// Merge the splits, normalise, apply the sigmoid output gate, write fp16 [rows][Hq * 256].
-// Grid (G * R, Hkv, B), 256 threads = head_dim.
-__global__ void __launch_bounds__(256) attn_combine_kernel(__half* out, const float* part_o, const float* part_ml,
-                                                           const __half* q_gate, int nsplit, int rows_per_seq, int hq,
-                                                           int hkv, int perm_out) {
-    griddep_prologue();
-    const int r = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z, d = threadIdx.x;
-    const int G = hq / hkv;
-    const int g = r / rows_per_seq, i = r % rows_per_seq;
-    const long long pbase = (static_cast<long long>(b) * hkv + kvh) * nsplit;
-    float m = -INFINITY;
-    for (int s = 0; s < nsplit; ++s) m = fmaxf(m, part_ml[(pbase + s) * (kAttnRows * 2) + r * 2]);
-    float acc = 0.f, l = 0.f;
-    for (int s = 0; s < nsplit; ++s) {
-        const float ms = part_ml[(pbase + s) * (kAttnRows * 2) + r * 2];
-        if (ms == -INFINITY) continue;
-        const float w = exp2f(ms - m);  // the partial maxima are in base-2 units
-        l += part_ml[(pbase + s) * (kAttnRows * 2) + r * 2 + 1] * w;
-        acc += part_o[(pbase + s) * (kAttnRows * 256) + r * 256 + d] * w;
-    }
-    const float inv = 1.0f / (l > 0.f ? l : 1.0f);
-    const long long row = static_cast<long long>(b) * rows_per_seq + i;
-    const int h = kvh * G + g;
-    // rounding point: the reference's SDPA writes fp16, the gate then multiplies in fp32
-    const float attn = __half2float(__float2half_rn(acc * inv));
-    if (!q_gate) {  // plain SDPA (the stand-alone entry point): no output gate
-        out[(row * hq + h) * 256 + d] = __float2half_rn(acc * inv);
-        return;
-    }
-    const float gate = __half2float(q_gate[(row * hq + h) * 512 + 256 + d]);
-    const float sig = 1.0f / (1.0f + expf(-gate));
-    out[(row * hq + h) * 256 + (perm_out ? perm8(d) : d)] = __float2half_rn(attn * sig);
 }
 
 // ------------------------------------------------------------------------------- causal conv1d + SiLU
@@ -769,8 +436,7 @@ __global__ void __launch_bounds__(512, 2) gdn_spec_kernel(__half* out, const __h
 }
 
 // ------------------------------------------------------------------------------- the same two mixers over a prompt chunk
-// Prefill keeps every row, so there is nothing to replay or to hold back.  Rows are found through chunk_row (the chunk's
-// group-by-group row order; with one sequence simply the positions).
+// Prefill keeps every row, so there is nothing to replay or to hold back.  Rows are [sequence][position].
 //
 // The convolution has no recurrence on its outputs (y_p needs the inputs p-3 .. p only): a thread takes V channels and
 // `span` consecutive positions with the window in registers.  The threads of the first positions are the only readers of
@@ -782,13 +448,14 @@ __global__ void __launch_bounds__(128) conv1d_chunk_kernel(__half* out, const __
                                                            int channels, int span) {
     griddep_prologue();
     const int c = (blockIdx.z * 128 + threadIdx.x) * V;
-    const int b = blockIdx.y, batch = gridDim.y, p0 = blockIdx.x * span;
+    const int b = blockIdx.y, p0 = blockIdx.x * span;
+    const long long seq0 = static_cast<long long>(b) * rc;
     if (c >= channels) return;
     float* st = state ? state + static_cast<long long>(b) * 3 * channels : nullptr;
     struct alignas(2 * V) Vec { __half h[V]; };
     auto load = [&](int p, float (&x)[V]) {  // the input at position p; negative: the state's slot 3 + p
         if (p >= 0) {
-            const Vec v = *reinterpret_cast<const Vec*>(in + chunk_row(p, b, batch, rc) * channels + c);
+            const Vec v = *reinterpret_cast<const Vec*>(in + (seq0 + p) * channels + c);
 #pragma unroll
             for (int e = 0; e < V; ++e) x[e] = __half2float(v.h[e]);
         } else {
@@ -823,7 +490,7 @@ __global__ void __launch_bounds__(128) conv1d_chunk_kernel(__half* out, const __
             x1[e] = x2[e];
             x2[e] = x[e];
         }
-        *reinterpret_cast<Vec*>(out + chunk_row(p, b, batch, rc) * channels + c) = o;
+        *reinterpret_cast<Vec*>(out + (seq0 + p) * channels + c) = o;
     }
     if (p0 == 0 && st) {
 #pragma unroll
@@ -879,7 +546,8 @@ __global__ void __cluster_dims__(kGdnSlices, 1, 1) __launch_bounds__(kGdnThreads
     __shared__ float4 sh_gate[2][kGdnBlock];                 // decay, beta, q.k
     __shared__ float sh_sq[2][kGdnSlices][kGdnBlock];        // sums of squares of the outputs, by column slice
     __shared__ float sh_s[128][kGdnCols + 1];
-    const int slice = blockIdx.x % kGdnSlices, h = blockIdx.x / kGdnSlices, b = blockIdx.y, batch = gridDim.y;
+    const int slice = blockIdx.x % kGdnSlices, h = blockIdx.x / kGdnSlices, b = blockIdx.y;
+    const long long seq0 = static_cast<long long>(b) * rc;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int cl = lane >> 3, rg = lane & 7, col = warp * 4 + cl;  // rows of a lane: 4 (rg + 8 m) + e, m, e = 0..3
     const int h_k = h / (hv / hk), channels = 2 * hk * 128 + hv * 128, value_dim = hv * 128;
@@ -919,13 +587,13 @@ __global__ void __cluster_dims__(kGdnSlices, 1, 1) __launch_bounds__(kGdnThreads
         for (int u = 0; u < kGdnBlock / 4; ++u) {
             const int p = p0 + warp + 4 * u;
             if (p < rc) {
-                const __half* cur = qkv + chunk_row(p, b, batch, rc) * channels + h_k * 128 + lane * 4;
+                const __half* cur = qkv + (seq0 + p) * channels + h_k * 128 + lane * 4;
                 rq[u] = *reinterpret_cast<const uint2*>(cur);
                 rk[u] = *reinterpret_cast<const uint2*>(cur + hk * 128);
             }
         }
         if (p0 + ot < rc) {
-            const long long row = chunk_row(p0 + ot, b, batch, rc);
+            const long long row = (seq0 + p0 + ot);
             rv = *reinterpret_cast<const __half2*>(qkv + row * channels + 2 * hk * 128 + h * 128 + col0 + oc);
             if ((tid & 7) == 0) { ra = aa[row * hv + h]; rb = bb[row * hv + h]; }
         }
@@ -971,7 +639,7 @@ __global__ void __cluster_dims__(kGdnSlices, 1, 1) __launch_bounds__(kGdnThreads
 #pragma unroll
             for (int r = 0; r < kGdnSlices; ++r) sq += sh_sq[buf][r][ot];
             const float inv_std = 1.0f / sqrtf(sq / 128.0f + 1e-6f);
-            const long long at = chunk_row(p0 + ot, b, batch, rc) * value_dim + h * 128 + col0 + oc;
+            const long long at = (seq0 + p0 + ot) * value_dim + h * 128 + col0 + oc;
             const float2 zv = __half22float2(*reinterpret_cast<const __half2*>(z + at));
             const float y0 = o0 * inv_std * nw0 * (zv.x / (1.0f + expf(-zv.x))), y1 = o1 * inv_std * nw1 * (zv.y / (1.0f + expf(-zv.y)));
             *reinterpret_cast<__half2*>(out + at) = __floats2half2_rn(y0, y1);
@@ -1107,7 +775,8 @@ __global__ void __launch_bounds__(128) gdn_block_kernel(GdnBlock* blocks, const 
     __shared__ float sh_lg[4][kScanBlock], sh_ik[4][kScanBlock], sh_iq[4][kScanBlock], sh_beta[4][kScanBlock];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int nblocks = (rc + kScanBlock - 1) / kScanBlock;
-    const int blk = blockIdx.x * 4 + warp, h = blockIdx.y, b = blockIdx.z, batch = gridDim.z;
+    const int blk = blockIdx.x * 4 + warp, h = blockIdx.y, b = blockIdx.z;
+    const long long seq0 = static_cast<long long>(b) * rc;
     if (blk >= nblocks) return;  // (no barrier below spans warps)
     const int p0 = blk * kScanBlock, h_k = h / (hv / hk), channels = 2 * hk * 128 + hv * 128;
     GdnBlock& out = blocks[(static_cast<long long>(b) * hv + h) * nblocks + blk];
@@ -1119,7 +788,7 @@ __global__ void __launch_bounds__(128) gdn_block_kernel(GdnBlock* blocks, const 
     for (int r = 0; r < 2; ++r) {
         const int p = p0 + g + 8 * r;
         live[r] = p < rc;
-        q_row[r] = qkv + chunk_row(live[r] ? p : p0, b, batch, rc) * channels + h_k * 128;
+        q_row[r] = qkv + (seq0 + (live[r] ? p : p0)) * channels + h_k * 128;
         k_row[r] = q_row[r] + hk * 128;
     }
     float kk[2][4] = {}, qk[2][4] = {}, k_sq[2] = {0.f, 0.f}, q_sq[2] = {0.f, 0.f};
@@ -1155,7 +824,7 @@ __global__ void __launch_bounds__(128) gdn_block_kernel(GdnBlock* blocks, const 
     // log of the cumulative decay and beta; positions behind the end decay nothing and write nothing
     float lg = 0.f, beta = 0.f;
     if (lane < kScanBlock && p0 + lane < rc) {
-        const long long row = chunk_row(p0 + lane, b, batch, rc);
+        const long long row = (seq0 + p0 + lane);
         const float a_val = __half2float(aa[row * hv + h]) + dt_bias[h];
         const float softplus = (a_val > 20.0f) ? a_val : logf(1.0f + expf(a_val));
         lg = -expf(A_log[h]) * softplus;
@@ -1233,7 +902,8 @@ __global__ void __cluster_dims__(kScanSlices, 1, 1) __launch_bounds__(32 * kScan
     griddep_prologue();
     __shared__ __align__(16) __half sh_q[2][kScanBlock][kScanPitch], sh_k[2][kScanBlock][kScanPitch];
     __shared__ float sh_sq[2][kScanSlices * kScanWarps][kScanBlock];  // sums of squares of the outputs, by warp of the cluster
-    const int slice = blockIdx.x % kScanSlices, h = blockIdx.x / kScanSlices, b = blockIdx.y, batch = gridDim.y;
+    const int slice = blockIdx.x % kScanSlices, h = blockIdx.x / kScanSlices, b = blockIdx.y;
+    const long long seq0 = static_cast<long long>(b) * rc;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int nblocks = (rc + kScanBlock - 1) / kScanBlock;
     const int h_k = h / (hv / hk), channels = 2 * hk * 128 + hv * 128, value_dim = hv * 128;
@@ -1247,7 +917,7 @@ __global__ void __cluster_dims__(kScanSlices, 1, 1) __launch_bounds__(32 * kScan
 #pragma unroll
         for (int u = 0; u < kScanBlock * 16 / (32 * kScanWarps); ++u) {
             const int idx = u * 32 * kScanWarps + tid, row = idx >> 4, c = (idx & 15) * 8, p = n * kScanBlock + row;
-            const __half* cur = qkv + chunk_row(p < rc ? p : n * kScanBlock, b, batch, rc) * channels + h_k * 128 + c;
+            const __half* cur = qkv + (seq0 + (p < rc ? p : n * kScanBlock)) * channels + h_k * 128 + c;
             const int bytes = p < rc ? 16 : 0;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(&sh_q[buf][row][c])), "l"(cur), "r"(bytes) : "memory");
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(&sh_k[buf][row][c])), "l"(cur + hk * 128), "r"(bytes) : "memory");
@@ -1262,7 +932,7 @@ __global__ void __cluster_dims__(kScanSlices, 1, 1) __launch_bounds__(32 * kScan
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int j = 8 * (i >> 1) + 2 * t + (i & 1), p = n * kScanBlock + j;
-            const __half* cur = qkv + chunk_row(p < rc ? p : n * kScanBlock, b, batch, rc) * channels + 2 * hk * 128 + h * 128 + c0;
+            const __half* cur = qkv + (seq0 + (p < rc ? p : n * kScanBlock)) * channels + 2 * hk * 128 + h * 128 + c0;
             rv[0][i] = p < rc ? cur[0] : __half(0.f);
             rv[1][i] = p < rc ? cur[8] : __half(0.f);
             rcoef[i] = __ldg(&blk[n].coef[j]);
@@ -1296,7 +966,7 @@ __global__ void __cluster_dims__(kScanSlices, 1, 1) __launch_bounds__(32 * kScan
     __half zv[2][4];
     auto out_row = [&](int n, int i) -> long long {
         const int p = n * kScanBlock + 8 * (i >> 1) + 2 * t + (i & 1);
-        return p < rc ? chunk_row(p, b, batch, rc) * value_dim + h * 128 + c0 : -1;
+        return p < rc ? (seq0 + p) * value_dim + h * 128 + c0 : -1;
     };
     auto fetch_z = [&](int n) {
 #pragma unroll
@@ -1550,55 +1220,10 @@ int attn_prep(cudaStream_t s, __half* q_out, __half* k_cache, __half* v_cache, c
 int attn_prep_ex(cudaStream_t s, __half* q_out, __half* k_cache, __half* v_cache, const __half* q_in, const __half* k_in,
                  const __half* v_in, const float* q_norm_w, const float* k_norm_w, const int* ctx, int batch,
                  int rows_per_seq, int hq, int hkv, long long max_seq, float eps, float rope_theta, int rope_dim,
-                 int q_head_stride, const long long* positions, int ctx_base, __half* k_out, int cache_batch) {
+                 int q_head_stride, const long long* positions, int ctx_base, __half* k_out) {
     dim3 grid(batch * rows_per_seq, hq + 2 * hkv);
     launch_pdl(attn_prep_kernel, dim3(grid), dim3(256), 0, s, q_out, k_cache, v_cache, q_in, k_in, v_in, q_norm_w, k_norm_w, ctx,
-               rows_per_seq, hq, hkv, max_seq, eps, logf(rope_theta), rope_dim, q_head_stride, positions, ctx_base, k_out, cache_batch);
-    return XB_LAUNCH_OK();
-}
-
-size_t attn_scratch_bytes(int batch, int hkv, int nsplit) {
-    return static_cast<size_t>(batch) * hkv * nsplit * (kAttnRows * 256 + kAttnRows * 2) * sizeof(float);
-}
-
-int attn_decode(cudaStream_t s, __half* out, const __half* q, const __half* q_gate, const __half* k_cache,
-                const __half* v_cache, const int* ctx, int batch, int rows_per_seq, int hq, int hkv, long long max_seq,
-                int nsplit, float* scratch) {
-    return attn_decode_ex(s, out, q, q_gate, k_cache, v_cache, ctx, batch, rows_per_seq, hq, hkv, max_seq, nsplit, scratch,
-                          1.0f / sqrtf(256.0f), 0, 0);
-}
-
-int attn_decode_ex(cudaStream_t s, __half* out, const __half* q, const __half* q_gate, const __half* k_cache,
-                   const __half* v_cache, const int* ctx, int batch, int rows_per_seq, int hq, int hkv, long long max_seq,
-                   int nsplit, float* scratch, float scale, int ctx_base, int perm_out, int cache_batch) {
-    if (hq % hkv != 0 || (hq / hkv) * rows_per_seq > kAttnRows) return -2;
-    // the shared-memory attribute belongs to the device's context: set it once per device
-    static bool configured_dev[64];
-    static std::mutex configured_mu;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
-    std::lock_guard<std::mutex> lock(configured_mu);
-    if (!configured_dev[dev]) {
-        const int bytes = static_cast<int>(sizeof(AttnSmem));
-        if (cudaFuncSetAttribute(attn_split_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
-            cudaFuncSetAttribute(attn_split_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
-            cudaFuncSetAttribute(attn_split_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
-            cudaFuncSetAttribute(attn_split_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
-            return -1;
-        configured_dev[dev] = true;
-    }
-    float* part_o = scratch;
-    float* part_ml = scratch + static_cast<size_t>(batch) * hkv * nsplit * (kAttnRows * 256);
-    dim3 grid(nsplit, hkv, batch);
-    switch (((hq / hkv) * rows_per_seq + 7) / 8) {
-        case 1: launch_pdl(attn_split_kernel<1>, dim3(grid), dim3(kAttnThreads), sizeof(AttnSmem), s, part_o, part_ml, q, k_cache, v_cache, ctx, rows_per_seq, hq, hkv, max_seq, scale, ctx_base, cache_batch); break;
-        case 2: launch_pdl(attn_split_kernel<2>, dim3(grid), dim3(kAttnThreads), sizeof(AttnSmem), s, part_o, part_ml, q, k_cache, v_cache, ctx, rows_per_seq, hq, hkv, max_seq, scale, ctx_base, cache_batch); break;
-        case 3: launch_pdl(attn_split_kernel<3>, dim3(grid), dim3(kAttnThreads), sizeof(AttnSmem), s, part_o, part_ml, q, k_cache, v_cache, ctx, rows_per_seq, hq, hkv, max_seq, scale, ctx_base, cache_batch); break;
-        default: launch_pdl(attn_split_kernel<4>, dim3(grid), dim3(kAttnThreads), sizeof(AttnSmem), s, part_o, part_ml, q, k_cache, v_cache, ctx, rows_per_seq, hq, hkv, max_seq, scale, ctx_base, cache_batch); break;
-    }
-    dim3 grid2((hq / hkv) * rows_per_seq, hkv, batch);
-    launch_pdl(attn_combine_kernel, dim3(grid2), dim3(256), 0, s, out, part_o, part_ml, q_gate, nsplit, rows_per_seq, hq, hkv,
-               (q_gate && perm_out) ? 1 : 0);
+               rows_per_seq, hq, hkv, max_seq, eps, logf(rope_theta), rope_dim, q_head_stride, positions, ctx_base, k_out);
     return XB_LAUNCH_OK();
 }
 

@@ -29,18 +29,24 @@ int attn_prep(cudaStream_t s, __half* q_out, __half* k_cache, __half* v_cache, c
 int attn_prep_ex(cudaStream_t s, __half* q_out, __half* k_cache, __half* v_cache, const __half* q_in, const __half* k_in,
                  const __half* v_in, const float* q_norm_w, const float* k_norm_w, const int* ctx, int batch,
                  int rows_per_seq, int hq, int hkv, long long max_seq, float eps, float rope_theta, int rope_dim,
-                 int q_head_stride, const long long* positions, int ctx_base, __half* k_out, int cache_batch = 0);
-size_t attn_scratch_bytes(int batch, int hkv, int nsplit);
-// causal GQA attention over the cache (row i of sequence b sees keys below ctx[b] + i + 1), then * sigmoid(gate)
-int attn_decode(cudaStream_t s, __half* out, const __half* q, const __half* q_gate, const __half* k_cache,
-                const __half* v_cache, const int* ctx, int batch, int rows_per_seq, int hq, int hkv, long long max_seq,
-                int nsplit, float* scratch);
-// with an explicit softmax scale, a host-side context length when ctx is null, and no output gate when q_gate is null.
-// cache_batch > 0 (here and in attn_prep_ex): entry e of the `batch` entries works on the cache of sequence
-// e % cache_batch with its own ctx[e], so one launch can take several row groups of every sequence (prefill).
-int attn_decode_ex(cudaStream_t s, __half* out, const __half* q, const __half* q_gate, const __half* k_cache,
-                   const __half* v_cache, const int* ctx, int batch, int rows_per_seq, int hq, int hkv, long long max_seq,
-                   int nsplit, float* scratch, float scale, int ctx_base, int perm_out = 0, int cache_batch = 0);
+                 int q_head_stride, const long long* positions, int ctx_base, __half* k_out);
+// Causal GQA attention over the cache (row i of sequence b sees keys below ctx[b] + i + 1), then * sigmoid(gate).
+struct AttnTiles {
+    __half* out = nullptr;             // [batch][rows_per_seq][hq][256]
+    const __half *q = nullptr, *k_cache = nullptr, *v_cache = nullptr;  // 16-byte aligned
+    const __half* q_gate = nullptr;    // [batch][rows_per_seq][hq][512], the gate in the upper 256, 16-byte aligned; null: no gate
+    const int* ctx = nullptr;          // per sequence; null: ctx_base
+    int ctx_base = 0;
+    int batch = 1, rows_per_seq = 1, hq = 1, hkv = 1;  // hq / hkv <= 128
+    // rows of a sequence's cache that hold keys (what is behind a row's own limit must still be finite), and its row stride
+    long long cache_rows = 0, cache_stride = 0;
+    float scale = 1.f;
+    int perm_out = 0;                  // see perm_out of rmsnorm_rows
+    int early = 0;                     // ctx, and the keys below it, were not written by the launch directly in front
+    float* scratch = nullptr;          // attn_tile_scratch_bytes
+};
+size_t attn_tile_scratch_bytes(int batch, int rows_per_seq, int hq, int hkv, int num_sms);
+int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status);
 
 // state [batch][3][channels], pending [batch][8][channels] fp32.  The first min(n_commit[b], prev_rows) pending
 // inputs of the previous call are committed to the state before the new rows are processed (n_commit null:
@@ -56,17 +62,8 @@ int gdn_spec(cudaStream_t s, __half* out, const __half* qkv, const __half* z, co
              float* pend_g, const int* n_commit, int batch, int rows_per_seq, int prev_rows, int hv, int hk, int nc_base = 0,
              int early_state = 0, int perm_out = 0);
 
-// Row of (position p, sequence b) in a prefill chunk of rc positions per sequence.  The step's mixer kernels take at
-// most a few rows per sequence and launch, laid out [sequence][row]; a projection does not care about the order of its
-// rows.  So a chunk's rows are stored group by group: group j holds positions 4j .. 4j+3 of every sequence as one
-// contiguous [sequence][row] block, which such a launch takes as it is.
-__host__ __device__ inline long long chunk_row(int p, int b, int batch, int rc) {
-    const int j = p >> 2, i = p & 3;
-    const int rj = (rc - 4 * j) < 4 ? (rc - 4 * j) : 4;
-    return static_cast<long long>(j) * batch * 4 + static_cast<long long>(b) * rj + i;
-}
-// The convolution and the gated delta rule over all rc positions of a prefill chunk in one launch each (rows in
-// chunk_row order, every row kept, the state read once and written back once; nothing pending afterwards).  A null
+// The convolution and the gated delta rule over all rc positions of a prefill chunk in one launch each (rows
+// [sequence][position], every row kept, the state read once and written back once; nothing pending afterwards).  A null
 // convolution state means zeros; zero_state starts the recurrence from zeros.
 int conv1d_chunk(cudaStream_t s, __half* out, const __half* in, const float* conv_w, float* state, int batch, int rc,
                  int channels);

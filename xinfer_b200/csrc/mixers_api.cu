@@ -23,7 +23,6 @@
 namespace {
 
 constexpr int kMaxDevices = 64;
-constexpr int kSdpaSplits = 8;
 
 // Scratch of the stand-alone entry points, per device, grown on demand (the speculative decoder has its own).
 struct MixerScratch {
@@ -125,20 +124,29 @@ int xinfer_sdpa_causal_cached_f16(xinfer_stream_t s, void* out, const void* Q, c
     const int hq = static_cast<int>(num_q_heads), hkv = static_cast<int>(num_kv_heads);
     const int group = hq / hkv;
     if (group > 32) return XINFER_ERR_INVALID_ARGUMENT;
-    const int rows_max = 32 / group;  // query rows that share a KV head fill at most 32 MMA columns per launch
-    float* scr = nullptr;
-    int rc = scratch(xb::attn_scratch_bytes(1, hkv, kSdpaSplits), &scr);
+    int *status = nullptr, num_sms = 0;
+    int rc = xb::device_facts(&status, &num_sms);
     if (rc != XINFER_OK) return rc;
-    const float sc = scale > 0.f ? scale : 1.0f / sqrtf(256.0f);  // src/ops/attention.cpp:165-167
-    const long long cap = max_seq_len > 0 ? max_seq_len : (1ll << 40);
-    const __half* q = static_cast<const __half*>(Q);
-    __half* o = static_cast<__half*>(out);
-    // the kernel takes the tokens of one launch as "rows of one sequence"; longer inputs go chunk by chunk
-    for (int64_t t0 = 0; t0 < num_q_tokens; t0 += rows_max) {
-        const int rows = static_cast<int>(num_q_tokens - t0 < rows_max ? num_q_tokens - t0 : rows_max);
-        rc = xb::attn_decode_ex(static_cast<cudaStream_t>(s), o + t0 * hq * 256, q + t0 * hq * 256, nullptr,
-                                static_cast<const __half*>(k_cache), static_cast<const __half*>(v_cache), nullptr, 1, rows, hq,
-                                hkv, cap, kSdpaSplits, scr, sc, static_cast<int>(start_pos + t0));
+    xb::AttnTiles a;
+    a.k_cache = static_cast<const __half*>(k_cache);
+    a.v_cache = static_cast<const __half*>(v_cache);
+    a.hq = hq;
+    a.hkv = hkv;
+    a.scale = scale > 0.f ? scale : 1.0f / sqrtf(256.0f);  // src/ops/attention.cpp:165-167
+    // pieces of rows that keep the count of (128-row tile, 64-key block) units of a launch well inside 32 bits
+    const int64_t tile_pos = 128 / group, blocks = (start_pos + num_q_tokens) / 64 + 1;
+    int64_t piece = (int64_t{1} << 29) / (blocks * hkv) * tile_pos;
+    piece = piece < tile_pos ? tile_pos : (piece < 65536 ? piece : 65536);
+    const int most = static_cast<int>(num_q_tokens < piece ? num_q_tokens : piece);
+    rc = scratch(xb::attn_tile_scratch_bytes(1, most, hq, hkv, num_sms), &a.scratch);
+    if (rc != XINFER_OK) return rc;
+    for (int64_t t0 = 0; t0 < num_q_tokens; t0 += piece) {
+        a.rows_per_seq = static_cast<int>(num_q_tokens - t0 < piece ? num_q_tokens - t0 : piece);
+        a.ctx_base = static_cast<int>(start_pos + t0);
+        a.cache_rows = a.cache_stride = start_pos + t0 + a.rows_per_seq;
+        a.out = static_cast<__half*>(out) + t0 * hq * 256;
+        a.q = static_cast<const __half*>(Q) + t0 * hq * 256;
+        rc = xb::attn_tiles(static_cast<cudaStream_t>(s), a, num_sms, status);
         if (rc != 0) return ok_or_cuda(rc);
     }
     return XINFER_OK;

@@ -83,33 +83,23 @@ __global__ void last_prompt_token_kernel(long long* cur_tok, const long long* pr
     if (b < batch) cur_tok[b] = prompt[static_cast<long long>(b) * T + T - 1];
 }
 
-// Prefill chunks: rows in chunk_row order (mixers.h).
+// Prefill chunks: rows are [sequence][position of the chunk].
 __global__ void gather_prompt_chunk_kernel(long long* rows, const long long* prompt, int batch, long long T, long long c0, int Rc) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= batch * Rc) return;
-    const int b = t / Rc, p = t % Rc;
-    rows[xb::chunk_row(p, b, batch, Rc)] = prompt[static_cast<long long>(b) * T + c0 + p];
+    if (t < batch * Rc) rows[t] = prompt[static_cast<long long>(t / Rc) * T + c0 + t % Rc];
 }
 // The hidden state in front of every row of a chunk: position 0 <- h_last[b], position p <- x at position p - 1.
 __global__ void shift_hidden_chunk_kernel(__half* out, const __half* h_last, const __half* x, int batch, int Rc, int H) {
     const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= static_cast<long long>(batch) * Rc * H) return;
-    const int col = static_cast<int>(t % H);
-    const long long bp = t / H;
-    const int b = static_cast<int>(bp / Rc), p = static_cast<int>(bp % Rc);
-    out[xb::chunk_row(p, b, batch, Rc) * H + col] =
-        p == 0 ? h_last[static_cast<long long>(b) * H + col] : x[xb::chunk_row(p - 1, b, batch, Rc) * H + col];
-}
-// entry e = group * batch + sequence of a chunk that starts at position c0: the keys in front of its first row
-__global__ void chunk_entry_ctx_kernel(int* entry_ctx, int entries, int batch, int c0) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < entries) entry_ctx[e] = c0 + 4 * (e / batch);
+    const int row = static_cast<int>(t / H), col = static_cast<int>(t % H);
+    out[t] = row % Rc == 0 ? h_last[static_cast<long long>(row / Rc) * H + col] : x[t - H];
 }
 __global__ void take_last_hidden_chunk_kernel(__half* h_last, const __half* x, int batch, int Rc, int H) {
     const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= static_cast<long long>(batch) * H) return;
     const int b = static_cast<int>(t / H), col = static_cast<int>(t % H);
-    h_last[t] = x[xb::chunk_row(Rc - 1, b, batch, Rc) * H + col];
+    h_last[t] = x[(static_cast<long long>(b) * Rc + Rc - 1) * H + col];
 }
 
 // A projection as this rank holds it: `n` output rows starting at row `row0` of the full [n_full][k] matrix
@@ -144,7 +134,9 @@ struct Layer {
 
 struct xinfer_spec_decoder {
     xinfer_model_config cfg{};
-    int batch = 0, k = 0, attn_splits = 8;
+    int batch = 0, k = 0;
+    int num_sms = 0;
+    int* status = nullptr;  // the device's status word
     int64_t max_seq = 0;
     uint64_t seed = 0;
     int device = 0;
@@ -190,10 +182,8 @@ struct xinfer_spec_decoder {
                *qbuf = nullptr, *kbuf = nullptr, *vbuf = nullptr, *mix_out = nullptr, *zbuf = nullptr, *bbuf = nullptr,
                *abuf = nullptr, *cat = nullptr, *hprev = nullptr;
         long long* tokens = nullptr;
-        int* entry_ctx = nullptr;        // context length in front of every (group, sequence) entry of a chunk
         void* gdn_scratch = nullptr;     // per-block operands of the delta rule
-        float* attn_scratch = nullptr;   // split partials of one attention launch over all entries
-        int attn_splits = 1;
+        float* attn_scratch = nullptr;   // partials of one attention launch
     } chunk;
     float top_p = 1.0f;               // < 1: nucleus sampling on both sides of the stochastic rule
     xb::Nucleus* nucleus = nullptr;   // [batch * (k + 1)] nuclei of the verify rows
@@ -377,16 +367,8 @@ void build_all(Dec* d) {
     d->delta_out = xalloc(d, static_cast<size_t>(M) * hv * 128);
     // (row, chunk) partials of the sampling kernels, one block per vocabulary slice
     d->partials = xalloc(d, static_cast<size_t>(d->world) * xb::sampling_scratch_bytes(M, d->vocab_local) / sizeof(__half));
-    {
-        // KV splits: with one attention CTA per SM, two waves of CTAs over (split, kv head, sequence)
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device);
-        const int units = d->bl * static_cast<int>(c.num_key_value_heads);
-        int splits = (2 * sms) / (units > 0 ? units : 1);
-        d->attn_splits = splits < 1 ? 1 : (splits > 16 ? 16 : splits);
-    }
-    d->attn_scratch = dalloc<float>(
-        d, xb::attn_scratch_bytes(d->bl, static_cast<int>(c.num_key_value_heads), d->attn_splits) / sizeof(float), true);
+    d->attn_scratch = dalloc<float>(d, xb::attn_tile_scratch_bytes(d->bl, k + 1, static_cast<int>(c.num_attention_heads),
+                                                                   static_cast<int>(c.num_key_value_heads), d->num_sms) / sizeof(float), true);
     if (d->sizing) d->seed = seed0;  // the real pass draws the same seeds again
 }
 
@@ -519,10 +501,23 @@ int layer_forward(Dec* d, cudaStream_t s, Layer& L, int R, __half* xr, const flo
                          d->q_gate.p + static_cast<size_t>(row0) * hq * 512, d->kbuf.p + static_cast<size_t>(row0) * hkv * 256,
                          d->vbuf.p + static_cast<size_t>(row0) * hkv * 256, L.q_norm, L.k_norm, ctx + d->b0, Bl, R, hq, hkv,
                          d->max_seq, c.rms_norm_eps, c.rope_theta, c.rope_dim));
-        NL(xb::attn_decode_ex(s, d->attn_out.p + static_cast<size_t>(row0) * hq * 256,
-                              d->qbuf + static_cast<size_t>(row0) * hq * 256, d->q_gate.p + static_cast<size_t>(row0) * hq * 512,
-                              L.k_cache, L.v_cache, ctx + d->b0, Bl, R, hq, hkv, d->max_seq, d->attn_splits, d->attn_scratch,
-                              1.0f / sqrtf(256.0f), 0, xperm_on()));
+        xb::AttnTiles at;
+        at.out = d->attn_out.p + static_cast<size_t>(row0) * hq * 256;
+        at.q = d->qbuf + static_cast<size_t>(row0) * hq * 256;
+        at.q_gate = d->q_gate.p + static_cast<size_t>(row0) * hq * 512;
+        at.k_cache = L.k_cache;
+        at.v_cache = L.v_cache;
+        at.ctx = ctx + d->b0;
+        at.batch = Bl;
+        at.rows_per_seq = R;
+        at.hq = hq;
+        at.hkv = hkv;
+        at.cache_rows = at.cache_stride = d->max_seq;
+        at.scale = 1.0f / sqrtf(256.0f);
+        at.perm_out = xperm_on();
+        at.early = 1;  // the context lengths and the keys below them were there before this layer's projections ran
+        at.scratch = d->attn_scratch;
+        NL(xb::attn_tiles(s, at, d->num_sms, d->status));
         d->launches_per_step += 3;
         CK(gather_rows(d, s, d->attn_out, row0, Ml, static_cast<int64_t>(hq) * 256));
         // x += mixer output, post-attention RMSNorm
@@ -659,11 +654,9 @@ int target_pass(Dec* d, cudaStream_t s, int R, const long long* tokens) {
 
 // ---------------------------------------------------------------------------------------------- prefill chunks
 // A prompt goes through the model in chunks of up to 512 rows (all sequences together), so that the projections see
-// M = hundreds of rows and run on the prefill GEMM.  Between them the attention kernels take the chunk four positions
-// at a time (their own row limit; the row order of a chunk, chunk_row, makes every such group a contiguous block, and
-// one launch takes all groups of all sequences as separate entries); the convolution
-// and the gated delta rule walk the whole chunk in one launch each (conv1d_chunk, gdn_chunk).  Natural feature
-// order everywhere (the permuted order of the decode step is a property of its 32-row kernel).
+// M = hundreds of rows and run on the prefill GEMM; attention, convolution and the gated delta rule take the whole chunk in
+// one launch each.  Natural feature order everywhere (the permuted order of the decode step is a property of its 32-row
+// kernel).
 
 int ensure_chunk_bufs(Dec* d, int rows) {
     auto& cb = d->chunk;
@@ -679,7 +672,7 @@ int ensure_chunk_bufs(Dec* d, int rows) {
     const size_t halves = (per_row + 64) * static_cast<size_t>(rows);
     if (cb.x) { cudaFree(cb.x); cudaFree(cb.attn_scratch); cudaFree(cb.gdn_scratch); cb = Dec::ChunkBufs(); }
     __half* base = nullptr;
-    if (cudaMalloc(&base, halves * sizeof(__half) + static_cast<size_t>(rows) * (sizeof(long long) + sizeof(int)) + 256) != cudaSuccess) {
+    if (cudaMalloc(&base, halves * sizeof(__half) + static_cast<size_t>(rows) * sizeof(long long) + 256) != cudaSuccess) {
         cudaGetLastError();
         return XINFER_ERR_OUT_OF_MEMORY;
     }
@@ -693,23 +686,14 @@ int ensure_chunk_bufs(Dec* d, int rows) {
     cb.qbuf = take(hq * 256); cb.kbuf = take(hkv * 256); cb.vbuf = take(hkv * 256); cb.mix_out = take(mix);
     cb.zbuf = take(hv * 128); cb.bbuf = take(hv); cb.abuf = take(hv); cb.cat = take(2 * H); cb.hprev = take(H);
     cb.tokens = reinterpret_cast<long long*>(base + ((off + 63) & ~static_cast<size_t>(63)));
-    cb.entry_ctx = reinterpret_cast<int*>(cb.tokens + rows);
-    // one attention launch takes every full group of four positions of every sequence as an entry of its own: enough
-    // entries fill the GPU without splitting the keys, few entries are split as in the step
-    const int entries = (rows + 3) / 4;
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device);
-    int ns = (2 * sms + entries * static_cast<int>(hkv) - 1) / (entries * static_cast<int>(hkv));
-    ns = ns < 1 ? 1 : (ns > d->attn_splits ? d->attn_splits : ns);
-    cb.attn_splits = ns;
-    if (cudaMalloc(&cb.attn_scratch, xb::attn_scratch_bytes(entries, static_cast<int>(hkv), ns)) != cudaSuccess) {
+    const int positions = (rows + d->batch - 1) / d->batch;  // of every sequence
+    if (cudaMalloc(&cb.attn_scratch, xb::attn_tile_scratch_bytes(d->batch, positions, static_cast<int>(hq), static_cast<int>(hkv), d->num_sms)) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(base);
         cb = Dec::ChunkBufs();
         return XINFER_ERR_OUT_OF_MEMORY;
     }
-    // (`rows` is a whole number of positions for every sequence, and no chunk holds more than that)
-    if (cudaMalloc(&cb.gdn_scratch, xb::gdn_chunk_scratch_bytes(d->batch, (rows + d->batch - 1) / d->batch, static_cast<int>(hv))) != cudaSuccess) {
+    if (cudaMalloc(&cb.gdn_scratch, xb::gdn_chunk_scratch_bytes(d->batch, positions, static_cast<int>(hv))) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(base);
         cudaFree(cb.attn_scratch);
@@ -734,7 +718,7 @@ int prefill_chunk(Dec* d, cudaStream_t s, const long long* prompt, int64_t T, in
     const int B = d->batch, M = B * Rc, H = static_cast<int>(c.hidden_size), F = static_cast<int>(c.intermediate_size);
     const int hq = static_cast<int>(c.num_attention_heads), hkv = static_cast<int>(c.num_key_value_heads);
     const int hv = static_cast<int>(c.linear_num_v_heads), hk = static_cast<int>(c.linear_num_k_heads);
-    const int ch = 2 * hk * 128 + hv * 128, groups = (Rc + 3) / 4;
+    const int ch = 2 * hk * 128 + hv * 128;
     const float eps = c.rms_norm_eps;
     void* st = s;
     auto desc = [](void* y, const Linear& l) {
@@ -742,11 +726,7 @@ int prefill_chunk(Dec* d, cudaStream_t s, const long long* prompt, int64_t T, in
         f.Y = y; f.W_int4 = l.w; f.scales = l.s; f.bias = nullptr; f.N = l.n;
         return f;
     };
-    const int full_groups = Rc / 4;
     gather_prompt_chunk_kernel<<<blocks_for(static_cast<size_t>(M), 128), 128, 0, s>>>(cb.tokens, prompt, B, T, c0, Rc);
-    if (full_groups > 0)
-        chunk_entry_ctx_kernel<<<blocks_for(static_cast<size_t>(full_groups) * B, 128), 128, 0, s>>>(cb.entry_ctx, full_groups * B, B,
-                                                                                                 static_cast<int>(c0));
     NL(xb::embed_rows(s, cb.x, d->embed, cb.tokens, M, H, c.vocab_size));
     NL(xb::rmsnorm_rows(s, cb.normed, H, cb.x, d->layers[0].input_norm, M, H, eps, 0));
     const size_t nl = d->layers.size();
@@ -755,26 +735,24 @@ int prefill_chunk(Dec* d, cudaStream_t s, const long long* prompt, int64_t T, in
         if (L.full) {
             const xinfer_fused_desc fd[3] = {desc(cb.wide, L.q_proj), desc(cb.kbuf, L.k_proj), desc(cb.vbuf, L.v_proj)};
             LIN(xinfer_linear_int4_fused_f16(st, cb.normed, fd, 3, M, H, 128));
-            // every full group of four positions of every sequence is one entry (rows [entry][4], its own context length,
-            // the cache of sequence entry % B): one launch each for the prologue, the split attention and the combine;
-            // a last short group goes through the same kernels on its own
-            if (full_groups > 0) {
-                NL(xb::attn_prep_ex(s, cb.qbuf, L.k_cache, L.v_cache, cb.wide, cb.kbuf, cb.vbuf, L.q_norm, L.k_norm, cb.entry_ctx,
-                                    full_groups * B, 4, hq, hkv, d->max_seq, eps, c.rope_theta, c.rope_dim, 512, nullptr, 0, nullptr, B));
-                NL(xb::attn_decode_ex(s, cb.mix_out, cb.qbuf, cb.wide, L.k_cache, L.v_cache, cb.entry_ctx, full_groups * B, 4, hq, hkv,
-                                      d->max_seq, cb.attn_splits, cb.attn_scratch, 1.0f / sqrtf(256.0f), 0, 0, B));
-            }
-            if (full_groups < groups) {
-                const int rj = Rc - 4 * full_groups;
-                const size_t r0 = static_cast<size_t>(full_groups) * B * 4;
-                const int pos0 = static_cast<int>(c0) + 4 * full_groups;
-                NL(xb::attn_prep_ex(s, cb.qbuf + r0 * hq * 256, L.k_cache, L.v_cache, cb.wide + r0 * hq * 512, cb.kbuf + r0 * hkv * 256,
-                                    cb.vbuf + r0 * hkv * 256, L.q_norm, L.k_norm, nullptr, B, rj, hq, hkv, d->max_seq, eps,
-                                    c.rope_theta, c.rope_dim, 512, nullptr, pos0, nullptr));
-                NL(xb::attn_decode_ex(s, cb.mix_out + r0 * hq * 256, cb.qbuf + r0 * hq * 256, cb.wide + r0 * hq * 512, L.k_cache,
-                                      L.v_cache, nullptr, B, rj, hq, hkv, d->max_seq, d->attn_splits, d->attn_scratch,
-                                      1.0f / sqrtf(256.0f), pos0, 0));
-            }
+            NL(xb::attn_prep_ex(s, cb.qbuf, L.k_cache, L.v_cache, cb.wide, cb.kbuf, cb.vbuf, L.q_norm, L.k_norm, nullptr, B, Rc, hq, hkv,
+                                d->max_seq, eps, c.rope_theta, c.rope_dim, 512, nullptr, static_cast<int>(c0), nullptr));
+            xb::AttnTiles at;
+            at.out = cb.mix_out;
+            at.q = cb.qbuf;
+            at.q_gate = cb.wide;
+            at.k_cache = L.k_cache;
+            at.v_cache = L.v_cache;
+            at.ctx_base = static_cast<int>(c0);
+            at.batch = B;
+            at.rows_per_seq = Rc;
+            at.hq = hq;
+            at.hkv = hkv;
+            at.cache_rows = c0 + Rc;
+            at.cache_stride = d->max_seq;
+            at.scale = 1.0f / sqrtf(256.0f);
+            at.scratch = cb.attn_scratch;
+            NL(xb::attn_tiles(s, at, d->num_sms, d->status));
             LIN(xinfer_linear_int4_f16f16(st, cb.proj_out, cb.mix_out, L.o_proj.w, L.o_proj.s, nullptr, M, L.o_proj.n, L.o_proj.k, 128));
         } else {
             const xinfer_fused_desc fd[4] = {desc(cb.wide, L.in_qkv), desc(cb.zbuf, L.in_z), desc(cb.bbuf, L.in_b), desc(cb.abuf, L.in_a)};
@@ -802,15 +780,8 @@ int prefill_chunk(Dec* d, cudaStream_t s, const long long* prompt, int64_t T, in
     NL(xb::rmsnorm_rows(s, cb.normed, H, cb.mix_out, ML.input_norm, M, H, eps, 0));
     const xinfer_fused_desc kv[2] = {desc(cb.kbuf, ML.k_proj), desc(cb.vbuf, ML.v_proj)};
     LIN(xinfer_linear_int4_fused_f16(st, cb.normed, kv, 2, M, H, 128));
-    if (full_groups > 0)
-        NL(xb::attn_prep_ex(s, cb.qbuf, ML.k_cache, ML.v_cache, cb.wide, cb.kbuf, cb.vbuf, ML.q_norm, ML.k_norm, cb.entry_ctx,
-                            full_groups * B, 4, 0, hkv, d->max_seq, eps, c.rope_theta, c.rope_dim, 512, nullptr, 0, nullptr, B));
-    if (full_groups < groups) {
-        const size_t r0 = static_cast<size_t>(full_groups) * B * 4;
-        NL(xb::attn_prep_ex(s, cb.qbuf, ML.k_cache, ML.v_cache, cb.wide, cb.kbuf + r0 * hkv * 256, cb.vbuf + r0 * hkv * 256, ML.q_norm,
-                            ML.k_norm, nullptr, B, Rc - 4 * full_groups, 0, hkv, d->max_seq, eps, c.rope_theta, c.rope_dim, 512,
-                            nullptr, static_cast<int>(c0) + 4 * full_groups, nullptr));
-    }
+    NL(xb::attn_prep_ex(s, cb.qbuf, ML.k_cache, ML.v_cache, cb.wide, cb.kbuf, cb.vbuf, ML.q_norm, ML.k_norm, nullptr, B, Rc, 0, hkv,
+                        d->max_seq, eps, c.rope_theta, c.rope_dim, 512, nullptr, static_cast<int>(c0), nullptr));
     take_last_hidden_chunk_kernel<<<blocks_for(static_cast<size_t>(B) * H, 256), 256, 0, s>>>(d->h_last, cb.x, B, Rc, H);
     CKCUDA(cudaGetLastError());
     return 0;
@@ -925,6 +896,10 @@ int xinfer_spec_decoder_create_tp(const xinfer_model_config* cfg, int batch, int
     d->bl = batch / world;
     d->b0 = rank * d->bl;
     cudaGetDevice(&d->device);
+    if (xb::device_facts(&d->status, &d->num_sms) != XINFER_OK) {
+        delete d;
+        return XINFER_ERR_NO_DEVICE;
+    }
     d->plan = xb::tc_plan_new();
     try {
         if (!d->plan) throw std::bad_alloc();
@@ -1148,8 +1123,8 @@ int xinfer_spec_decoder_set_top_p(xinfer_spec_decoder* d, float top_p) {
 
 // Builds the context from a prompt: tokens [batch][T] (host), all sequences the same length, starting from the empty
 // context of reset(0, seed).  Positions 0 .. T-2 go through the target model in chunks of up to 512 rows over all
-// sequences (prefill_chunk: projections on the prefill GEMM, mixers four positions at a time with every row kept,
-// so KV caches, Gated-DeltaNet and convolution state advance as in steps whose drafts were all accepted), the MTP
+// sequences (prefill_chunk: every row kept, so KV caches, Gated-DeltaNet and convolution state advance as in steps whose
+// drafts were all accepted), the MTP
 // head's KV slots of the same positions are written from (token, hidden state in front of it; zeros in front of
 // position 0), and the last prompt token becomes the current token.  Afterwards ctx = T - 1 and
 // xinfer_spec_decoder_step continues from there.  Stands where the reference's chunked prefill does

@@ -44,6 +44,8 @@ bool gemm_eligible(const void* x, const TcProj* proj, int num, bool swiglu, long
 size_t gemm_partial_bytes(int num_sms);
 int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num, bool swiglu, bool out_f32, long long m,
                 long long k, int* status, long long wait_limit, int x_stage_limit, int num_sms, float* partials, int* counters);
+// The current device's status word (what xinfer_device_status reads) and number of SMs; a XINFER_* code.
+int device_facts(int** status, int* num_sms);
 // Records a message for xinfer_last_cuda_error() on the calling thread (c_api.cu).
 void set_last_error(const char* msg);
 // Programmatic dependent launch (on unless XINFER_PDL=0): kernels are launched with the stream-serialization
