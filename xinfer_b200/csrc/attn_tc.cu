@@ -11,15 +11,20 @@
 //                 rarely rescaled), fp32 sums, fp16 probabilities back into tensor memory;
 //   O += P V      M = 128, N = 256 dims, K = 64 keys, A from tensor memory, V as it lies in the cache (its 256 dims are
 //                 contiguous: an MN-major operand), O in 256 tensor-memory columns.
-// K and V blocks arrive by TMA two blocks ahead (2 x 64 KB beside 64 KB of queries).
+// K and V blocks of 32 KB arrive by TMA, a warp each: three slots of keys and two of values beside 64 KB of queries, three and
+// three where the queries are at most 32 rows and take 16 KB.
 //
-// Tiles x 64-key blocks are cut evenly over one CTA per SM on the device, from the context lengths that lie there: a CTA
-// takes a contiguous range of (tile, block) units.  What covers a whole tile is written out, the two ends of a range as fp32
-// partials for attn_tile_combine_kernel.
+// (sequence, tile) x 64-key blocks are cut evenly over groups of Hkv CTAs, one per KV head and together one per SM, on the
+// device, from the context lengths that lie there: a CTA takes a contiguous range of (tile, block) units.  What covers a whole
+// tile is written out, the two ends of a range as fp32 partials for attn_tile_combine_kernel.  The CTAs of a group walk the
+// same keys in step: in the cache the heads of a key lie
+// side by side.
 //
 // Bounds.  Prefill: per block the tensor core needs 128 * 64 * 256 * 4 flop = 1024 clocks at its full rate, the exponentials
-// 512.  Decode (24 of the 128 rows in use): 64 KB of cache per block are 2900 clocks of an SM's share of HBM, so the padded
-// rows cost nothing.
+// 512; measured 2500 (8192 keys, 512 rows: 130 us, 770 TFLOP/s; 4.9 ms five rows a launch), the S product at N = 64 being
+// bound by its shared-memory reads.  Decode (24 of the 128 rows in use): 64 KB of cache per block are 2900 clocks of an SM's
+// share of HBM, so the padded rows cost nothing; 269 MB of cache take 56 us in the step, 47 of them at the 5.8 TB/s that a
+// longer context settles at.  (Pulling the blocks into L2 ahead in 32 KB runs of all heads made it slower, 60 to 70 us.)
 //
 // Every wait is bounded (WaitState); one that runs out sets the device status word and the CTA leaves through its normal exit.
 #include <cuda.h>
@@ -40,26 +45,33 @@ namespace xb {
 namespace {
 
 constexpr int kTileRows = 128, kTileKeys = 64, kDim = 256, kDimBlocks = kDim / 64;
-constexpr int kSoftmaxThreads = 128, kTileThreads = kSoftmaxThreads + 64;
-constexpr int kTmaWarp = 4, kMmaWarp = 5;
-constexpr int kKvSlots = 2;
-constexpr int kQBytes = kTileRows * kDim * 2, kKvBytes = kTileKeys * kDim * 2;
+constexpr int kSoftmaxThreads = 128, kTileThreads = kSoftmaxThreads + 96;
+constexpr int kKWarp = 4, kVWarp = 5, kMmaWarp = 6;  // two TMA warps: keys (and queries), values
+constexpr int kKvBytes = kTileKeys * kDim * 2;
+constexpr int kKSlots = 3;
+constexpr int tile_v_slots(int rows) { return rows <= 32 ? 3 : 2; }
+// Bytes of a 64-dim block of the queries.  At 32 rows the MMA, which always takes 128, reads on into what lies behind: rows of
+// S that nobody looks at.
+constexpr int tile_q_block(int rows) { return (rows <= 32 ? 32 : kTileRows) * 128; }
 // tensor memory columns
 constexpr uint32_t kColO = 0, kColS = 256, kColP = 384, kTileTmemCols = 512;
 constexpr float kLazyRescale = 8.0f;  // in base-2 units: probabilities stay below 2^8
 
 struct TileCtrl {
-    uint64_t q_full, q_empty, o_free, k_full[kKvSlots], k_empty[kKvSlots], v_full[kKvSlots], v_empty[kKvSlots];
+    uint64_t q_full, q_empty, o_free, k_full[kKSlots], k_empty[kKSlots], v_full[3], v_empty[3];
     uint64_t s_full[2], s_free[2], p_ready[2], pv_done[2];
     uint32_t tmem_base;
     WaitState ws;
 };
-constexpr size_t kTileSmemBytes = 1024 + kQBytes + 2 * kKvSlots * kKvBytes + sizeof(TileCtrl);
+constexpr size_t tile_smem_bytes(int rows) {
+    return 1024 + kDimBlocks * tile_q_block(rows) + (kKSlots + tile_v_slots(rows)) * kKvBytes + sizeof(TileCtrl);
+}
+static_assert(tile_smem_bytes(32) <= 227 * 1024 && tile_smem_bytes(kTileRows) <= 227 * 1024, "shared memory");
 
 struct TileShape {          // what both kernels need to find their work
     const int* ctx;         // keys in front of each sequence's first row; null: ctx_base
     int ctx_base;
-    int rows_per_seq, hq, hkv, group, tile_pos, tiles, items;  // items = batch * hkv * tiles, tiles fastest
+    int rows_per_seq, hq, hkv, group, tile_pos, tiles, items;  // items = batch * tiles, tiles fastest
     long long max_seq;
 };
 struct TileParams {
@@ -71,7 +83,7 @@ struct TileParams {
     int early;              // keys below ctx, and ctx itself, do not come from the launch in front of this one
     float scale2;           // softmax scale * log2 e
     float *part_o, *part_ml;  // [CTA][2][row][256], [CTA][2][row][max, sum]
-    int* table;             // [items] first unit of every item, then the number of units and of CTAs at work
+    int2* table;            // [items] first and last group at work on every item
     long long wait_limit;
     int* status;
 };
@@ -157,25 +169,25 @@ __device__ __forceinline__ void store8(__half* dst, const uint4& v, int vec) {
 }
 
 // Keys in front of item e's first row, and its number of 64-key blocks (at least one).
-__device__ __forceinline__ int item_ctx(const TileShape& sh, int e) { return sh.ctx ? __ldg(sh.ctx + e / (sh.hkv * sh.tiles)) : sh.ctx_base; }
+__device__ __forceinline__ int item_ctx(const TileShape& sh, int e) { return sh.ctx ? __ldg(sh.ctx + e / sh.tiles) : sh.ctx_base; }
 __device__ __forceinline__ int item_blocks(const TileShape& sh, int e) {
     const int end = (e % sh.tiles + 1) * sh.tile_pos;
     long long keys = static_cast<long long>(item_ctx(sh, e)) + (end < sh.rows_per_seq ? end : sh.rows_per_seq);
     if (keys > sh.max_seq) keys = sh.max_seq;
     return static_cast<int>((keys + kTileKeys - 1) / kTileKeys);
 }
-__device__ __forceinline__ int range_begin(int cta, int total, int ctas) { return static_cast<int>(static_cast<long long>(cta) * total / ctas); }
-// The CTA whose range holds unit u: the largest c with floor(c total / ctas) <= u.
-__device__ __forceinline__ int unit_owner(int u, int total, int ctas) {
-    return static_cast<int>((static_cast<long long>(u + 1) * ctas - 1) / total);
+__device__ __forceinline__ int range_begin(int group, int total, int groups) { return static_cast<int>(static_cast<long long>(group) * total / groups); }
+// The group whose range holds unit u: the largest c with floor(c total / groups) <= u.
+__device__ __forceinline__ int unit_owner(int u, int total, int groups) {
+    return static_cast<int>((static_cast<long long>(u + 1) * groups - 1) / total);
 }
 
-// A CTA's walk through its units, a run of blocks of one item at a time.
+// A group's walk through its units, a run of blocks of one item at a time.
 struct TileWalk {
-    int item, off, u, u_end, total, ctas;  // next item, next block of it, next unit
+    int item, off, u, u_end, total, groups;  // next item, next block of it, next unit
     int kb0, n, blocks;                    // the current run
     // Every lane of a warp calls it.
-    __device__ void start(const TileShape& sh, int cta, int grid) {
+    __device__ void start(const TileShape& sh, int group, int most_groups) {
         const int lane = threadIdx.x & 31;
         total = 0;
         for (int e0 = 0; e0 < sh.items; e0 += 32) {
@@ -183,10 +195,10 @@ struct TileWalk {
             total += __reduce_add_sync(0xffffffffu, mine);
         }
         // Below two blocks a CTA, the partials cost more than the additional CTAs bring.
-        ctas = total / 2 < 1 ? 1 : (total / 2 < grid ? total / 2 : grid);
+        groups = total / 2 < 1 ? 1 : (total / 2 < most_groups ? total / 2 : most_groups);
         item = off = 0;
-        u = cta < ctas ? range_begin(cta, total, ctas) : total;
-        u_end = cta < ctas ? range_begin(cta + 1, total, ctas) : total;
+        u = group < groups ? range_begin(group, total, groups) : total;
+        u_end = group < groups ? range_begin(group + 1, total, groups) : total;
         int before = 0;
         for (int e0 = 0; e0 < sh.items && u < u_end; e0 += 32) {
             const int mine = e0 + lane < sh.items ? item_blocks(sh, e0 + lane) : 0;
@@ -225,14 +237,14 @@ struct TileWalk {
 __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid_constant__ TileParams p) {
     extern __shared__ uint8_t tile_smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tile_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    uint8_t* q_smem = smem;                          // [dim block][128 rows][128 B]
-    uint8_t* k_smem = q_smem + kQBytes;              // [slot][dim block][64 keys][128 B]
-    uint8_t* v_smem = k_smem + kKvSlots * kKvBytes;
-    TileCtrl* ctrl = reinterpret_cast<TileCtrl*>(v_smem + kKvSlots * kKvBytes);
+    const TileShape& sh = p.sh;
+    const int rows = sh.group * sh.tile_pos, live_warps = (rows + 31) / 32, v_slots = tile_v_slots(rows), q_block = tile_q_block(rows);
+    uint8_t* q_smem = smem;                          // [dim block][rows][128 B]
+    uint8_t* k_smem = q_smem + kDimBlocks * q_block; // [slot][dim block][64 keys][128 B]
+    uint8_t* v_smem = k_smem + kKSlots * kKvBytes;
+    TileCtrl* ctrl = reinterpret_cast<TileCtrl*>(v_smem + v_slots * kKvBytes);
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const TileShape& sh = p.sh;
-    const int rows = sh.group * sh.tile_pos, live_warps = (rows + 31) / 32;
     volatile WaitState* ws = &ctrl->ws;
     griddep_launch_dependents();
 
@@ -240,11 +252,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
         mbar_init(smem_u32(&ctrl->q_full), 1);
         mbar_init(smem_u32(&ctrl->q_empty), 1);
         mbar_init(smem_u32(&ctrl->o_free), live_warps);
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 3; ++i) {
             mbar_init(smem_u32(&ctrl->k_full[i]), 1);
             mbar_init(smem_u32(&ctrl->k_empty[i]), 1);
             mbar_init(smem_u32(&ctrl->v_full[i]), 1);
             mbar_init(smem_u32(&ctrl->v_empty[i]), 1);
+        }
+        for (int i = 0; i < 2; ++i) {
             mbar_init(smem_u32(&ctrl->s_full[i]), 1);
             mbar_init(smem_u32(&ctrl->s_free[i]), live_warps);
             mbar_init(smem_u32(&ctrl->p_ready[i]), live_warps);
@@ -265,71 +279,66 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
     const uint32_t tmem = ctrl->tmem_base;
     if (!p.early) griddep_wait();
     TileWalk walk;
-    walk.start(sh, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
+    const int kvh = static_cast<int>(blockIdx.x) % sh.hkv;
+    walk.start(sh, static_cast<int>(blockIdx.x) / sh.hkv, static_cast<int>(gridDim.x) / sh.hkv);
     const int units = walk.u_end - walk.u;
 
-    if (warp == kTmaWarp) {
-        // ------------------------------------------------------------------ TMA producer (whole warp waits, one lane issues)
+    if (warp == kKWarp || warp == kVWarp) {
+        // ------------------------------------------------------------------ TMA producers (whole warp waits, one lane issues)
+        const bool keys = warp == kKWarp;
         const bool leader = elect_one_sync();
+        const CUtensorMap* map = keys ? &p.k_map : &p.v_map;
         if (leader) {
-            tma_prefetch_desc(&p.q_map);
-            tma_prefetch_desc(&p.k_map);
-            tma_prefetch_desc(&p.v_map);
+            tma_prefetch_desc(map);
+            if (keys) tma_prefetch_desc(&p.q_map);
         }
-        const uint64_t pol_q = l2_policy_evict_first(), pol_kv = l2_policy_evict_last();
-        auto load_kv = [&](const CUtensorMap* map, uint64_t* full, uint8_t* ring, int i, int block, int item) {
+        // keys and values are read once by a decode pass, by every tile of a prompt
+        const uint64_t pol_q = l2_policy_evict_first(), pol_kv = sh.tiles == 1 ? l2_policy_evict_first() : l2_policy_evict_last();
+        uint64_t *full = keys ? ctrl->k_full : ctrl->v_full, *empty = keys ? ctrl->k_empty : ctrl->v_empty;
+        const uint32_t ring = smem_u32(keys ? k_smem : v_smem);
+        const int slots = keys ? kKSlots : v_slots;
+        auto load = [&](int slot, int block, int item) {
             if (leader) {
-                const int slot = i % kKvSlots, b = item / (sh.hkv * sh.tiles), kvh = item / sh.tiles % sh.hkv;
+                const int b = item / sh.tiles;
                 const uint32_t bar = smem_u32(&full[slot]);
                 mbar_arrive_expect_tx(bar, kKvBytes);
                 for (int d = 0; d < kDimBlocks; ++d)
-                    tma_load_3d(smem_u32(ring) + slot * kKvBytes + d * (kTileKeys * 128), map, bar, kvh * kDim + d * 64, block * kTileKeys, b, pol_kv);
+                    tma_load_3d(ring + slot * kKvBytes + d * (kTileKeys * 128), map, bar, kvh * kDim + d * 64, block * kTileKeys, b, pol_kv);
             }
         };
-        int i = 0, ahead = 0, nk = 0, nv = 0, nq = 0;
+        int i = 0, ahead = 0, nq = 0, slot = 0;
+        uint32_t parity = 1;  // under which a slot's first use passes at once
         bool ok = true;
         if (p.early) {
             // the first blocks while the launch in front of this one, which writes the newest keys and the queries, finishes
             if (walk.next(sh)) {
                 const int old_blocks = item_ctx(sh, walk.item) / kTileKeys;
-                for (; ahead < kKvSlots && ahead < walk.n && walk.kb0 + ahead < old_blocks; ++ahead) {
-                    load_kv(&p.k_map, ctrl->k_full, k_smem, ahead, walk.kb0 + ahead, walk.item);
-                    load_kv(&p.v_map, ctrl->v_full, v_smem, ahead, walk.kb0 + ahead, walk.item);
-                }
+                for (; ahead < slots && ahead < walk.n && walk.kb0 + ahead < old_blocks; ++ahead) load(ahead, walk.kb0 + ahead, walk.item);
             }
             griddep_wait();
         }
-        if (leader) ws->dep_ready = 1;
+        if (leader && keys) ws->dep_ready = 1;
         __syncwarp();
-        nk = nv = ahead;
         for (int run = 0; ok && walk.next(sh); ++run) {
-            for (int j = 0; j < walk.n && ok; ++j, ++i) {
-                const int slot = i % kKvSlots;
-                const uint32_t parity = ((i / kKvSlots) & 1u) ^ 1u;
+            for (int j = 0; j < walk.n && ok; ++j) {
                 if (i >= ahead) {
-                    ok = warp_wait_parked(&ctrl->k_empty[slot], parity, ws);
+                    ok = warp_wait_parked(&empty[slot], parity, ws);
                     if (!ok) break;
-                    load_kv(&p.k_map, ctrl->k_full, k_smem, i, walk.kb0 + j, walk.item);
-                    ++nk;
+                    load(slot, walk.kb0 + j, walk.item);
                 }
-                if (j == 0) {
+                ++i;
+                if (++slot == slots) { slot = 0; parity ^= 1u; }
+                if (j == 0 && keys) {
                     ok = run == 0 || warp_wait_parked(&ctrl->q_empty, (run & 1u) ^ 1u, ws);
                     if (!ok) break;
                     if (leader) {
-                        const int b = walk.item / (sh.hkv * sh.tiles), kvh = walk.item / sh.tiles % sh.hkv;
+                        const int b = walk.item / sh.tiles;
                         const uint32_t bar = smem_u32(&ctrl->q_full);
                         mbar_arrive_expect_tx(bar, static_cast<uint32_t>(rows) * kDim * 2);
                         for (int d = 0; d < kDimBlocks; ++d)
-                            tma_load_4d(smem_u32(q_smem) + d * (kTileRows * 128), &p.q_map, bar, d * 64, kvh * sh.group,
-                                        walk.item % sh.tiles * sh.tile_pos, b, pol_q);
+                            tma_load_4d(smem_u32(q_smem) + d * q_block, &p.q_map, bar, d * 64, kvh * sh.group, walk.item % sh.tiles * sh.tile_pos, b, pol_q);
                     }
                     ++nq;
-                }
-                if (i >= ahead) {
-                    ok = warp_wait_parked(&ctrl->v_empty[slot], parity, ws);
-                    if (!ok) break;
-                    load_kv(&p.v_map, ctrl->v_full, v_smem, i, walk.kb0 + j, walk.item);
-                    ++nv;
                 }
             }
             walk.advance();
@@ -337,17 +346,14 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
         if (ws->abort_flag) {
             // give the copies still in flight a bounded chance to land before the CTA exits
             const long long t0 = clock64();
-            auto landed = [&](uint64_t* bars, int count) {
-                for (int s = 0; s < kKvSlots && s < count; ++s) {
-                    const int k = count - 1 - s;
-                    while (!mbar_try_wait(smem_u32(&bars[k % kKvSlots]), (k / kKvSlots) & 1u) && clock64() - t0 < p.wait_limit / 8) {
-                    }
+            const int loaded = i > ahead ? i : ahead;
+            for (int c = 0; c < slots && c < loaded; ++c) {
+                const int k = loaded - 1 - c;
+                while (!mbar_try_wait(smem_u32(&full[k % slots]), (k / slots) & 1u) && clock64() - t0 < p.wait_limit / 8) {
                 }
-            };
+            }
             while (nq > 0 && !mbar_try_wait(smem_u32(&ctrl->q_full), (nq - 1) & 1u) && clock64() - t0 < p.wait_limit / 8) {
             }
-            landed(ctrl->k_full, nk);
-            landed(ctrl->v_full, nv);
         }
         __syncwarp();
     } else if (warp == kMmaWarp) {
@@ -361,15 +367,17 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
         constexpr uint32_t lo_k = 1u << 16, lo_v = static_cast<uint32_t>((kTileKeys * 128) >> 4) << 16;
         const uint32_t q_lo = (smem_u32(q_smem) >> 4) & 0x3FFFu, k_lo = (smem_u32(k_smem) >> 4) & 0x3FFFu, v_lo = (smem_u32(v_smem) >> 4) & 0x3FFFu;
         auto desc = [&](uint32_t lo) { return (static_cast<uint64_t>(desc_hi) << 32) | lo; };
+        uint32_t k_slot = 0, k_phase = 0, v_slot = 0, v_phase = 0;
         auto issue_s = [&](int i, bool last_of_run) {
-            const uint32_t buf = static_cast<uint32_t>(i & 1), slot = static_cast<uint32_t>(i % kKvSlots);
-            if (!warp_wait_parked(&ctrl->k_full[slot], (i / kKvSlots) & 1u, ws)) return false;
+            const uint32_t buf = static_cast<uint32_t>(i & 1), slot = k_slot;
+            if (!warp_wait_parked(&ctrl->k_full[slot], k_phase, ws)) return false;
+            if (++k_slot == kKSlots) { k_slot = 0; k_phase ^= 1u; }
             if (i >= 2 && !warp_wait_parked(&ctrl->s_free[buf], ((i >> 1) & 1u) ^ 1u, ws)) return false;
             tc_fence_after_sync();
             if (leader) {
 #pragma unroll
                 for (int k = 0; k < kDim / 16; ++k) {
-                    const uint32_t a = q_lo + (((k >> 2) * (kTileRows * 128) + (k & 3) * 32) >> 4);
+                    const uint32_t a = q_lo + (((k >> 2) * q_block + (k & 3) * 32) >> 4);
                     const uint32_t c = k_lo + ((slot * kKvBytes + (k >> 2) * (kTileKeys * 128) + (k & 3) * 32) >> 4);
                     umma_ss_f16(tmem + kColS + buf * kTileKeys, desc(lo_k | a), desc(lo_k | c), idesc_s, k > 0 ? 1u : 0u);
                 }
@@ -382,8 +390,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
         };
         // `run` >= 0: the block is the first of that run and overwrites O, which the run before must have been read from
         auto issue_o = [&](int i, int run) {
-            const uint32_t buf = static_cast<uint32_t>(i & 1), slot = static_cast<uint32_t>(i % kKvSlots);
-            if (!warp_wait_parked(&ctrl->v_full[slot], (i / kKvSlots) & 1u, ws)) return false;
+            const uint32_t buf = static_cast<uint32_t>(i & 1), slot = v_slot;
+            if (!warp_wait_parked(&ctrl->v_full[slot], v_phase, ws)) return false;
+            if (++v_slot == static_cast<uint32_t>(v_slots)) { v_slot = 0; v_phase ^= 1u; }
             if (!warp_wait_parked(&ctrl->p_ready[buf], (i >> 1) & 1u, ws)) return false;
             if (run > 0 && !warp_wait_parked(&ctrl->o_free, (run & 1u) ^ 1u, ws)) return false;
             tc_fence_after_sync();
@@ -419,7 +428,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
         bool ok = true;
         int i = 0;
         while (ok && walk.next(sh)) {
-            const int item = walk.item, b = item / (sh.hkv * sh.tiles), kvh = item / sh.tiles % sh.hkv, pos = item % sh.tiles * sh.tile_pos + pr;
+            const int item = walk.item, b = item / sh.tiles, pos = item % sh.tiles * sh.tile_pos + pr;
             const bool valid = r < rows && pos < sh.rows_per_seq;
             long long lim = static_cast<long long>(item_ctx(sh, item)) + pos + 1;
             if (lim > sh.max_seq) lim = sh.max_seq;
@@ -520,15 +529,12 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
                 __syncwarp();
             }
             if (!whole && valid) *reinterpret_cast<float2*>(p.part_ml + slot * 2) = make_float2(m, l);
-            if (tid == 0 && walk.kb0 == 0) p.table[item] = walk.u;
+            if (tid == 0 && kvh == 0 && walk.kb0 == 0)
+                p.table[item] = make_int2(static_cast<int>(blockIdx.x) / sh.hkv, unit_owner(walk.u + walk.blocks - 1, walk.total, walk.groups));
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&ctrl->o_free));
             walk.advance();
-        }
-        if (blockIdx.x == 0 && tid == 0) {
-            p.table[sh.items] = walk.total;
-            p.table[sh.items + 1] = walk.ctas;
         }
     } else if (p.early) {
         griddep_wait();
@@ -545,36 +551,87 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
     }
 }
 
-// Merges the parts of the items that were cut.  Grid (items, row blocks of 8), a warp per row, eight dims per lane.
-__global__ void __launch_bounds__(256) attn_tile_combine_kernel(__half* out, const float* part_o, const float* part_ml, const int* table,
-                                                                const __half* q_gate, const TileShape sh, int perm_out, int out_vec) {
+// Merges the parts of the items that were cut.  A warp takes every kWarpsPerRow-th part of a row, eight dims per lane; grid
+// (items * Hkv, row blocks).  A row of few long sequences has up to one part per group (37 at one sequence): eight warps, a row
+// a block (8192 keys, one row: 4 us, 8 with a warp a row).  Otherwise there are a few parts and many rows: a warp each.
+template <int kWarpsPerRow>
+__global__ void __launch_bounds__(256, 4) attn_tile_combine_kernel(__half* out, const float* part_o, const float* part_ml, const int2* table,
+                                                                   const __half* q_gate, const TileShape sh, int perm_out, int out_vec) {
     griddep_prologue();
-    const int item = blockIdx.x, rows = sh.group * sh.tile_pos, r = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const int total = table[sh.items], ctas = table[sh.items + 1], u = table[item];
-    const int u_end = item + 1 < sh.items ? table[item + 1] : total;
-    const int c0 = unit_owner(u, total, ctas), c1 = unit_owner(u_end - 1, total, ctas);
-    const int b = item / (sh.hkv * sh.tiles), kvh = item / sh.tiles % sh.hkv, pos = item % sh.tiles * sh.tile_pos + r / sh.group;
-    if (c0 == c1 || r >= rows || pos >= sh.rows_per_seq) return;
-    auto slot = [&](int c) { return (static_cast<size_t>(c) * 2 + (c == c0 ? 1 : 0)) * rows + r; };
+    constexpr int kBatch = 4;  // parts whose loads are in flight together
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = warp % kWarpsPerRow;
+    const int item = blockIdx.x / sh.hkv, kvh = blockIdx.x % sh.hkv, rows = sh.group * sh.tile_pos;
+    const int r = blockIdx.y * (8 / kWarpsPerRow) + warp / kWarpsPerRow;
+    const int2 who = table[item];
+    const int b = item / sh.tiles, pos = item % sh.tiles * sh.tile_pos + r / sh.group;
+    const long long at = (static_cast<long long>(b) * sh.rows_per_seq + pos) * sh.hq + kvh * sh.group + r % sh.group;
+    const bool gated = q_gate && r < rows && pos < sh.rows_per_seq && sub == 0;
+    uint4 gate = make_uint4(0, 0, 0, 0);  // (asked for here: its way from memory is the parts')
+    if (gated) gate = __ldg(reinterpret_cast<const uint4*>(q_gate + at * 512 + 256 + lane * 8));
+    const int c0 = who.x, c1 = who.y;
+    if (c0 == c1 || r >= rows || pos >= sh.rows_per_seq) return;  // (the same for all warps of a row)
+    auto slot = [&](int c) { return ((static_cast<size_t>(c) * sh.hkv + kvh) * 2 + (c == c0 ? 1 : 0)) * rows + r; };
     float m = -INFINITY, l = 0.f, acc[8] = {};
-    for (int c = c0 + lane; c <= c1; c += 32) m = fmaxf(m, __ldcg(part_ml + slot(c) * 2));
+    for (int c = c0 + sub; c <= c1; c += kBatch * kWarpsPerRow) {
+        float2 ml[kBatch];
+        float4 v[kBatch][2];
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-#pragma unroll 4
-    for (int c = c0; c <= c1; ++c) {
-        const float2 ml = __ldcg(reinterpret_cast<const float2*>(part_ml + slot(c) * 2));
-        const float w = ml.x == -INFINITY ? 0.f : exp2_ftz(ml.x - m);
-        l += ml.y * w;
-        const float4* src = reinterpret_cast<const float4*>(part_o + slot(c) * kDim + lane * 8);
-        const float4 a = __ldcg(src), d = __ldcg(src + 1);
-        acc[0] += a.x * w; acc[1] += a.y * w; acc[2] += a.z * w; acc[3] += a.w * w;
-        acc[4] += d.x * w; acc[5] += d.y * w; acc[6] += d.z * w; acc[7] += d.w * w;
+        for (int i = 0; i < kBatch; ++i) {
+            ml[i] = make_float2(-INFINITY, 0.f);
+            const int ci = c + i * kWarpsPerRow;
+            if (ci <= c1) {
+                ml[i] = __ldcg(reinterpret_cast<const float2*>(part_ml + slot(ci) * 2));
+                const float4* src = reinterpret_cast<const float4*>(part_o + slot(ci) * kDim + lane * 8);
+                v[i][0] = __ldcg(src);
+                v[i][1] = __ldcg(src + 1);
+            }
+        }
+        float top = m;
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) top = fmaxf(top, ml[i].x);
+        const float w0 = m == -INFINITY ? 0.f : exp2_ftz(m - top);
+        m = top;
+        l *= w0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] *= w0;
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+            if (ml[i].x == -INFINITY) continue;
+            const float w = exp2_ftz(ml[i].x - m);
+            l += ml[i].y * w;
+            acc[0] += v[i][0].x * w; acc[1] += v[i][0].y * w; acc[2] += v[i][0].z * w; acc[3] += v[i][0].w * w;
+            acc[4] += v[i][1].x * w; acc[5] += v[i][1].y * w; acc[6] += v[i][1].z * w; acc[7] += v[i][1].w * w;
+        }
+    }
+    if constexpr (kWarpsPerRow > 1) {
+        static_assert(kWarpsPerRow == 8, "a row is a block");
+        __shared__ float2 sh_ml[8];
+        __shared__ __align__(16) float sh_acc[8][kDim];
+        if (lane == 0) sh_ml[warp] = make_float2(m, l);
+        *reinterpret_cast<float4*>(&sh_acc[warp][lane * 8]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        *reinterpret_cast<float4*>(&sh_acc[warp][lane * 8 + 4]) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+        __syncthreads();
+        if (warp > 0) return;
+        float w[8];
+#pragma unroll
+        for (int i = 1; i < 8; ++i) m = fmaxf(m, sh_ml[i].x);
+        l = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            w[i] = sh_ml[i].x == -INFINITY ? 0.f : exp2_ftz(sh_ml[i].x - m);
+            l += sh_ml[i].y * w[i];
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            acc[j] = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[j] += sh_acc[i][lane * 8 + j] * w[i];
+        }
     }
     const float inv = 1.0f / (l > 0.f ? l : 1.0f);
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] *= inv;
-    const long long at = (static_cast<long long>(b) * sh.rows_per_seq + pos) * sh.hq + kvh * sh.group + r % sh.group;
-    store8(out + at * kDim + lane * 8, finish8(acc, q_gate ? q_gate + at * 512 + 256 + lane * 8 : nullptr, perm_out != 0), out_vec);
+    store8(out + at * kDim + lane * 8, finish8(acc, gated ? reinterpret_cast<const __half*>(&gate) : nullptr, perm_out != 0), out_vec);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -599,6 +656,8 @@ bool encode_half(CUtensorMap* map, const __half* base, int rank, const cuuint64_
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// One CTA per SM, in whole groups of one per KV head.
+int tile_ctas(int hkv, int num_sms) { return (num_sms / hkv > 0 ? num_sms / hkv : 1) * hkv; }
 struct TileDims { int tile_pos, tiles, rows; long long items; };
 TileDims tile_dims(int batch, int rows_per_seq, int hq, int hkv) {
     TileDims d;
@@ -606,7 +665,7 @@ TileDims tile_dims(int batch, int rows_per_seq, int hq, int hkv) {
     d.tiles = (rows_per_seq + kTileRows / group - 1) / (kTileRows / group);
     d.tile_pos = (rows_per_seq + d.tiles - 1) / d.tiles;  // evenly filled
     d.rows = d.tile_pos * group;
-    d.items = static_cast<long long>(batch) * hkv * d.tiles;
+    d.items = static_cast<long long>(batch) * d.tiles;
     return d;
 }
 
@@ -617,7 +676,7 @@ TileDims tile_dims(int batch, int rows_per_seq, int hq, int hkv) {
 size_t attn_tile_scratch_bytes(int batch, int rows_per_seq, int hq, int hkv, int num_sms) {
     const int group = hq / hkv, most_pos = kTileRows / group < rows_per_seq ? kTileRows / group : rows_per_seq;
     const TileDims d = tile_dims(batch, rows_per_seq, hq, hkv);
-    return static_cast<size_t>(num_sms) * 2 * (most_pos * group) * (kDim + 2) * sizeof(float) + (static_cast<size_t>(d.items) + 2) * sizeof(int);
+    return static_cast<size_t>(tile_ctas(hkv, num_sms)) * 2 * (most_pos * group) * (kDim + 2) * sizeof(float) + static_cast<size_t>(d.items) * sizeof(int2);
 }
 
 int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status) {
@@ -625,7 +684,7 @@ int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status) {
     memset(&p, 0, sizeof(p));
     const int group = a.hq / a.hkv;
     const TileDims d = tile_dims(a.batch, a.rows_per_seq, a.hq, a.hkv);
-    if (d.items > (1 << 24)) return -2;
+    if (d.items * a.hkv > (1 << 24)) return -2;
     {
         const cuuint64_t head = kDim * 2, pos = head * a.hq;
         const cuuint64_t dims[4] = {kDim, static_cast<cuuint64_t>(a.hq), static_cast<cuuint64_t>(a.rows_per_seq), static_cast<cuuint64_t>(a.batch)};
@@ -657,8 +716,9 @@ int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status) {
     p.early = a.early;
     p.scale2 = a.scale * 1.4426950408889634f;
     p.part_o = a.scratch;
-    p.part_ml = a.scratch + static_cast<size_t>(num_sms) * 2 * d.rows * kDim;
-    p.table = reinterpret_cast<int*>(p.part_ml + static_cast<size_t>(num_sms) * 2 * d.rows * 2);
+    const int ctas = tile_ctas(a.hkv, num_sms);
+    p.part_ml = a.scratch + static_cast<size_t>(ctas) * 2 * d.rows * kDim;
+    p.table = reinterpret_cast<int2*>(p.part_ml + static_cast<size_t>(ctas) * 2 * d.rows * 2);
     p.wait_limit = tc_wait_limit();
     p.status = status;
     {
@@ -668,14 +728,18 @@ int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status) {
         if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
         std::lock_guard<std::mutex> lock(mu);
         if (!configured[dev]) {
-            if (cudaFuncSetAttribute(attn_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTileSmemBytes)) != cudaSuccess)
+            if (cudaFuncSetAttribute(attn_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
                 return -1;
             configured[dev] = true;
         }
     }
-    if (launch_pdl(attn_tile_kernel, dim3(num_sms), dim3(kTileThreads), kTileSmemBytes, s, p) != cudaSuccess) return -1;
-    if (launch_pdl(attn_tile_combine_kernel, dim3(p.sh.items, (d.rows + 7) / 8), dim3(256), 0, s, a.out, static_cast<const float*>(p.part_o),
-                   static_cast<const float*>(p.part_ml), static_cast<const int*>(p.table), a.q_gate, p.sh, a.perm_out, p.out_vec) != cudaSuccess)
+    if (launch_pdl(attn_tile_kernel, dim3(ctas), dim3(kTileThreads), tile_smem_bytes(d.rows), s, p) != cudaSuccess) return -1;
+    // (every item a single block: nothing was cut)
+    if (!a.ctx && static_cast<long long>(a.ctx_base) + a.rows_per_seq <= kTileKeys) return 0;
+    const bool wide = d.tiles == 1 && ctas >= 8 * a.batch * a.hkv;  // eight parts a row
+    if (launch_pdl(wide ? attn_tile_combine_kernel<8> : attn_tile_combine_kernel<1>, dim3(p.sh.items * a.hkv, wide ? d.rows : (d.rows + 7) / 8),
+                   dim3(256), 0, s, a.out, static_cast<const float*>(p.part_o), static_cast<const float*>(p.part_ml),
+                   static_cast<const int2*>(p.table), a.q_gate, p.sh, a.perm_out, p.out_vec) != cudaSuccess)
         return -1;
     return 0;
 }
