@@ -139,6 +139,11 @@ int run_linear(xinfer_stream_t s, const void* x, xb::ActType in, bool out_f32, c
         if (r == -1) return fail_cuda(cudaGetLastError());
         // r < -1: the problem could not be described to the tensor-core kernel; use CUDA cores
     }
+    if (in == xb::ActType::F32 && out_f32 && xb::f32_eligible(x, proj, num, swiglu, m, k, group_size)) {
+        const int f = xb::f32_launch(stream, x, proj, num, swiglu, m, k, c->num_sms);
+        if (f == 0) { g_last_path = 2; return XINFER_OK; }
+        if (f == -1) return fail_cuda(cudaGetLastError());
+    }
     int r = xb::simt_launch(stream, x, in, out_f32, proj, num, swiglu, m, k, group_size);
     if (r != 0) return fail_cuda(cudaGetLastError());
     g_last_path = 2;

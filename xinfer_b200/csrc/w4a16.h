@@ -75,6 +75,10 @@ int tc_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num, b
 constexpr int kTcXPermuted = 1;
 constexpr int kTcYPermuted = 2;
 
+// ---- fp32 activations (w4a16_f32.cu): any m, k % 128 == 0, 16-byte aligned operands
+bool f32_eligible(const void* x, const TcProj* proj, int num, bool swiglu, long long m, long long k, int group_size);
+int f32_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms);
+
 // ---- CUDA-core path (w4a16_simt.cu): any m, fp16 or fp32 activations, any shape the reference accepts
 enum class ActType { F16, F32 };
 int simt_launch(cudaStream_t stream, const void* x, ActType in, bool out_f32, const TcProj* proj, int num,

@@ -1,6 +1,5 @@
-// W4A16 linear on CUDA cores: the path for fp32 activations (the reference's "reference and oracle
-// testing" overloads), for M beyond the tensor-core kernel's 32 rows, and for shapes the tensor-core
-// kernel does not take (K not a multiple of 128, unaligned pointers, group sizes other than 128).
+// W4A16 linear on CUDA cores: the path for shapes the tensor-core kernels do not take (K not a multiple of 128, unaligned
+// pointers, group sizes other than 128).
 //
 // Same contracts as the reference's kernels:
 //   linear_int4 / splitk_int4_impl   src/ops/linear.cpp:33-305
@@ -69,18 +68,6 @@ __device__ __forceinline__ void load_x32(const __half* x, float* out) {
         }
     }
 }
-__device__ __forceinline__ void load_x32(const float* x, float* out) {
-    const float4* p = reinterpret_cast<const float4*>(x);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const float4 v = __ldg(p + i);
-        out[i * 4] = v.x;
-        out[i * 4 + 1] = v.y;
-        out[i * 4 + 2] = v.z;
-        out[i * 4 + 3] = v.w;
-    }
-}
-
 // fp32 dot of 32 activations with 32 int4 weights (16 bytes), nibble i of word j <-> k = 8 j + i,
 // value = (int32(word) << (28 - 4 i)) >> 28 as in src/ops/linear.cpp:100-110.
 __device__ __forceinline__ float dot32(const uint4& wv, const float* x) {
@@ -98,7 +85,7 @@ __device__ __forceinline__ float dot32(const uint4& wv, const float* x) {
     return dot;
 }
 
-template <typename InT, typename OutT, int MB>
+template <typename OutT, int MB>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) w4a16_simt_kernel(const SimtParams p) {
     const int lane = threadIdx.x & 31;
     const long long pair = static_cast<long long>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -123,7 +110,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) w4a16_simt_kernel(const S
     const uint8_t* wb = has_b ? pb.w + row_b * row_bytes : nullptr;
     const __half* sa = pa.scales + row_a * p.groups;
     const __half* sb = has_b ? pb.scales + row_b * p.groups : nullptr;
-    const InT* x = static_cast<const InT*>(p.x);
+    const __half* x = static_cast<const __half*>(p.x);
 
     float acc_a[MB], acc_b[MB];
 #pragma unroll
@@ -227,24 +214,27 @@ __global__ void w4a16_generic_kernel(const SimtParams p) {
 }
 
 template <typename InT, typename OutT>
-cudaError_t launch_typed(cudaStream_t stream, const SimtParams& p, bool fast) {
-    if (!fast) {
-        long long total_n = 0;
-        for (int i = 0; i < (p.swiglu ? 1 : p.num); ++i) total_n += p.proj[i].n;
-        const long long total = p.m * total_n;
-        const int threads = 128;
-        w4a16_generic_kernel<InT, OutT><<<static_cast<unsigned>((total + threads - 1) / threads), threads, 0, stream>>>(p);
-        return cudaGetLastError();
-    }
+cudaError_t launch_generic(cudaStream_t stream, const SimtParams& p) {
+    long long total_n = 0;
+    for (int i = 0; i < (p.swiglu ? 1 : p.num); ++i) total_n += p.proj[i].n;
+    const long long total = p.m * total_n;
+    const int threads = 128;
+    w4a16_generic_kernel<InT, OutT><<<static_cast<unsigned>((total + threads - 1) / threads), threads, 0, stream>>>(p);
+    return cudaGetLastError();
+}
+
+template <typename OutT>
+cudaError_t launch_half(cudaStream_t stream, const SimtParams& p, bool fast) {
+    if (!fast) return launch_generic<__half, OutT>(stream, p);
     const unsigned blocks = static_cast<unsigned>((p.pairs + kWarpsPerBlock - 1) / kWarpsPerBlock);
     const int threads = kWarpsPerBlock * 32;
     if (p.m == 1) {
-        w4a16_simt_kernel<InT, OutT, 1><<<dim3(blocks, 1), threads, 0, stream>>>(p);
+        w4a16_simt_kernel<OutT, 1><<<dim3(blocks, 1), threads, 0, stream>>>(p);
     } else if (p.m == 2) {
-        w4a16_simt_kernel<InT, OutT, 2><<<dim3(blocks, 1), threads, 0, stream>>>(p);
+        w4a16_simt_kernel<OutT, 2><<<dim3(blocks, 1), threads, 0, stream>>>(p);
     } else {
         const unsigned my = static_cast<unsigned>((p.m + 3) / 4);
-        w4a16_simt_kernel<InT, OutT, 4><<<dim3(blocks, my), threads, 0, stream>>>(p);
+        w4a16_simt_kernel<OutT, 4><<<dim3(blocks, my), threads, 0, stream>>>(p);
     }
     return cudaGetLastError();
 }
@@ -283,9 +273,9 @@ int simt_launch(cudaStream_t stream, const void* x, ActType in, bool out_f32, co
     if (p.groups <= 0 || pairs <= 0) return 0;
     cudaError_t e;
     if (in == ActType::F16) {
-        e = out_f32 ? launch_typed<__half, float>(stream, p, fast) : launch_typed<__half, __half>(stream, p, fast);
+        e = out_f32 ? launch_half<float>(stream, p, fast) : launch_half<__half>(stream, p, fast);
     } else {
-        e = out_f32 ? launch_typed<float, float>(stream, p, fast) : launch_typed<float, __half>(stream, p, fast);
+        e = out_f32 ? launch_generic<float, float>(stream, p) : launch_generic<float, __half>(stream, p);
     }
     return e == cudaSuccess ? 0 : -1;
 }
