@@ -27,11 +27,12 @@ struct DeviceCtx {
     bool ready = false;
     int num_sms = 0;
     float* workspace = nullptr;   // split-K partials
-    int* counters = nullptr;      // tile arrival counters, zero between launches
+    int* counters = nullptr;      // tile arrival counters and the synchronous acceptance's, zero between launches
     int* status = nullptr;        // device status word
     void* sampling = nullptr;     // (row, chunk) partials
-    long long* small_dev = nullptr;   // staging for the synchronous sampling calls
-    long long* small_host = nullptr;  // pinned
+    long long* small_host = nullptr;  // pinned: the results of the synchronous sampling calls
+    std::mutex accept_mutex;          // of the synchronous acceptance call
+    unsigned accept_ticket = 0;
     int forced_path = 0;              // xinfer_set_linear_path, per device
     float* gemm_partials = nullptr;   // fp32 partial sums of the prefill GEMM's K splits (taken at its first use)
     bool gemm_partials_tried = false;
@@ -67,12 +68,12 @@ int get_ctx(DeviceCtx** out) {
             c.num_sms = prop.multiProcessorCount;
             const size_t ws = xb::tc_workspace_bytes(c.num_sms);
             if ((e = cudaMalloc(&c.workspace, ws)) != cudaSuccess) return fail_cuda(e);
-            if ((e = cudaMalloc(&c.counters, kCounterCapacity * sizeof(int))) != cudaSuccess) return fail_cuda(e);
+            if ((e = cudaMalloc(&c.counters, (kCounterCapacity + 1) * sizeof(int))) != cudaSuccess) return fail_cuda(e);
             if ((e = cudaMalloc(&c.status, sizeof(int))) != cudaSuccess) return fail_cuda(e);
             if ((e = cudaMalloc(&c.sampling, kSamplingScratchBytes)) != cudaSuccess) return fail_cuda(e);
-            if ((e = cudaMalloc(&c.small_dev, kSmallBytes)) != cudaSuccess) return fail_cuda(e);
             if ((e = cudaMallocHost(&c.small_host, kSmallBytes)) != cudaSuccess) return fail_cuda(e);
-            if ((e = cudaMemset(c.counters, 0, kCounterCapacity * sizeof(int))) != cudaSuccess) return fail_cuda(e);
+            memset(c.small_host, 0, kSmallBytes);
+            if ((e = cudaMemset(c.counters, 0, (kCounterCapacity + 1) * sizeof(int))) != cudaSuccess) return fail_cuda(e);
             if ((e = cudaMemset(c.status, 0, sizeof(int))) != cudaSuccess) return fail_cuda(e);
             if ((e = cudaDeviceSynchronize()) != cudaSuccess) return fail_cuda(e);
             c.ready = true;
@@ -343,15 +344,14 @@ int64_t xinfer_argmax(xinfer_stream_t s, const float* logits, int64_t vocab, flo
     if (get_ctx(&c) != XINFER_OK) return -1;
     if (xb::sampling_scratch_bytes(1, vocab) > kSamplingScratchBytes) return -1;
     cudaStream_t stream = static_cast<cudaStream_t>(s);
-    if (xb::argmax_rows(stream, logits, vocab, 1, vocab, c->sampling, c->small_dev, partial_max,
+    if (xb::argmax_rows(stream, logits, vocab, 1, vocab, c->sampling, c->small_host + kSmallBytes / 16, partial_max,
                         reinterpret_cast<long long*>(partial_idx)) != 0) {
         fail_cuda(cudaGetLastError());
         return -1;
     }
-    cudaError_t e = cudaMemcpyAsync(c->small_host, c->small_dev, sizeof(long long), cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    cudaError_t e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) { fail_cuda(e); return -1; }
-    return c->small_host[0];
+    return c->small_host[kSmallBytes / 16];
 }
 
 int xinfer_speculative_accept_reject_batched(xinfer_stream_t s, const int64_t* draft_tokens, const float* logits,
@@ -421,32 +421,36 @@ int xinfer_speculative_accept_reject(xinfer_stream_t s, const int64_t* draft_tok
     DeviceCtx* c = nullptr;
     int rc = get_ctx(&c);
     if (rc != XINFER_OK) return rc;
-    cudaStream_t stream = static_cast<cudaStream_t>(s);
-    // staging layout in the pinned / device small buffers (8-byte words):
-    //   [0, n) tokens | [n, 2n) probs (floats, first half of the words) | [2n, 3n) uniforms | record after
-    long long* h = c->small_host;
-    memcpy(h, draft_tokens, n * sizeof(int64_t));
-    float* h_probs = reinterpret_cast<float*>(h + n);
-    float* h_unif = reinterpret_cast<float*>(h + 2 * n);
-    if (draft_probs) memcpy(h_probs, draft_probs, n * sizeof(float));
+    if (xb::sampling_scratch_bytes(static_cast<long long>(n), vocab) > kSamplingScratchBytes) return XINFER_ERR_INVALID_ARGUMENT;
+    static_assert(XINFER_MAX_DRAFT_TOKENS <= xb::kAcceptHostMax, "argument block");
+    xb::AcceptHostArgs args;
+    memset(&args, 0, sizeof(args));
+    args.n = static_cast<int>(n);
+    args.stochastic = draft_probs ? 1 : 0;
+    memcpy(args.tokens, draft_tokens, n * sizeof(int64_t));
     if (draft_probs) {
-        if (rand_uniform) memcpy(h_unif, rand_uniform, n * sizeof(float));
-        else memset(h_unif, 0, n * sizeof(float));  // missing uniforms mean r = 0, sampling.cpp:130
+        memcpy(args.probs, draft_probs, n * sizeof(float));
+        if (rand_uniform) memcpy(args.uniforms, rand_uniform, n * sizeof(float));  // missing uniforms mean r = 0, sampling.cpp:130
     }
-    cudaError_t e = cudaMemcpyAsync(c->small_dev, h, 3 * n * sizeof(long long), cudaMemcpyHostToDevice, stream);
-    if (e != cudaSuccess) return fail_cuda(e);
-    long long* d = c->small_dev;
-    xinfer_accept_record* d_rec = reinterpret_cast<xinfer_accept_record*>(d + 3 * n);
-    rc = xinfer_speculative_accept_reject_batched(
-        s, reinterpret_cast<const int64_t*>(d), logits, vocab, vocab,
-        draft_probs ? reinterpret_cast<const float*>(d + n) : nullptr,
-        draft_probs ? reinterpret_cast<const float*>(d + 2 * n) : nullptr, 1.0f, 1, static_cast<int>(n),
-        static_cast<int>(n), static_cast<int>(n) - 1, d_rec);
-    if (rc != XINFER_OK) return rc;
-    xinfer_accept_record* h_rec = reinterpret_cast<xinfer_accept_record*>(h + 3 * n);
-    e = cudaMemcpyAsync(h_rec, d_rec, sizeof(*h_rec), cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return fail_cuda(e);
+    xb::AcceptOut rec;
+    {
+        // one call at a time per device: the slot, the counter and the partials are the device's
+        std::lock_guard<std::mutex> lock(c->accept_mutex);
+        xb::AcceptHostSlot* slot = reinterpret_cast<xb::AcceptHostSlot*>(c->small_host);
+        const unsigned ticket = ++c->accept_ticket;
+        if (xb::accept_host(static_cast<cudaStream_t>(s), logits, vocab, args, c->sampling, c->counters + kCounterCapacity, slot, ticket) != 0)
+            return fail_cuda(cudaGetLastError());
+        const volatile unsigned* seen = &slot->ticket;
+        for (int spins = 0; *seen != ticket; ++spins) {
+            if ((spins & 1023) != 1023) continue;
+            // (every so often: has the stream come to an end without the record, or with an error?)
+            const cudaError_t e = cudaStreamQuery(static_cast<cudaStream_t>(s));
+            if (e != cudaErrorNotReady && *seen != ticket) return fail_cuda(e == cudaSuccess ? cudaErrorUnknown : e);
+        }
+        __sync_synchronize();
+        rec = slot->record;
+    }
+    const xb::AcceptOut* h_rec = &rec;
     out->bonus_or_resampled_token = h_rec->bonus_or_resampled_token;
     out->rejected_token = h_rec->rejected_token;
     out->num_accepted = h_rec->num_accepted;

@@ -18,6 +18,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "sampling.h"
 
 namespace xb {
@@ -63,13 +64,8 @@ __device__ __forceinline__ unsigned long long nucleus_weight(float scaled, float
     return __float2ull_rn(expf(scaled - max_scaled) * 4294967296.0f);
 }
 
-// grid = (chunks, rows).  `row_stride` is the distance between logit rows in floats.
-__global__ void __launch_bounds__(kThreads) logits_partials_kernel(const float* __restrict__ logits, long long row_stride,
-                                                                   int vocab, float inv_t, int want_sum,
-                                                                   Partial* __restrict__ out, int chunks, int idx_offset) {
-    const int row = blockIdx.y;
-    const int chunk = blockIdx.x;
-    const float* l = logits + static_cast<long long>(row) * row_stride;
+// The partial of one chunk of the row at `l`, by a block; every thread gets it.
+__device__ __forceinline__ Partial chunk_partial(const float* l, int chunk, int vocab, float inv_t, int want_sum, int idx_offset) {
     const int base = chunk * kChunk;
     const int end = min(vocab, base + kChunk);
 
@@ -159,6 +155,15 @@ __global__ void __launch_bounds__(kThreads) logits_partials_kernel(const float* 
         res.max_scaled = ms;
         res.sum_exp = se;
     }
+    return res;
+}
+
+// grid = (chunks, rows).  `row_stride` is the distance between logit rows in floats.
+__global__ void __launch_bounds__(kThreads) logits_partials_kernel(const float* logits, long long row_stride, int vocab, float inv_t,
+                                                                   int want_sum, Partial* out, int chunks, int idx_offset) {
+    griddep_prologue();
+    const int row = blockIdx.y, chunk = blockIdx.x;
+    const Partial res = chunk_partial(logits + static_cast<long long>(row) * row_stride, chunk, vocab, inv_t, want_sum, idx_offset);
     if (threadIdx.x == 0) out[static_cast<long long>(row) * chunks + chunk] = res;
 }
 
@@ -201,11 +206,20 @@ __device__ __forceinline__ void merge_row(const Partial* p, int chunks, int nsli
 
 __global__ void argmax_finish_kernel(const Partial* partials, int chunks, int nslices, long long slice_stride,
                                      long long* out) {
+    griddep_prologue();
     const int row = blockIdx.x;
     float mx, ms, se;
     int idx;
     merge_row(partials + static_cast<long long>(row) * chunks, chunks, nslices, slice_stride, threadIdx.x, mx, idx, ms, se);
     if (threadIdx.x == 0) out[row] = idx < 0 ? 0 : idx;
+}
+
+// Whether draft token d is kept where the target's argmax is t: the reference's rule (src/ops/sampling.cpp:117-157).
+template <typename F>
+__device__ __forceinline__ bool keep_draft(long long d, int t, bool stochastic, float p_draft, float r, F p_target) {
+    if (!stochastic || p_draft <= 0.f) return d == t;
+    if (d == t && r <= 0.f) return true;
+    return r < (p_target() / p_draft);
 }
 
 // One warp per sequence.  Rows of sequence b are b * rows_per_seq + i.
@@ -214,6 +228,7 @@ __global__ void accept_finish_kernel(const Partial* partials, int chunks, int ns
                                      int vocab, float inv_t, const long long* draft_tokens, const float* draft_probs,
                                      const float* uniforms, int num_draft, int rows_per_seq, int bonus_row,
                                      const Nucleus* nucleus, AcceptOut* out) {
+    griddep_prologue();
     const int b = blockIdx.x;
     const int lane = threadIdx.x;
     AcceptOut r;
@@ -231,33 +246,19 @@ __global__ void accept_finish_kernel(const Partial* partials, int chunks, int ns
         int t;
         merge_row(partials + row * chunks, chunks, nslices, slice_stride, lane, mx, t, ms, se);
         const long long d = draft_tokens[static_cast<long long>(b) * num_draft + i];
-        bool accepted;
-        if (!draft_probs) {
-            accepted = (d == t);
-        } else {
-            const float p_draft = draft_probs[static_cast<long long>(b) * num_draft + i];
-            const float rr = uniforms ? uniforms[static_cast<long long>(b) * num_draft + i] : 0.f;
-            if (p_draft <= 0.f) {
-                accepted = (d == t);
-            } else if (d == t && rr <= 0.f) {
-                accepted = true;
-            } else {
-                float p_target = 0.f;
-                if (nucleus) {
-                    // the target's distribution cut to its nucleus: zero outside, w / Z_nucleus inside
-                    const Nucleus q = nucleus[row];
-                    if (d >= 0 && d < vocab && q.z > 0) {
-                        const float sv = logits[row * row_stride + d] * inv_t;
-                        if (order_key(sv) >= q.thr_key)
-                            p_target = static_cast<float>(static_cast<double>(nucleus_weight(sv, q.max_scaled)) /
-                                                          static_cast<double>(q.z));
-                    }
-                } else if (d >= 0 && d < vocab && se > 0.f) {
-                    p_target = expf(logits[row * row_stride + d] * inv_t - ms) / se;
-                }
-                accepted = rr < (p_target / p_draft);
+        const float p_draft = draft_probs ? draft_probs[static_cast<long long>(b) * num_draft + i] : 0.f;
+        const float rr = draft_probs && uniforms ? uniforms[static_cast<long long>(b) * num_draft + i] : 0.f;
+        const bool accepted = keep_draft(d, t, draft_probs != nullptr, p_draft, rr, [&]() -> float {
+            if (d < 0 || d >= vocab) return 0.f;
+            const float sv = logits[row * row_stride + d] * inv_t;
+            if (nucleus) {
+                // the target's distribution cut to its nucleus: zero outside, w / Z_nucleus inside
+                const Nucleus q = nucleus[row];
+                if (q.z == 0 || order_key(sv) < q.thr_key) return 0.f;
+                return static_cast<float>(static_cast<double>(nucleus_weight(sv, q.max_scaled)) / static_cast<double>(q.z));
             }
-        }
+            return se > 0.f ? expf(sv - ms) / se : 0.f;
+        });
         if (accepted) {
             r.num_accepted++;
         } else {
@@ -293,6 +294,59 @@ __device__ __forceinline__ void philox4x32_10(uint32_t c[4], uint32_t k0, uint32
         k0 += 0x9E3779B9u;
         k1 += 0xBB67AE85u;
     }
+}
+
+// The synchronous call for one sequence, in one launch and without a copy in either direction: the host's values come as
+// launch parameters, the block that finishes last merges the rows (a warp each) and runs the scan, and the record goes into
+// the host's pinned memory with a ticket behind it that the host polls.  (Copy in, two kernels, copy out and a stream
+// synchronisation before: 44 us a call from Python against 25, a third of that Python.)
+__global__ void __launch_bounds__(kThreads) accept_host_kernel(const float* logits, int vocab, const __grid_constant__ AcceptHostArgs a,
+                                                               Partial* partials, int chunks, int* counter, AcceptHostSlot* slot,
+                                                               unsigned ticket) {
+    griddep_prologue();
+    __shared__ float s_ms[kAcceptHostMax], s_se[kAcceptHostMax];
+    __shared__ int s_t[kAcceptHostMax], s_last;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const Partial res = chunk_partial(logits + static_cast<long long>(blockIdx.y) * vocab, blockIdx.x, vocab, 1.0f, a.stochastic, 0);
+    if (threadIdx.x == 0) {
+        partials[static_cast<long long>(blockIdx.y) * chunks + blockIdx.x] = res;
+        __threadfence();
+        const int total = gridDim.x * gridDim.y;
+        s_last = atomicAdd(counter, 1) == total - 1;
+        if (s_last) *counter = 0;  // as the next launch expects it
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
+    for (int i = warp; i < a.n; i += kThreads / 32) {
+        float mx, ms, se;
+        int t;
+        merge_row(partials + static_cast<long long>(i) * chunks, chunks, 1, 0, lane, mx, t, ms, se);
+        if (lane == 0) { s_ms[i] = ms; s_se[i] = se; s_t[i] = t; }
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    AcceptOut r = {-1, -1, 0, 0, 0, 0, 0, 0};
+    for (int i = 0; i < a.n; ++i) {
+        const long long d = a.tokens[i];
+        if (keep_draft(d, s_t[i], a.stochastic, a.probs[i], a.uniforms[i], [&]() -> float {
+                return d >= 0 && d < vocab && s_se[i] > 0.f ? expf(logits[static_cast<long long>(i) * vocab + d] - s_ms[i]) / s_se[i] : 0.f;
+            })) {
+            r.num_accepted++;
+            continue;
+        }
+        r.has_rejected_token = 1;
+        r.rejected_token = d;
+        r.num_rejected = 1;
+        r.bonus_or_resampled_token = s_t[i];
+        r.num_resampled = 1;
+        r.num_remaining = a.n - (r.num_accepted + 1);
+        break;
+    }
+    if (!r.has_rejected_token) r.bonus_or_resampled_token = s_t[a.n - 1];
+    slot->record = r;
+    __threadfence_system();
+    *const_cast<volatile unsigned*>(&slot->ticket) = ticket;
 }
 
 __global__ void philox_uniform_kernel(float* out, long long n, unsigned long long seed, unsigned long long subseq) {
@@ -741,16 +795,15 @@ size_t sampling_scratch_bytes(long long rows, long long vocab) {
 int sampling_partials(cudaStream_t stream, const float* logits, long long row_stride, int rows, long long vocab,
                       float inv_temperature, bool want_sum, long long idx_offset, void* partials_out) {
     const int chunks = sampling_chunks(vocab);
-    logits_partials_kernel<<<dim3(chunks, rows), kThreads, 0, stream>>>(
-        logits, row_stride, static_cast<int>(vocab), inv_temperature, want_sum ? 1 : 0, static_cast<Partial*>(partials_out),
-        chunks, static_cast<int>(idx_offset));
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_pdl(logits_partials_kernel, dim3(chunks, rows), dim3(kThreads), 0, stream, logits, row_stride, static_cast<int>(vocab),
+                      inv_temperature, want_sum ? 1 : 0, static_cast<Partial*>(partials_out), chunks,
+                      static_cast<int>(idx_offset)) == cudaSuccess ? 0 : -1;
 }
 
 int argmax_finish(cudaStream_t stream, const void* partials, int chunks, int nslices, long long slice_stride, int rows,
                   long long* out_dev) {
-    argmax_finish_kernel<<<rows, 32, 0, stream>>>(static_cast<const Partial*>(partials), chunks, nslices, slice_stride, out_dev);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_pdl(argmax_finish_kernel, dim3(rows), dim3(32), 0, stream, static_cast<const Partial*>(partials), chunks, nslices,
+                      slice_stride, out_dev) == cudaSuccess ? 0 : -1;
 }
 
 int accept_finish(cudaStream_t stream, const void* partials, int chunks, int nslices, long long slice_stride,
@@ -758,10 +811,9 @@ int accept_finish(cudaStream_t stream, const void* partials, int chunks, int nsl
                   const long long* draft_tokens, const float* draft_probs, const float* uniforms, int batch,
                   int num_draft, int rows_per_seq, int bonus_row, AcceptOut* out_dev, const Nucleus* nucleus) {
     if (nslices > 1 && draft_probs) return -2;  // the stochastic rule reads the draft token's logit: one slice only
-    accept_finish_kernel<<<batch, 32, 0, stream>>>(static_cast<const Partial*>(partials), chunks, nslices, slice_stride, logits,
-                                                   row_stride, static_cast<int>(vocab), inv_temperature, draft_tokens,
-                                                   draft_probs, uniforms, num_draft, rows_per_seq, bonus_row, nucleus, out_dev);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_pdl(accept_finish_kernel, dim3(batch), dim3(32), 0, stream, static_cast<const Partial*>(partials), chunks, nslices,
+                      slice_stride, logits, row_stride, static_cast<int>(vocab), inv_temperature, draft_tokens, draft_probs, uniforms,
+                      num_draft, rows_per_seq, bonus_row, nucleus, out_dev) == cudaSuccess ? 0 : -1;
 }
 
 int argmax_rows(cudaStream_t stream, const float* logits, long long row_stride, int rows, long long vocab,
@@ -784,6 +836,13 @@ int accept_reject_batched(cudaStream_t stream, const float* logits, long long ro
         return -1;
     return accept_finish(stream, scratch, chunks, 1, 0, logits, row_stride, vocab, inv_temperature, draft_tokens,
                          draft_probs, uniforms, batch, num_draft, rows_per_seq, bonus_row, out_dev);
+}
+
+int accept_host(cudaStream_t stream, const float* logits, long long vocab, const AcceptHostArgs& args, void* scratch, int* counter,
+                AcceptHostSlot* slot, unsigned ticket) {
+    const int chunks = sampling_chunks(vocab);
+    return launch_pdl(accept_host_kernel, dim3(chunks, args.n), dim3(kThreads), 0, stream, logits, static_cast<int>(vocab), args,
+                      static_cast<Partial*>(scratch), chunks, counter, slot, ticket) == cudaSuccess ? 0 : -1;
 }
 
 int philox_uniform(cudaStream_t stream, float* out, long long n, unsigned long long seed, unsigned long long subseq) {

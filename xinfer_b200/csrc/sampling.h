@@ -57,6 +57,21 @@ int accept_reject_batched(cudaStream_t stream, const float* logits, long long ro
                           const float* uniforms, int batch, int num_draft, int rows_per_seq, int bonus_row,
                           void* scratch, AcceptOut* out_dev);
 
+// The synchronous form for one sequence (bonus row n - 1, no temperature): `slot` is pinned host memory, which the kernel fills
+// with the record and then the ticket; `counter` a zeroed int, left zeroed.
+constexpr int kAcceptHostMax = 64;
+struct AcceptHostArgs {
+    long long tokens[kAcceptHostMax];
+    float probs[kAcceptHostMax], uniforms[kAcceptHostMax];
+    int n, stochastic;
+};
+struct AcceptHostSlot {
+    AcceptOut record;
+    unsigned ticket;
+};
+int accept_host(cudaStream_t stream, const float* logits, long long vocab, const AcceptHostArgs& args, void* scratch, int* counter,
+                AcceptHostSlot* slot, unsigned ticket);
+
 int philox_uniform(cudaStream_t stream, float* out, long long n, unsigned long long seed, unsigned long long subseq);
 // the subsequence read from device memory at run time (a counter that add_counter advances): graph-replay safe
 int philox_uniform_counter(cudaStream_t stream, float* out, long long n, unsigned long long seed,

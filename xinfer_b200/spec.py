@@ -9,6 +9,7 @@ import torch
 
 from . import _lib
 from ._lib import ModelConfig, check, lib
+from .ops import _stream
 
 
 @dataclass
@@ -171,13 +172,13 @@ class SpecDecoder:
         check(lib().xinfer_spec_decoder_override_drafts(self._h, t.ctypes.data_as(C.c_void_p)), "override_drafts")
 
     def step(self):
-        code = lib().xinfer_spec_decoder_step(self._h, torch.cuda.current_stream().cuda_stream)
+        code = lib().xinfer_spec_decoder_step(self._h, _stream())
         if code < 0:
             raise _lib.XInferError(code, "spec_decoder_step: " + self._err())
 
     def enqueue_linears(self):
         """Measurement: only the W4A16 launches of one step, on the current stream."""
-        code = lib().xinfer_spec_decoder_enqueue_linears(self._h, torch.cuda.current_stream().cuda_stream)
+        code = lib().xinfer_spec_decoder_enqueue_linears(self._h, _stream())
         if code < 0:
             raise _lib.XInferError(code, "enqueue_linears: " + self._err())
 
@@ -188,7 +189,7 @@ class SpecDecoder:
 
     def results(self):
         """(emitted [batch, k+1] int64 with -1 padding, counts [batch]); synchronises the stream."""
-        check(lib().xinfer_spec_decoder_results(self._h, torch.cuda.current_stream().cuda_stream,
+        check(lib().xinfer_spec_decoder_results(self._h, _stream(),
                                                 self._emitted.ctypes.data_as(C.c_void_p),
                                                 self._counts.ctypes.data_as(C.c_void_p)), "spec_decoder_results")
         return self._emitted.copy(), self._counts.copy()
