@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include "launch.cuh"
+#include "ptx_sm100.cuh"
 #include "sampling.h"
 
 namespace xb {
@@ -528,12 +529,31 @@ __device__ __forceinline__ void nucleus_for_each(const float* l, int i0, int i1,
 // every cluster barrier.
 constexpr int kNucCluster = 8;
 constexpr int kNucCand = 4096;
+// Rows of up to 8 * 20 * 1024 tokens stay in registers.  The list of those within kNucCut[i] of the maximum for the smallest
+// i that holds the nucleus is short for a trained model's logits; up to kNucShort of them the leader selects and draws alone.
+constexpr int kNucRegs = 20, kNucCuts = 7, kNucShort = 256;
+__device__ __forceinline__ float nucleus_cut(int i) { return i < 4 ? 1.0f + i : (i == 4 ? 6.0f : (i == 5 ? 8.0f : 11.0f)); }
+
+// The weight the nucleus has to reach, and the point of the running sum over its tokens that a uniform picks.
+__device__ __forceinline__ unsigned long long nucleus_target(float top_p, unsigned long long total) {
+    const double want = ceil(static_cast<double>(top_p) * static_cast<double>(total));
+    const unsigned long long target = want <= 1.0 ? 1ull : static_cast<unsigned long long>(want);
+    return target > total ? total : target;
+}
+__device__ __forceinline__ unsigned long long nucleus_draw(float uniform, unsigned long long z) {
+    const double pos = floor(static_cast<double>(uniform) * static_cast<double>(z));
+    const unsigned long long t = pos <= 0.0 ? 0ull : static_cast<unsigned long long>(pos);
+    return t >= z ? z - 1 : t;
+}
 
 struct NucShared {
     unsigned long long hist[4096];   // bucket limbs (24 KB) / candidate keys (16 KB) + list histogram / row histograms
     unsigned long long wsum[32];
     unsigned long long csum[kNucCluster];   // leader: per-CTA sums
-    float cmax[kNucCluster];                // leader: per-CTA maxima
+    float cmax[kNucCluster];                // per-CTA maxima
+    unsigned long long cz[kNucCluster];     // per-CTA sums of weights
+    float ccut[kNucCluster][kNucCuts], wcut[32][kNucCuts];
+    uint32_t ids[kNucShort];                // leader: token ids of a short candidate list
     float wmax[32];
     unsigned long long above, target, z_nuc;   // leader: results of a level / of the selection
     int bin, count;
@@ -554,24 +574,166 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
     const int cspan = (((vocab + kNucCluster - 1) / kNucCluster) + 31) & ~31;
     const int c0 = min(vocab, crank * cspan), c1 = min(vocab, c0 + cspan);
 
+    const bool in_regs = cspan <= kNucRegs * kNucThreads;
+    float v[kNucRegs];  // scaled logits of the tokens c0 + j * 1024 + tid
+
     // maximum of the scaled logits
     float mx = -INFINITY;
-    nucleus_for_each(l, c0, c1, inv_t, tid, [&](int, float sv) { mx = fmaxf(mx, sv); });
+    if (in_regs) {
+#pragma unroll
+        for (int j = 0; j < kNucRegs; ++j) {
+            const int i = c0 + j * kNucThreads + tid;
+            v[j] = i < c1 ? l[i] : -INFINITY;
+        }
+#pragma unroll
+        for (int j = 0; j < kNucRegs; ++j) {
+            v[j] *= inv_t;
+            mx = fmaxf(mx, v[j]);
+        }
+    } else {
+        nucleus_for_each(l, c0, c1, inv_t, tid, [&](int, float sv) { mx = fmaxf(mx, sv); });
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (lane == 0) sh.wmax[warp] = mx;
-    for (int i = tid; i < 4096; i += kNucThreads) sh.hist[i] = 0;
     if (tid == 0) sh.count = 0;
     __syncthreads();
-    if (tid == 0) {
-        float m = sh.wmax[0];
-        for (int w = 1; w < 32; ++w) m = fmaxf(m, sh.wmax[w]);
-        lead->cmax[crank] = m;
+    if (warp == 0) {
+        float m = sh.wmax[lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane < kNucCluster) cluster.map_shared_rank(&sh, lane)->cmax[crank] = m;
     }
     cluster.sync();
-    float ms = lead->cmax[0];
+    float ms = sh.cmax[0];
 #pragma unroll
-    for (int r = 1; r < kNucCluster; ++r) ms = fmaxf(ms, lead->cmax[r]);
+    for (int r = 1; r < kNucCluster; ++r) ms = fmaxf(ms, sh.cmax[r]);
+
+    unsigned long long above = 0, target = 0;
+    bool listed = false;  // the leader's list holds every token of the nucleus
+    int count = 0;
+    if (in_regs) {
+        // the row's weight, and (in fp32, to choose the cut by) the weight within each distance of the maximum
+        unsigned long long z = 0;
+        float cut[kNucCuts] = {};
+#pragma unroll
+        for (int j = 0; j < kNucRegs; ++j) {
+            z += nucleus_weight(v[j], ms);
+            const float d = ms - v[j];
+            if (d <= nucleus_cut(kNucCuts - 1)) {
+                const float e = expf(v[j] - ms);
+#pragma unroll
+                for (int i = 0; i < kNucCuts; ++i) cut[i] += d <= nucleus_cut(i) ? e : 0.f;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            z += shfl_u64(z, lane ^ o);
+#pragma unroll
+            for (int i = 0; i < kNucCuts; ++i) cut[i] += __shfl_xor_sync(0xffffffffu, cut[i], o);
+        }
+        if (lane == 0) {
+            sh.wsum[warp] = z;
+#pragma unroll
+            for (int i = 0; i < kNucCuts; ++i) sh.wcut[warp][i] = cut[i];
+        }
+        __syncthreads();
+        if (warp <= kNucCuts) {  // warp i < kNucCuts: cut i; the next one: the weight
+            if (warp < kNucCuts) {
+                float c = sh.wcut[lane][warp];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+                if (lane < kNucCluster) cluster.map_shared_rank(&sh, lane)->ccut[crank][warp] = c;
+            } else {
+                unsigned long long t = sh.wsum[lane];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) t += shfl_u64(t, lane ^ o);
+                if (lane < kNucCluster) cluster.map_shared_rank(&sh, lane)->cz[crank] = t;
+            }
+        }
+        cluster.sync();
+        unsigned long long tot = 0;
+#pragma unroll
+        for (int r = 0; r < kNucCluster; ++r) tot += sh.cz[r];
+        target = nucleus_target(top_p, tot);
+        float reach = -1.f;
+#pragma unroll
+        for (int i = kNucCuts - 1; i >= 0; --i) {
+            float c = 0.f;
+#pragma unroll
+            for (int r = 0; r < kNucCluster; ++r) c += sh.ccut[r][i];
+            // (sums of at most 2^18 positive terms, each rounded to 2^-24: well within the margin)
+            if (tot > 0 && c * 0.999f >= static_cast<float>(target) * (1.0f / 4294967296.0f)) reach = nucleus_cut(i);
+        }
+        if (reach >= 0.f) {  // (the same in every CTA)
+            uint32_t* keys = reinterpret_cast<uint32_t*>(lead->hist);
+#pragma unroll
+            for (int j = 0; j < kNucRegs; ++j) {
+                if (ms - v[j] <= reach && nucleus_weight(v[j], ms)) {
+                    const int at = atomicAdd(&lead->count, 1);
+                    if (at < kNucCand) keys[at] = order_key(v[j]);
+                    if (at < kNucShort) lead->ids[at] = static_cast<uint32_t>(c0 + j * kNucThreads + tid);
+                }
+            }
+            cluster.sync();
+            count = lead->count;
+            listed = count <= kNucCand;
+            if (count <= kNucShort) {
+                cluster_arrive();  // (the leader stays until everybody has read its count)
+                if (crank == 0) {
+                    const uint32_t* key = reinterpret_cast<const uint32_t*>(sh.hist);
+                    unsigned long long* weight = sh.hist + kNucCand / 2;  // behind the keys
+                    const uint32_t mine = tid < count ? key[tid] : 0u;
+                    const unsigned long long w = tid < count ? nucleus_weight(key_to_float(mine), ms) : 0ull;
+                    if (tid < count) weight[tid] = w;
+                    __syncthreads();
+                    // the weight at or above each candidate; the threshold is the largest key at which it reaches the target
+                    unsigned long long sum = 0;
+                    if (tid < count)
+                        for (int q = 0; q < count; ++q) sum += key[q] >= mine ? weight[q] : 0ull;
+                    if (warp < kNucShort / 32) {
+                        const uint32_t best = __reduce_max_sync(0xffffffffu, tid < count && sum >= target ? mine : 0u);
+                        if (lane == 0) sh.wmax[warp] = __uint_as_float(best);
+                    }
+                    __syncthreads();
+                    uint32_t thr = 0;
+#pragma unroll
+                    for (int q = 0; q < kNucShort / 32; ++q) thr = max(thr, __float_as_uint(sh.wmax[q]));
+                    if (tid < count && mine == thr) sh.z_nuc = sum;
+                    __syncthreads();
+                    const unsigned long long z_nuc = sh.z_nuc;
+                    if (tid == 0 && nuc_out) {
+                        Nucleus q;
+                        q.z = z_nuc;
+                        q.max_scaled = ms;
+                        q.thr_key = thr;
+                        nuc_out[row] = q;
+                    }
+                    if (uniforms && tid < count && mine >= thr) {
+                        // the candidate in whose range of the running sum over the token ids the draw falls
+                        const unsigned long long t2 = nucleus_draw(uniforms[static_cast<long long>(row) * u_stride], z_nuc);
+                        const uint32_t id = sh.ids[tid];
+                        unsigned long long before = 0;
+                        for (int q = 0; q < count; ++q) before += key[q] >= thr && sh.ids[q] < id ? weight[q] : 0ull;
+                        if (before <= t2 && t2 < before + w) {
+                            tok_out[row] = id;
+                            prob_out[static_cast<long long>(row) * prob_stride] =
+                                static_cast<float>(static_cast<double>(w) / static_cast<double>(z_nuc));
+                        }
+                    }
+                    __syncwarp();
+                    cluster_wait();
+                }
+                return;
+            }
+        }
+        cluster.sync();  // (every CTA has read the count and the sums)
+    }
+    int b0 = 0;
+    if (!listed) {
+    if (tid == 0) sh.count = 0;
+    for (int i = tid; i < 4096; i += kNucThreads) sh.hist[i] = 0;
+    __syncthreads();
 
     // level 0: total weight and a histogram over the distance to the maximum, 64 buckets per unit of scaled logit
     // (the keys themselves crowd into a few exponents: their top bits would send every token of the row to a
@@ -614,9 +776,7 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
         if (warp == 0) {
             unsigned long long tot = 0;
             for (int r = 0; r < kNucCluster; ++r) tot += sh.csum[r];
-            double want = ceil(static_cast<double>(top_p) * static_cast<double>(tot));
-            unsigned long long target = want <= 1.0 ? 1ull : static_cast<unsigned long long>(want);
-            if (target > tot) target = tot;
+            const unsigned long long target = nucleus_target(top_p, tot);
             if (lane == 0) sh.target = target;
             find_bin_desc(
                 [&](int bk) -> unsigned long long {
@@ -627,9 +787,9 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
         }
     }
     cluster.sync();
-    const int b0 = lead->bin;
-    unsigned long long above = lead->above;
-    unsigned long long target = lead->target - above;
+    b0 = lead->bin;
+    above = lead->above;
+    target = lead->target - above;
     cluster.sync();   // (every CTA has read the leader's results and the leader has read every histogram)
 
     // The tokens of bucket b0 (a few dozen of a 150 000-token row, unless many logits are equal) are gathered into a
@@ -644,7 +804,8 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
         }
     });
     cluster.sync();
-    const int count = lead->count;
+    count = lead->count;
+    }
     uint32_t prefix = 0;           // the key bits decided so far
     unsigned long long last = 0;   // weight of the threshold's own bin at the last level
     if (count <= kNucCand) {
@@ -751,9 +912,7 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
     unsigned long long before = 0;
     for (int r = 0; r < crank; ++r) before += lead->csum[r];
     for (int w = 0; w < warp; ++w) before += sh.wsum[w];
-    double pos = floor(static_cast<double>(uniforms[static_cast<long long>(row) * u_stride]) * static_cast<double>(z_nuc));
-    unsigned long long t2 = pos <= 0.0 ? 0ull : static_cast<unsigned long long>(pos);
-    if (t2 >= z_nuc) t2 = z_nuc - 1;
+    const unsigned long long t2 = nucleus_draw(uniforms[static_cast<long long>(row) * u_stride], z_nuc);
     if (mine > 0 && before <= t2 && t2 < before + mine) {   // warp-uniform: exactly one warp of one CTA
         unsigned long long cum = before;
         for (int base = w0; base < w1; base += 32) {
