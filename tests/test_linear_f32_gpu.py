@@ -1,0 +1,38 @@
+"""The fp32 linear at the edges of its tiles (32 weight rows, 8 activation rows) and of its cut over K (clusters of one to eight
+CTAs, groups that do not fill the warps), with activations over a wide range; fused and SwiGLU forms.  Against fp64."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def weights(torch, g, n, k):
+    w = torch.randint(0, 256, (n, k // 2), generator=g, device="cuda", dtype=torch.uint8)
+    s = (torch.randn((n, k // 128), generator=g, device="cuda").abs() * 0.02 / 7).half()
+    q = torch.stack([w & 15, w >> 4], -1).reshape(n, k).double()
+    q = torch.where(q > 7, q - 16, q)
+    return w, s, (q.view(n, -1, 128) * s.double()[..., None]).view(n, k)
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 128, 1), (1, 128, 32), (7, 256, 33), (8, 1024, 31), (9, 1152, 65), (17, 5120, 100), (2, 17408, 96), (33, 640, 5000)])
+def test_linear_f32(M, K, N):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    import xinfer_b200.ops as ops
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    x = torch.randn((M, K), generator=g, device="cuda") * torch.exp(3 * torch.randn((M, K), generator=g, device="cuda"))
+    bias = torch.randn(N, generator=g, device="cuda")
+    (w, s, d), (w2, s2, d2) = weights(torch, g, N, K), weights(torch, g, N, K)
+    rel = lambda got, want: ((got.double() - want).norm() / want.norm()).item()  # noqa: E731
+    # fp32 sums of K products: 2^-24 each step, growing with the root of the number of steps (128 in a group, then the groups)
+    bound = 2 ** -24 * (128 + K / 128) ** 0.5 * 2
+    y = torch.full((M, N), float("nan"), device="cuda")
+    assert ops.linear_int4(y, x, w, s, bias, M, N, K) == 0
+    assert rel(y, x.double() @ d.T + bias.double()) <= bound
+    ys = [torch.full((M, N), float("nan"), device="cuda") for _ in range(2)]
+    assert ops.linear_int4_fused(x, [{"Y": ys[0], "W_int4": w, "scales": s, "N": N}, {"Y": ys[1], "W_int4": w2, "scales": s2, "N": N}], M, K) == 0
+    assert rel(ys[0], x.double() @ d.T) <= bound and rel(ys[1], x.double() @ d2.T) <= bound
+    x /= x.abs().amax()  # (so that the gate neither vanishes nor overflows)
+    assert ops.mlp_gate_up_swiglu_int4(y, x, w, s, w2, s2, M, N, K) == 0
+    gate = x.double() @ d.T
+    assert rel(y, gate / (1 + torch.exp(-gate)) * (x.double() @ d2.T)) <= 4 * bound

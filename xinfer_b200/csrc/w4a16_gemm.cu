@@ -58,7 +58,7 @@ constexpr int kGemmParkPitch = 9;
 constexpr int kGemmParkBytes = 2 * 256 * kGemmParkPitch * 4;  // gate/up exchange: [2][fold thread][8 columns]
 constexpr int kGemmMaxProj = 4;
 // Register split of the launch's 512 x 128: the fold keeps 128 sums per thread.
-constexpr int kFoldRegs = 184, kUnpackRegs = 88, kCtrlRegs = 48;
+constexpr int kFoldRegs = 208, kUnpackRegs = 64, kCtrlRegs = 32;
 static_assert(kFoldRegs * 256 + kUnpackRegs * 128 + kCtrlRegs * 128 <= 65536, "register split");
 
 struct GemmCtrl {
