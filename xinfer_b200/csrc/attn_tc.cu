@@ -305,6 +305,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
                 for (int d = 0; d < kDimBlocks; ++d)
                     tma_load_3d(ring + slot * kKvBytes + d * (kTileKeys * 128), map, bar, kvh * kDim + d * 64, block * kTileKeys, b, pol_kv);
             }
+            __syncwarp();  // (or the other lanes wait for the next slot before this one's load is issued)
         };
         int i = 0, ahead = 0, nq = 0, slot = 0;
         uint32_t parity = 1;  // under which a slot's first use passes at once
@@ -338,6 +339,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
                         for (int d = 0; d < kDimBlocks; ++d)
                             tma_load_4d(smem_u32(q_smem) + d * q_block, &p.q_map, bar, d * 64, kvh * sh.group, walk.item % sh.tiles * sh.tile_pos, b, pol_q);
                     }
+                    __syncwarp();
                     ++nq;
                 }
             }

@@ -46,16 +46,18 @@ constexpr int kGemmThreads = kGemmFoldThreads + kGemmUnpackThreads + 128;  // + 
 constexpr int kGemmUnpackWarp0 = 8, kGemmXWarp = 12, kGemmMmaWarp = 13, kGemmWWarp = 14;
 constexpr int kGemmTileN = 128;   // weight rows of one CTA of a pair (gate/up: 64 of each)
 constexpr int kGemmTileM = 256;   // most activation rows per tile (the MMA's N)
-constexpr int kGemmStageK = 64;   // k per operand slot: one 128-byte swizzle row of fp16
-constexpr int kOpSlots = 5;       // operand ring: a slot holds 64 k of unpacked weights and of activations
-// The packed weights come from HBM, a microsecond and more away: their ring takes what the activations leave of shared
-// memory (6 slots at 256 activation rows), and further groups are pulled into L2 ahead of it.
-constexpr int kWSlotsMax = 10, kWPrefetch = 8;
-constexpr int kWSlotBytes = kGemmTileN * 64;                // 8 KB of packed weights: one 128-k group
-constexpr int kASlotBytes = kGemmTileN * kGemmStageK * 2;   // 16 KB of fp16 weights
+constexpr int kSwizzleK = 64;     // k of one 128-byte swizzle row of fp16
+// Operand ring: a slot holds a whole 128-k group of unpacked weights and of activations.  The MMA warp's own loop - waits, issue
+// and commits, each a hundred clocks or two - is what every stage goes through, and with 64-k slots it took longer than the
+// tensor core: at M = 512 900 TFLOP/s with three waits a slot (weights and activations apart), 1120 now.
+// Accumulator tiles: tiles of at most 128 rows have four, the larger ones two (all of tensor memory).
+constexpr int kOpSlotsMax = 4, kDBufsMax = 4, kWSlotsMax = 8;
+constexpr int kWSlotBytes = kGemmTileN * 64;                    // 8 KB of packed weights: one group
+constexpr int kAHalfBytes = kGemmTileN * kSwizzleK * 2;         // 16 KB: 64 k of unpacked weights
+constexpr int kASlotBytes = 2 * kAHalfBytes;
 constexpr int kGemmTmemCols = 512;
 constexpr int kGemmParkPitch = 9;
-constexpr int kGemmParkBytes = 2 * 256 * kGemmParkPitch * 4;  // gate/up exchange: [2][fold thread][8 columns]
+constexpr int kGemmParkBytes = 256 * kGemmParkPitch * 4;  // gate/up exchange: [fold thread][8 columns]
 constexpr int kGemmMaxProj = 4;
 // Register split of the launch's 512 x 128: the fold keeps 128 sums per thread.
 constexpr int kFoldRegs = 208, kUnpackRegs = 64, kCtrlRegs = 32;
@@ -63,21 +65,27 @@ static_assert(kFoldRegs * 256 + kUnpackRegs * 128 + kCtrlRegs * 128 <= 65536, "r
 
 struct GemmCtrl {
     uint64_t w_full[kWSlotsMax], w_empty[kWSlotsMax];
-    uint64_t a_ready[kOpSlots], x_full[kOpSlots], op_empty[kOpSlots];
-    uint64_t d_full[2], d_empty[2];
+    uint64_t op_full[kOpSlotsMax], op_empty[kOpSlotsMax];  // full: the pair's unpack warps and the activations' bytes
+    uint64_t d_full[kDBufsMax], d_empty[kDBufsMax];
     uint32_t tmem_base;
     int last_arrival;
     WaitState ws;
 };
 
-// [alignment slack] [A ring] [X ring: kOpSlots x tile_m / 2 x 128 bytes] [W ring] [park] [control]
+// [alignment slack] [A ring] [X ring: slots x 2 x tile_m / 2 x 128 bytes] [W ring] [park] [control]
 constexpr int kGemmSmemBytes = 227 * 1024;
-constexpr int kGemmSmemFixed = 1024 + kOpSlots * kASlotBytes + kGemmParkBytes + static_cast<int>(sizeof(GemmCtrl));
+constexpr int kGemmSmemFixed = 1024 + kGemmParkBytes + static_cast<int>(sizeof(GemmCtrl));
+constexpr int gemm_slots_bytes(int tile_m, int slots) { return slots * (kASlotBytes + tile_m * 2 * kSwizzleK); }
+constexpr int gemm_op_slots(int tile_m) {
+    return kGemmSmemFixed + gemm_slots_bytes(tile_m, 4) + 3 * kWSlotBytes <= kGemmSmemBytes ? 4 : 3;
+}
+// (the packed weights come from HBM, a microsecond and more away: their ring takes the rest)
 constexpr int gemm_w_slots(int tile_m) {
-    const int n = (kGemmSmemBytes - kGemmSmemFixed - kOpSlots * tile_m * kGemmStageK) / kWSlotBytes;
+    const int n = (kGemmSmemBytes - kGemmSmemFixed - gemm_slots_bytes(tile_m, gemm_op_slots(tile_m))) / kWSlotBytes;
     return n < kWSlotsMax ? n : kWSlotsMax;
 }
-static_assert(gemm_w_slots(kGemmTileM) >= 4, "shared memory");
+constexpr int gemm_d_bufs(int tile_m) { return tile_m > 128 ? 2 : kDBufsMax; }
+static_assert(gemm_w_slots(kGemmTileM) >= 3 && gemm_w_slots(128) >= 3, "shared memory");
 
 struct GemmProj {
     const __half* scales[2];  // gate/up: of both
@@ -214,9 +222,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
     // the swizzled operand tiles want 1024-byte alignment
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint8_t* a_ring = smem;
-    uint8_t* x_ring = a_ring + kOpSlots * kASlotBytes;
-    const uint32_t x_slot_bytes = static_cast<uint32_t>(p.tile_m) * kGemmStageK;  // this CTA's half of the rows
-    uint8_t* w_ring = x_ring + kOpSlots * x_slot_bytes;
+    const int op_slots = gemm_op_slots(p.tile_m), d_bufs = gemm_d_bufs(p.tile_m), d_shift = d_bufs == 2 ? 1 : 2, d_cols = kGemmTmemCols / d_bufs;
+    uint8_t* x_ring = a_ring + op_slots * kASlotBytes;
+    const uint32_t x_half_bytes = static_cast<uint32_t>(p.tile_m) * kSwizzleK;  // 64 k of this CTA's half of the rows
+    uint8_t* w_ring = x_ring + op_slots * 2 * x_half_bytes;
     const int w_slots = p.w_slots;
     float* park = reinterpret_cast<float*>(w_ring + w_slots * kWSlotBytes);
     GemmCtrl* ctrl = reinterpret_cast<GemmCtrl*>(w_ring + w_slots * kWSlotBytes + kGemmParkBytes);
@@ -230,12 +239,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
 
     if (tid == 0) {
         for (int i = 0; i < w_slots; ++i) { mbar_init(smem_u32(&ctrl->w_full[i]), 1); mbar_init(smem_u32(&ctrl->w_empty[i]), kGemmUnpackThreads / 32); }
-        for (int i = 0; i < kOpSlots; ++i) {
-            mbar_init(smem_u32(&ctrl->a_ready[i]), 2 * kGemmUnpackThreads / 32);
-            mbar_init(smem_u32(&ctrl->x_full[i]), 1);
+        for (int i = 0; i < op_slots; ++i) {
+            mbar_init(smem_u32(&ctrl->op_full[i]), 2 * kGemmUnpackThreads / 32 + 1);
             mbar_init(smem_u32(&ctrl->op_empty[i]), 1);
         }
-        for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&ctrl->d_full[i]), 1); mbar_init(smem_u32(&ctrl->d_empty[i]), 2 * kGemmFoldThreads / 32); }
+        for (int i = 0; i < d_bufs; ++i) { mbar_init(smem_u32(&ctrl->d_full[i]), 1); mbar_init(smem_u32(&ctrl->d_empty[i]), 2 * kGemmFoldThreads / 32); }
         ctrl->ws.abort_flag = 0;
         ctrl->ws.dep_ready = 0;
         ctrl->ws.limit = p.wait_limit;
@@ -258,47 +266,33 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
         setmaxnreg_dec<kCtrlRegs>();
         if (warp == kGemmWWarp) {
             // -------------------------------------------------------------- TMA: packed weights (whole warp waits, one lane issues)
-            // They do not depend on the kernel in front of this one.
+            // They do not depend on the kernel in front of this one.  (Both TMA warps find a tile's coordinates once per tile: with the
+            // projection, the divisions and the address of its map worked out per stage, 500 clocks each, they held everybody up.)
             const bool leader = elect_one_sync();
             if (leader)
                 for (int i = 0; i < (p.swiglu ? 2 : p.num_proj); ++i) tma_prefetch_desc(&p.w_map[i]);
             const uint64_t pol_w = l2_policy_evict_first();
-            // two cursors into the unit list: the one that loads, and one that pulls into L2 ahead of it
-            struct Cursor { int tile, group; } at = {first_tile, first_group}, ahead = at;
-            auto visit = [&](Cursor& c, bool load, uint32_t dst, uint32_t full) {
-                const int pr = proj_of_tile(p, c.tile);
-                const int rel = c.tile - p.proj[pr].tile0, nt2 = rel / p.m_tiles, nt = nt2 * 2 + static_cast<int>(rank);
-                if (leader) {
-                    if (load) {
-                        if (p.swiglu) {
-                            tma_load_2d(dst, &p.w_map[0], full, c.group * 64, nt * 64, pol_w);
-                            tma_load_2d(dst + kWSlotBytes / 2, &p.w_map[1], full, c.group * 64, nt * 64, pol_w);
-                        } else {
-                            tma_load_2d(dst, &p.w_map[pr], full, c.group * 64, nt * kGemmTileN, pol_w);
-                        }
-                    } else if (rel == nt2 * p.m_tiles) {  // the tiles over further activation rows find them there
-                        if (p.swiglu) {
-                            tma_prefetch_l2_2d(&p.w_map[0], c.group * 64, nt * 64);
-                            tma_prefetch_l2_2d(&p.w_map[1], c.group * 64, nt * 64);
-                        } else {
-                            tma_prefetch_l2_2d(&p.w_map[pr], c.group * 64, nt * kGemmTileN);
-                        }
-                    }
-                }
-                if (++c.group == p.groups) { c.group = 0; ++c.tile; }
-            };
-            int slot = 0, n = 0, na = 0;
+            const uint32_t ring = smem_u32(w_ring), full0 = smem_u32(&ctrl->w_full[0]), empty0 = smem_u32(&ctrl->w_empty[0]);
+            int slot = 0, n = 0, group = first_group;
             uint32_t phase = 1;  // parity under which a slot's first use passes at once
-            for (; n < U; ++n) {
-                const uint32_t full = smem_u32(&ctrl->w_full[slot]);
-                if (!mbar_wait_parked(smem_u32(&ctrl->w_empty[slot]), phase, ws)) break;
-                if (leader) mbar_arrive_expect_tx(full, kWSlotBytes);
-                visit(at, true, smem_u32(w_ring) + slot * kWSlotBytes, full);
-                if (++slot == w_slots) { slot = 0; phase ^= 1u; }
-                if (n + 1 >= w_slots) {
-                    if (na <= n) { na = n + 1; ahead = at; }
-                    for (; na < U && na <= n + kWPrefetch; ++na) visit(ahead, false, 0, 0);
+            bool ok = true;
+            for (int tile = first_tile; n < U && ok; ++tile) {
+                const int pr = proj_of_tile(p, tile), nt = (tile - p.proj[pr].tile0) / p.m_tiles * 2 + static_cast<int>(rank);
+                const CUtensorMap *map0 = &p.w_map[p.swiglu ? 0 : pr], *map1 = &p.w_map[1];
+                const int y = nt * (p.swiglu ? 64 : kGemmTileN), end = U - n < p.groups - group ? group + (U - n) : p.groups;
+                for (; group < end; ++group, ++n) {
+                    const uint32_t full = full0 + slot * 8, dst = ring + slot * kWSlotBytes;
+                    ok = mbar_wait_parked(empty0 + slot * 8, phase, ws);
+                    if (!ok) break;
+                    if (leader) {
+                        mbar_arrive_expect_tx(full, kWSlotBytes);
+                        tma_load_2d(dst, map0, full, group * 64, y, pol_w);
+                        if (p.swiglu) tma_load_2d(dst + kWSlotBytes / 2, map1, full, group * 64, y, pol_w);
+                    }
+                    __syncwarp();  // (or the other lanes wait for the next slot before this one's load is issued)
+                    if (++slot == w_slots) { slot = 0; phase ^= 1u; }
                 }
+                group = 0;
             }
             if (ws->abort_flag) {
                 // give the copies still in flight a bounded chance to land before the CTA exits
@@ -315,32 +309,35 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
             const bool leader = elect_one_sync();
             if (leader) tma_prefetch_desc(&p.x_map);
             const uint64_t pol_x = l2_policy_evict_last();
-            int tile = first_tile, group = first_group;
-            const int S = 2 * U;  // 64-k stages, two per unit
-            const int SX = (p.x_stage_limit >= 0 && p.x_stage_limit < S) ? p.x_stage_limit : S;
+            const int SX = (p.x_stage_limit >= 0 && p.x_stage_limit < U) ? p.x_stage_limit : U;
+            const uint32_t ring = smem_u32(x_ring), full0 = smem_u32(&ctrl->op_full[0]), empty0 = smem_u32(&ctrl->op_empty[0]);
+            // both halves of the rows are counted on the even CTA's barrier, where the MMAs are issued
+            const uint32_t pair_full0 = mapa_shared_cluster(full0, 0);
             griddep_wait();
             if (leader) ws->dep_ready = 1;
-            int nx = 0, slot = 0;
+            int nx = 0, slot = 0, k0 = first_group * 128;
             uint32_t phase = 1;
-            for (; nx < SX; ++nx) {
-                if (!mbar_wait_parked(smem_u32(&ctrl->op_empty[slot]), phase, ws)) break;
-                const uint32_t full = smem_u32(&ctrl->x_full[slot]);
-                const int pr = proj_of_tile(p, tile);
-                const int m0 = ((tile - p.proj[pr].tile0) % p.m_tiles) * p.tile_m + static_cast<int>(rank) * (p.tile_m >> 1);
-                if (leader) {
-                    // both halves of the rows are counted on the even CTA's barrier, where the MMAs are issued
-                    if (rank == 0) mbar_arrive_expect_tx(full, 2 * x_slot_bytes);
-                    tma_load_2d_pair(smem_u32(x_ring) + slot * x_slot_bytes, &p.x_map, mapa_shared_cluster(full, 0),
-                                     group * 128 + (nx & 1) * kGemmStageK, m0, pol_x);
+            bool ok = true;
+            for (int tile = first_tile; nx < SX && ok; ++tile) {
+                const int m0 = (tile - p.proj[proj_of_tile(p, tile)].tile0) % p.m_tiles * p.tile_m + static_cast<int>(rank) * (p.tile_m >> 1);
+                for (; k0 < p.groups * 128 && nx < SX; k0 += 128, ++nx) {
+                    ok = mbar_wait_parked(empty0 + slot * 8, phase, ws);
+                    if (!ok) break;
+                    if (leader) {
+                        if (rank == 0) mbar_arrive_expect_tx(full0 + slot * 8, 4 * x_half_bytes);
+                        tma_load_2d_pair(ring + slot * 2 * x_half_bytes, &p.x_map, pair_full0 + slot * 8, k0, m0, pol_x);
+                        tma_load_2d_pair(ring + slot * 2 * x_half_bytes + x_half_bytes, &p.x_map, pair_full0 + slot * 8, k0 + kSwizzleK, m0, pol_x);
+                    }
+                    __syncwarp();
+                    if (++slot == op_slots) { slot = 0; phase ^= 1u; }
                 }
-                if ((nx & 1) && ++group == p.groups) { group = 0; ++tile; }
-                if (++slot == kOpSlots) { slot = 0; phase ^= 1u; }
+                k0 = 0;
             }
             if (ws->abort_flag) {
                 const long long t0 = clock64();
-                for (int i = 0; i < kOpSlots && i < nx; ++i) {
+                for (int i = 0; i < op_slots && i < nx; ++i) {
                     const int k = nx - 1 - i;
-                    while (!mbar_try_wait(smem_u32(&ctrl->x_full[k % kOpSlots]), (k / kOpSlots) & 1u) && clock64() - t0 < p.wait_limit / 8) {
+                    while (!mbar_try_wait(smem_u32(&ctrl->op_full[k % op_slots]), (k / op_slots) & 1u) && clock64() - t0 < p.wait_limit / 8) {
                     }
                 }
             }
@@ -357,28 +354,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
             bool ok = true;
             uint32_t slot = 0, phase = 0;
             for (int i = 0; i < U && ok; ++i) {
-                const uint32_t buf = static_cast<uint32_t>(i & 1);
-                if (i >= 2 && !mbar_wait_parked(smem_u32(&ctrl->d_empty[buf]), ((i >> 1) & 1u) ^ 1u, ws)) break;
-#pragma unroll 1
-                for (int half = 0; half < 2; ++half) {
-                    ok = mbar_wait_parked(smem_u32(&ctrl->x_full[slot]), phase, ws) &&
-                         mbar_wait_parked(smem_u32(&ctrl->a_ready[slot]), phase, ws);
-                    if (!ok) break;
-                    tc_fence_after_sync();
-                    if (leader) {
+                const uint32_t buf = static_cast<uint32_t>(i & (d_bufs - 1));
+                if (i >= d_bufs && !mbar_wait_parked(smem_u32(&ctrl->d_empty[buf]), ((i >> d_shift) & 1u) ^ 1u, ws)) break;
+                ok = mbar_wait_parked(smem_u32(&ctrl->op_full[slot]), phase, ws);
+                if (!ok) break;
+                tc_fence_after_sync();
+                if (leader) {
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const uint32_t alo = desc_lo_const | (a_lo0 + ((slot * kASlotBytes + k * 32) >> 4));
-                            const uint32_t xlo = desc_lo_const | (x_lo0 + ((slot * x_slot_bytes + k * 32) >> 4));
-                            umma_ss_f16_pair(tmem_base + buf * 256, (static_cast<uint64_t>(desc_hi) << 32) | alo,
-                                             (static_cast<uint64_t>(desc_hi) << 32) | xlo, idesc, (half > 0 || k > 0) ? 1u : 0u);
-                        }
-                        umma_commit_pair(smem_u32(&ctrl->op_empty[slot]));
-                        if (half) umma_commit_pair(smem_u32(&ctrl->d_full[buf]));
+                    for (int k = 0; k < 8; ++k) {
+                        const uint32_t alo = desc_lo_const | (a_lo0 + ((slot * kASlotBytes + (k >> 2) * kAHalfBytes + (k & 3) * 32) >> 4));
+                        const uint32_t xlo = desc_lo_const | (x_lo0 + ((slot * 2 * x_half_bytes + (k >> 2) * x_half_bytes + (k & 3) * 32) >> 4));
+                        umma_ss_f16_pair(tmem_base + buf * d_cols, (static_cast<uint64_t>(desc_hi) << 32) | alo,
+                                         (static_cast<uint64_t>(desc_hi) << 32) | xlo, idesc, k > 0 ? 1u : 0u);
                     }
-                    __syncwarp();
-                    if (++slot == kOpSlots) { slot = 0; phase ^= 1u; }
+                    umma_commit_pair(smem_u32(&ctrl->op_empty[slot]));
+                    umma_commit_pair(smem_u32(&ctrl->d_full[buf]));
                 }
+                __syncwarp();
+                if (++slot == static_cast<uint32_t>(op_slots)) { slot = 0; phase ^= 1u; }
             }
         }
     } else if (warp >= kGemmUnpackWarp0) {
@@ -388,40 +381,35 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
         // raw rows of 64 bytes under the 64-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ ((r >> 1) & 3)
         const uint32_t w_row = static_cast<uint32_t>(r) * 64, w_sw = static_cast<uint32_t>((r >> 1) & 3);
         const uint32_t a_row = static_cast<uint32_t>((r >> 3) * 1024 + (r & 7) * 128), a_sw = static_cast<uint32_t>(r & 7);
-        bool ok = true;
         int wslot = 0, aslot = 0;
         uint32_t w_phase = 0, a_phase = 1;
-        for (int i = 0; i < U && ok; ++i) {
+        for (int i = 0; i < U; ++i) {
             if (!mbar_wait(smem_u32(&ctrl->w_full[wslot]), w_phase, ws)) break;
             const uint32_t wsrc = smem_u32(w_ring) + wslot * kWSlotBytes + w_row;
             uint4 v[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) v[c] = lds128(wsrc + ((static_cast<uint32_t>(c) ^ w_sw) << 4));
+            if (!mbar_wait(smem_u32(&ctrl->op_empty[aslot]), a_phase, ws)) break;
+            const uint32_t adst = smem_u32(a_ring) + aslot * kASlotBytes + a_row;
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                if (!mbar_wait(smem_u32(&ctrl->op_empty[aslot]), a_phase, ws)) { ok = false; break; }
-                const uint32_t adst = smem_u32(a_ring) + aslot * kASlotBytes + a_row;
-                const uint32_t words[8] = {v[2 * half].x, v[2 * half].y, v[2 * half].z, v[2 * half].w,
-                                           v[2 * half + 1].x, v[2 * half + 1].y, v[2 * half + 1].z, v[2 * half + 1].w};
-#pragma unroll
-                for (int w = 0; w < 8; ++w) {
-                    uint32_t q[4];
-                    dequant_word(words[w], q);  // (k0,k4) (k1,k5) (k2,k6) (k3,k7)
-                    uint4 o;
-                    o.x = prmt(q[0], q[1], 0x5410u);  // (k0,k1)
-                    o.y = prmt(q[2], q[3], 0x5410u);  // (k2,k3)
-                    o.z = prmt(q[0], q[1], 0x7632u);  // (k4,k5)
-                    o.w = prmt(q[2], q[3], 0x7632u);  // (k6,k7)
-                    sts128(adst + ((static_cast<uint32_t>(w) ^ a_sw) << 4), o);
-                }
-                fence_proxy_async_smem();  // the tensor core reads this tile through the async proxy
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive_cluster(mapa_shared_cluster(smem_u32(&ctrl->a_ready[aslot]), 0));
-                    if (half) mbar_arrive(smem_u32(&ctrl->w_empty[wslot]));
-                }
-                if (++aslot == kOpSlots) { aslot = 0; a_phase ^= 1u; }
+            for (int w = 0; w < 16; ++w) {
+                const uint4& vw = v[w >> 2];
+                uint32_t q[4];
+                dequant_word((w & 3) == 0 ? vw.x : (w & 3) == 1 ? vw.y : (w & 3) == 2 ? vw.z : vw.w, q);  // (k0,k4) (k1,k5) (k2,k6) (k3,k7)
+                uint4 o;
+                o.x = prmt(q[0], q[1], 0x5410u);  // (k0,k1)
+                o.y = prmt(q[2], q[3], 0x5410u);  // (k2,k3)
+                o.z = prmt(q[0], q[1], 0x7632u);  // (k4,k5)
+                o.w = prmt(q[2], q[3], 0x7632u);  // (k6,k7)
+                sts128(adst + (w >> 3) * kAHalfBytes + ((static_cast<uint32_t>(w & 7) ^ a_sw) << 4), o);
             }
+            fence_proxy_async_smem();  // the tensor core reads this tile through the async proxy
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive_cluster(mapa_shared_cluster(smem_u32(&ctrl->op_full[aslot]), 0));
+                mbar_arrive(smem_u32(&ctrl->w_empty[wslot]));
+            }
+            if (++aslot == op_slots) { aslot = 0; a_phase ^= 1u; }
             if (++wslot == w_slots) { wslot = 0; w_phase ^= 1u; }
         }
     } else {
@@ -456,10 +444,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
                     q_cur = q_next;
                     q_next = load_scales(sp, group + 9, p.groups);
                 }
-                const uint32_t buf = static_cast<uint32_t>(i & 1);
-                if (dead || !mbar_wait_parked(smem_u32(&ctrl->d_full[buf]), (i >> 1) & 1u, ws)) { dead = true; continue; }
+                const uint32_t buf = static_cast<uint32_t>(i & (d_bufs - 1));
+                if (dead || !mbar_wait_parked(smem_u32(&ctrl->d_full[buf]), (i >> d_shift) & 1u, ws)) { dead = true; continue; }
                 tc_fence_after_sync();
-                const uint32_t src = d_addr + buf * 256;
+                const uint32_t src = d_addr + buf * d_cols;
                 // 32 columns a read (one tcgen05.ld; with two of 16 the whole kernel is 20 % slower at M = 512).  A tile of
                 // fewer columns reads on into columns that are allocated and not used.
 #pragma unroll
@@ -539,10 +527,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
                             }
                         } else {
                             // Gate and up of one feature sit in different warps, which trade halves of the 16 columns: the
-                            // gate thread finishes columns 0-7, the up thread 8-15.  Two buffers, one barrier a chunk.
-                            float* buf = park + (c & 1) * (kGemmParkBytes / 8);
-                            float* mine = buf + (ch * 128 + r) * kGemmParkPitch;
-                            const float* theirs = buf + (ch * 128 + (r ^ 64)) * kGemmParkPitch;
+                            // gate thread finishes columns 0-7, the up thread 8-15.
+                            float* mine = park + tid * kGemmParkPitch;
+                            const float* theirs = park + (tid ^ 64) * kGemmParkPitch;
 #pragma unroll
                             for (int j = 0; j < 8; ++j) mine[j] = up_row ? acc[c * 16 + j] : acc[c * 16 + 8 + j];
                             fold_barrier();
@@ -554,6 +541,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
                                     if (mc + j + (up_row ? 8 : 0) < p.m) store_out(out, (g / (1.0f + expf(-g))) * u);
                                 }
                             }
+                            fold_barrier();
                         }
                     }
                 }
@@ -608,7 +596,7 @@ bool encode_gemm_w(CUtensorMap* map, const uint8_t* w, long long n, long long k,
 bool encode_gemm_x(CUtensorMap* map, const __half* x, long long m, long long k, int tile_m) {
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(m)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k) * 2};
-    const cuuint32_t box[2] = {kGemmStageK, static_cast<cuuint32_t>(tile_m / 2)};
+    const cuuint32_t box[2] = {kSwizzleK, static_cast<cuuint32_t>(tile_m / 2)};
     const cuuint32_t estr[2] = {1, 1};
     return gemm_encode_fn() &&
            gemm_encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(x), dims, strides, box, estr,
