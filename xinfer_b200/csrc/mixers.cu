@@ -71,35 +71,55 @@ __device__ __forceinline__ float block_sum(float v, float* smem) {
     return t;
 }
 
-// ------------------------------------------------------------------------------- embedding
-__global__ void embed_kernel(__half* out, const uint16_t* table_bf16, const long long* tokens, int hidden, long long vocab) {
-    griddep_prologue();
-    const int row = blockIdx.x;
-    const long long tok = tokens[row];
-    const bool ok = tok >= 0 && (vocab <= 0 || tok < vocab);
-    for (int d = threadIdx.x; d < hidden; d += blockDim.x) {
-        float v = 0.f;
-        if (ok) v = __uint_as_float(static_cast<uint32_t>(table_bf16[tok * hidden + d]) << 16);
-        out[static_cast<long long>(row) * hidden + d] = __float2half_rn(v);
-    }
-}
-
 // ------------------------------------------------------------------------------- RMSNorm family
-// mode 0: out = rmsnorm(in) * w
-// mode 1: x = half(float(x) + float(delta)); out = rmsnorm(x) * w   (residual add, then norm)
+// out = rmsnorm(x) * w, where x is read
+//   from `x`                                                  (plain)
+//   as half(x + delta), also written back to x                (residual add, then norm)
+//   from row `tokens[row]` of the bf16 table, also written to x when x is given   (embedding, then norm)
 // `out` may have a wider row (ld_out) and a column offset so that two norms can fill one concatenated row.
-__global__ void __launch_bounds__(256) rmsnorm_kernel(__half* out, long long ld_out, __half* x, const __half* delta,
-                                                      const float* w, int hidden, float eps, int perm_out) {
+// One or two such jobs per launch (blockIdx.y).  Bound by latency at a step's 1 to 32 rows (2.6 us a launch): what counts
+// is the number of launches and of dependent trips to memory.  An embedding of its own, 2 bytes per load, took 10 us.
+struct NormJob {
+    __half* out;
+    __half* x;
+    const __half* delta;
+    const float* w;
+    const uint16_t* table;    // embedding rows (bf16), or null
+    const long long* tokens;  // one per row
+    long long vocab;          // tokens outside [0, vocab) read as zeros
+    long long* token_copy;    // tokens[row] also goes to token_copy[row * token_ld], if given
+    int token_ld;
+    const int* pos_in;        // pos_out[row] = pos_in[row] + pos_add, if given
+    int* pos_out;
+    int pos_add;
+};
+
+// The table row of a job's token (null: none, or no table); the first thread keeps the job's books.
+__device__ __forceinline__ const uint16_t* norm_tokens(const NormJob& job, long long row, int hidden) {
+    if (!job.table) return nullptr;
+    const long long tok = job.tokens[row];
+    if (threadIdx.x == 0) {
+        if (job.token_copy) job.token_copy[row * job.token_ld] = tok;
+        if (job.pos_out) job.pos_out[row] = job.pos_in[row] + job.pos_add;
+    }
+    return (tok >= 0 && (job.vocab <= 0 || tok < job.vocab)) ? job.table + tok * hidden : nullptr;
+}
+__device__ __forceinline__ __half bf16_to_half(uint32_t bits) { return __float2half_rn(__uint_as_float(bits << 16)); }
+
+__global__ void __launch_bounds__(256) rmsnorm_kernel(const __grid_constant__ NormJob job0, const __grid_constant__ NormJob job1,
+                                                      long long ld_out, int hidden, float eps, int perm_out) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ float red[32];
+    const NormJob& job = blockIdx.y ? job1 : job0;
+    const float* w = job.w;
     const long long row = blockIdx.x;
-    __half* xr = x + row * hidden;
-    const __half* dr = delta ? delta + row * hidden : nullptr;
-    __half* orow = out + row * ld_out;
+    __half* xr = job.x ? job.x + row * hidden : nullptr;
+    const __half* dr = job.delta ? job.delta + row * hidden : nullptr;
+    __half* orow = job.out + row * ld_out;
     const int nvec = hidden >> 3;
-    const bool vec_ok = (hidden & 7) == 0 && nvec <= 4 * 256 && ((reinterpret_cast<uintptr_t>(xr) & 15) == 0) &&
-                        ((reinterpret_cast<uintptr_t>(orow) & 15) == 0) &&
-                        (!dr || (reinterpret_cast<uintptr_t>(dr) & 15) == 0);
+    const bool vec_ok = (hidden & 7) == 0 && nvec <= 4 * 256 &&
+                        ((reinterpret_cast<uintptr_t>(xr) | reinterpret_cast<uintptr_t>(orow) | reinterpret_cast<uintptr_t>(dr) |
+                          reinterpret_cast<uintptr_t>(job.table) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
     if (vec_ok) {
         // The norm weights do not depend on the previous kernel in the stream: they are fetched before waiting
         // for it, so that only the activations' latency is left on the critical path.
@@ -113,6 +133,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(__half* out, long long ld_
             }
         }
         asm volatile("griddepcontrol.wait;" ::: "memory");
+        const uint16_t* tr = norm_tokens(job, row, hidden);
         // one pass: each thread keeps its (up to four) 8-element vectors in registers
         uint4 v[4];
         float ss = 0.f;
@@ -120,8 +141,21 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(__half* out, long long ld_
         for (int it = 0; it < 4; ++it) {
             const int i = threadIdx.x + it * 256;
             if (i < nvec) {
-                v[it] = *reinterpret_cast<const uint4*>(xr + i * 8);
+                if (!job.table) v[it] = *reinterpret_cast<const uint4*>(xr + i * 8);
+                else v[it] = tr ? __ldg(reinterpret_cast<const uint4*>(tr + i * 8)) : make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+            const int i = threadIdx.x + it * 256;
+            if (i < nvec) {
                 __half2* h = reinterpret_cast<__half2*>(&v[it]);
+                if (job.table) {
+                    const uint32_t e[4] = {v[it].x, v[it].y, v[it].z, v[it].w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) h[j] = __halves2half2(bf16_to_half(e[j] & 0xFFFFu), bf16_to_half(e[j] >> 16));
+                    if (xr) *reinterpret_cast<uint4*>(xr + i * 8) = v[it];
+                }
                 if (dr) {
                     const uint4 dv = *reinterpret_cast<const uint4*>(dr + i * 8);
                     const __half2* dh = reinterpret_cast<const __half2*>(&dv);
@@ -161,20 +195,20 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(__half* out, long long ld_
         return;
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint16_t* tr = norm_tokens(job, row, hidden);
+    auto element = [&](int i) { return job.table ? (tr ? bf16_to_half(tr[i]) : __float2half_rn(0.f)) : xr[i]; };
     float ss = 0.f;
     for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
-        float v = __half2float(xr[i]);
-        if (dr) {
-            const __half s = __float2half_rn(v + __half2float(dr[i]));
-            xr[i] = s;
-            v = __half2float(s);
-        }
+        __half e = element(i);
+        if (dr) e = __float2half_rn(__half2float(e) + __half2float(dr[i]));
+        if (xr && (dr || job.table)) xr[i] = e;
+        const float v = __half2float(e);
         ss += v * v;
     }
     const float total = block_sum(ss, red);
     const float r = 1.0f / sqrtf(total / static_cast<float>(hidden) + eps);
     for (int i = threadIdx.x; i < hidden; i += blockDim.x)
-        orow[(perm_out && (hidden & 7) == 0) ? perm8(i) : i] = __float2half_rn(__half2float(xr[i]) * r * w[i]);
+        orow[(perm_out && (hidden & 7) == 0) ? perm8(i) : i] = __float2half_rn(__half2float(xr ? xr[i] : element(i)) * r * w[i]);
 }
 
 // ------------------------------------------------------------------------------- attention prologue
@@ -257,22 +291,27 @@ __global__ void conv1d_spec_kernel(__half* out, const __half* in, const float* c
     if (c >= channels) return;
     float* st = state + static_cast<long long>(b) * 3 * channels;
     float* pd = pending + static_cast<long long>(b) * 8 * channels;
-    float s0 = st[c], s1 = st[channels + c], s2 = st[2 * channels + c];
     int nc = n_commit ? n_commit[b] : nc_base;
     if (nc > prev_rows) nc = prev_rows;
-    for (int i = 0; i < nc; ++i) {  // replay the accepted inputs of the previous step
-        s0 = s1;
-        s1 = s2;
-        s2 = pd[i * channels + c];
-    }
+    // the last three inputs, with the accepted ones of the previous step behind the committed ones
+    float s0 = nc < 3 ? st[nc * channels + c] : pd[(nc - 3) * channels + c];
+    float s1 = nc < 2 ? st[(nc + 1) * channels + c] : pd[(nc - 2) * channels + c];
+    float s2 = nc < 1 ? st[2 * channels + c] : pd[(nc - 1) * channels + c];
     st[c] = s0;
     st[channels + c] = s1;
     st[2 * channels + c] = s2;
     const float w0 = conv_w[c * 4], w1 = conv_w[c * 4 + 1], w2 = conv_w[c * 4 + 2], w3 = conv_w[c * 4 + 3];
     if (early_state) asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int i = 0; i < rows_per_seq; ++i) {
+    // all rows (eight at most) are requested before the first is used: one trip to memory instead of one per row
+    __half xs[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        if (i < rows_per_seq) xs[i] = in[(static_cast<long long>(b) * rows_per_seq + i) * channels + c];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        if (i >= rows_per_seq) break;
         const long long row = static_cast<long long>(b) * rows_per_seq + i;
-        const float x = __half2float(in[row * channels + c]);
+        const float x = __half2float(xs[i]);
         const float sum = w0 * s0 + w1 * s1 + w2 * s2 + w3 * x;
         out[row * channels + c] = __float2half_rn(sum / (1.0f + expf(-sum)));
         pd[i * channels + c] = x;
@@ -1182,31 +1221,60 @@ __global__ void fill_int_kernel(int* p, int n, int v) {
     if (i < n) p[i] = v;
 }
 
-__global__ void copy_token_column_kernel(long long* draft, const long long* argmax_out, int k, int col) {
-    griddep_prologue();
-    const int b = threadIdx.x + blockIdx.x * blockDim.x;
-    draft[b * k + col] = argmax_out[b];
-}
-
 }  // namespace
 
 #define XB_LAUNCH_OK() (cudaGetLastError() == cudaSuccess ? 0 : -1)
 
-int embed_rows(cudaStream_t s, __half* out, const void* table_bf16, const long long* tokens, int rows, int hidden,
-               long long vocab) {
-    launch_pdl(embed_kernel, dim3(rows), dim3(256), 0, s, out, static_cast<const uint16_t*>(table_bf16), tokens, hidden, vocab);
+int embed_norm_rows(cudaStream_t s, __half* out, __half* x, const void* table_bf16, const long long* tokens, const float* w, int rows,
+                    int hidden, long long vocab, float eps, int perm_out) {
+    NormJob j = {};
+    j.out = out;
+    j.x = x;
+    j.w = w;
+    j.table = static_cast<const uint16_t*>(table_bf16);
+    j.tokens = tokens;
+    j.vocab = vocab;
+    launch_pdl(rmsnorm_kernel, dim3(rows), dim3(256), 0, s, j, j, static_cast<long long>(hidden), hidden, eps, perm_out);
+    return XB_LAUNCH_OK();
+}
+
+int head_input_rows(cudaStream_t s, const HeadInput& h, int rows, int hidden, float eps, int perm_out) {
+    NormJob e = {}, p = {};
+    e.out = h.cat;
+    e.w = h.embed_norm;
+    e.table = static_cast<const uint16_t*>(h.table_bf16);
+    e.tokens = h.tokens;
+    e.vocab = h.vocab;
+    e.token_copy = h.token_copy;
+    e.token_ld = h.token_ld;
+    e.pos_in = h.pos_in;
+    e.pos_out = h.pos_out;
+    e.pos_add = h.pos_add;
+    p.out = h.cat + hidden;
+    p.x = const_cast<__half*>(h.hidden_rows);
+    p.w = h.hidden_norm;
+    launch_pdl(rmsnorm_kernel, dim3(rows, 2), dim3(256), 0, s, e, p, 2LL * hidden, hidden, eps, perm_out);
     return XB_LAUNCH_OK();
 }
 
 int rmsnorm_rows(cudaStream_t s, __half* out, long long ld_out, const __half* in, const float* w, int rows, int hidden,
                  float eps, int perm_out) {
-    launch_pdl(rmsnorm_kernel, dim3(rows), dim3(256), 0, s, out, ld_out, const_cast<__half*>(in), nullptr, w, hidden, eps, perm_out);
+    NormJob j = {};
+    j.out = out;
+    j.x = const_cast<__half*>(in);
+    j.w = w;
+    launch_pdl(rmsnorm_kernel, dim3(rows), dim3(256), 0, s, j, j, ld_out, hidden, eps, perm_out);
     return XB_LAUNCH_OK();
 }
 
 int add_rmsnorm_rows(cudaStream_t s, __half* out, __half* x, const __half* delta, const float* w, int rows, int hidden,
                      float eps, int perm_out) {
-    launch_pdl(rmsnorm_kernel, dim3(rows), dim3(256), 0, s, out, hidden, x, delta, w, hidden, eps, perm_out);
+    NormJob j = {};
+    j.out = out;
+    j.x = x;
+    j.delta = delta;
+    j.w = w;
+    launch_pdl(rmsnorm_kernel, dim3(rows), dim3(256), 0, s, j, j, static_cast<long long>(hidden), hidden, eps, perm_out);
     return XB_LAUNCH_OK();
 }
 
@@ -1299,11 +1367,6 @@ int build_verify_tokens(cudaStream_t s, long long* out, const long long* cur_tok
 
 int fill_int(cudaStream_t s, int* p, int n, int v) {
     launch_pdl(fill_int_kernel, dim3((n + 127) / 128), dim3(128), 0, s, p, n, v);
-    return XB_LAUNCH_OK();
-}
-
-int copy_token_column(cudaStream_t s, long long* draft, const long long* argmax_out, int batch, int k, int col) {
-    launch_pdl(copy_token_column_kernel, dim3(1), dim3(batch), 0, s, draft, argmax_out, k, col);
     return XB_LAUNCH_OK();
 }
 

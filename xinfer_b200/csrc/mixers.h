@@ -8,13 +8,30 @@
 
 namespace xb {
 
-int embed_rows(cudaStream_t s, __half* out, const void* table_bf16, const long long* tokens, int rows, int hidden,
-               long long vocab);
 // perm_out (here and below): write the output with every block of eight features in the order the int4 unpack of
 // the W4A16 kernel yields them, (0,4,1,5,2,6,3,7): such a buffer is only good as the X of a projection launched
 // with kTcXPermuted (w4a16.h).
 int rmsnorm_rows(cudaStream_t s, __half* out, long long ld_out, const __half* in, const float* w, int rows, int hidden,
                  float eps, int perm_out = 0);
+// x = embedding rows (bf16 table) of the tokens, out = rmsnorm(x) * w
+int embed_norm_rows(cudaStream_t s, __half* out, __half* x, const void* table_bf16, const long long* tokens, const float* w, int rows,
+                    int hidden, long long vocab, float eps, int perm_out = 0);
+// cat[row] = [rmsnorm(embedding of tokens[row]) * embed_norm ; rmsnorm(hidden_rows[row]) * hidden_norm], and on the way
+// token_copy[row * token_ld] = tokens[row] and pos_out[row] = pos_in[row] + pos_add (each if its target is given)
+struct HeadInput {
+    __half* cat = nullptr;  // [rows][2 hidden]
+    const void* table_bf16 = nullptr;
+    const long long* tokens = nullptr;
+    long long vocab = 0;
+    const float *embed_norm = nullptr, *hidden_norm = nullptr;
+    const __half* hidden_rows = nullptr;
+    long long* token_copy = nullptr;
+    int token_ld = 1;
+    const int* pos_in = nullptr;
+    int* pos_out = nullptr;
+    int pos_add = 0;
+};
+int head_input_rows(cudaStream_t s, const HeadInput& h, int rows, int hidden, float eps, int perm_out = 0);
 // x = half(x + delta) in place, out = rmsnorm(x) * w
 int add_rmsnorm_rows(cudaStream_t s, __half* out, __half* x, const __half* delta, const float* w, int rows, int hidden,
                      float eps, int perm_out = 0);
@@ -80,6 +97,5 @@ int spec_commit(cudaStream_t s, const void* accept_records, const long long* dra
 int build_verify_tokens(cudaStream_t s, long long* out, const long long* cur_tok, const long long* draft, int batch,
                         int k);
 int fill_int(cudaStream_t s, int* p, int n, int v);
-int copy_token_column(cudaStream_t s, long long* draft, const long long* argmax_out, int batch, int k, int col);
 
 }  // namespace xb

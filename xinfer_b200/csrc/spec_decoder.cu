@@ -74,10 +74,6 @@ __global__ void init_tokens_kernel(long long* p, int n, uint64_t seed, long long
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) p[i] = static_cast<long long>(mix32(seed * 0x9E3779B97F4A7C15ULL + i)) % vocab;
 }
-__global__ void add_int_kernel(int* out, const int* in, int n, int v) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = in[i] + v;
-}
 __global__ void last_prompt_token_kernel(long long* cur_tok, const long long* prompt, int batch, long long T) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < batch) cur_tok[b] = prompt[static_cast<long long>(b) * T + T - 1];
@@ -159,7 +155,7 @@ struct xinfer_spec_decoder {
     __half *h_last = nullptr, *mtp_hidden = nullptr;
     xinfer_accept_record* records = nullptr;
     // activations (rows up to batch * (k + 1)); XBufs are written by other ranks under tensor parallelism
-    __half *x = nullptr, *emb = nullptr, *normed = nullptr, *qbuf = nullptr, *qkv_conv = nullptr, *bbuf = nullptr,
+    __half *x = nullptr, *normed = nullptr, *qbuf = nullptr, *qkv_conv = nullptr, *bbuf = nullptr,
            *abuf = nullptr, *cat = nullptr;
     XBuf x_mtp, proj_out, mlp, q_gate, kbuf, vbuf, attn_out, qkv_raw, zbuf, delta_out, partials;
     float *logits = nullptr, *attn_scratch = nullptr;
@@ -346,7 +342,6 @@ void build_all(Dec* d) {
     d->nucleus = dalloc<xb::Nucleus>(d, static_cast<size_t>(M), true);
     const int64_t hv = c.linear_num_v_heads, hk = c.linear_num_k_heads, ch = 2 * hk * 128 + hv * 128;
     d->x = dalloc<__half>(d, static_cast<size_t>(M) * H, true);
-    d->emb = dalloc<__half>(d, static_cast<size_t>(batch) * H, true);
     d->normed = dalloc<__half>(d, static_cast<size_t>(M) * H, true);
     d->qbuf = dalloc<__half>(d, static_cast<size_t>(M) * c.num_attention_heads * 256, true);
     d->qkv_conv = dalloc<__half>(d, static_cast<size_t>(M) * ch, true);
@@ -586,14 +581,25 @@ int draft_pass(Dec* d, cudaStream_t s, int i, bool full) {
     const auto& c = d->cfg;
     const int B = d->batch, H = static_cast<int>(c.hidden_size);
     const long long* tok = (i == 0) ? d->cur_tok : d->argmax_out;
-    const __half* hprev = (i == 0) ? d->h_last : d->mtp_hidden;
+    const __half* hprev = (i == 0) ? d->h_last : d->world > 1 ? d->mtp_hidden : d->x_mtp.p;
     // cat = [rmsnorm(embed(tok)) ; rmsnorm(h_prev)]  ->  fc  ->  x
-    NL(xb::embed_rows(s, d->emb, d->embed, tok, B, H, c.vocab_size));
-    NL(xb::rmsnorm_rows(s, d->cat, 2 * H, d->emb, d->mtp_enorm, B, H, c.rms_norm_eps, xperm_on()));
-    NL(xb::rmsnorm_rows(s, d->cat + H, 2 * H, hprev, d->mtp_hnorm, B, H, c.rms_norm_eps, xperm_on()));
+    // (the same launch takes down the token, which the previous pass drew, as that pass's draft, and this pass's positions)
+    xb::HeadInput hi;
+    hi.cat = d->cat;
+    hi.table_bf16 = d->embed;
+    hi.tokens = tok;
+    hi.vocab = c.vocab_size;
+    hi.embed_norm = d->mtp_enorm;
+    hi.hidden_norm = d->mtp_hnorm;
+    hi.hidden_rows = hprev;
+    if (i > 0) hi.token_copy = d->draft + (i - 1);
+    hi.token_ld = d->k;
+    hi.pos_in = d->ctx;
+    hi.pos_out = d->ctx_draft;
+    hi.pos_add = i;
+    NL(xb::head_input_rows(s, hi, B, H, c.rms_norm_eps, xperm_on()));
     CK(lin(d, s, d->x_mtp, d->cat, d->mtp_fc, B, kAll));
-    if (!d->linears_only) add_int_kernel<<<1, 64, 0, s>>>(d->ctx_draft, d->ctx, B, i);
-    d->launches_per_step += 4;
+    d->launches_per_step += 1;
     if (!full) {
         // input norm -> k, v projections of the head's layer -> head norm, RoPE, cache write
         Layer& L = d->mtp_layer;
@@ -615,8 +621,9 @@ int draft_pass(Dec* d, cudaStream_t s, int i, bool full) {
     NL(xb::rmsnorm_rows(s, d->normed, H, d->x_mtp.p, d->mtp_layer.input_norm, B, H, c.rms_norm_eps, xperm_on()));
     ++d->launches_per_step;
     CK(layer_forward(d, s, d->mtp_layer, 1, d->x_mtp.p, d->final_norm, d->ctx_draft, d->n_commit_zero, 0));
-    // keep the head's output hidden (pre final norm) for the next draft pass
-    if (!d->linears_only)
+    // the head's output hidden (pre final norm) is the next draft pass's; another rank may already be writing that pass's
+    // x_mtp here while this one still reads, so with several ranks it is set aside
+    if (!d->linears_only && d->world > 1)
         CKCUDA(cudaMemcpyAsync(d->mtp_hidden, d->x_mtp.p, static_cast<size_t>(B) * H * sizeof(__half), cudaMemcpyDeviceToDevice, s));
     CK(lm_head_and_partials(d, s, B));
     if (d->temperature > 0.f) {
@@ -631,17 +638,15 @@ int draft_pass(Dec* d, cudaStream_t s, int i, bool full) {
         NL(xb::argmax_finish(s, d->partials.p, xb::sampling_chunks(d->vocab_local), d->world, partial_slice_stride(d, B), B,
                              d->argmax_out));
     }
-    NL(xb::copy_token_column(s, d->draft, d->argmax_out, B, d->k, i));
-    d->launches_per_step += 4;
+    d->launches_per_step += 1;
     return 0;
 }
 
 int target_pass(Dec* d, cudaStream_t s, int R, const long long* tokens) {
     const auto& c = d->cfg;
     const int M = d->batch * R, H = static_cast<int>(c.hidden_size);
-    NL(xb::embed_rows(s, d->x, d->embed, tokens, M, H, c.vocab_size));
-    NL(xb::rmsnorm_rows(s, d->normed, H, d->x, d->layers[0].input_norm, M, H, c.rms_norm_eps, xperm_on()));
-    d->launches_per_step += 2;
+    NL(xb::embed_norm_rows(s, d->normed, d->x, d->embed, tokens, d->layers[0].input_norm, M, H, c.vocab_size, c.rms_norm_eps, xperm_on()));
+    d->launches_per_step += 1;
     const size_t nl = d->layers.size();
     for (size_t l = 0; l < nl; ++l)
         CK(layer_forward(d, s, d->layers[l], R, d->x, l + 1 < nl ? d->layers[l + 1].input_norm : d->final_norm, d->ctx,
@@ -727,8 +732,7 @@ int prefill_chunk(Dec* d, cudaStream_t s, const long long* prompt, int64_t T, in
         return f;
     };
     gather_prompt_chunk_kernel<<<blocks_for(static_cast<size_t>(M), 128), 128, 0, s>>>(cb.tokens, prompt, B, T, c0, Rc);
-    NL(xb::embed_rows(s, cb.x, d->embed, cb.tokens, M, H, c.vocab_size));
-    NL(xb::rmsnorm_rows(s, cb.normed, H, cb.x, d->layers[0].input_norm, M, H, eps, 0));
+    NL(xb::embed_norm_rows(s, cb.normed, cb.x, d->embed, cb.tokens, d->layers[0].input_norm, M, H, c.vocab_size, eps));
     const size_t nl = d->layers.size();
     for (size_t l = 0; l < nl; ++l) {
         Layer& L = d->layers[l];
@@ -773,9 +777,15 @@ int prefill_chunk(Dec* d, cudaStream_t s, const long long* prompt, int64_t T, in
     Layer& ML = d->mtp_layer;
     const size_t nH = static_cast<size_t>(M) * H;
     shift_hidden_chunk_kernel<<<blocks_for(nH, 256), 256, 0, s>>>(cb.hprev, d->h_last, cb.x, B, Rc, H);
-    NL(xb::embed_rows(s, cb.proj_out, d->embed, cb.tokens, M, H, c.vocab_size));
-    NL(xb::rmsnorm_rows(s, cb.cat, 2 * H, cb.proj_out, d->mtp_enorm, M, H, eps, 0));
-    NL(xb::rmsnorm_rows(s, cb.cat + H, 2 * H, cb.hprev, d->mtp_hnorm, M, H, eps, 0));
+    xb::HeadInput hi;
+    hi.cat = cb.cat;
+    hi.table_bf16 = d->embed;
+    hi.tokens = cb.tokens;
+    hi.vocab = c.vocab_size;
+    hi.embed_norm = d->mtp_enorm;
+    hi.hidden_norm = d->mtp_hnorm;
+    hi.hidden_rows = cb.hprev;
+    NL(xb::head_input_rows(s, hi, M, H, eps));
     LIN(xinfer_linear_int4_f16f16(st, cb.mix_out, cb.cat, d->mtp_fc.w, d->mtp_fc.s, nullptr, M, d->mtp_fc.n, d->mtp_fc.k, 128));
     NL(xb::rmsnorm_rows(s, cb.normed, H, cb.mix_out, ML.input_norm, M, H, eps, 0));
     const xinfer_fused_desc kv[2] = {desc(cb.kbuf, ML.k_proj), desc(cb.vbuf, ML.v_proj)};
