@@ -96,7 +96,6 @@ struct NormJob {
 
 // The table row of a job's token (null: none, or no table); the first thread keeps the job's books.
 __device__ __forceinline__ const uint16_t* norm_tokens(const NormJob& job, long long row, int hidden) {
-    if (!job.table) return nullptr;
     const long long tok = job.tokens[row];
     if (threadIdx.x == 0) {
         if (job.token_copy) job.token_copy[row * job.token_ld] = tok;
@@ -106,11 +105,14 @@ __device__ __forceinline__ const uint16_t* norm_tokens(const NormJob& job, long 
 }
 __device__ __forceinline__ __half bf16_to_half(uint32_t bits) { return __float2half_rn(__uint_as_float(bits << 16)); }
 
+// TABLE: some job of the launch reads the embedding table
+template <bool TABLE>
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const __grid_constant__ NormJob job0, const __grid_constant__ NormJob job1,
                                                       long long ld_out, int hidden, float eps, int perm_out) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    __shared__ float red[32];
-    const NormJob& job = blockIdx.y ? job1 : job0;
+    __shared__ __align__(16) float red[32];
+    const NormJob& job = TABLE && blockIdx.y ? job1 : job0;
+    const bool table = TABLE && job.table;
     const float* w = job.w;
     const long long row = blockIdx.x;
     __half* xr = job.x ? job.x + row * hidden : nullptr;
@@ -133,52 +135,57 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __grid_constant__ No
             }
         }
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        const uint16_t* tr = norm_tokens(job, row, hidden);
-        // one pass: each thread keeps its (up to four) 8-element vectors in registers
-        uint4 v[4];
+        const uint16_t* tr = table ? norm_tokens(job, row, hidden) : nullptr;
+        // one pass: each thread keeps its (up to four) 8-element vectors in registers.  Every load goes out before the first
+        // value is used and before any store (which the compiler must take for a possible alias of the later loads): with
+        // the residual stored in between, each further vector was another trip to memory (2.9 us a launch against 2.5).
+        uint4 v[4], dv[4];
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+            const int i = threadIdx.x + it * 256;
+            if (i < nvec) {
+                if (!table) v[it] = *reinterpret_cast<const uint4*>(xr + i * 8);
+                else v[it] = tr ? __ldg(reinterpret_cast<const uint4*>(tr + i * 8)) : make_uint4(0u, 0u, 0u, 0u);
+                if (dr) dv[it] = *reinterpret_cast<const uint4*>(dr + i * 8);
+            }
+        }
         float ss = 0.f;
 #pragma unroll
         for (int it = 0; it < 4; ++it) {
             const int i = threadIdx.x + it * 256;
             if (i < nvec) {
-                if (!job.table) v[it] = *reinterpret_cast<const uint4*>(xr + i * 8);
-                else v[it] = tr ? __ldg(reinterpret_cast<const uint4*>(tr + i * 8)) : make_uint4(0u, 0u, 0u, 0u);
-            }
-        }
-#pragma unroll
-        for (int it = 0; it < 4; ++it) {
-            const int i = threadIdx.x + it * 256;
-            if (i < nvec) {
                 __half2* h = reinterpret_cast<__half2*>(&v[it]);
-                if (job.table) {
+                if (table) {
                     const uint32_t e[4] = {v[it].x, v[it].y, v[it].z, v[it].w};
 #pragma unroll
                     for (int j = 0; j < 4; ++j) h[j] = __halves2half2(bf16_to_half(e[j] & 0xFFFFu), bf16_to_half(e[j] >> 16));
-                    if (xr) *reinterpret_cast<uint4*>(xr + i * 8) = v[it];
                 }
                 if (dr) {
-                    const uint4 dv = *reinterpret_cast<const uint4*>(dr + i * 8);
-                    const __half2* dh = reinterpret_cast<const __half2*>(&dv);
+                    const __half2* dh = reinterpret_cast<const __half2*>(&dv[it]);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const float2 a = __half22float2(h[j]), b = __half22float2(dh[j]);
                         h[j] = __halves2half2(__float2half_rn(a.x + b.x), __float2half_rn(a.y + b.y));
                     }
-                    *reinterpret_cast<uint4*>(xr + i * 8) = v[it];
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float2 a = __half22float2(h[j]);
-                    ss += a.x * a.x + a.y * a.y;
+                    ss = fmaf(a.y, a.y, fmaf(a.x, a.x, ss));
                 }
             }
         }
-        const float total = block_sum(ss, red);
+        ss = warp_sum(ss);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+        __syncthreads();
+        const float4 r0 = *reinterpret_cast<const float4*>(red), r1 = *reinterpret_cast<const float4*>(red + 4);
+        const float total = ((r0.x + r1.x) + (r0.z + r1.z)) + ((r0.y + r1.y) + (r0.w + r1.w));
         const float r = 1.0f / sqrtf(total / static_cast<float>(hidden) + eps);
 #pragma unroll
         for (int it = 0; it < 4; ++it) {
             const int i = threadIdx.x + it * 256;
             if (i < nvec) {
+                if (xr && (dr || table)) *reinterpret_cast<uint4*>(xr + i * 8) = v[it];
                 const __half2* h = reinterpret_cast<const __half2*>(&v[it]);
                 const float4 w0 = wv[it][0], w1 = wv[it][1];
                 const float ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
@@ -195,13 +202,13 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __grid_constant__ No
         return;
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const uint16_t* tr = norm_tokens(job, row, hidden);
-    auto element = [&](int i) { return job.table ? (tr ? bf16_to_half(tr[i]) : __float2half_rn(0.f)) : xr[i]; };
+    const uint16_t* tr = table ? norm_tokens(job, row, hidden) : nullptr;
+    auto element = [&](int i) { return table ? (tr ? bf16_to_half(tr[i]) : __float2half_rn(0.f)) : xr[i]; };
     float ss = 0.f;
     for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
         __half e = element(i);
         if (dr) e = __float2half_rn(__half2float(e) + __half2float(dr[i]));
-        if (xr && (dr || job.table)) xr[i] = e;
+        if (xr && (dr || table)) xr[i] = e;
         const float v = __half2float(e);
         ss += v * v;
     }
@@ -321,155 +328,243 @@ __global__ void conv1d_spec_kernel(__half* out, const __half* in, const float* c
     }
 }
 
+// ------------------------------------------------------------------------------- two fp32 operations per instruction
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float sum_f32x2(uint64_t a) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));
+    return lo + hi;
+}
+
 // ------------------------------------------------------------------------------- Gated DeltaNet recurrence
-// Grid (v heads, B), 512 threads: thread (part, j) keeps rows [32 part, 32 part + 32) of column j of the
-// 128 x 128 fp32 state in registers.  Everything that does not depend on the state (q/k L2 norms, beta, the
-// decay factor) is computed for all tokens at once before the recurrence, and the gated RMSNorm of the
-// outputs for all tokens after it, so the sequential part is one barrier and 64 FMAs per token.
-// pend_k [B][Hv][8][128] normalised keys, pend_d [B][Hv][8][128] deltas, pend_g [B][Hv][8] decay factors of
-// the previous step: replaying them touches each state element with the same two operations, in the same
-// order, as the step that produced them, so the committed state is bit-identical.
-__global__ void __launch_bounds__(512, 2) gdn_spec_kernel(__half* out, const __half* qkv, const __half* z,
-                                                          const __half* bb, const __half* aa, const float* A_log,
-                                                          const float* dt_bias, const float* norm_w, float* state,
-                                                          float* pend_k, float* pend_d, float* pend_g,
-                                                          const int* n_commit, int rows_per_seq, int prev_rows, int hv,
-                                                          int hk, int nc_base, int early_state, int perm_out) {
+// One CTA per (v head, sequence).  pend_k [B][Hv][8][128] normalised keys, pend_d [B][Hv][8][128] deltas, pend_g [B][Hv][8]
+// decay factors of the previous step: replaying the accepted ones of them touches each state element with the same two
+// operations in the same order every time, and gives the committed state.
+//
+// The state streams through: element by element it is replayed, written back and multiplied with the keys and queries of
+// all tokens, and the recurrence itself is solved on those products.  With G_t the product of the decay factors up to t,
+//     delta_t = beta_t (v_t - G_t k_t.S - sum_{s<t} (G_t / G_s) (k_t.k_s) delta_s)
+//     out_t   =             G_t q_t.S + sum_{s<=t} (G_t / G_s) (q_t.k_s) delta_s
+// (the factors G_t / G_s are products of the decays in between, never quotients).  Thread (part, j) takes 128 / PARTS rows
+// of column j, BATCH at a time with the next BATCH in flight; TOKENS >= rows_per_seq.
+//
+// A pass is latency with few heads and memory with many (128 KB of state moved per head).  PARTS = 4, BATCH = 32: every
+// load of a head is in flight at once.  PARTS = 2, BATCH = 16: three CTAs per SM, so that 384 heads (48 heads, eight
+// sequences, 50 MB) are one wave.  A kernel that kept the state in registers through the tokens needed 64 registers and
+// 512 threads a head, ran those 384 heads in two waves and paid a barrier per token: 23.3 us against 13.0, and with one
+// sequence of four tokens 11.8 against 6.7.
+constexpr int kGdnTokens = 8;  // rows_per_seq at most, and entries of the pending buffers
+
+// sum of squares of 128 values, lane l holding l, l + 32, l + 64 and l + 96
+__device__ __forceinline__ float warp_sum_sq(const float (&v)[4]) {
+    float s[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s[i] = warp_sum(v[i] * v[i]);
+    return ((s[0] + s[1]) + s[2]) + s[3];
+}
+
+template <int PARTS, int BATCH, int TOKENS>
+__global__ void __launch_bounds__(128 * PARTS, PARTS == 2 ? (TOKENS <= 4 ? 3 : 2) : 1) gdn_spec_kernel(
+    __half* out, const __half* qkv, const __half* z, const __half* bb, const __half* aa, const float* A_log,
+    const float* dt_bias, const float* norm_w, float* state, float* pend_k, float* pend_d, float* pend_g,
+    const int* n_commit, int rows_per_seq, int prev_rows, int hv, int hk, int nc_base, int early_state, int perm_out) {
     // The recurrent state, the previous step's pending updates and the per-head constants were written many
     // launches ago (by this layer's kernel of the previous pass, and by the commit at the end of the previous step):
-    // they are fetched BEFORE waiting for the kernel in front of this one, so that the bulk of this kernel's memory
-    // traffic overlaps the projection and convolution that precede it.  Only q/k/v/z/b/a come from those.
-    // (early_state = 0: the caller's previous launch wrote the state - the stand-alone op entry point chaining
-    // chunks of one sequence - so everything waits.)
+    // they are requested BEFORE waiting for the kernel in front of this one.  Only q/k/v/z/b/a come from it.
+    // (early_state = 0: the caller's previous launch wrote the state - the stand-alone op entry point
+    // chaining chunks of one sequence - so everything waits.)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (!early_state) asm volatile("griddepcontrol.wait;" ::: "memory");
-    __shared__ __align__(16) float sh_q[8][128], sh_k[8][128];
-    __shared__ float sh_beta[8], sh_eg[8], red[2][16];
-    __shared__ float part_sum[2][4][128], attn_all[8][4][128];
+    constexpr int kRows = 128 / PARTS, kThreads = 128 * PARTS, kWarps = 4 * PARTS;
+    static_assert(TOKENS <= kWarps, "a warp per token");
+    __shared__ __align__(16) float sh_q[TOKENS][128], sh_k[TOKENS][128], sh_pk[kGdnTokens][128];
+    __shared__ float sh_v[TOKENS][128], sh_z[TOKENS][128], sh_pd[kGdnTokens][128], sh_pg[kGdnTokens];
+    __shared__ float sums[PARTS][TOKENS][128];
+    __shared__ float sh_nw[128], sh_beta[TOKENS], sh_eg[TOKENS];
+    __shared__ float gram[2][TOKENS][TOKENS];  // k_t.k_s and q_t.k_s
     const int h = blockIdx.x, b = blockIdx.y;
-    const int j = threadIdx.x & 127, part = threadIdx.x >> 7;  // part doubles as the token group in phases 0 and 2
-    const int lane = threadIdx.x & 31, wig = (threadIdx.x >> 5) & 3;
-    const int i0 = part * 32;
+    const int j = threadIdx.x & 127, part = threadIdx.x >> 7;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i0 = part * kRows;
     const int h_k = h / (hv / hk);
     const int channels = 2 * hk * 128 + hv * 128;
     const int value_dim = hv * 128;
-    float* S = state + (static_cast<long long>(b) * hv + h) * (128 * 128);
-    const long long pbase = (static_cast<long long>(b) * hv + h) * 8;
-    float col[32];
+    float* S = state + (static_cast<long long>(b) * hv + h) * (128 * 128) + i0 * 128 + j;
+    const long long pbase = (static_cast<long long>(b) * hv + h) * kGdnTokens;
+
+    float next[BATCH];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) col[i] = S[(i0 + i) * 128 + j];
-    const float exp_a_log = expf(A_log[h]);
-    const float dtb = dt_bias[h];
+    for (int i = 0; i < BATCH; ++i) next[i] = S[i * 128];
     int nc = n_commit ? n_commit[b] : nc_base;
     if (nc > prev_rows) nc = prev_rows;
+    for (int e = threadIdx.x; e < nc * 128; e += kThreads) {
+        sh_pk[0][e] = pend_k[pbase * 128 + e];
+        sh_pd[0][e] = pend_d[pbase * 128 + e];
+    }
+    if (threadIdx.x < nc) sh_pg[threadIdx.x] = pend_g[pbase + threadIdx.x];
+    if (part == 0) sh_nw[j] = norm_w[j];
     if (early_state) asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    // ---- phase 0: per-token quantities that do not depend on the state (token tt handled by thread group tt % 4)
-    for (int t0 = 0; t0 < rows_per_seq; t0 += 4) {
-        const int tt = t0 + part;
-        float raw_q = 0.f, raw_k = 0.f;
-        if (tt < rows_per_seq) {
-            const __half* cur = qkv + (static_cast<long long>(b) * rows_per_seq + tt) * channels;
-            raw_q = __half2float(cur[h_k * 128 + j]);
-            raw_k = __half2float(cur[hk * 128 + h_k * 128 + j]);
-        }
-        const float wq = warp_sum(raw_q * raw_q), wk = warp_sum(raw_k * raw_k);
-        __syncthreads();
-        if (lane == 0) { red[0][part * 4 + wig] = wq; red[1][part * 4 + wig] = wk; }
-        __syncthreads();
-        if (tt < rows_per_seq) {
-            const float q_sq = ((red[0][part * 4] + red[0][part * 4 + 1]) + red[0][part * 4 + 2]) + red[0][part * 4 + 3];
-            const float k_sq = ((red[1][part * 4] + red[1][part * 4 + 1]) + red[1][part * 4 + 2]) + red[1][part * 4 + 3];
-            sh_q[tt][j] = (raw_q * (1.0f / sqrtf(q_sq + 1e-6f))) * 0.08838834764f;
-            sh_k[tt][j] = raw_k * (1.0f / sqrtf(k_sq + 1e-6f));
-            if (j == 0) {
-                const long long row = static_cast<long long>(b) * rows_per_seq + tt;
+    // ---- per-token quantities that do not depend on the state: one warp per token
+    if (warp < TOKENS) {
+        const int t = warp;
+        float q[4] = {}, k[4] = {}, v[4] = {}, zz[4] = {};  // (zeros beyond rows_per_seq)
+        if (t < rows_per_seq) {
+            const long long row = static_cast<long long>(b) * rows_per_seq + t;
+            const __half* cur = qkv + row * channels;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int d = lane + 32 * i;
+                q[i] = __half2float(cur[h_k * 128 + d]);
+                k[i] = __half2float(cur[hk * 128 + h_k * 128 + d]);
+                v[i] = __half2float(cur[2 * hk * 128 + h * 128 + d]);
+                zz[i] = __half2float(z[row * value_dim + h * 128 + d]);
+            }
+            if (lane == 0) {
                 const float b_val = __half2float(bb[row * hv + h]);
-                sh_beta[tt] = 1.0f / (1.0f + expf(-b_val));
-                const float a_val = __half2float(aa[row * hv + h]) + dtb;
+                const float a_val = __half2float(aa[row * hv + h]) + dt_bias[h];
                 const float softplus = (a_val > 20.0f) ? a_val : logf(1.0f + expf(a_val));
-                sh_eg[tt] = expf(-exp_a_log * softplus);
+                sh_beta[t] = 1.0f / (1.0f + expf(-b_val));
+                sh_eg[t] = expf(-expf(A_log[h]) * softplus);
             }
         }
-    }
-
-    // ---- replay of the previous step's accepted updates, then write the committed state
-    if (nc > 0) {
-        for (int t = 0; t < nc; ++t) {
-            const float eg = pend_g[pbase + t];
-            const float dj = pend_d[(pbase + t) * 128 + j];
-            const float* pk = pend_k + (pbase + t) * 128 + i0;
+        const float q_sq = warp_sum_sq(q), k_sq = warp_sum_sq(k);
+        const float rq = 1.0f / sqrtf(q_sq + 1e-6f), rk = 1.0f / sqrtf(k_sq + 1e-6f);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                const float sv = col[i] * eg;
-                col[i] = sv + __ldg(pk + i) * dj;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 32; ++i) S[(i0 + i) * 128 + j] = col[i];
-    }
-    __syncthreads();  // phase 0 results visible; replay reads of pend_* are done before they are overwritten
-
-    // ---- phase 1: the recurrence
-    for (int t = 0; t < rows_per_seq; ++t) {
-        const long long row = static_cast<long long>(b) * rows_per_seq + t;
-        const float v = __half2float(qkv[row * channels + 2 * hk * 128 + h * 128 + j]);
-        const float eg = sh_eg[t];
-        float kv_mem = 0.f;
-        const float4* k4 = reinterpret_cast<const float4*>(&sh_k[t][i0]);  // 16-byte broadcast reads
-        const float4* q4 = reinterpret_cast<const float4*>(&sh_q[t][i0]);
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            const float4 kk = k4[m];
-            const float kv[4] = {kk.x, kk.y, kk.z, kk.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float sv = col[m * 4 + e] * eg;
-                col[m * 4 + e] = sv;
-                kv_mem += sv * kv[e];
-            }
-        }
-        part_sum[t & 1][part][j] = kv_mem;
-        __syncthreads();
-        const float* ps = &part_sum[t & 1][0][j];
-        const float delta = (v - (((ps[0] + ps[128]) + ps[256]) + ps[384])) * sh_beta[t];
-        float attn = 0.f;
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            const float4 kk = k4[m], qq = q4[m];
-            const float kv[4] = {kk.x, kk.y, kk.z, kk.w}, qv[4] = {qq.x, qq.y, qq.z, qq.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float ns = col[m * 4 + e] + kv[e] * delta;
-                col[m * 4 + e] = ns;
-                attn += ns * qv[e];
-            }
-        }
-        attn_all[t][part][j] = attn;
-        if (part == 0) {
-            pend_k[(pbase + t) * 128 + j] = sh_k[t][j];
-            pend_d[(pbase + t) * 128 + j] = delta;
-            if (j == 0) pend_g[pbase + t] = eg;
+        for (int i = 0; i < 4; ++i) {
+            const int d = lane + 32 * i;
+            sh_q[t][d] = (q[i] * rq) * 0.08838834764f;
+            sh_k[t][d] = k[i] * rk;
+            sh_v[t][d] = v[i];
+            sh_z[t][d] = zz[i] / (1.0f + expf(-zz[i]));
         }
     }
     __syncthreads();
 
-    // ---- phase 2: gated RMSNorm of every token's output (token tt handled by thread group tt % 4)
-    for (int t0 = 0; t0 < rows_per_seq; t0 += 4) {
-        const int tt = t0 + part;
-        float attn = 0.f;
-        if (tt < rows_per_seq) attn = ((attn_all[tt][0][j] + attn_all[tt][1][j]) + attn_all[tt][2][j]) + attn_all[tt][3][j];
-        const float wsq = warp_sum(attn * attn);
-        __syncthreads();
-        if (lane == 0) red[0][part * 4 + wig] = wsq;
-        __syncthreads();
-        if (tt < rows_per_seq) {
-            const float sq = ((red[0][part * 4] + red[0][part * 4 + 1]) + red[0][part * 4 + 2]) + red[0][part * 4 + 3];
-            const float inv_std = 1.0f / sqrtf(sq / 128.0f + 1e-6f);
-            const long long row = static_cast<long long>(b) * rows_per_seq + tt;
-            const float zv = __half2float(z[row * value_dim + h * 128 + j]);
-            const float silu_z = zv / (1.0f + expf(-zv));
-            out[row * value_dim + h * 128 + (perm_out ? perm8(j) : j)] = __float2half_rn(attn * inv_std * norm_w[j] * silu_z);
+    // ---- the state streams through
+    uint64_t ks[TOKENS], qs[TOKENS];  // sums over the even and the odd rows
+#pragma unroll
+    for (int t = 0; t < TOKENS; ++t) ks[t] = qs[t] = 0;
+#pragma unroll 1
+    for (int r0 = 0; r0 < kRows; r0 += BATCH) {
+        uint64_t cur[BATCH / 2];
+#pragma unroll
+        for (int i = 0; i < BATCH / 2; ++i) cur[i] = pack_f32x2(next[2 * i], next[2 * i + 1]);
+        if (r0 + BATCH < kRows) {
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) next[i] = S[(r0 + BATCH + i) * 128];
+        }
+        if (nc > 0) {
+#pragma unroll 1
+            for (int t = 0; t < nc; ++t) {  // the previous step's accepted updates
+                const uint64_t eg = pack_f32x2(sh_pg[t], sh_pg[t]), dj = pack_f32x2(sh_pd[t][j], sh_pd[t][j]);
+                const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(&sh_pk[t][i0 + r0]);
+#pragma unroll
+                for (int m = 0; m < BATCH / 4; ++m) {
+                    const ulonglong2 kk = k4[m];
+                    cur[2 * m] = fma_f32x2(kk.x, dj, mul_f32x2(cur[2 * m], eg));
+                    cur[2 * m + 1] = fma_f32x2(kk.y, dj, mul_f32x2(cur[2 * m + 1], eg));
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < BATCH / 2; ++i) {
+                S[(r0 + 2 * i) * 128] = __uint_as_float(static_cast<uint32_t>(cur[i]));
+                S[(r0 + 2 * i + 1) * 128] = __uint_as_float(static_cast<uint32_t>(cur[i] >> 32));
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < BATCH / 4; ++m) {
+#pragma unroll
+            for (int t = 0; t < TOKENS; ++t) {
+                const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(&sh_k[t][i0 + r0 + 4 * m]);
+                const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(&sh_q[t][i0 + r0 + 4 * m]);
+                ks[t] = fma_f32x2(cur[2 * m + 1], kk.y, fma_f32x2(cur[2 * m], kk.x, ks[t]));
+                qs[t] = fma_f32x2(cur[2 * m + 1], qq.y, fma_f32x2(cur[2 * m], qq.x, qs[t]));
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < TOKENS; ++t) sums[part][t][j] = sum_f32x2(ks[t]);
+    // products among the tokens: k or q of a token with the keys up to it
+    for (int e = warp; e < 2 * TOKENS; e += kWarps) {
+        const int t = e >> 1;
+        const float* a = (e & 1) ? sh_q[t] : sh_k[t];
+        const float a0 = a[lane], a1 = a[lane + 32], a2 = a[lane + 64], a3 = a[lane + 96];
+        for (int u = 0; u <= t && t < rows_per_seq; ++u) {
+            const float g = warp_sum((a0 * sh_k[u][lane] + a1 * sh_k[u][lane + 32]) + (a2 * sh_k[u][lane + 64] + a3 * sh_k[u][lane + 96]));
+            if (lane == 0) gram[e & 1][t][u] = g;
+        }
+    }
+    __syncthreads();
+    float kS[TOKENS];
+    auto column_sum = [&](int t) {
+        float v = sums[0][t][j] + sums[1][t][j];
+        if constexpr (PARTS == 4) v += sums[2][t][j] + sums[3][t][j];
+        return v;
+    };
+    if (part == 0) {
+#pragma unroll
+        for (int t = 0; t < TOKENS; ++t) kS[t] = column_sum(t);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < TOKENS; ++t) sums[part][t][j] = sum_f32x2(qs[t]);
+    __syncthreads();
+
+    // ---- the recurrence on the products; part 0 keeps the deltas
+    if (part == 0) {
+        float delta[TOKENS], decay[TOKENS];  // decay[u]: from token u to the present one
+        float G = 1.f;
+#pragma unroll
+        for (int t = 0; t < TOKENS; ++t) {
+            if (t >= rows_per_seq) break;
+            const float eg = sh_eg[t];
+            G *= eg;
+            float mem = G * kS[t], att = G * column_sum(t);
+#pragma unroll
+            for (int u = 0; u < t; ++u) {
+                decay[u] *= eg;
+                const float d = decay[u] * delta[u];
+                mem += gram[0][t][u] * d;
+                att += gram[1][t][u] * d;
+            }
+            decay[t] = 1.f;
+            delta[t] = (sh_v[t][j] - mem) * sh_beta[t];
+            sums[0][t][j] = att + gram[1][t][t] * delta[t];
+            pend_d[(pbase + t) * 128 + j] = delta[t];
+            if (j == 0) pend_g[pbase + t] = eg;
+        }
+    } else if (part == 1) {
+        for (int t = 0; t < rows_per_seq; ++t) pend_k[(pbase + t) * 128 + j] = sh_k[t][j];
+    }
+    __syncthreads();
+
+    // ---- gated RMSNorm of every token's output: one warp per token
+    if (warp < rows_per_seq) {
+        const int t = warp;
+        const float* at = sums[0][t];
+        const float a[4] = {at[lane], at[lane + 32], at[lane + 64], at[lane + 96]};
+        const float sq = warp_sum_sq(a);
+        const float inv_std = 1.0f / sqrtf(sq / 128.0f + 1e-6f);
+        __half* orow = out + (static_cast<long long>(b) * rows_per_seq + t) * value_dim + h * 128;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int d = lane + 32 * i;
+            orow[perm_out ? perm8(d) : d] = __float2half_rn(a[i] * inv_std * sh_nw[d] * sh_z[t][d]);
         }
     }
 }
@@ -555,26 +650,6 @@ __global__ void __launch_bounds__(128) conv1d_chunk_kernel(__half* out, const __
 constexpr int kGdnWalkRows = 16;
 constexpr int kGdnCols = 16, kGdnBlock = 16, kGdnSlices = 128 / kGdnCols, kGdnThreads = kGdnCols * 8;
 
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
-    uint64_t d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-__device__ __forceinline__ float sum_f32x2(uint64_t a) {
-    float lo, hi;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));
-    return lo + hi;
-}
 
 __global__ void __cluster_dims__(kGdnSlices, 1, 1) __launch_bounds__(kGdnThreads) gdn_walk_kernel(
     __half* out, const __half* qkv, const __half* z, const __half* bb, const __half* aa, const float* A_log, const float* dt_bias,
@@ -1234,7 +1309,7 @@ int embed_norm_rows(cudaStream_t s, __half* out, __half* x, const void* table_bf
     j.table = static_cast<const uint16_t*>(table_bf16);
     j.tokens = tokens;
     j.vocab = vocab;
-    launch_pdl(rmsnorm_kernel, dim3(rows), dim3(256), 0, s, j, j, static_cast<long long>(hidden), hidden, eps, perm_out);
+    launch_pdl(rmsnorm_kernel<true>, dim3(rows), dim3(256), 0, s, j, j, static_cast<long long>(hidden), hidden, eps, perm_out);
     return XB_LAUNCH_OK();
 }
 
@@ -1253,7 +1328,7 @@ int head_input_rows(cudaStream_t s, const HeadInput& h, int rows, int hidden, fl
     p.out = h.cat + hidden;
     p.x = const_cast<__half*>(h.hidden_rows);
     p.w = h.hidden_norm;
-    launch_pdl(rmsnorm_kernel, dim3(rows, 2), dim3(256), 0, s, e, p, 2LL * hidden, hidden, eps, perm_out);
+    launch_pdl(rmsnorm_kernel<true>, dim3(rows, 2), dim3(256), 0, s, e, p, 2LL * hidden, hidden, eps, perm_out);
     return XB_LAUNCH_OK();
 }
 
@@ -1263,7 +1338,7 @@ int rmsnorm_rows(cudaStream_t s, __half* out, long long ld_out, const __half* in
     j.out = out;
     j.x = const_cast<__half*>(in);
     j.w = w;
-    launch_pdl(rmsnorm_kernel, dim3(rows), dim3(256), 0, s, j, j, ld_out, hidden, eps, perm_out);
+    launch_pdl(rmsnorm_kernel<false>, dim3(rows), dim3(256), 0, s, j, j, ld_out, hidden, eps, perm_out);
     return XB_LAUNCH_OK();
 }
 
@@ -1274,7 +1349,7 @@ int add_rmsnorm_rows(cudaStream_t s, __half* out, __half* x, const __half* delta
     j.x = x;
     j.delta = delta;
     j.w = w;
-    launch_pdl(rmsnorm_kernel, dim3(rows), dim3(256), 0, s, j, j, static_cast<long long>(hidden), hidden, eps, perm_out);
+    launch_pdl(rmsnorm_kernel<false>, dim3(rows), dim3(256), 0, s, j, j, static_cast<long long>(hidden), hidden, eps, perm_out);
     return XB_LAUNCH_OK();
 }
 
@@ -1305,10 +1380,15 @@ int conv1d_spec(cudaStream_t s, __half* out, const __half* in, const float* conv
 int gdn_spec(cudaStream_t s, __half* out, const __half* qkv, const __half* z, const __half* b, const __half* a,
              const float* A_log, const float* dt_bias, const float* norm_w, float* state, float* pend_k, float* pend_d,
              float* pend_g, const int* n_commit, int batch, int rows_per_seq, int prev_rows, int hv, int hk, int nc_base,
-             int early_state, int perm_out) {
-    dim3 grid(hv, batch);
-    launch_pdl(gdn_spec_kernel, dim3(grid), dim3(512), 0, s, out, qkv, z, b, a, A_log, dt_bias, norm_w, state, pend_k, pend_d, pend_g,
-                                         n_commit, rows_per_seq, prev_rows, hv, hk, nc_base, early_state, perm_out);
+             int early_state, int perm_out, int num_sms) {
+    // more heads than SMs: several per SM, whose streams overlap each other (144 heads: 6.7 us with 512 threads a head and
+    // 9.2 with 256; 192 heads: 13.5 and 9.4)
+    const bool many = hv * batch > num_sms;
+    const bool few_tokens = rows_per_seq <= 4;
+    launch_pdl(many ? (few_tokens ? gdn_spec_kernel<2, 16, 4> : gdn_spec_kernel<2, 16, 8>)
+                    : (few_tokens ? gdn_spec_kernel<4, 32, 4> : gdn_spec_kernel<4, 32, 8>),
+               dim3(hv, batch), dim3(many ? 256 : 512), 0, s, out, qkv, z, b, a, A_log, dt_bias, norm_w, state, pend_k, pend_d, pend_g,
+               n_commit, rows_per_seq, prev_rows, hv, hk, nc_base, early_state, perm_out);
     return XB_LAUNCH_OK();
 }
 

@@ -73,11 +73,11 @@ int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status);
 int conv1d_spec(cudaStream_t s, __half* out, const __half* in, const float* conv_w, float* state, float* pending,
                 const int* n_commit, int batch, int rows_per_seq, int prev_rows, int channels, int nc_base = 0,
                 int early_state = 0);
-// state [batch][hv][128][128], pend_k / pend_d [batch][hv][8][128], pend_g [batch][hv][8] fp32
+// state [batch][hv][128][128], pend_k / pend_d [batch][hv][8][128], pend_g [batch][hv][8] fp32; rows_per_seq <= 8
 int gdn_spec(cudaStream_t s, __half* out, const __half* qkv, const __half* z, const __half* b, const __half* a,
              const float* A_log, const float* dt_bias, const float* norm_w, float* state, float* pend_k, float* pend_d,
-             float* pend_g, const int* n_commit, int batch, int rows_per_seq, int prev_rows, int hv, int hk, int nc_base = 0,
-             int early_state = 0, int perm_out = 0);
+             float* pend_g, const int* n_commit, int batch, int rows_per_seq, int prev_rows, int hv, int hk, int nc_base,
+             int early_state, int perm_out, int num_sms);
 
 // The convolution and the gated delta rule over all rc positions of a prefill chunk in one launch each (rows
 // [sequence][position], every row kept, the state read once and written back once; nothing pending afterwards).  A null

@@ -195,7 +195,10 @@ int xinfer_recurrent_gated_delta_net_f16(xinfer_stream_t s, void* out, const voi
     // pointers that the vector accesses of the chunk kernel do not fit: eight tokens a launch through the step's kernel
     const size_t pk = static_cast<size_t>(hv) * 8 * 128;
     float* scr = nullptr;
-    int rc = scratch((2 * pk + static_cast<size_t>(hv) * 8) * sizeof(float), &scr);
+    int *status = nullptr, num_sms = 0;
+    int rc = xb::device_facts(&status, &num_sms);
+    if (rc != XINFER_OK) return rc;
+    rc = scratch((2 * pk + static_cast<size_t>(hv) * 8) * sizeof(float), &scr);
     if (rc != XINFER_OK) return rc;
     float *pend_k = scr, *pend_d = scr + pk, *pend_g = scr + 2 * pk;
     cudaStream_t st = static_cast<cudaStream_t>(s);
@@ -210,12 +213,12 @@ int xinfer_recurrent_gated_delta_net_f16(xinfer_stream_t s, void* out, const voi
     for (int64_t t0 = 0; t0 < seq_len; t0 += 8) {
         const int rows = static_cast<int>(seq_len - t0 < 8 ? seq_len - t0 : 8);
         rc = xb::gdn_spec(st, o + t0 * vd, q + t0 * ch, zz + t0 * vd, bb + t0 * hv, aa + t0 * hv, A_log, dt_bias, norm_weight,
-                          state_buffer, pend_k, pend_d, pend_g, nullptr, 1, rows, prev, hv, hk, prev);
+                          state_buffer, pend_k, pend_d, pend_g, nullptr, 1, rows, prev, hv, hk, prev, 0, 0, num_sms);
         if (rc != 0) return ok_or_cuda(rc);
         prev = rows;
     }
     return ok_or_cuda(xb::gdn_spec(st, o, q, zz, bb, aa, A_log, dt_bias, norm_weight, state_buffer, pend_k, pend_d, pend_g, nullptr,
-                                   1, 0, prev, hv, hk, prev));
+                                   1, 0, prev, hv, hk, prev, 0, 0, num_sms));
 }
 
 /* ---- plain device memory and streams, for hosts that do not link the CUDA runtime themselves --------------- */

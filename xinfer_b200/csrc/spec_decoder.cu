@@ -532,7 +532,7 @@ int layer_forward(Dec* d, cudaStream_t s, Layer& L, int R, __half* xr, const flo
         NL(xb::gdn_spec(s, d->delta_out.p + static_cast<size_t>(row0) * hv * 128, d->qkv_conv + static_cast<size_t>(row0) * ch,
                         d->zbuf.p + static_cast<size_t>(row0) * hv * 128, d->bbuf + static_cast<size_t>(row0) * hv,
                         d->abuf + static_cast<size_t>(row0) * hv, L.A_log, L.dt_bias, L.gdn_norm, L.S, L.pend_k, L.pend_d,
-                        L.pend_g, n_commit + d->b0, Bl, R, prev_rows, hv, hk, 0, 1, xperm_on()));
+                        L.pend_g, n_commit + d->b0, Bl, R, prev_rows, hv, hk, 0, 1, xperm_on(), d->num_sms));
         d->launches_per_step += 2;
         CK(gather_rows(d, s, d->delta_out, row0, Ml, static_cast<int64_t>(hv) * 128));
         CK(lin_add_norm(d, s, d->proj_out, d->delta_out.p, L.out_proj, M, xr, L.post_norm));
