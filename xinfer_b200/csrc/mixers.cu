@@ -842,8 +842,11 @@ __global__ void __cluster_dims__(kGdnSlices, 1, 1) __launch_bounds__(kGdnThreads
 // tf32 operands the same kernel ran at a quarter of the rate: mma.sync of that type does 90 multiply-adds per clock and SM.)
 // Transposed products (state S^T, with the value columns as the MMA's rows) let a warp keep its 16 x 128 slice of the state
 // in accumulators that are A operands as they stand.
-// 512 tokens, one sequence, 48 heads: 160 us, 1.5 ms through the step's kernel eight tokens a launch, 300 us with
-// gdn_walk_kernel; bound by the latency of a block (1800 instructions per warp at 0.2 per clock, one warp per scheduler).
+// Bound by the latency of a block, one warp per scheduler, so nothing that the next block does not wait for stays in the walk:
+// it leaves the raw outputs in fp32, and gdn_norm_kernel does their gated RMSNorm, which spans all columns of a head, for all
+// tokens at once (with a cluster adding up the squares inside the walk the scan took 145 us).
+// 512 tokens, one sequence, 48 heads: 67 us, 1.5 ms through the step's kernel eight tokens a launch, 300 us with
+// gdn_walk_kernel.
 constexpr int kScanBlock = 16, kScanWarps = 2, kScanCols = 16 * kScanWarps, kScanSlices = 128 / kScanCols, kScanPitch = 136;
 constexpr float kSplitDown = 0.0625f, kSplitUp = 16.0f, kMidUp = 2048.0f, kMidDown = 1.0f / 2048.0f;
 struct GdnBlock {                         // one block of one head, written by gdn_block_kernel
@@ -1010,12 +1013,12 @@ __global__ void __launch_bounds__(128) gdn_block_kernel(GdnBlock* blocks, const 
     }
 }
 
-__global__ void __cluster_dims__(kScanSlices, 1, 1) __launch_bounds__(32 * kScanWarps) gdn_scan_kernel(
-    __half* out, const __half* qkv, const __half* z, const GdnBlock* blocks, const float* norm_w, float* state, int rc, int hv, int hk,
-    int zero_state) {
+__global__ void __launch_bounds__(32 * kScanWarps) gdn_scan_kernel(float* raw, const __half* qkv, const GdnBlock* blocks, float* state,
+                                                                   int rc, int hv, int hk, int zero_state) {
     griddep_prologue();
     __shared__ __align__(16) __half sh_q[2][kScanBlock][kScanPitch], sh_k[2][kScanBlock][kScanPitch];
-    __shared__ float sh_sq[2][kScanSlices * kScanWarps][kScanBlock];  // sums of squares of the outputs, by warp of the cluster
+    __shared__ __align__(16) __half sh_v[2][kScanBlock][kScanCols + 8];
+    __shared__ __align__(16) GdnBlock sh_blk[2];
     const int slice = blockIdx.x % kScanSlices, h = blockIdx.x / kScanSlices, b = blockIdx.y;
     const long long seq0 = static_cast<long long>(b) * rc;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -1025,7 +1028,9 @@ __global__ void __cluster_dims__(kScanSlices, 1, 1) __launch_bounds__(32 * kScan
     const GdnBlock* blk = blocks + (static_cast<long long>(b) * hv + h) * nblocks;
     float* S = state + (static_cast<long long>(b) * hv + h) * (128 * 128);
 
-    // a block's q and k: 16-byte pieces straight into shared memory, zeros behind the end
+    // A block's q, k, v, matrices and factors: 16-byte pieces straight into shared memory, zeros behind the end.  (The small
+    // operands were fetched to registers a block ahead before, but with 255 of them in use the compiler moved the loads down to
+    // where they are needed: a trip to L2 in every block, 85 us against 67.)
     auto stage = [&](int n) {
         const int buf = n & 1;
 #pragma unroll
@@ -1036,35 +1041,24 @@ __global__ void __cluster_dims__(kScanSlices, 1, 1) __launch_bounds__(32 * kScan
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(&sh_q[buf][row][c])), "l"(cur), "r"(bytes) : "memory");
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(&sh_k[buf][row][c])), "l"(cur + hk * 128), "r"(bytes) : "memory");
         }
+        constexpr int kVPieces = kScanCols / 8, kBlkPieces = static_cast<int>(sizeof(GdnBlock) / 16);
+#pragma unroll
+        for (int u = 0; u < (kScanBlock * kVPieces + 32 * kScanWarps - 1) / (32 * kScanWarps); ++u) {
+            const int idx = u * 32 * kScanWarps + tid, row = idx / kVPieces, c = (idx % kVPieces) * 8, p = n * kScanBlock + row;
+            const __half* cur = qkv + (seq0 + (p < rc ? p : n * kScanBlock)) * channels + 2 * hk * 128 + h * 128 + slice * kScanCols + c;
+            if (row < kScanBlock)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(&sh_v[buf][row][c])), "l"(cur), "r"(p < rc ? 16 : 0) : "memory");
+        }
+#pragma unroll
+        for (int u = 0; u < (kBlkPieces + 32 * kScanWarps - 1) / (32 * kScanWarps); ++u) {
+            const int idx = u * 32 * kScanWarps + tid;
+            if (idx < kBlkPieces)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&sh_blk[buf]) + idx * 16),
+                             "l"(reinterpret_cast<const char*>(blk + n) + idx * 16) : "memory");
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    // its small operands: v of the thread's two columns and four tokens 8 (i / 2) + 2t + i % 2, the block's matrices and factors
-    __half rv[2][4];
-    uint32_t rt[2][2][2], rp[2][2][2];  // [hi, mid][i tile][j half]
-    float4 rcoef[4];
-    auto fetch = [&](int n) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int j = 8 * (i >> 1) + 2 * t + (i & 1), p = n * kScanBlock + j;
-            const __half* cur = qkv + (seq0 + (p < rc ? p : n * kScanBlock)) * channels + 2 * hk * 128 + h * 128 + c0;
-            rv[0][i] = p < rc ? cur[0] : __half(0.f);
-            rv[1][i] = p < rc ? cur[8] : __half(0.f);
-            rcoef[i] = __ldg(&blk[n].coef[j]);
-        }
-#pragma unroll
-        for (int w = 0; w < 2; ++w) {
-#pragma unroll
-            for (int it = 0; it < 2; ++it) {
-#pragma unroll
-                for (int jh = 0; jh < 2; ++jh) {
-                    rt[w][it][jh] = __ldg(reinterpret_cast<const uint32_t*>(&blk[n].t[w][it * 8 + g][jh * 8 + 2 * t]));
-                    rp[w][it][jh] = __ldg(reinterpret_cast<const uint32_t*>(&blk[n].p[w][it * 8 + g][jh * 8 + 2 * t]));
-                }
-            }
-        }
-    };
     stage(0);
-    fetch(0);
 
     float s[16][4];  // 2^-4 S^T: s[n][e] = 2^-4 S[8n + 2t + (e & 1)][c0 + 8 (e >> 1)]
 #pragma unroll
@@ -1072,78 +1066,16 @@ __global__ void __cluster_dims__(kScanSlices, 1, 1) __launch_bounds__(32 * kScan
 #pragma unroll
         for (int e = 0; e < 4; ++e) s[n][e] = zero_state ? 0.f : kSplitDown * S[(8 * n + 2 * t + (e & 1)) * 128 + c0 + 8 * (e >> 1)];
     }
-    const float nw[2] = {norm_w[c0], norm_w[c0 + 8]};
-
-    // The block whose norm is under way: its outputs [token tile][fragment], gates and rows.  Its stores are issued behind
-    // the next cluster barrier's arrive, which is a release and would wait for them.
-    float o[2][4];
-    __half zv[2][4];
-    auto out_row = [&](int n, int i) -> long long {
-        const int p = n * kScanBlock + 8 * (i >> 1) + 2 * t + (i & 1);
-        return p < rc ? (seq0 + p) * value_dim + h * 128 + c0 : -1;
-    };
-    auto fetch_z = [&](int n) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const long long at = out_row(n, i);
-            zv[0][i] = at >= 0 ? z[at] : __half(0.f);
-            zv[1][i] = at >= 0 ? z[at + 8] : __half(0.f);
-        }
-    };
-    __half y[2][4];
-    auto norm = [&](int n) {
-        cluster_wait();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float sq = 0.f;
-#pragma unroll
-            for (int r = 0; r < kScanSlices * kScanWarps; ++r) sq += sh_sq[n & 1][r][8 * (i >> 1) + 2 * t + (i & 1)];
-            const float inv_std = 1.0f / sqrtf(sq / 128.0f + 1e-6f);
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const float zf = __half2float(zv[c][i]);
-                y[c][i] = __float2half_rn(o[i >> 1][2 * c + (i & 1)] * inv_std * nw[c] * (zf / (1.0f + expf(-zf))));
-            }
-        }
-    };
-    auto store = [&](int n) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const long long at = out_row(n, i);
-            if (at >= 0) {
-                out[at] = y[0][i];
-                out[at + 8] = y[1][i];
-            }
-        }
-    };
     // ldmatrix addresses: [token][state row] tiles, (token halves) x (row halves), plain and transposed
     const uint32_t lm_row = static_cast<uint32_t>(((lane >> 4) & 1) * 8 + (lane & 7)), lm_col = static_cast<uint32_t>(((lane >> 3) & 1) * 8);
     const uint32_t lt_row = static_cast<uint32_t>(((lane >> 3) & 1) * 8 + (lane & 7)), lt_col = static_cast<uint32_t>(((lane >> 4) & 1) * 8);
 
     for (int n = 0; n < nblocks; ++n) {
         const int buf = n & 1;
-        // this block's small operands, before the next block's take their registers
-        float v[2][4];
-        float4 coef[4];
-        uint32_t tm[2][2][2], pm[2][2][2];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            v[0][i] = __half2float(rv[0][i]);
-            v[1][i] = __half2float(rv[1][i]);
-            coef[i] = rcoef[i];
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            tm[i >> 2][(i >> 1) & 1][i & 1] = rt[i >> 2][(i >> 1) & 1][i & 1];
-            pm[i >> 2][(i >> 1) & 1][i & 1] = rp[i >> 2][(i >> 1) & 1][i & 1];
-        }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        if (n > 0) fetch_z(n - 1);
-        if (n + 1 < nblocks) {
-            stage(n + 1);
-            fetch(n + 1);
-        }
+        if (n + 1 < nblocks) stage(n + 1);
+        const GdnBlock& here = sh_blk[buf];
 
         // (K S0)^T and (Q S0)^T: 16 value columns x 16 tokens, contraction over the 128 state rows
         float ks[2][2][4] = {}, qs[2][2][4] = {};  // [hi, mid][token tile]
@@ -1161,6 +1093,22 @@ __global__ void __cluster_dims__(kScanSlices, 1, 1) __launch_bounds__(32 * kScan
                 mma_f16(ks[1][nt], mid, kb[2 * nt], kb[2 * nt + 1]);
                 mma_f16(qs[1][nt], mid, qb[2 * nt], qb[2 * nt + 1]);
             }
+        }
+        float v[2][4];  // the thread's two columns, tokens 8 (i / 2) + 2t + i % 2
+        float4 coef[4];
+        uint32_t tm[2][2][2], pm[2][2][2];  // [hi, mid][i tile][j half]
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int j = 8 * (i >> 1) + 2 * t + (i & 1);
+            v[0][i] = __half2float(sh_v[buf][j][warp * 16 + g]);
+            v[1][i] = __half2float(sh_v[buf][j][warp * 16 + g + 8]);
+            coef[i] = here.coef[j];
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int w = i >> 2, it = (i >> 1) & 1, jh = i & 1;
+            tm[w][it][jh] = *reinterpret_cast<const uint32_t*>(&here.t[w][it * 8 + g][jh * 8 + 2 * t]);
+            pm[w][it][jh] = *reinterpret_cast<const uint32_t*>(&here.p[w][it * 8 + g][jh * 8 + 2 * t]);
         }
         // 2^-4 delta^T = (2^-4 (V - diag(G / |k|) K S0))^T T^T
         float delta[2][4] = {}, acc[2][4] = {}, u[2][4];
@@ -1219,38 +1167,44 @@ __global__ void __cluster_dims__(kScanSlices, 1, 1) __launch_bounds__(32 * kScan
                 for (int e = 0; e < 4; ++e) sn[e] = fmaf(low[e], kMidDown, sn[e]);
             }
         }
-        if (n > 0) norm(n - 1);
-        // sums of squares over this warp's 16 columns, to every CTA of the cluster
-        float sq[4];
 #pragma unroll
         for (int jt = 0; jt < 2; ++jt) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                o[jt][e] = coef[jt * 2 + (e & 1)].y * (qs[0][jt][e] + kMidDown * qs[1][jt][e]) + kSplitUp * (od[jt][e] + kMidDown * acc[jt][e]);
+            for (int e = 0; e < 4; ++e) {
+                const int p = n * kScanBlock + 8 * jt + 2 * t + (e & 1);
+                const float o = coef[jt * 2 + (e & 1)].y * (qs[0][jt][e] + kMidDown * qs[1][jt][e]) + kSplitUp * (od[jt][e] + kMidDown * acc[jt][e]);
+                if (p < rc) raw[((seq0 + p) * hv + h) * 128 + c0 + 8 * (e >> 1)] = o;
+            }
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float a = o[i >> 1][i & 1], c = o[i >> 1][2 + (i & 1)];
-            sq[i] = a * a + c * c;
-#pragma unroll
-            for (int off = 4; off < 32; off <<= 1) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], off);
-        }
-        if (g < kScanSlices) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                st_shared_cluster_f32(mapa_shared_cluster(smem_u32(&sh_sq[buf][slice * kScanWarps + warp][8 * (i >> 1) + 2 * t + (i & 1)]), g), sq[i]);
-        }
-        cluster_arrive();
-        if (n > 0) store(n - 1);
     }
-    fetch_z(nblocks - 1);
-    norm(nblocks - 1);
-    store(nblocks - 1);
 #pragma unroll
     for (int n = 0; n < 16; ++n) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) S[(8 * n + 2 * t + (e & 1)) * 128 + c0 + 8 * (e >> 1)] = kSplitUp * s[n][e];
     }
+}
+
+// out = rmsnorm(raw) * w * silu(z) over the 128 values of a head: a warp per (row, head), memory bound (14 bytes a value moved,
+// most of them still in L2).
+__global__ void __launch_bounds__(256) gdn_norm_kernel(__half* out, const float* raw, const __half* z, const float* norm_w, long long heads) {
+    const int lane = threadIdx.x & 31;
+    const long long head = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5), at = head * 128 + 4 * lane;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    float w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = norm_w[4 * lane + i];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (head >= heads) return;
+    const float4 x = *reinterpret_cast<const float4*>(raw + at);
+    const __half2 z0 = *reinterpret_cast<const __half2*>(z + at), z1 = *reinterpret_cast<const __half2*>(z + at + 2);
+    const float v[4] = {x.x, x.y, x.z, x.w}, g[4] = {__low2float(z0), __high2float(z0), __low2float(z1), __high2float(z1)};
+    const float sq = warp_sum((v[0] * v[0] + v[1] * v[1]) + (v[2] * v[2] + v[3] * v[3]));
+    const float inv_std = 1.0f / sqrtf(sq / 128.0f + 1e-6f);
+    float y[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) y[i] = v[i] * inv_std * w[i] * (g[i] / (1.0f + expf(-g[i])));
+    *reinterpret_cast<__half2*>(out + at) = __floats2half2_rn(y[0], y[1]);
+    *reinterpret_cast<__half2*>(out + at + 2) = __floats2half2_rn(y[2], y[3]);
 }
 
 // ------------------------------------------------------------------------------- speculative bookkeeping
@@ -1412,7 +1366,8 @@ bool gdn_chunk_aligned(const void* out, const void* qkv, const void* z, const vo
 }
 
 size_t gdn_chunk_scratch_bytes(int batch, int rc, int hv) {
-    return static_cast<size_t>(batch) * hv * ((rc + kScanBlock - 1) / kScanBlock) * sizeof(GdnBlock);
+    const size_t heads = static_cast<size_t>(batch) * hv;
+    return heads * rc * 128 * sizeof(float) + heads * ((rc + kScanBlock - 1) / kScanBlock) * sizeof(GdnBlock);  // outputs, blocks
 }
 
 int gdn_chunk(cudaStream_t s, __half* out, const __half* qkv, const __half* z, const __half* b, const __half* a,
@@ -1423,11 +1378,14 @@ int gdn_chunk(cudaStream_t s, __half* out, const __half* qkv, const __half* z, c
                    state, rc, hv, hk, zero_state);
         return XB_LAUNCH_OK();
     }
-    GdnBlock* blocks = static_cast<GdnBlock*>(scratch);
+    const long long heads = static_cast<long long>(batch) * rc * hv;
+    float* raw = static_cast<float*>(scratch);
+    GdnBlock* blocks = reinterpret_cast<GdnBlock*>(raw + heads * 128);
     const int nblocks = (rc + kScanBlock - 1) / kScanBlock;
     launch_pdl(gdn_block_kernel, dim3((nblocks + 3) / 4, hv, batch), dim3(128), 0, s, blocks, qkv, b, a, A_log, dt_bias, rc, hv, hk);
-    launch_pdl(gdn_scan_kernel, dim3(hv * kScanSlices, batch), dim3(32 * kScanWarps), 0, s, out, qkv, z, static_cast<const GdnBlock*>(blocks),
-               norm_w, state, rc, hv, hk, zero_state);
+    launch_pdl(gdn_scan_kernel, dim3(hv * kScanSlices, batch), dim3(32 * kScanWarps), 0, s, raw, qkv, static_cast<const GdnBlock*>(blocks),
+               state, rc, hv, hk, zero_state);
+    launch_pdl(gdn_norm_kernel, dim3(static_cast<unsigned>((heads + 7) / 8)), dim3(256), 0, s, out, static_cast<const float*>(raw), z, norm_w, heads);
     return XB_LAUNCH_OK();
 }
 

@@ -176,8 +176,8 @@ int xinfer_recurrent_gated_delta_net_f16(xinfer_stream_t s, void* out, const voi
     if (!out || !qkv || !z || !b || !a || !A_log || !dt_bias || !norm_weight || !state_buffer) return XINFER_ERR_INVALID_ARGUMENT;
     const int hv = static_cast<int>(num_v_heads), hk = static_cast<int>(num_k_heads);
     if (xb::gdn_chunk_aligned(out, qkv, z, state_buffer)) {
-        // pieces of 4096 rows bound the scratch (29 MB at 48 heads)
-        const int64_t piece = 4096, ch = 2 * static_cast<int64_t>(hk) * 128 + static_cast<int64_t>(hv) * 128, vd = static_cast<int64_t>(hv) * 128;
+        // pieces of 1024 rows bound the scratch (32 MB at 48 heads)
+        const int64_t piece = 1024, ch = 2 * static_cast<int64_t>(hk) * 128 + static_cast<int64_t>(hv) * 128, vd = static_cast<int64_t>(hv) * 128;
         float* blocks = nullptr;
         const int most = static_cast<int>(seq_len < piece ? seq_len : piece);
         const int rc = scratch(xb::gdn_chunk_scratch_bytes(1, most, hv), &blocks);
