@@ -56,8 +56,6 @@ constexpr int kWSlotBytes = kGemmTileN * 64;                    // 8 KB of packe
 constexpr int kAHalfBytes = kGemmTileN * kSwizzleK * 2;         // 16 KB: 64 k of unpacked weights
 constexpr int kASlotBytes = 2 * kAHalfBytes;
 constexpr int kGemmTmemCols = 512;
-constexpr int kGemmParkPitch = 9;
-constexpr int kGemmParkBytes = 256 * kGemmParkPitch * 4;  // gate/up exchange: [fold thread][8 columns]
 constexpr int kGemmMaxProj = 4;
 // Register split of the launch's 512 x 128: the fold keeps 128 sums per thread.
 constexpr int kFoldRegs = 208, kUnpackRegs = 64, kCtrlRegs = 32;
@@ -72,9 +70,9 @@ struct GemmCtrl {
     WaitState ws;
 };
 
-// [alignment slack] [A ring] [X ring: slots x 2 x tile_m / 2 x 128 bytes] [W ring] [park] [control]
+// [alignment slack] [A ring] [X ring: slots x 2 x tile_m / 2 x 128 bytes] [W ring] [control]
 constexpr int kGemmSmemBytes = 227 * 1024;
-constexpr int kGemmSmemFixed = 1024 + kGemmParkBytes + static_cast<int>(sizeof(GemmCtrl));
+constexpr int kGemmSmemFixed = 1024 + static_cast<int>(sizeof(GemmCtrl));
 constexpr int gemm_slots_bytes(int tile_m, int slots) { return slots * (kASlotBytes + tile_m * 2 * kSwizzleK); }
 constexpr int gemm_op_slots(int tile_m) {
     return kGemmSmemFixed + gemm_slots_bytes(tile_m, 4) + 3 * kWSlotBytes <= kGemmSmemBytes ? 4 : 3;
@@ -109,11 +107,11 @@ struct GemmParams {
     long long units;     // tiles * groups
     int pairs;           // CTA pairs of the launch
     int whole_tiles;     // cut between tiles only
-    int swiglu;      // rows 0-63 of a CTA = gate, 64-127 = up of the same 64 features; y = silu(gate) * up
+    int swiglu;      // a CTA's rows: gate and up of the same 64 features, sixteen and sixteen; y = silu(gate) * up
     long long wait_limit;
     int* status;
     int x_stage_limit;  // test hook: activation stages (of a CTA) from this index on are never requested (-1: off)
-    float* partials;    // [CTA][2][column][fold thread]: fp32 sums of the tiles a CTA holds a part of
+    float* partials;    // [CTA][2][column / 4][fold thread][4]: fp32 sums of the tiles a CTA holds a part of
     int* counters;      // [CTA]: groups of the tile that starts in that pair's range and ends behind it, added up so far
 };
 
@@ -227,8 +225,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
     const uint32_t x_half_bytes = static_cast<uint32_t>(p.tile_m) * kSwizzleK;  // 64 k of this CTA's half of the rows
     uint8_t* w_ring = x_ring + op_slots * 2 * x_half_bytes;
     const int w_slots = p.w_slots;
-    float* park = reinterpret_cast<float*>(w_ring + w_slots * kWSlotBytes);
-    GemmCtrl* ctrl = reinterpret_cast<GemmCtrl*>(w_ring + w_slots * kWSlotBytes + kGemmParkBytes);
+    GemmCtrl* ctrl = reinterpret_cast<GemmCtrl*>(w_ring + w_slots * kWSlotBytes);
 
     const int tid = threadIdx.x;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -380,7 +377,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
         const int r = tid - kGemmFoldThreads;
         // raw rows of 64 bytes under the 64-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ ((r >> 1) & 3)
         const uint32_t w_row = static_cast<uint32_t>(r) * 64, w_sw = static_cast<uint32_t>((r >> 1) & 3);
-        const uint32_t a_row = static_cast<uint32_t>((r >> 3) * 1024 + (r & 7) * 128), a_sw = static_cast<uint32_t>(r & 7);
+        // gate/up: the raw tile is 64 rows of each, the operand sixteen and sixteen, so that a feature's two sums meet in one warp
+        const int ra = p.swiglu ? ((r & 48) << 1) + ((r >> 6) << 4) + (r & 15) : r;
+        const uint32_t a_row = static_cast<uint32_t>((ra >> 3) * 1024 + (ra & 7) * 128), a_sw = static_cast<uint32_t>(ra & 7);
         int wslot = 0, aslot = 0;
         uint32_t w_phase = 0, a_phase = 1;
         for (int i = 0; i < U; ++i) {
@@ -418,7 +417,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
         const int r = tid & 127, ch = tid >> 7;          // tile row, column half
         const int half_cols = p.tile_m >> 1;             // a multiple of 16
         const uint32_t d_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(ch * half_cols);
-        const bool up_row = p.swiglu && r >= 64;
+        const bool up_row = p.swiglu && (r & 16);
         float acc[kGemmTileM / 2];
         int i = 0, tile = first_tile, group = first_group;
         bool dead = false;
@@ -427,7 +426,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
             const int pr = proj_of_tile(p, tile);
             const GemmProj& pj = p.proj[pr];
             const int rel = tile - pj.tile0, nt = rel / p.m_tiles * 2 + static_cast<int>(rank), m0 = (rel % p.m_tiles) * p.tile_m;
-            const int row = p.swiglu ? nt * 64 + (r & 63) : nt * kGemmTileN + r;
+            const int row = p.swiglu ? nt * 64 + ((r & 96) >> 1) + (r & 15) : nt * kGemmTileN + r;
             const bool valid = row < pj.n;
             const unsigned short* sp = reinterpret_cast<const unsigned short*>(pj.scales[up_row ? 1 : 0]) +
                                        static_cast<long long>(valid ? row : 0) * p.groups;
@@ -476,72 +475,108 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
                 c_first = unit_owner(p, tu);
                 c_last = unit_owner(p, tu + p.groups - 1);
                 const size_t slot_floats = static_cast<size_t>(kGemmTileN) * kGemmTileM;
-                float* mine = p.partials + (static_cast<size_t>(blockIdx.x) * 2 + (seg_begin > 0 ? 0 : 1)) * slot_floats + tid;
-#pragma unroll
-                for (int j = 0; j < kGemmTileM / 2; ++j)
-                    if (j < half_cols) __stcg(mine + j * kGemmFoldThreads, acc[j]);
-                __threadfence();
-                fold_barrier();
-                if (tid == 0) {
-                    const int n = seg_end - seg_begin, old = atomicAdd(p.counters + c_first * 2 + rank, n);
-                    const bool last = old + n == p.groups;
-                    if (last) p.counters[c_first * 2 + rank] = 0;  // as the next launch expects it
-                    ctrl->last_arrival = last ? 1 : 0;
-                    __threadfence();
+                int* counter = p.counters + c_first * 2 + rank;
+                const int n = seg_end - seg_begin;
+                // A tile cut once: the second pair met its part at the start of its range, long ago.  If it has indeed arrived, this
+                // one's sums stay in registers (writing them, the fence behind it and reading them back took 3 us of 42 at N = 5120,
+                // M = 512).
+                bool kept = false;
+                if (pair == c_first && c_last == c_first + 1) {
+                    if (tid == 0) {
+                        const bool last = atomicAdd(counter, 0) + n == p.groups;
+                        if (last) *counter = 0;  // as the next launch expects it
+                        ctrl->last_arrival = last ? 1 : 0;
+                        __threadfence();
+                    }
+                    fold_barrier();
+                    kept = ctrl->last_arrival != 0;
+                    fold_barrier();
                 }
-                fold_barrier();
+                if (!kept) {
+                    float4* mine = reinterpret_cast<float4*>(p.partials + (static_cast<size_t>(blockIdx.x) * 2 + (seg_begin > 0 ? 0 : 1)) * slot_floats) + tid;
+#pragma unroll
+                    for (int j = 0; j < kGemmTileM / 2; j += 4)
+                        if (j < half_cols) __stcg(mine + j / 4 * kGemmFoldThreads, make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]));
+                    __threadfence();
+                    fold_barrier();
+                    if (tid == 0) {
+                        const bool last = atomicAdd(counter, n) + n == p.groups;
+                        if (last) *counter = 0;
+                        ctrl->last_arrival = last ? 1 : 0;
+                        __threadfence();
+                    }
+                    fold_barrier();
+                }
+                if (ctrl->last_arrival) {
+                    // The parts are added in pair order, whoever is last; this pair's own comes back from memory too, which leaves
+                    // the registers free to request a whole part, or half of one, at once.  (Sixteen columns at a time, each a
+                    // trip to L2, cost 8 us a part: N = 5120, M = 256 took 43 us and takes 34.)
+                    __threadfence();
+                    const float* base = p.partials + static_cast<size_t>(rank) * 2 * slot_floats + tid * 4;
+                    if (!kept) {
+                        // a contributor's part of this tile: slot 1 if the tile starts in its range, else slot 0
+                        const float4* src = reinterpret_cast<const float4*>(base + static_cast<size_t>(c_first) * 4 * slot_floats + slot_floats);
+#pragma unroll
+                        for (int j = 0; j < kGemmTileM / 2; j += 4) {
+                            if (j < half_cols) {
+                                const float4 t = __ldcg(src + j / 4 * kGemmFoldThreads);
+                                acc[j] = t.x;
+                                acc[j + 1] = t.y;
+                                acc[j + 2] = t.z;
+                                acc[j + 3] = t.w;
+                            }
+                        }
+                    }
+#pragma unroll 1
+                    for (int o = c_first + 1; o <= c_last; ++o) {
+                        const float4* src = reinterpret_cast<const float4*>(base + static_cast<size_t>(o) * 4 * slot_floats);
+#pragma unroll
+                        for (int c = 0; c < kGemmTileM / 2; c += 64) {
+                            if (c < half_cols) {
+                                float4 t[16];
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) t[j] = __ldcg(src + (c / 4 + j) * kGemmFoldThreads);
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) {
+                                    acc[c + j * 4] += t[j].x;
+                                    acc[c + j * 4 + 1] += t[j].y;
+                                    acc[c + j * 4 + 2] += t[j].z;
+                                    acc[c + j * 4 + 3] += t[j].w;
+                                }
+                            }
+                        }
+                    }
+                }
             }
             if (!split || ctrl->last_arrival) {
                 const float bias = (valid && pj.bias && !p.swiglu) ? pj.bias[row] : 0.f;
-                if (split) __threadfence();
 #pragma unroll
                 for (int c = 0; c < kGemmTileM / 32; ++c) {
                     if (c * 16 < half_cols) {
-                        if (split) {
-                            float sum[16];
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) sum[j] = 0.f;
-                            for (int o = c_first; o <= c_last; ++o) {
-                                if (o == pair) {
-#pragma unroll
-                                    for (int j = 0; j < 16; ++j) sum[j] += acc[c * 16 + j];
-                                } else {
-                                    // a contributor's part of this tile: slot 1 if the tile starts in its range, else slot 0
-                                    const float* src = p.partials +
-                                                       ((static_cast<size_t>(o) * 2 + rank) * 2 + (o == c_first ? 1 : 0)) * kGemmTileN * kGemmTileM +
-                                                       static_cast<size_t>(c) * 16 * kGemmFoldThreads + tid;
-#pragma unroll
-                                    for (int j = 0; j < 16; ++j) sum[j] += __ldcg(src + j * kGemmFoldThreads);
-                                }
-                            }
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) acc[c * 16 + j] = sum[j];
-                        }
                         const int mc = m0 + ch * half_cols + c * 16;
                         OutT* out = static_cast<OutT*>(pj.y) + static_cast<long long>(mc) * pj.ldy + row;
                         if (!p.swiglu) {
-                            if (valid) {
+                            const int live = valid ? p.m - mc : 0;
 #pragma unroll
-                                for (int j = 0; j < 16; ++j, out += pj.ldy)
-                                    if (mc + j < p.m) store_out(out, acc[c * 16 + j] + bias);
-                            }
+                            for (int j = 0; j < 16; ++j, out += pj.ldy)
+                                if (j < live) store_out(out, acc[c * 16 + j] + bias);
                         } else {
-                            // Gate and up of one feature sit in different warps, which trade halves of the 16 columns: the
-                            // gate thread finishes columns 0-7, the up thread 8-15.
-                            float* mine = park + tid * kGemmParkPitch;
-                            const float* theirs = park + (tid ^ 64) * kGemmParkPitch;
+                            // Gate and up of one feature sit sixteen lanes apart, which trade halves of the 16 columns: the gate
+                            // lane finishes columns 0-7, the up lane 8-15.  (Through shared memory, with two barriers per 16
+                            // columns, the trade took 4 us a tile.)
+                            float y[8];  // (all of them before the first store: inside its condition each would wait for the last)
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) mine[j] = up_row ? acc[c * 16 + j] : acc[c * 16 + 8 + j];
-                            fold_barrier();
-                            if (up_row) out += 8 * pj.ldy;
-                            if (valid) {
-#pragma unroll
-                                for (int j = 0; j < 8; ++j, out += pj.ldy) {
-                                    const float g = up_row ? theirs[j] : acc[c * 16 + j], u = up_row ? acc[c * 16 + 8 + j] : theirs[j];
-                                    if (mc + j + (up_row ? 8 : 0) < p.m) store_out(out, (g / (1.0f + expf(-g))) * u);
-                                }
+                            for (int j = 0; j < 8; ++j) {
+                                const float a = acc[c * 16 + j], b = acc[c * 16 + 8 + j];
+                                const float theirs = __shfl_xor_sync(0xffffffffu, up_row ? a : b, 16);
+                                const float g = up_row ? theirs : a, u = up_row ? b : theirs;
+                                y[j] = (g / (1.0f + expf(-g))) * u;
                             }
-                            fold_barrier();
+                            if (up_row) out += 8 * pj.ldy;
+                            const int live = valid ? p.m - mc - (up_row ? 8 : 0) : 0;
+#pragma unroll
+                            for (int j = 0; j < 8; ++j, out += pj.ldy)
+                                if (j < live) store_out(out, y[j]);
                         }
                     }
                 }
@@ -687,7 +722,7 @@ int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num,
     p.counters = counters;
     // One pair per two SMs.  Cutting tiles evens the pairs' work out and costs the exchange of partial sums, about as
     // much as kCutCost groups; a small problem takes fewer pairs (below eight groups each, the pipeline's fill dominates).
-    constexpr long long kCutCost = 10;
+    constexpr long long kCutCost = 16;
     const long long max_pairs = num_sms / 2;
     const long long whole = (tiles + max_pairs - 1) / max_pairs * p.groups;
     long long cut_pairs = p.units / 8;
