@@ -675,9 +675,14 @@ int ensure_chunk_bufs(Dec* d, int rows) {
     const size_t wide = mx(hq * 512, ch), mix = mx(mx(hq * 256, hv * 128), H);
     const size_t per_row = 3 * H + F + wide + ch + hq * 256 + 2 * hkv * 256 + mix + hv * 128 + 2 * hv + 2 * H + H;
     const size_t halves = (per_row + 64) * static_cast<size_t>(rows);
-    if (cb.x) { cudaFree(cb.x); cudaFree(cb.attn_scratch); cudaFree(cb.gdn_scratch); cb = Dec::ChunkBufs(); }
+    if (cb.x) { cudaFree(cb.x); cb = Dec::ChunkBufs(); }
+    // one block: activations, tokens, the attention's and the delta rule's scratch
+    const int positions = (rows + d->batch - 1) / d->batch;  // of every sequence
+    const size_t attn_bytes = xb::attn_tile_scratch_bytes(d->batch, positions, static_cast<int>(hq), static_cast<int>(hkv), d->num_sms);
+    const size_t front = (halves * sizeof(__half) + static_cast<size_t>(rows) * sizeof(long long) + 256 + 255) & ~static_cast<size_t>(255);
+    const size_t attn_end = (front + attn_bytes + 255) & ~static_cast<size_t>(255);
     __half* base = nullptr;
-    if (cudaMalloc(&base, halves * sizeof(__half) + static_cast<size_t>(rows) * sizeof(long long) + 256) != cudaSuccess) {
+    if (cudaMalloc(&base, attn_end + xb::gdn_chunk_scratch_bytes(d->batch, positions, static_cast<int>(hv))) != cudaSuccess) {
         cudaGetLastError();
         return XINFER_ERR_OUT_OF_MEMORY;
     }
@@ -691,20 +696,8 @@ int ensure_chunk_bufs(Dec* d, int rows) {
     cb.qbuf = take(hq * 256); cb.kbuf = take(hkv * 256); cb.vbuf = take(hkv * 256); cb.mix_out = take(mix);
     cb.zbuf = take(hv * 128); cb.bbuf = take(hv); cb.abuf = take(hv); cb.cat = take(2 * H); cb.hprev = take(H);
     cb.tokens = reinterpret_cast<long long*>(base + ((off + 63) & ~static_cast<size_t>(63)));
-    const int positions = (rows + d->batch - 1) / d->batch;  // of every sequence
-    if (cudaMalloc(&cb.attn_scratch, xb::attn_tile_scratch_bytes(d->batch, positions, static_cast<int>(hq), static_cast<int>(hkv), d->num_sms)) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(base);
-        cb = Dec::ChunkBufs();
-        return XINFER_ERR_OUT_OF_MEMORY;
-    }
-    if (cudaMalloc(&cb.gdn_scratch, xb::gdn_chunk_scratch_bytes(d->batch, positions, static_cast<int>(hv))) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(base);
-        cudaFree(cb.attn_scratch);
-        cb = Dec::ChunkBufs();
-        return XINFER_ERR_OUT_OF_MEMORY;
-    }
+    cb.attn_scratch = reinterpret_cast<float*>(reinterpret_cast<char*>(base) + front);
+    cb.gdn_scratch = reinterpret_cast<char*>(base) + attn_end;
     cb.rows = rows;
     return 0;
 }
@@ -948,7 +941,7 @@ void xinfer_spec_decoder_destroy(xinfer_spec_decoder* d) {
     if (d->graph) cudaGraphDestroy(d->graph);
     if (d->plan) xb::tc_plan_delete(d->plan);  // the recorded plan points into this decoder's weights
     if (d->arena) xinfer_arena_destroy(d->arena);
-    if (d->chunk.x) { cudaFree(d->chunk.x); cudaFree(d->chunk.attn_scratch); cudaFree(d->chunk.gdn_scratch); }
+    if (d->chunk.x) cudaFree(d->chunk.x);
     if (d->h_emitted) cudaFreeHost(d->h_emitted);
     if (d->h_emitted_n) cudaFreeHost(d->h_emitted_n);
     delete d;
