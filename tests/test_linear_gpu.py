@@ -345,6 +345,39 @@ def test_prefill_swiglu_and_fused_projections(cuda, M):
         assert rel_err(Ys[i].float().cpu().numpy(), ref) <= 2e-3
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [1024, 5120, 1152])
+@pytest.mark.parametrize("M", [1, 129])
+def test_scales_at_any_two_byte_address(cuda, M, K):
+    """Scales that start one element behind a 16-byte boundary (a view into a packed checkpoint): plain, fused and SwiGLU form
+    give what the same scales give at an aligned address."""
+    N = 384
+    X, Wg, Sg, _ = synth_linear(M, K, N, seed=K)
+    _, Wu, Su, _ = synth_linear(1, K, N, seed=K + 1)
+    Xd, Wgd, Wud = dev(X), dev(Wg), dev(Wu)
+
+    def outputs(lead):
+        def place(S, lead):
+            buf = torch.empty(S.size + 8, dtype=torch.float16, device="cuda")
+            view = buf[lead:lead + S.size].view(S.shape)
+            view.copy_(dev(S))
+            assert view.data_ptr() % 16 == 2 * lead
+            return view
+        got = []
+        for lead_g, lead_u in ((lead, lead), (0, lead)):   # (gate/up: also with only one of the two off the boundary)
+            sg, su = place(Sg, lead_g), place(Su, lead_u)
+            y = [torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda") for _ in range(4)]
+            assert cuda.linear_int4(y[0], Xd, Wgd, sg, None, M, N, K) == 0
+            descs = [{"Y": y[1 + i], "W_int4": w, "scales": s, "bias": None, "N": N} for i, (w, s) in enumerate(((Wgd, sg), (Wud, su)))]
+            assert cuda.linear_int4_fused(Xd, descs, M, K) == 0
+            assert cuda.mlp_gate_up_swiglu_int4(y[3], Xd, Wgd, sg, Wud, su, M, N, K) == 0
+            got += y
+        torch.cuda.synchronize()
+        assert cuda.last_linear_path() == (TC if M <= 32 else GEMM) and cuda.device_status(0) == 0
+        return torch.stack(got)
+    assert torch.equal(outputs(1), outputs(0))
+
+
 # ------------------------------------------------------------------ fused launches at layer shapes
 def test_fused_layer_shapes(cuda):
     K, M = 5120, 32

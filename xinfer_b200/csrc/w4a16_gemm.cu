@@ -92,6 +92,7 @@ struct GemmProj {
     long long ldy;
     int n;           // output features
     int tile0;       // index of its first tile in the launch
+    int scales_vec;  // every row of its scales starts on a 16-byte boundary
 };
 
 struct GemmParams {
@@ -176,11 +177,12 @@ __device__ __forceinline__ void fold_barrier() { asm volatile("bar.sync 1, %0;" 
 __device__ __forceinline__ void store_out(float* y, float v) { *y = v; }
 __device__ __forceinline__ void store_out(__half* y, float v) { *y = __float2half_rn(v); }
 
-// Scales of the groups g .. g + 7 of one weight row (g a multiple of 8; zero behind the last), and on to the next one.
-__device__ __forceinline__ uint4 load_scales(const unsigned short* sp, int g, int groups) {
+// Scales of the groups g .. g + 7 of one weight row (g a multiple of 8; zero behind the last), and on to the next one.  `vec`:
+// the row starts on a 16-byte boundary and has a multiple of eight of them; a caller's scales may lie anywhere.
+__device__ __forceinline__ uint4 load_scales(const unsigned short* sp, int g, int groups, int vec) {
     uint4 q = make_uint4(0, 0, 0, 0);
     if (g >= groups) return q;
-    if ((groups & 7) == 0) return __ldg(reinterpret_cast<const uint4*>(sp + g));
+    if (vec) return __ldg(reinterpret_cast<const uint4*>(sp + g));
     uint32_t h[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) h[j] = g + j < groups ? __ldg(sp + g + j) : 0u;
@@ -434,14 +436,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
 #pragma unroll
             for (int j = 0; j < kGemmTileM / 2; ++j) acc[j] = 0.f;
             // scales eight groups at a time, a block of eight ahead of its use (one group ahead, their latency is the loop's)
-            uint4 q_cur = load_scales(sp, seg_begin & ~7, p.groups), q_next = load_scales(sp, (seg_begin & ~7) + 8, p.groups);
+            uint4 q_cur = load_scales(sp, seg_begin & ~7, p.groups, pj.scales_vec), q_next = load_scales(sp, (seg_begin & ~7) + 8, p.groups, pj.scales_vec);
             for (int j = 0; j < (seg_begin & 7); ++j) shift_scales(q_cur);
             for (; group < seg_end; ++group, ++i) {
                 const float sc = __half2float(__ushort_as_half(static_cast<unsigned short>(q_cur.x & 0xFFFFu)));
                 shift_scales(q_cur);
                 if ((group & 7) == 7) {
                     q_cur = q_next;
-                    q_next = load_scales(sp, group + 9, p.groups);
+                    q_next = load_scales(sp, group + 9, p.groups, pj.scales_vec);
                 }
                 const uint32_t buf = static_cast<uint32_t>(i & (d_bufs - 1));
                 if (dead || !mbar_wait_parked(smem_u32(&ctrl->d_full[buf]), (i >> d_shift) & 1u, ws)) { dead = true; continue; }
@@ -706,6 +708,7 @@ int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num,
         p.proj[i].y = a.y;
         p.proj[i].ldy = a.ldy > 0 ? a.ldy : a.n;
         p.proj[i].n = static_cast<int>(a.n);
+        p.proj[i].scales_vec = p.groups % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.scales) | reinterpret_cast<uintptr_t>(p.proj[i].scales[1])) & 15) == 0;
         p.proj[i].tile0 = static_cast<int>(tiles);
         const int rows = swiglu ? kGemmTileN : 2 * kGemmTileN;  // of a pair
         tiles += (a.n + rows - 1) / rows * p.m_tiles;
