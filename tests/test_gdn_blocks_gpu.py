@@ -71,6 +71,48 @@ def test_delta_rule_blocks(cuda, T, kind):
     assert rel(S_d.cpu().numpy(), S_want) <= 6e-8 * 128 ** 0.5 * (T if kind == "slow decay" else 8) ** 0.5
 
 
+@pytest.mark.parametrize("T", [17, 40])
+@pytest.mark.parametrize("kind", ["1e-4", "1e-5", "small beta", "zero keys", "tiny keys", "large state", "large state, small values"])
+def test_delta_rule_blocks_range(cuda, T, kind):
+    """Magnitudes far from one, head by head: small states and values, keys at and near zero beside large values, states beyond
+    fp16's range, a state that grows from zero by small updates."""
+    import torch
+    hv, hk = 6, 2
+    rng = np.random.default_rng(T)
+    qkv = rng.normal(0, 1, (T, 2 * hk * 128 + hv * 128))
+    k, v = qkv[:, hk * 128:2 * hk * 128], qkv[:, 2 * hk * 128:]
+    z, b, a = (rng.normal(0, 1, (T, n)).astype(np.float16) for n in (hv * 128, hv, hv))
+    size = 0.05
+    if kind in ("1e-4", "1e-5"):
+        size = float(kind)
+        v *= size
+    elif kind == "small beta":
+        b, size = (b - 12).astype(np.float16), 0.0
+    elif kind == "zero keys":
+        k[2::5] = 0
+        v *= 1e4
+    elif kind == "tiny keys":
+        k *= 1e-4
+        v *= 100
+    else:  # (with the strong decay of the other kinds the large state is gone after a few tokens)
+        a, size = (a - 6).astype(np.float16), 1e7
+        if kind == "large state, small values":
+            v *= 1e-3
+    qkv = qkv.astype(np.float16)
+    A_log, dt_bias = (rng.normal(0, 0.5, hv).astype(np.float32) for _ in range(2))
+    norm_w = rng.normal(1, 0.02, 128).astype(np.float32)
+    S = (size * rng.normal(0, 1, (hv, 128, 128))).astype(np.float32)
+    want, S_want = delta_rule_f64(qkv, z, b, a, A_log, dt_bias, norm_w, S, hv, hk)
+    out, S_d = torch.full((T, hv * 128), float("nan"), dtype=torch.float16, device="cuda"), dev(S)
+    assert cuda.recurrent_gated_delta_net(out, dev(qkv), dev(z), dev(b), dev(a), dev(A_log), dev(dt_bias), dev(norm_w), S_d, T, size == 0, hv, hk) == 0
+    torch.cuda.synchronize()
+    got, S_got = out.double().cpu().numpy(), S_d.double().cpu().numpy()
+    # as above, and half a step of fp16's subnormals on every output
+    assert np.linalg.norm(got - want) <= 5e-4 * np.linalg.norm(want) + 2 ** -25 * want.size ** 0.5
+    for h in range(hv):
+        assert np.linalg.norm(S_got[h] - S_want[h]) <= 6e-8 * 128 ** 0.5 * T ** 0.5 * np.linalg.norm(S_want[h]), h
+
+
 @pytest.mark.parametrize("T,C", [(1, 4), (2, 10), (3, 516), (8, 513), (9, 512), (40, 1028)])
 def test_conv1d_spans(cuda, T, C):
     """One and several spans of positions, channel counts with and without vector access, in place, with and without state."""

@@ -918,26 +918,33 @@ __global__ void __cluster_dims__(kGdnSlices, 1, 1) __launch_bounds__(kGdnThreads
 //   S = G_15 S0 + K^T diag(G_15 / G_j) delta
 // which is the same arithmetic, token for token, in another order (the blocked form of the delta rule published as
 // "Parallelizing Linear Transformers with the Delta Rule over Sequence Length", Yang et al. 2024).  What does not involve the
-// state - (I + L)^-1 diag(beta), P, the norms and the decays - is computed for all blocks of all heads at once by
+// state - (I + L)^-1 - I, P, the norms and the decays - is computed for all blocks of all heads at once by
 // gdn_block_kernel, a warp per block; gdn_scan_kernel then walks the blocks.
 //
 // Everything keeps fp32's precision: k and q enter as their raw fp16 values (their norms are row factors), every other
-// operand x as two fp16 values, hi = rn(2^-4 x) and mid = rn(2^11 (2^-4 x - hi)), 22 significant bits and the sign of mid,
-// which is fp32 to its last bit, in the range of +-2^20; the products with mid are summed apart and scaled back.  (With
-// tf32 operands the same kernel ran at a quarter of the rate: mma.sync of that type does 90 multiply-adds per clock and SM.)
+// operand x as two fp16 values, hi = rn(x) and mid = rn(2^11 (x - hi)); the products with mid are summed apart and scaled back.
+// Together they hold x to 2^-24 of itself from 2^-12 upwards and to 2^-36 below, so what is proportional to the state is carried
+// times a power of two f, which a warp chooses for its sixteen value columns: when the largest of f |S| and f beta |v| of the
+// coming block has left [2^-4, 2], f brings it back to [1/2, 1).  The rule enlarges nothing (beta <= 1, |k| <= 1), so f |delta|
+// stays below 32 inside a block and its product with 1 / |k| <= 1000 inside fp16.  (A fixed factor of 2^-4 before: states of
+// 1e-4 were carried to 1e-4 of themselves, a key near zero beside large values or a state above 2^20 gave NaN.  The choice costs 4
+// of the scan's 46 us at 512 tokens.)  What falls by more than 2^12 within sixteen tokens is, in those, held to 2^-36 of where it
+// came from.  delta is (r + ((I + L)^-1 - I) r): the tensor core's sums, which truncate, only get the smaller part.
+// (With tf32 operands the same kernel ran at a quarter of the rate: mma.sync of that type does 90 multiply-adds per clock and SM.)
 // Transposed products (state S^T, with the value columns as the MMA's rows) let a warp keep its 16 x 128 slice of the state
 // in accumulators that are A operands as they stand.
 // Bound by the latency of a block, one warp per scheduler, so nothing that the next block does not wait for stays in the walk:
 // it leaves the raw outputs in fp32, and gdn_norm_kernel does their gated RMSNorm, which spans all columns of a head, for all
 // tokens at once (with a cluster adding up the squares inside the walk the scan took 145 us).
-// 512 tokens, one sequence, 48 heads: 67 us, 1.5 ms through the step's kernel eight tokens a launch, 300 us with
+// 512 tokens, one sequence, 48 heads: 61 us, 1.5 ms through the step's kernel eight tokens a launch, 300 us with
 // gdn_walk_kernel.
 constexpr int kScanBlock = 16, kScanWarps = 2, kScanCols = 16 * kScanWarps, kScanSlices = 128 / kScanCols, kScanPitch = 136;
-constexpr float kSplitDown = 0.0625f, kSplitUp = 16.0f, kMidUp = 2048.0f, kMidDown = 1.0f / 2048.0f;
+constexpr float kMidUp = 2048.0f, kMidDown = 1.0f / 2048.0f;
 struct GdnBlock {                         // one block of one head, written by gdn_block_kernel
-    __half t[2][kScanBlock][kScanBlock];  // (I + L)^-1 diag(beta): rn(x), rn(2^11 (x - hi))
+    __half t[2][kScanBlock][kScanBlock];  // (I + L)^-1 - I: rn(x), rn(2^11 (x - hi))
     __half p[2][kScanBlock][kScanBlock];
-    float4 coef[kScanBlock];              // per token: 16 G_i / |k_i|, 16 G_i / (|q_i| sqrt(128)), G_15 / G_i / |k_i|, G_15
+    float4 coef[kScanBlock];              // per token: beta_i G_i / |k_i|, G_i / (|q_i| sqrt(128)), G_15 / G_i / |k_i|, beta_i
+    float decay, most, pad[2];            // G_15; the largest beta_i |v_i|
 };
 
 __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -945,7 +952,7 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], u
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// Two already scaled values as fp16 pairs hi and mid.
+// Two values as fp16 pairs hi and mid.
 __device__ __forceinline__ void split_f16x2(float x, float y, uint32_t& hi, uint32_t& mid) {
     const __half2 h = __floats2half2_rn(x, y);
     const float2 f = __half22float2(h);
@@ -969,10 +976,13 @@ __device__ __forceinline__ void ldsm4_trans(uint32_t addr, uint32_t (&r)[4]) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
+// The largest of the lanes' values, none of them negative.
+__device__ __forceinline__ float warp_most(float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v))); }
+
 // One warp per (block, value head, sequence).
 __global__ void __launch_bounds__(128) gdn_block_kernel(GdnBlock* blocks, const __half* qkv, const __half* bb, const __half* aa,
                                                         const float* A_log, const float* dt_bias, int rc, int hv, int hk) {
-    griddep_prologue();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float sh_l[4][kScanBlock][kScanBlock + 1];
     __shared__ float sh_lg[4][kScanBlock], sh_ik[4][kScanBlock], sh_iq[4][kScanBlock], sh_beta[4][kScanBlock];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -992,6 +1002,16 @@ __global__ void __launch_bounds__(128) gdn_block_kernel(GdnBlock* blocks, const 
         live[r] = p < rc;
         q_row[r] = qkv + (seq0 + (live[r] ? p : p0)) * channels + h_k * 128;
         k_row[r] = q_row[r] + hk * 128;
+    }
+    // the largest |v| of eight values of rows 2u + lane / 16
+    float v_most[kScanBlock / 2];
+#pragma unroll
+    for (int u = 0; u < kScanBlock / 2; ++u) {
+        const int p = p0 + 2 * u + (lane >> 4);
+        const uint4 v = *reinterpret_cast<const uint4*>(qkv + (seq0 + (p < rc ? p : p0)) * channels + 2 * hk * 128 + h * 128 + (lane & 15) * 8);
+        const __half2* v2 = reinterpret_cast<const __half2*>(&v);
+        const __half2 m = __hmax2(__hmax2(__habs2(v2[0]), __habs2(v2[1])), __hmax2(__habs2(v2[2]), __habs2(v2[3])));
+        v_most[u] = fminf(fmaxf(__low2float(m), __high2float(m)), 65504.f);  // (an infinity takes only its own column along)
     }
     float kk[2][4] = {}, qk[2][4] = {}, k_sq[2] = {0.f, 0.f}, q_sq[2] = {0.f, 0.f};
 #pragma unroll
@@ -1087,15 +1107,27 @@ __global__ void __launch_bounds__(128) gdn_block_kernel(GdnBlock* blocks, const 
         const float bj = sh_beta[warp][j];
 #pragma unroll
         for (int i = 0; i < kScanBlock; ++i) {
-            const float v = x[i] * bj;
+            const float v = i > j ? x[i] : 0.f;
             const __half hi = __float2half_rn(v);
             out.t[0][i][j] = hi;
             out.t[1][i][j] = __float2half_rn((v - __half2float(hi)) * kMidUp);
         }
         const float gj = expf(prefix);
-        out.coef[j] = make_float4(kSplitUp * gj * sh_ik[warp][j], kSplitUp * gj * sh_iq[warp][j], expf(suffix) * sh_ik[warp][j],
-                                  expf(prefix + suffix));
+        out.coef[j] = make_float4(bj * gj * sh_ik[warp][j], gj * sh_iq[warp][j], expf(suffix) * sh_ik[warp][j], bj);
+        if (lane == 0) out.decay = expf(prefix + suffix);
     }
+    // the largest beta |v|: sixteen lanes a row
+    float most = 0.f;
+#pragma unroll
+    for (int u = 0; u < kScanBlock / 2; ++u) {
+        const int i = 2 * u + (lane >> 4);
+        most = fmaxf(most, sh_beta[warp][i] * v_most[u]);  // (beta is 0 behind the end)
+    }
+    most = warp_most(most);
+    if (lane == 0) out.most = most;
+    // Only now: CTAs of the scan that are placed between this kernel's end up two and three on one SM beside empty ones, and the
+    // fullest SM sets the scan's time (128 tokens: 38 us for the three launches with the signal at the front, 25 with it here).
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 __global__ void __launch_bounds__(32 * kScanWarps) gdn_scan_kernel(float* raw, const __half* qkv, const GdnBlock* blocks, float* state,
@@ -1145,12 +1177,19 @@ __global__ void __launch_bounds__(32 * kScanWarps) gdn_scan_kernel(float* raw, c
     };
     stage(0);
 
-    float s[16][4];  // 2^-4 S^T: s[n][e] = 2^-4 S[8n + 2t + (e & 1)][c0 + 8 (e >> 1)]
+    float s[16][4];  // f S^T: s[n][e] = f S[8n + 2t + (e & 1)][c0 + 8 (e >> 1)]
+    float f = 1.f, inv_f = 1.f;  // powers of two
+    float most = blk[0].most;       // the largest of f |S| and f beta |v|
+
 #pragma unroll
     for (int n = 0; n < 16; ++n) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[n][e] = zero_state ? 0.f : kSplitDown * S[(8 * n + 2 * t + (e & 1)) * 128 + c0 + 8 * (e >> 1)];
+        for (int e = 0; e < 4; ++e) {
+            s[n][e] = zero_state ? 0.f : S[(8 * n + 2 * t + (e & 1)) * 128 + c0 + 8 * (e >> 1)];
+            most = fmaxf(most, fabsf(s[n][e]));
+        }
     }
+    most = warp_most(most);
     // ldmatrix addresses: [token][state row] tiles, (token halves) x (row halves), plain and transposed
     const uint32_t lm_row = static_cast<uint32_t>(((lane >> 4) & 1) * 8 + (lane & 7)), lm_col = static_cast<uint32_t>(((lane >> 3) & 1) * 8);
     const uint32_t lt_row = static_cast<uint32_t>(((lane >> 3) & 1) * 8 + (lane & 7)), lt_col = static_cast<uint32_t>(((lane >> 4) & 1) * 8);
@@ -1161,6 +1200,21 @@ __global__ void __launch_bounds__(32 * kScanWarps) gdn_scan_kernel(float* raw, c
         __syncthreads();
         if (n + 1 < nblocks) stage(n + 1);
         const GdnBlock& here = sh_blk[buf];
+        if ((most > 2.0f && most < INFINITY) || (most < 0.0625f && most > 0.f)) {  // (the same for the warp)
+            int step = 126 - static_cast<int>(__float_as_uint(most) >> 23);
+            const int now = static_cast<int>(__float_as_uint(f) >> 23) - 127;  // (f stays within 2^-100 .. 2^100)
+            step = now + step > 100 ? 100 - now : (now + step < -100 ? -100 - now : step);
+            const float by = __uint_as_float(static_cast<uint32_t>(127 + step) << 23);
+            f *= by;
+            inv_f *= __uint_as_float(static_cast<uint32_t>(127 - step) << 23);
+#pragma unroll
+            for (int m = 0; m < 16; ++m) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[m][e] *= by;
+            }
+        }
+        most = n + 1 < nblocks ? f * blk[n + 1].most : 0.f;
+        float s_most[2] = {0.f, 0.f};
 
         // (K S0)^T and (Q S0)^T: 16 value columns x 16 tokens, contraction over the 128 state rows
         float ks[2][2][4] = {}, qs[2][2][4] = {};  // [hi, mid][token tile]
@@ -1179,15 +1233,15 @@ __global__ void __launch_bounds__(32 * kScanWarps) gdn_scan_kernel(float* raw, c
                 mma_f16(qs[1][nt], mid, qb[2 * nt], qb[2 * nt + 1]);
             }
         }
-        float v[2][4];  // the thread's two columns, tokens 8 (i / 2) + 2t + i % 2
+        float v[2][4];  // f beta v of the thread's two columns, tokens 8 (i / 2) + 2t + i % 2
         float4 coef[4];
         uint32_t tm[2][2][2], pm[2][2][2];  // [hi, mid][i tile][j half]
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int j = 8 * (i >> 1) + 2 * t + (i & 1);
-            v[0][i] = __half2float(sh_v[buf][j][warp * 16 + g]);
-            v[1][i] = __half2float(sh_v[buf][j][warp * 16 + g + 8]);
             coef[i] = here.coef[j];
+            v[0][i] = f * coef[i].w * __half2float(sh_v[buf][j][warp * 16 + g]);
+            v[1][i] = f * coef[i].w * __half2float(sh_v[buf][j][warp * 16 + g + 8]);
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -1195,16 +1249,16 @@ __global__ void __launch_bounds__(32 * kScanWarps) gdn_scan_kernel(float* raw, c
             tm[w][it][jh] = *reinterpret_cast<const uint32_t*>(&here.t[w][it * 8 + g][jh * 8 + 2 * t]);
             pm[w][it][jh] = *reinterpret_cast<const uint32_t*>(&here.p[w][it * 8 + g][jh * 8 + 2 * t]);
         }
-        // 2^-4 delta^T = (2^-4 (V - diag(G / |k|) K S0))^T T^T
+        // f delta^T = (f diag(beta) (V - diag(G / |k|) K S0))^T T^T
         float delta[2][4] = {}, acc[2][4] = {}, u[2][4];
+        float r[2][4];
         uint32_t ahi[4], amid[4];
         {
-            float r[2][4];
 #pragma unroll
             for (int jt = 0; jt < 2; ++jt) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    r[jt][e] = kSplitDown * (v[e >> 1][jt * 2 + (e & 1)] - coef[jt * 2 + (e & 1)].x * (ks[0][jt][e] + kMidDown * ks[1][jt][e]));
+                    r[jt][e] = v[e >> 1][jt * 2 + (e & 1)] - coef[jt * 2 + (e & 1)].x * (ks[0][jt][e] + kMidDown * ks[1][jt][e]);
             }
             split_frag(r[0], r[1], ahi, amid);
         }
@@ -1218,7 +1272,7 @@ __global__ void __launch_bounds__(32 * kScanWarps) gdn_scan_kernel(float* raw, c
         for (int jt = 0; jt < 2; ++jt) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                delta[jt][e] += kMidDown * acc[jt][e];
+                delta[jt][e] = r[jt][e] + (delta[jt][e] + kMidDown * acc[jt][e]);
                 u[jt][e] = delta[jt][e] * coef[jt * 2 + (e & 1)].z;
                 acc[jt][e] = 0.f;
             }
@@ -1233,7 +1287,7 @@ __global__ void __launch_bounds__(32 * kScanWarps) gdn_scan_kernel(float* raw, c
             mma_f16(acc[it], amid, pm[0][it][0], pm[0][it][1]);
         }
         // S^T = G_15 S^T + (diag(G_15 / G_j / |k_j|) delta)^T K
-        const float ge = coef[0].w;
+        const float ge = here.decay;
         const uint32_t kt_base = smem_u32(&sh_k[buf][lt_row][lt_col]);
         split_frag(u[0], u[1], ahi, amid);
 #pragma unroll
@@ -1249,15 +1303,19 @@ __global__ void __launch_bounds__(32 * kScanWarps) gdn_scan_kernel(float* raw, c
                 mma_f16(sn, ahi, kb[2 * nt], kb[2 * nt + 1]);
                 mma_f16(low, amid, kb[2 * nt], kb[2 * nt + 1]);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) sn[e] = fmaf(low[e], kMidDown, sn[e]);
+                for (int e = 0; e < 4; ++e) {
+                    sn[e] = fmaf(low[e], kMidDown, sn[e]);
+                    s_most[nt] = fmaxf(s_most[nt], fabsf(sn[e]));
+                }
             }
         }
+        most = warp_most(fmaxf(fmaxf(s_most[0], s_most[1]), most));
 #pragma unroll
         for (int jt = 0; jt < 2; ++jt) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int p = n * kScanBlock + 8 * jt + 2 * t + (e & 1);
-                const float o = coef[jt * 2 + (e & 1)].y * (qs[0][jt][e] + kMidDown * qs[1][jt][e]) + kSplitUp * (od[jt][e] + kMidDown * acc[jt][e]);
+                const float o = inv_f * (coef[jt * 2 + (e & 1)].y * (qs[0][jt][e] + kMidDown * qs[1][jt][e]) + (od[jt][e] + kMidDown * acc[jt][e]));
                 if (p < rc) raw[((seq0 + p) * hv + h) * 128 + c0 + 8 * (e >> 1)] = o;
             }
         }
@@ -1265,7 +1323,7 @@ __global__ void __launch_bounds__(32 * kScanWarps) gdn_scan_kernel(float* raw, c
 #pragma unroll
     for (int n = 0; n < 16; ++n) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[(8 * n + 2 * t + (e & 1)) * 128 + c0 + 8 * (e >> 1)] = kSplitUp * s[n][e];
+        for (int e = 0; e < 4; ++e) S[(8 * n + 2 * t + (e & 1)) * 128 + c0 + 8 * (e >> 1)] = inv_f * s[n][e];
     }
 }
 
