@@ -31,3 +31,39 @@ def test_step_forms_match_oracle(batch, k, v_heads, k_heads):
             overrides.append(cont)
         assert compare_step(dec, model, seqs, shape_cfg, overrides, tag=f"keep{keep}") == [keep] * batch
     dec.close()
+
+
+@pytest.mark.parametrize("batch,k", [(1, 7), (3, 4)])
+def test_drafts_across_a_key_block(batch, k):
+    """The head's context length grows with every draft and here passes a multiple of 64 keys inside a step, on a model so small
+    that several launches of a draft pass are on the GPU at once: eager and replayed steps give the same drafts, logits and
+    hidden rows, and the eager ones the oracle's."""
+    from xinfer_b200.spec import Shape, SpecDecoder
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    shape_cfg = Shape(hidden_size=512, intermediate_size=512, num_hidden_layers=4, num_attention_heads=4, num_key_value_heads=2,
+                      vocab_size=2048, linear_num_v_heads=6, linear_num_k_heads=2)
+    dec = SpecDecoder(shape_cfg, batch=batch, k=k, max_seq=256, seed=3)
+    dec.reset(59, seed=8)
+    model = pull_model(dec, shape_cfg, k)
+    seqs = pull_state(dec, model, shape_cfg, batch, dec.max_seq)
+    for i in range(3):
+        compare_step(dec, model, seqs, shape_cfg, tag=f"step{i}")
+
+    def run(graph):
+        dec.reset(59, seed=8)
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            if graph:
+                dec.capture(stream)        # (one eager step, then the capture)
+            else:
+                dec.step()
+            got = [dec.results()]
+            for _ in range(12):
+                dec.step()
+                got.append(dec.results())
+        torch.cuda.synchronize()
+        return got
+    for (e0, n0), (e1, n1) in zip(run(False), run(True)):
+        assert np.array_equal(e0, e1) and np.array_equal(n0, n1)
+    dec.close()

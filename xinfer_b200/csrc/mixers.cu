@@ -373,9 +373,8 @@ __global__ void __launch_bounds__(256) attn_prep_rows_kernel(__half* q_out, __ha
 __global__ void conv1d_spec_kernel(__half* out, const __half* in, const float* conv_w, float* state, float* pending,
                                    const int* n_commit, int rows_per_seq, int prev_rows, int channels, int nc_base,
                                    int early_state) {
-    // state, pending inputs and weights do not depend on the kernel in front of this one: they are read, and the
-    // committed state written, before waiting for it (only `in` comes from that kernel).  early_state = 0: the
-    // caller's previous launch wrote them, so everything waits.
+    // early_state: state, pending inputs and weights are read, and the committed state written, before waiting for the kernel
+    // in front of this one, from which only `in` comes (mixers.h says when that is sound).  0: everything waits.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (!early_state) asm volatile("griddepcontrol.wait;" ::: "memory");
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -467,11 +466,9 @@ __global__ void __launch_bounds__(128 * PARTS, PARTS == 2 ? (TOKENS <= 4 ? 3 : 2
     __half* out, const __half* qkv, const __half* z, const __half* bb, const __half* aa, const float* A_log,
     const float* dt_bias, const float* norm_w, float* state, float* pend_k, float* pend_d, float* pend_g,
     const int* n_commit, int rows_per_seq, int prev_rows, int hv, int hk, int nc_base, int early_state, int perm_out) {
-    // The recurrent state, the previous step's pending updates and the per-head constants were written many
-    // launches ago (by this layer's kernel of the previous pass, and by the commit at the end of the previous step):
-    // they are requested BEFORE waiting for the kernel in front of this one.  Only q/k/v/z/b/a come from it.
-    // (early_state = 0: the caller's previous launch wrote the state - the stand-alone op entry point
-    // chaining chunks of one sequence - so everything waits.)
+    // early_state: the recurrent state, the previous step's pending updates and the per-head constants (written by this layer's
+    // kernel of the previous pass, and by the commit at the end of the previous step) are requested BEFORE waiting for the
+    // kernel in front of this one, from which only q/k/v/z/b/a come (mixers.h says when that is sound).  0: everything waits.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (!early_state) asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int kRows = 128 / PARTS, kThreads = 128 * PARTS, kWarps = 4 * PARTS;
@@ -1379,9 +1376,12 @@ __global__ void spec_commit_kernel(const AcceptRec* rec, const long long* draft_
     for (int d = threadIdx.x; d < hidden; d += blockDim.x) h_last[static_cast<long long>(b) * hidden + d] = src[d];
 }
 
-// rows of the verify pass: row (b, 0) = current token, rows (b, 1..k) = draft tokens
+// rows of the verify pass: row (b, 0) = current token, rows (b, 1..k) = draft tokens.  Signals its dependents only after its own
+// wait: everything in front of it is complete before a launch of the verify pass starts, which reads the step before's context
+// lengths, keys and states ahead of its own wait (mixers.h).
 __global__ void build_verify_tokens_kernel(long long* out, const long long* cur_tok, const long long* draft, int k) {
-    griddep_prologue();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int b = blockIdx.x, i = threadIdx.x;
     if (i == 0) out[b * (k + 1)] = cur_tok[b];
     else if (i <= k) out[b * (k + 1) + i] = draft[b * k + i - 1];

@@ -59,7 +59,7 @@ struct AttnTiles {
     long long cache_rows = 0, cache_stride = 0;
     float scale = 1.f;
     int perm_out = 0;                  // see perm_out of rmsnorm_rows
-    int early = 0;                     // ctx, and the keys below it, were not written by the launch directly in front
+    int early = 0;                     // see below
     float* scratch = nullptr;          // attn_tile_scratch_bytes
 };
 size_t attn_tile_scratch_bytes(int batch, int rows_per_seq, int hq, int hkv, int num_sms);
@@ -70,6 +70,12 @@ int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status);
 // nc_base of them).  rows_per_seq = 0 only commits.  early_state = 1 (both kernels): state, pending updates and
 // weights were NOT written by the launch directly in front of this one in the stream, so the kernel may fetch
 // them while that launch is still running (programmatic dependent launch).
+//
+// early / early_state: the kernel reads its context lengths and the keys below them, or its state, pending updates and n_commit
+// (conv1d_spec also writes its state), before it waits for the launch in front of it.  Kernels of the step signal their
+// dependents first and wait afterwards, so several launches may be under way at once, and "some launches ago" says nothing.
+// What is read early must have been written before a launch of this stream that signals only after its own wait
+// (build_verify_tokens; any launch or copy outside programmatic dependent launch), with that launch in front of this one.
 int conv1d_spec(cudaStream_t s, __half* out, const __half* in, const float* conv_w, float* state, float* pending,
                 const int* n_commit, int batch, int rows_per_seq, int prev_rows, int channels, int nc_base = 0,
                 int early_state = 0);

@@ -510,7 +510,9 @@ int layer_forward(Dec* d, cudaStream_t s, Layer& L, int R, __half* xr, const flo
         at.cache_rows = at.cache_stride = d->max_seq;
         at.scale = 1.0f / sqrtf(256.0f);
         at.perm_out = xperm_on();
-        at.early = 1;  // the context lengths and the keys below them were there before this layer's projections ran
+        // The verify pass: lengths and keys are the step before's, and build_verify_tokens stands in front.  A draft pass counts its
+        // lengths itself, a few launches ahead of this one, and its newest keys are the pass before's.
+        at.early = ctx == d->ctx;
         at.scratch = d->attn_scratch;
         NL(xb::attn_tiles(s, at, d->num_sms, d->status));
         d->launches_per_step += 3;
