@@ -44,7 +44,8 @@ XINFER_EXPORT int xinfer_b200_init(int device);
 XINFER_EXPORT int xinfer_b200_init_current(void); /* the same for the calling thread's current device */
 /* 0 when no bounded device-side wait has given up on `device` since the last call, else
  * XINFER_ERR_DEVICE_TIMEOUT.  Covers every entry point, xinfer_linear_int4_f16f16_noalloc included; reading
- * clears the record.  The output of a launch that reported a timeout is undefined. */
+ * clears the record, after waiting for the device, and makes the next launches sound again.  The output of a launch that
+ * reported a timeout, and of launches between it and this call, is undefined. */
 XINFER_EXPORT int xinfer_device_status(int device);
 XINFER_EXPORT const char* xinfer_last_cuda_error(void);
 XINFER_EXPORT const char* xinfer_b200_version(void);

@@ -500,3 +500,34 @@ def test_prefill_gemm_wait_runs_out_and_is_reported(cuda):
     assert cuda.device_status(0) == 0
     again, _ = run_linear(cuda, X, W, S, out_dtype=torch.float16, path=GEMM)
     assert np.array_equal(again, good)
+
+
+def test_cut_tiles_after_a_timeout(cuda):
+    """A GEMM whose tiles are cut between CTAs gives up after some of its parts have been counted.  Once the status has been
+    read, the next cut GEMM and the next stream-K linear of the decode kernel are right again."""
+    from xinfer_b200 import _lib
+    M, K, N = 512, 5120, 5120
+    X, W, S, _ = synth_linear(M, K, N, seed=4)
+    Xd, Wd, Sd = dev(X), dev(W), dev(S)
+    wide = synth_linear(4, 512, 40000, seed=5)
+
+    def both():
+        y = torch.full((M, N), float("nan"), device="cuda")
+        assert cuda.linear_int4(y, Xd, Wd, Sd, None, M, N, K) == 0
+        torch.cuda.synchronize()
+        assert cuda.last_linear_path() == GEMM
+        return y, run_linear(cuda, *wide[:3])[0]
+    good = both()
+    assert cuda.device_status(0) == 0
+    for stage in (3, 12, 20):                # (of the 21 or 22 groups of a pair)
+        cuda.set_wait_hooks(8_000_000, stage)
+        try:
+            y = torch.empty((M, N), device="cuda")
+            assert cuda.linear_int4(y, Xd, Wd, Sd, None, M, N, K) == 0
+            torch.cuda.synchronize()
+        finally:
+            cuda.set_wait_hooks(0, -1)
+        assert cuda.device_status(0) == _lib.ERR_DEVICE_TIMEOUT
+        again = both()
+        assert cuda.device_status(0) == 0
+        assert torch.equal(again[0], good[0]) and np.array_equal(again[1], good[1])

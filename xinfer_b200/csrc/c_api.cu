@@ -255,7 +255,13 @@ int xinfer_device_status(int device) {
     cudaError_t e = cudaSuccess;
     if (g_ctx[device].ready) {
         e = cudaMemcpy(&v, g_ctx[device].status, sizeof(int), cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess && v != 0) cudaMemset(g_ctx[device].status, 0, sizeof(int));
+        if (e == cudaSuccess && v != 0) {
+            // a launch that gave up may have left tiles half counted: the counters are zeroed with the record, and the device is
+            // idle meanwhile (the caller's streams need not order themselves with these copies)
+            if ((e = cudaDeviceSynchronize()) == cudaSuccess) e = cudaMemset(g_ctx[device].counters, 0, (kCounterCapacity + 1) * sizeof(int));
+            if (e == cudaSuccess) e = cudaMemset(g_ctx[device].status, 0, sizeof(int));
+            if (e == cudaSuccess) e = cudaDeviceSynchronize();
+        }
     }
     // the allocation-free entry point keeps its own status word (in its in-library array)
     const int v2 = xb::tc_noalloc_take_status(device);
