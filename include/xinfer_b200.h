@@ -53,10 +53,10 @@ XINFER_EXPORT const char* xinfer_b200_version(void);
  * kernel), 2 CUDA cores (fp32 activations, odd shapes), 3 tcgen05 GEMM (M > 32: prefill chunks through the same entry
  * points, forward_prefill_chunk of src/targets/qwen3_8/forward.cpp:402-554). */
 XINFER_EXPORT int xinfer_last_linear_path(void);
-/* Test hook for the bounded device-side waits of the tcgen05 linear kernel.  limit_clocks: SM clocks after
- * which a wait gives up (<= 0 restores the default, about one second).  withhold_x_from_stage >= 0: the
- * kernel's loader never requests the activation stages from that index on, so the waits for them run out,
- * the kernel returns through its abort path and xinfer_device_status reports the timeout (-1: off).
+/* Test hook for the bounded device-side waits of the tcgen05 kernels.  limit_clocks: SM clocks after
+ * which a wait gives up (<= 0 restores the default, about one second).  withhold_x_from_stage >= 0: a
+ * linear's loader never requests the activation stages from that index on, the attention's never its queries, so
+ * the waits for them run out, the kernel returns through its abort path and xinfer_device_status reports the timeout (-1: off).
  * Process-wide; applies to launches enqueued afterwards.  No counterpart in the reference. */
 XINFER_EXPORT void xinfer_debug_set_wait_hooks(int64_t limit_clocks, int withhold_x_from_stage);
 /* Force a kernel family for the linear entry points on the current device: 0 = automatic (fp16 activations: the

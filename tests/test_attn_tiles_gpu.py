@@ -42,3 +42,32 @@ def test_attention_tiles(hq, hkv, T, start, amp):
         assert ((got - want).norm() / want.norm()).item() <= 2 * 2 ** -11
         rms = want.pow(2).mean().sqrt()
         assert ((got - want).abs() / torch.maximum(want.abs(), rms)).max().item() <= 8 * 2 ** -11
+
+
+@pytest.mark.parametrize("T,start", [(1, 3000), (200, 333)])
+def test_attention_wait_runs_out_and_is_reported(T, start):
+    """The loader withholds the queries: the launch comes back, the merge behind it stays inside its buffers although the table of
+    parts was not written, the status reports it once, and the next call is right."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    import xinfer_b200.ops as ops
+    from xinfer_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(T)
+    q = torch.randn((T, 24, 256), generator=g, device="cuda").half()
+    k, v = (torch.randn((start + T, 4, 256), generator=g, device="cuda").half() for _ in range(2))
+
+    def call():
+        out = torch.full((T, 24, 256), float("nan"), device="cuda", dtype=torch.float16)
+        assert ops.sdpa_causal_cached(out, q, k, v, start, T, 24, 4, 256) == 0
+        torch.cuda.synchronize()
+        return out
+    good = call()
+    ops.set_wait_hooks(8_000_000, 0)           # about 4 ms
+    try:
+        call()
+    finally:
+        ops.set_wait_hooks(0, -1)
+    assert ops.device_status(0) == _lib.ERR_DEVICE_TIMEOUT
+    assert torch.equal(call(), good)
+    assert ops.device_status(0) == 0

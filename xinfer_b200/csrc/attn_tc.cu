@@ -85,6 +85,7 @@ struct TileParams {
     float *part_o, *part_ml;  // [CTA][2][row][256], [CTA][2][row][max, sum]
     int2* table;            // [items] first and last group at work on every item
     long long wait_limit;
+    int withhold;           // test hook: the queries are never requested
     int* status;
 };
 
@@ -332,7 +333,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
                 if (j == 0 && keys) {
                     ok = run == 0 || warp_wait_parked(&ctrl->q_empty, (run & 1u) ^ 1u, ws);
                     if (!ok) break;
-                    if (leader) {
+                    if (leader && !p.withhold) {
                         const int b = walk.item / sh.tiles;
                         const uint32_t bar = smem_u32(&ctrl->q_full);
                         mbar_arrive_expect_tx(bar, static_cast<uint32_t>(rows) * kDim * 2);
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
                             tma_load_4d(smem_u32(q_smem) + d * q_block, &p.q_map, bar, d * 64, kvh * sh.group, walk.item % sh.tiles * sh.tile_pos, b, pol_q);
                     }
                     __syncwarp();
-                    ++nq;
+                    nq += !p.withhold;
                 }
             }
             walk.advance();
@@ -554,11 +555,12 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
 }
 
 // Merges the parts of the items that were cut.  A warp takes every kWarpsPerRow-th part of a row, eight dims per lane; grid
-// (items * Hkv, row blocks).  A row of few long sequences has up to one part per group (37 at one sequence): eight warps, a row
+// (items * Hkv, row blocks).  What the table says is kept inside the `groups` of the launch in front: one that gave up has not
+// written all of it.  A row of few long sequences has up to one part per group (37 at one sequence): eight warps, a row
 // a block (8192 keys, one row: 4 us, 8 with a warp a row).  Otherwise there are a few parts and many rows: a warp each.
 template <int kWarpsPerRow>
 __global__ void __launch_bounds__(256, 4) attn_tile_combine_kernel(__half* out, const float* part_o, const float* part_ml, const int2* table,
-                                                                   const __half* q_gate, const TileShape sh, int perm_out, int out_vec) {
+                                                                   const __half* q_gate, const TileShape sh, int groups, int perm_out, int out_vec) {
     griddep_prologue();
     constexpr int kBatch = 4;  // parts whose loads are in flight together
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = warp % kWarpsPerRow;
@@ -570,7 +572,7 @@ __global__ void __launch_bounds__(256, 4) attn_tile_combine_kernel(__half* out, 
     const bool gated = q_gate && r < rows && pos < sh.rows_per_seq && sub == 0;
     uint4 gate = make_uint4(0, 0, 0, 0);  // (asked for here: its way from memory is the parts')
     if (gated) gate = __ldg(reinterpret_cast<const uint4*>(q_gate + at * 512 + 256 + lane * 8));
-    const int c0 = who.x, c1 = who.y;
+    const int c0 = min(max(who.x, 0), groups - 1), c1 = min(max(who.y, c0), groups - 1);
     if (c0 == c1 || r >= rows || pos >= sh.rows_per_seq) return;  // (the same for all warps of a row)
     auto slot = [&](int c) { return ((static_cast<size_t>(c) * sh.hkv + kvh) * 2 + (c == c0 ? 1 : 0)) * rows + r; };
     float m = -INFINITY, l = 0.f, acc[8] = {};
@@ -722,6 +724,7 @@ int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status) {
     p.part_ml = a.scratch + static_cast<size_t>(ctas) * 2 * d.rows * kDim;
     p.table = reinterpret_cast<int2*>(p.part_ml + static_cast<size_t>(ctas) * 2 * d.rows * 2);
     p.wait_limit = tc_wait_limit();
+    p.withhold = tc_x_stage_limit() >= 0;
     p.status = status;
     {
         static bool configured[64];
@@ -741,7 +744,7 @@ int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status) {
     const bool wide = d.tiles == 1 && ctas >= 8 * a.batch * a.hkv;  // eight parts a row
     if (launch_pdl(wide ? attn_tile_combine_kernel<8> : attn_tile_combine_kernel<1>, dim3(p.sh.items * a.hkv, wide ? d.rows : (d.rows + 7) / 8),
                    dim3(256), 0, s, a.out, static_cast<const float*>(p.part_o), static_cast<const float*>(p.part_ml),
-                   static_cast<const int2*>(p.table), a.q_gate, p.sh, a.perm_out, p.out_vec) != cudaSuccess)
+                   static_cast<const int2*>(p.table), a.q_gate, p.sh, ctas / a.hkv, a.perm_out, p.out_vec) != cudaSuccess)
         return -1;
     return 0;
 }

@@ -34,7 +34,7 @@ void tc_set_wait_hooks(long long limit_clocks, int withhold_x_from_stage);
 // Status word of the allocation-free entry point on `device` (which must be current): read and cleared.
 int tc_noalloc_take_status(int device);
 long long tc_wait_limit();  // clocks after which a device-side wait gives up (tc_set_wait_hooks)
-int tc_x_stage_limit();     // test hook of tc_set_wait_hooks: first activation stage that is never requested (-1: off)
+int tc_x_stage_limit();     // test hook of tc_set_wait_hooks: first activation stage that is never requested (-1: off; for the attention, its queries)
 
 // Dense GEMM for more than 32 activation rows (prefill chunks) on tcgen05, both operands from shared memory
 // (w4a16_gemm.cu).  One launch for all projections that share X; gate and up of the fused MLP are one pair.
