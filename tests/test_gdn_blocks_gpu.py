@@ -71,6 +71,27 @@ def test_delta_rule_blocks(cuda, T, kind):
     assert rel(S_d.cpu().numpy(), S_want) <= 6e-8 * 128 ** 0.5 * (T if kind == "slow decay" else 8) ** 0.5
 
 
+@pytest.mark.parametrize("T", [2, 7, 8, 9, 15])
+@pytest.mark.parametrize("zero", [False, True])
+def test_delta_rule_short_calls(cuda, T, zero):
+    """Calls that a single block of the token-by-token kernel covers, none of them full."""
+    import torch
+    hv, hk = 9, 3
+    rng = np.random.default_rng(T)
+    qkv = rng.normal(0, 1, (T, 2 * hk * 128 + hv * 128)).astype(np.float16)
+    z, b, a = (rng.normal(0, 1, (T, n)).astype(np.float16) for n in (hv * 128, hv, hv))
+    A_log, dt_bias = (rng.normal(0, 0.5, hv).astype(np.float32) for _ in range(2))
+    norm_w = rng.normal(1, 0.02, 128).astype(np.float32)
+    S = rng.normal(0, 0.05, (hv, 128, 128)).astype(np.float32)
+    want, S_want = delta_rule_f64(qkv, z, b, a, A_log, dt_bias, norm_w, 0 * S if zero else S, hv, hk)
+    out, S_d = torch.full((T, hv * 128), float("nan"), dtype=torch.float16, device="cuda"), dev(S)
+    assert cuda.recurrent_gated_delta_net(out, dev(qkv), dev(z), dev(b), dev(a), dev(A_log), dev(dt_bias), dev(norm_w), S_d, T, zero, hv, hk) == 0
+    torch.cuda.synchronize()
+    rel = lambda x, y: np.linalg.norm(np.asarray(x, np.float64) - y) / np.linalg.norm(y)  # noqa: E731
+    assert rel(out.float().cpu().numpy(), want) <= 5e-4                       # (the bounds of the longer calls)
+    assert rel(S_d.cpu().numpy(), S_want) <= 6e-8 * 128 ** 0.5 * 8 ** 0.5
+
+
 @pytest.mark.parametrize("T", [17, 40])
 @pytest.mark.parametrize("kind", ["1e-4", "1e-5", "small beta", "zero keys", "tiny keys", "large state", "large state, small values"])
 def test_delta_rule_blocks_range(cuda, T, kind):

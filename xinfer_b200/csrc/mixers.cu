@@ -736,6 +736,7 @@ constexpr int kGdnCols = 16, kGdnBlock = 16, kGdnSlices = 128 / kGdnCols, kGdnTh
 __global__ void __cluster_dims__(kGdnSlices, 1, 1) __launch_bounds__(kGdnThreads) gdn_walk_kernel(
     __half* out, const __half* qkv, const __half* z, const __half* bb, const __half* aa, const float* A_log, const float* dt_bias,
     const float* norm_w, float* state, int rc, int hv, int hk, int zero_state) {
+    cluster_arrive();  // (a CTA may write into another one's shared memory once that one has started)
     griddep_prologue();
     __shared__ __align__(16) float sh_q[2][kGdnBlock][128], sh_k[2][kGdnBlock][128];
     __shared__ float sh_v[2][kGdnBlock][kGdnCols], sh_out[kGdnBlock][kGdnCols + 1];
@@ -885,6 +886,7 @@ __global__ void __cluster_dims__(kGdnSlices, 1, 1) __launch_bounds__(kGdnThreads
         float sq = o0 * o0 + o1 * o1;
 #pragma unroll
         for (int off = 1; off < 8; off <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+        if (n == 0) cluster_wait();
         st_shared_cluster_f32(mapa_shared_cluster(smem_u32(&sh_sq[buf][slice][ot]), tid & 7), sq);
         cluster_arrive();
         if (p0 + kGdnBlock < rc) stage(p0 + kGdnBlock, buf ^ 1);

@@ -566,6 +566,7 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ NucShared sh;
+    cluster_arrive();  // (a CTA may write into another one's shared memory once that one has started)
     const int crank = static_cast<int>(cluster.block_rank());
     const int row = blockIdx.x / kNucCluster, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float* l = logits + static_cast<long long>(row) * row_stride;
@@ -598,6 +599,7 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
     if (lane == 0) sh.wmax[warp] = mx;
     if (tid == 0) sh.count = 0;
     __syncthreads();
+    cluster_wait();
     if (warp == 0) {
         float m = sh.wmax[lane];
 #pragma unroll
