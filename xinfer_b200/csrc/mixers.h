@@ -92,7 +92,7 @@ int conv1d_chunk(cudaStream_t s, __half* out, const __half* in, const float* con
                  int channels);
 int gdn_chunk(cudaStream_t s, __half* out, const __half* qkv, const __half* z, const __half* b, const __half* a,
               const float* A_log, const float* dt_bias, const float* norm_w, float* state, int batch, int rc, int hv, int hk,
-              void* scratch, int zero_state = 0);
+              void* scratch, int num_sms, int zero_state = 0);
 size_t gdn_chunk_scratch_bytes(int batch, int rc, int hv);  // of `scratch`, 16-byte aligned
 // Whether the vector accesses of gdn_chunk fit these pointers.
 bool gdn_chunk_aligned(const void* out, const void* qkv, const void* z, const void* state);

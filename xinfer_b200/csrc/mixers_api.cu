@@ -175,19 +175,22 @@ int xinfer_recurrent_gated_delta_net_f16(xinfer_stream_t s, void* out, const voi
     if (num_v_heads <= 0 || num_k_heads <= 0 || num_v_heads % num_k_heads) return XINFER_ERR_INVALID_ARGUMENT;
     if (!out || !qkv || !z || !b || !a || !A_log || !dt_bias || !norm_weight || !state_buffer) return XINFER_ERR_INVALID_ARGUMENT;
     const int hv = static_cast<int>(num_v_heads), hk = static_cast<int>(num_k_heads);
+    int *status = nullptr, num_sms = 0;
+    int rc = xb::device_facts(&status, &num_sms);
+    if (rc != XINFER_OK) return rc;
     if (xb::gdn_chunk_aligned(out, qkv, z, state_buffer)) {
         // pieces of 1024 rows bound the scratch (32 MB at 48 heads)
         const int64_t piece = 1024, ch = 2 * static_cast<int64_t>(hk) * 128 + static_cast<int64_t>(hv) * 128, vd = static_cast<int64_t>(hv) * 128;
         float* blocks = nullptr;
         const int most = static_cast<int>(seq_len < piece ? seq_len : piece);
-        const int rc = scratch(xb::gdn_chunk_scratch_bytes(1, most, hv), &blocks);
+        rc = scratch(xb::gdn_chunk_scratch_bytes(1, most, hv), &blocks);
         if (rc != XINFER_OK) return rc;
         for (int64_t t0 = 0; t0 < seq_len; t0 += piece) {
             const int rows = static_cast<int>(seq_len - t0 < piece ? seq_len - t0 : piece);
             const int r = xb::gdn_chunk(static_cast<cudaStream_t>(s), static_cast<__half*>(out) + t0 * vd, static_cast<const __half*>(qkv) + t0 * ch,
                                         static_cast<const __half*>(z) + t0 * vd, static_cast<const __half*>(b) + t0 * hv,
                                         static_cast<const __half*>(a) + t0 * hv, A_log, dt_bias, norm_weight, state_buffer, 1, rows, hv, hk,
-                                        blocks, zero_state && t0 == 0);
+                                        blocks, num_sms, zero_state && t0 == 0);
             if (r != 0) return ok_or_cuda(r);
         }
         return XINFER_OK;
@@ -195,9 +198,6 @@ int xinfer_recurrent_gated_delta_net_f16(xinfer_stream_t s, void* out, const voi
     // pointers that the vector accesses of the chunk kernel do not fit: eight tokens a launch through the step's kernel
     const size_t pk = static_cast<size_t>(hv) * 8 * 128;
     float* scr = nullptr;
-    int *status = nullptr, num_sms = 0;
-    int rc = xb::device_facts(&status, &num_sms);
-    if (rc != XINFER_OK) return rc;
     rc = scratch((2 * pk + static_cast<size_t>(hv) * 8) * sizeof(float), &scr);
     if (rc != XINFER_OK) return rc;
     float *pend_k = scr, *pend_d = scr + pk, *pend_g = scr + 2 * pk;

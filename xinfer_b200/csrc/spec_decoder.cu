@@ -757,7 +757,8 @@ int prefill_chunk(Dec* d, cudaStream_t s, const long long* prompt, int64_t T, in
             const xinfer_fused_desc fd[4] = {desc(cb.wide, L.in_qkv), desc(cb.zbuf, L.in_z), desc(cb.bbuf, L.in_b), desc(cb.abuf, L.in_a)};
             LIN(xinfer_linear_int4_fused_f16(st, cb.normed, fd, 4, M, H, 128));
             NL(xb::conv1d_chunk(s, cb.wide2, cb.wide, L.conv_w, L.conv_state, B, Rc, ch));
-            NL(xb::gdn_chunk(s, cb.mix_out, cb.wide2, cb.zbuf, cb.bbuf, cb.abuf, L.A_log, L.dt_bias, L.gdn_norm, L.S, B, Rc, hv, hk, cb.gdn_scratch));
+            NL(xb::gdn_chunk(s, cb.mix_out, cb.wide2, cb.zbuf, cb.bbuf, cb.abuf, L.A_log, L.dt_bias, L.gdn_norm, L.S, B, Rc, hv, hk, cb.gdn_scratch,
+                             d->num_sms));
             LIN(xinfer_linear_int4_f16f16(st, cb.proj_out, cb.mix_out, L.out_proj.w, L.out_proj.s, nullptr, M, L.out_proj.n,
                                           L.out_proj.k, 128));
         }
