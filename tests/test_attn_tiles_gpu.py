@@ -71,3 +71,30 @@ def test_attention_wait_runs_out_and_is_reported(T, start):
     assert ops.device_status(0) == _lib.ERR_DEVICE_TIMEOUT
     assert torch.equal(call(), good)
     assert ops.device_status(0) == 0
+
+
+@pytest.mark.parametrize("hq,hkv,T,start", [(24, 4, 1, 1023), (8, 2, 1, 1099), (24, 4, 5, 3000), (24, 4, 77, 0), (12, 2, 22, 900)])
+def test_attention_repeats_itself(hq, hkv, T, start):
+    """The same call gives the same bits whatever ran in between, and a position the same as in a call without those behind it
+    where both cut the keys alike (one block)."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    import xinfer_b200.ops as ops
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rand = lambda *s: torch.randn(s, generator=g, device="cuda").half()  # noqa: E731
+    q, k, v = 3 * rand(T, hq, 256), rand(start + T, hkv, 256), rand(start + T, hkv, 256)
+
+    def call(q, k, v, T, start):
+        out = torch.full((T, hq, 256), float("nan"), device="cuda", dtype=torch.float16)
+        assert ops.sdpa_causal_cached(out, q, k, v, start, T, hq, hkv, 256) == 0
+        return out
+    first = call(q, k, v, T, start)
+    for i in range(12):
+        for other in (1, 3, 40):  # (other contents of the kernel's shared memory)
+            call((2 + i) * rand(other, hq, 256), (1 + i) * rand(500, hkv, 256), rand(500, hkv, 256), other, 500 - other)
+        assert torch.equal(call(q, k, v, T, start), first), i
+    few = min(T, 5)
+    short = call(q[:few].contiguous(), k, v, few, 20)
+    for t in range(few):
+        assert torch.equal(call(q[t:t + 1].contiguous(), k, v, 1, 20 + t)[0], short[t]), t

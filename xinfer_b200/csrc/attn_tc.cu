@@ -463,10 +463,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
                     mx3 = fmaxf(mx3, __uint_as_float(raw[c + 3]));
                 }
                 const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale2;
-                if (__any_sync(0xffffffffu, mx > m + kLazyRescale || (m == -INFINITY && mx > m))) {
-                    const float m_new = fmaxf(m, mx), alpha = m == -INFINITY ? 0.f : exp2_ftz(m - m_new);
+                // Each row by its own scores: what its neighbours hold, or the rows of S behind the last, which are products of whatever
+                // lies in shared memory there, must not show in its rounding.
+                const bool raise = valid && (mx > m + kLazyRescale || (m == -INFINITY && mx > m));
+                if (__any_sync(0xffffffffu, raise)) {
+                    const float alpha = !raise ? 1.f : (m == -INFINITY ? 0.f : exp2_ftz(m - mx));
                     l *= alpha;
-                    m = m_new;
+                    if (raise) m = mx;
                     if (j > 0) {
                         // O holds the blocks before this one once their products are done
                         if (!warp_wait(&ctrl->pv_done[buf ^ 1u], ((i - 1) >> 1) & 1u, ws)) { ok = false; break; }
