@@ -190,3 +190,37 @@ def test_shape_validation_like_the_reference(cuda):
     with pytest.raises(_lib.XInferError) as e:
         cuda.recurrent_gated_delta_net(None, None, None, None, None, None, None, None, None, 1, False, 32, 5)
     assert e.value.code == _lib.ERR_INVALID_ARGUMENT
+
+
+def test_captured_decode_layer_after_a_long_prompt(cuda):
+    """Attention and delta rule of a single token captured as a graph, then the same ops on a prompt, then the graph again: what it
+    holds of the library's scratch has not moved."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    n = lambda *s: torch.randn(s, generator=g, device="cuda").half()  # noqa: E731
+    hq, hkv, hv, hk, cap, T = 8, 2, 6, 2, 1200, 1100
+    q, kc, vc = n(T, hq, 256), n(cap, hkv, 256), n(cap, hkv, 256)
+    qkv, z, b, a = n(T, 2 * hk * 128 + hv * 128), n(T, hv * 128), n(T, hv), n(T, hv)
+    A_log, dt_bias, norm_w = (torch.randn(i, generator=g, device="cuda") for i in (hv, hv, 128))
+    state0 = torch.randn((hv, 128, 128), generator=g, device="cuda")
+    o1, o2, state = torch.empty(hq * 256, device="cuda").half(), torch.empty(hv * 128, device="cuda").half(), state0.clone()
+
+    def one():
+        assert cuda.sdpa_causal_cached(o1, q, kc, vc, 1099, 1, hq, hkv, 256, max_seq_len=cap) == 0
+        assert cuda.recurrent_gated_delta_net(o2, qkv, z, b, a, A_log, dt_bias, norm_w, state, 1, False, hv, hk) == 0
+    one()
+    torch.cuda.synchronize()
+    want = o1.clone(), o2.clone(), state.clone()
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=stream):
+        one()
+    out, out2 = torch.empty((T, hq * 256), device="cuda").half(), torch.empty((T, hv * 128), device="cuda").half()
+    long_state = state0.clone()
+    assert cuda.sdpa_causal_cached(out, q, kc, vc, 0, T, hq, hkv, 256, max_seq_len=cap) == 0
+    assert cuda.recurrent_gated_delta_net(out2, qkv, z, b, a, A_log, dt_bias, norm_w, long_state, T, False, hv, hk) == 0
+    torch.cuda.synchronize()
+    for x in (o1, o2):
+        x.fill_(float("nan"))
+    state.copy_(state0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, y) for x, y in zip((o1, o2, state), want))

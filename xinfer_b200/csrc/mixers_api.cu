@@ -24,32 +24,41 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 
-// Scratch of the stand-alone entry points, per device, grown on demand (the speculative decoder has its own).
+// Scratch of the stand-alone entry points, a block per device and op (the speculative decoder has its own).  A block is taken at
+// the most that any call with the same heads needs (39 MB for the attention and 32 MB for the delta rule at the 27B shapes): it
+// stays where it is whatever the row counts, so a graph captured around one call stays good when another one has more rows.
+// Only more heads than before move it.
 struct MixerScratch {
     float* buf = nullptr;
     size_t bytes = 0;
 };
-MixerScratch g_scratch[kMaxDevices];
+enum ScratchOf { kAttention, kDelta, kScratches };
+MixerScratch g_scratch[kMaxDevices][kScratches];
 std::mutex g_mu;
 
-int scratch(size_t bytes, float** out) {
+// `bytes`: what this call needs; `most`: what any call with these heads needs.
+int scratch(ScratchOf which, size_t bytes, size_t most, float** out) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return XINFER_ERR_NO_DEVICE;
     std::lock_guard<std::mutex> lock(g_mu);
-    MixerScratch& m = g_scratch[dev];
+    MixerScratch& m = g_scratch[dev][which];
     if (m.bytes < bytes) {
-        // a larger request: the old block may still be in use by work already enqueued, so wait for it first
+        // more heads: the old block may still be in use by work already enqueued, so wait for it first
         if (m.buf) {
             cudaDeviceSynchronize();
             cudaFree(m.buf);
             m.buf = nullptr;
             m.bytes = 0;
         }
-        if (cudaMalloc(reinterpret_cast<void**>(&m.buf), bytes) != cudaSuccess) {
+        for (size_t size : {most, bytes}) {  // (on a full device the call still gets what it needs)
+            if (cudaMalloc(reinterpret_cast<void**>(&m.buf), size) == cudaSuccess) {
+                m.bytes = size;
+                break;
+            }
             cudaGetLastError();
-            return XINFER_ERR_OUT_OF_MEMORY;
+            m.buf = nullptr;
         }
-        m.bytes = bytes;
+        if (!m.buf) return XINFER_ERR_OUT_OF_MEMORY;
     }
     *out = m.buf;
     return XINFER_OK;
@@ -136,9 +145,11 @@ int xinfer_sdpa_causal_cached_f16(xinfer_stream_t s, void* out, const void* Q, c
     // pieces of rows that keep the count of (128-row tile, 64-key block) units of a launch well inside 32 bits
     const int64_t tile_pos = 128 / group, blocks = (start_pos + num_q_tokens) / 64 + 1;
     int64_t piece = (int64_t{1} << 29) / (blocks * hkv) * tile_pos;
-    piece = piece < tile_pos ? tile_pos : (piece < 65536 ? piece : 65536);
+    constexpr int64_t kMostRows = 65536;
+    piece = piece < tile_pos ? tile_pos : (piece < kMostRows ? piece : kMostRows);
     const int most = static_cast<int>(num_q_tokens < piece ? num_q_tokens : piece);
-    rc = scratch(xb::attn_tile_scratch_bytes(1, most, hq, hkv, num_sms), &a.scratch);
+    rc = scratch(kAttention, xb::attn_tile_scratch_bytes(1, most, hq, hkv, num_sms), xb::attn_tile_scratch_bytes(1, kMostRows, hq, hkv, num_sms),
+                 &a.scratch);
     if (rc != XINFER_OK) return rc;
     for (int64_t t0 = 0; t0 < num_q_tokens; t0 += piece) {
         a.rows_per_seq = static_cast<int>(num_q_tokens - t0 < piece ? num_q_tokens - t0 : piece);
@@ -183,7 +194,7 @@ int xinfer_recurrent_gated_delta_net_f16(xinfer_stream_t s, void* out, const voi
         const int64_t piece = 1024, ch = 2 * static_cast<int64_t>(hk) * 128 + static_cast<int64_t>(hv) * 128, vd = static_cast<int64_t>(hv) * 128;
         float* blocks = nullptr;
         const int most = static_cast<int>(seq_len < piece ? seq_len : piece);
-        rc = scratch(xb::gdn_chunk_scratch_bytes(1, most, hv), &blocks);
+        rc = scratch(kDelta, xb::gdn_chunk_scratch_bytes(1, most, hv), xb::gdn_chunk_scratch_bytes(1, static_cast<int>(piece), hv), &blocks);
         if (rc != XINFER_OK) return rc;
         for (int64_t t0 = 0; t0 < seq_len; t0 += piece) {
             const int rows = static_cast<int>(seq_len - t0 < piece ? seq_len - t0 : piece);
@@ -198,7 +209,8 @@ int xinfer_recurrent_gated_delta_net_f16(xinfer_stream_t s, void* out, const voi
     // pointers that the vector accesses of the chunk kernel do not fit: eight tokens a launch through the step's kernel
     const size_t pk = static_cast<size_t>(hv) * 8 * 128;
     float* scr = nullptr;
-    rc = scratch((2 * pk + static_cast<size_t>(hv) * 8) * sizeof(float), &scr);
+    const size_t pending = (2 * pk + static_cast<size_t>(hv) * 8) * sizeof(float);
+    rc = scratch(kDelta, pending, xb::gdn_chunk_scratch_bytes(1, 1024, hv), &scr);
     if (rc != XINFER_OK) return rc;
     float *pend_k = scr, *pend_d = scr + pk, *pend_g = scr + 2 * pk;
     cudaStream_t st = static_cast<cudaStream_t>(s);
