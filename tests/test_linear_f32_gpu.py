@@ -36,3 +36,34 @@ def test_linear_f32(M, K, N):
     assert ops.mlp_gate_up_swiglu_int4(y, x, w, s, w2, s2, M, N, K) == 0
     gate = x.double() @ d.T
     assert rel(y, gate / (1 + torch.exp(-gate)) * (x.double() @ d2.T)) <= 4 * bound
+
+
+def test_linear_f32_carries_infinities_and_nan():
+    """An infinite activation gives infinities of the weights' signs, as fp32 arithmetic does, NaN gives NaN, the largest finite
+    values neither; other rows stay untouched."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    import xinfer_b200.ops as ops
+    M, K, N = 6, 256, 40
+    g = torch.Generator(device="cuda").manual_seed(1)
+    w, s, d = weights(torch, g, N, K)
+    w[w & 0x0F == 0] |= 0x01            # (no zero weights: infinity times zero is NaN)
+    w[w & 0xF0 == 0] |= 0x10
+    q = torch.stack([w & 15, w >> 4], -1).reshape(N, K).double()
+    d = (torch.where(q > 7, q - 16, q).view(N, -1, 128) * s.double()[..., None]).view(N, K)
+    x = torch.randn((M, K), generator=g, device="cuda")
+    x[1, 5], x[2, 200], x[3, 7] = float("inf"), float("-inf"), float("nan")
+    x[4, 9] = torch.tensor(0x7F800001, dtype=torch.int32, device="cuda").view(torch.float32)   # a NaN whose leading half is an infinity's
+    x[5] *= 1e36
+    y = torch.empty((M, N), device="cuda")
+    assert ops.linear_int4(y, x, w, s, None, M, N, K) == 0
+    want = x.double() @ d.T
+    assert torch.equal(y[1:3].double(), want[1:3]) and torch.isinf(y[1:3]).all()
+    assert torch.isnan(y[3:5]).all()
+    for r in (0, 5):
+        assert ((y[r].double() - want[r]).norm() / want[r].norm()).item() <= 2 ** -24 * (128 + K / 128) ** 0.5 * 2
+    silu = torch.empty((3, N), device="cuda")
+    assert ops.mlp_gate_up_swiglu_int4(silu, x[:3].contiguous(), w, s, w, s, 3, N, K) == 0
+    gate = y[1:3]
+    assert torch.equal(silu[1:3].isnan(), (gate / (1 + torch.exp(-gate)) * gate).isnan())
