@@ -346,6 +346,41 @@ def test_prefill_swiglu_and_fused_projections(cuda, M):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,K,Ns,glu,path", [
+    (33, 5120, [17408], True, TC), (40, 5120, [17408], True, TC), (64, 5120, [17408], True, GEMM), (33, 6144, [5120], False, TC),
+    (40, 6144, [5120], False, TC), (64, 6144, [5120], False, GEMM), (33, 5120, [12288, 1024, 1024], False, GEMM), (64, 5632, [2048], False, TC),
+    (65, 5632, [2048], False, GEMM)])
+def test_33_to_64_rows_take_the_cheaper_route(cuda, M, K, Ns, glu, path):
+    """Two 32-row slices of the decode kernel or the GEMM, by modelled time: the route that the rule means to take, and the same
+    outputs as through the GEMM to the fp16 rounding of either."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn((M, K), generator=g, device="cuda").half()
+    w = [(torch.randint(0, 256, (n, K // 2), generator=g, device="cuda", dtype=torch.uint8),
+          (torch.rand((n, K // 128), generator=g, device="cuda") * 0.01).half()) for n in (Ns * 2 if glu else Ns)]
+
+    def run():
+        ys = [torch.full((M, n), float("nan"), dtype=torch.float16, device="cuda") for n in Ns]
+        if glu:
+            assert cuda.mlp_gate_up_swiglu_int4(ys[0], x, *w[0], *w[1], M, Ns[0], K) == 0
+        elif len(Ns) == 1:
+            assert cuda.linear_int4(ys[0], x, *w[0], None, M, Ns[0], K) == 0
+        else:
+            assert cuda.linear_int4_fused(x, [{"Y": y, "W_int4": a, "scales": s, "N": n} for y, (a, s), n in zip(ys, w, Ns)], M, K) == 0
+        torch.cuda.synchronize()
+        return ys, cuda.last_linear_path()
+    got, used = run()
+    assert used == path
+    cuda.set_linear_path(GEMM)
+    try:
+        want, used = run()
+    finally:
+        cuda.set_linear_path(0)
+    assert used == GEMM and cuda.device_status(0) == 0
+    for a, b in zip(got, want):
+        assert ((a.double() - b.double()).norm() / b.double().norm()).item() <= 2 ** -11
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("K", [1024, 5120, 1152])
 @pytest.mark.parametrize("M", [1, 129])
 def test_scales_at_any_two_byte_address(cuda, M, K):

@@ -20,8 +20,21 @@ constexpr int kMaxDevices = 64;
 constexpr int kCounterCapacity = 8192;
 constexpr size_t kSamplingScratchBytes = 4u << 20;  // rows * chunks * 16 B
 // 33 .. 128 rows on few weights run as 32-row slices of the decode kernel: a problem this small is all pipeline fill, and
-// the decode kernel spreads it over more CTAs.
-constexpr int64_t kSliceRowsMax = 128, kSliceWeightsMax = 4 << 20;
+// the decode kernel spreads it over more CTAs.  On more weights two slices (33 .. 64 rows) are taken where they cost less than the
+// GEMM by what both were measured at, in us (W in millions of weights):
+//   two slices    13 + W (0.21, 0.24 or 0.28 with up to 8, 16 or 32 rows in the second)
+//   the GEMM      xb::gemm_modelled_us
+// 33 / 48 / 64 rows, slices and GEMM: gate/up of 5120 x 17408 49 and 55 / 53 and 53 / 55 and 53; 6144 x 5120 19 and 21 / 21 and 21 /
+// 22 and 21; q/k/v of 5120 x 8192 22 and 23 / 23 and 23 / 25 and 23; 17408 x 5120 34 and 34 / 36 and 34 / 38 and 34.  From 65 rows on
+// the third slice decides for the GEMM everywhere (33 and 25 for q/k/v, 77 and 60 for gate/up).  The models are good to 6 %, which
+// is the margin that the slices need.
+constexpr int64_t kSliceRowsMax = 128, kSliceWeightsMax = 4 << 20, kTwoSlices = 64;
+bool slices_cost_less(const xb::TcProj* proj, int num, bool swiglu, int64_t m, int64_t k, int64_t weights, int num_sms) {
+    if (weights <= kSliceWeightsMax) return true;
+    if (m > kTwoSlices) return false;
+    const double per_million = m - 32 <= 8 ? 0.21 : (m - 32 <= 16 ? 0.24 : 0.28);
+    return 13.0 + per_million * 1e-6 * static_cast<double>(weights) < 0.94 * xb::gemm_modelled_us(proj, num, swiglu, m, k, num_sms);
+}
 
 struct DeviceCtx {
     bool ready = false;
@@ -91,8 +104,8 @@ int run_linear(xinfer_stream_t s, const void* x, xb::ActType in, bool out_f32, c
     cudaStream_t stream = static_cast<cudaStream_t>(s);
     int64_t weights = 0;
     for (int i = 0; i < (swiglu ? 2 : num); ++i) weights += proj[i].n * k;
-    if (c->forced_path != 2 && c->forced_path != 3 && in == xb::ActType::F16 && m > 32 && m <= kSliceRowsMax && weights <= kSliceWeightsMax &&
-        xb::tc_eligible(x, proj, num, swiglu, 32, k, group_size)) {
+    if (c->forced_path != 2 && c->forced_path != 3 && in == xb::ActType::F16 && m > 32 && m <= kSliceRowsMax &&
+        xb::tc_eligible(x, proj, num, swiglu, 32, k, group_size) && slices_cost_less(proj, num, swiglu, m, k, weights, c->num_sms)) {
         const int cnt = swiglu ? 2 : num;
         const size_t ybytes = out_f32 ? 4 : 2;
         for (int64_t r0 = 0; r0 < m; r0 += 32) {

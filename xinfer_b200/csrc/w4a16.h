@@ -44,6 +44,8 @@ bool gemm_eligible(const void* x, const TcProj* proj, int num, bool swiglu, long
 size_t gemm_partial_bytes(int num_sms);
 int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num, bool swiglu, bool out_f32, long long m,
                 long long k, int* status, long long wait_limit, int x_stage_limit, int num_sms, float* partials, int* counters);
+// About how long a launch of at most 256 rows takes, in microseconds.
+double gemm_modelled_us(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms);
 // The current device's status word (what xinfer_device_status reads) and number of SMs; a XINFER_* code.
 int device_facts(int** status, int* num_sms);
 // Records a message for xinfer_last_cuda_error() on the calling thread (c_api.cu).

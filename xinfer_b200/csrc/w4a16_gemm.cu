@@ -679,6 +679,47 @@ bool gemm_eligible(const void* x, const TcProj* proj, int num, bool swiglu, long
     return true;
 }
 
+namespace {
+
+// How a launch's tiles are dealt to the CTA pairs.  One pair per two SMs.  Cutting tiles evens the pairs' work out and costs the
+// exchange of partial sums, about as much as kCutCost groups; a small problem takes fewer pairs (below eight groups each, the
+// pipeline's fill dominates).
+constexpr long long kCutCost = 16;
+struct GemmDeal {
+    long long tiles, units, pairs;
+    bool whole_tiles;
+};
+GemmDeal gemm_deal(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms, bool may_cut) {
+    GemmDeal d;
+    const long long groups = k / 128, m_tiles = (m + kGemmTileM - 1) / kGemmTileM, rows = swiglu ? kGemmTileN : 2 * kGemmTileN;  // of a pair
+    d.tiles = 0;
+    for (int i = 0; i < (swiglu ? 1 : num); ++i) d.tiles += (proj[i].n + rows - 1) / rows * m_tiles;
+    d.units = d.tiles * groups;
+    const long long max_pairs = num_sms / 2, whole = (d.tiles + max_pairs - 1) / max_pairs * groups;
+    long long cut_pairs = d.units / 8;
+    if (cut_pairs < 1) cut_pairs = 1;
+    if (cut_pairs > max_pairs) cut_pairs = max_pairs;
+    d.whole_tiles = !may_cut || whole <= (d.units + cut_pairs - 1) / cut_pairs + kCutCost;
+    d.pairs = !d.whole_tiles ? cut_pairs : (d.tiles < max_pairs ? d.tiles : max_pairs);
+    return d;
+}
+
+}  // namespace
+
+// 5.8 us a tile of a pair (fill, read-out and stores) and 0.53 us a group; a cut costs kCutCost groups, or six where it falls on
+// equal parts of every tile.  Within 6 % of most of 18 shapes at 33 .. 64 rows; off by more for the narrowest (5120 x 2048 and
+// narrower: within 3 us) and for few tiles in many parts (16384 x 1024: 21 us, modelled 13).
+double gemm_modelled_us(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms) {
+    const GemmDeal d = gemm_deal(proj, num, swiglu, m, k, num_sms, true);
+    const long long groups = k / 128;
+    if (d.whole_tiles) {
+        const long long tiles = (d.tiles + d.pairs - 1) / d.pairs;
+        return 5.8 * static_cast<double>(tiles) + 0.53 * static_cast<double>(tiles * groups);
+    }
+    const bool even = d.units % d.pairs == 0 && groups % (d.units / d.pairs) == 0;
+    return 5.8 + 0.53 * (static_cast<double>(d.units) / static_cast<double>(d.pairs) + (even ? 6.0 : static_cast<double>(kCutCost)));
+}
+
 size_t gemm_partial_bytes(int num_sms) {
     return static_cast<size_t>(num_sms) * 2 * kGemmTileN * kGemmTileM * sizeof(float);
 }
@@ -713,28 +754,20 @@ int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num,
         const int rows = swiglu ? kGemmTileN : 2 * kGemmTileN;  // of a pair
         tiles += (a.n + rows - 1) / rows * p.m_tiles;
     }
-    if (tiles > (1 << 30)) return -2;
+    const GemmDeal deal = gemm_deal(proj, num, swiglu, m, k, num_sms, partials != nullptr);
+    if (deal.tiles > (1 << 30)) return -2;
     if (!encode_gemm_x(&p.x_map, static_cast<const __half*>(x), m, k, p.tile_m)) return -2;
     p.m = static_cast<int>(m);
-    p.units = tiles * p.groups;
+    p.units = deal.units;
     p.swiglu = swiglu ? 1 : 0;
     p.wait_limit = wait_limit;
     p.x_stage_limit = x_stage_limit;
     p.status = status;
     p.partials = partials;
     p.counters = counters;
-    // One pair per two SMs.  Cutting tiles evens the pairs' work out and costs the exchange of partial sums, about as
-    // much as kCutCost groups; a small problem takes fewer pairs (below eight groups each, the pipeline's fill dominates).
-    constexpr long long kCutCost = 16;
-    const long long max_pairs = num_sms / 2;
-    const long long whole = (tiles + max_pairs - 1) / max_pairs * p.groups;
-    long long cut_pairs = p.units / 8;
-    if (cut_pairs < 1) cut_pairs = 1;
-    if (cut_pairs > max_pairs) cut_pairs = max_pairs;
-    p.whole_tiles = (!partials || whole <= (p.units + cut_pairs - 1) / cut_pairs + kCutCost) ? 1 : 0;
-    const long long pairs = p.whole_tiles ? (tiles < max_pairs ? tiles : max_pairs) : cut_pairs;
-    p.pairs = static_cast<int>(pairs);
-    const dim3 grid(static_cast<unsigned>(2 * pairs));
+    p.whole_tiles = deal.whole_tiles ? 1 : 0;
+    p.pairs = static_cast<int>(deal.pairs);
+    const dim3 grid(static_cast<unsigned>(2 * deal.pairs));
     const cudaError_t e = out_f32 ? gemm_configure_and_launch<float>(p, grid, stream) : gemm_configure_and_launch<__half>(p, grid, stream);
     return e == cudaSuccess ? 0 : -1;
 }
