@@ -92,7 +92,6 @@ struct GemmProj {
     long long ldy;
     int n;           // output features
     int tile0;       // index of its first tile in the launch
-    int scales_vec;  // every row of its scales starts on a 16-byte boundary
 };
 
 struct GemmParams {
@@ -105,6 +104,7 @@ struct GemmParams {
     int w_slots;     // slots of the packed-weight ring
     int m_tiles;
     int groups;      // k / 128
+    int scales_vec;  // every row of scales starts on a 16-byte boundary
     long long units;     // tiles * groups
     int pairs;           // CTA pairs of the launch
     int whole_tiles;     // cut between tiles only
@@ -436,14 +436,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
 #pragma unroll
             for (int j = 0; j < kGemmTileM / 2; ++j) acc[j] = 0.f;
             // scales eight groups at a time, a block of eight ahead of its use (one group ahead, their latency is the loop's)
-            uint4 q_cur = load_scales(sp, seg_begin & ~7, p.groups, pj.scales_vec), q_next = load_scales(sp, (seg_begin & ~7) + 8, p.groups, pj.scales_vec);
+            uint4 q_cur = load_scales(sp, seg_begin & ~7, p.groups, p.scales_vec), q_next = load_scales(sp, (seg_begin & ~7) + 8, p.groups, p.scales_vec);
             for (int j = 0; j < (seg_begin & 7); ++j) shift_scales(q_cur);
             for (; group < seg_end; ++group, ++i) {
                 const float sc = __half2float(__ushort_as_half(static_cast<unsigned short>(q_cur.x & 0xFFFFu)));
                 shift_scales(q_cur);
                 if ((group & 7) == 7) {
                     q_cur = q_next;
-                    q_next = load_scales(sp, group + 9, p.groups, pj.scales_vec);
+                    q_next = load_scales(sp, group + 9, p.groups, p.scales_vec);
                 }
                 const uint32_t buf = static_cast<uint32_t>(i & (d_bufs - 1));
                 if (dead || !mbar_wait_parked(smem_u32(&ctrl->d_full[buf]), (i >> d_shift) & 1u, ws)) { dead = true; continue; }
@@ -741,6 +741,7 @@ int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num,
         p.proj[0].scales[1] = static_cast<const __half*>(proj[1].scales);
     }
     p.num_proj = swiglu ? 1 : num;
+    p.scales_vec = p.groups % 8 == 0;  // (one flag a launch: read for every projection it cost the kernel 1 to 2 %)
     for (int i = 0; i < p.num_proj; ++i) {
         const TcProj& a = proj[i];
         if (!swiglu && !encode_gemm_w(&p.w_map[i], a.w, a.n, k, kGemmTileN)) return -2;
@@ -749,7 +750,7 @@ int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num,
         p.proj[i].y = a.y;
         p.proj[i].ldy = a.ldy > 0 ? a.ldy : a.n;
         p.proj[i].n = static_cast<int>(a.n);
-        p.proj[i].scales_vec = p.groups % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.scales) | reinterpret_cast<uintptr_t>(p.proj[i].scales[1])) & 15) == 0;
+        if (((reinterpret_cast<uintptr_t>(a.scales) | reinterpret_cast<uintptr_t>(p.proj[i].scales[1])) & 15) != 0) p.scales_vec = 0;
         p.proj[i].tile0 = static_cast<int>(tiles);
         const int rows = swiglu ? kGemmTileN : 2 * kGemmTileN;  // of a pair
         tiles += (a.n + rows - 1) / rows * p.m_tiles;
