@@ -38,6 +38,36 @@ def test_linear_f32(M, K, N):
     assert rel(y, gate / (1 + torch.exp(-gate)) * (x.double() @ d2.T)) <= 4 * bound
 
 
+@pytest.mark.parametrize("M,K,N", [(8, 5120, 512), (8, 6144, 512), (2, 17408, 640)])
+@pytest.mark.parametrize("spread", [0.0, 3.0])
+def test_linear_f32_is_as_close_as_a_chain_of_fmas(M, K, N, spread):
+    """Error against 64 bits beside that of fp32 arithmetic in the reference's association - a chain of 128 fused multiply-adds per
+    group, a chain over the groups - for activations of one magnitude and of many; mean of four draws."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    import xinfer_b200.ops as ops
+    ours, chain = 0.0, 0.0
+    for seed in range(4):
+        g = torch.Generator(device="cuda").manual_seed(seed + K)
+        x = torch.randn((M, K), generator=g, device="cuda") * torch.exp(spread * torch.randn((M, K), generator=g, device="cuda"))
+        w, s, d = weights(torch, g, N, K)
+        y = torch.empty((M, N), device="cuda")
+        assert ops.linear_int4(y, x, w, s, None, M, N, K) == 0
+        want = x.double() @ d.T
+        sd = s.double()
+        q = torch.round(d.view(N, -1, 128) / sd.clamp_min(1e-9)[..., None])          # the integers
+        xg, dot = x.double().view(M, 1, -1, 128), torch.zeros((M, N, K // 128), device="cuda", dtype=torch.float64)
+        for i in range(128):
+            dot = (dot + xg[..., i] * q[None, ..., i]).float().double()              # a product is exact in 64 bits: one rounding
+        acc = torch.zeros((M, N), device="cuda", dtype=torch.float64)
+        for j in range(K // 128):
+            acc = (acc + dot[..., j] * sd[:, j]).float().double()
+        ours += ((y.double() - want).norm() / want.norm()).item()
+        chain += ((acc - want).norm() / want.norm()).item()
+    assert ours <= 1.25 * chain, (ours / 4, chain / 4)
+
+
 def test_linear_f32_carries_infinities_and_nan():
     """An infinite activation gives infinities of the weights' signs, as fp32 arithmetic does, NaN gives NaN, the largest finite
     values neither; other rows stay untouched."""
