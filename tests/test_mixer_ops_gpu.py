@@ -192,9 +192,10 @@ def test_shape_validation_like_the_reference(cuda):
     assert e.value.code == _lib.ERR_INVALID_ARGUMENT
 
 
-def test_captured_decode_layer_after_a_long_prompt(cuda):
-    """Attention and delta rule of a single token captured as a graph, then the same ops on a prompt, then the graph again: what it
-    holds of the library's scratch has not moved."""
+@pytest.mark.parametrize("other", [None, (24, 4, 48, 16), (64, 2, 80, 16)])
+def test_captured_decode_layer_after_a_long_prompt(cuda, other):
+    """Attention and delta rule of a single token captured as a graph, then the same ops on a prompt, or with other heads, then the
+    graph again: what it holds of the library's scratch is still there."""
     g = torch.Generator(device="cuda").manual_seed(5)
     n = lambda *s: torch.randn(s, generator=g, device="cuda").half()  # noqa: E731
     hq, hkv, hv, hk, cap, T = 8, 2, 6, 2, 1200, 1100
@@ -217,6 +218,12 @@ def test_captured_decode_layer_after_a_long_prompt(cuda):
     long_state = state0.clone()
     assert cuda.sdpa_causal_cached(out, q, kc, vc, 0, T, hq, hkv, 256, max_seq_len=cap) == 0
     assert cuda.recurrent_gated_delta_net(out2, qkv, z, b, a, A_log, dt_bias, norm_w, long_state, T, False, hv, hk) == 0
+    if other:
+        hq, hkv, hv, hk = other
+        T = 600
+        assert cuda.sdpa_causal_cached(n(T, hq, 256), n(T, hq, 256), n(T, hkv, 256), n(T, hkv, 256), 0, T, hq, hkv, 256) == 0
+        assert cuda.recurrent_gated_delta_net(n(T, hv * 128), n(T, 2 * hk * 128 + hv * 128), n(T, hv * 128), n(T, hv), n(T, hv), n(hv).float(),
+                                              n(hv).float(), norm_w, n(hv, 128, 128).float(), T, False, hv, hk) == 0
     torch.cuda.synchronize()
     for x in (o1, o2):
         x.fill_(float("nan"))

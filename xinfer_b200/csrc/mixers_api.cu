@@ -25,12 +25,12 @@ namespace {
 constexpr int kMaxDevices = 64;
 
 // Scratch of the stand-alone entry points, a block per device and op (the speculative decoder has its own).  A block is taken at
-// the most that any call with the same heads needs (39 MB for the attention and 32 MB for the delta rule at the 27B shapes): it
-// stays where it is whatever the row counts, so a graph captured around one call stays good when another one has more rows.
-// Only more heads than before move it.
+// the most that any call with the same heads needs (39 MB for the attention and 32 MB for the delta rule at the 27B shapes), so it
+// stays where it is whatever the row counts.  Other heads may need a larger one.  Then the old one is kept, since a captured graph
+// may hold it; sizes are powers of two, so that all of an op's blocks together are less than twice the largest.
 struct MixerScratch {
     float* buf = nullptr;
-    size_t bytes = 0;
+    size_t bytes = 0, refused = SIZE_MAX;  // `refused`: the smallest request that there was no memory for
 };
 enum ScratchOf { kAttention, kDelta, kScratches };
 MixerScratch g_scratch[kMaxDevices][kScratches];
@@ -42,24 +42,21 @@ int scratch(ScratchOf which, size_t bytes, size_t most, float** out) {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return XINFER_ERR_NO_DEVICE;
     std::lock_guard<std::mutex> lock(g_mu);
     MixerScratch& m = g_scratch[dev][which];
-    if (m.bytes < bytes) {
-        // more heads: the old block may still be in use by work already enqueued, so wait for it first
-        if (m.buf) {
-            cudaDeviceSynchronize();
-            cudaFree(m.buf);
-            m.buf = nullptr;
-            m.bytes = 0;
+    for (size_t want : {most, bytes}) {  // (on a full device the call still gets what it needs)
+        if (m.bytes >= want) break;
+        if (want == most && most != bytes && want >= m.refused) continue;
+        size_t size = size_t{1} << 20;
+        while (size < want) size *= 2;
+        float* buf = nullptr;
+        if (cudaMalloc(reinterpret_cast<void**>(&buf), size) == cudaSuccess) {
+            m.buf = buf;
+            m.bytes = size;
+            break;
         }
-        for (size_t size : {most, bytes}) {  // (on a full device the call still gets what it needs)
-            if (cudaMalloc(reinterpret_cast<void**>(&m.buf), size) == cudaSuccess) {
-                m.bytes = size;
-                break;
-            }
-            cudaGetLastError();
-            m.buf = nullptr;
-        }
-        if (!m.buf) return XINFER_ERR_OUT_OF_MEMORY;
+        cudaGetLastError();
+        if (want < m.refused) m.refused = want;
     }
+    if (m.bytes < bytes) return XINFER_ERR_OUT_OF_MEMORY;
     *out = m.buf;
     return XINFER_OK;
 }
