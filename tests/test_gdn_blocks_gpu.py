@@ -151,3 +151,30 @@ def test_conv1d_spans(cuda, T, C):
             assert np.all(np.abs(y.float().cpu().numpy() - want) <= 2 ** -10 * np.maximum(np.abs(want), 2 ** -14))
             if state is not None:
                 assert np.array_equal(st_d.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("with_state", [True, False])
+def test_conv1d_beyond_32_bit_positions(cuda, with_state):
+    """A sequence of more than 2^31 positions (two channels) gives, at its end and at a seam, what that part alone gives."""
+    import torch
+    C, T, tail, seam = 2, 2 ** 31 + 21, 64, 2 ** 30
+    if torch.cuda.mem_get_info()[0] < 24 << 30:
+        pytest.skip("needs 24 GB")
+    x = torch.full((T, C), 0.5, dtype=torch.float16, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(0)
+    for at in (seam - 32, T - tail):
+        x[at:at + tail] = torch.randn((tail, C), generator=g, device="cuda").half()
+    w, st = torch.randn((C, 4), generator=g, device="cuda"), torch.randn((3, C), generator=g, device="cuda")
+    y, last = torch.empty_like(x), st.clone() if with_state else None
+    assert cuda.causal_conv1d_silu(y, x, w, T, last, C) == 0
+    for at in (seam - 32, T - tail):
+        y2, st2 = torch.empty((tail, C), dtype=torch.float16, device="cuda"), torch.full_like(st, 0.5)
+        assert cuda.causal_conv1d_silu(y2, x[at:at + tail].contiguous(), w, tail, st2, C) == 0
+        assert torch.equal(y[at:at + tail], y2)
+    if with_state:
+        assert torch.equal(last, st2)
+    head = torch.empty((64, C), dtype=torch.float16, device="cuda")
+    assert cuda.causal_conv1d_silu(head, x[:64].contiguous(), w, 64, st.clone() if with_state else None, C) == 0
+    assert torch.equal(y[:64], head)
+    del x, y
+    torch.cuda.empty_cache()

@@ -32,7 +32,7 @@ struct MixerScratch {
     float* buf = nullptr;
     size_t bytes = 0, refused = SIZE_MAX;  // `refused`: the smallest request that there was no memory for
 };
-enum ScratchOf { kAttention, kDelta, kScratches };
+enum ScratchOf { kAttention, kDelta, kConvState, kScratches };
 MixerScratch g_scratch[kMaxDevices][kScratches];
 std::mutex g_mu;
 
@@ -167,9 +167,23 @@ int xinfer_causal_conv1d_silu_f16(xinfer_stream_t s, void* out_qkv, const void* 
     if (num_channels <= 0 || num_channels > INT32_MAX) return XINFER_ERR_INVALID_ARGUMENT;
     if (seq_len <= 0) return XINFER_NOOP_INVALID_SHAPE;
     if (!out_qkv || !in_qkv || !conv_w) return XINFER_ERR_INVALID_ARGUMENT;
-    if (seq_len > INT32_MAX) return XINFER_ERR_INVALID_ARGUMENT;
-    return ok_or_cuda(xb::conv1d_chunk(static_cast<cudaStream_t>(s), static_cast<__half*>(out_qkv), static_cast<const __half*>(in_qkv),
-                                       conv_w, conv_state, 1, static_cast<int>(seq_len), static_cast<int>(num_channels)));
+    // pieces that 32-bit positions reach; the state carries from one to the next
+    constexpr int64_t kPiece = int64_t{1} << 30;
+    float* state = conv_state;
+    if (!state && seq_len > kPiece) {
+        const size_t bytes = 3 * sizeof(float) * static_cast<size_t>(num_channels);
+        const int rc = scratch(kConvState, bytes, bytes, &state);
+        if (rc != XINFER_OK) return rc;
+        if (cudaMemsetAsync(state, 0, bytes, static_cast<cudaStream_t>(s)) != cudaSuccess) return ok_or_cuda(-1);
+    }
+    for (int64_t t0 = 0; t0 < seq_len; t0 += kPiece) {
+        const int rows = static_cast<int>(seq_len - t0 < kPiece ? seq_len - t0 : kPiece);
+        const int r = xb::conv1d_chunk(static_cast<cudaStream_t>(s), static_cast<__half*>(out_qkv) + t0 * num_channels,
+                                       static_cast<const __half*>(in_qkv) + t0 * num_channels, conv_w, state, 1, rows,
+                                       static_cast<int>(num_channels));
+        if (r != 0) return ok_or_cuda(r);
+    }
+    return XINFER_OK;
 }
 
 int xinfer_recurrent_gated_delta_net_f16(xinfer_stream_t s, void* out, const void* qkv, const void* z, const void* b,
