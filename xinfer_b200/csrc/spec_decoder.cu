@@ -1142,10 +1142,9 @@ int xinfer_spec_decoder_prefill(xinfer_spec_decoder* d, xinfer_stream_t stream, 
     if (d->ctx_upper != 0) { d->error = "prefill starts from the empty context (reset(0, seed))"; return XINFER_ERR_INVALID_ARGUMENT; }
     if (T - 1 + 2 * R > d->max_seq) { d->error = "prompt does not fit the cache"; return XINFER_ERR_INVALID_ARGUMENT; }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // positions per sequence and chunk: 512 rows over all sequences, a multiple of the mixers' four
-    int Cp = (512 / B) & ~3;
-    if (Cp < 4) Cp = 4;
-    if (T - 1 < Cp) Cp = static_cast<int>(((T - 1) + 3) & ~3LL);
+    // positions per sequence and chunk: 512 rows over all sequences
+    int Cp = 512 / B > 0 ? 512 / B : 1;
+    if (T - 1 < Cp) Cp = static_cast<int>(T - 1);
     if (Cp > 0) {
         int rc0 = ensure_chunk_bufs(d, B * Cp);
         if (rc0 < 0) return rc0;
