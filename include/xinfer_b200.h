@@ -60,7 +60,8 @@ XINFER_EXPORT int xinfer_last_linear_path(void);
  * Process-wide; applies to launches enqueued afterwards.  No counterpart in the reference. */
 XINFER_EXPORT void xinfer_debug_set_wait_hooks(int64_t limit_clocks, int withhold_x_from_stage);
 /* Force a kernel family for the linear entry points on the current device: 0 = automatic (fp16 activations: the
- * tcgen05 decode kernel up to 32 rows, 32-row slices of it up to 128 rows, the tcgen05 GEMM above), 1 = the same,
+ * tcgen05 decode kernel up to 32 rows; above, the tcgen05 GEMM or, where it costs less - up to 128 rows on at most 4 M
+ * weights, up to 64 rows by a model of both - 32-row slices of the decode kernel), 1 = the same,
  * 2 = CUDA cores only, 3 = the GEMM for every M > 32.  For measurements and tests. */
 XINFER_EXPORT void xinfer_set_linear_path(int path);
 

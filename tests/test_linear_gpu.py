@@ -247,12 +247,12 @@ GEMM = 3
 @pytest.mark.parametrize("M,K,N", [(33, 128, 16), (64, 512, 96), (256, 1024, 1000), (300, 5120, 1024), (512, 5120, 6144),
                                    (512, 17408, 5120), (513, 256, 300)])
 def test_prefill_gemm_against_oracle(cuda, M, K, N):
-    """More than 32 rows go to the tensor-core GEMM (scale * weight enters the MMA as an exact hi + lo pair of fp16
-    operands; sums in fp32 over all of K): same bound as the decode kernels."""
+    """More than 32 rows go to the tensor-core GEMM (the weights enter the MMA as exact fp16 integers, a 128-k group at a
+    time, and are folded with the group's scale in fp32): same bound as the decode kernels."""
     X, W, S, _ = synth_linear(M, K, N, seed=M + N)
     bias = np.random.default_rng(1).normal(0, 0.1, size=N).astype(np.float32)
     ref = oracle.linear_int4_f64(X.astype(np.float32), W, S, bias)
-    got, used = run_linear(cuda, X, W, S, bias=bias, path=GEMM)   # (forced: up to 128 rows the default is the decode kernel)
+    got, used = run_linear(cuda, X, W, S, bias=bias, path=GEMM)   # (forced: few weights default to the decode kernel up to 128 rows)
     assert used == GEMM
     # (one tensor-core accumulation over all of K instead of one per 128-k group; its fp32 adds truncate, so the
     # error grows with K: 3.7e-5 measured at K = 5120, 1.3e-4 at K = 17408; the stated bound is 1e-3 relative)
@@ -263,7 +263,7 @@ def test_prefill_gemm_against_oracle(cuda, M, K, N):
     # the CUDA-core path of the same call agrees
     simt, used = run_linear(cuda, X, W, S, bias=bias, path=SIMT)
     assert used == SIMT and rel_err(got, simt) <= 3e-4
-    # the default: 32-row slices of the decode kernel up to 128 rows (the reference's association), the GEMM above
+    # the default on few weights: 32-row slices of the decode kernel up to 128 rows, the GEMM above
     auto, used = run_linear(cuda, X, W, S, bias=bias)
     assert used == (TC if M <= 128 else GEMM)
     assert rel_err(auto, ref) <= (2e-5 if M <= 128 else 3e-4)
@@ -325,7 +325,7 @@ def test_prefill_swiglu_and_fused_projections(cuda, M):
         cuda.set_linear_path(0)
     torch.cuda.synchronize()
     assert cuda.last_linear_path() == GEMM and cuda.device_status(0) == 0
-    if M <= 128:   # the default for this many rows: slices through the decode kernel, fused and SwiGLU forms included
+    if M <= 128:   # the default for this many rows on few weights: slices through the decode kernel, fused and SwiGLU forms included
         Y2 = torch.empty((M, N), dtype=torch.float16, device="cuda")
         assert cuda.mlp_gate_up_swiglu_int4(Y2, dev(X), dev(Wg), dev(Sg), dev(Wu), dev(Su), M, N, K) == 0
         torch.cuda.synchronize()

@@ -9,8 +9,8 @@
 //   * a pair of CTAs (tcgen05 cta_group::2) owns 256 weight rows (the MMA's M, 128 per CTA) x up to 256 activation rows
 //     (its N, of which each CTA loads half: one CTA alone would have to pull 64 KB of activations through L2 per 128-k
 //     group, 18 TB/s over the chip at full tensor rate);
-//   * the int4 values go into the MMA as exact fp16 integers.  One 128-k group accumulates into one of two tensor-memory
-//     tiles (2 x 256 columns), and while the tensor core works on the next group eight warps read the finished one back
+//   * the int4 values go into the MMA as exact fp16 integers.  One 128-k group accumulates into one of two
+//     tensor-memory tiles of 256 columns (four of 128 up to 128 rows), and while the tensor core works on the next group eight warps read the finished one back
 //     and fold it into fp32 registers with the group's scale: acc += d * scale, the reference's own association
 //     (src/ops/linear.cpp:239-287).  So every product is exact and every weight costs one MMA (the form before this one
 //     put scale * weight into the MMA as a high and a low fp16 operand, two MMAs per k step, because it kept one
