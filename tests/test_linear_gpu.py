@@ -254,8 +254,8 @@ def test_prefill_gemm_against_oracle(cuda, M, K, N):
     ref = oracle.linear_int4_f64(X.astype(np.float32), W, S, bias)
     got, used = run_linear(cuda, X, W, S, bias=bias, path=GEMM)   # (forced: few weights default to the decode kernel up to 128 rows)
     assert used == GEMM
-    # (one tensor-core accumulation over all of K instead of one per 128-k group; its fp32 adds truncate, so the
-    # error grows with K: 3.7e-5 measured at K = 5120, 1.3e-4 at K = 17408; the stated bound is 1e-3 relative)
+    # (the bound of one tensor-core accumulation over all of K, whose fp32 adds truncate; with one per 128-k group 1e-7
+    # is measured at K = 5120 and 17408)
     assert rel_err(got, ref) <= 3e-4
     got16, used = run_linear(cuda, X, W, S, bias=bias, out_dtype=torch.float16, path=GEMM)
     assert used == GEMM
