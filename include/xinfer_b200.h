@@ -304,7 +304,8 @@ XINFER_EXPORT int xinfer_attention_write_kv_cache_f16(xinfer_stream_t s, void* k
                                                       int64_t num_tokens, int64_t num_kv_heads, int64_t head_dim,
                                                       int64_t max_seq_len);
 /* Causal GQA attention of num_q_tokens query rows at positions start_pos... over the cache: row i sees keys
- * 0 .. start_pos + i.  scale <= 0 means 1/sqrt(head_dim).  Replaces ops::sdpa_causal_cached (half),
+ * 0 .. start_pos + i.  scale <= 0 means 1/sqrt(head_dim).  The V rows of this call's own positions must be finite: keys
+ * are taken 64 at a time, and a later row's enters an earlier one's sum with weight 0.  Replaces ops::sdpa_causal_cached (half),
  * src/ops/attention.h:102-113 (also the body of sdpa_causal_verify). */
 XINFER_EXPORT int xinfer_sdpa_causal_cached_f16(xinfer_stream_t s, void* out_f16, const void* Q_f16,
                                                 const void* k_cache_f16, const void* v_cache_f16, int64_t start_pos,
