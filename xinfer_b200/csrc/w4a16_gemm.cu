@@ -70,7 +70,7 @@ struct GemmCtrl {
     WaitState ws;
 };
 
-// [alignment slack] [A ring] [X ring: slots x 2 x tile_m / 2 x 128 bytes] [W ring] [control]
+// [control] [alignment slack] [A ring] [X ring: slots x 2 x tile_m / 2 x 128 bytes] [W ring]
 constexpr int kGemmSmemBytes = 227 * 1024;
 constexpr int kGemmSmemFixed = 1024 + static_cast<int>(sizeof(GemmCtrl));
 constexpr int gemm_slots_bytes(int tile_m, int slots) { return slots * (kASlotBytes + tile_m * 2 * kSwizzleK); }
@@ -216,18 +216,20 @@ __device__ __forceinline__ int proj_of_tile(const GemmParams& p, int tile) {
     return i;
 }
 
-template <typename OutT>
+// NC: 32-column reads a fold thread makes of an accumulator tile, ceil(tile_m / 64).
+template <int NC, typename OutT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __grid_constant__ GemmParams p) {
     extern __shared__ uint8_t gemm_smem_raw[];
+    // (the control block first: its addresses are then constants, and the fold, which needs every register, holds none of them)
+    GemmCtrl* ctrl = reinterpret_cast<GemmCtrl*>(gemm_smem_raw);
     // the swizzled operand tiles want 1024-byte alignment
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    uint8_t* a_ring = smem;
-    const int op_slots = gemm_op_slots(p.tile_m), d_bufs = gemm_d_bufs(p.tile_m), d_shift = d_bufs == 2 ? 1 : 2, d_cols = kGemmTmemCols / d_bufs;
+    uint8_t* a_ring = gemm_smem_raw + (((smem_u32(gemm_smem_raw) + sizeof(GemmCtrl) + 1023u) & ~1023u) - smem_u32(gemm_smem_raw));
+    constexpr int d_bufs = gemm_d_bufs(NC * 64), d_shift = d_bufs == 2 ? 1 : 2, d_cols = kGemmTmemCols / d_bufs;
+    const int op_slots = gemm_op_slots(p.tile_m);
     uint8_t* x_ring = a_ring + op_slots * kASlotBytes;
     const uint32_t x_half_bytes = static_cast<uint32_t>(p.tile_m) * kSwizzleK;  // 64 k of this CTA's half of the rows
     uint8_t* w_ring = x_ring + op_slots * 2 * x_half_bytes;
     const int w_slots = p.w_slots;
-    GemmCtrl* ctrl = reinterpret_cast<GemmCtrl*>(w_ring + w_slots * kWSlotBytes);
 
     const int tid = threadIdx.x;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -253,7 +255,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
     __syncthreads();
     cluster_sync_all();  // the other CTA's barriers are initialised too
     tc_fence_after_sync();
-    const uint32_t tmem_base = ctrl->tmem_base;
+    const uint32_t tmem_base = *const_cast<volatile uint32_t*>(&ctrl->tmem_base);
 
     // this pair's units (tile, 128-k group), tile-major; ring slots and phases count from its first unit
     const int pair = static_cast<int>(blockIdx.x >> 1);
@@ -420,7 +422,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
         const int half_cols = p.tile_m >> 1;             // a multiple of 16
         const uint32_t d_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(ch * half_cols);
         const bool up_row = p.swiglu && (r & 16);
-        float acc[kGemmTileM / 2];
+        float acc[NC * 32];
         int i = 0, tile = first_tile, group = first_group;
         bool dead = false;
         while (i < U) {
@@ -434,7 +436,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
                                        static_cast<long long>(valid ? row : 0) * p.groups;
             const int seg_begin = group, seg_end = (U - i < p.groups - group) ? group + (U - i) : p.groups;
 #pragma unroll
-            for (int j = 0; j < kGemmTileM / 2; ++j) acc[j] = 0.f;
+            for (int j = 0; j < NC * 32; ++j) acc[j] = 0.f;
             // scales eight groups at a time, a block of eight ahead of its use (one group ahead, their latency is the loop's)
             uint4 q_cur = load_scales(sp, seg_begin & ~7, p.groups, p.scales_vec), q_next = load_scales(sp, (seg_begin & ~7) + 8, p.groups, p.scales_vec);
             for (int j = 0; j < (seg_begin & 7); ++j) shift_scales(q_cur);
@@ -452,12 +454,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
                 // 32 columns a read (one tcgen05.ld; with two of 16 the whole kernel is 20 % slower at M = 512).  A tile of
                 // fewer columns reads on into columns that are allocated and not used.
 #pragma unroll
-                for (int c = 0; c < kGemmTileM / 64; ++c) {
-                    if (c * 32 < half_cols) {
+                for (int c = 0; c < NC; ++c) {
+                    // (always true; without a branch between them the compiler sets up a read beside the additions of the one before it,
+                    // runs out of registers and keeps launch-wide values in memory, which costs every warp of the CTA: 12 % at M = 512)
+                    if (NC < 4 || c * 32 < half_cols) {
                         uint32_t d[32];
                         tmem_ld32(src + c * 32, d);
                         tmem_wait_ld();
-                        if (c * 32 + 32 >= half_cols) {  // the last read of this group: the MMA warp may have the columns
+                        if (c == NC - 1) {  // the last read of this group: the MMA warp may have the columns
                             tc_fence_before_sync();
                             __syncwarp();
                             if (lane == 0) mbar_arrive_cluster(mapa_shared_cluster(smem_u32(&ctrl->d_empty[buf]), 0));
@@ -497,7 +501,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
                 if (!kept) {
                     float4* mine = reinterpret_cast<float4*>(p.partials + (static_cast<size_t>(blockIdx.x) * 2 + (seg_begin > 0 ? 0 : 1)) * slot_floats) + tid;
 #pragma unroll
-                    for (int j = 0; j < kGemmTileM / 2; j += 4)
+                    for (int j = 0; j < NC * 32; j += 4)
                         if (j < half_cols) __stcg(mine + j / 4 * kGemmFoldThreads, make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]));
                     __threadfence();
                     fold_barrier();
@@ -519,7 +523,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
                         // a contributor's part of this tile: slot 1 if the tile starts in its range, else slot 0
                         const float4* src = reinterpret_cast<const float4*>(base + static_cast<size_t>(c_first) * 4 * slot_floats + slot_floats);
 #pragma unroll
-                        for (int j = 0; j < kGemmTileM / 2; j += 4) {
+                        for (int j = 0; j < NC * 32; j += 4) {
                             if (j < half_cols) {
                                 const float4 t = __ldcg(src + j / 4 * kGemmFoldThreads);
                                 acc[j] = t.x;
@@ -533,13 +537,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
                     for (int o = c_first + 1; o <= c_last; ++o) {
                         const float4* src = reinterpret_cast<const float4*>(base + static_cast<size_t>(o) * 4 * slot_floats);
 #pragma unroll
-                        for (int c = 0; c < kGemmTileM / 2; c += 64) {
+                        for (int c = 0; c < NC * 32; c += 64) {
                             if (c < half_cols) {
                                 float4 t[16];
 #pragma unroll
-                                for (int j = 0; j < 16; ++j) t[j] = __ldcg(src + (c / 4 + j) * kGemmFoldThreads);
+                                for (int j = 0; j < 16; ++j)
+                                    if (c + j * 4 < NC * 32) t[j] = __ldcg(src + (c / 4 + j) * kGemmFoldThreads);
 #pragma unroll
                                 for (int j = 0; j < 16; ++j) {
+                                    if (c + j * 4 >= NC * 32) continue;
                                     acc[c + j * 4] += t[j].x;
                                     acc[c + j * 4 + 1] += t[j].y;
                                     acc[c + j * 4 + 2] += t[j].z;
@@ -553,7 +559,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
             if (!split || ctrl->last_arrival) {
                 const float bias = (valid && pj.bias && !p.swiglu) ? pj.bias[row] : 0.f;
 #pragma unroll
-                for (int c = 0; c < kGemmTileM / 32; ++c) {
+                for (int c = 0; c < NC * 2; ++c) {
                     if (c * 16 < half_cols) {
                         const int mc = m0 + ch * half_cols + c * 16;
                         OutT* out = static_cast<OutT*>(pj.y) + static_cast<long long>(mc) * pj.ldy + row;
@@ -572,7 +578,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
                                 const float a = acc[c * 16 + j], b = acc[c * 16 + 8 + j];
                                 const float theirs = __shfl_xor_sync(0xffffffffu, up_row ? a : b, 16);
                                 const float g = up_row ? theirs : a, u = up_row ? b : theirs;
-                                y[j] = (g / (1.0f + expf(-g))) * u;
+                                // (The exact division has a branch, so that the eight came one after the other: 1500 clocks per 16 columns,
+                                // 12000 between two tiles of 256 rows.  Two units in the last place of fp32, before the rounding to fp16.)
+                                y[j] = __fdividef(g, 1.0f + expf(-g)) * u;
                             }
                             if (up_row) out += 8 * pj.ldy;
                             const int live = valid ? p.m - mc - (up_row ? 8 : 0) : 0;
@@ -591,11 +599,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();  // the pair's MMAs read both CTAs' shared memory, and each arrives on the other's barriers
-    if (tid == 0 && ctrl->ws.abort_flag && p.status) atomicExch(p.status, kStatusWaitTimeout);
-    if (warp == kGemmMmaWarp) {
+    uint32_t t;  // (again, rather than through the fold)
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    if (t == 0 && ctrl->ws.abort_flag && p.status) atomicExch(p.status, kStatusWaitTimeout);
+    if (t >> 5 == kGemmMmaWarp) {
         __syncwarp();
         tc_fence_after_sync();
-        tmem_dealloc_pair(tmem_base, kGemmTmemCols);
+        tmem_dealloc_pair(*const_cast<volatile uint32_t*>(&ctrl->tmem_base), kGemmTmemCols);
     }
 }
 
@@ -641,7 +651,7 @@ bool encode_gemm_x(CUtensorMap* map, const __half* x, long long m, long long k, 
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename OutT>
+template <int NC, typename OutT>
 cudaError_t gemm_configure_and_launch(const GemmParams& p, dim3 grid, cudaStream_t stream) {
     static bool configured[64];
     static std::mutex mu;
@@ -654,16 +664,26 @@ cudaError_t gemm_configure_and_launch(const GemmParams& p, dim3 grid, cudaStream
         if (!configured[dev]) {
             // the register re-split draws on what the block was launched with: a request above that would wait forever
             cudaFuncAttributes a;
-            e = cudaFuncGetAttributes(&a, w4a16_gemm_kernel<OutT>);
+            e = cudaFuncGetAttributes(&a, w4a16_gemm_kernel<NC, OutT>);
             if (e != cudaSuccess) return e;
             if (a.numRegs * kGemmThreads < kFoldRegs * kGemmFoldThreads + kUnpackRegs * kGemmUnpackThreads + kCtrlRegs * 128)
                 return cudaErrorLaunchOutOfResources;
-            e = cudaFuncSetAttribute(w4a16_gemm_kernel<OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemBytes);
+            e = cudaFuncSetAttribute(w4a16_gemm_kernel<NC, OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemBytes);
             if (e != cudaSuccess) return e;
             configured[dev] = true;
         }
     }
-    return launch_pdl(w4a16_gemm_kernel<OutT>, grid, dim3(kGemmThreads), kGemmSmemBytes, stream, p);
+    return launch_pdl(w4a16_gemm_kernel<NC, OutT>, grid, dim3(kGemmThreads), kGemmSmemBytes, stream, p);
+}
+
+template <typename OutT>
+cudaError_t gemm_configure_and_launch(const GemmParams& p, dim3 grid, cudaStream_t stream) {
+    switch ((p.tile_m + 63) / 64) {
+        case 1: return gemm_configure_and_launch<1, OutT>(p, grid, stream);
+        case 2: return gemm_configure_and_launch<2, OutT>(p, grid, stream);
+        case 3: return gemm_configure_and_launch<3, OutT>(p, grid, stream);
+        default: return gemm_configure_and_launch<4, OutT>(p, grid, stream);
+    }
 }
 
 }  // namespace
