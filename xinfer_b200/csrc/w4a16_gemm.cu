@@ -43,7 +43,12 @@ namespace {
 constexpr int kGemmFoldThreads = 256;    // two per weight row: each folds half of the tile's activation columns
 constexpr int kGemmUnpackThreads = 128;  // one per weight row
 constexpr int kGemmThreads = kGemmFoldThreads + kGemmUnpackThreads + 128;  // + a warpgroup with the two TMA warps and the MMA warp
-constexpr int kGemmUnpackWarp0 = 8, kGemmXWarp = 12, kGemmMmaWarp = 13, kGemmWWarp = 14;
+constexpr int kGemmUnpackWarp0 = 8, kGemmXWarp = 12, kGemmMmaWarp = 13, kGemmWWarp = 14, kGemmUnpackWarp1 = 16;
+// Sets of unpacking warps, which take the groups in turn.  A set needs 1100 clocks a group (600 of work, the rest two waits and the
+// fences); at more than 128 rows the MMAs take as long.  Up to 128 rows a second
+// set brings gate/up 5120 x 17408 from 49.7 to 46.9 us at 77 rows and from 52.2 to 48.0 at 128, 5120 x 14336 at 128 from 26.7 to 24.2.
+constexpr int gemm_unpack_sets(int nc) { return nc <= 2 ? 2 : 1; }
+constexpr int gemm_threads(int nc) { return kGemmThreads + (gemm_unpack_sets(nc) - 1) * kGemmUnpackThreads; }
 constexpr int kGemmTileN = 128;   // weight rows of one CTA of a pair (gate/up: 64 of each)
 constexpr int kGemmTileM = 256;   // most activation rows per tile (the MMA's N)
 constexpr int kSwizzleK = 64;     // k of one 128-byte swizzle row of fp16
@@ -57,9 +62,11 @@ constexpr int kAHalfBytes = kGemmTileN * kSwizzleK * 2;         // 16 KB: 64 k o
 constexpr int kASlotBytes = 2 * kAHalfBytes;
 constexpr int kGemmTmemCols = 512;
 constexpr int kGemmMaxProj = 4;
-// Register split of the launch's 512 x 128: the fold keeps 128 sums per thread.
-constexpr int kFoldRegs = 208, kUnpackRegs = 64, kCtrlRegs = 32;
-static_assert(kFoldRegs * 256 + kUnpackRegs * 128 + kCtrlRegs * 128 <= 65536, "register split");
+// Register split of the launch's 512 x 128, or 640 x 96: the fold keeps 128, or 64, sums per thread.
+constexpr int kUnpackRegs = 64, kCtrlRegs = 32;
+constexpr int gemm_fold_regs(int nc) { return nc <= 2 ? 144 : 208; }
+constexpr int gemm_split_regs(int nc) { return gemm_fold_regs(nc) * 256 + kUnpackRegs * 128 * gemm_unpack_sets(nc) + kCtrlRegs * 128; }
+static_assert(gemm_split_regs(4) <= 512 * 128 && gemm_split_regs(2) <= 640 * 96, "register split");
 
 struct GemmCtrl {
     uint64_t w_full[kWSlotsMax], w_empty[kWSlotsMax];
@@ -218,7 +225,7 @@ __device__ __forceinline__ int proj_of_tile(const GemmParams& p, int tile) {
 
 // NC: 32-column reads a fold thread makes of an accumulator tile, ceil(tile_m / 64).
 template <int NC, typename OutT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a16_gemm_kernel(const __grid_constant__ GemmParams p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1) w4a16_gemm_kernel(const __grid_constant__ GemmParams p) {
     extern __shared__ uint8_t gemm_smem_raw[];
     // (the control block first: its addresses are then constants, and the fold, which needs every register, holds none of them)
     GemmCtrl* ctrl = reinterpret_cast<GemmCtrl*>(gemm_smem_raw);
@@ -263,7 +270,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
     const int U = static_cast<int>(u1 - u0);
     const int first_tile = static_cast<int>(u0 / p.groups), first_group = static_cast<int>(u0 - static_cast<long long>(first_tile) * p.groups);
 
-    if (warp >= kGemmXWarp) {
+    constexpr int kSets = gemm_unpack_sets(NC);
+    if (warp >= kGemmXWarp && warp < kGemmUnpackWarp1) {
         setmaxnreg_dec<kCtrlRegs>();
         if (warp == kGemmWWarp) {
             // -------------------------------------------------------------- TMA: packed weights (whole warp waits, one lane issues)
@@ -378,15 +386,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
     } else if (warp >= kGemmUnpackWarp0) {
         // ------------------------------------------------------------------ unpack: one thread per weight row of the tile
         setmaxnreg_dec<kUnpackRegs>();
-        const int r = tid - kGemmFoldThreads;
+        const int r = tid & (kGemmUnpackThreads - 1), set = warp >= kGemmUnpackWarp1 ? 1 : 0;
         // raw rows of 64 bytes under the 64-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ ((r >> 1) & 3)
         const uint32_t w_row = static_cast<uint32_t>(r) * 64, w_sw = static_cast<uint32_t>((r >> 1) & 3);
         // gate/up: the raw tile is 64 rows of each, the operand sixteen and sixteen, so that a feature's two sums meet in one warp
         const int ra = p.swiglu ? ((r & 48) << 1) + ((r >> 6) << 4) + (r & 15) : r;
         const uint32_t a_row = static_cast<uint32_t>((ra >> 3) * 1024 + (ra & 7) * 128), a_sw = static_cast<uint32_t>(ra & 7);
-        int wslot = 0, aslot = 0;
+        int wslot = set, aslot = set;  // (both rings have three slots at least)
         uint32_t w_phase = 0, a_phase = 1;
-        for (int i = 0; i < U; ++i) {
+        for (int i = set; i < U; i += kSets) {
             if (!mbar_wait(smem_u32(&ctrl->w_full[wslot]), w_phase, ws)) break;
             const uint32_t wsrc = smem_u32(w_ring) + wslot * kWSlotBytes + w_row;
             uint4 v[4];
@@ -412,12 +420,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) w4a
                 mbar_arrive_cluster(mapa_shared_cluster(smem_u32(&ctrl->op_full[aslot]), 0));
                 mbar_arrive(smem_u32(&ctrl->w_empty[wslot]));
             }
-            if (++aslot == op_slots) { aslot = 0; a_phase ^= 1u; }
-            if (++wslot == w_slots) { wslot = 0; w_phase ^= 1u; }
+            if ((aslot += kSets) >= op_slots) { aslot -= op_slots; a_phase ^= 1u; }
+            if ((wslot += kSets) >= w_slots) { wslot -= w_slots; w_phase ^= 1u; }
         }
     } else {
         // ------------------------------------------------------------------ fold, then write: two threads per weight row
-        setmaxnreg_inc<kFoldRegs>();
+        setmaxnreg_inc<gemm_fold_regs(NC)>();
         const int r = tid & 127, ch = tid >> 7;          // tile row, column half
         const int half_cols = p.tile_m >> 1;             // a multiple of 16
         const uint32_t d_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(ch * half_cols);
@@ -666,14 +674,13 @@ cudaError_t gemm_configure_and_launch(const GemmParams& p, dim3 grid, cudaStream
             cudaFuncAttributes a;
             e = cudaFuncGetAttributes(&a, w4a16_gemm_kernel<NC, OutT>);
             if (e != cudaSuccess) return e;
-            if (a.numRegs * kGemmThreads < kFoldRegs * kGemmFoldThreads + kUnpackRegs * kGemmUnpackThreads + kCtrlRegs * 128)
-                return cudaErrorLaunchOutOfResources;
+            if (a.numRegs * gemm_threads(NC) < gemm_split_regs(NC)) return cudaErrorLaunchOutOfResources;
             e = cudaFuncSetAttribute(w4a16_gemm_kernel<NC, OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemBytes);
             if (e != cudaSuccess) return e;
             configured[dev] = true;
         }
     }
-    return launch_pdl(w4a16_gemm_kernel<NC, OutT>, grid, dim3(kGemmThreads), kGemmSmemBytes, stream, p);
+    return launch_pdl(w4a16_gemm_kernel<NC, OutT>, grid, dim3(gemm_threads(NC)), kGemmSmemBytes, stream, p);
 }
 
 template <typename OutT>
