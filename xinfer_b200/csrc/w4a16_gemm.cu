@@ -126,22 +126,28 @@ struct GemmParams {
 // D[tmem] (+)= A[smem descriptor] * B[smem descriptor], kind::f16, on a CTA pair: A and D rows 0-127 in the even CTA,
 // 128-255 in the odd one; B rows half and half, each CTA's at the descriptor's offset.  Issued by one thread of the even CTA.
 __device__ __forceinline__ void umma_ss_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                 uint32_t accumulate) {
+                                                 uint32_t accumulate, uint32_t issue) {
     asm volatile(
         "{\n\t"
-        ".reg .pred p;\n\t"
+        ".reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
         "}"
         :
-        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(issue)
         : "memory");
 }
 // Arrives on the mbarrier at this offset in both CTAs of the pair when every MMA issued so far has completed.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-                 "h"(static_cast<uint16_t>(3))
-                 : "memory");
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint32_t issue) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t"
+        "}" ::"r"(bar),
+        "h"(static_cast<uint16_t>(3)), "r"(issue)
+        : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
@@ -364,21 +370,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
             uint32_t slot = 0, phase = 0;
             for (int i = 0; i < U && ok; ++i) {
                 const uint32_t buf = static_cast<uint32_t>(i & (d_bufs - 1));
-                if (i >= d_bufs && !mbar_wait_parked(smem_u32(&ctrl->d_empty[buf]), ((i >> d_shift) & 1u) ^ 1u, ws)) break;
-                ok = mbar_wait_parked(smem_u32(&ctrl->op_full[slot]), phase, ws);
+                // (both asked before either answer is looked at: an answer takes a hundred clocks, also where there is nothing to wait for)
+                const uint32_t d_bar = smem_u32(&ctrl->d_empty[buf]), d_phase = ((i >> d_shift) & 1u) ^ 1u, op_bar = smem_u32(&ctrl->op_full[slot]);
+                const bool d_ready = mbar_try_wait(d_bar, d_phase), op_ready = mbar_try_wait(op_bar, phase);  // (an unused tile is ready)
+                ok = (d_ready || mbar_wait_parked(d_bar, d_phase, ws)) && (op_ready || mbar_wait_parked(op_bar, phase, ws));
                 if (!ok) break;
                 tc_fence_after_sync();
-                if (leader) {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const uint32_t alo = desc_lo_const | (a_lo0 + ((slot * kASlotBytes + (k >> 2) * kAHalfBytes + (k & 3) * 32) >> 4));
-                        const uint32_t xlo = desc_lo_const | (x_lo0 + ((slot * 2 * x_half_bytes + (k >> 2) * x_half_bytes + (k & 3) * 32) >> 4));
-                        umma_ss_f16_pair(tmem_base + buf * d_cols, (static_cast<uint64_t>(desc_hi) << 32) | alo,
-                                         (static_cast<uint64_t>(desc_hi) << 32) | xlo, idesc, k > 0 ? 1u : 0u);
-                    }
-                    umma_commit_pair(smem_u32(&ctrl->op_empty[slot]));
-                    umma_commit_pair(smem_u32(&ctrl->d_full[buf]));
+                for (int k = 0; k < 8; ++k) {
+                    const uint32_t alo = desc_lo_const | (a_lo0 + ((slot * kASlotBytes + (k >> 2) * kAHalfBytes + (k & 3) * 32) >> 4));
+                    const uint32_t xlo = desc_lo_const | (x_lo0 + ((slot * 2 * x_half_bytes + (k >> 2) * x_half_bytes + (k & 3) * 32) >> 4));
+                    umma_ss_f16_pair(tmem_base + buf * d_cols, (static_cast<uint64_t>(desc_hi) << 32) | alo,
+                                     (static_cast<uint64_t>(desc_hi) << 32) | xlo, idesc, k > 0 ? 1u : 0u, leader);
                 }
+                umma_commit_pair(smem_u32(&ctrl->op_empty[slot]), leader);
+                umma_commit_pair(smem_u32(&ctrl->d_full[buf]), leader);
                 __syncwarp();
                 if (++slot == static_cast<uint32_t>(op_slots)) { slot = 0; phase ^= 1u; }
             }
@@ -395,12 +401,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
         int wslot = set, aslot = set;  // (both rings have three slots at least)
         uint32_t w_phase = 0, a_phase = 1;
         for (int i = set; i < U; i += kSets) {
-            if (!mbar_wait(smem_u32(&ctrl->w_full[wslot]), w_phase, ws)) break;
+            const uint32_t w_bar = smem_u32(&ctrl->w_full[wslot]), a_bar = smem_u32(&ctrl->op_empty[aslot]);
+            const bool w_ready = mbar_try_wait(w_bar, w_phase), a_ready = mbar_try_wait(a_bar, a_phase);  // (as in the MMA warp)
+            if (!w_ready && !mbar_wait(w_bar, w_phase, ws)) break;
             const uint32_t wsrc = smem_u32(w_ring) + wslot * kWSlotBytes + w_row;
             uint4 v[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) v[c] = lds128(wsrc + ((static_cast<uint32_t>(c) ^ w_sw) << 4));
-            if (!mbar_wait(smem_u32(&ctrl->op_empty[aslot]), a_phase, ws)) break;
+            if (!a_ready && !mbar_wait(a_bar, a_phase, ws)) break;
             const uint32_t adst = smem_u32(a_ring) + aslot * kASlotBytes + a_row;
 #pragma unroll
             for (int w = 0; w < 16; ++w) {
