@@ -94,6 +94,7 @@ struct Cfg {
     static constexpr int kCtrlBytes = 512;
     static constexpr int kSmemBytes = kWRingBytes + kXRingBytes + kXchgBytes + kCtrlBytes + 1024;  // + align slack
     static_assert(kSmemBytes <= 196 * 1024, "rings sized to leave L1 for the scale loads");
+    static_assert(kStages <= 4 && kXStages <= 6, "barriers of the control block");
 };
 
 struct Seg {
@@ -140,14 +141,17 @@ struct Params {
 };
 
 struct Ctrl {
-    uint64_t full[8];     // weights of a stage have landed
-    uint64_t empty[8];    // every consumer warp has unpacked them
-    uint64_t x_full[8];   // activations of a stage have landed
-    uint64_t x_ready[8];  // the reorder warp has rewritten them in the unpack's k order
-    uint64_t x_empty[8];  // both halves' MMAs that read them have completed
+    uint64_t full[4];     // weights of a stage have landed
+    uint64_t empty[4];    // every consumer warp has unpacked them
+    uint64_t x_full[6];   // activations of a stage have landed
+    uint64_t x_ready[6];  // the reorder warp has rewritten them in the unpack's k order
+    uint64_t x_empty[6];  // both halves' MMAs that read them have completed
     uint64_t a_full[2][2];
     uint64_t d_full[2][2];
     uint64_t epi;         // epilogue barrier of the consumer warps
+    uint64_t epi_groups[8];  // whole tiles: the two warps of 32 rows (one per group) have traded their sums
+    uint64_t epi_halves[8];  // ... the gate and the up warp of 32 features theirs
+    uint64_t epi_read[4];    // ... and the four warps of a quarter have read what the others left
     uint64_t red;         // counts the bytes of split-K partials that other CTAs of the cluster store here
     uint32_t tmem_base;
     int is_last;
@@ -253,6 +257,10 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                 mbar_init(smem_u32(&ctrl->d_full[w][b]), 1);
             }
         mbar_init(smem_u32(&ctrl->epi), kConsumerThreads / 32);
+        if (NREAD > 8 && p.cluster == 1) {
+            for (int i = 0; i < 8; ++i) { mbar_init(smem_u32(&ctrl->epi_groups[i]), 2); mbar_init(smem_u32(&ctrl->epi_halves[i]), 2); }
+            for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&ctrl->epi_read[i]), 4);
+        }
         mbar_init(smem_u32(&ctrl->red), 1);
         if (p.cluster > 1) {
             // bytes this CTA will receive: every CTA of the cluster (itself included) sends 256 floats for each
@@ -553,10 +561,15 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
             }
         };
 
+        // The scale of this warp's group is fetched two stages ahead as a raw 16-bit value and only
+        // converted when its stage starts, so the load latency never sits in the loop's critical path; a tile's first two
+        // are asked for before the epilogue of the tile in front of it.
+        uint32_t q0 = 0u, q1 = 0u;
+        uint32_t quick_phase = 0;   // of the whole tiles' barriers
+        bool stage_acc_free = true; // nobody else may still be reading stage_acc
         long long u = u_begin;
+        int tile = static_cast<int>(u_begin / S), s0 = static_cast<int>(u_begin - static_cast<long long>(tile) * S);
         while (u < u_end && ok) {
-            const int tile = static_cast<int>(u / S);
-            const int s0 = static_cast<int>(u - static_cast<long long>(tile) * S);
             const int s1 = static_cast<int>(min(static_cast<long long>(S), s0 + (u_end - u)));
             const TileInfo ti = locate_tile(p, tile);
             const Seg& sg = p.seg[p.swiglu ? wg : ti.seg];
@@ -584,16 +597,16 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
 #pragma unroll
             for (int j = 0; j < NREAD; ++j) acc[j] = 0.f;
 
-            // The scale of this warp's group is fetched two stages ahead as a raw 16-bit value and only
-            // converted when its stage starts, so the load latency never sits in the loop's critical path.
             // The loop's bookkeeping is kept to running pointers and counters: the SM is issue-bound here and
             // every instruction of a consumer warp is paid sixteen-fold.
             const unsigned short* sp = reinterpret_cast<const unsigned short*>(my_scales) + 2 * s0 + gi;  // this stage's scale
             // stages [s0, s_lim) have a scale for this thread (none for rows beyond N; K/128 odd: group 1 of the last)
             const int s_lim = min(s1, (gmax - gi + 1) >> 1);
             float sc_pend = 0.f;
-            uint32_t q0 = (s0 < s_lim) ? static_cast<uint32_t>(__ldg(sp)) : 0u;
-            uint32_t q1 = (s0 + 1 < s_lim) ? static_cast<uint32_t>(__ldg(sp + 2)) : 0u;
+            if (u == u_begin) {
+                q0 = (s0 < s_lim) ? static_cast<uint32_t>(__ldg(sp)) : 0u;
+                q1 = (s0 + 1 < s_lim) ? static_cast<uint32_t>(__ldg(sp + 2)) : 0u;
+            }
             bool have_prev = false;
             uint32_t slot = n % C::kStages;                 // weight-ring slot and phase of stage n
             uint32_t full_phase = (n / C::kStages) & 1u;
@@ -652,6 +665,16 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                 have_prev = true;
             }
             if (!ok) break;
+            const long long u_next = u + (s1 - s0);
+            if (u_next < u_end) {
+                const TileInfo tn = locate_tile(p, tile + 1);
+                const Seg& sn = p.seg[p.swiglu ? wg : tn.seg];
+                const int row_n = p.swiglu ? tn.row0 + t : tn.row0 + rt;
+                const unsigned short* sq = reinterpret_cast<const unsigned short*>(sn.scales) + static_cast<long long>(row_n) * p.groups + gi;
+                const int lim = row_n < sn.n ? static_cast<int>(min(static_cast<long long>((p.groups - gi + 1) >> 1), u_end - u_next)) : 0;
+                q0 = lim > 0 ? static_cast<uint32_t>(__ldg(sq)) : 0u;
+                q1 = lim > 1 ? static_cast<uint32_t>(__ldg(sq + 2)) : 0u;
+            }
             // drain the tile's last stage (n already counts it)
             if (!mbar_wait(dfull, (n - 1) & 1u, abort_flag)) { ok = false; break; }
             tc_fence_after_sync();
@@ -666,6 +689,78 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
             const int m_rows = p.m < NREAD ? p.m : NREAD;
             const bool whole = (s0 == 0 && s1 == S);
             const bool direct_xchg = !whole && p.cluster > 1 && p.xchg_direct;
+            if (NREAD > 8 && whole && p.cluster == 1 && p.seg[p.swiglu ? 0 : ti.seg].push == 0) {
+                // A whole tile's sums never leave their four warps.  The two that share a row trade halves of the activation rows (each
+                // adds what the other one left for it); of gate/up, the gate and the up warp then trade halves of those, so that each of
+                // the four finishes a quarter.  Barriers of two warps, and stores straight from registers: through the parked rows
+                // below, with barriers of all sixteen warps, a tile of 32 activation rows took 8000 clocks after its twenty stages of
+                // 2000 each.
+                constexpr int H = NREAD / 2;
+                if (!stage_acc_free) {
+                    if (!consumer_sync()) break;
+                    stage_acc_free = true;
+                } else if (!mbar_wait(smem_u32(&ctrl->epi_read[quarter]), quick_phase ^ 1u, abort_flag)) {  // (passes at once the first time)
+                    ok = false;
+                    break;
+                }
+                float* const cell = stage_acc + rt;  // of activation row j: cell[j * kTileRows]
+                float sum[H];
+#pragma unroll
+                for (int j = 0; j < H; ++j) {
+                    cell[(gi == 0 ? H + j : j) * kTileRows] = gi == 0 ? acc[H + j] : acc[j];
+                    sum[j] = gi == 0 ? acc[j] : acc[H + j];
+                }
+                auto trade = [&](uint64_t* bar) -> bool {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(bar));
+                    return mbar_wait(smem_u32(bar), quick_phase, abort_flag);
+                };
+                if (!trade(&ctrl->epi_groups[wg * 4 + quarter])) { ok = false; break; }
+#pragma unroll
+                for (int j = 0; j < H; ++j) sum[j] += cell[(gi * H + j) * kTileRows];
+                OutT* const y = static_cast<OutT*>(p.seg[p.swiglu ? 0 : ti.seg].y) + my_col;
+                const long long ldy = p.seg[p.swiglu ? 0 : ti.seg].ldy;
+                if (!p.swiglu) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&ctrl->epi_read[quarter]));
+                    const float b = (valid && sg.bias) ? sg.bias[my_row] : 0.f;
+                    const int live = valid ? m_rows - gi * H : 0;
+                    OutT* o = y + gi * H * ldy;
+#pragma unroll
+                    for (int j = 0; j < H; ++j, o += ldy)
+                        if (j < live) store_out<OutT>(o, sum[j] + b);
+                } else {
+                    constexpr int Q = H / 2;
+                    // the up warp finishes the second half of this group's activation rows, the gate warp the first
+                    float mine[Q];
+#pragma unroll
+                    for (int j = 0; j < Q; ++j) {
+                        cell[(gi * H + (wg == 0 ? Q + j : j)) * kTileRows] = wg == 0 ? sum[Q + j] : sum[j];
+                        mine[j] = wg == 0 ? sum[j] : sum[Q + j];
+                    }
+                    if (!trade(&ctrl->epi_halves[gi * 4 + quarter])) { ok = false; break; }
+                    const float* const theirs = stage_acc + (wg == 0 ? kHalfRows + t : t) + (gi * H + wg * Q) * kTileRows;
+                    const int live = valid ? m_rows - gi * H - wg * Q : 0;
+                    OutT* o = y + (gi * H + wg * Q) * ldy;
+                    float v[Q];  // (all before the first store; no branch in the division: an exact one each in turn)
+#pragma unroll
+                    for (int j = 0; j < Q; ++j) {
+                        const float other = theirs[j * kTileRows];
+                        const float g = wg == 0 ? mine[j] : other, up = wg == 0 ? other : mine[j];
+                        v[j] = __fdividef(g, 1.0f + expf(-g)) * up;
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&ctrl->epi_read[quarter]));
+#pragma unroll
+                    for (int j = 0; j < Q; ++j, o += ldy)
+                        if (j < live) store_out<OutT>(o, v[j]);
+                }
+                quick_phase ^= 1u;
+                u += s1 - s0;
+                s0 = 0;
+                ++tile;
+                continue;
+            }
             if (!direct_xchg) {
             if (!consumer_sync()) break;  // previous tile's readers of stage_acc are done
             if (gi == 0) {
@@ -857,7 +952,10 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                         store_row<OutT>(p, sg, my_col + static_cast<long long>(j) * ldy, j, stage_acc[j * kTileRows + rt] + b);
                 }
             }
+            stage_acc_free = false;
             u += (s1 - s0);
+            s0 = 0;
+            ++tile;
         }
         // every thread of a cluster passes both cluster barriers exactly once, also when a wait gave up
         if (p.cluster > 1) {
