@@ -32,7 +32,7 @@
 // split evenly over one CTA per SM; a tile finished by several CTAs is summed by the last one to
 // arrive, in CTA order, from fp32 partials in a scratch buffer (deterministic, no float atomics).
 // With fewer tiles, each tile's K range is split over a thread-block cluster that sums through
-// distributed shared memory (bulk copies that count bytes on the receiver's mbarrier).
+// distributed shared memory (plain remote stores between two cluster barriers).
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -126,7 +126,6 @@ struct Params {
     long long wait_limit;  // SM clocks after which a device-side wait gives up
     int x_stage_limit;     // test hook: activation stages beyond this index are never requested (-1: off)
     TpLink tp;             // N-split exchange (world <= 1: none)
-    int xchg_direct;       // cluster split-K partials go by plain remote stores (1) or by bulk copies (0)
     int x_perm;            // X is stored in the unpack's k order already: no in-kernel reorder of the staged activations
     int y_perm;            // write Y with its columns in that order (it is the X of another such launch)
     // Optional: the first weight stages of the NEXT tensor-core launch in the stream, pulled into L2 while this
@@ -149,10 +148,9 @@ struct Ctrl {
     uint64_t a_full[2][2];
     uint64_t d_full[2][2];
     uint64_t epi;         // epilogue barrier of the consumer warps
-    uint64_t epi_groups[8];  // whole tiles: the two warps of 32 rows (one per group) have traded their sums
-    uint64_t epi_halves[8];  // ... the gate and the up warp of 32 features theirs
+    uint64_t epi_groups[8];  // whole tiles, cluster splits: the two warps of 32 rows (one per group) have traded their sums
+    uint64_t epi_halves[8];  // whole tiles: the gate and the up warp of 32 features theirs
     uint64_t epi_read[4];    // ... and the four warps of a quarter have read what the others left
-    uint64_t red;         // counts the bytes of split-K partials that other CTAs of the cluster store here
     uint32_t tmem_base;
     int is_last;
     WaitState ws;
@@ -257,20 +255,12 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                 mbar_init(smem_u32(&ctrl->d_full[w][b]), 1);
             }
         mbar_init(smem_u32(&ctrl->epi), kConsumerThreads / 32);
-        if (NREAD > 8 && p.cluster == 1) {
-            for (int i = 0; i < 8; ++i) { mbar_init(smem_u32(&ctrl->epi_groups[i]), 2); mbar_init(smem_u32(&ctrl->epi_halves[i]), 2); }
-            for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&ctrl->epi_read[i]), 4);
-        }
-        mbar_init(smem_u32(&ctrl->red), 1);
-        if (p.cluster > 1) {
-            // bytes this CTA will receive: every CTA of the cluster (itself included) sends 256 floats for each
-            // activation row this CTA finishes (a contiguous block of ceil(m / cluster) rows per rank)
-            const int m_rows = p.m < NREAD ? p.m : NREAD;
-            const int rank = static_cast<int>(cluster_ctarank());
-            const int rows_cap = (m_rows + p.cluster - 1) / p.cluster;
-            int owned = m_rows - rank * rows_cap;
-            owned = owned < 0 ? 0 : (owned > rows_cap ? rows_cap : owned);
-            mbar_arrive_expect_tx(smem_u32(&ctrl->red), static_cast<uint32_t>(p.cluster * owned * kTileRows * 4));
+        if (NREAD > 8) {
+            for (int i = 0; i < 8; ++i) mbar_init(smem_u32(&ctrl->epi_groups[i]), 2);
+            if (p.cluster == 1) {
+                for (int i = 0; i < 8; ++i) mbar_init(smem_u32(&ctrl->epi_halves[i]), 2);
+                for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&ctrl->epi_read[i]), 4);
+            }
         }
         ctrl->ws.abort_flag = 0;
         ctrl->ws.dep_ready = 0;
@@ -688,7 +678,6 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
             float* stage_acc = xchg;  // [NREAD][256] fp32, row rt's values at [j][rt]
             const int m_rows = p.m < NREAD ? p.m : NREAD;
             const bool whole = (s0 == 0 && s1 == S);
-            const bool direct_xchg = !whole && p.cluster > 1 && p.xchg_direct;
             if (NREAD > 8 && whole && p.cluster == 1 && p.seg[p.swiglu ? 0 : ti.seg].push == 0) {
                 // A whole tile's sums never leave their four warps.  The two that share a row trade halves of the activation rows (each
                 // adds what the other one left for it); of gate/up, the gate and the up warp then trade halves of those, so that each of
@@ -761,42 +750,60 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                 ++tile;
                 continue;
             }
-            if (!direct_xchg) {
-            if (!consumer_sync()) break;  // previous tile's readers of stage_acc are done
-            if (gi == 0) {
+            if (p.cluster == 1) {
+                if (!consumer_sync()) break;  // previous tile's readers of stage_acc are done
+                if (gi == 0) {
 #pragma unroll
-                for (int j = 0; j < NREAD; ++j) stage_acc[j * kTileRows + rt] = acc[j];
-            }
-            if (!consumer_sync()) break;
-            if (gi == 1) {
+                    for (int j = 0; j < NREAD; ++j) stage_acc[j * kTileRows + rt] = acc[j];
+                }
+                if (!consumer_sync()) break;
+                if (gi == 1) {
 #pragma unroll
-                for (int j = 0; j < NREAD; ++j) stage_acc[j * kTileRows + rt] += acc[j];
-            }
-            fence_proxy_async_smem();  // the copy engine may read the parked rows (split-K exchange)
-            if (!consumer_sync()) break;
+                    for (int j = 0; j < NREAD; ++j) stage_acc[j * kTileRows + rt] += acc[j];
+                }
+                if (!consumer_sync()) break;
             }
             bool finish = whole;
             int j0 = gi, jstep = 2, jend = m_rows;  // activation rows this thread finishes: j0, j0 + jstep, ... < jend
-            if (direct_xchg) {
+            if (p.cluster > 1) {
                 // K splits of one tile form a thread-block cluster.  CTA r of the cluster finishes a contiguous block
                 // of activation rows (ceil(m / cluster) of them).  Every thread stores its fp32 partials straight from
                 // its registers into the owner's shared memory (the weight ring, free once every CTA has arrived at
-                // barrier A): [sender][group][row of the block][256 features].  One cluster barrier later the owner
-                // adds the two groups of every sender and then the senders in rank order (deterministic).
+                // barrier A).  One cluster barrier later the owner adds the senders in rank order (deterministic).
+                // Up to eight activation rows: [sender][group][row of the block][256 features], the owner adds a sender's two
+                // groups.  More: the two warps of a row first trade halves of the activation rows and each sends the sums of its half,
+                // [sender][row][256].  (Parked rows sent by the copy engine, one copy per receiver, took 2.3 us from the last stage to
+                // the sums at 32 rows; this 1.3.)
                 float* part = reinterpret_cast<float*>(smem);
                 const uint32_t my_rank = cluster_ctarank();
                 const uint32_t csz = static_cast<uint32_t>(p.cluster);
                 const uint32_t rows_cap = (static_cast<uint32_t>(m_rows) + csz - 1) / csz;
+                constexpr bool kPairSums = NREAD > 8;
+                constexpr int kSend = kPairSums ? NREAD / 2 : NREAD;
+                const uint32_t first = kPairSums ? gi * kSend : 0;  // activation rows first .. first + kSend - 1 are this thread's to send
+                if constexpr (kPairSums) {
+                    float* const cell = stage_acc + rt;  // of activation row j: cell[j * kTileRows]
+#pragma unroll
+                    for (int j = 0; j < kSend; ++j) {
+                        cell[(gi == 0 ? kSend + j : j) * kTileRows] = gi == 0 ? acc[kSend + j] : acc[j];
+                        if (gi == 1) acc[j] = acc[kSend + j];
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&ctrl->epi_groups[wg * 4 + quarter]));
+                    if (!mbar_wait(smem_u32(&ctrl->epi_groups[wg * 4 + quarter]), 0u, abort_flag)) { ok = false; break; }  // (one tile a launch)
+#pragma unroll
+                    for (int j = 0; j < kSend; ++j) acc[j] += cell[(first + j) * kTileRows];
+                }
                 if (cl_steps == 0) { cluster_arrive(); cl_steps = 1; }
                 cluster_wait();  // (A) every CTA of the cluster has finished reading its weight ring
                 cl_steps = 2;
                 {
-                    const uint32_t local = smem_u32(part) + (((my_rank * 2 + gi) * rows_cap) * kTileRows + rt) * 4;
-                    uint32_t owner = 0, jl = 0;
-                    uint32_t dst = mapa_shared_cluster(local, 0);
+                    const uint32_t local = smem_u32(part) + (((kPairSums ? my_rank : my_rank * 2 + gi) * rows_cap) * kTileRows + rt) * 4;
+                    uint32_t owner = first / rows_cap, jl = first - owner * rows_cap;
+                    uint32_t dst = mapa_shared_cluster(local, owner < csz ? owner : 0) + jl * (kTileRows * 4);
 #pragma unroll
-                    for (int j = 0; j < NREAD; ++j) {
-                        if (j < m_rows) {
+                    for (int j = 0; j < kSend; ++j) {
+                        if (static_cast<int>(first) + j < m_rows) {
                             st_shared_cluster_f32(dst, acc[j]);
                             dst += kTileRows * 4;
                             if (++jl == rows_cap) {
@@ -812,58 +819,6 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                 cluster_wait();    // ... and acquires everyone's: this CTA's block is complete
                 cl_steps = 4;
                 {
-                    const bool direct = !p.swiglu && valid;
-                    const long long ldy = sg.ldy;
-                    const float bias = (direct && sg.bias) ? sg.bias[my_row] : 0.f;
-                    const uint32_t jfirst = my_rank * rows_cap;
-                    uint32_t jlast = jfirst + rows_cap;
-                    jlast = jlast > static_cast<uint32_t>(m_rows) ? static_cast<uint32_t>(m_rows) : jlast;
-                    uint32_t j = jfirst + gi;
-                    long long yoff = my_col + static_cast<long long>(j) * ldy;
-                    uint32_t pa = smem_u32(part) + (gi * kTileRows + rt) * 4;  // row gi of the block, sender 0, group 0
-                    const uint32_t gstep = rows_cap * (kTileRows * 4);           // group 0 -> group 1 of one sender
-                    float* sa = stage_acc + j * kTileRows + rt;
-#pragma unroll 1
-                    for (; j < jlast; j += 2, pa += 2 * kTileRows * 4, yoff += 2 * ldy, sa += 2 * kTileRows) {
-                        float sum = 0.f;
-                        uint32_t a = pa;
-#pragma unroll 2
-                        for (uint32_t r = 0; r < csz; ++r, a += 2 * gstep) sum += lds_f32(a) + lds_f32(a + gstep);
-                        if (direct) store_row<OutT>(p, sg, yoff, static_cast<int>(j), sum + bias);
-                        else *sa = sum;
-                    }
-                    j0 = static_cast<int>(jfirst) + gi;
-                    jend = static_cast<int>(jlast);
-                    finish = p.swiglu != 0;  // plain projections are already written
-                }
-            } else if (!whole && p.cluster > 1) {
-                // K splits of one tile form a thread-block cluster.  CTA r of the cluster finishes a contiguous
-                // block of activation rows (ceil(m / cluster) of them): every CTA sends its fp32 partials of
-                // that block, contiguous in the parked accumulators, into r's shared memory with ONE bulk copy
-                // that counts its bytes on r's mbarrier, so r waits for exactly its incoming data.  It then sums
-                // the `cluster` copies in rank order (deterministic).
-                float* part = reinterpret_cast<float*>(smem);  // the weight ring, free once every CTA has arrived
-                const uint32_t my_rank = cluster_ctarank();
-                const uint32_t csz = static_cast<uint32_t>(p.cluster);
-                const uint32_t rows_cap = (static_cast<uint32_t>(m_rows) + csz - 1) / csz;
-                if (cl_steps == 0) { cluster_arrive(); cl_steps = 1; }
-                cluster_wait();  // (A) every CTA of the cluster has finished reading its weight ring
-                cl_steps = 2;
-                if (warp == 0 && lane < static_cast<int>(csz)) {  // lane r sends the block owned by CTA r
-                    int nr = m_rows - lane * static_cast<int>(rows_cap);
-                    nr = nr > static_cast<int>(rows_cap) ? static_cast<int>(rows_cap) : nr;
-                    if (nr > 0) {
-                        const uint32_t dst = smem_u32(part) + (my_rank * rows_cap) * (kTileRows * 4);
-                        bulk_copy_to_cluster(mapa_shared_cluster(dst, lane),
-                                             smem_u32(stage_acc) + lane * rows_cap * (kTileRows * 4), nr * (kTileRows * 4),
-                                             mapa_shared_cluster(smem_u32(&ctrl->red), lane));
-                    }
-                }
-                if (!mbar_wait(smem_u32(&ctrl->red), 0u, abort_flag)) { ok = false; break; }
-                // (B) this CTA has all its incoming rows, so the senders' sources may go away; waited for at exit
-                cluster_arrive();
-                cl_steps = 3;
-                {
                     // this CTA's block of rows; the two threads of a tile row take every other one
                     const bool direct = !p.swiglu && valid;
                     const long long ldy = sg.ldy;
@@ -873,15 +828,25 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                     jlast = jlast > static_cast<uint32_t>(m_rows) ? static_cast<uint32_t>(m_rows) : jlast;
                     uint32_t j = jfirst + gi;
                     long long yoff = my_col + static_cast<long long>(j) * ldy;
-                    uint32_t pa = smem_u32(part) + (gi * kTileRows + rt) * 4;
-                    const uint32_t rstep = rows_cap * (kTileRows * 4);
+                    uint32_t pa = smem_u32(part) + (gi * kTileRows + rt) * 4;  // row gi of the block, sender 0, group 0
+                    const uint32_t gstep = rows_cap * (kTileRows * 4);           // group 0 -> group 1 of one sender, or the next sender
                     float* sa = stage_acc + j * kTileRows + rt;
 #pragma unroll 1
                     for (; j < jlast; j += 2, pa += 2 * kTileRows * 4, yoff += 2 * ldy, sa += 2 * kTileRows) {
                         float sum = 0.f;
-                        uint32_t a = pa;
+                        if constexpr (kPairSums) {
+                            float in[8];  // (every sender's requested before the first is added: the additions are a chain)
+#pragma unroll
+                            for (uint32_t r = 0; r < 8; ++r)
+                                if (r < csz) in[r] = lds_f32(pa + r * gstep);
+#pragma unroll
+                            for (uint32_t r = 0; r < 8; ++r)
+                                if (r < csz) sum += in[r];
+                        } else {
+                            uint32_t a = pa;
 #pragma unroll 2
-                        for (uint32_t r = 0; r < csz; ++r, a += rstep) sum += lds_f32(a);
+                            for (uint32_t r = 0; r < csz; ++r, a += 2 * gstep) sum += lds_f32(a) + lds_f32(a + gstep);
+                        }
                         if (direct) store_row<OutT>(p, sg, yoff, static_cast<int>(j), sum + bias);
                         else *sa = sum;
                     }
@@ -1316,9 +1281,6 @@ int tc_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num, b
         if (p.tp.wait_limit <= 0) p.tp.wait_limit = g_wait_limit;
     }
     p.x_stage_limit = g_x_stage_limit;
-    // few activation rows: the partials go by plain remote stores (less latency than parking them and starting a
-    // bulk copy per peer); more rows: the copy engine moves them (fewer instructions per CTA)
-    p.xchg_direct = m <= 8 ? 1 : 0;
     TcPlan& pl = cur_plan();
     if (pl.recording) {
         pl.entries.push_back(make_entry(proj, num, swiglu, out_f32, m, k));
