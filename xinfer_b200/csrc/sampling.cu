@@ -65,7 +65,7 @@ __device__ __forceinline__ unsigned long long nucleus_weight(float scaled, float
     return __float2ull_rn(expf(scaled - max_scaled) * 4294967296.0f);
 }
 
-// The partial of one chunk of the row at `l`, by a block; every thread gets it.
+// The partial of one chunk of the row at `l`, by a block, once in a launch; every thread gets it.
 __device__ __forceinline__ Partial chunk_partial(const float* l, int chunk, int vocab, float inv_t, int want_sum, int idx_offset) {
     const int base = chunk * kChunk;
     const int end = min(vocab, base + kChunk);
@@ -92,53 +92,39 @@ __device__ __forceinline__ Partial chunk_partial(const float* l, int chunk, int 
             }
         }
     }
-    // block argmax (value, lowest index)
-    __shared__ float s_v[kThreads / 32];
+    // Block argmax (value, lowest index) and, for the sum, the maximum of the scaled logits: scaling by a positive factor is monotone,
+    // also where it rounds two values together, so that is the scaled maximum.  (NaNs are passed over there and turn up in the sum.)
+    // Every thread merges the warps' values itself: one barrier here and one for the sum, where there were seven.
+    __shared__ float s_v[kThreads / 32], s_m[kThreads / 32], s_f[kThreads / 32];
     __shared__ int s_i[kThreads / 32];
-    __shared__ float s_f[kThreads / 32];
+    float ms = vals[0];
+#pragma unroll
+    for (int r = 1; r < 16; ++r) ms = fmaxf(ms, vals[r]);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, best, off);
         const int oi = __shfl_xor_sync(0xffffffffu, best_i, off);
         better(best, best_i, ov, oi);
+        ms = fmaxf(ms, __shfl_xor_sync(0xffffffffu, ms, off));
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) { s_v[warp] = best; s_i[warp] = best_i; }
+    if (lane == 0) { s_v[warp] = best; s_i[warp] = best_i; s_m[warp] = ms; }
     __syncthreads();
-    if (warp == 0) {
-        float v = (lane < kThreads / 32) ? s_v[lane] : -INFINITY;
-        int i = (lane < kThreads / 32) ? s_i[lane] : -1;
+    best = s_v[0];
+    best_i = s_i[0];
+    ms = s_m[0];
 #pragma unroll
-        for (int off = 4; off > 0; off >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, v, off);
-            const int oi = __shfl_xor_sync(0xffffffffu, i, off);
-            better(v, i, ov, oi);
-        }
-        if (lane == 0) { s_v[0] = v; s_i[0] = i; }
+    for (int w = 1; w < kThreads / 32; ++w) {
+        better(best, best_i, s_v[w], s_i[w]);
+        ms = fmaxf(ms, s_m[w]);
     }
-    __syncthreads();
     Partial res;
-    res.max_raw = s_v[0];
-    res.idx = s_i[0] < 0 ? -1 : s_i[0] + idx_offset;  // vocabulary slice of an N-split LM head: global token id
+    res.max_raw = best;
+    res.idx = best_i < 0 ? -1 : best_i + idx_offset;  // vocabulary slice of an N-split LM head: global token id
     res.max_scaled = 0.f;
     res.sum_exp = 0.f;
     if (want_sum) {
-        // maximum of the scaled logits: scaling by a positive factor is monotone but may round two
-        // values together, so take the maximum of the scaled values themselves
-        float ms = -INFINITY;
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            const int idx = base + ((r >> 2) * kThreads + threadIdx.x) * 4 + (r & 3);
-            if (idx < end) ms = fmaxf(ms, vals[r] * inv_t);
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) ms = fmaxf(ms, __shfl_xor_sync(0xffffffffu, ms, off));
-        __syncthreads();
-        if (lane == 0) s_f[warp] = ms;
-        __syncthreads();
-        ms = s_f[0];
-#pragma unroll
-        for (int w = 1; w < kThreads / 32; ++w) ms = fmaxf(ms, s_f[w]);
+        ms = fmaxf(ms, -INFINITY) * inv_t;  // (nothing but NaNs: -inf)
         float se = 0.f;
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
@@ -147,7 +133,6 @@ __device__ __forceinline__ Partial chunk_partial(const float* l, int chunk, int 
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) se += __shfl_xor_sync(0xffffffffu, se, off);
-        __syncthreads();
         if (lane == 0) s_f[warp] = se;
         __syncthreads();
         se = 0.f;
@@ -390,26 +375,39 @@ __global__ void __launch_bounds__(kThreads) sample_finish_kernel(const Partial* 
     const int row = blockIdx.x, tid = threadIdx.x;
     const Partial* P = partials + static_cast<long long>(row) * chunks;
     const float* l = logits + static_cast<long long>(row) * row_stride;
-    __shared__ float s_m, s_z, s_rest;
+    __shared__ float s_z, s_rest;
     __shared__ int s_chunk, s_thread;
     __shared__ float s_local[kThreads], s_prefix;
+    griddep_prologue();
+    // The chunks' maxima, sums and factors, read and worked out by as many threads as there are chunks; the sums over them are one
+    // thread's, in chunk order.  (More chunks than threads - a vocabulary beyond a million - are read as they come.)
+    __shared__ float s_cmax[kThreads], s_csum[kThreads], s_cexp[kThreads];
+    const bool staged = chunks <= kThreads;
+    if (staged && tid < chunks) {
+        s_cmax[tid] = P[tid].max_scaled;
+        s_csum[tid] = P[tid].sum_exp;
+    }
+    __syncthreads();
+    float m = -INFINITY;
+    for (int c = 0; c < chunks; ++c) m = fmaxf(m, staged ? s_cmax[c] : P[c].max_scaled);
+    if (staged && tid < chunks) s_cexp[tid] = expf(s_cmax[tid] - m);
+    __syncthreads();
     if (tid == 0) {
-        float m = -INFINITY;
-        for (int c = 0; c < chunks; ++c) m = fmaxf(m, P[c].max_scaled);
+        auto sum_of = [&](int c) { return staged ? s_csum[c] : P[c].sum_exp; };
+        auto factor = [&](int c) { return staged ? s_cexp[c] : expf(P[c].max_scaled - m); };
         float z = 0.f;
-        for (int c = 0; c < chunks; ++c) z += P[c].sum_exp * expf(P[c].max_scaled - m);
+        for (int c = 0; c < chunks; ++c) z += sum_of(c) * factor(c);
         const float target = uniforms[static_cast<long long>(row) * u_stride] * z;
         float before = 0.f;
         int pick = chunks - 1;
         for (int c = 0; c < chunks; ++c) {
-            const float w = P[c].sum_exp * expf(P[c].max_scaled - m);
+            const float w = sum_of(c) * factor(c);
             if (before + w > target) { pick = c; break; }
             if (c + 1 < chunks) before += w;
         }
-        s_m = m; s_z = z; s_chunk = pick; s_rest = target - before;
+        s_z = z; s_chunk = pick; s_rest = target - before;
     }
     __syncthreads();
-    const float m = s_m;
     const int base = s_chunk * kChunk + tid * 16;
     float e[16];
     float local = 0.f;
@@ -575,6 +573,7 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
     const int cspan = (((vocab + kNucCluster - 1) / kNucCluster) + 31) & ~31;
     const int c0 = min(vocab, crank * cspan), c1 = min(vocab, c0 + cspan);
 
+    griddep_prologue();
     const bool in_regs = cspan <= kNucRegs * kNucThreads;
     float v[kNucRegs];  // scaled logits of the tokens c0 + j * 1024 + tid
 
@@ -1030,17 +1029,14 @@ int add_counter(cudaStream_t stream, unsigned long long* counter_dev, unsigned l
 int sample_finish(cudaStream_t stream, const void* partials, int chunks, const float* logits, long long row_stride,
                   long long vocab, float inv_temperature, const float* uniforms, int u_stride, int rows, long long* tok_out,
                   float* prob_out, int prob_stride) {
-    sample_finish_kernel<<<rows, kThreads, 0, stream>>>(static_cast<const Partial*>(partials), chunks, logits, row_stride,
-                                                        static_cast<int>(vocab), inv_temperature, uniforms, u_stride, tok_out,
-                                                        prob_out, prob_stride);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_pdl(sample_finish_kernel, dim3(rows), dim3(kThreads), 0, stream, static_cast<const Partial*>(partials), chunks, logits,
+                      row_stride, static_cast<int>(vocab), inv_temperature, uniforms, u_stride, tok_out, prob_out, prob_stride) == cudaSuccess ? 0 : -1;
 }
 int nucleus_rows(cudaStream_t stream, const float* logits, long long row_stride, int rows, long long vocab,
                  float inv_temperature, float top_p, const float* uniforms, int u_stride, Nucleus* nucleus_out,
                  long long* tok_out, float* prob_out, int prob_stride) {
     if (rows <= 0) return 0;
-    nucleus_kernel<<<rows * kNucCluster, kNucThreads, 0, stream>>>(logits, row_stride, static_cast<int>(vocab), inv_temperature, top_p,
-                                                     uniforms, u_stride, nucleus_out, tok_out, prob_out, prob_stride);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_pdl(nucleus_kernel, dim3(rows * kNucCluster), dim3(kNucThreads), 0, stream, logits, row_stride, static_cast<int>(vocab),
+                      inv_temperature, top_p, uniforms, u_stride, nucleus_out, tok_out, prob_out, prob_stride) == cudaSuccess ? 0 : -1;
 }
 }  // namespace xb
