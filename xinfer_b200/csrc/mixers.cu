@@ -42,6 +42,10 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// x / (1 + exp(-x)) on its way to an fp16 value.  Two units in the last place of fp32, and no branch: the exact division has one, so that
+// a thread's values came one after the other, 150 clocks and more each.
+__device__ __forceinline__ float silu(float x) { return __fdividef(x, 1.0f + expf(-x)); }
+
 // Outputs that feed a W4A16 projection can be written with every block of eight features in the order the int4
 // unpack yields them, (0,4,1,5,2,6,3,7), which saves the projection kernel its in-flight rewrite of the staged
 // activations.  perm8: where feature n goes;  perm8_vec: eight consecutive features (one 16-byte vector) reordered.
@@ -404,7 +408,7 @@ __global__ void conv1d_spec_kernel(__half* out, const __half* in, const float* c
         const long long row = static_cast<long long>(b) * rows_per_seq + i;
         const float x = __half2float(xs[i]);
         const float sum = w0 * s0 + w1 * s1 + w2 * s2 + w3 * x;
-        out[row * channels + c] = __float2half_rn(sum / (1.0f + expf(-sum)));
+        out[row * channels + c] = __float2half_rn(silu(sum));
         pd[i * channels + c] = x;
         s0 = s1;
         s1 = s2;
@@ -532,7 +536,7 @@ __global__ void __launch_bounds__(128 * PARTS, PARTS == 2 ? (TOKENS <= 4 ? 3 : 2
             sh_q[t][d] = (q[i] * rq) * 0.08838834764f;
             sh_k[t][d] = k[i] * rk;
             sh_v[t][d] = v[i];
-            sh_z[t][d] = zz[i] / (1.0f + expf(-zz[i]));
+            sh_z[t][d] = silu(zz[i]);
         }
     }
     __syncthreads();
@@ -655,18 +659,24 @@ __global__ void __launch_bounds__(128 * PARTS, PARTS == 2 ? (TOKENS <= 4 ? 3 : 2
 // Prefill keeps every row, so there is nothing to replay or to hold back.  Rows are [sequence][position].
 //
 // The convolution has no recurrence on its outputs (y_p needs the inputs p-3 .. p only): a thread takes V channels and
-// `span` consecutive positions with the window in registers.  The threads of the first positions are the only readers of
-// the state and also the ones that replace it by the chunk's last three inputs, so one launch does both.  (span = rc when
-// the output overwrites the input.)  Bound by its memory traffic; 512 x 10240 in 8 us against 35 with a thread per element
+// SPAN consecutive positions with the window in registers.  The threads of the first positions are the only readers of
+// the state and also the ones that replace it by the chunk's last three inputs, so one launch does both.  (SPAN 0: all of
+// them, when the output overwrites the input.)  Bound by its memory traffic; 512 x 10240 in 8 us against 35 with a thread per element
 // and a second launch for the state.
-template <int V>
+template <int V, int SPAN>
 __global__ void __launch_bounds__(128) conv1d_chunk_kernel(__half* out, const __half* in, const float* conv_w, float* state, int rc,
-                                                           int channels, int span) {
+                                                           int channels) {
     griddep_prologue();
     const int c = (blockIdx.z * 128 + threadIdx.x) * V;
-    const int b = blockIdx.y, p0 = blockIdx.x * span;
+    const int b = blockIdx.y, p0 = blockIdx.x * SPAN;
     const long long seq0 = static_cast<long long>(b) * rc;
     if (c >= channels) return;
+    float w[V][4];
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) w[e][t] = conv_w[(c + e) * 4 + t];
+    }
     float* st = state ? state + static_cast<long long>(b) * 3 * channels : nullptr;
     struct alignas(2 * V) Vec { __half h[V]; };
     auto load = [&](int p, float (&x)[V]) {  // the input at position p; negative: the state's slot 3 + p
@@ -679,12 +689,7 @@ __global__ void __launch_bounds__(128) conv1d_chunk_kernel(__half* out, const __
             for (int e = 0; e < V; ++e) x[e] = st ? st[(3 + p) * static_cast<long long>(channels) + c + e] : 0.f;
         }
     };
-    float w[V][4], x0[V], x1[V], x2[V], tail[3][V];
-#pragma unroll
-    for (int e = 0; e < V; ++e) {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) w[e][t] = conv_w[(c + e) * 4 + t];
-    }
+    float x0[V], x1[V], x2[V], tail[3][V];
     load(p0 - 3, x0);
     load(p0 - 2, x1);
     load(p0 - 1, x2);
@@ -692,21 +697,38 @@ __global__ void __launch_bounds__(128) conv1d_chunk_kernel(__half* out, const __
 #pragma unroll
         for (int t = 0; t < 3; ++t) load(rc - 3 + t, tail[t]);
     }
-    const int p1 = p0 + span < rc ? p0 + span : rc;
-#pragma unroll 4
-    for (int p = p0; p < p1; ++p) {
-        float x[V];
-        load(p, x);
+    auto emit = [&](int p, const float (&x)[V]) {
         Vec o;
 #pragma unroll
         for (int e = 0; e < V; ++e) {
             const float sum = w[e][0] * x0[e] + w[e][1] * x1[e] + w[e][2] * x2[e] + w[e][3] * x[e];
-            o.h[e] = __float2half_rn(sum / (1.0f + expf(-sum)));
+            o.h[e] = __float2half_rn(silu(sum));
             x0[e] = x1[e];
             x1[e] = x2[e];
             x2[e] = x[e];
         }
         *reinterpret_cast<Vec*>(out + (seq0 + p) * channels + c) = o;
+    };
+    if constexpr (SPAN > 0) {  // every position requested before the first is used
+        Vec raw[SPAN];
+#pragma unroll
+        for (int i = 0; i < SPAN; ++i)
+            if (p0 + i < rc) raw[i] = *reinterpret_cast<const Vec*>(in + (seq0 + p0 + i) * channels + c);
+#pragma unroll
+        for (int i = 0; i < SPAN; ++i) {
+            if (p0 + i < rc) {
+                float x[V];
+#pragma unroll
+                for (int e = 0; e < V; ++e) x[e] = __half2float(raw[i].h[e]);
+                emit(p0 + i, x);
+            }
+        }
+    } else {
+        for (int p = 0; p < rc; ++p) {
+            float x[V];
+            load(p, x);
+            emit(p, x);
+        }
     }
     if (p0 == 0 && st) {
 #pragma unroll
@@ -878,7 +900,7 @@ __global__ void __cluster_dims__(kGdnSlices, 1, 1) __launch_bounds__(kGdnThreads
         const float inv_std = 1.0f / sqrtf(total / 128.0f + 1e-6f);
         const long long at = (seq0 + ot) * value_dim + h * 128 + col0 + oc;
         const float2 zv = __half22float2(*reinterpret_cast<const __half2*>(z + at));
-        const float y0 = o0 * inv_std * nw0 * (zv.x / (1.0f + expf(-zv.x))), y1 = o1 * inv_std * nw1 * (zv.y / (1.0f + expf(-zv.y)));
+        const float y0 = o0 * inv_std * nw0 * silu(zv.x), y1 = o1 * inv_std * nw1 * silu(zv.y);
         *reinterpret_cast<__half2*>(out + at) = __floats2half2_rn(y0, y1);
     }
 }
@@ -1318,7 +1340,7 @@ __global__ void __launch_bounds__(256) gdn_norm_kernel(__half* out, const float*
     const float inv_std = 1.0f / sqrtf(sq / 128.0f + 1e-6f);
     float y[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) y[i] = v[i] * inv_std * w[i] * (g[i] / (1.0f + expf(-g[i])));
+    for (int i = 0; i < 4; ++i) y[i] = v[i] * inv_std * w[i] * silu(g[i]);
     *reinterpret_cast<__half2*>(out + at) = __floats2half2_rn(y[0], y[1]);
     *reinterpret_cast<__half2*>(out + at + 2) = __floats2half2_rn(y[2], y[3]);
 }
@@ -1473,11 +1495,12 @@ int conv1d_chunk(cudaStream_t s, __half* out, const __half* in, const float* con
     // Eight positions per thread; all of them when the output lies over the input (a position's inputs are its neighbours').
     const size_t bytes = static_cast<size_t>(batch) * rc * channels * sizeof(__half);
     const char *o = reinterpret_cast<const char*>(out), *i = reinterpret_cast<const char*>(in);
-    const int span = (o < i + bytes && i < o + bytes) ? rc : 8;
+    const bool overlap = o < i + bytes && i < o + bytes;
     const bool vec = channels % 4 == 0 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in)) & 7) == 0;
     const int per_block = 128 * (vec ? 4 : 1);
-    dim3 grid((rc + span - 1) / span, batch, (channels + per_block - 1) / per_block);
-    launch_pdl(vec ? conv1d_chunk_kernel<4> : conv1d_chunk_kernel<1>, grid, dim3(128), 0, s, out, in, conv_w, state, rc, channels, span);
+    dim3 grid(overlap ? 1 : (rc + 7) / 8, batch, (channels + per_block - 1) / per_block);
+    launch_pdl(overlap ? (vec ? conv1d_chunk_kernel<4, 0> : conv1d_chunk_kernel<1, 0>) : (vec ? conv1d_chunk_kernel<4, 8> : conv1d_chunk_kernel<1, 8>),
+               grid, dim3(128), 0, s, out, in, conv_w, state, rc, channels);
     return XB_LAUNCH_OK();
 }
 
