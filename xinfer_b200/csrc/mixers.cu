@@ -1460,7 +1460,10 @@ int attn_prep_ex(cudaStream_t s, __half* q_out, __half* k_cache, __half* v_cache
                  int rows_per_seq, int hq, int hkv, long long max_seq, float eps, float rope_theta, int rope_dim,
                  int q_head_stride, const long long* positions, int ctx_base, __half* k_out) {
     const int rows = batch * rows_per_seq, slots = hq + 2 * hkv;
-    const bool many = static_cast<long long>(rows) * slots > 4096;  // above, a block per head is several waves (see attn_prep_rows_kernel)
+    // A block per head or a warp per head, in us: rotary embedding of 24 + 4 heads 8 rows 1.9 and 2.0, 32 rows 2.4 and 2.4, 77 rows 4.1 and
+    // 3.1, 128 rows 5.7 and 3.3; cache write of 4 heads 32 rows 1.7 and 1.6, 512 rows 5.3 and 2.3.  With head norms a warp's own
+    // sums are the longer chain (32 rows of 32 slots 3.6 and 5.6), and the block stays the faster until it is several waves.
+    const bool many = static_cast<long long>(rows) * slots > (q_norm_w || k_norm_w ? 4096 : 1024);
     launch_pdl(many ? attn_prep_rows_kernel : attn_prep_kernel, many ? dim3(rows, (slots + 7) / 8) : dim3(rows, slots), dim3(256), 0, s,
                q_out, k_cache, v_cache, q_in, k_in, v_in, q_norm_w, k_norm_w, ctx, rows_per_seq, hq, hkv, max_seq, eps, logf(rope_theta),
                rope_dim, q_head_stride, positions, ctx_base, k_out);
