@@ -148,9 +148,9 @@ struct Ctrl {
     uint64_t a_full[2][2];
     uint64_t d_full[2][2];
     uint64_t epi;         // epilogue barrier of the consumer warps
-    uint64_t epi_groups[8];  // whole tiles, cluster splits: the two warps of 32 rows (one per group) have traded their sums
-    uint64_t epi_halves[8];  // whole tiles: the gate and the up warp of 32 features theirs
-    uint64_t epi_read[4];    // ... and the four warps of a quarter have read what the others left
+    uint64_t epi_groups[8];  // the two warps of 32 rows (one per group) have traded their sums
+    uint64_t epi_halves[8];  // the gate and the up warp of 32 features theirs
+    uint64_t epi_read[4];    // the four warps of a quarter have read what the others left
     uint32_t tmem_base;
     int is_last;
     WaitState ws;
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
         // converted when its stage starts, so the load latency never sits in the loop's critical path; a tile's first two
         // are asked for before the epilogue of the tile in front of it.
         uint32_t q0 = 0u, q1 = 0u;
-        uint32_t quick_phase = 0;   // of the whole tiles' barriers
+        uint32_t quick_phase = 0, halves_phase = 0;  // of the barriers of a tile's four warps
         bool stage_acc_free = true; // nobody else may still be reading stage_acc
         long long u = u_begin;
         int tile = static_cast<int>(u_begin / S), s0 = static_cast<int>(u_begin - static_cast<long long>(tile) * S);
@@ -678,8 +678,10 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
             float* stage_acc = xchg;  // [NREAD][256] fp32, row rt's values at [j][rt]
             const int m_rows = p.m < NREAD ? p.m : NREAD;
             const bool whole = (s0 == 0 && s1 == S);
-            if (NREAD > 8 && whole && p.cluster == 1 && p.seg[p.swiglu ? 0 : ti.seg].push == 0) {
-                // A whole tile's sums never leave their four warps.  The two that share a row trade halves of the activation rows (each
+            // (Cut tiles with up to 16 activation rows go the other way: this one's code costs the main loop of gate/up 1.5 % there and gains
+            // the LM head 0.4.)
+            if (NREAD > 8 && (NREAD > 16 || whole) && p.cluster == 1 && p.seg[p.swiglu ? 0 : ti.seg].push == 0) {
+                // A tile's sums stay with their four warps.  The two that share a row trade halves of the activation rows (each
                 // adds what the other one left for it); of gate/up, the gate and the up warp then trade halves of those, so that each of
                 // the four finishes a quarter.  Barriers of two warps, and stores straight from registers: through the parked rows
                 // below, with barriers of all sixteen warps, a tile of 32 activation rows took 8000 clocks after its twenty stages of
@@ -699,19 +701,60 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                     cell[(gi == 0 ? H + j : j) * kTileRows] = gi == 0 ? acc[H + j] : acc[j];
                     sum[j] = gi == 0 ? acc[j] : acc[H + j];
                 }
-                auto trade = [&](uint64_t* bar) -> bool {
+                auto trade = [&](uint64_t* bar, uint32_t phase) -> bool {
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(bar));
-                    return mbar_wait(smem_u32(bar), quick_phase, abort_flag);
+                    return mbar_wait(smem_u32(bar), phase, abort_flag);
                 };
-                if (!trade(&ctrl->epi_groups[wg * 4 + quarter])) { ok = false; break; }
+                if (!trade(&ctrl->epi_groups[wg * 4 + quarter], quick_phase)) { ok = false; break; }
 #pragma unroll
                 for (int j = 0; j < H; ++j) sum[j] += cell[(gi * H + j) * kTileRows];
-                OutT* const y = static_cast<OutT*>(p.seg[p.swiglu ? 0 : ti.seg].y) + my_col;
-                const long long ldy = p.seg[p.swiglu ? 0 : ti.seg].ldy;
-                if (!p.swiglu) {
+                auto cells_read = [&] {
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&ctrl->epi_read[quarter]));
+                };
+                if (!p.swiglu) cells_read();
+                bool last = whole;
+                if (NREAD > 16 && !whole) {
+                    // A tile cut between CTAs (units cut evenly over one CTA per SM): the partial sums go through the scratch buffer and
+                    // the last CTA to arrive adds all of them, its own too, in CTA order.
+                    const int wslot = blockIdx.x * 2 + (tile == static_cast<int>(u_begin / S) ? 0 : 1);
+                    float* ws = p.workspace + static_cast<long long>(wslot) * (32 * kTileRows) + gi * H * kTileRows + rt;
+#pragma unroll
+                    for (int j = 0; j < H; ++j)
+                        if (gi * H + j < m_rows) ws[j * kTileRows] = sum[j];
+                    __threadfence();
+                    if (!consumer_sync()) break;
+                    const long long t_lo = static_cast<long long>(tile) * S;
+                    const int c_lo = unit_owner(t_lo, p.total_units, ctas), c_hi = unit_owner(t_lo + S - 1, p.total_units, ctas);
+                    if (tid == 0) {
+                        const int old = atomicAdd(&p.counters[tile], 1);
+                        ctrl->is_last = (old == c_hi - c_lo) ? 1 : 0;
+                    }
+                    if (!consumer_sync()) break;
+                    last = ctrl->is_last != 0;
+                    if (last) {
+                        __threadfence();
+#pragma unroll
+                        for (int j = 0; j < H; ++j) sum[j] = 0.f;
+#pragma unroll 1
+                        for (int c = c_lo; c <= c_hi; ++c) {
+                            const int c_first_tile = static_cast<int>(unit_begin(c, p.total_units, ctas) / S);
+                            const float* src = p.workspace + static_cast<long long>(c * 2 + (tile == c_first_tile ? 0 : 1)) * (32 * kTileRows) +
+                                               gi * H * kTileRows + rt;
+#pragma unroll
+                            for (int j = 0; j < H; ++j)
+                                if (gi * H + j < m_rows) sum[j] += __ldcg(src + j * kTileRows);
+                        }
+                        if (tid == 0) p.counters[tile] = 0;
+                    } else if (p.swiglu) {
+                        cells_read();
+                    }
+                }
+                OutT* const y = static_cast<OutT*>(p.seg[p.swiglu ? 0 : ti.seg].y) + my_col;
+                const long long ldy = p.seg[p.swiglu ? 0 : ti.seg].ldy;
+                if (!last) {
+                } else if (!p.swiglu) {
                     const float b = (valid && sg.bias) ? sg.bias[my_row] : 0.f;
                     const int live = valid ? m_rows - gi * H : 0;
                     OutT* o = y + gi * H * ldy;
@@ -727,7 +770,8 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                         cell[(gi * H + (wg == 0 ? Q + j : j)) * kTileRows] = wg == 0 ? sum[Q + j] : sum[j];
                         mine[j] = wg == 0 ? sum[j] : sum[Q + j];
                     }
-                    if (!trade(&ctrl->epi_halves[gi * 4 + quarter])) { ok = false; break; }
+                    if (!trade(&ctrl->epi_halves[gi * 4 + quarter], halves_phase)) { ok = false; break; }
+                    halves_phase ^= 1u;
                     const float* const theirs = stage_acc + (wg == 0 ? kHalfRows + t : t) + (gi * H + wg * Q) * kTileRows;
                     const int live = valid ? m_rows - gi * H - wg * Q : 0;
                     OutT* o = y + (gi * H + wg * Q) * ldy;
@@ -738,8 +782,7 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                         const float g = wg == 0 ? mine[j] : other, up = wg == 0 ? other : mine[j];
                         v[j] = __fdividef(g, 1.0f + expf(-g)) * up;
                     }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&ctrl->epi_read[quarter]));
+                    cells_read();
 #pragma unroll
                     for (int j = 0; j < Q; ++j, o += ldy)
                         if (j < live) store_out<OutT>(o, v[j]);
