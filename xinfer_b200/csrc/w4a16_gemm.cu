@@ -54,7 +54,8 @@ constexpr int kGemmTileM = 256;   // most activation rows per tile (the MMA's N)
 constexpr int kSwizzleK = 64;     // k of one 128-byte swizzle row of fp16
 // Operand ring: a slot holds a whole 128-k group of unpacked weights and of activations.  The MMA warp's own loop - waits, issue
 // and commits, each a hundred clocks or two - is what every stage goes through, and with 64-k slots it took longer than the
-// tensor core: at M = 512 900 TFLOP/s with three waits a slot (weights and activations apart), 1120 now.
+// tensor core: at M = 512 900 TFLOP/s with three waits a slot (weights and activations apart), 1120 with one, 1150 to
+// 1280 with its instructions predicated and its two waits side by side (umma_ss_f16_pair, the MMA warp).
 // Accumulator tiles: tiles of at most 128 rows have four, the larger ones two (all of tensor memory).
 constexpr int kOpSlotsMax = 4, kDBufsMax = 4, kWSlotsMax = 8;
 constexpr int kWSlotBytes = kGemmTileN * 64;                    // 8 KB of packed weights: one group
@@ -123,6 +124,8 @@ struct GemmParams {
     int* counters;      // [CTA]: groups of the tile that starts in that pair's range and ends behind it, added up so far
 };
 
+// (This and the commit are executed by a whole warp under uniform control flow; the lane with `issue` set issues.  Inside `if (leader)`
+// the descriptors were moved to uniform registers for every instruction: the eight of a group took 500 clocks, and 400 this way.)
 // D[tmem] (+)= A[smem descriptor] * B[smem descriptor], kind::f16, on a CTA pair: A and D rows 0-127 in the even CTA,
 // 128-255 in the odd one; B rows half and half, each CTA's at the descriptor's offset.  Issued by one thread of the even CTA.
 __device__ __forceinline__ void umma_ss_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
@@ -741,7 +744,7 @@ GemmDeal gemm_deal(const TcProj* proj, int num, bool swiglu, long long m, long l
 
 }  // namespace
 
-// 5.8 us a tile of a pair (fill, read-out and stores) and 0.53 us a group; a cut costs kCutCost groups, or six where it falls on
+// As the kernel was when the routes of 33 to 64 rows were drawn (c_api.cu): 5.8 us a tile of a pair (fill, read-out and stores) and 0.53 us a group; a cut costs kCutCost groups, or six where it falls on
 // equal parts of every tile.  Within 6 % of most of 18 shapes at 33 .. 64 rows; off by more for the narrowest (5120 x 2048 and
 // narrower: within 3 us) and for few tiles in many parts (16384 x 1024: 21 us, modelled 13).
 double gemm_modelled_us(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms) {
