@@ -61,8 +61,12 @@ __device__ __forceinline__ int nucleus_bucket(float scaled, float max_scaled) {
 __device__ __forceinline__ float key_to_float(uint32_t k) {
     return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k);
 }
+// (At most 2^32, and only exp(0) gets there: a 32-bit conversion, which saturates one short of it, and a carry.  The 64-bit one made
+// the pass over a row's weights 5800 clocks at 19 a thread.  Its answer to a NaN stays.)
 __device__ __forceinline__ unsigned long long nucleus_weight(float scaled, float max_scaled) {
-    return __float2ull_rn(expf(scaled - max_scaled) * 4294967296.0f);
+    const float x = expf(scaled - max_scaled) * 4294967296.0f;
+    const unsigned long long w = static_cast<unsigned long long>(__float2uint_rn(x)) + (x >= 4294967296.0f ? 1u : 0u);
+    return x != x ? 0x8000000000000000ull : w;
 }
 
 // The partial of one chunk of the row at `l`, by a block, once in a launch; every thread gets it.
@@ -529,7 +533,7 @@ constexpr int kNucCluster = 8;
 constexpr int kNucCand = 4096;
 // Rows of up to 8 * 20 * 1024 tokens stay in registers.  The list of those within kNucCut[i] of the maximum for the smallest
 // i that holds the nucleus is short for a trained model's logits; up to kNucShort of them the leader selects and draws alone.
-constexpr int kNucRegs = 20, kNucCuts = 7, kNucShort = 256;
+constexpr int kNucRegs = 20, kNucCuts = 7, kNucShort = kNucThreads / 4;
 __device__ __forceinline__ float nucleus_cut(int i) { return i < 4 ? 1.0f + i : (i == 4 ? 6.0f : (i == 5 ? 8.0f : 11.0f)); }
 
 // The weight the nucleus has to reach, and the point of the running sum over its tokens that a uniform picks.
@@ -555,6 +559,7 @@ struct NucShared {
     float wmax[32];
     unsigned long long above, target, z_nuc;   // leader: results of a level / of the selection
     int bin, count;
+    int listed, list_at;                    // this CTA's candidates: how many, and where they go in the leader's list
     uint32_t thr;
 };
 
@@ -596,7 +601,7 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (lane == 0) sh.wmax[warp] = mx;
-    if (tid == 0) sh.count = 0;
+    if (tid == 0) sh.count = sh.listed = 0;
     __syncthreads();
     cluster_wait();
     if (warp == 0) {
@@ -667,13 +672,25 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
             if (tot > 0 && c * 0.999f >= static_cast<float>(target) * (1.0f / 4294967296.0f)) reach = nucleus_cut(i);
         }
         if (reach >= 0.f) {  // (the same in every CTA)
+            // A CTA counts its candidates first and asks the leader for their places once (an atomic per candidate on the leader's shared
+            // memory, each a trip there and back, took 5300 clocks for some fifty).  Weights are not zero this close to the maximum.
             uint32_t* keys = reinterpret_cast<uint32_t*>(lead->hist);
+            int mine = 0;
 #pragma unroll
-            for (int j = 0; j < kNucRegs; ++j) {
-                if (ms - v[j] <= reach && nucleus_weight(v[j], ms)) {
-                    const int at = atomicAdd(&lead->count, 1);
-                    if (at < kNucCand) keys[at] = order_key(v[j]);
-                    if (at < kNucShort) lead->ids[at] = static_cast<uint32_t>(c0 + j * kNucThreads + tid);
+            for (int j = 0; j < kNucRegs; ++j) mine += ms - v[j] <= reach ? 1 : 0;
+            int at = mine ? atomicAdd(&sh.listed, mine) : 0;
+            __syncthreads();
+            if (tid == 0) sh.list_at = sh.listed ? atomicAdd(&lead->count, sh.listed) : 0;
+            __syncthreads();
+            if (mine) {
+                at += sh.list_at;
+#pragma unroll
+                for (int j = 0; j < kNucRegs; ++j) {
+                    if (ms - v[j] <= reach) {
+                        if (at < kNucCand) keys[at] = order_key(v[j]);
+                        if (at < kNucShort) lead->ids[at] = static_cast<uint32_t>(c0 + j * kNucThreads + tid);
+                        ++at;
+                    }
                 }
             }
             cluster.sync();
@@ -682,25 +699,29 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
             if (count <= kNucShort) {
                 cluster_arrive();  // (the leader stays until everybody has read its count)
                 if (crank == 0) {
+                    // four threads a candidate (of at most 256), each with every fourth of the others
+                    const float uniform = uniforms ? uniforms[static_cast<long long>(row) * u_stride] : 0.f;
                     const uint32_t* key = reinterpret_cast<const uint32_t*>(sh.hist);
                     unsigned long long* weight = sh.hist + kNucCand / 2;  // behind the keys
-                    const uint32_t mine = tid < count ? key[tid] : 0u;
-                    const unsigned long long w = tid < count ? nucleus_weight(key_to_float(mine), ms) : 0ull;
-                    if (tid < count) weight[tid] = w;
+                    if (tid < count) weight[tid] = nucleus_weight(key_to_float(key[tid]), ms);
                     __syncthreads();
+                    const int at = tid >> 2, part = tid & 3;
+                    const bool live = at < count;
+                    const uint32_t mine = live ? key[at] : 0u;
+                    auto four = [](unsigned long long s) {
+                        s += __shfl_xor_sync(0xffffffffu, s, 1);
+                        return s + __shfl_xor_sync(0xffffffffu, s, 2);
+                    };
                     // the weight at or above each candidate; the threshold is the largest key at which it reaches the target
                     unsigned long long sum = 0;
-                    if (tid < count)
-                        for (int q = 0; q < count; ++q) sum += key[q] >= mine ? weight[q] : 0ull;
-                    if (warp < kNucShort / 32) {
-                        const uint32_t best = __reduce_max_sync(0xffffffffu, tid < count && sum >= target ? mine : 0u);
-                        if (lane == 0) sh.wmax[warp] = __uint_as_float(best);
-                    }
+                    if (live)
+                        for (int q = part; q < count; q += 4) sum += key[q] >= mine ? weight[q] : 0ull;
+                    sum = four(sum);
+                    const uint32_t best = __reduce_max_sync(0xffffffffu, live && sum >= target ? mine : 0u);
+                    if (lane == 0) sh.wmax[warp] = __uint_as_float(best);
                     __syncthreads();
-                    uint32_t thr = 0;
-#pragma unroll
-                    for (int q = 0; q < kNucShort / 32; ++q) thr = max(thr, __float_as_uint(sh.wmax[q]));
-                    if (tid < count && mine == thr) sh.z_nuc = sum;
+                    const uint32_t thr = __reduce_max_sync(0xffffffffu, __float_as_uint(sh.wmax[lane]));
+                    if (live && part == 0 && mine == thr) sh.z_nuc = sum;
                     __syncthreads();
                     const unsigned long long z_nuc = sh.z_nuc;
                     if (tid == 0 && nuc_out) {
@@ -710,13 +731,16 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
                         q.thr_key = thr;
                         nuc_out[row] = q;
                     }
-                    if (uniforms && tid < count && mine >= thr) {
+                    if (uniforms) {
                         // the candidate in whose range of the running sum over the token ids the draw falls
-                        const unsigned long long t2 = nucleus_draw(uniforms[static_cast<long long>(row) * u_stride], z_nuc);
-                        const uint32_t id = sh.ids[tid];
+                        const unsigned long long t2 = nucleus_draw(uniform, z_nuc);
+                        const uint32_t id = live ? sh.ids[at] : 0u;
                         unsigned long long before = 0;
-                        for (int q = 0; q < count; ++q) before += key[q] >= thr && sh.ids[q] < id ? weight[q] : 0ull;
-                        if (before <= t2 && t2 < before + w) {
+                        if (live && mine >= thr)
+                            for (int q = part; q < count; q += 4) before += key[q] >= thr && sh.ids[q] < id ? weight[q] : 0ull;
+                        before = four(before);
+                        const unsigned long long w = live ? weight[at] : 0ull;
+                        if (live && part == 0 && mine >= thr && before <= t2 && t2 < before + w) {
                             tok_out[row] = id;
                             prob_out[static_cast<long long>(row) * prob_stride] =
                                 static_cast<float>(static_cast<double>(w) / static_cast<double>(z_nuc));
