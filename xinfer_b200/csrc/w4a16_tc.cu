@@ -815,8 +815,8 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                 // barrier A).  One cluster barrier later the owner adds the senders in rank order (deterministic).
                 // Up to eight activation rows: [sender][group][row of the block][256 features], the owner adds a sender's two
                 // groups.  More: the two warps of a row first trade halves of the activation rows and each sends the sums of its half,
-                // [sender][row][256].  (Parked rows sent by the copy engine, one copy per receiver, took 2.3 us from the last stage to
-                // the sums at 32 rows; this 1.3.)
+                // [sender][row][256].  (Parked rows sent by the copy engine, one copy per receiver, took 4.4 us from the last stage to
+                // the outputs at 32 rows; a launch of 6144 x 5120 went from 11.3 to 10.45 us.)
                 float* part = reinterpret_cast<float*>(smem);
                 const uint32_t my_rank = cluster_ctarank();
                 const uint32_t csz = static_cast<uint32_t>(p.cluster);
