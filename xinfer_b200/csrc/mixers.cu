@@ -31,6 +31,7 @@
 #include "launch.cuh"
 #include "mixers.h"
 #include "ptx_sm100.cuh"
+#include "silu.cuh"
 
 namespace xb {
 
@@ -41,10 +42,6 @@ __device__ __forceinline__ float warp_sum(float v) {
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
     return v;
 }
-
-// x / (1 + exp(-x)) on its way to an fp16 value.  Two units in the last place of fp32, and no branch: the exact division has one, so that
-// a thread's values came one after the other, 150 clocks and more each.
-__device__ __forceinline__ float silu(float x) { return __fdividef(x, 1.0f + expf(-x)); }
 
 // Outputs that feed a W4A16 projection can be written with every block of eight features in the order the int4
 // unpack yields them, (0,4,1,5,2,6,3,7), which saves the projection kernel its in-flight rewrite of the staged

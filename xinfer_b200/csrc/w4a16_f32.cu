@@ -17,6 +17,7 @@
 #include <stdint.h>
 
 #include "ptx_sm100.cuh"
+#include "silu.cuh"
 #include "w4a16.h"
 
 namespace xb {
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(kF32Threads, 2) w4a16_f32_kernel(const __grid_
         parts[0][tid] = sum;  // (this thread's own slot; the others' sums of it are in)
         __syncthreads();
         if (row >= 16) return;
-        sum = (sum / (1.0f + expf(-sum))) * parts[0][tid + 16];
+        sum = silu(sum) * parts[0][tid + 16];
     }
     const F32Proj& pj = p.proj[pi];
     if (base + row < pj.n && m0 + col < p.m) {

@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "silu.cuh"
 #include "w4a16.h"
 
 namespace xb {
@@ -150,8 +151,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) w4a16_simt_kernel(const S
             if (m >= p.m) continue;
             if (p.swiglu) {
                 const float g = acc_a[mi];
-                const float silu = g / (1.0f + expf(-g));
-                put<OutT>(pa.y, m * pa.ldy + row_a, silu * acc_b[mi]);
+                put<OutT>(pa.y, m * pa.ldy + row_a, silu(g) * acc_b[mi]);
             } else {
                 float va = acc_a[mi];
                 if (pa.bias) va += pa.bias[row_a];
@@ -204,8 +204,7 @@ __global__ void w4a16_generic_kernel(const SimtParams p) {
     }
     const SimtProj& po = p.proj[p.swiglu ? 0 : pi];
     if (p.swiglu) {
-        const float silu = res[0] / (1.0f + expf(-res[0]));
-        put<OutT>(po.y, m * po.ldy + n, silu * res[1]);
+        put<OutT>(po.y, m * po.ldy + n, silu(res[0]) * res[1]);
     } else {
         float v = res[0];
         if (po.bias) v += po.bias[n];

@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "ptx_sm100.cuh"
+#include "silu.cuh"
 #include "w4a16.h"
 
 namespace xb {
@@ -775,12 +776,12 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                     const float* const theirs = stage_acc + (wg == 0 ? kHalfRows + t : t) + (gi * H + wg * Q) * kTileRows;
                     const int live = valid ? m_rows - gi * H - wg * Q : 0;
                     OutT* o = y + (gi * H + wg * Q) * ldy;
-                    float v[Q];  // (all before the first store; no branch in the division: an exact one each in turn)
+                    float v[Q];  // (all before the first store)
 #pragma unroll
                     for (int j = 0; j < Q; ++j) {
                         const float other = theirs[j * kTileRows];
                         const float g = wg == 0 ? mine[j] : other, up = wg == 0 ? other : mine[j];
-                        v[j] = __fdividef(g, 1.0f + expf(-g)) * up;
+                        v[j] = silu(g) * up;
                     }
                     cells_read();
 #pragma unroll
@@ -949,7 +950,7 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
                             const float g = stage_acc[j * kTileRows + t];
                             const float up = stage_acc[j * kTileRows + kHalfRows + t];
                             store_row<OutT>(p, p.seg[0], my_col + static_cast<long long>(j) * ldy, j,
-                                            (g / (1.0f + expf(-g))) * up);
+                                            silu(g) * up);
                         }
                     }
                 } else if (valid) {
