@@ -153,6 +153,20 @@ def test_conv1d_spans(cuda, T, C):
                 assert np.array_equal(st_d.cpu().numpy(), ref)
 
 
+@pytest.mark.parametrize("T", [1, 2, 3, 7, 8, 9, 16, 17, 61])
+@pytest.mark.parametrize("C", [512, 515])
+def test_conv1d_in_place(cuda, T, C):
+    """A thread's walk over all positions against one that takes eight: the same bits."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn((T, C), generator=g, device="cuda").half()
+    w, st = torch.randn((C, 4), generator=g, device="cuda"), torch.randn((3, C), generator=g, device="cuda")
+    apart, st2 = torch.empty_like(x), st.clone()
+    assert cuda.causal_conv1d_silu(apart, x, w, T, st, C) == 0
+    assert cuda.causal_conv1d_silu(x, x, w, T, st2, C) == 0
+    assert torch.equal(x, apart) and torch.equal(st, st2)
+
+
 @pytest.mark.parametrize("with_state", [True, False])
 def test_conv1d_beyond_32_bit_positions(cuda, with_state):
     """A sequence of more than 2^31 positions (two channels) gives, at its end and at a seam, what that part alone gives."""
