@@ -93,6 +93,17 @@ constexpr int gemm_w_slots(int tile_m) {
 }
 constexpr int gemm_d_bufs(int tile_m) { return tile_m > 128 ? 2 : kDBufsMax; }
 static_assert(gemm_w_slots(kGemmTileM) >= 3 && gemm_w_slots(128) >= 3, "shared memory");
+// Sets of unpacking warps that take the groups in turn keep to slots of their own: the rings' lengths are multiples of their number.
+// Otherwise a set would come to a slot that the other one used last, and a wait for a parity that tells its own last use from the next
+// would be let through by a use that lies between them, before the bytes have landed.
+constexpr bool gemm_sets_keep_their_slots() {
+    for (int tile_m = 32; tile_m <= kGemmTileM; tile_m += 32) {
+        const int sets = gemm_unpack_sets((tile_m + 63) / 64);
+        if (gemm_op_slots(tile_m) % sets || gemm_w_slots(tile_m) % sets) return false;
+    }
+    return true;
+}
+static_assert(gemm_sets_keep_their_slots(), "ring lengths");
 
 struct GemmProj {
     const __half* scales[2];  // gate/up: of both
@@ -402,7 +413,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
         // gate/up: the raw tile is 64 rows of each, the operand sixteen and sixteen, so that a feature's two sums meet in one warp
         const int ra = p.swiglu ? ((r & 48) << 1) + ((r >> 6) << 4) + (r & 15) : r;
         const uint32_t a_row = static_cast<uint32_t>((ra >> 3) * 1024 + (ra & 7) * 128), a_sw = static_cast<uint32_t>(ra & 7);
-        int wslot = set, aslot = set;  // (both rings have three slots at least)
+        int wslot = set, aslot = set;  // (a set's own slots: gemm_sets_keep_their_slots)
         uint32_t w_phase = 0, a_phase = 1;
         for (int i = set; i < U; i += kSets) {
             const uint32_t w_bar = smem_u32(&ctrl->w_full[wslot]), a_bar = smem_u32(&ctrl->op_empty[aslot]);
