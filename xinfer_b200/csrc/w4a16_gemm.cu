@@ -17,7 +17,7 @@
 //     accumulator over all of K: 113 us at M = 512, K = 5120, N = 17408);
 //   * both operands from shared memory: the activations land by TMA in the canonical 128-byte-swizzled K-major layout,
 //     the packed weights land raw (64 bytes per row and group) and four warps, one thread per weight row, unpack them
-//     into the same layout;
+//     into the same layout (up to 128 rows eight, four to every other group);
 //   * the work of one launch - all tiles of all its projections x K / 128 groups - is dealt to one pair per two SMs, whole
 //     tiles or, where that leaves the last wave too empty, cut evenly.  A tile that straddles a cut is finished by the CTA
 //     that arrives last, which adds the others' fp32 partials in pair order (the result does not depend on who is last).
@@ -756,9 +756,10 @@ GemmDeal gemm_deal(const TcProj* proj, int num, bool swiglu, long long m, long l
 
 }  // namespace
 
-// As the kernel was when the routes of 33 to 64 rows were drawn (c_api.cu): 5.8 us a tile of a pair (fill, read-out and stores) and 0.53 us a group; a cut costs kCutCost groups, or six where it falls on
-// equal parts of every tile.  Within 6 % of most of 18 shapes at 33 .. 64 rows; off by more for the narrowest (5120 x 2048 and
-// narrower: within 3 us) and for few tiles in many parts (16384 x 1024: 21 us, modelled 13).
+// The kernel as it was when the routes of 33 to 64 rows were drawn (c_api.cu), up to 30 % slower than now: 5.8 us a tile of a pair (fill,
+// read-out and stores) and 0.53 us a group; a cut costs kCutCost groups, or six where it falls on equal parts of every tile.  It was
+// within 6 % of most of 18 shapes at 33 .. 64 rows, and off by more for the narrowest (5120 x 2048 and narrower: within 3 us) and
+// for few tiles in many parts (16384 x 1024: 21 us, modelled 13).
 double gemm_modelled_us(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms) {
     const GemmDeal d = gemm_deal(proj, num, swiglu, m, k, num_sms, true);
     const long long groups = k / 128;

@@ -672,10 +672,10 @@ __global__ void __launch_bounds__(kThreads, 1) w4a16_tc_kernel(const __grid_cons
             fold(sc_pend, (n - 1) & 1u);
 
             // ---------------------------------------------------------------- tile epilogue
-            // Runs once per tile, so its instructions are cold in the instruction caches: the accumulators
-            // are parked in shared memory and everything after that is written as rolled loops (a fully
-            // unrolled epilogue cost ~10 us in instruction fetches alone).  The two threads of a row first
-            // add their groups' partial sums there; afterwards they split the activation rows by parity.
+            // Runs once per tile, so its instructions are cold in the instruction caches.  Above 8 activation rows a tile that one CTA
+            // finishes keeps its sums in registers, unrolled; the others (few rows, cut tiles of up to 16, values that go to
+            // peers) are parked in shared memory and what follows is written as rolled loops: the two threads of a row first add
+            // their groups' partial sums there, afterwards they split the activation rows by parity.
             float* stage_acc = xchg;  // [NREAD][256] fp32, row rt's values at [j][rt]
             const int m_rows = p.m < NREAD ? p.m : NREAD;
             const bool whole = (s0 == 0 && s1 == S);
