@@ -222,10 +222,11 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __grid_constant__ No
 // ------------------------------------------------------------------------------- attention prologue
 // A rotation is two products and a sum; one product is rounded before the sum, and left to the compiler it was another one in each of
 // the two forms below.  Here it is the sine's, in both.  Calls of more than 4096 heads, which have only ever had the second form, keep
-// what that gave them: the cosine's for a pair's second value (`sine_fused`).
-__device__ __forceinline__ float rotated(bool second, float v0, float v1, float c, float s, bool sine_fused) {
+// what that gave them: the cosine's for a pair's second value (SINE_FUSED).
+template <bool SINE_FUSED>
+__device__ __forceinline__ float rotated(bool second, float v0, float v1, float c, float s) {
     if (!second) return fmaf(v0, c, -__fmul_rn(v1, s));
-    return sine_fused ? fmaf(v0, s, __fmul_rn(v1, c)) : fmaf(v1, c, __fmul_rn(v0, s));
+    return SINE_FUSED ? fmaf(v0, s, __fmul_rn(v1, c)) : fmaf(v1, c, __fmul_rn(v0, s));
 }
 
 // One block per (row, head slot); head slots 0..Hq-1 are query heads, Hq..Hq+Hkv-1 key heads,
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(__half* q_out, __half* k
         const float angle = static_cast<float>(pos) * freq;
         const float c = cosf(angle), s = sinf(angle);
         const float v0 = vals[pair], v1 = vals[pair + half_rot];
-        outv = rotated(d >= half_rot, v0, v1, c, s, false);
+        outv = rotated<false>(d >= half_rot, v0, v1, c, s);
     }
     const __half o = __float2half_rn(outv);
     if (is_q) {
@@ -294,12 +295,13 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(__half* q_out, __half* k
 // The same for many heads: a warp per (row, head slot), eight slots of a row per block; lane l holds dims l, l + 32, ...  Same
 // sums in the same order.  No block barriers, and a prompt's heads are two waves of blocks instead of fourteen: 512 rows and 24
 // query heads 13.9 -> 5 us.  A warp's own chain is longer: 32 heads of 32 rows take 5.6 us against 3.6.
+template <bool SINE_FUSED>
 __global__ void __launch_bounds__(256) attn_prep_rows_kernel(__half* q_out, __half* k_cache, __half* v_cache,
                                                         const __half* q_gate, const __half* k_in, const __half* v_in,
                                                         const float* q_norm_w, const float* k_norm_w, const int* ctx,
                                                         int rows_per_seq, int hq, int hkv, long long max_seq,
                                                         float eps, float log_theta, int rope_dim, int q_head_stride,
-                                                        const long long* positions, int ctx_base, __half* k_out, bool sine_fused) {
+                                                        const long long* positions, int ctx_base, __half* k_out) {
     griddep_prologue();
     __shared__ float sh[8][256];
     __shared__ float2 sh_cs[8][128];
@@ -370,7 +372,7 @@ __global__ void __launch_bounds__(256) attn_prep_rows_kernel(__half* q_out, __ha
             const int pair = d < half_rot ? d : d - half_rot;
             const float c = cs[pair].x, s = cs[pair].y;
             const float v0 = vals[pair], v1 = vals[pair + half_rot];
-            outv = rotated(d >= half_rot, v0, v1, c, s, sine_fused);
+            outv = rotated<SINE_FUSED>(d >= half_rot, v0, v1, c, s);
         }
         if (store) to[d] = __float2half_rn(outv);
     }
@@ -1466,12 +1468,14 @@ int attn_prep_ex(cudaStream_t s, __half* q_out, __half* k_cache, __half* v_cache
     const int rows = batch * rows_per_seq, slots = hq + 2 * hkv;
     // A block per head or a warp per head, in us: rotary embedding of 24 + 4 heads 8 rows 1.9 and 2.0, 32 rows 2.4 and 2.4, 77 rows 4.1 and
     // 3.1, 128 rows 5.7 and 3.3; cache write of 4 heads 32 rows 1.7 and 1.6, 512 rows 5.3 and 2.3.  With head norms a warp's own
-    // sums are the longer chain (32 rows of 32 slots 3.6 and 5.6), and the block stays the faster until it is several waves.
+    // sums are the longer chain (32 rows of 32 slots 3.6 and 5.6), and the block stays the faster until it is several waves.  So it does
+    // for a single head a row, where seven warps of eight would have nothing to do (1100 rows 3.1 and 3.8, 4000 rows 6.6 and 7.2; of two
+    // heads 4.6 and 3.8).
     const long long heads = static_cast<long long>(rows) * slots;
-    if (heads > (q_norm_w || k_norm_w ? 4096 : 1024))
-        launch_pdl(attn_prep_rows_kernel, dim3(rows, (slots + 7) / 8), dim3(256), 0, s, q_out, k_cache, v_cache, q_in, k_in, v_in, q_norm_w,
-                   k_norm_w, ctx, rows_per_seq, hq, hkv, max_seq, eps, logf(rope_theta), rope_dim, q_head_stride, positions, ctx_base, k_out,
-                   heads > 4096);
+    if (heads > (q_norm_w || k_norm_w || slots == 1 ? 4096 : 1024))
+        launch_pdl(heads > 4096 ? attn_prep_rows_kernel<true> : attn_prep_rows_kernel<false>, dim3(rows, (slots + 7) / 8), dim3(256), 0, s,
+                   q_out, k_cache, v_cache, q_in, k_in, v_in, q_norm_w, k_norm_w, ctx, rows_per_seq, hq, hkv, max_seq, eps, logf(rope_theta),
+                   rope_dim, q_head_stride, positions, ctx_base, k_out);
     else
         launch_pdl(attn_prep_kernel, dim3(rows, slots), dim3(256), 0, s, q_out, k_cache, v_cache, q_in, k_in, v_in, q_norm_w, k_norm_w, ctx,
                    rows_per_seq, hq, hkv, max_seq, eps, logf(rope_theta), rope_dim, q_head_stride, positions, ctx_base, k_out);
