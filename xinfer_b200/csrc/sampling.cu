@@ -69,7 +69,7 @@ __device__ __forceinline__ unsigned long long nucleus_weight(float scaled, float
     return x != x ? 0x8000000000000000ull : w;
 }
 
-// The partial of one chunk of the row at `l`, by a block, once in a launch; every thread gets it.
+// The partial of one chunk of the row at `l`, by a block, once in a launch; thread 0 gets it.
 __device__ __forceinline__ Partial chunk_partial(const float* l, int chunk, int vocab, float inv_t, int want_sum, int idx_offset) {
     const int base = chunk * kChunk;
     const int end = min(vocab, base + kChunk);
@@ -98,29 +98,31 @@ __device__ __forceinline__ Partial chunk_partial(const float* l, int chunk, int 
     }
     // Block argmax (value, lowest index) and, for the sum, the maximum of the scaled logits: scaling by a positive factor is monotone,
     // also where it rounds two values together, so that is the scaled maximum.  (NaNs are passed over there and turn up in the sum.)
-    // Every thread merges the warps' values itself: one barrier here and one for the sum, where there were seven.
+    // Every warp merges the warps' values itself: one barrier here and one for the sum, where there were seven.
     __shared__ float s_v[kThreads / 32], s_m[kThreads / 32], s_f[kThreads / 32];
     __shared__ int s_i[kThreads / 32];
-    float ms = vals[0];
+    float ms = -INFINITY;
+    if (want_sum) {
 #pragma unroll
-    for (int r = 1; r < 16; ++r) ms = fmaxf(ms, vals[r]);
+        for (int r = 0; r < 16; ++r) ms = fmaxf(ms, vals[r]);
+    }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, best, off);
         const int oi = __shfl_xor_sync(0xffffffffu, best_i, off);
         better(best, best_i, ov, oi);
-        ms = fmaxf(ms, __shfl_xor_sync(0xffffffffu, ms, off));
+        if (want_sum) ms = fmaxf(ms, __shfl_xor_sync(0xffffffffu, ms, off));
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) { s_v[warp] = best; s_i[warp] = best_i; s_m[warp] = ms; }
     __syncthreads();
-    best = s_v[0];
-    best_i = s_i[0];
-    ms = s_m[0];
+    best = s_v[lane & (kThreads / 32 - 1)];
+    best_i = s_i[lane & (kThreads / 32 - 1)];
 #pragma unroll
-    for (int w = 1; w < kThreads / 32; ++w) {
-        better(best, best_i, s_v[w], s_i[w]);
-        ms = fmaxf(ms, s_m[w]);
+    for (int off = kThreads / 64; off > 0; off >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, best, off);
+        const int oi = __shfl_xor_sync(0xffffffffu, best_i, off);
+        better(best, best_i, ov, oi);
     }
     Partial res;
     res.max_raw = best;
@@ -128,7 +130,9 @@ __device__ __forceinline__ Partial chunk_partial(const float* l, int chunk, int 
     res.max_scaled = 0.f;
     res.sum_exp = 0.f;
     if (want_sum) {
-        ms = fmaxf(ms, -INFINITY) * inv_t;  // (nothing but NaNs: -inf)
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) ms = fmaxf(ms, s_m[w]);
+        ms *= inv_t;  // (nothing but NaNs: -inf)
         float se = 0.f;
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
