@@ -61,9 +61,13 @@ __device__ __forceinline__ int nucleus_bucket(float scaled, float max_scaled) {
 __device__ __forceinline__ float key_to_float(uint32_t k) {
     return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k);
 }
-// (At most 2^32, and only exp(0) gets there: a 32-bit conversion, which saturates one short of it, and a carry.  The 64-bit one made
-// the pass over a row's weights 5800 clocks at 19 a thread.  Its answer to a NaN stays.)
 __device__ __forceinline__ unsigned long long nucleus_weight(float scaled, float max_scaled) {
+    return __float2ull_rn(expf(scaled - max_scaled) * 4294967296.0f);
+}
+// The same value (at most 2^32, and only exp(0) gets there) by a 32-bit conversion, which saturates one short of it, and a carry; the
+// 64-bit one's answer to a NaN stays.  For a pass over weights that are in registers, which the 64-bit conversions made 5800 clocks at
+// 19 a thread; where the logits are read again they hide behind the loads, and this form's instructions cost 3 % (400000 tokens).
+__device__ __forceinline__ unsigned long long nucleus_weight_in_regs(float scaled, float max_scaled) {
     const float x = expf(scaled - max_scaled) * 4294967296.0f;
     const unsigned long long w = static_cast<unsigned long long>(__float2uint_rn(x)) + (x >= 4294967296.0f ? 1u : 0u);
     return x != x ? 0x8000000000000000ull : w;
@@ -628,7 +632,7 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
         float cut[kNucCuts] = {};
 #pragma unroll
         for (int j = 0; j < kNucRegs; ++j) {
-            z += nucleus_weight(v[j], ms);
+            z += nucleus_weight_in_regs(v[j], ms);
             const float d = ms - v[j];
             if (d <= nucleus_cut(kNucCuts - 1)) {
                 const float e = expf(v[j] - ms);
@@ -707,7 +711,7 @@ nucleus_kernel(const float* logits, long long row_stride, int vocab, float inv_t
                     const float uniform = uniforms ? uniforms[static_cast<long long>(row) * u_stride] : 0.f;
                     const uint32_t* key = reinterpret_cast<const uint32_t*>(sh.hist);
                     unsigned long long* weight = sh.hist + kNucCand / 2;  // behind the keys
-                    if (tid < count) weight[tid] = nucleus_weight(key_to_float(key[tid]), ms);
+                    if (tid < count) weight[tid] = nucleus_weight_in_regs(key_to_float(key[tid]), ms);
                     __syncthreads();
                     const int at = tid >> 2, part = tid & 3;
                     const bool live = at < count;
