@@ -7,17 +7,23 @@
 // ~2000 flop per weight byte), so this kernel is built around the tensor pipe:
 //
 //   * a pair of CTAs (tcgen05 cta_group::2) owns 256 weight rows (the MMA's M, 128 per CTA) x up to 256 activation rows
-//     (its N, of which each CTA loads half: one CTA alone would have to pull 64 KB of activations through L2 per 128-k
-//     group, 18 TB/s over the chip at full tensor rate);
-//   * the int4 values go into the MMA as exact fp16 integers.  One 128-k group accumulates into one of two
-//     tensor-memory tiles of 256 columns (four of 128 up to 128 rows), and while the tensor core works on the next group eight warps read the finished one back
-//     and fold it into fp32 registers with the group's scale: acc += d * scale, the reference's own association
-//     (src/ops/linear.cpp:239-287).  So every product is exact and every weight costs one MMA (the form before this one
-//     put scale * weight into the MMA as a high and a low fp16 operand, two MMAs per k step, because it kept one
-//     accumulator over all of K: 113 us at M = 512, K = 5120, N = 17408);
-//   * both operands from shared memory: the activations land by TMA in the canonical 128-byte-swizzled K-major layout,
-//     the packed weights land raw (64 bytes per row and group) and four warps, one thread per weight row, unpack them
-//     into the same layout (up to 128 rows eight, four to every other group);
+//     (of which each CTA loads half: one CTA alone would have to pull 64 KB of activations through L2 per 128-k group, 18 TB/s
+//     over the chip at full tensor rate);
+//   * the int4 values go into the MMA as exact fp16 integers.  One 128-k group accumulates into a tensor-memory tile of up to 192
+//     columns (above 192 activation rows two such tiles of half the rows each, one after the other).  There are two or three, and while
+//     the tensor core works on the next one eight warps read the finished one back and fold it into fp32 registers with the group's
+//     scale: acc += d * scale, the reference's own association (src/ops/linear.cpp:239-287).  So every product is exact and every weight
+//     costs one MMA;
+//   * the weights are the operand in tensor memory, the activations the one in shared memory.  Activations land by TMA in the
+//     canonical 128-byte-swizzled K-major layout; the packed weights land raw (64 bytes per row and group) and four warps, one
+//     thread per weight row, unpack them into their lanes of tensor memory (up to 128 rows eight, four to every other group).
+//     With both operands in shared memory its bandwidth was the pace: of 128 bytes a clock, a CTA's group moved 8 KB of packed
+//     weights in and out, 32 KB of unpacked ones in and out, and its half of the activations in and out, 900 clocks at 96 rows
+//     (measured: 860 a group, the MMAs of it 384) and 1270 at 256 (1215; 1024).  The unpacked weights were 512 of either.
+//     What is the pace now: up to 128 rows issue slots, 70 % of which are taken, most of all on the scheduler that the MMA warp shares
+//     with two fold and two unpacking warps (700 to 900 clocks a group); at 256 rows the MMAs, at the clock that the power limit
+//     leaves (720 to 780 ns a group: 1.6 to 1.7 PFLOP/s, what the library's GEMM reaches in a burst).  Gate/up 5120 x 17408, one GPU
+//     in turn: 77 rows 45.0 -> 40.7 us, 96 44.5 -> 43.2, 160 56.4 -> 53.2, 352 115.8 -> 108.1, 512 141.5 -> 138.6;
 //   * the work of one launch - all tiles of all its projections x K / 128 groups - is dealt to one pair per two SMs, whole
 //     tiles or, where that leaves the last wave too empty, cut evenly.  A tile that straddles a cut is finished by the CTA
 //     that arrives last, which adds the others' fp32 partials in pair order (the result does not depend on who is last).
@@ -45,65 +51,71 @@ constexpr int kGemmFoldThreads = 256;    // two per weight row: each folds half 
 constexpr int kGemmUnpackThreads = 128;  // one per weight row
 constexpr int kGemmThreads = kGemmFoldThreads + kGemmUnpackThreads + 128;  // + a warpgroup with the two TMA warps and the MMA warp
 constexpr int kGemmUnpackWarp0 = 8, kGemmXWarp = 12, kGemmMmaWarp = 13, kGemmWWarp = 14, kGemmUnpackWarp1 = 16;
-// Sets of unpacking warps, which take the groups in turn.  A set needs 1100 clocks a group (600 of work, the rest two waits and the
-// fences); at more than 128 rows the MMAs take as long.  Up to 128 rows a second
-// set brings gate/up 5120 x 17408 from 49.7 to 46.9 us at 77 rows and from 52.2 to 48.0 at 128, 5120 x 14336 at 128 from 26.7 to 24.2.
-constexpr int gemm_unpack_sets(int nc) { return nc <= 2 ? 2 : 1; }
-constexpr int gemm_threads(int nc) { return kGemmThreads + (gemm_unpack_sets(nc) - 1) * kGemmUnpackThreads; }
 constexpr int kGemmTileN = 128;   // weight rows of one CTA of a pair (gate/up: 64 of each)
-constexpr int kGemmTileM = 256;   // most activation rows per tile (the MMA's N)
+constexpr int kGemmTileM = 256;   // most activation rows per tile
 constexpr int kSwizzleK = 64;     // k of one 128-byte swizzle row of fp16
-// Operand ring: a slot holds a whole 128-k group of unpacked weights and of activations.  The MMA warp's own loop - waits, issue
-// and commits, each a hundred clocks or two - is what every stage goes through, and with 64-k slots it took longer than the
-// tensor core: at M = 512 900 TFLOP/s with three waits a slot (weights and activations apart), 1120 with one, 1150 to
-// 1280 with its instructions predicated and its two waits side by side (umma_ss_f16_pair, the MMA warp).
-// Accumulator tiles: tiles of at most 128 rows have four, the larger ones two (all of tensor memory).
-constexpr int kOpSlotsMax = 4, kDBufsMax = 4, kWSlotsMax = 8;
+// Shapes of a kernel: H accumulator tiles per group of C times 16 columns (the MMA's N).  Up to 192 activation rows are one accumulator
+// tile, of which tensor memory has room for two beside two slots of unpacked weights, up to 128 rows for three; more rows are two tiles of
+// half of them each.  The rows are a multiple of 16 * H, so that the rows of an accumulator tile that each CTA holds are whole 8-row
+// swizzle atoms.
+constexpr int kGemmTmemCols = 512, kASlotCols = 64, kDBufsMax = 3;
+constexpr int gemm_halves(int tile_m) { return tile_m > 192 ? 2 : 1; }
+constexpr int gemm_d_bufs(int c) { return c <= 8 ? 3 : 2; }
+constexpr int gemm_a_slots(int c) { return gemm_d_bufs(c) * c * 16 + 4 * kASlotCols <= kGemmTmemCols ? 4 : 2; }  // (at the end of it)
+// Up to 80 rows the two fold threads of a row take the groups in turn, all columns of each, and add their sums up when the tile is
+// done; with more, sums for all columns do not fit the registers and each takes half of the columns of every group.
+constexpr bool gemm_fold_in_turn(int h, int c) { return h == 1 && c <= 5; }
+// Sets of unpacking warps, which take the groups in turn.  Up to 128 rows the MMAs of a group take up to 512 clocks, less than a set needs.
+constexpr int gemm_unpack_sets(int h, int c) { return h == 1 && c <= 8 ? 2 : 1; }
+constexpr int gemm_threads(int h, int c) { return kGemmThreads + (gemm_unpack_sets(h, c) - 1) * kGemmUnpackThreads; }
+// Shared memory: a slot of either ring holds a whole 128-k group.
+constexpr int kXSlotsMax = 8, kWSlotsMax = 12, kASlotsMax = 4;
 constexpr int kWSlotBytes = kGemmTileN * 64;                    // 8 KB of packed weights: one group
-constexpr int kAHalfBytes = kGemmTileN * kSwizzleK * 2;         // 16 KB: 64 k of unpacked weights
-constexpr int kASlotBytes = 2 * kAHalfBytes;
-constexpr int kGemmTmemCols = 512;
 constexpr int kGemmMaxProj = 4;
-// Register split of the launch's 512 x 128, or 640 x 96: the fold keeps 128, or 64, sums per thread.
-constexpr int kUnpackRegs = 64, kCtrlRegs = 32;
-constexpr int gemm_fold_regs(int nc) { return nc <= 2 ? 144 : 208; }
-constexpr int gemm_split_regs(int nc) { return gemm_fold_regs(nc) * 256 + kUnpackRegs * 128 * gemm_unpack_sets(nc) + kCtrlRegs * 128; }
-static_assert(gemm_split_regs(4) <= 512 * 128 && gemm_split_regs(2) <= 640 * 96, "register split");
+// Register split of the launch's 512 x 128, or 640 x 96: the fold keeps up to 128, or 96, sums per thread.
+constexpr int kCtrlRegs = 32, kUnpackRegs = 64;
+constexpr int gemm_fold_regs(int h, int c) { return gemm_unpack_sets(h, c) == 2 ? 160 : 208; }
+constexpr int gemm_split_regs(int h, int c) { return gemm_fold_regs(h, c) * 256 + kUnpackRegs * 128 * gemm_unpack_sets(h, c) + kCtrlRegs * 128; }
+static_assert(gemm_split_regs(2, 8) <= 512 * 128 && gemm_split_regs(1, 12) <= 512 * 128 && gemm_split_regs(1, 8) <= 640 * 96, "register split");
 
 struct GemmCtrl {
     uint64_t w_full[kWSlotsMax], w_empty[kWSlotsMax];
-    uint64_t op_full[kOpSlotsMax], op_empty[kOpSlotsMax];  // full: the pair's unpack warps and the activations' bytes
-    uint64_t d_full[kDBufsMax], d_empty[kDBufsMax];
+    uint64_t x_full[kXSlotsMax];  // the activations' bytes, both CTAs'
+    // A group's MMAs are done: its accumulator tile (the second one of two) may be read, its slots of weights and activations be filled
+    // again.  One commit for all three: the ring has the length of the activations' and those who wait look up the group they wait for.
+    uint64_t done[kXSlotsMax], half_done[kXSlotsMax];
+    uint64_t a_full[kASlotsMax];  // the pair's unpacking warps
+    uint64_t d_empty[kDBufsMax];
     uint32_t tmem_base;
     int last_arrival;
     WaitState ws;
 };
 
-// [control] [alignment slack] [A ring] [X ring: slots x 2 x tile_m / 2 x 128 bytes] [W ring]
+// [control] [alignment slack] [X ring] [W ring] [sums that the two fold threads of a row trade]
 constexpr int kGemmSmemBytes = 227 * 1024;
 constexpr int kGemmSmemFixed = 1024 + static_cast<int>(sizeof(GemmCtrl));
-constexpr int gemm_slots_bytes(int tile_m, int slots) { return slots * (kASlotBytes + tile_m * 2 * kSwizzleK); }
-constexpr int gemm_op_slots(int tile_m) {
-    return kGemmSmemFixed + gemm_slots_bytes(tile_m, 4) + 3 * kWSlotBytes <= kGemmSmemBytes ? 4 : 3;
-}
+constexpr int gemm_x_slots(int h, int c) { return h * c <= 8 ? 8 : 4; }
+constexpr int gemm_x_half_bytes(int h, int c) { return h * c * 8 * 2 * kSwizzleK; }  // 64 k of a CTA's half of the rows
+constexpr int gemm_trade_bytes(int h, int c) { return gemm_fold_in_turn(h, c) ? kGemmFoldThreads * c * 8 * 4 : 0; }
 // (the packed weights come from HBM, a microsecond and more away: their ring takes the rest)
-constexpr int gemm_w_slots(int tile_m) {
-    const int n = (kGemmSmemBytes - kGemmSmemFixed - gemm_slots_bytes(tile_m, gemm_op_slots(tile_m))) / kWSlotBytes;
+constexpr int gemm_w_slots(int h, int c) {
+    const int n = (kGemmSmemBytes - kGemmSmemFixed - gemm_x_slots(h, c) * 2 * gemm_x_half_bytes(h, c) - gemm_trade_bytes(h, c)) / kWSlotBytes & ~1;
     return n < kWSlotsMax ? n : kWSlotsMax;
 }
-constexpr int gemm_d_bufs(int tile_m) { return tile_m > 128 ? 2 : kDBufsMax; }
-static_assert(gemm_w_slots(kGemmTileM) >= 3 && gemm_w_slots(128) >= 3, "shared memory");
-// Sets of unpacking warps that take the groups in turn keep to slots of their own: the rings' lengths are multiples of their number.
-// Otherwise a set would come to a slot that the other one used last, and a wait for a parity that tells its own last use from the next
-// would be let through by a use that lies between them, before the bytes have landed.
-constexpr bool gemm_sets_keep_their_slots() {
-    for (int tile_m = 32; tile_m <= kGemmTileM; tile_m += 32) {
-        const int sets = gemm_unpack_sets((tile_m + 63) / 64);
-        if (gemm_op_slots(tile_m) % sets || gemm_w_slots(tile_m) % sets) return false;
+// Who waits for a phase of a barrier by its parity must have seen the phase before it end, and the phase after it must not end before he
+// has looked.  Sets of unpacking warps that take the groups in turn come to every slot of the packed weights, and to every entry of
+// `done`, by themselves if the rings' lengths are multiples of their number; no group's MMAs are issued before those of the group that
+// lies as many before as there are accumulator tiles, or slots of unpacked weights, have been seen done: the ring is no shorter.
+constexpr bool gemm_rings_keep_in_step() {
+    for (int tile_m = 16; tile_m <= kGemmTileM; tile_m += 16 * gemm_halves(tile_m + 1)) {
+        const int h = gemm_halves(tile_m), c = tile_m / h / 16, sets = gemm_unpack_sets(h, c);
+        const int x = gemm_x_slots(h, c), w = gemm_w_slots(h, c), a = gemm_a_slots(c), d = gemm_d_bufs(c);
+        if (x % sets || w % sets || a % sets || x < d || x < a || x > kXSlotsMax || a > kASlotsMax || d > kDBufsMax || w < 8) return false;
+        if (d * c * 16 + a * kASlotCols > kGemmTmemCols) return false;
     }
     return true;
 }
-static_assert(gemm_sets_keep_their_slots(), "ring lengths");
+static_assert(gemm_rings_keep_in_step(), "ring lengths");
 
 struct GemmProj {
     const __half* scales[2];  // gate/up: of both
@@ -120,15 +132,14 @@ struct GemmParams {
     GemmProj proj[kGemmMaxProj];
     int num_proj;
     int m;           // activation rows
-    int tile_m;      // activation rows per tile, a multiple of 32
-    int w_slots;     // slots of the packed-weight ring
+    int tile_m;      // activation rows per tile, a multiple of 16 up to 192 and of 32 above
+    int pair_stores; // two neighbouring features of every output lie in one aligned word (fp16)
     int m_tiles;
     int groups;      // k / 128
     int scales_vec;  // every row of scales starts on a 16-byte boundary
     long long units;     // tiles * groups
     int pairs;           // CTA pairs of the launch
     int whole_tiles;     // cut between tiles only
-    int swiglu;      // a CTA's rows: gate and up of the same 64 features, sixteen and sixteen; y = silu(gate) * up
     long long wait_limit;
     int* status;
     int x_stage_limit;  // test hook: activation stages (of a CTA) from this index on are never requested (-1: off)
@@ -138,19 +149,19 @@ struct GemmParams {
 
 // (This and the commit are executed by a whole warp under uniform control flow; the lane with `issue` set issues.  Inside `if (leader)`
 // the descriptors were moved to uniform registers for every instruction: the eight of a group took 500 clocks, and 400 this way.)
-// D[tmem] (+)= A[smem descriptor] * B[smem descriptor], kind::f16, on a CTA pair: A and D rows 0-127 in the even CTA,
-// 128-255 in the odd one; B rows half and half, each CTA's at the descriptor's offset.  Issued by one thread of the even CTA.
-__device__ __forceinline__ void umma_ss_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+// D[tmem] (+)= A[tmem] * B[smem descriptor], kind::f16, on a CTA pair: A and D rows 0-127 in the even CTA's tensor memory,
+// 128-255 in the odd one's; B rows half and half, each CTA's at the descriptor's offset.  Issued by one thread of the even CTA.
+__device__ __forceinline__ void umma_ts_f16_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                                  uint32_t accumulate, uint32_t issue) {
     asm volatile(
         "{\n\t"
         ".reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "setp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
         "}"
         :
-        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(issue)
+        : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(issue)
         : "memory");
 }
 // Arrives on the mbarrier at this offset in both CTAs of the pair when every MMA issued so far has completed.
@@ -204,6 +215,39 @@ __device__ __forceinline__ void fold_barrier() { asm volatile("bar.sync 1, %0;" 
 
 __device__ __forceinline__ void store_out(float* y, float v) { *y = v; }
 __device__ __forceinline__ void store_out(__half* y, float v) { *y = __float2half_rn(v); }
+// `live` (of at most eight) activation rows of one output feature, from `y` on.  Neighbouring lanes trade four of their eight, so that each
+// stores two features of four rows: half the stores, each of four bytes.  `pairs`: such words are aligned, and neighbouring lanes agree
+// about `live`.  All lanes call.
+template <typename OutT>
+__device__ __forceinline__ void store_rows(OutT* y, long long ldy, const float* v, int live, bool pairs, int lane) {
+    if constexpr (sizeof(OutT) == 2) {
+        const bool odd = lane & 1;
+        uint32_t h[4], even_f[2], odd_f[2];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const __half2 t = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
+            h[j] = *reinterpret_cast<const uint32_t*>(&t);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const uint32_t theirs = __shfl_xor_sync(0xffffffffu, odd ? h[2 * j] : h[2 * j + 1], 1), mine = odd ? h[2 * j + 1] : h[2 * j];
+            even_f[j] = odd ? theirs : mine;
+            odd_f[j] = odd ? mine : theirs;
+        }
+        if (pairs && live >= 8) {
+            OutT* out = odd ? y - 1 + 2 * ldy : y;
+#pragma unroll
+            for (int j = 0; j < 2; ++j, out += 4 * ldy) {
+                *reinterpret_cast<uint32_t*>(out) = prmt(even_f[j], odd_f[j], 0x5410u);
+                *reinterpret_cast<uint32_t*>(out + ldy) = prmt(even_f[j], odd_f[j], 0x7632u);
+            }
+            return;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j, y += ldy)
+        if (j < live) store_out(y, v[j]);
+}
 
 // Scales of the groups g .. g + 7 of one weight row (g a multiple of 8; zero behind the last), and on to the next one.  `vec`:
 // the row starts on a 16-byte boundary and has a multiple of eight of them; a caller's scales may lie anywhere.
@@ -215,6 +259,11 @@ __device__ __forceinline__ uint4 load_scales(const unsigned short* sp, int g, in
 #pragma unroll
     for (int j = 0; j < 8; ++j) h[j] = g + j < groups ? __ldg(sp + g + j) : 0u;
     return make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, h[6] | h[7] << 16);
+}
+__device__ __forceinline__ void next_word(uint4& q) {
+    q.x = q.y;
+    q.y = q.z;
+    q.z = q.w;
 }
 __device__ __forceinline__ void shift_scales(uint4& q) {
     q.x = __funnelshift_r(q.x, q.y, 16);
@@ -244,20 +293,62 @@ __device__ __forceinline__ int proj_of_tile(const GemmParams& p, int tile) {
     return i;
 }
 
-// NC: 32-column reads a fold thread makes of an accumulator tile, ceil(tile_m / 64).
-template <int NC, typename OutT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1) w4a16_gemm_kernel(const __grid_constant__ GemmParams p) {
+// Eight packed int4 (k0 in the lowest nibble) -> (k0,k1) (k2,k3) (k4,k5) (k6,k7) as fp16 pairs.  As dequant_word, but each byte is first
+// copied into both halves of a register, its low nibble used of the one and its high nibble of the other, which leaves them in k order.
+// (Volatile: the words of a group are to be ready in registers when its slot of tensor memory becomes free.)
+__device__ __forceinline__ void dequant_word_in_order(uint32_t w, uint32_t* q) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        asm volatile(
+            "{\n\t"
+            ".reg .b32 t;\n\t"
+            "prmt.b32 t, %1, 0, %2;\n\t"
+            "lop3.b32 t, t, 0x00F0000F, %3, 0x6A;\n\t"
+            "sub.f16x2 %0, t, %3;\n\t"
+            "}"
+            : "=r"(q[j])
+            : "r"(w), "r"(0x4040u | static_cast<uint32_t>(j * 0x101)), "r"(0x54806408u));
+}
+
+// acc0 += d0 * sc, acc1 += d1 * sc: two roundings each as fmaf has, one instruction.  (Volatile: it stays where it stands between the reads.)
+__device__ __forceinline__ void fma_pair(float& acc0, float& acc1, uint32_t d0, uint32_t d1, float sc) {
+    asm volatile(
+        "{\n\t"
+        ".reg .b64 a, b, c;\n\t"
+        "mov.b64 a, {%0, %1};\n\t"
+        "mov.b64 b, {%2, %3};\n\t"
+        "mov.b64 c, {%4, %4};\n\t"
+        "fma.rn.f32x2 a, b, c, a;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t"
+        "}"
+        : "+f"(acc0), "+f"(acc1)
+        : "r"(d0), "r"(d1), "f"(sc));
+}
+// f(Step<0>()) ... f(Step<N - 1>()): a loop whose index is a constant.
+template <int I>
+struct Step { static constexpr int value = I; };
+template <int N, int I = 0, typename F>
+__device__ __forceinline__ void for_steps(F&& f) {
+    if constexpr (I < N) {
+        f(Step<I>());
+        for_steps<N, I + 1>(f);
+    }
+}
+
+// H accumulator tiles a group of C times 16 columns each.  kSwiglu: a CTA's rows are gate and up of the same
+// 64 features, sixteen and sixteen; y = silu(gate) * up.
+template <int H, int C, typename OutT, bool kSwiglu>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(H, C), 1) w4a16_gemm_kernel(const __grid_constant__ GemmParams p) {
     extern __shared__ uint8_t gemm_smem_raw[];
     // (the control block first: its addresses are then constants, and the fold, which needs every register, holds none of them)
     GemmCtrl* ctrl = reinterpret_cast<GemmCtrl*>(gemm_smem_raw);
     // the swizzled operand tiles want 1024-byte alignment
-    uint8_t* a_ring = gemm_smem_raw + (((smem_u32(gemm_smem_raw) + sizeof(GemmCtrl) + 1023u) & ~1023u) - smem_u32(gemm_smem_raw));
-    constexpr int d_bufs = gemm_d_bufs(NC * 64), d_shift = d_bufs == 2 ? 1 : 2, d_cols = kGemmTmemCols / d_bufs;
-    const int op_slots = gemm_op_slots(p.tile_m);
-    uint8_t* x_ring = a_ring + op_slots * kASlotBytes;
-    const uint32_t x_half_bytes = static_cast<uint32_t>(p.tile_m) * kSwizzleK;  // 64 k of this CTA's half of the rows
-    uint8_t* w_ring = x_ring + op_slots * 2 * x_half_bytes;
-    const int w_slots = p.w_slots;
+    uint8_t* x_ring = gemm_smem_raw + (((smem_u32(gemm_smem_raw) + sizeof(GemmCtrl) + 1023u) & ~1023u) - smem_u32(gemm_smem_raw));
+    constexpr int acc_cols = C * 16, half_cols = C * 8, tile_m = H * acc_cols;
+    constexpr int x_slots = gemm_x_slots(H, C), x_shift = x_slots == 8 ? 3 : 2, w_slots = gemm_w_slots(H, C), a_slots = gemm_a_slots(C);
+    constexpr int d_bufs = gemm_d_bufs(C);
+    constexpr uint32_t x_half_bytes = gemm_x_half_bytes(H, C);
+    uint8_t* w_ring = x_ring + x_slots * 2 * x_half_bytes;
 
     const int tid = threadIdx.x;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -268,11 +359,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
 
     if (tid == 0) {
         for (int i = 0; i < w_slots; ++i) { mbar_init(smem_u32(&ctrl->w_full[i]), 1); mbar_init(smem_u32(&ctrl->w_empty[i]), kGemmUnpackThreads / 32); }
-        for (int i = 0; i < op_slots; ++i) {
-            mbar_init(smem_u32(&ctrl->op_full[i]), 2 * kGemmUnpackThreads / 32 + 1);
-            mbar_init(smem_u32(&ctrl->op_empty[i]), 1);
+        for (int i = 0; i < x_slots; ++i) {
+            mbar_init(smem_u32(&ctrl->x_full[i]), 1);
+            mbar_init(smem_u32(&ctrl->done[i]), 1);
+            mbar_init(smem_u32(&ctrl->half_done[i]), 1);
         }
-        for (int i = 0; i < d_bufs; ++i) { mbar_init(smem_u32(&ctrl->d_full[i]), 1); mbar_init(smem_u32(&ctrl->d_empty[i]), 2 * kGemmFoldThreads / 32); }
+        for (int i = 0; i < a_slots; ++i) mbar_init(smem_u32(&ctrl->a_full[i]), 2 * kGemmUnpackThreads / 32);
+        for (int i = 0; i < d_bufs; ++i) mbar_init(smem_u32(&ctrl->d_empty[i]), 2 * kGemmFoldThreads / 32 / (gemm_fold_in_turn(H, C) ? 2 : 1));
         ctrl->ws.abort_flag = 0;
         ctrl->ws.dep_ready = 0;
         ctrl->ws.limit = p.wait_limit;
@@ -291,7 +384,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
     const int U = static_cast<int>(u1 - u0);
     const int first_tile = static_cast<int>(u0 / p.groups), first_group = static_cast<int>(u0 - static_cast<long long>(first_tile) * p.groups);
 
-    constexpr int kSets = gemm_unpack_sets(NC);
+    constexpr int kSets = gemm_unpack_sets(H, C);
+    const uint32_t a_base = tmem_base + kGemmTmemCols - static_cast<uint32_t>(a_slots * kASlotCols);
     if (warp >= kGemmXWarp && warp < kGemmUnpackWarp1) {
         setmaxnreg_dec<kCtrlRegs>();
         if (warp == kGemmWWarp) {
@@ -300,7 +394,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
             // projection, the divisions and the address of its map worked out per stage, 500 clocks each, they held everybody up.)
             const bool leader = elect_one_sync();
             if (leader)
-                for (int i = 0; i < (p.swiglu ? 2 : p.num_proj); ++i) tma_prefetch_desc(&p.w_map[i]);
+                for (int i = 0; i < (kSwiglu ? 2 : p.num_proj); ++i) tma_prefetch_desc(&p.w_map[i]);
             const uint64_t pol_w = l2_policy_evict_first();
             const uint32_t ring = smem_u32(w_ring), full0 = smem_u32(&ctrl->w_full[0]), empty0 = smem_u32(&ctrl->w_empty[0]);
             int slot = 0, n = 0, group = first_group;
@@ -308,16 +402,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
             bool ok = true;
             for (int tile = first_tile; n < U && ok; ++tile) {
                 const int pr = proj_of_tile(p, tile), nt = (tile - p.proj[pr].tile0) / p.m_tiles * 2 + static_cast<int>(rank);
-                const CUtensorMap *map0 = &p.w_map[p.swiglu ? 0 : pr], *map1 = &p.w_map[1];
-                const int y = nt * (p.swiglu ? 64 : kGemmTileN), end = U - n < p.groups - group ? group + (U - n) : p.groups;
+                const CUtensorMap *map0 = &p.w_map[kSwiglu ? 0 : pr], *map1 = &p.w_map[1];
+                const int y = nt * (kSwiglu ? 64 : kGemmTileN), end = U - n < p.groups - group ? group + (U - n) : p.groups;
                 for (; group < end; ++group, ++n) {
                     const uint32_t full = full0 + slot * 8, dst = ring + slot * kWSlotBytes;
                     ok = mbar_wait_parked(empty0 + slot * 8, phase, ws);
+                    // (all CTAs start together: without a pause the first group would come back interleaved with the whole ring of every CTA)
+                    if (n == 3) ok = ok && mbar_wait_parked(full0, 0, ws);
                     if (!ok) break;
                     if (leader) {
                         mbar_arrive_expect_tx(full, kWSlotBytes);
                         tma_load_2d(dst, map0, full, group * 64, y, pol_w);
-                        if (p.swiglu) tma_load_2d(dst + kWSlotBytes / 2, map1, full, group * 64, y, pol_w);
+                        if (kSwiglu) tma_load_2d(dst + kWSlotBytes / 2, map1, full, group * 64, y, pol_w);
                     }
                     __syncwarp();  // (or the other lanes wait for the next slot before this one's load is issued)
                     if (++slot == w_slots) { slot = 0; phase ^= 1u; }
@@ -340,7 +436,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
             if (leader) tma_prefetch_desc(&p.x_map);
             const uint64_t pol_x = l2_policy_evict_last();
             const int SX = (p.x_stage_limit >= 0 && p.x_stage_limit < U) ? p.x_stage_limit : U;
-            const uint32_t ring = smem_u32(x_ring), full0 = smem_u32(&ctrl->op_full[0]), empty0 = smem_u32(&ctrl->op_empty[0]);
+            const uint32_t ring = smem_u32(x_ring), full0 = smem_u32(&ctrl->x_full[0]), empty0 = smem_u32(&ctrl->done[0]);
             // both halves of the rows are counted on the even CTA's barrier, where the MMAs are issued
             const uint32_t pair_full0 = mapa_shared_cluster(full0, 0);
             griddep_wait();
@@ -349,25 +445,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
             uint32_t phase = 1;
             bool ok = true;
             for (int tile = first_tile; nx < SX && ok; ++tile) {
-                const int m0 = (tile - p.proj[proj_of_tile(p, tile)].tile0) % p.m_tiles * p.tile_m + static_cast<int>(rank) * (p.tile_m >> 1);
+                const int m0 = (tile - p.proj[proj_of_tile(p, tile)].tile0) % p.m_tiles * tile_m + static_cast<int>(rank) * (tile_m >> 1);
                 for (; k0 < p.groups * 128 && nx < SX; k0 += 128, ++nx) {
                     ok = mbar_wait_parked(empty0 + slot * 8, phase, ws);
                     if (!ok) break;
                     if (leader) {
-                        if (rank == 0) mbar_arrive_expect_tx(full0 + slot * 8, 4 * x_half_bytes);
+                        if (rank == 0) mbar_arrive_expect_tx(full0 + slot * 8, tile_m * 256u);
                         tma_load_2d_pair(ring + slot * 2 * x_half_bytes, &p.x_map, pair_full0 + slot * 8, k0, m0, pol_x);
                         tma_load_2d_pair(ring + slot * 2 * x_half_bytes + x_half_bytes, &p.x_map, pair_full0 + slot * 8, k0 + kSwizzleK, m0, pol_x);
                     }
                     __syncwarp();
-                    if (++slot == op_slots) { slot = 0; phase ^= 1u; }
+                    if (++slot == x_slots) { slot = 0; phase ^= 1u; }
                 }
                 k0 = 0;
             }
             if (ws->abort_flag) {
                 const long long t0 = clock64();
-                for (int i = 0; i < op_slots && i < nx; ++i) {
+                for (int i = 0; i < x_slots && i < nx; ++i) {
                     const int k = nx - 1 - i;
-                    while (!mbar_try_wait(smem_u32(&ctrl->op_full[k % op_slots]), (k / op_slots) & 1u) && clock64() - t0 < p.wait_limit / 8) {
+                    while (!mbar_try_wait(smem_u32(&ctrl->x_full[k % x_slots]), (k / x_slots) & 1u) && clock64() - t0 < p.wait_limit / 8) {
                     }
                 }
             }
@@ -375,134 +471,238 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
         } else if (warp == kGemmMmaWarp && rank == 0) {
             // -------------------------------------------------------------- MMA issuer of the pair
             const bool leader = elect_one_sync();
-            const uint32_t idesc = umma_idesc_f16_f32(256, 0) | (static_cast<uint32_t>(p.tile_m >> 3) << 17);
+            const uint32_t idesc = umma_idesc_f16_f32(256, 0) | (static_cast<uint32_t>(acc_cols >> 3) << 17);
             // K-major, 128-byte swizzle: rows of 64 k, 8-row groups 1024 bytes apart; descriptor version 1
             constexpr uint32_t desc_hi = ((1024u >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);
             constexpr uint32_t desc_lo_const = 1u << 16;
-            const uint32_t a_lo0 = (smem_u32(a_ring) >> 4) & 0x3FFFu;
             const uint32_t x_lo0 = (smem_u32(x_ring) >> 4) & 0x3FFFu;
-            bool ok = true;
-            uint32_t slot = 0, phase = 0;
+            // (Barriers are asked in the middle of the group before, all before any answer is looked at: an answer takes a hundred clocks, also
+            // where there is nothing to wait for, and the tensor core has little more than that to do when a group's last MMA is issued.)
+            const uint32_t x_bar0 = smem_u32(&ctrl->x_full[0]), a_bar0 = smem_u32(&ctrl->a_full[0]), d_bar0 = smem_u32(&ctrl->d_empty[0]);
+            bool ok = true, x_ready = false, a_ready = false, d_ready = true;  // (an unused accumulator tile is ready)
+            uint32_t xslot = 0, x_phase = 0, aslot = 0, a_phase = 0, buf = 0, d_phase = 1;
             for (int i = 0; i < U && ok; ++i) {
-                const uint32_t buf = static_cast<uint32_t>(i & (d_bufs - 1));
-                // (both asked before either answer is looked at: an answer takes a hundred clocks, also where there is nothing to wait for)
-                const uint32_t d_bar = smem_u32(&ctrl->d_empty[buf]), d_phase = ((i >> d_shift) & 1u) ^ 1u, op_bar = smem_u32(&ctrl->op_full[slot]);
-                const bool d_ready = mbar_try_wait(d_bar, d_phase), op_ready = mbar_try_wait(op_bar, phase);  // (an unused tile is ready)
-                ok = (d_ready || mbar_wait_parked(d_bar, d_phase, ws)) && (op_ready || mbar_wait_parked(op_bar, phase, ws));
-                if (!ok) break;
-                tc_fence_after_sync();
+                const uint32_t x_now = x_lo0 + xslot * (2 * x_half_bytes >> 4), a_now = a_base + aslot * kASlotCols;
+                ok = (x_ready || mbar_wait_parked(x_bar0 + xslot * 8, x_phase, ws)) && (a_ready || mbar_wait_parked(a_bar0 + aslot * 8, a_phase, ws));
+                const uint32_t done_bar = smem_u32(&ctrl->done[0]) + xslot * 8, half_bar = smem_u32(&ctrl->half_done[0]) + xslot * 8;
+                if (++xslot == static_cast<uint32_t>(x_slots)) { xslot = 0; x_phase ^= 1u; }
+                if (++aslot == static_cast<uint32_t>(a_slots)) { aslot = 0; a_phase ^= 1u; }
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const uint32_t alo = desc_lo_const | (a_lo0 + ((slot * kASlotBytes + (k >> 2) * kAHalfBytes + (k & 3) * 32) >> 4));
-                    const uint32_t xlo = desc_lo_const | (x_lo0 + ((slot * 2 * x_half_bytes + (k >> 2) * x_half_bytes + (k & 3) * 32) >> 4));
-                    umma_ss_f16_pair(tmem_base + buf * d_cols, (static_cast<uint64_t>(desc_hi) << 32) | alo,
-                                     (static_cast<uint64_t>(desc_hi) << 32) | xlo, idesc, k > 0 ? 1u : 0u, leader);
+                for (int h = 0; h < H; ++h) {
+                    ok = ok && (d_ready || mbar_wait_parked(d_bar0 + buf * 8, d_phase, ws));
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    const uint32_t d_now = tmem_base + buf * acc_cols;
+                    const uint32_t b_now = desc_lo_const | (x_now + (h ? static_cast<uint32_t>(acc_cols) * 64 >> 4 : 0u));
+                    if (++buf == d_bufs) { buf = 0; d_phase ^= 1u; }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        if (k == 4) {
+                            d_ready = mbar_test_wait(d_bar0 + buf * 8, d_phase);
+                            if (h == H - 1) {
+                                x_ready = mbar_test_wait(x_bar0 + xslot * 8, x_phase);
+                                a_ready = mbar_test_wait(a_bar0 + aslot * 8, a_phase);
+                            }
+                        }
+                        umma_ts_f16_pair(d_now, a_now + k * 8, (static_cast<uint64_t>(desc_hi) << 32) | (b_now + ((k >> 2) * x_half_bytes + (k & 3) * 32 >> 4)),
+                                         idesc, k > 0 ? 1u : 0u, leader);
+                    }
+                    umma_commit_pair(h == H - 1 ? done_bar : half_bar, leader);
+                    __syncwarp();
                 }
-                umma_commit_pair(smem_u32(&ctrl->op_empty[slot]), leader);
-                umma_commit_pair(smem_u32(&ctrl->d_full[buf]), leader);
-                __syncwarp();
-                if (++slot == static_cast<uint32_t>(op_slots)) { slot = 0; phase ^= 1u; }
             }
         }
     } else if (warp >= kGemmUnpackWarp0) {
         // ------------------------------------------------------------------ unpack: one thread per weight row of the tile
         setmaxnreg_dec<kUnpackRegs>();
         const int r = tid & (kGemmUnpackThreads - 1), set = warp >= kGemmUnpackWarp1 ? 1 : 0;
-        // raw rows of 64 bytes under the 64-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ ((r >> 1) & 3)
-        const uint32_t w_row = static_cast<uint32_t>(r) * 64, w_sw = static_cast<uint32_t>((r >> 1) & 3);
         // gate/up: the raw tile is 64 rows of each, the operand sixteen and sixteen, so that a feature's two sums meet in one warp
-        const int ra = p.swiglu ? ((r & 48) << 1) + ((r >> 6) << 4) + (r & 15) : r;
-        const uint32_t a_row = static_cast<uint32_t>((ra >> 3) * 1024 + (ra & 7) * 128), a_sw = static_cast<uint32_t>(ra & 7);
-        int wslot = set, aslot = set;  // (a set's own slots: gemm_sets_keep_their_slots)
-        uint32_t w_phase = 0, a_phase = 1;
+        const int rr = kSwiglu ? ((r >> 5) << 4) + (r & 15) + ((r & 16) << 2) : r;
+        // raw rows of 64 bytes under the 64-byte swizzle: 16-byte chunk c of row rr sits at chunk c ^ ((rr >> 1) & 3)
+        const uint32_t w_row = smem_u32(w_ring) + static_cast<uint32_t>(rr) * 64, w_sw = static_cast<uint32_t>((rr >> 1) & 3);
+        const uint32_t a_row = a_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+        int wslot = set;  // (a set's own slots: gemm_rings_keep_in_step)
+        uint32_t w_phase = 0;
+        constexpr int kAhead = 8;  // of a group's sixteen words, those unpacked before its slot is asked for
         for (int i = set; i < U; i += kSets) {
-            const uint32_t w_bar = smem_u32(&ctrl->w_full[wslot]), a_bar = smem_u32(&ctrl->op_empty[aslot]);
-            const bool w_ready = mbar_try_wait(w_bar, w_phase), a_ready = mbar_try_wait(a_bar, a_phase);  // (as in the MMA warp)
-            if (!w_ready && !mbar_wait(w_bar, w_phase, ws)) break;
-            const uint32_t wsrc = smem_u32(w_ring) + wslot * kWSlotBytes + w_row;
+            // the slot's last user: the group a_slots before this one
+            const int last = i - a_slots;
+            const uint32_t w_bar = smem_u32(&ctrl->w_full[wslot]), a_bar = smem_u32(&ctrl->done[last & (x_slots - 1)]);
+            const uint32_t a_phase = static_cast<uint32_t>(last >> x_shift) & 1u;
+            if (!__all_sync(0xffffffffu, mbar_wait(w_bar, w_phase, ws))) break;
+            const uint32_t wsrc = w_row + wslot * kWSlotBytes;
             uint4 v[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) v[c] = lds128(wsrc + ((static_cast<uint32_t>(c) ^ w_sw) << 4));
-            if (!a_ready && !mbar_wait(a_bar, a_phase, ws)) break;
-            const uint32_t adst = smem_u32(a_ring) + aslot * kASlotBytes + a_row;
+            const uint32_t adst = a_row + static_cast<uint32_t>(i & (a_slots - 1)) * kASlotCols;
+            uint32_t q[kAhead * 4];
 #pragma unroll
-            for (int w = 0; w < 16; ++w) {
+            for (int w = 0; w < kAhead; ++w) {
                 const uint4& vw = v[w >> 2];
-                uint32_t q[4];
-                dequant_word((w & 3) == 0 ? vw.x : (w & 3) == 1 ? vw.y : (w & 3) == 2 ? vw.z : vw.w, q);  // (k0,k4) (k1,k5) (k2,k6) (k3,k7)
-                uint4 o;
-                o.x = prmt(q[0], q[1], 0x5410u);  // (k0,k1)
-                o.y = prmt(q[2], q[3], 0x5410u);  // (k2,k3)
-                o.z = prmt(q[0], q[1], 0x7632u);  // (k4,k5)
-                o.w = prmt(q[2], q[3], 0x7632u);  // (k6,k7)
-                sts128(adst + (w >> 3) * kAHalfBytes + ((static_cast<uint32_t>(w & 7) ^ a_sw) << 4), o);
+                dequant_word_in_order((w & 3) == 0 ? vw.x : (w & 3) == 1 ? vw.y : (w & 3) == 2 ? vw.z : vw.w, q + w * 4);
             }
-            fence_proxy_async_smem();  // the tensor core reads this tile through the async proxy
+            if (!__all_sync(0xffffffffu, last < 0 || mbar_wait(a_bar, a_phase, ws))) break;  // (tcgen05.st wants the whole warp)
+            tc_fence_after_sync();
+#pragma unroll
+            for (int w = 0; w < kAhead; w += 2) tmem_st8(adst + w * 4, q + w * 4);
+#pragma unroll
+            for (int w = kAhead; w < 16; w += 2) {
+                uint32_t t[8];
+                const uint4& vw = v[w >> 2];
+                dequant_word_in_order((w & 2) ? vw.z : vw.x, t);
+                dequant_word_in_order((w & 2) ? vw.w : vw.y, t + 4);
+                tmem_st8(adst + w * 4, t);
+            }
+            if (lane == 0) mbar_arrive(smem_u32(&ctrl->w_empty[wslot]));
+            tmem_wait_st();
+            tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive_cluster(mapa_shared_cluster(smem_u32(&ctrl->op_full[aslot]), 0));
-                mbar_arrive(smem_u32(&ctrl->w_empty[wslot]));
-            }
-            if ((aslot += kSets) >= op_slots) { aslot -= op_slots; a_phase ^= 1u; }
+            if (lane == 0) mbar_arrive_cluster(mapa_shared_cluster(smem_u32(&ctrl->a_full[i & (a_slots - 1)]), 0));
             if ((wslot += kSets) >= w_slots) { wslot -= w_slots; w_phase ^= 1u; }
         }
     } else {
         // ------------------------------------------------------------------ fold, then write: two threads per weight row
-        setmaxnreg_inc<gemm_fold_regs(NC)>();
-        const int r = tid & 127, ch = tid >> 7;          // tile row, column half
-        const int half_cols = p.tile_m >> 1;             // a multiple of 16
-        const uint32_t d_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(ch * half_cols);
-        const bool up_row = p.swiglu && (r & 16);
-        float acc[NC * 32];
+        setmaxnreg_inc<gemm_fold_regs(H, C)>();
+        const int r = tid & 127, ch = tid >> 7;  // tile row, and which of the row's two threads
+        constexpr bool kInTurn = gemm_fold_in_turn(H, C);
+        const uint32_t d_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + (kInTurn ? 0u : static_cast<uint32_t>(ch * half_cols));
+        const uint32_t d_empty0 = mapa_shared_cluster(smem_u32(&ctrl->d_empty[0]), 0);
+        const bool up_row = kSwiglu && (r & 16);
+        // (accumulator tile h holds, of each CTA's activation rows, those from h * half_cols on: a thread's columns are rows in sequence)
+        constexpr int kCols = kInTurn ? half_cols : (half_cols + 15) / 16 * 16;  // of an accumulator tile, as they are written
+        float acc[kInTurn ? acc_cols : H * kCols];
+        uint32_t buf = kInTurn ? static_cast<uint32_t>(ch) : 0u;
         int i = 0, tile = first_tile, group = first_group;
         bool dead = false;
+        auto wait_tile = [&](int n, int h) {  // (tcgen05.ld wants the whole warp)
+            const uint32_t bar = smem_u32(h == H - 1 ? &ctrl->done[0] : &ctrl->half_done[0]) + static_cast<uint32_t>(n & (x_slots - 1)) * 8;
+            dead = !__all_sync(0xffffffffu, !dead && mbar_wait_parked(bar, static_cast<uint32_t>(n >> x_shift) & 1u, ws));
+            if (!dead) tc_fence_after_sync();
+            return !dead;
+        };
+        auto release_tile = [&]() {  // the MMA warp may have the columns
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(d_empty0 + buf * 8);
+        };
         while (i < U) {
             // one tile, or the part of it that lies in this pair's range
             const int pr = proj_of_tile(p, tile);
             const GemmProj& pj = p.proj[pr];
-            const int rel = tile - pj.tile0, nt = rel / p.m_tiles * 2 + static_cast<int>(rank), m0 = (rel % p.m_tiles) * p.tile_m;
-            const int row = p.swiglu ? nt * 64 + ((r & 96) >> 1) + (r & 15) : nt * kGemmTileN + r;
+            const int rel = tile - pj.tile0, nt = rel / p.m_tiles * 2 + static_cast<int>(rank), m0 = (rel % p.m_tiles) * tile_m;
+            const int row = kSwiglu ? nt * 64 + ((r & 96) >> 1) + (r & 15) : nt * kGemmTileN + r;
             const bool valid = row < pj.n;
             const unsigned short* sp = reinterpret_cast<const unsigned short*>(pj.scales[up_row ? 1 : 0]) +
                                        static_cast<long long>(valid ? row : 0) * p.groups;
             const int seg_begin = group, seg_end = (U - i < p.groups - group) ? group + (U - i) : p.groups;
 #pragma unroll
-            for (int j = 0; j < NC * 32; ++j) acc[j] = 0.f;
-            // scales eight groups at a time, a block of eight ahead of its use (one group ahead, their latency is the loop's)
-            uint4 q_cur = load_scales(sp, seg_begin & ~7, p.groups, p.scales_vec), q_next = load_scales(sp, (seg_begin & ~7) + 8, p.groups, p.scales_vec);
-            for (int j = 0; j < (seg_begin & 7); ++j) shift_scales(q_cur);
-            for (; group < seg_end; ++group, ++i) {
-                const float sc = __half2float(__ushort_as_half(static_cast<unsigned short>(q_cur.x & 0xFFFFu)));
-                shift_scales(q_cur);
-                if ((group & 7) == 7) {
-                    q_cur = q_next;
-                    q_next = load_scales(sp, group + 9, p.groups, p.scales_vec);
-                }
-                const uint32_t buf = static_cast<uint32_t>(i & (d_bufs - 1));
-                if (dead || !mbar_wait_parked(smem_u32(&ctrl->d_full[buf]), (i >> d_shift) & 1u, ws)) { dead = true; continue; }
-                tc_fence_after_sync();
-                const uint32_t src = d_addr + buf * d_cols;
-                // 32 columns a read (one tcgen05.ld; with two of 16 the whole kernel is 20 % slower at M = 512).  A tile of
-                // fewer columns reads on into columns that are allocated and not used.
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    // (always true; without a branch between them the compiler sets up a read beside the additions of the one before it,
-                    // runs out of registers and keeps launch-wide values in memory, which costs every warp of the CTA: 12 % at M = 512)
-                    if (NC < 4 || c * 32 < half_cols) {
-                        uint32_t d[32];
-                        tmem_ld32(src + c * 32, d);
+            for (int j = 0; j < static_cast<int>(sizeof(acc) / sizeof(acc[0])); ++j) acc[j] = 0.f;
+            // Scales eight groups at a time, a block of eight ahead of its use (one group ahead, their latency is the loop's).
+            // One read of tensor memory is in flight while the one before it is added up, and a tile is handed back before its last columns
+            // are added: the slowest fold warp of the pair, which shares its scheduler with the MMA warp, is the pace.
+            if constexpr (kInTurn) {
+                const int n0 = i + ((i ^ ch) & 1), g0 = group + (n0 - i);  // this thread's first group
+                uint4 q_cur = load_scales(sp, g0 & ~7, p.groups, p.scales_vec), q_next = load_scales(sp, (g0 & ~7) + 8, p.groups, p.scales_vec);
+                const uint32_t pick = g0 & 1 ? 0x4432u : 0x4410u;  // its scales lie in the same half of every word
+                for (int j = 0; j < (g0 & 7) >> 1; ++j) next_word(q_cur);
+                constexpr int kOdd = C == 4 ? 32 : 16, kSteps = C <= 4 ? 2 : 3;  // 32 and 16, 32 and 32, or 32, 16 and 32 columns
+                uint32_t d0[32], d1[kOdd];
+                auto read = [&](auto step) {
+                    constexpr int t = decltype(step)::value, c = t / 2 * 48 + (t & 1) * 32;
+                    if constexpr (!(t & 1)) tmem_ld32(d_addr + buf * acc_cols + c, d0);
+                    else if constexpr (kOdd == 32) tmem_ld32(d_addr + buf * acc_cols + c, d1);
+                    else tmem_ld16(d_addr + buf * acc_cols + c, d1);
+                };
+                for (int g = g0, n = n0; g < seg_end; g += 2, n += 2) {
+                    const float sc = __half2float(__ushort_as_half(static_cast<unsigned short>(prmt(q_cur.x, 0u, pick))));
+                    next_word(q_cur);
+                    if ((g & 6) == 6) {
+                        q_cur = q_next;
+                        q_next = load_scales(sp, (g & ~7) + 16, p.groups, p.scales_vec);
+                    }
+                    if (!wait_tile(n, 0)) break;
+                    read(Step<0>());
+                    for_steps<kSteps>([&](auto step) {
+                        constexpr int t = decltype(step)::value, c = t / 2 * 48 + (t & 1) * 32, width = t & 1 ? kOdd : 32;
                         tmem_wait_ld();
-                        if (c == NC - 1) {  // the last read of this group: the MMA warp may have the columns
-                            tc_fence_before_sync();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive_cluster(mapa_shared_cluster(smem_u32(&ctrl->d_empty[buf]), 0));
-                        }
+                        if constexpr (t + 1 < kSteps) read(Step<t + 1>());
+                        else release_tile();
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) acc[c * 32 + j] = fmaf(__uint_as_float(d[j]), sc, acc[c * 32 + j]);
+                        for (int j = 0; j < width; j += 2) {
+                            if constexpr (t & 1) fma_pair(acc[c + j], acc[c + j + 1], d1[j], d1[j + 1], sc);
+                            else fma_pair(acc[c + j], acc[c + j + 1], d0[j], d0[j + 1], sc);
+                        }
+                    });
+                    buf = buf == 0 ? d_bufs - 1 : buf - 1;  // two further
+                }
+                i += seg_end - group;
+                group = seg_end;
+            } else {
+                uint4 q_cur = load_scales(sp, seg_begin & ~7, p.groups, p.scales_vec), q_next = load_scales(sp, (seg_begin & ~7) + 8, p.groups, p.scales_vec);
+                for (int j = 0; j < (seg_begin & 7); ++j) shift_scales(q_cur);
+                constexpr int kRead = H == 1 ? 32 : 16, kReads = (kCols + kRead - 1) / kRead, kSteps = H * kReads;
+                constexpr bool kAcross = kSteps % 2 == 0;  // (else the two buffers would change places from group to group)
+                uint32_t d[2][kRead];
+                auto read = [&](auto step) {
+                    constexpr int t = decltype(step)::value, c = t % kReads * kRead;
+                    // (a tile of fewer columns reads on into columns that are allocated and not used)
+                    if constexpr (kRead == 32 && kCols - c >= 32) tmem_ld32(d_addr + buf * acc_cols + c, d[t & 1]);
+                    else tmem_ld16(d_addr + buf * acc_cols + c, d[t & 1]);
+                };
+                if (wait_tile(i, 0)) {
+                    read(Step<0>());
+                    for (; group < seg_end && !dead; ++group, ++i) {
+                        const float sc = __half2float(__ushort_as_half(static_cast<unsigned short>(q_cur.x & 0xFFFFu)));
+                        shift_scales(q_cur);
+                        if ((group & 7) == 7) {
+                            q_cur = q_next;
+                            q_next = load_scales(sp, group + 9, p.groups, p.scales_vec);
+                        }
+                        for_steps<kSteps>([&](auto step) {
+                            constexpr int t = decltype(step)::value, h = t / kReads, c = t % kReads * kRead;
+                            tmem_wait_ld();
+                            if constexpr (t % kReads < kReads - 1) {
+                                read(Step<t + 1>());
+                            } else {
+                                release_tile();
+                                buf = buf == d_bufs - 1 ? 0 : buf + 1;
+                                if (t < kSteps - 1 || (kAcross && group + 1 < seg_end)) {
+                                    if (wait_tile(t < kSteps - 1 ? i : i + 1, (h + 1) % H)) read(Step<(t + 1) % kSteps>());
+                                }
+                            }
+#pragma unroll
+                            for (int j = 0; j < kRead && c + j < kCols; j += 2)
+                                fma_pair(acc[h * kCols + c + j], acc[h * kCols + c + j + 1], d[t & 1][j], d[t & 1][j + 1], sc);
+                            if constexpr (!kAcross && t == kSteps - 1) {
+                                if (group + 1 < seg_end && wait_tile(i + 1, 0)) read(Step<0>());
+                            }
+                        });
                     }
                 }
             }
             if (fold_barrier_or(dead || ws->abort_flag != 0)) break;
+
+            if constexpr (kInTurn) {
+                // The row's other thread has the other groups' sums: each passes half of its columns on and finishes the other half.  (The
+                // barrier above: the trade of the tile before has been read.)
+                float4* trade = reinterpret_cast<float4*>(w_ring + w_slots * kWSlotBytes);
+#pragma unroll
+                for (int j = 0; j < half_cols; j += 4) {
+                    const int k = half_cols + j;
+                    trade[j / 4 * kGemmFoldThreads + tid] = make_float4(ch ? acc[j] : acc[k], ch ? acc[j + 1] : acc[k + 1], ch ? acc[j + 2] : acc[k + 2],
+                                                                        ch ? acc[j + 3] : acc[k + 3]);
+                }
+                fold_barrier();
+#pragma unroll
+                for (int j = 0; j < half_cols; j += 4) {
+                    const int k = half_cols + j;
+                    const float4 t = trade[j / 4 * kGemmFoldThreads + (tid ^ 128)];
+                    acc[j] = (ch ? acc[k] : acc[j]) + t.x;
+                    acc[j + 1] = (ch ? acc[k + 1] : acc[j + 1]) + t.y;
+                    acc[j + 2] = (ch ? acc[k + 2] : acc[j + 2]) + t.z;
+                    acc[j + 3] = (ch ? acc[k + 3] : acc[j + 3]) + t.w;
+                }
+            }
 
             // ------------------------------------------------------------ a straddling tile: the last CTA to arrive finishes it
             int c_first = 0, c_last = 0;
@@ -532,8 +732,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
                 if (!kept) {
                     float4* mine = reinterpret_cast<float4*>(p.partials + (static_cast<size_t>(blockIdx.x) * 2 + (seg_begin > 0 ? 0 : 1)) * slot_floats) + tid;
 #pragma unroll
-                    for (int j = 0; j < NC * 32; j += 4)
-                        if (j < half_cols) __stcg(mine + j / 4 * kGemmFoldThreads, make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]));
+                    for (int j = 0; j < H * kCols; j += 4)
+                        __stcg(mine + j / 4 * kGemmFoldThreads, make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]));
                     __threadfence();
                     fold_barrier();
                     if (tid == 0) {
@@ -554,51 +754,56 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
                         // a contributor's part of this tile: slot 1 if the tile starts in its range, else slot 0
                         const float4* src = reinterpret_cast<const float4*>(base + static_cast<size_t>(c_first) * 4 * slot_floats + slot_floats);
 #pragma unroll
-                        for (int j = 0; j < NC * 32; j += 4) {
-                            if (j < half_cols) {
-                                const float4 t = __ldcg(src + j / 4 * kGemmFoldThreads);
-                                acc[j] = t.x;
-                                acc[j + 1] = t.y;
-                                acc[j + 2] = t.z;
-                                acc[j + 3] = t.w;
-                            }
+                        for (int j = 0; j < H * kCols; j += 4) {
+                            const float4 t = __ldcg(src + j / 4 * kGemmFoldThreads);
+                            acc[j] = t.x;
+                            acc[j + 1] = t.y;
+                            acc[j + 2] = t.z;
+                            acc[j + 3] = t.w;
                         }
                     }
+                    constexpr int kBatch = 12;
 #pragma unroll 1
                     for (int o = c_first + 1; o <= c_last; ++o) {
                         const float4* src = reinterpret_cast<const float4*>(base + static_cast<size_t>(o) * 4 * slot_floats);
 #pragma unroll
-                        for (int c = 0; c < NC * 32; c += 64) {
-                            if (c < half_cols) {
-                                float4 t[16];
+                        for (int c = 0; c < H * kCols / 4; c += kBatch) {
+                            float4 t[kBatch];
 #pragma unroll
-                                for (int j = 0; j < 16; ++j)
-                                    if (c + j * 4 < NC * 32) t[j] = __ldcg(src + (c / 4 + j) * kGemmFoldThreads);
+                            for (int j = 0; j < kBatch; ++j)
+                                if (c + j < H * kCols / 4) t[j] = __ldcg(src + (c + j) * kGemmFoldThreads);
 #pragma unroll
-                                for (int j = 0; j < 16; ++j) {
-                                    if (c + j * 4 >= NC * 32) continue;
-                                    acc[c + j * 4] += t[j].x;
-                                    acc[c + j * 4 + 1] += t[j].y;
-                                    acc[c + j * 4 + 2] += t[j].z;
-                                    acc[c + j * 4 + 3] += t[j].w;
-                                }
+                            for (int j = 0; j < kBatch; ++j) {
+                                if (c + j >= H * kCols / 4) continue;
+                                float* to = acc + (c + j) * 4;
+                                to[0] += t[j].x;
+                                to[1] += t[j].y;
+                                to[2] += t[j].z;
+                                to[3] += t[j].w;
                             }
                         }
                     }
                 }
             }
             if (!split || ctrl->last_arrival) {
-                const float bias = (valid && pj.bias && !p.swiglu) ? pj.bias[row] : 0.f;
+                const float bias = (valid && pj.bias && !kSwiglu) ? pj.bias[row] : 0.f;
 #pragma unroll
-                for (int c = 0; c < NC * 2; ++c) {
-                    if (c * 16 < half_cols) {
-                        const int mc = m0 + ch * half_cols + c * 16;
+                for (int c = 0; c < H * ((kCols + 15) / 16); ++c) {
+                    constexpr int kBlocks = (kCols + 15) / 16;
+                    const int col = c % kBlocks * 16, at = c / kBlocks * kCols + col;  // of its accumulator tile, in `acc`
+                    if (col < half_cols) {
+                        const int mc = m0 + ch * (tile_m >> 1) + c / kBlocks * half_cols + col;
+                        const int rows = p.m - mc < half_cols - col ? p.m - mc : half_cols - col;
                         OutT* out = static_cast<OutT*>(pj.y) + static_cast<long long>(mc) * pj.ldy + row;
-                        if (!p.swiglu) {
-                            const int live = valid ? p.m - mc : 0;
+                        if (!kSwiglu) {
 #pragma unroll
-                            for (int j = 0; j < 16; ++j, out += pj.ldy)
-                                if (j < live) store_out(out, acc[c * 16 + j] + bias);
+                            for (int b = 0; b < 16; b += 8) {
+                                float y[8];
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) y[j] = at + b + j < H * kCols ? acc[at + b + j] + bias : 0.f;
+                                if (b < half_cols - col) store_rows(out, pj.ldy, y, valid ? rows - b : 0, p.pair_stores, lane);
+                                out += 8 * pj.ldy;
+                            }
                         } else {
                             // Gate and up of one feature sit sixteen lanes apart, which trade halves of the 16 columns: the gate
                             // lane finishes columns 0-7, the up lane 8-15.  (Through shared memory, with two barriers per 16
@@ -606,7 +811,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
                             float y[8];  // (all of them before the first store: inside its condition each would wait for the last)
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
-                                const float a = acc[c * 16 + j], b = acc[c * 16 + 8 + j];
+                                const float a = acc[at + j], b = at + 8 + j < H * kCols ? acc[at + 8 + j] : 0.f;
                                 const float theirs = __shfl_xor_sync(0xffffffffu, up_row ? a : b, 16);
                                 const float g = up_row ? theirs : a, u = up_row ? b : theirs;
                                 // (With the compiler's division, which has a branch, the eight came one after the other: 1500 clocks per 16
@@ -614,10 +819,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(NC), 1)
                                 y[j] = silu(g) * u;
                             }
                             if (up_row) out += 8 * pj.ldy;
-                            const int live = valid ? p.m - mc - (up_row ? 8 : 0) : 0;
-#pragma unroll
-                            for (int j = 0; j < 8; ++j, out += pj.ldy)
-                                if (j < live) store_out(out, y[j]);
+                            store_rows(out, pj.ldy, y, valid ? rows - (up_row ? 8 : 0) : 0, p.pair_stores, lane);
                         }
                     }
                 }
@@ -682,7 +884,7 @@ bool encode_gemm_x(CUtensorMap* map, const __half* x, long long m, long long k, 
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int NC, typename OutT>
+template <int H, int C, typename OutT, bool kSwiglu>
 cudaError_t gemm_configure_and_launch(const GemmParams& p, dim3 grid, cudaStream_t stream) {
     static bool configured[64];
     static std::mutex mu;
@@ -695,24 +897,33 @@ cudaError_t gemm_configure_and_launch(const GemmParams& p, dim3 grid, cudaStream
         if (!configured[dev]) {
             // the register re-split draws on what the block was launched with: a request above that would wait forever
             cudaFuncAttributes a;
-            e = cudaFuncGetAttributes(&a, w4a16_gemm_kernel<NC, OutT>);
+            e = cudaFuncGetAttributes(&a, w4a16_gemm_kernel<H, C, OutT, kSwiglu>);
             if (e != cudaSuccess) return e;
-            if (a.numRegs * gemm_threads(NC) < gemm_split_regs(NC)) return cudaErrorLaunchOutOfResources;
-            e = cudaFuncSetAttribute(w4a16_gemm_kernel<NC, OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemBytes);
+            if (a.numRegs * gemm_threads(H, C) < gemm_split_regs(H, C)) return cudaErrorLaunchOutOfResources;
+            e = cudaFuncSetAttribute(w4a16_gemm_kernel<H, C, OutT, kSwiglu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemBytes);
             if (e != cudaSuccess) return e;
             configured[dev] = true;
         }
     }
-    return launch_pdl(w4a16_gemm_kernel<NC, OutT>, grid, dim3(gemm_threads(NC)), kGemmSmemBytes, stream, p);
+    return launch_pdl(w4a16_gemm_kernel<H, C, OutT, kSwiglu>, grid, dim3(gemm_threads(H, C)), kGemmSmemBytes, stream, p);
 }
 
-template <typename OutT>
+template <typename OutT, bool kSwiglu>
 cudaError_t gemm_configure_and_launch(const GemmParams& p, dim3 grid, cudaStream_t stream) {
-    switch ((p.tile_m + 63) / 64) {
-        case 1: return gemm_configure_and_launch<1, OutT>(p, grid, stream);
-        case 2: return gemm_configure_and_launch<2, OutT>(p, grid, stream);
-        case 3: return gemm_configure_and_launch<3, OutT>(p, grid, stream);
-        default: return gemm_configure_and_launch<4, OutT>(p, grid, stream);
+    switch (p.tile_m) {
+        case 48: return gemm_configure_and_launch<1, 3, OutT, kSwiglu>(p, grid, stream);
+        case 64: return gemm_configure_and_launch<1, 4, OutT, kSwiglu>(p, grid, stream);
+        case 80: return gemm_configure_and_launch<1, 5, OutT, kSwiglu>(p, grid, stream);
+        case 96: return gemm_configure_and_launch<1, 6, OutT, kSwiglu>(p, grid, stream);
+        case 112: return gemm_configure_and_launch<1, 7, OutT, kSwiglu>(p, grid, stream);
+        case 128: return gemm_configure_and_launch<1, 8, OutT, kSwiglu>(p, grid, stream);
+        case 144: return gemm_configure_and_launch<1, 9, OutT, kSwiglu>(p, grid, stream);
+        case 160: return gemm_configure_and_launch<1, 10, OutT, kSwiglu>(p, grid, stream);
+        case 176: return gemm_configure_and_launch<1, 11, OutT, kSwiglu>(p, grid, stream);
+        case 192: return gemm_configure_and_launch<1, 12, OutT, kSwiglu>(p, grid, stream);
+        case 224: return gemm_configure_and_launch<2, 7, OutT, kSwiglu>(p, grid, stream);
+        case 256: return gemm_configure_and_launch<2, 8, OutT, kSwiglu>(p, grid, stream);
+        default: return cudaErrorInvalidValue;  // (33 rows and more, in the steps of gemm_launch: none)
     }
 }
 
@@ -781,17 +992,21 @@ int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num,
                 long long k, int* status, long long wait_limit, int x_stage_limit, int num_sms, float* partials, int* counters) {
     GemmParams p;
     memset(&p, 0, sizeof(p));
-    // rows per tile: as few tiles as 256 rows allow, evenly filled, in steps of 32 (a fold thread reads 16 columns at a time)
+    // rows per tile: as few tiles as 256 rows allow, evenly filled, in steps of what the accumulator tiles' halves need
     p.m_tiles = static_cast<int>((m + kGemmTileM - 1) / kGemmTileM);
-    p.tile_m = static_cast<int>(((m + p.m_tiles - 1) / p.m_tiles + 31) / 32 * 32);
-    p.w_slots = gemm_w_slots(p.tile_m);
+    const int rows = static_cast<int>((m + p.m_tiles - 1) / p.m_tiles), step = 16 * gemm_halves(rows);
+    p.tile_m = (rows + step - 1) / step * step;
     p.groups = static_cast<int>(k / 128);
+    // (two or three groups: summed in turn, with the products of the second thread's first group rounded by themselves, the error against 64
+    // bits is a tenth larger than in sequence; from five groups on it is smaller, 0.91 to 0.99 of it)
+    if (p.groups < 5 && gemm_fold_in_turn(1, p.tile_m / 16)) p.tile_m = 96;
     long long tiles = 0;
     if (swiglu) {
         if (!encode_gemm_w(&p.w_map[0], proj[0].w, proj[0].n, k, 64) || !encode_gemm_w(&p.w_map[1], proj[1].w, proj[1].n, k, 64)) return -2;
         p.proj[0].scales[1] = static_cast<const __half*>(proj[1].scales);
     }
     p.num_proj = swiglu ? 1 : num;
+    p.pair_stores = out_f32 ? 0 : 1;
     p.scales_vec = p.groups % 8 == 0;  // (one flag a launch: read for every projection it cost the kernel 1 to 2 %)
     for (int i = 0; i < p.num_proj; ++i) {
         const TcProj& a = proj[i];
@@ -802,6 +1017,7 @@ int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num,
         p.proj[i].ldy = a.ldy > 0 ? a.ldy : a.n;
         p.proj[i].n = static_cast<int>(a.n);
         if (((reinterpret_cast<uintptr_t>(a.scales) | reinterpret_cast<uintptr_t>(p.proj[i].scales[1])) & 15) != 0) p.scales_vec = 0;
+        if ((reinterpret_cast<uintptr_t>(a.y) & 3) || (p.proj[i].ldy & 1) || (a.n & 1)) p.pair_stores = 0;
         p.proj[i].tile0 = static_cast<int>(tiles);
         const int rows = swiglu ? kGemmTileN : 2 * kGemmTileN;  // of a pair
         tiles += (a.n + rows - 1) / rows * p.m_tiles;
@@ -811,7 +1027,6 @@ int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num,
     if (!encode_gemm_x(&p.x_map, static_cast<const __half*>(x), m, k, p.tile_m)) return -2;
     p.m = static_cast<int>(m);
     p.units = deal.units;
-    p.swiglu = swiglu ? 1 : 0;
     p.wait_limit = wait_limit;
     p.x_stage_limit = x_stage_limit;
     p.status = status;
@@ -820,7 +1035,10 @@ int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num,
     p.whole_tiles = deal.whole_tiles ? 1 : 0;
     p.pairs = static_cast<int>(deal.pairs);
     const dim3 grid(static_cast<unsigned>(2 * deal.pairs));
-    const cudaError_t e = out_f32 ? gemm_configure_and_launch<float>(p, grid, stream) : gemm_configure_and_launch<__half>(p, grid, stream);
+    if (swiglu && out_f32) return -2;  // (fp16 activations give fp16 results there)
+    const cudaError_t e = swiglu    ? gemm_configure_and_launch<__half, true>(p, grid, stream)
+                          : out_f32 ? gemm_configure_and_launch<float, false>(p, grid, stream)
+                                    : gemm_configure_and_launch<__half, false>(p, grid, stream);
     return e == cudaSuccess ? 0 : -1;
 }
 
