@@ -39,7 +39,7 @@ int tc_x_stage_limit();     // test hook of tc_set_wait_hooks: first activation 
 // Dense GEMM for more than 32 activation rows (prefill chunks) on tcgen05, both operands from shared memory
 // (w4a16_gemm.cu).  One launch for all projections that share X; gate and up of the fused MLP are one pair.
 bool gemm_eligible(const void* x, const TcProj* proj, int num, bool swiglu, long long m, long long k, int group_size);
-// `partials` (gemm_partial_bytes) and `counters` (one zeroed int per SM, left zeroed): scratch for tiles whose K range
+// `partials` (gemm_partial_bytes) and `counters` (eight zeroed ints per SM, left zeroed): scratch for tiles whose K range
 // is cut between CTAs (partials null: tiles are not cut).
 size_t gemm_partial_bytes(int num_sms);
 int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num, bool swiglu, bool out_f32, long long m,

@@ -72,6 +72,7 @@ constexpr int gemm_threads(int h, int c) { return kGemmThreads + (gemm_unpack_se
 constexpr int kXSlotsMax = 8, kWSlotsMax = 12, kASlotsMax = 4;
 constexpr int kWSlotBytes = kGemmTileN * 64;                    // 8 KB of packed weights: one group
 constexpr int kGemmMaxProj = 4;
+constexpr long long kOthersWait = 3000;  // clocks
 // Register split of the launch's 512 x 128, or 640 x 96: the fold keeps up to 128, or 96, sums per thread.
 constexpr int kCtrlRegs = 32, kUnpackRegs = 64;
 constexpr int gemm_fold_regs(int h, int c) { return gemm_unpack_sets(h, c) == 2 ? 160 : 208; }
@@ -87,7 +88,6 @@ struct GemmCtrl {
     uint64_t a_full[kASlotsMax];  // the pair's unpacking warps
     uint64_t d_empty[kDBufsMax];
     uint32_t tmem_base;
-    int last_arrival;
     WaitState ws;
 };
 
@@ -139,12 +139,13 @@ struct GemmParams {
     int scales_vec;  // every row of scales starts on a 16-byte boundary
     long long units;     // tiles * groups
     int pairs;           // CTA pairs of the launch
-    int whole_tiles;     // cut between tiles only
+    long long deal_quot; // what is dealt to each pair: whole tiles (deal_size groups) or single groups, the remainder spread evenly
+    int deal_rem, deal_size;
     long long wait_limit;
     int* status;
     int x_stage_limit;  // test hook: activation stages (of a CTA) from this index on are never requested (-1: off)
     float* partials;    // [CTA][2][column / 4][fold thread][4]: fp32 sums of the tiles a CTA holds a part of
-    int* counters;      // [CTA]: groups of the tile that starts in that pair's range and ends behind it, added up so far
+    int* counters;      // [CTA][fold warp]: groups of the tile that starts in that pair's range and ends behind it, added up so far
 };
 
 // (This and the commit are executed by a whole warp under uniform control flow; the lane with `issue` set issues.  Inside `if (leader)`
@@ -272,21 +273,8 @@ __device__ __forceinline__ void shift_scales(uint4& q) {
     q.w >>= 16;
 }
 
-// First unit of pair c: units cut evenly, or whole tiles only.
-__device__ __forceinline__ long long unit_begin(const GemmParams& p, long long c) {
-    if (p.whole_tiles) {
-        const long long tiles = p.units / p.groups;
-        return c * tiles / p.pairs * p.groups;
-    }
-    return c * p.units / p.pairs;
-}
-// The pair whose range holds unit u.
-__device__ __forceinline__ int unit_owner(const GemmParams& p, long long u) {
-    int c = static_cast<int>(u * p.pairs / p.units);
-    while (c + 1 < p.pairs && unit_begin(p, c + 1) <= u) ++c;
-    while (c > 0 && unit_begin(p, c) > u) --c;
-    return c;
-}
+// First unit of pair c: floor(c * tiles / pairs) tiles on, or floor(c * units / pairs) units (the division by host, but for its remainder).
+__device__ __forceinline__ long long unit_begin(const GemmParams& p, int c) { return (c * p.deal_quot + c * p.deal_rem / p.pairs) * p.deal_size; }
 __device__ __forceinline__ int proj_of_tile(const GemmParams& p, int tile) {
     int i = 0;
     while (i + 1 < p.num_proj && tile >= p.proj[i + 1].tile0) ++i;
@@ -323,6 +311,17 @@ __device__ __forceinline__ void fma_pair(float& acc0, float& acc1, uint32_t d0, 
         "}"
         : "+f"(acc0), "+f"(acc1)
         : "r"(d0), "r"(d1), "f"(sc));
+}
+__device__ __forceinline__ int load_acquire(const int* p) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void add4(float* acc, const float4& t) {
+    acc[0] += t.x;
+    acc[1] += t.y;
+    acc[2] += t.z;
+    acc[3] += t.w;
 }
 // f(Step<0>()) ... f(Step<N - 1>()): a loop whose index is a constant.
 template <int I>
@@ -380,7 +379,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(H, C), 
 
     // this pair's units (tile, 128-k group), tile-major; ring slots and phases count from its first unit
     const int pair = static_cast<int>(blockIdx.x >> 1);
-    const long long u0 = unit_begin(p, pair), u1 = unit_begin(p, static_cast<long long>(pair) + 1);
+    const long long u0 = unit_begin(p, pair), u1 = unit_begin(p, pair + 1);
     const int U = static_cast<int>(u1 - u0);
     const int first_tile = static_cast<int>(u0 / p.groups), first_group = static_cast<int>(u0 - static_cast<long long>(first_tile) * p.groups);
 
@@ -705,87 +704,96 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(H, C), 
             }
 
             // ------------------------------------------------------------ a straddling tile: the last CTA to arrive finishes it
-            int c_first = 0, c_last = 0;
             const bool split = seg_begin > 0 || seg_end < p.groups;
+            bool last = true;
             if (split) {
                 const long long tu = static_cast<long long>(tile) * p.groups;
-                c_first = unit_owner(p, tu);
-                c_last = unit_owner(p, tu + p.groups - 1);
+                int c_first = pair, c_last = pair;
+                if (seg_begin > 0)
+                    do --c_first;
+                    while (unit_begin(p, c_first) > tu);
+                if (seg_end < p.groups)
+                    do ++c_last;
+                    while (unit_begin(p, c_last + 1) < tu + p.groups);
                 const size_t slot_floats = static_cast<size_t>(kGemmTileN) * kGemmTileM;
-                int* counter = p.counters + c_first * 2 + rank;
+                // (every fold warp exchanges its own rows and columns with the same warp of the others, without the CTA's other warps)
+                int* counter = p.counters + (c_first * 2 + static_cast<int>(rank)) * (kGemmFoldThreads / 32) + warp;
                 const int n = seg_end - seg_begin;
-                // A tile cut once: the second pair met its part at the start of its range, long ago.  If it has indeed arrived, this
-                // one's sums stay in registers (writing them, the fence behind it and reading them back took 3 us of 42 at N = 5120,
-                // M = 512).
-                bool kept = false;
-                if (pair == c_first && c_last == c_first + 1) {
-                    if (tid == 0) {
-                        const bool last = atomicAdd(counter, 0) + n == p.groups;
-                        if (last) *counter = 0;  // as the next launch expects it
-                        ctrl->last_arrival = last ? 1 : 0;
-                        __threadfence();
-                    }
-                    fold_barrier();
-                    kept = ctrl->last_arrival != 0;
-                    fold_barrier();
+                // The pair in whose range a tile starts comes to it last of all it does, after an exchange more than the pairs with one part
+                // only: the others have mostly arrived or are about to.  If they have, its sums stay in registers (writing them, with the
+                // fence behind it, takes 3.5 us at 256 rows: worth a wait of half of that).
+                last = false;
+                if (seg_begin == 0) {
+                    // (the whole warp asks: a loop of one lane's own costs the epilogue registers)
+                    const long long t0 = clock64();
+                    int have;
+                    do have = load_acquire(counter);
+                    while (__any_sync(0xffffffffu, have + n != p.groups && clock64() - t0 < kOthersWait));
+                    last = __all_sync(0xffffffffu, have + n == p.groups);
+                    if (last && lane == 0) *counter = 0;  // as the next launch expects it
                 }
-                if (!kept) {
+                if (!last) {
                     float4* mine = reinterpret_cast<float4*>(p.partials + (static_cast<size_t>(blockIdx.x) * 2 + (seg_begin > 0 ? 0 : 1)) * slot_floats) + tid;
 #pragma unroll
                     for (int j = 0; j < H * kCols; j += 4)
                         __stcg(mine + j / 4 * kGemmFoldThreads, make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]));
                     __threadfence();
-                    fold_barrier();
-                    if (tid == 0) {
-                        const bool last = atomicAdd(counter, n) + n == p.groups;
-                        if (last) *counter = 0;
-                        ctrl->last_arrival = last ? 1 : 0;
-                        __threadfence();
+                    __syncwarp();
+                    int have = 0;
+                    if (lane == 0) {
+                        have = atomicAdd(counter, n);
+                        if (have + n == p.groups) *counter = 0;
                     }
-                    fold_barrier();
+                    last = __any_sync(0xffffffffu, lane == 0 && have + n == p.groups);
                 }
-                if (ctrl->last_arrival) {
-                    // The parts are added in pair order, whoever is last; this pair's own comes back from memory too, which leaves
-                    // the registers free to request a whole part, or half of one, at once.  (Sixteen columns at a time, each a
-                    // trip to L2, cost 8 us a part: N = 5120, M = 256 took 43 us and takes 34.)
+                if (last) {
+                    // The parts are added in pair order, whoever is last: those in front of this pair's own, it, those behind.
                     __threadfence();
                     const float* base = p.partials + static_cast<size_t>(rank) * 2 * slot_floats + tid * 4;
-                    if (!kept) {
-                        // a contributor's part of this tile: slot 1 if the tile starts in its range, else slot 0
-                        const float4* src = reinterpret_cast<const float4*>(base + static_cast<size_t>(c_first) * 4 * slot_floats + slot_floats);
+                    auto part = [&](int o) {  // a contributor's part of this tile: slot 1 if the tile starts in its range, else slot 0
+                        return reinterpret_cast<const float4*>(base + static_cast<size_t>(o) * 4 * slot_floats + (o == c_first ? slot_floats : 0));
+                    };
+                    constexpr int kParts = H * kCols / 4, kBatch = 12;
+                    if (c_first < pair) {
 #pragma unroll
-                        for (int j = 0; j < H * kCols; j += 4) {
-                            const float4 t = __ldcg(src + j / 4 * kGemmFoldThreads);
-                            acc[j] = t.x;
-                            acc[j + 1] = t.y;
-                            acc[j + 2] = t.z;
-                            acc[j + 3] = t.w;
-                        }
-                    }
-                    constexpr int kBatch = 12;
-#pragma unroll 1
-                    for (int o = c_first + 1; o <= c_last; ++o) {
-                        const float4* src = reinterpret_cast<const float4*>(base + static_cast<size_t>(o) * 4 * slot_floats);
-#pragma unroll
-                        for (int c = 0; c < H * kCols / 4; c += kBatch) {
+                        for (int c = 0; c < kParts; c += kBatch) {
                             float4 t[kBatch];
 #pragma unroll
                             for (int j = 0; j < kBatch; ++j)
-                                if (c + j < H * kCols / 4) t[j] = __ldcg(src + (c + j) * kGemmFoldThreads);
+                                if (c + j < kParts) t[j] = __ldcg(part(c_first) + (c + j) * kGemmFoldThreads);
+#pragma unroll 1
+                            for (int o = c_first + 1; o < pair; ++o) {
 #pragma unroll
-                            for (int j = 0; j < kBatch; ++j) {
-                                if (c + j >= H * kCols / 4) continue;
-                                float* to = acc + (c + j) * 4;
-                                to[0] += t[j].x;
-                                to[1] += t[j].y;
-                                to[2] += t[j].z;
-                                to[3] += t[j].w;
+                                for (int j = 0; j < kBatch; ++j)
+                                    if (c + j < kParts) {
+                                        const float4 u = __ldcg(part(o) + (c + j) * kGemmFoldThreads);
+                                        t[j].x += u.x;
+                                        t[j].y += u.y;
+                                        t[j].z += u.z;
+                                        t[j].w += u.w;
+                                    }
                             }
+#pragma unroll
+                            for (int j = 0; j < kBatch; ++j)
+                                if (c + j < kParts) add4(acc + (c + j) * 4, t[j]);
+                        }
+                    }
+#pragma unroll 1
+                    for (int o = pair + 1; o <= c_last; ++o) {
+#pragma unroll
+                        for (int c = 0; c < kParts; c += kBatch) {
+                            float4 t[kBatch];
+#pragma unroll
+                            for (int j = 0; j < kBatch; ++j)
+                                if (c + j < kParts) t[j] = __ldcg(part(o) + (c + j) * kGemmFoldThreads);
+#pragma unroll
+                            for (int j = 0; j < kBatch; ++j)
+                                if (c + j < kParts) add4(acc + (c + j) * 4, t[j]);
                         }
                     }
                 }
             }
-            if (!split || ctrl->last_arrival) {
+            if (last) {
                 const float bias = (valid && pj.bias && !kSwiglu) ? pj.bias[row] : 0.f;
 #pragma unroll
                 for (int c = 0; c < H * ((kCols + 15) / 16); ++c) {
@@ -943,8 +951,9 @@ bool gemm_eligible(const void* x, const TcProj* proj, int num, bool swiglu, long
 namespace {
 
 // How a launch's tiles are dealt to the CTA pairs.  One pair per two SMs.  Cutting tiles evens the pairs' work out and costs the
-// exchange of partial sums, about as much as kCutCost groups; a small problem takes fewer pairs (below eight groups each, the
-// pipeline's fill dominates).
+// exchange of partial sums, about as much as kCutCost groups (with 12, 8 or 4 in its place 14336 x 5120 is cut up to 256 rows and takes
+// 35.7 -> 37 to 40 us there, and nothing else gains; of the exchange's 12 us at 512 rows, 4 are writing the part met first, 4 reading
+// the others' two, 2 the outputs); a small problem takes fewer pairs (below eight groups each, the pipeline's fill dominates).
 constexpr long long kCutCost = 16;
 struct GemmDeal {
     long long tiles, units, pairs;
@@ -1032,8 +1041,11 @@ int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num,
     p.status = status;
     p.partials = partials;
     p.counters = counters;
-    p.whole_tiles = deal.whole_tiles ? 1 : 0;
     p.pairs = static_cast<int>(deal.pairs);
+    const long long dealt = deal.whole_tiles ? deal.tiles : deal.units;
+    p.deal_quot = dealt / deal.pairs;
+    p.deal_rem = static_cast<int>(dealt % deal.pairs);
+    p.deal_size = deal.whole_tiles ? p.groups : 1;
     const dim3 grid(static_cast<unsigned>(2 * deal.pairs));
     if (swiglu && out_f32) return -2;  // (fp16 activations give fp16 results there)
     const cudaError_t e = swiglu    ? gemm_configure_and_launch<__half, true>(p, grid, stream)
