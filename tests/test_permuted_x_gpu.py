@@ -1,0 +1,27 @@
+"""Long launches of more than 16 activation rows have X written in the unpack's order by a small launch in front of them; the allocation-free
+entry point never has.  The sums are the same in the same order, so the two agree to the bit on either side of the rule's lines."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [16, 17, 24, 31, 32])
+@pytest.mark.parametrize("K,N", [
+    (12160, 38144),   # 48 stages per CTA (the last of one group), 149 tiles on 148 SMs
+    (12032, 38144),   # 47
+    (12288, 37888),   # 148 tiles: none is cut
+    (5120, 151936),   # an LM head
+])
+def test_same_bits_as_without(cuda, M, K, N):
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    w = torch.randint(0, 256, (N, K // 2), generator=g, device="cuda", dtype=torch.uint8)
+    s = torch.rand((N, K // 128), generator=g, device="cuda").mul_(0.01).half()
+    x = torch.randn((M, K), generator=g, device="cuda").half()
+    got, want = (torch.full((M, N), float("nan"), device="cuda", dtype=torch.float16) for _ in range(2))
+    for _ in range(2):  # (twice: the second call's copy of X follows the first call's reads of it)
+        assert cuda.linear_int4(got, x, w, s, None, M, N, K) == 0
+    assert cuda.linear_int4_noalloc(want, x, w, s, None, M, N, K) == 0
+    torch.cuda.synchronize()
+    assert cuda.device_status(0) == 0
+    assert torch.equal(got, want) and not torch.isnan(got).any()

@@ -42,6 +42,7 @@ struct DeviceCtx {
     bool ready = false;
     int num_sms = 0;
     float* workspace = nullptr;   // split-K partials
+    void* x_scratch = nullptr;    // activations in the decode kernel's order, of launches that use `workspace` too
     int* counters = nullptr;      // tile arrival counters and the synchronous acceptance's, zero between launches
     int* status = nullptr;        // device status word
     void* sampling = nullptr;     // (row, chunk) partials
@@ -83,6 +84,7 @@ int get_ctx(DeviceCtx** out) {
             c.num_sms = prop.multiProcessorCount;
             const size_t ws = xb::tc_workspace_bytes(c.num_sms);
             if ((e = cudaMalloc(&c.workspace, ws)) != cudaSuccess) return fail_cuda(e);
+            if ((e = cudaMalloc(&c.x_scratch, xb::tc_x_scratch_bytes())) != cudaSuccess) return fail_cuda(e);
             if ((e = cudaMalloc(&c.counters, (kCounterCapacity + 1) * sizeof(int))) != cudaSuccess) return fail_cuda(e);
             if ((e = cudaMalloc(&c.status, sizeof(int))) != cudaSuccess) return fail_cuda(e);
             if ((e = cudaMalloc(&c.sampling, kSamplingScratchBytes)) != cudaSuccess) return fail_cuda(e);
@@ -149,8 +151,10 @@ int run_linear(xinfer_stream_t s, const void* x, xb::ActType in, bool out_f32, c
     const bool want_tc = (c->forced_path != 2) && in == xb::ActType::F16 &&
                          xb::tc_eligible(x, proj, num, swiglu, m, k, group_size);
     if (want_tc) {
-        int r = xb::tc_launch(stream, x, proj, num, swiglu, out_f32, m, k, c->num_sms, c->workspace, c->counters,
-                              kCounterCapacity, c->status);
+        const bool permuted = xb::tc_wants_permuted_x(proj, num, swiglu, m, k, c->num_sms);
+        if (permuted && xb::tc_permute_x(stream, x, c->x_scratch, m, k) != 0) return fail_cuda(cudaGetLastError());
+        int r = xb::tc_launch(stream, permuted ? c->x_scratch : x, proj, num, swiglu, out_f32, m, k, c->num_sms, c->workspace, c->counters,
+                              kCounterCapacity, c->status, nullptr, permuted ? xb::kTcXPermuted : 0);
         if (r == 0) { g_last_path = 1; return XINFER_OK; }
         if (r == -1) return fail_cuda(cudaGetLastError());
         // r < -1: the problem could not be described to the tensor-core kernel; use CUDA cores

@@ -28,6 +28,10 @@ struct TcProj {
 
 // ---- tcgen05 path (w4a16_tc.cu): fp16 activations, 1 <= m <= 32, k % 128 == 0
 size_t tc_workspace_bytes(int ctas);
+// X in the order kTcXPermuted names, written once in front of a launch that is worth it (tc_x_scratch_bytes of scratch).
+size_t tc_x_scratch_bytes();
+bool tc_wants_permuted_x(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms);
+int tc_permute_x(cudaStream_t stream, const void* x, void* scratch, long long m, long long k);
 // Test hooks for the bounded device-side waits: their clock limit (<= 0 restores the one-second default)
 // and the first activation stage that the producer never requests (-1: all are requested).
 void tc_set_wait_hooks(long long limit_clocks, int withhold_x_from_stage);

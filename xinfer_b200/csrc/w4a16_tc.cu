@@ -44,6 +44,7 @@
 #include <new>
 #include <vector>
 
+#include "launch.cuh"
 #include "ptx_sm100.cuh"
 #include "silu.cuh"
 #include "w4a16.h"
@@ -1270,6 +1271,41 @@ bool tc_eligible(const void* x, const TcProj* proj, int num, bool swiglu, long l
         if (reinterpret_cast<uintptr_t>(proj[i].w) & 15) return false;
     }
     return true;
+}
+
+namespace {
+constexpr long long kXScratchK = 32768;      // longest row that has room in the scratch
+constexpr long long kPermuteStages = 48;     // stages of 256 k per CTA
+// X with every block of eight features in the order the int4 unpack yields them, (0,4,1,5,2,6,3,7): sixteen bytes a thread.
+__global__ void __launch_bounds__(256) permute_x_kernel(const uint4* x, uint4* out, int blocks) {
+    griddep_prologue();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= blocks) return;
+    const uint4 v = __ldg(x + i);
+    out[i] = make_uint4(prmt(v.x, v.z, 0x5410u), prmt(v.x, v.z, 0x7632u), prmt(v.y, v.w, 0x5410u), prmt(v.y, v.w, 0x7632u));
+}
+}  // namespace
+
+size_t tc_x_scratch_bytes() { return static_cast<size_t>(32) * kXScratchK * sizeof(__half); }
+
+// Whether a launch is worth a small one in front of it that writes X in the unpack's order once, instead of one warp of every CTA doing so
+// for each of its stages.  With more than 16 rows that warp is the pace of a stage (1900 clocks against 1700), but the small launch costs
+// 1.5 us: at 32 rows 80 stages per CTA (5120 x 151936) take 100.9 -> 97.8 us, 21 (5120 x 40000) 35.6 -> 36.1, 16 (2560 x 60000)
+// 30.8 -> 32.1; at 16 rows there is nothing to gain (88.7 both).  The line lies above the 33 stages where the two meet.
+bool tc_wants_permuted_x(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms) {
+    if (m <= 16 || k > kXScratchK) return false;
+    long long tiles = 0;
+    const int rows = swiglu ? kHalfRows : kTileRows;
+    for (int i = 0; i < (swiglu ? 1 : num); ++i) tiles += (proj[i].n + rows - 1) / rows;
+    // (cut tiles only: those launches use the device's scratch buffer already, others may run beside each other on several streams)
+    if (tiles < num_sms || tiles % num_sms == 0) return false;
+    return tiles * ((k / 128 + 1) / 2) >= kPermuteStages * num_sms;
+}
+
+int tc_permute_x(cudaStream_t stream, const void* x, void* scratch, long long m, long long k) {
+    const int blocks = static_cast<int>(m * k / 8);
+    return launch_pdl(permute_x_kernel, dim3((blocks + 255) / 256), dim3(256), 0, stream, static_cast<const uint4*>(x), static_cast<uint4*>(scratch),
+                      blocks) == cudaSuccess ? 0 : -1;
 }
 
 // Launches the tensor-core kernel.  `scratch` holds tc_workspace_bytes(ctas) bytes of partials followed by
