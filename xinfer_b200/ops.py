@@ -157,23 +157,22 @@ def speculative_accept_reject(draft_tokens: Sequence[int], num_draft_tokens: int
     std::logic_error.
     """
     n = int(num_draft_tokens)
-    toks = (C.c_int64 * max(n, 1))(*[int(t) for t in draft_tokens][:n]) if draft_tokens is not None else None
-    probs = (C.c_float * max(n, 1))(*[float(p) for p in draft_probs][:n]) if draft_probs is not None else None
-    unif = (C.c_float * max(n, 1))(*[float(u) for u in rand_uniform][:n]) if rand_uniform is not None else None
+    # (arrays go into a void* argument as they are; C.cast and a comprehension per array took half of this function's 8 us)
+    toks = (C.c_int64 * max(n, 1))(*[*map(int, draft_tokens)][:n]) if draft_tokens is not None else None
+    probs = (C.c_float * max(n, 1))(*[*map(float, draft_probs)][:n]) if draft_probs is not None else None
+    unif = (C.c_float * max(n, 1))(*[*map(float, rand_uniform)][:n]) if rand_uniform is not None else None
     res = AcceptResult()
-    check(lib().xinfer_speculative_accept_reject(
-        _stream(), C.cast(toks, C.c_void_p) if toks is not None else None, n, _ptr(target_logits), vocab_size,
-        C.cast(probs, C.c_void_p) if probs is not None else None,
-        C.cast(unif, C.c_void_p) if unif is not None else None, C.byref(res)), "speculative_accept_reject")
+    check(lib().xinfer_speculative_accept_reject(_stream(), toks, n, _ptr(target_logits), vocab_size, probs, unif, C.byref(res)),
+          "speculative_accept_reject")
     return {
-        "accepted_tokens": [int(res.accepted_tokens[i]) for i in range(res.num_accepted)],
-        "bonus_or_resampled_token": int(res.bonus_or_resampled_token),
+        "accepted_tokens": res.accepted_tokens[:res.num_accepted],
+        "bonus_or_resampled_token": res.bonus_or_resampled_token,
         "has_rejected_token": bool(res.has_rejected_token),
-        "rejected_token": int(res.rejected_token),
-        "num_accepted": int(res.num_accepted),
-        "num_rejected": int(res.num_rejected),
-        "num_resampled": int(res.num_resampled),
-        "num_remaining": int(res.num_remaining),
+        "rejected_token": res.rejected_token,
+        "num_accepted": res.num_accepted,
+        "num_rejected": res.num_rejected,
+        "num_resampled": res.num_resampled,
+        "num_remaining": res.num_remaining,
     }
 
 
