@@ -367,6 +367,20 @@ __device__ __forceinline__ uint32_t hfma2_u32(uint32_t a, uint32_t b, uint32_t c
     asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
+// acc0 += d0 * sc, acc1 += d1 * sc: two roundings each as fmaf has, one instruction.  (Volatile: it stays where it stands between the reads.)
+__device__ __forceinline__ void fma_pair(float& acc0, float& acc1, uint32_t d0, uint32_t d1, float sc) {
+    asm volatile(
+        "{\n\t"
+        ".reg .b64 a, b, c;\n\t"
+        "mov.b64 a, {%0, %1};\n\t"
+        "mov.b64 b, {%2, %3};\n\t"
+        "mov.b64 c, {%4, %4};\n\t"
+        "fma.rn.f32x2 a, b, c, a;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t"
+        "}"
+        : "+f"(acc0), "+f"(acc1)
+        : "r"(d0), "r"(d1), "f"(sc));
+}
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     uint32_t d;
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));

@@ -298,20 +298,6 @@ __device__ __forceinline__ void dequant_word_in_order(uint32_t w, uint32_t* q) {
             : "r"(w), "r"(0x4040u | static_cast<uint32_t>(j * 0x101)), "r"(0x54806408u));
 }
 
-// acc0 += d0 * sc, acc1 += d1 * sc: two roundings each as fmaf has, one instruction.  (Volatile: it stays where it stands between the reads.)
-__device__ __forceinline__ void fma_pair(float& acc0, float& acc1, uint32_t d0, uint32_t d1, float sc) {
-    asm volatile(
-        "{\n\t"
-        ".reg .b64 a, b, c;\n\t"
-        "mov.b64 a, {%0, %1};\n\t"
-        "mov.b64 b, {%2, %3};\n\t"
-        "mov.b64 c, {%4, %4};\n\t"
-        "fma.rn.f32x2 a, b, c, a;\n\t"
-        "mov.b64 {%0, %1}, a;\n\t"
-        "}"
-        : "+f"(acc0), "+f"(acc1)
-        : "r"(d0), "r"(d1), "f"(sc));
-}
 __device__ __forceinline__ int load_acquire(const int* p) {
     int v;
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
