@@ -78,7 +78,7 @@ __device__ __forceinline__ float block_sum(float v, float* smem) {
 //   as half(x + delta), also written back to x                (residual add, then norm)
 //   from row `tokens[row]` of the bf16 table, also written to x when x is given   (embedding, then norm)
 // `out` may have a wider row (ld_out) and a column offset so that two norms can fill one concatenated row.
-// One or two such jobs per launch (blockIdx.y).  Bound by latency at a step's 1 to 32 rows (2.6 us a launch): what counts
+// One or two such jobs per launch (blockIdx.y).  Bound by latency at a step's 1 to 32 rows (2.3 us a launch): what counts
 // is the number of launches and of dependent trips to memory.  An embedding of its own, 2 bytes per load, took 10 us.
 struct NormJob {
     __half* out;
@@ -106,12 +106,19 @@ __device__ __forceinline__ const uint16_t* norm_tokens(const NormJob& job, long 
 }
 __device__ __forceinline__ __half bf16_to_half(uint32_t bits) { return __float2half_rn(__uint_as_float(bits << 16)); }
 
-// TABLE: some job of the launch reads the embedding table
-template <bool TABLE>
-__global__ void __launch_bounds__(256) rmsnorm_kernel(const __grid_constant__ NormJob job0, const __grid_constant__ NormJob job1,
+constexpr int kNormWideRows = 148, kNormNarrow = 2048;
+// TABLE: some job of the launch reads the embedding table.  VECS: most 8-element vectors of a thread: four of 256 threads (and the path for
+// rows that are not vectors), or one of up to 1024.
+// One vector a thread is the shorter way through a row, which is what counts as long as every row has an SM to itself, and where 256
+// threads would not all have one: 5120 features with the residual added, 1 row 2.30 -> 2.03 us, 32 rows 2.57 -> 2.30, 148 rows 2.58 -> 2.31;
+// 1024 features, 2796 rows 8.9 -> 4.9.  With more rows the 640 threads of a wide row leave an SM three rows at a time, and four vectors a
+// thread are better: 1024 x 5120 5.93 us against 6.83 without the addition, 2796 x 5120 12.6 against 15.7 (between 148 and 512 rows
+// either may be, by up to 0.3 us).
+template <bool TABLE, int VECS>
+__global__ void __launch_bounds__(VECS == 1 ? 1024 : 256) rmsnorm_kernel(const __grid_constant__ NormJob job0, const __grid_constant__ NormJob job1,
                                                       long long ld_out, int hidden, float eps, int perm_out) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    __shared__ __align__(16) float red[32];
+    __shared__ __align__(16) float red[32];  // of every warp
     const NormJob& job = TABLE && blockIdx.y ? job1 : job0;
     const bool table = TABLE && job.table;
     const float* w = job.w;
@@ -120,15 +127,15 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __grid_constant__ No
     const __half* dr = job.delta ? job.delta + row * hidden : nullptr;
     __half* orow = job.out + row * ld_out;
     const int nvec = hidden >> 3;
-    const bool vec_ok = (hidden & 7) == 0 && nvec <= 4 * 256 &&
+    const bool vec_ok = (hidden & 7) == 0 && nvec <= VECS * static_cast<int>(blockDim.x) &&
                         ((reinterpret_cast<uintptr_t>(xr) | reinterpret_cast<uintptr_t>(orow) | reinterpret_cast<uintptr_t>(dr) |
                           reinterpret_cast<uintptr_t>(job.table) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
     if (vec_ok) {
         // The norm weights do not depend on the previous kernel in the stream: they are fetched before waiting
         // for it, so that only the activations' latency is left on the critical path.
-        float4 wv[4][2];
+        float4 wv[VECS][2];
 #pragma unroll
-        for (int it = 0; it < 4; ++it) {
+        for (int it = 0; it < VECS; ++it) {
             const int i = threadIdx.x + it * 256;
             if (i < nvec) {
                 wv[it][0] = __ldg(reinterpret_cast<const float4*>(w + i * 8));
@@ -140,9 +147,9 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __grid_constant__ No
         // one pass: each thread keeps its (up to four) 8-element vectors in registers.  Every load goes out before the first
         // value is used and before any store (which the compiler must take for a possible alias of the later loads): with
         // the residual stored in between, each further vector was another trip to memory (2.9 us a launch against 2.5).
-        uint4 v[4], dv[4];
+        uint4 v[VECS], dv[VECS];
 #pragma unroll
-        for (int it = 0; it < 4; ++it) {
+        for (int it = 0; it < VECS; ++it) {
             const int i = threadIdx.x + it * 256;
             if (i < nvec) {
                 if (!table) v[it] = *reinterpret_cast<const uint4*>(xr + i * 8);
@@ -152,7 +159,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __grid_constant__ No
         }
         float ss = 0.f;
 #pragma unroll
-        for (int it = 0; it < 4; ++it) {
+        for (int it = 0; it < VECS; ++it) {
             const int i = threadIdx.x + it * 256;
             if (i < nvec) {
                 __half2* h = reinterpret_cast<__half2*>(&v[it]);
@@ -178,12 +185,17 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __grid_constant__ No
         }
         ss = warp_sum(ss);
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+        if (VECS == 1 && threadIdx.x < 32 && threadIdx.x >= (blockDim.x >> 5)) red[threadIdx.x] = 0.f;
         __syncthreads();
-        const float4 r0 = *reinterpret_cast<const float4*>(red), r1 = *reinterpret_cast<const float4*>(red + 4);
-        const float total = ((r0.x + r1.x) + (r0.z + r1.z)) + ((r0.y + r1.y) + (r0.w + r1.w));
+        float total = 0.f;
+#pragma unroll
+        for (int w = 0; w < (VECS == 1 ? 32 : 8); w += 8) {
+            const float4 r0 = *reinterpret_cast<const float4*>(red + w), r1 = *reinterpret_cast<const float4*>(red + w + 4);
+            total += ((r0.x + r1.x) + (r0.z + r1.z)) + ((r0.y + r1.y) + (r0.w + r1.w));
+        }
         const float r = 1.0f / sqrtf(total / static_cast<float>(hidden) + eps);
 #pragma unroll
-        for (int it = 0; it < 4; ++it) {
+        for (int it = 0; it < VECS; ++it) {
             const int i = threadIdx.x + it * 256;
             if (i < nvec) {
                 if (xr && (dr || table)) *reinterpret_cast<uint4*>(xr + i * 8) = v[it];
@@ -1401,6 +1413,16 @@ __global__ void fill_int_kernel(int* p, int n, int v) {
 
 #define XB_LAUNCH_OK() (cudaGetLastError() == cudaSuccess ? 0 : -1)
 
+namespace {
+template <bool TABLE>
+void launch_norm(cudaStream_t s, dim3 grid, const NormJob& a, const NormJob& b, long long ld_out, int hidden, float eps, int perm_out) {
+    if (hidden % 8 == 0 && hidden <= 8 * 1024 && (static_cast<int>(grid.x) <= kNormWideRows || hidden <= kNormNarrow))
+        launch_pdl(rmsnorm_kernel<TABLE, 1>, grid, dim3((hidden / 8 + 31) / 32 * 32), 0, s, a, b, ld_out, hidden, eps, perm_out);
+    else
+        launch_pdl(rmsnorm_kernel<TABLE, 4>, grid, dim3(256), 0, s, a, b, ld_out, hidden, eps, perm_out);
+}
+}  // namespace
+
 int embed_norm_rows(cudaStream_t s, __half* out, __half* x, const void* table_bf16, const long long* tokens, const float* w, int rows,
                     int hidden, long long vocab, float eps, int perm_out) {
     NormJob j = {};
@@ -1410,7 +1432,7 @@ int embed_norm_rows(cudaStream_t s, __half* out, __half* x, const void* table_bf
     j.table = static_cast<const uint16_t*>(table_bf16);
     j.tokens = tokens;
     j.vocab = vocab;
-    launch_pdl(rmsnorm_kernel<true>, dim3(rows), dim3(256), 0, s, j, j, static_cast<long long>(hidden), hidden, eps, perm_out);
+    launch_norm<true>(s, dim3(rows), j, j, static_cast<long long>(hidden), hidden, eps, perm_out);
     return XB_LAUNCH_OK();
 }
 
@@ -1429,7 +1451,7 @@ int head_input_rows(cudaStream_t s, const HeadInput& h, int rows, int hidden, fl
     p.out = h.cat + hidden;
     p.x = const_cast<__half*>(h.hidden_rows);
     p.w = h.hidden_norm;
-    launch_pdl(rmsnorm_kernel<true>, dim3(rows, 2), dim3(256), 0, s, e, p, 2LL * hidden, hidden, eps, perm_out);
+    launch_norm<true>(s, dim3(rows, 2), e, p, 2LL * hidden, hidden, eps, perm_out);
     return XB_LAUNCH_OK();
 }
 
@@ -1439,7 +1461,7 @@ int rmsnorm_rows(cudaStream_t s, __half* out, long long ld_out, const __half* in
     j.out = out;
     j.x = const_cast<__half*>(in);
     j.w = w;
-    launch_pdl(rmsnorm_kernel<false>, dim3(rows), dim3(256), 0, s, j, j, ld_out, hidden, eps, perm_out);
+    launch_norm<false>(s, dim3(rows), j, j, ld_out, hidden, eps, perm_out);
     return XB_LAUNCH_OK();
 }
 
@@ -1450,7 +1472,7 @@ int add_rmsnorm_rows(cudaStream_t s, __half* out, __half* x, const __half* delta
     j.x = x;
     j.delta = delta;
     j.w = w;
-    launch_pdl(rmsnorm_kernel<false>, dim3(rows), dim3(256), 0, s, j, j, static_cast<long long>(hidden), hidden, eps, perm_out);
+    launch_norm<false>(s, dim3(rows), j, j, static_cast<long long>(hidden), hidden, eps, perm_out);
     return XB_LAUNCH_OK();
 }
 
