@@ -1,0 +1,29 @@
+"""The convolution over a chunk with one and with four channels a thread, on either side of the line between them, with weights that can be
+loaded as vectors and with weights that cannot: the same bits, and those of a row-by-row reference within one rounding."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 8, 9, 63, 64, 65, 72, 200])
+@pytest.mark.parametrize("channels", [4, 512, 1028, 1030])
+def test_rows_and_channels(cuda, rows, channels):
+    g = torch.Generator(device="cuda").manual_seed(rows * 7 + channels)
+    x = torch.randn((rows, channels), generator=g, device="cuda").half()
+    shifted = torch.randn(channels * 4 + 1, generator=g, device="cuda")[1:].view(channels, 4)  # four bytes behind a boundary
+    state = torch.randn((3, channels), generator=g, device="cuda")
+    out, states = [], []
+    for weights, inplace in ((shifted.clone(), False), (shifted, False), (shifted.clone(), True)):
+        st = state.clone()
+        o = x.clone() if inplace else torch.full_like(x, float("nan"))
+        assert cuda.causal_conv1d_silu(o, o if inplace else x, weights, rows, st, channels) == 0
+        out.append(o)
+        states.append(st)
+    assert all(torch.equal(out[0], o) for o in out) and all(torch.equal(states[0], s) for s in states)
+    seen = torch.cat([state.double(), x.double()])
+    assert torch.equal(states[0], seen[-3:].float())
+    y = sum(shifted[:, t].double() * seen[t:t + rows] for t in range(4))
+    want = y / (1 + torch.exp(-y))
+    bound = sum((shifted[:, t].double() * seen[t:t + rows]).abs() for t in range(4))  # four fp32 roundings of sums this large at most
+    assert torch.all((out[0].double() - want).abs() <= 2.0 ** -11 * 1.01 * want.abs() + 8 * 2.0 ** -24 * bound + 2.0 ** -24)

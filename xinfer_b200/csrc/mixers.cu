@@ -679,11 +679,12 @@ __global__ void __launch_bounds__(128 * PARTS, PARTS == 2 ? (TOKENS <= 4 ? 3 : 2
 //
 // The convolution has no recurrence on its outputs (y_p needs the inputs p-3 .. p only): a thread takes V channels and
 // SPAN consecutive positions with the window in registers.  The threads of the first positions are the only readers of
-// the state and also the ones that replace it by the chunk's last three inputs, so one launch does both.  512 x 10240 in 11.9 us
-// (its 21 MB take 3.2 at the copy's rate).
+// the state and also the ones that replace it by the chunk's last three inputs, so one launch does both.  512 x 10240 in 9.7 us
+// (its 21 MB take 3.2 at the copy's rate; 11.9 with the weights loaded one by one).
 // SPAN 0: all positions, when the output overwrites the input (a position's inputs are its neighbours').  A store may not pass the
-// loads behind it, so the inputs are read kAhead positions at a time there too: 512 x 10240 in 86 us, position by position in 172.
-constexpr int kAhead = 8;
+// loads behind it, so the inputs are read kAhead positions at a time there too: 512 x 10240 in 65 us, four channels a thread in 86,
+// position by position in 172.
+constexpr int kAhead = 8, kConvNarrowRows = 64;
 template <int V, int SPAN>
 __global__ void __launch_bounds__(128) conv1d_chunk_kernel(__half* out, const __half* in, const float* conv_w, float* state, int rc,
                                                            int channels) {
@@ -692,11 +693,23 @@ __global__ void __launch_bounds__(128) conv1d_chunk_kernel(__half* out, const __
     const int b = blockIdx.y, p0 = blockIdx.x * SPAN;
     const long long seq0 = static_cast<long long>(b) * rc;
     if (c >= channels) return;
+    // (a channel's four weights in one load: one by one, sixteen bytes apart, the lanes' requests were more than the activations')
     float w[V][4];
+    if ((reinterpret_cast<uintptr_t>(conv_w) & 15) == 0) {
 #pragma unroll
-    for (int e = 0; e < V; ++e) {
+        for (int e = 0; e < V; ++e) {
+            const float4 q = __ldg(reinterpret_cast<const float4*>(conv_w) + c + e);
+            w[e][0] = q.x;
+            w[e][1] = q.y;
+            w[e][2] = q.z;
+            w[e][3] = q.w;
+        }
+    } else {
 #pragma unroll
-        for (int t = 0; t < 4; ++t) w[e][t] = conv_w[(c + e) * 4 + t];
+        for (int e = 0; e < V; ++e) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) w[e][t] = conv_w[(c + e) * 4 + t];
+        }
     }
     float* st = state ? state + static_cast<long long>(b) * 3 * channels : nullptr;
     struct alignas(2 * V) Vec { __half h[V]; };
@@ -1533,10 +1546,13 @@ int conv1d_chunk(cudaStream_t s, __half* out, const __half* in, const float* con
     const size_t bytes = static_cast<size_t>(batch) * rc * channels * sizeof(__half);
     const char *o = reinterpret_cast<const char*>(out), *i = reinterpret_cast<const char*>(in);
     const bool overlap = o < i + bytes && i < o + bytes;
-    const bool vec = channels % 4 == 0 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in)) & 7) == 0;
+    // One channel a thread is the shorter chain, which counts while a launch is no more than that: few rows (10240 channels, us a launch with
+    // four channels a thread and with one: 1 row 2.36 and 2.05, 8 rows 3.25 and 2.63, 33 rows 3.86 and 3.45, 77 rows 5.0 and 5.1, 509 rows 9.7
+    // and 14.0), or every position of a channel one after the other (in place, 509 rows 84 and 65).
+    const bool vec = !overlap && static_cast<long long>(batch) * rc > kConvNarrowRows && channels % 4 == 0 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in)) & 7) == 0;
     const int per_block = 128 * (vec ? 4 : 1);
     dim3 grid(overlap ? 1 : (rc + kAhead - 1) / kAhead, batch, (channels + per_block - 1) / per_block);
-    launch_pdl(overlap ? (vec ? conv1d_chunk_kernel<4, 0> : conv1d_chunk_kernel<1, 0>) : (vec ? conv1d_chunk_kernel<4, kAhead> : conv1d_chunk_kernel<1, kAhead>),
+    launch_pdl(overlap ? conv1d_chunk_kernel<1, 0> : (vec ? conv1d_chunk_kernel<4, kAhead> : conv1d_chunk_kernel<1, kAhead>),
                grid, dim3(128), 0, s, out, in, conv_w, state, rc, channels);
     return XB_LAUNCH_OK();
 }
