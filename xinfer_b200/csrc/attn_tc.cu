@@ -171,6 +171,30 @@ __device__ __forceinline__ void store8(__half* dst, const uint4& v, int vec) {
     }
 }
 
+// Four lanes' four pieces each, transposed: lane q's t[k] becomes what t[q] of lane k of the four was.
+__device__ __forceinline__ uint4 shfl_xor4(const uint4& v, int mask) {
+    return make_uint4(__shfl_xor_sync(0xffffffffu, v.x, mask), __shfl_xor_sync(0xffffffffu, v.y, mask), __shfl_xor_sync(0xffffffffu, v.z, mask),
+                      __shfl_xor_sync(0xffffffffu, v.w, mask));
+}
+__device__ __forceinline__ uint4 pick4(bool first, const uint4& a, const uint4& b) {
+    return make_uint4(first ? a.x : b.x, first ? a.y : b.y, first ? a.z : b.z, first ? a.w : b.w);
+}
+__device__ __forceinline__ void transpose4(uint4 (&t)[4], int lane) {
+    const bool b1 = lane & 2, b0 = lane & 1;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const uint4 got = shfl_xor4(pick4(b1, t[j], t[j + 2]), 2);
+        t[j] = pick4(b1, got, t[j]);
+        t[j + 2] = pick4(b1, t[j + 2], got);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j += 2) {
+        const uint4 got = shfl_xor4(pick4(b0, t[j], t[j + 1]), 1);
+        t[j] = pick4(b0, got, t[j]);
+        t[j + 1] = pick4(b0, t[j + 1], got);
+    }
+}
+
 // Keys in front of item e's first row, and its number of 64-key blocks (at least one).
 __device__ __forceinline__ int item_ctx(const TileShape& sh, int e) { return sh.ctx ? __ldg(sh.ctx + e / sh.tiles) : sh.ctx_base; }
 __device__ __forceinline__ int item_blocks(const TileShape& sh, int e) {
@@ -514,27 +538,53 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
             const size_t slot = (static_cast<size_t>(blockIdx.x) * 2 + (walk.kb0 > 0 ? 0 : 1)) * rows + r;
             const long long at = (static_cast<long long>(b) * sh.rows_per_seq + pos) * sh.hq + kvh * sh.group + head_in_group;
             const float inv = whole ? 1.0f / (l > 0.f ? l : 1.0f) : 1.0f;
+            // A part of a tile of many rows is stored by four lanes a row, sixteen bytes each: a thread's own row piece by piece, every store is 32
+            // lines of memory and half a sector of each (24 heads, us: 512 rows behind 1536 50.3 -> 44.1, 77 behind 2000 30.8 -> 24.8).  Few rows
+            // do not pay for the shuffles (1 row behind 1023 10.6 and 11.3, 8 rows of 48 queries 13.8 and 13.5), finished fp16 rows, whose
+            // stores are half as many, neither (77 rows 15.8 and 19.3).
+            if (!whole && rows > 32) {
+                const int quad = lane & ~3, q = lane & 3;
+                const uint32_t live = __ballot_sync(0xffffffffu, valid) >> quad;
 #pragma unroll 1
-            for (int c = 0; c < kDim; c += 32) {
-                uint32_t o[32];
-                tmem_ld32(tmem + lanes + kColO + c, o);
-                tmem_wait_ld();
-                if (valid) {
-                    float v[32];
+                for (int c = 0; c < kDim; c += 32) {
+                    uint32_t o[32];
+                    tmem_ld32(tmem + lanes + kColO + c, o);
+                    tmem_wait_ld();
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(o[e]) * inv;
-                    if (whole) {
-                        __half* dst = p.out + at * kDim + c;
-                        const __half* gate = p.q_gate ? p.q_gate + at * 512 + 256 + c : nullptr;
+                    for (int e = 0; e < 32; e += 16) {
+                        uint4 t[4];
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) store8(dst + 8 * e, finish8(v + 8 * e, gate ? gate + 8 * e : nullptr, p.perm_out != 0), p.out_vec);
-                    } else {
-                        float4* dst = reinterpret_cast<float4*>(p.part_o + slot * kDim + c);
+                        for (int k = 0; k < 4; ++k) t[k] = make_uint4(o[e + 4 * k], o[e + 4 * k + 1], o[e + 4 * k + 2], o[e + 4 * k + 3]);
+                        transpose4(t, lane);
+                        float* dst = p.part_o + (slot - q) * kDim + c + e + 4 * q;  // (rows follow one another)
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) __stcg(dst + e, make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]));
+                        for (int k = 0; k < 4; ++k)
+                            if (live >> k & 1u) __stcg(reinterpret_cast<uint4*>(dst + k * kDim), t[k]);
                     }
                 }
-                __syncwarp();
+            } else {
+#pragma unroll 1
+                for (int c = 0; c < kDim; c += 32) {
+                    uint32_t o[32];
+                    tmem_ld32(tmem + lanes + kColO + c, o);
+                    tmem_wait_ld();
+                    if (valid) {
+                        float v[32];
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(o[e]) * inv;
+                        if (whole) {
+                            __half* dst = p.out + at * kDim + c;
+                            const __half* gate = p.q_gate ? p.q_gate + at * 512 + 256 + c : nullptr;
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) store8(dst + 8 * e, finish8(v + 8 * e, gate ? gate + 8 * e : nullptr, p.perm_out != 0), p.out_vec);
+                        } else {
+                            float4* dst = reinterpret_cast<float4*>(p.part_o + slot * kDim + c);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) __stcg(dst + e, make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]));
+                        }
+                    }
+                    __syncwarp();
+                }
             }
             if (!whole && valid) *reinterpret_cast<float2*>(p.part_ml + slot * 2) = make_float2(m, l);
             if (tid == 0 && kvh == 0 && walk.kb0 == 0)
