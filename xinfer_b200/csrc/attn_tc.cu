@@ -75,6 +75,7 @@ struct TileShape {          // what both kernels need to find their work
     int ctx_base;
     int rows_per_seq, hq, hkv, group, tile_pos, tiles, items;  // items = batch * tiles, tiles fastest
     long long max_seq;
+    int by_item;            // a group of CTAs to every item, none cut (whole_items)
 };
 struct TileParams {
     CUtensorMap q_map, k_map, v_map;
@@ -217,6 +218,13 @@ struct TileWalk {
     __device__ void start(const TileShape& sh, int group, int most_groups) {
         const int lane = threadIdx.x & 31;
         total = 0;
+        if (sh.by_item) {
+            groups = sh.items;
+            item = group;
+            off = u = 0;
+            u_end = group < groups ? item_blocks(sh, group) : 0;
+            return;
+        }
         for (int e0 = 0; e0 < sh.items; e0 += 32) {
             const int mine = e0 + lane < sh.items ? item_blocks(sh, e0 + lane) : 0;
             total += __reduce_add_sync(0xffffffffu, mine);
@@ -588,7 +596,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
             }
             if (!whole && valid) *reinterpret_cast<float2*>(p.part_ml + slot * 2) = make_float2(m, l);
             if (tid == 0 && kvh == 0 && walk.kb0 == 0)
-                p.table[item] = make_int2(static_cast<int>(blockIdx.x) / sh.hkv, unit_owner(walk.u + walk.blocks - 1, walk.total, walk.groups));
+                p.table[item] = make_int2(static_cast<int>(blockIdx.x) / sh.hkv, sh.by_item ? static_cast<int>(blockIdx.x) / sh.hkv
+                                                                                   : unit_owner(walk.u + walk.blocks - 1, walk.total, walk.groups));
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&ctrl->o_free));
@@ -730,6 +739,26 @@ TileDims tile_dims(int batch, int rows_per_seq, int hq, int hkv) {
 
 }  // namespace
 
+namespace {
+// Whether every item is better left whole, with a group of CTAs for each.  Cut evenly, a group has two blocks or more, of one item or of two
+// (which it then reads out one after the other), and the parts are merged by another launch: with several tiles a sequence that costs
+// as much as kCutBlocks more blocks of the largest item, with one, which few groups share, kOneTileBlocks blocks are as long as two and the merge.
+// 24 heads, us cut and whole: 77 rows behind none 15.4 and 8.8, behind 400 18.7 and 16.1, behind 600 19.1 and 19.7; 128 behind none 17.4 and 9.3;
+// 512 behind none 27.0 and 17.6, behind 256 26.8 and 22.6; 2 rows behind 126 10.5 and 8.3, 1 behind 200 10.2 and 10.4, 4 behind 380 10.5 and 12.6.
+constexpr long long kCutBlocks = 7, kOneTileBlocks = 3;
+bool whole_items(const AttnTiles& a, const TileDims& d, int groups) {
+    if (a.ctx || d.items > groups) return false;  // (only the device knows the number of keys)
+    long long most = 0, total = 0;
+    for (int t = 0; t < d.tiles; ++t) {
+        const long long end = static_cast<long long>(t + 1) * d.tile_pos;
+        most = (a.ctx_base + (end < a.rows_per_seq ? end : a.rows_per_seq) + kTileKeys - 1) / kTileKeys;
+        total += most * a.batch;
+    }
+    if (d.tiles == 1) return most <= kOneTileBlocks;
+    return most <= (total > 2 * groups ? total / groups : 2) + kCutBlocks;
+}
+}  // namespace
+
 // Enough for every launch of at most `rows_per_seq` rows (tiles of fewer rows may each hold more of them: 128 positions are
 // 7 tiles of 19, 59 are 3 of 20).
 size_t attn_tile_scratch_bytes(int batch, int rows_per_seq, int hq, int hkv, int num_sms) {
@@ -776,6 +805,7 @@ int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status) {
     p.scale2 = a.scale * 1.4426950408889634f;
     p.part_o = a.scratch;
     const int ctas = tile_ctas(a.hkv, num_sms);
+    p.sh.by_item = whole_items(a, d, ctas / a.hkv);
     p.part_ml = a.scratch + static_cast<size_t>(ctas) * 2 * d.rows * kDim;
     p.table = reinterpret_cast<int2*>(p.part_ml + static_cast<size_t>(ctas) * 2 * d.rows * 2);
     p.wait_limit = tc_wait_limit();
@@ -794,8 +824,8 @@ int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status) {
         }
     }
     if (launch_pdl(attn_tile_kernel, dim3(ctas), dim3(kTileThreads), tile_smem_bytes(d.rows), s, p) != cudaSuccess) return -1;
-    // (every item a single block: nothing was cut)
-    if (!a.ctx && static_cast<long long>(a.ctx_base) + a.rows_per_seq <= kTileKeys) return 0;
+    // (nothing was cut, or every item is a single block)
+    if (p.sh.by_item || (!a.ctx && static_cast<long long>(a.ctx_base) + a.rows_per_seq <= kTileKeys)) return 0;
     const bool wide = d.tiles == 1 && ctas >= 8 * a.batch * a.hkv;  // eight parts a row
     if (launch_pdl(wide ? attn_tile_combine_kernel<8> : attn_tile_combine_kernel<1>, dim3(p.sh.items * a.hkv, wide ? d.rows : (d.rows + 7) / 8),
                    dim3(256), 0, s, a.out, static_cast<const float*>(p.part_o), static_cast<const float*>(p.part_ml),
