@@ -449,8 +449,8 @@ XINFER_EXPORT int xinfer_spec_decoder_set_sampling(xinfer_spec_decoder* d, float
  * capture. */
 XINFER_EXPORT int xinfer_spec_decoder_set_top_p(xinfer_spec_decoder* d, float top_p);
 /* Builds the context from a prompt, tokens[batch][T] on the host (every sequence the same length), starting from the
- * empty context of xinfer_spec_decoder_reset(d, 0, seed): positions 0 .. T-2 go through the target in chunks of up to
- * 512 rows over all sequences (the projections of a chunk run as one M = 512 GEMM each, attention, convolution and the
+ * empty context of xinfer_spec_decoder_reset(d, 0, seed): positions 0 .. T-2 go through the target in chunks of one length and up to
+ * 4096 rows over all sequences, fewer where the device's memory does not hold that (the projections of a chunk run as one GEMM each, attention, convolution and the
  * gated delta rule take it in one launch each), the MTP head's KV slots of those positions are filled, the last prompt
  * token becomes the current token; ctx = T - 1 afterwards and xinfer_spec_decoder_step continues from there.  Stands
  * where the reference's chunked prefill does (forward_prefill_chunk, src/targets/qwen3_8/forward.cpp:402-554;
