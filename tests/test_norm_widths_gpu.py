@@ -1,4 +1,4 @@
-"""RMSNorm with one 8-element vector a thread (few rows, or narrow ones) and with up to four: on either side of the lines between them, at
+"""RMSNorm with one 8-element vector a thread (few rows, or narrow ones), with two and with up to four: on either side of the lines between them, at
 widths that leave the last warp, or the last vector, incomplete, against 64 bits."""
 import pytest
 import torch
@@ -23,3 +23,9 @@ def test_rows_and_widths(cuda, rows, hidden):
     assert torch.equal(res, total)
     want = total.double() * torch.rsqrt(total.double().pow(2).mean(1, keepdim=True) + 1e-6) * w.double()
     assert torch.all((out.double() - want).abs() <= 2.0 ** -11 * 1.01 * want.abs() + 2.0 ** -24)
+
+
+@pytest.mark.parametrize("rows", [444, 445, 592, 593, 888, 889])
+@pytest.mark.parametrize("hidden", [2048, 2056, 2560, 4096, 4104, 5120, 6136, 6144, 6152])
+def test_two_vectors_a_thread(cuda, rows, hidden):
+    test_rows_and_widths(cuda, rows, hidden)

@@ -106,16 +106,21 @@ __device__ __forceinline__ const uint16_t* norm_tokens(const NormJob& job, long 
 }
 __device__ __forceinline__ __half bf16_to_half(uint32_t bits) { return __float2half_rn(__uint_as_float(bits << 16)); }
 
-constexpr int kNormWideRows = 148, kNormNarrow = 2048;
+constexpr int kNormSms = 148, kNormNarrow = 2048, kNormPairs = 6144;
 // TABLE: some job of the launch reads the embedding table.  VECS: most 8-element vectors of a thread: four of 256 threads (and the path for
-// rows that are not vectors), or one of up to 1024.
+// rows that are not vectors), two of up to 512, or one of up to 1024.  FEW: no row shares its SM.  Bound by latency, then by the rows in flight.
 // One vector a thread is the shorter way through a row, which is what counts as long as every row has an SM to itself, and where 256
-// threads would not all have one: 5120 features with the residual added, 1 row 2.30 -> 2.03 us, 32 rows 2.57 -> 2.30, 148 rows 2.58 -> 2.31;
-// 1024 features, 2796 rows 8.9 -> 4.9.  With more rows the 640 threads of a wide row leave an SM three rows at a time, and four vectors a
-// thread are better: 1024 x 5120 5.93 us against 6.83 without the addition, 2796 x 5120 12.6 against 15.7 (between 148 and 512 rows
-// either may be, by up to 0.3 us).
-template <bool TABLE, int VECS>
-__global__ void __launch_bounds__(VECS == 1 ? 1024 : 256) rmsnorm_kernel(const __grid_constant__ NormJob job0, const __grid_constant__ NormJob job1,
+// threads would not all have one: 5120 features with the residual added, 1 row 2.30 -> 1.84 us, 32 rows 2.57 -> 2.13, 148 rows 2.58 -> 2.24;
+// 1024 features, 2796 rows 8.9 -> 4.9.  (0.07 to 0.12 us of it since the compiler may use 64 registers, where otherwise it fits two rows of 1024
+// threads on an SM; with many narrow rows those are worth as much: 1024 features, 2796 rows 4.47 against 4.71.)  With more rows the 640
+// threads of a wide row leave an SM three rows at a time: 1024 x 5120 5.93 us with four vectors, 6.83 with one.
+// Two vectors, the weights read behind the sum (another trip to L2, but 40 registers in place of 77), put four rows of 5120 or 6144 features on an
+// SM in place of three and leave no thread idle: where rows are many, and where four an SM are a single wave.  5120 features with the residual
+// added: 296..444 rows 3.8 us with four vectors and 4.5 with two, 445..592 5.2 and 4.4, 740 5.9 and 6.4, 1480 9.8 and 9.1, 2796 17.7 and 15.9;
+// 2560 features, 740 rows 4.3 and 4.7, 2796 11.8 and 8.0.  At 7168 and more, two rows an SM, 740 rows 5.3 and 6.1, 2796 15.8 and 16.2; at 2048
+// one vector is better up to 1024 rows (3.1 and 3.9).
+template <bool TABLE, int VECS, bool FEW>
+__global__ void __launch_bounds__(VECS == 1 ? 1024 : VECS == 2 ? 512 : 256, VECS == 2 ? 3 : FEW ? 1 : 0) rmsnorm_kernel(const __grid_constant__ NormJob job0, const __grid_constant__ NormJob job1,
                                                       long long ld_out, int hidden, float eps, int perm_out) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ __align__(16) float red[32];  // of every warp
@@ -127,6 +132,7 @@ __global__ void __launch_bounds__(VECS == 1 ? 1024 : 256) rmsnorm_kernel(const _
     const __half* dr = job.delta ? job.delta + row * hidden : nullptr;
     __half* orow = job.out + row * ld_out;
     const int nvec = hidden >> 3;
+    constexpr bool kLateW = VECS == 2;
     const bool vec_ok = (hidden & 7) == 0 && nvec <= VECS * static_cast<int>(blockDim.x) &&
                         ((reinterpret_cast<uintptr_t>(xr) | reinterpret_cast<uintptr_t>(orow) | reinterpret_cast<uintptr_t>(dr) |
                           reinterpret_cast<uintptr_t>(job.table) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
@@ -136,8 +142,8 @@ __global__ void __launch_bounds__(VECS == 1 ? 1024 : 256) rmsnorm_kernel(const _
         float4 wv[VECS][2];
 #pragma unroll
         for (int it = 0; it < VECS; ++it) {
-            const int i = threadIdx.x + it * 256;
-            if (i < nvec) {
+            const int i = threadIdx.x + it * (VECS == 2 ? blockDim.x : 256);
+            if (i < nvec && !kLateW) {
                 wv[it][0] = __ldg(reinterpret_cast<const float4*>(w + i * 8));
                 wv[it][1] = __ldg(reinterpret_cast<const float4*>(w + i * 8 + 4));
             }
@@ -150,7 +156,7 @@ __global__ void __launch_bounds__(VECS == 1 ? 1024 : 256) rmsnorm_kernel(const _
         uint4 v[VECS], dv[VECS];
 #pragma unroll
         for (int it = 0; it < VECS; ++it) {
-            const int i = threadIdx.x + it * 256;
+            const int i = threadIdx.x + it * (VECS == 2 ? blockDim.x : 256);
             if (i < nvec) {
                 if (!table) v[it] = *reinterpret_cast<const uint4*>(xr + i * 8);
                 else v[it] = tr ? __ldg(reinterpret_cast<const uint4*>(tr + i * 8)) : make_uint4(0u, 0u, 0u, 0u);
@@ -160,7 +166,7 @@ __global__ void __launch_bounds__(VECS == 1 ? 1024 : 256) rmsnorm_kernel(const _
         float ss = 0.f;
 #pragma unroll
         for (int it = 0; it < VECS; ++it) {
-            const int i = threadIdx.x + it * 256;
+            const int i = threadIdx.x + it * (VECS == 2 ? blockDim.x : 256);
             if (i < nvec) {
                 __half2* h = reinterpret_cast<__half2*>(&v[it]);
                 if (table) {
@@ -185,22 +191,23 @@ __global__ void __launch_bounds__(VECS == 1 ? 1024 : 256) rmsnorm_kernel(const _
         }
         ss = warp_sum(ss);
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-        if (VECS == 1 && threadIdx.x < 32 && threadIdx.x >= (blockDim.x >> 5)) red[threadIdx.x] = 0.f;
+        if (VECS <= 2 && threadIdx.x < 32 && threadIdx.x >= (blockDim.x >> 5)) red[threadIdx.x] = 0.f;
         __syncthreads();
         float total = 0.f;
 #pragma unroll
-        for (int w = 0; w < (VECS == 1 ? 32 : 8); w += 8) {
+        for (int w = 0; w < (VECS == 1 ? 32 : VECS == 2 ? 16 : 8); w += 8) {
             const float4 r0 = *reinterpret_cast<const float4*>(red + w), r1 = *reinterpret_cast<const float4*>(red + w + 4);
             total += ((r0.x + r1.x) + (r0.z + r1.z)) + ((r0.y + r1.y) + (r0.w + r1.w));
         }
         const float r = 1.0f / sqrtf(total / static_cast<float>(hidden) + eps);
 #pragma unroll
         for (int it = 0; it < VECS; ++it) {
-            const int i = threadIdx.x + it * 256;
+            const int i = threadIdx.x + it * (VECS == 2 ? blockDim.x : 256);
             if (i < nvec) {
                 if (xr && (dr || table)) *reinterpret_cast<uint4*>(xr + i * 8) = v[it];
                 const __half2* h = reinterpret_cast<const __half2*>(&v[it]);
-                const float4 w0 = wv[it][0], w1 = wv[it][1];
+                const float4 w0 = kLateW ? __ldg(reinterpret_cast<const float4*>(w + i * 8)) : wv[it][0];
+                const float4 w1 = kLateW ? __ldg(reinterpret_cast<const float4*>(w + i * 8 + 4)) : wv[it][1];
                 const float ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
                 uint4 o;
                 __half2* oh = reinterpret_cast<__half2*>(&o);
@@ -1429,10 +1436,18 @@ __global__ void fill_int_kernel(int* p, int n, int v) {
 namespace {
 template <bool TABLE>
 void launch_norm(cudaStream_t s, dim3 grid, const NormJob& a, const NormJob& b, long long ld_out, int hidden, float eps, int perm_out) {
-    if (hidden % 8 == 0 && hidden <= 8 * 1024 && (static_cast<int>(grid.x) <= kNormWideRows || hidden <= kNormNarrow))
-        launch_pdl(rmsnorm_kernel<TABLE, 1>, grid, dim3((hidden / 8 + 31) / 32 * 32), 0, s, a, b, ld_out, hidden, eps, perm_out);
+    const int rows = static_cast<int>(grid.x), warps_of_one = (hidden / 8 + 31) / 32, warps_of_two = (hidden / 8 + 63) / 64;
+    const bool vectors = hidden % 8 == 0 && hidden <= 8 * 1024;
+    const bool pairs = hidden > kNormNarrow && hidden <= kNormPairs &&
+                       (rows > 6 * kNormSms || (hidden > 4096 && rows > 3 * kNormSms && rows <= 4 * kNormSms));
+    if (vectors && rows <= kNormSms)
+        launch_pdl(rmsnorm_kernel<TABLE, 1, true>, grid, dim3(warps_of_one * 32), 0, s, a, b, ld_out, hidden, eps, perm_out);
+    else if (vectors && hidden <= kNormNarrow)
+        launch_pdl(rmsnorm_kernel<TABLE, 1, false>, grid, dim3(warps_of_one * 32), 0, s, a, b, ld_out, hidden, eps, perm_out);
+    else if (vectors && pairs)
+        launch_pdl(rmsnorm_kernel<TABLE, 2, false>, grid, dim3(warps_of_two * 32), 0, s, a, b, ld_out, hidden, eps, perm_out);
     else
-        launch_pdl(rmsnorm_kernel<TABLE, 4>, grid, dim3(256), 0, s, a, b, ld_out, hidden, eps, perm_out);
+        launch_pdl(rmsnorm_kernel<TABLE, 4, false>, grid, dim3(256), 0, s, a, b, ld_out, hidden, eps, perm_out);
 }
 }  // namespace
 
