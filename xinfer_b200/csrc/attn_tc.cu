@@ -75,7 +75,6 @@ struct TileShape {          // what both kernels need to find their work
     int ctx_base;
     int rows_per_seq, hq, hkv, group, tile_pos, tiles, items;  // items = batch * tiles, tiles fastest
     long long max_seq;
-    int by_item;            // a group of CTAs to every item, none cut (whole_items)
 };
 struct TileParams {
     CUtensorMap q_map, k_map, v_map;
@@ -214,11 +213,12 @@ __device__ __forceinline__ int unit_owner(int u, int total, int groups) {
 struct TileWalk {
     int item, off, u, u_end, total, groups;  // next item, next block of it, next unit
     int kb0, n, blocks;                    // the current run
-    // Every lane of a warp calls it.
+    // Every lane of a warp calls it.  BY_ITEM: a group to every item, none cut (whole_items).
+    template <bool BY_ITEM>
     __device__ void start(const TileShape& sh, int group, int most_groups) {
         const int lane = threadIdx.x & 31;
         total = 0;
-        if (sh.by_item) {
+        if constexpr (BY_ITEM) {
             groups = sh.items;
             item = group;
             off = u = 0;
@@ -269,6 +269,9 @@ struct TileWalk {
     __device__ bool whole() const { return kb0 == 0 && n == blocks; }
 };
 
+// BY_ITEM: whole_items.  FOUR: parts are stored by four lanes a row.  Both are compiled apart from the form of a step's rows, which is slower by
+// the mere presence of either (8 x 8192 keys: 56.6 us, 58.6 beside FOUR, 60.3 beside both).
+template <bool BY_ITEM, bool FOUR>
 __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid_constant__ TileParams p) {
     extern __shared__ uint8_t tile_smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tile_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -315,7 +318,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
     if (!p.early) griddep_wait();
     TileWalk walk;
     const int kvh = static_cast<int>(blockIdx.x) % sh.hkv;
-    walk.start(sh, static_cast<int>(blockIdx.x) / sh.hkv, static_cast<int>(gridDim.x) / sh.hkv);
+    walk.start<BY_ITEM>(sh, static_cast<int>(blockIdx.x) / sh.hkv, static_cast<int>(gridDim.x) / sh.hkv);
     const int units = walk.u_end - walk.u;
 
     if (warp == kKWarp || warp == kVWarp) {
@@ -542,7 +545,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
             ok = ok && mbar_wait(smem_u32(&ctrl->pv_done[(i - 1) & 1]), ((i - 1) >> 1) & 1u, ws);
             if (!ok) break;
             tc_fence_after_sync();
-            const bool whole = walk.whole();
+            const bool whole = BY_ITEM || walk.whole();
             const size_t slot = (static_cast<size_t>(blockIdx.x) * 2 + (walk.kb0 > 0 ? 0 : 1)) * rows + r;
             const long long at = (static_cast<long long>(b) * sh.rows_per_seq + pos) * sh.hq + kvh * sh.group + head_in_group;
             const float inv = whole ? 1.0f / (l > 0.f ? l : 1.0f) : 1.0f;
@@ -550,7 +553,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
             // lines of memory and half a sector of each (24 heads, us: 512 rows behind 1536 50.3 -> 44.1, 77 behind 2000 30.8 -> 24.8).  Few rows
             // do not pay for the shuffles (1 row behind 1023 10.6 and 11.3, 8 rows of 48 queries 13.8 and 13.5), finished fp16 rows, whose
             // stores are half as many, neither (77 rows 15.8 and 19.3).
-            if (!whole && rows > 32) {
+            if (FOUR && !whole) {
                 const int quad = lane & ~3, q = lane & 3;
                 const uint32_t live = __ballot_sync(0xffffffffu, valid) >> quad;
 #pragma unroll 1
@@ -595,9 +598,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) attn_tile_kernel(const __grid
                 }
             }
             if (!whole && valid) *reinterpret_cast<float2*>(p.part_ml + slot * 2) = make_float2(m, l);
-            if (tid == 0 && kvh == 0 && walk.kb0 == 0)
-                p.table[item] = make_int2(static_cast<int>(blockIdx.x) / sh.hkv, sh.by_item ? static_cast<int>(blockIdx.x) / sh.hkv
-                                                                                   : unit_owner(walk.u + walk.blocks - 1, walk.total, walk.groups));
+            if (!BY_ITEM && tid == 0 && kvh == 0 && walk.kb0 == 0)
+                p.table[item] = make_int2(static_cast<int>(blockIdx.x) / sh.hkv, unit_owner(walk.u + walk.blocks - 1, walk.total, walk.groups));
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&ctrl->o_free));
@@ -743,8 +745,8 @@ namespace {
 // Whether every item is better left whole, with a group of CTAs for each.  Cut evenly, a group has two blocks or more, of one item or of two
 // (which it then reads out one after the other), and the parts are merged by another launch: with several tiles a sequence that costs
 // as much as kCutBlocks more blocks of the largest item, with one, which few groups share, kOneTileBlocks blocks are as long as two and the merge.
-// 24 heads, us cut and whole: 77 rows behind none 15.4 and 8.8, behind 400 18.7 and 16.1, behind 600 19.1 and 19.7; 128 behind none 17.4 and 9.3;
-// 512 behind none 27.0 and 17.6, behind 256 26.8 and 22.6; 2 rows behind 126 10.5 and 8.3, 1 behind 200 10.2 and 10.4, 4 behind 380 10.5 and 12.6.
+// 24 heads, us cut and whole: 77 rows behind none 15.4 and 8.4, behind 400 18.7 and 15.6, behind 600 19.1 and 19.7; 128 behind none 17.4 and 8.9;
+// 512 behind none 27.0 and 17.1, behind 256 26.8 and 22.1; 2 rows behind 126 10.5 and 8.3, 1 behind 200 10.2 and 10.4, 4 behind 380 10.5 and 12.6.
 constexpr long long kCutBlocks = 7, kOneTileBlocks = 3;
 bool whole_items(const AttnTiles& a, const TileDims& d, int groups) {
     if (a.ctx || d.items > groups) return false;  // (only the device knows the number of keys)
@@ -805,7 +807,7 @@ int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status) {
     p.scale2 = a.scale * 1.4426950408889634f;
     p.part_o = a.scratch;
     const int ctas = tile_ctas(a.hkv, num_sms);
-    p.sh.by_item = whole_items(a, d, ctas / a.hkv);
+    const bool by_item = whole_items(a, d, ctas / a.hkv);
     p.part_ml = a.scratch + static_cast<size_t>(ctas) * 2 * d.rows * kDim;
     p.table = reinterpret_cast<int2*>(p.part_ml + static_cast<size_t>(ctas) * 2 * d.rows * 2);
     p.wait_limit = tc_wait_limit();
@@ -818,14 +820,15 @@ int attn_tiles(cudaStream_t s, const AttnTiles& a, int num_sms, int* status) {
         if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
         std::lock_guard<std::mutex> lock(mu);
         if (!configured[dev]) {
-            if (cudaFuncSetAttribute(attn_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
-                return -1;
+            for (auto* f : {attn_tile_kernel<false, false>, attn_tile_kernel<false, true>, attn_tile_kernel<true, false>})
+                if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return -1;
             configured[dev] = true;
         }
     }
-    if (launch_pdl(attn_tile_kernel, dim3(ctas), dim3(kTileThreads), tile_smem_bytes(d.rows), s, p) != cudaSuccess) return -1;
+    auto* kernel = by_item ? attn_tile_kernel<true, false> : d.rows > 32 ? attn_tile_kernel<false, true> : attn_tile_kernel<false, false>;
+    if (launch_pdl(kernel, dim3(ctas), dim3(kTileThreads), tile_smem_bytes(d.rows), s, p) != cudaSuccess) return -1;
     // (nothing was cut, or every item is a single block)
-    if (p.sh.by_item || (!a.ctx && static_cast<long long>(a.ctx_base) + a.rows_per_seq <= kTileKeys)) return 0;
+    if (by_item || (!a.ctx && static_cast<long long>(a.ctx_base) + a.rows_per_seq <= kTileKeys)) return 0;
     const bool wide = d.tiles == 1 && ctas >= 8 * a.batch * a.hkv;  // eight parts a row
     if (launch_pdl(wide ? attn_tile_combine_kernel<8> : attn_tile_combine_kernel<1>, dim3(p.sh.items * a.hkv, wide ? d.rows : (d.rows + 7) / 8),
                    dim3(256), 0, s, a.out, static_cast<const float*>(p.part_o), static_cast<const float*>(p.part_ml),
