@@ -25,3 +25,24 @@ def test_same_bits_as_without(cuda, M, K, N):
     torch.cuda.synchronize()
     assert cuda.device_status(0) == 0
     assert torch.equal(got, want) and not torch.isnan(got).any()
+
+
+def test_uncut_launches_share_no_scratch(cuda):
+    """7105 tiles of one stage: long enough for the rule, but no tile is cut, so that such launches may run on several streams at once."""
+    M, K, N = 32, 256, 7105 * 256
+    g = torch.Generator(device="cuda").manual_seed(3)
+    w = torch.randint(0, 256, (N, K // 2), generator=g, device="cuda", dtype=torch.uint8)
+    s = torch.rand((N, K // 128), generator=g, device="cuda").mul_(0.01).half()
+    xs = [torch.randn((M, K), generator=g, device="cuda").half() for _ in range(2)]
+    want, got = ([torch.empty((M, N), device="cuda", dtype=torch.float16) for _ in range(2)] for _ in range(2))
+    for x, y in zip(xs, want):
+        assert cuda.linear_int4_noalloc(y, x, w, s, None, M, N, K) == 0
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for _ in range(5):
+        for stream, x, y in zip(streams, xs, got):
+            with torch.cuda.stream(stream):
+                assert cuda.linear_int4(y, x, w, s, None, M, N, K) == 0
+    torch.cuda.synchronize()
+    assert cuda.device_status(0) == 0
+    assert all(torch.equal(a, b) for a, b in zip(want, got))

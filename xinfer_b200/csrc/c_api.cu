@@ -151,7 +151,7 @@ int run_linear(xinfer_stream_t s, const void* x, xb::ActType in, bool out_f32, c
     const bool want_tc = (c->forced_path != 2) && in == xb::ActType::F16 &&
                          xb::tc_eligible(x, proj, num, swiglu, m, k, group_size);
     if (want_tc) {
-        const bool permuted = xb::tc_wants_permuted_x(proj, num, swiglu, m, k, c->num_sms);
+        const bool permuted = xb::tc_wants_permuted_x(proj, num, swiglu, m, k, c->num_sms, kCounterCapacity);
         if (permuted && xb::tc_permute_x(stream, x, c->x_scratch, m, k) != 0) return fail_cuda(cudaGetLastError());
         int r = xb::tc_launch(stream, permuted ? c->x_scratch : x, proj, num, swiglu, out_f32, m, k, c->num_sms, c->workspace, c->counters,
                               kCounterCapacity, c->status, nullptr, permuted ? xb::kTcXPermuted : 0);

@@ -30,7 +30,7 @@ struct TcProj {
 size_t tc_workspace_bytes(int ctas);
 // X in the order kTcXPermuted names, written once in front of a launch that is worth it (tc_x_scratch_bytes of scratch).
 size_t tc_x_scratch_bytes();
-bool tc_wants_permuted_x(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms);
+bool tc_wants_permuted_x(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms, int counter_capacity);
 int tc_permute_x(cudaStream_t stream, const void* x, void* scratch, long long m, long long k);
 // Test hooks for the bounded device-side waits: their clock limit (<= 0 restores the one-second default)
 // and the first activation stage that the producer never requests (-1: all are requested).

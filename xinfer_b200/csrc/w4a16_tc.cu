@@ -1294,14 +1294,16 @@ size_t tc_x_scratch_bytes() { return static_cast<size_t>(32) * kXScratchK * size
 // for each of its stages.  With more than 16 rows that warp is the pace of a stage (1900 clocks against 1700), but the small launch costs
 // 1.5 us: at 32 rows 80 stages per CTA (5120 x 151936) take 100.9 -> 97.8 us, 21 (5120 x 40000) 35.6 -> 36.1, 16 (2560 x 60000)
 // 30.8 -> 32.1; at 16 rows there is nothing to gain (88.7 both).  The line lies above the 33 stages where the two meet.
-bool tc_wants_permuted_x(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms) {
+bool tc_wants_permuted_x(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms, int counter_capacity) {
     if (m <= 16 || k > kXScratchK) return false;
     long long tiles = 0;
+    const long long stages = (k / 128 + 1) / 2;
     const int rows = swiglu ? kHalfRows : kTileRows;
     for (int i = 0; i < (swiglu ? 1 : num); ++i) tiles += (proj[i].n + rows - 1) / rows;
-    // (cut tiles only: those launches use the device's scratch buffer already, others may run beside each other on several streams)
-    if (tiles < num_sms || tiles % num_sms == 0) return false;
-    return tiles * ((k / 128 + 1) / 2) >= kPermuteStages * num_sms;
+    // Cut tiles only: those launches use the device's scratch buffer already, others may run beside each other on several streams.  (A tile of
+    // one stage cannot be cut, and more tiles than counters are refused by tc_launch.)
+    if (tiles < num_sms || tiles % num_sms == 0 || stages < 2 || tiles > counter_capacity) return false;
+    return tiles * stages >= kPermuteStages * num_sms;
 }
 
 int tc_permute_x(cudaStream_t stream, const void* x, void* scratch, long long m, long long k) {
