@@ -46,3 +46,25 @@ def test_uncut_launches_share_no_scratch(cuda):
     torch.cuda.synchronize()
     assert cuda.device_status(0) == 0
     assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+def test_x_written_by_the_launch_in_front(cuda):
+    """The small launch starts while the norm in front of it, whose output it reads, still runs; every call has another X."""
+    M, K, N = 32, 5120, 151936
+    g = torch.Generator(device="cuda").manual_seed(9)
+    w = torch.randint(0, 256, (N, K // 2), generator=g, device="cuda", dtype=torch.uint8)
+    s = torch.rand((N, K // 128), generator=g, device="cuda").mul_(0.01).half()
+    norm_w = torch.randn(K, generator=g, device="cuda")
+    xs = [torch.randn((M, K), generator=g, device="cuda").half() for _ in range(6)]
+    normed = torch.empty_like(xs[0])
+    got, want = ([torch.empty((M, N), device="cuda", dtype=torch.float16) for _ in xs] for _ in range(2))
+    for x, y in zip(xs, got):
+        assert cuda.rmsnorm(normed, x, norm_w, M, K) == 0
+        assert cuda.linear_int4(y, normed, w, s, None, M, N, K) == 0
+    for x, y in zip(xs, want):
+        assert cuda.rmsnorm(normed, x, norm_w, M, K) == 0
+        torch.cuda.synchronize()
+        assert cuda.linear_int4_noalloc(y, normed, w, s, None, M, N, K) == 0
+    torch.cuda.synchronize()
+    assert cuda.device_status(0) == 0
+    assert all(torch.equal(a, b) for a, b in zip(want, got))

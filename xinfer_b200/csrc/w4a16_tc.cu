@@ -1283,7 +1283,7 @@ __global__ void __launch_bounds__(256) permute_x_kernel(const uint4* x, uint4* o
     griddep_prologue();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= blocks) return;
-    const uint4 v = __ldg(x + i);
+    const uint4 v = x[i];  // (not by the read-only path: the launch in front may still have been writing X when this grid started)
     out[i] = make_uint4(prmt(v.x, v.z, 0x5410u), prmt(v.x, v.z, 0x7632u), prmt(v.y, v.w, 0x5410u), prmt(v.y, v.w, 0x7632u));
 }
 }  // namespace
