@@ -27,3 +27,23 @@ def test_rows_and_channels(cuda, rows, channels):
     want = y / (1 + torch.exp(-y))
     bound = sum((shifted[:, t].double() * seen[t:t + rows]).abs() for t in range(4))  # four fp32 roundings of sums this large at most
     assert torch.all((out[0].double() - want).abs() <= 2.0 ** -11 * 1.01 * want.abs() + 8 * 2.0 ** -24 * bound + 2.0 ** -24)
+
+
+@pytest.mark.parametrize("rows", [1, 3])
+@pytest.mark.parametrize("inplace", [False, True])
+def test_more_channels_than_blocks_of_one_channel_a_thread(cuda, rows, inplace):
+    """65535 blocks of 128 channels and four channels more: too many for a grid with one channel a thread, not for one with four."""
+    channels = 65535 * 128 + 4
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn((rows, channels), generator=g, device="cuda").half()
+    weights = torch.randn((channels, 4), generator=g, device="cuda")
+    state = torch.randn((3, channels), generator=g, device="cuda")
+    seen = torch.cat([state, x.float()])
+    o = x.clone() if inplace else torch.empty_like(x)
+    assert cuda.causal_conv1d_silu(o, o if inplace else x, weights, rows, state, channels) == 0
+    assert torch.equal(state, seen[-3:])
+    terms = [weights[:, t] * seen[t:t + rows] for t in range(4)]
+    y = sum(terms).double()
+    want = y / (1 + torch.exp(-y))
+    bound = sum(t.abs() for t in terms).double()  # four fp32 roundings of sums this large at most, here and in the expectation
+    assert torch.all((o.double() - want).abs() <= 2.0 ** -11 * 1.01 * want.abs() + 16 * 2.0 ** -24 * bound + 2.0 ** -24)

@@ -1563,11 +1563,13 @@ int conv1d_chunk(cudaStream_t s, __half* out, const __half* in, const float* con
     const bool overlap = o < i + bytes && i < o + bytes;
     // One channel a thread is the shorter chain, which counts while a launch is no more than that: few rows (10240 channels, us a launch with
     // four channels a thread and with one: 1 row 2.36 and 2.05, 8 rows 3.25 and 2.63, 33 rows 3.86 and 3.45, 77 rows 5.0 and 5.1, 509 rows 9.7
-    // and 14.0), or every position of a channel one after the other (in place, 509 rows 84 and 65).
-    const bool vec = !overlap && static_cast<long long>(batch) * rc > kConvNarrowRows && channels % 4 == 0 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in)) & 7) == 0;
+    // and 14.0), or every position of a channel one after the other (in place, 509 rows 84 and 65).  More than 65535 blocks of 128 channels
+    // do not fit the grid's third dimension.
+    const bool vec_ok = channels % 4 == 0 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in)) & 7) == 0;
+    const bool vec = vec_ok && (channels > 65535 * 128 || (!overlap && static_cast<long long>(batch) * rc > kConvNarrowRows));
     const int per_block = 128 * (vec ? 4 : 1);
     dim3 grid(overlap ? 1 : (rc + kAhead - 1) / kAhead, batch, (channels + per_block - 1) / per_block);
-    launch_pdl(overlap ? conv1d_chunk_kernel<1, 0> : (vec ? conv1d_chunk_kernel<4, kAhead> : conv1d_chunk_kernel<1, kAhead>),
+    launch_pdl(overlap ? (vec ? conv1d_chunk_kernel<4, 0> : conv1d_chunk_kernel<1, 0>) : (vec ? conv1d_chunk_kernel<4, kAhead> : conv1d_chunk_kernel<1, kAhead>),
                grid, dim3(128), 0, s, out, in, conv_w, state, rc, channels);
     return XB_LAUNCH_OK();
 }
