@@ -274,7 +274,8 @@ XINFER_EXPORT int xinfer_spec_decoder_override_drafts(xinfer_spec_decoder* d, co
 XINFER_EXPORT int xinfer_spec_decoder_enqueue_linears(xinfer_spec_decoder* d, xinfer_stream_t stream);
 /* what: 0 weight bytes, 1 state bytes, 2 kernel launches per step, 3 graph captured,
  * 4 algorithmic bytes of the step's linear launches (this rank's), 5 number of linear launches per step,
- * 6 inter-rank exchanges per step, 7 bytes of the decoder's one device block */
+ * 6 inter-rank exchanges per step, 7 bytes of the decoder's one device block, 8 chunks of the last prompt,
+ * 9 bytes of the buffers of prompt chunks, kept from the first prompt on until the decoder is destroyed */
 XINFER_EXPORT int64_t xinfer_spec_decoder_info(const xinfer_spec_decoder* d, int what);
 XINFER_EXPORT void* xinfer_spec_decoder_tensor(xinfer_spec_decoder* d, int layer, const char* name, int64_t* bytes);
 XINFER_EXPORT const char* xinfer_spec_decoder_error(const xinfer_spec_decoder* d);
@@ -449,14 +450,18 @@ XINFER_EXPORT int xinfer_spec_decoder_set_sampling(xinfer_spec_decoder* d, float
  * capture. */
 XINFER_EXPORT int xinfer_spec_decoder_set_top_p(xinfer_spec_decoder* d, float top_p);
 /* Builds the context from a prompt, tokens[batch][T] on the host (every sequence the same length), starting from the
- * empty context of xinfer_spec_decoder_reset(d, 0, seed): positions 0 .. T-2 go through the target in chunks of one length and up to
- * 4096 rows over all sequences, fewer where the device's memory does not hold that (the projections of a chunk run as one GEMM each, attention, convolution and the
- * gated delta rule take it in one launch each), the MTP head's KV slots of those positions are filled, the last prompt
- * token becomes the current token; ctx = T - 1 afterwards and xinfer_spec_decoder_step continues from there.  Stands
+ * empty context of xinfer_spec_decoder_reset(d, 0, seed): positions 0 .. T-2 go through the target in chunks of one length and
+ * up to 4096 rows over all sequences, fewer (down to 512) where the buffers of a chunk would take more than a quarter of the
+ * device's free memory (the projections of a chunk run as one GEMM each, attention, convolution and the gated delta rule take it
+ * in one launch each), the MTP head's KV slots of those positions are filled, the last prompt token becomes the current token;
+ * ctx = T - 1 afterwards and xinfer_spec_decoder_step continues from there.  Stands
  * where the reference's chunked prefill does (forward_prefill_chunk, src/targets/qwen3_8/forward.cpp:402-554;
  * prefill_chunk_size = 512, include/xinfer/engine.h:34; engine.cpp:330-398).  Synchronous; one GPU only. */
 XINFER_EXPORT int xinfer_spec_decoder_prefill(xinfer_spec_decoder* d, xinfer_stream_t stream, const int64_t* prompt_host,
                                               int64_t T);
+/* Test hook of this decoder's prompts: chunks have at most that many rows (0: 4096), and that many bytes of device memory are taken
+ * for free (0: what the device reports). */
+XINFER_EXPORT int xinfer_debug_set_chunk_hooks(xinfer_spec_decoder* d, int64_t most_rows, int64_t free_bytes);
 /* The device side of Engine::generate's speculative loop (src/runtime/engine.cpp:262-560) for `batch` prompts of one
  * length T (host, [batch][T]): the reference's argument checks (max_new_tokens > 0, temperature >= 0, 0 < top_p <= 1 and top_p < 1 only with temperature > 0,
  * prompt + completion within the cache; messages in xinfer_spec_decoder_error), reset to the empty context, prefill,

@@ -34,3 +34,38 @@ def test_chunks_against_one_sequence(cuda, batch, tokens):
             err = np.sqrt(np.mean((whole[name][b] - one[name][0]) ** 2) / np.mean(one[name][0] ** 2))
             assert err < 36 ** 0.5 * 2.0 ** -11, name
     assert cuda.device_status(0) == 0
+
+
+def test_chunks_leave_the_device_most_of_its_memory(cuda):
+    """Buffers for more than 512 rows take a quarter of the free memory at most, their own block, which they replace, counted as free;
+    with less, chunks are halved, down to 512 rows whatever that leaves."""
+    from xinfer_b200.spec import Shape, SpecDecoder
+    shape_cfg = Shape(hidden_size=512, intermediate_size=512, num_hidden_layers=4, num_attention_heads=8, num_key_value_heads=2,
+                      vocab_size=1024, linear_num_v_heads=3, linear_num_k_heads=1)
+    batch, tokens = 4, 1025  # 4096 rows
+    prompts = np.random.default_rng(1).integers(0, 1024, size=(batch, tokens)).astype(np.int64)
+    dec = SpecDecoder(shape_cfg, batch=batch, k=3, max_seq=tokens + 32, seed=4)
+
+    def run(free):
+        dec.set_chunk_hooks(free_bytes=free)
+        dec.reset(0, seed=2)
+        dec.prefill(prompts)
+        return dec.info(8), dec.info(9), dec.tensor(-1, "h_last", np.float16).astype(np.float64)
+
+    chunks, bytes_512, want = run(1)
+    assert chunks == 8
+    free = 4 * bytes_512
+    seen = {}
+    while chunks > 1:  # (a little more free memory each time: the chunks get longer one step after the other)
+        chunks, taken, got = run(free)
+        assert chunks in (1, 2, 4, 8) and chunks <= min(seen, default=8)
+        if chunks not in seen and chunks < 8:
+            assert 4 * taken <= free + max(seen.values(), default=bytes_512)
+            seen[chunks] = taken
+        # a few dozen fp16 roundings (2^-12 rms each, relative) on the way, whose sums come in another order
+        assert np.sqrt(np.mean((got - want) ** 2) / np.mean(want ** 2)) < 36 ** 0.5 * 2.0 ** -11
+        free += free // 8
+    assert sorted(seen) == [1, 2, 4]
+    assert run(1)[:2] == (1, seen[1])  # (buffers that are there already are used)
+    dec.close()
+    assert cuda.device_status(0) == 0

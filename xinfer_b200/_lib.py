@@ -121,6 +121,7 @@ SIGNATURES = {
     "xinfer_spec_decoder_exchange_bytes": (_sz, [_vp, _i32, _i32, _i32]),
     "xinfer_spec_decoder_load_artifact": (_i32, [_vp, _vp, _i32]),
     "xinfer_spec_decoder_prefill": (_i32, [_vp, _vp, _vp, _i64]),
+    "xinfer_debug_set_chunk_hooks": (_i32, [_vp, _i64, _i64]),
     "xinfer_spec_decoder_set_sampling": (_i32, [_vp, _f32, _u64]),
     "xinfer_spec_decoder_generate": (_i32, [_vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp]),
     "xinfer_sample_tokens_top_p": (_i32, [_vp, _vp, _i64, _i64, _i32, _f32, _f32, _vp, _vp, _vp]),

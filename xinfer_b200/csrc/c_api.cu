@@ -100,6 +100,21 @@ int get_ctx(DeviceCtx** out) {
     return XINFER_OK;
 }
 
+// Scratch for K splits of the GEMM: taken once per device, outside any stream capture (a failed or refused allocation just means no
+// K split).
+void take_gemm_partials(DeviceCtx* c, cudaStream_t stream) {
+    if (c->gemm_partials || c->gemm_partials_tried) return;
+    c->gemm_partials_tried = true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+        void* ptr = nullptr;
+        if (cudaMalloc(&ptr, xb::gemm_partial_bytes(c->num_sms)) == cudaSuccess) c->gemm_partials = static_cast<float*>(ptr);
+        else cudaGetLastError();
+    } else {
+        c->gemm_partials_tried = false;  // try again on a call that is not being captured
+    }
+}
+
 int run_linear(xinfer_stream_t s, const void* x, xb::ActType in, bool out_f32, const xb::TcProj* proj, int num,
                bool swiglu, int64_t m, int64_t k, int group_size) {
     DeviceCtx* c = nullptr;
@@ -130,19 +145,7 @@ int run_linear(xinfer_stream_t s, const void* x, xb::ActType in, bool out_f32, c
     }
     if (c->forced_path != 2 && in == xb::ActType::F16 && xb::gemm_eligible(x, proj, num, swiglu, m, k, group_size)) {
         // more than 32 rows (prefill chunks): the compute-bound tcgen05 GEMM
-        // scratch for K splits of the GEMM: taken once per device, outside any stream capture (a failed or refused
-        // allocation just means no K split)
-        if (!c->gemm_partials && !c->gemm_partials_tried) {
-            c->gemm_partials_tried = true;
-            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-            if (cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
-                void* ptr = nullptr;
-                if (cudaMalloc(&ptr, xb::gemm_partial_bytes(c->num_sms)) == cudaSuccess) c->gemm_partials = static_cast<float*>(ptr);
-                else cudaGetLastError();
-            } else {
-                c->gemm_partials_tried = false;  // try again on a call that is not being captured
-            }
-        }
+        take_gemm_partials(c, stream);
         const int r = xb::gemm_launch(stream, x, proj, num, swiglu, out_f32, m, k, c->status, xb::tc_wait_limit(), xb::tc_x_stage_limit(), c->num_sms,
                                       c->gemm_partials, c->counters);
         if (r == 0) { g_last_path = 3; return XINFER_OK; }
@@ -232,6 +235,11 @@ int device_facts(int** status, int* num_sms) {
     *status = c->status;
     *num_sms = c->num_sms;
     return XINFER_OK;
+}
+
+void take_gemm_scratch(cudaStream_t s) {
+    DeviceCtx* c = nullptr;
+    if (get_ctx(&c) == XINFER_OK) take_gemm_partials(c, s);
 }
 
 int run_tc_linear(cudaStream_t s, const void* x, const TcProj* proj, int num, bool swiglu, bool out_f32, long long m,

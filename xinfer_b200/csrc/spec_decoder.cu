@@ -174,6 +174,7 @@ struct xinfer_spec_decoder {
     // activation rows of a prefill chunk (allocated by the first long prompt, freed with the decoder)
     struct ChunkBufs {
         int rows = 0;
+        size_t bytes = 0;
         __half *x = nullptr, *normed = nullptr, *proj_out = nullptr, *mlp = nullptr, *wide = nullptr, *wide2 = nullptr,
                *qbuf = nullptr, *kbuf = nullptr, *vbuf = nullptr, *mix_out = nullptr, *zbuf = nullptr, *bbuf = nullptr,
                *abuf = nullptr, *cat = nullptr, *hprev = nullptr;
@@ -181,6 +182,9 @@ struct xinfer_spec_decoder {
         void* gdn_scratch = nullptr;     // per-block operands of the delta rule
         float* attn_scratch = nullptr;   // partials of one attention launch
     } chunk;
+    int chunk_rows_hook = 0;              // xinfer_debug_set_chunk_hooks
+    int64_t chunk_free_hook = 0;
+    int prompt_chunks = 0;                // of the last prompt
     float top_p = 1.0f;               // < 1: nucleus sampling on both sides of the stochastic rule
     xb::Nucleus* nucleus = nullptr;   // [batch * (k + 1)] nuclei of the verify rows
     int prev_rows = 0;       // rows of the previous target pass (for the lazy state commit)
@@ -667,11 +671,15 @@ int target_pass(Dec* d, cudaStream_t s, int R, const long long* tokens) {
 
 // A chunk's launches cost the same whatever its length (filling and draining a GEMM and the exchange of its cut tiles 6 to 16 us, the
 // others 2 to 3): with 512 / 1024 / 2048 / 4096 rows, prompts of 4 x 700 tokens through 8 layers and a few decoding steps take 23.5 / 21.9 /
-// 21.3 / 20.5 ms, 1 x 768 7.2 / 6.5 / 6.5 / 6.5.  A row takes 180 KB of buffers; where the device has no room for them, chunks are halved
-// down to kLeastChunkRows.
+// 21.3 / 20.5 ms, 1 x 768 7.2 / 6.5 / 6.5 / 6.5.  A row takes 214 KB at the 27B shapes (183 of activations, 31 of the delta rule's operands) and
+// a launch of the attention 39 MB whatever the rows, which the decoder keeps: 0.92 GB for 4096 rows, 0.15 for 512.  So that a prompt
+// does not take from its host what that counts on, chunks of more than kLeastChunkRows rows take no more than a kChunkShare-th of the memory
+// that is free (their own block, which they replace, counted in); they are halved until they do.
 constexpr int kChunkRows = 4096, kLeastChunkRows = 512;
+constexpr size_t kChunkShare = 4;
 
-int ensure_chunk_bufs(Dec* d, int rows) {
+// Buffers for chunks of `rows` rows: at any price (`must`), or if the device has memory to spare, else the present ones stay.
+int ensure_chunk_bufs(Dec* d, int rows, bool must) {
     auto& cb = d->chunk;
     if (cb.rows >= rows) return 0;
     const auto& c = d->cfg;
@@ -683,14 +691,21 @@ int ensure_chunk_bufs(Dec* d, int rows) {
     const size_t wide = mx(hq * 512, ch), mix = mx(mx(hq * 256, hv * 128), H);
     const size_t per_row = 3 * H + F + wide + ch + hq * 256 + 2 * hkv * 256 + mix + hv * 128 + 2 * hv + 2 * H + H;
     const size_t halves = (per_row + 64) * static_cast<size_t>(rows);
-    if (cb.x) { cudaFree(cb.x); cb = Dec::ChunkBufs(); }
     // one block: activations, tokens, the attention's and the delta rule's scratch
     const int positions = (rows + d->batch - 1) / d->batch;  // of every sequence
     const size_t attn_bytes = xb::attn_tile_scratch_bytes(d->batch, positions, static_cast<int>(hq), static_cast<int>(hkv), d->num_sms);
     const size_t front = (halves * sizeof(__half) + static_cast<size_t>(rows) * sizeof(long long) + 256 + 255) & ~static_cast<size_t>(255);
     const size_t attn_end = (front + attn_bytes + 255) & ~static_cast<size_t>(255);
+    const size_t bytes = attn_end + xb::gdn_chunk_scratch_bytes(d->batch, positions, static_cast<int>(hv));
+    if (!must) {
+        size_t free_bytes = 0, total = 0;
+        if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) { cudaGetLastError(); return XINFER_ERR_OUT_OF_MEMORY; }
+        if (d->chunk_free_hook > 0) free_bytes = static_cast<size_t>(d->chunk_free_hook);
+        if (bytes > (free_bytes + cb.bytes) / kChunkShare) return XINFER_ERR_OUT_OF_MEMORY;
+    }
+    if (cb.x) { cudaFree(cb.x); cb = Dec::ChunkBufs(); }
     __half* base = nullptr;
-    if (cudaMalloc(&base, attn_end + xb::gdn_chunk_scratch_bytes(d->batch, positions, static_cast<int>(hv))) != cudaSuccess) {
+    if (cudaMalloc(&base, bytes) != cudaSuccess) {
         cudaGetLastError();
         return XINFER_ERR_OUT_OF_MEMORY;
     }
@@ -707,6 +722,7 @@ int ensure_chunk_bufs(Dec* d, int rows) {
     cb.attn_scratch = reinterpret_cast<float*>(reinterpret_cast<char*>(base) + front);
     cb.gdn_scratch = reinterpret_cast<char*>(base) + attn_end;
     cb.rows = rows;
+    cb.bytes = bytes;
     return 0;
 }
 
@@ -1105,6 +1121,8 @@ int64_t xinfer_spec_decoder_info(const xinfer_spec_decoder* d, int what) {
         case 5: return d->linear_launches;
         case 6: return d->exchanges_per_step;
         case 7: return d->arena ? static_cast<int64_t>(xinfer_arena_capacity(d->arena)) : 0;
+        case 8: return d->prompt_chunks;
+        case 9: return static_cast<int64_t>(d->chunk.bytes);
         default: return -1;
     }
 }
@@ -1133,6 +1151,13 @@ int xinfer_spec_decoder_set_top_p(xinfer_spec_decoder* d, float top_p) {
     return XINFER_OK;
 }
 
+int xinfer_debug_set_chunk_hooks(xinfer_spec_decoder* d, int64_t most_rows, int64_t free_bytes) {
+    if (!d || most_rows < 0 || most_rows > kChunkRows || free_bytes < 0) return XINFER_ERR_INVALID_ARGUMENT;
+    d->chunk_rows_hook = static_cast<int>(most_rows);
+    d->chunk_free_hook = free_bytes;
+    return XINFER_OK;
+}
+
 // Builds the context from a prompt: tokens [batch][T] (host), all sequences the same length, starting from the empty
 // context of reset(0, seed).  Positions 0 .. T-2 go through the target model in chunks of up to 4096 rows over all
 // sequences (prefill_chunk: every row kept, so KV caches, Gated-DeltaNet and convolution state advance as in steps whose
@@ -1148,20 +1173,34 @@ int xinfer_spec_decoder_prefill(xinfer_spec_decoder* d, xinfer_stream_t stream, 
     if (d->ctx_upper != 0) { d->error = "prefill starts from the empty context (reset(0, seed))"; return XINFER_ERR_INVALID_ARGUMENT; }
     if (T - 1 + 2 * R > d->max_seq) { d->error = "prompt does not fit the cache"; return XINFER_ERR_INVALID_ARGUMENT; }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    // What a prompt needs whatever the length of its chunks comes first: its tokens (a block of an earlier prompt's chunks gives way to
+    // them), and the scratch of the device's GEMM.
+    long long* prompt = nullptr;
+    const size_t pbytes = static_cast<size_t>(B) * T * sizeof(long long);
+    if (cudaMalloc(&prompt, pbytes) != cudaSuccess) {
+        cudaGetLastError();
+        if (!d->chunk.x) return XINFER_ERR_OUT_OF_MEMORY;
+        cudaFree(d->chunk.x);
+        d->chunk = Dec::ChunkBufs();
+        if (cudaMalloc(&prompt, pbytes) != cudaSuccess) { cudaGetLastError(); return XINFER_ERR_OUT_OF_MEMORY; }
+    }
+    if (B * (T - 1) > 32) xb::take_gemm_scratch(s);
     // positions per sequence and chunk: as few chunks as kChunkRows rows over all sequences allow, of one length but for the last, in whole
     // blocks of the delta rule
     int Cp = 0;
-    for (int rows = kChunkRows; T > 1; rows /= 2) {
+    d->prompt_chunks = 0;
+    for (int rows = d->chunk_rows_hook > 0 ? d->chunk_rows_hook : kChunkRows; T > 1; rows /= 2) {
         const int64_t most = rows / B > 16 ? rows / B / 16 * 16 : 16, chunks = (T - 1 + most - 1) / most;
         Cp = static_cast<int>(((T - 1 + chunks - 1) / chunks + 15) / 16 * 16);
         if (T - 1 < Cp) Cp = static_cast<int>(T - 1);
-        const int rc0 = ensure_chunk_bufs(d, B * Cp);
+        d->prompt_chunks = static_cast<int>((T - 1 + Cp - 1) / Cp);
+        const int rc0 = ensure_chunk_bufs(d, B * Cp, rows <= kLeastChunkRows);
         if (rc0 == 0) break;
-        if (rc0 != XINFER_ERR_OUT_OF_MEMORY || rows <= kLeastChunkRows) return rc0;
+        if (rc0 != XINFER_ERR_OUT_OF_MEMORY || rows <= kLeastChunkRows) {
+            cudaFree(prompt);
+            return rc0;
+        }
     }
-    long long* prompt = nullptr;
-    const size_t pbytes = static_cast<size_t>(B) * T * sizeof(long long);
-    if (cudaMalloc(&prompt, pbytes) != cudaSuccess) { cudaGetLastError(); return XINFER_ERR_OUT_OF_MEMORY; }
     int prev_r = 0;
     int rc = [&]() -> int {
         CKCUDA(cudaMemcpyAsync(prompt, prompt_host, pbytes, cudaMemcpyHostToDevice, s));

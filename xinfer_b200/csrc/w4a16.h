@@ -52,6 +52,8 @@ int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num,
 double gemm_modelled_us(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms);
 // The current device's status word (what xinfer_device_status reads) and number of SMs; a XINFER_* code.
 int device_facts(int** status, int* num_sms);
+// The GEMM's scratch of the current device, if it has not been taken yet: for callers with large allocations of their own to make.
+void take_gemm_scratch(cudaStream_t s);
 // Records a message for xinfer_last_cuda_error() on the calling thread (c_api.cu).
 void set_last_error(const char* msg);
 // Programmatic dependent launch (on unless XINFER_PDL=0): kernels are launched with the stream-serialization

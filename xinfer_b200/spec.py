@@ -114,6 +114,10 @@ class SpecDecoder:
         if code != 0:
             raise _lib.XInferError(code, "spec_decoder_prefill: " + self._err())
 
+    def set_chunk_hooks(self, most_rows: int = 0, free_bytes: int = 0) -> None:
+        """Test hook of the prompts' chunks: their most rows, and the device memory taken for free (0 restores either)."""
+        _lib.check(lib().xinfer_debug_set_chunk_hooks(self._h, most_rows, free_bytes), "debug_set_chunk_hooks")
+
     def generate(self, prompt, max_new_tokens: int = 256, temperature: float = 0.0, top_p: float = 1.0,
                  eos_token_id: int = -1, im_end_token_id: int = -1, seed: int = 0, stream=None):
         """The speculative generate loop for ``prompt`` (int64 [batch][T]) with the fields of the reference's
