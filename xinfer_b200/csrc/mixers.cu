@@ -26,6 +26,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "launch.cuh"
@@ -106,7 +107,7 @@ __device__ __forceinline__ const uint16_t* norm_tokens(const NormJob& job, long 
 }
 __device__ __forceinline__ __half bf16_to_half(uint32_t bits) { return __float2half_rn(__uint_as_float(bits << 16)); }
 
-constexpr int kNormSms = 148, kNormNarrow = 2048, kNormPairs = 6144;
+constexpr int kNormNarrow = 2048, kNormPairs = 6144;
 // TABLE: some job of the launch reads the embedding table.  VECS: most 8-element vectors of a thread: four of 256 threads (and the path for
 // rows that are not vectors), two of up to 512, or one of up to 1024.  FEW: no row shares its SM.  Bound by latency, then by the rows in flight.
 // One vector a thread is the shorter way through a row, which is what counts as long as every row has an SM to itself, and where 256
@@ -1434,13 +1435,28 @@ __global__ void fill_int_kernel(int* p, int n, int v) {
 #define XB_LAUNCH_OK() (cudaGetLastError() == cudaSuccess ? 0 : -1)
 
 namespace {
+// SMs of the current device.  (Asked of the runtime and kept: a norm may be the first call on a device, also under capture, where the
+// library's own record of it cannot be set up.)
+int sm_count() {
+    static std::atomic<int> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    int n = known[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 148;
+        known[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 template <bool TABLE>
 void launch_norm(cudaStream_t s, dim3 grid, const NormJob& a, const NormJob& b, long long ld_out, int hidden, float eps, int perm_out) {
-    const int rows = static_cast<int>(grid.x), warps_of_one = (hidden / 8 + 31) / 32, warps_of_two = (hidden / 8 + 63) / 64;
+    const long long rows = static_cast<long long>(grid.x) * grid.y, sms = sm_count();  // (a block for every row of every job)
+    const int warps_of_one = (hidden / 8 + 31) / 32, warps_of_two = (hidden / 8 + 63) / 64;
     const bool vectors = hidden % 8 == 0 && hidden <= 8 * 1024;
     const bool pairs = hidden > kNormNarrow && hidden <= kNormPairs &&
-                       (rows > 6 * kNormSms || (hidden > 4096 && rows > 3 * kNormSms && rows <= 4 * kNormSms));
-    if (vectors && rows <= kNormSms)
+                       (rows > 6 * sms || (hidden > 4096 && rows > 3 * sms && rows <= 4 * sms));
+    if (vectors && rows <= sms)
         launch_pdl(rmsnorm_kernel<TABLE, 1, true>, grid, dim3(warps_of_one * 32), 0, s, a, b, ld_out, hidden, eps, perm_out);
     else if (vectors && hidden <= kNormNarrow)
         launch_pdl(rmsnorm_kernel<TABLE, 1, false>, grid, dim3(warps_of_one * 32), 0, s, a, b, ld_out, hidden, eps, perm_out);
