@@ -47,3 +47,12 @@ def test_more_channels_than_blocks_of_one_channel_a_thread(cuda, rows, inplace):
     want = y / (1 + torch.exp(-y))
     bound = sum(t.abs() for t in terms).double()  # four fp32 roundings of sums this large at most, here and in the expectation
     assert torch.all((o.double() - want).abs() <= 2.0 ** -11 * 1.01 * want.abs() + 16 * 2.0 ** -24 * bound + 2.0 ** -24)
+
+
+@pytest.mark.parametrize("rows,channels", [
+    (40, 10240), (41, 10240),  # 400 and 480 blocks of 128 channels and eight positions: one channel a thread below 444 of them
+    (392, 1028), (393, 1028),  # 441 and 450
+    (880, 512), (881, 512),    # 440 and 444
+])
+def test_number_of_blocks(cuda, rows, channels):
+    test_rows_and_channels(cuda, rows, channels)

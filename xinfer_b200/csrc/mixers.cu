@@ -692,7 +692,7 @@ __global__ void __launch_bounds__(128 * PARTS, PARTS == 2 ? (TOKENS <= 4 ? 3 : 2
 // SPAN 0: all positions, when the output overwrites the input (a position's inputs are its neighbours').  A store may not pass the
 // loads behind it, so the inputs are read kAhead positions at a time there too: 512 x 10240 in 65 us, four channels a thread in 86,
 // position by position in 172.
-constexpr int kAhead = 8, kConvNarrowRows = 64;
+constexpr int kAhead = 8, kConvNarrowBlocks = 3;
 template <int V, int SPAN>
 __global__ void __launch_bounds__(128) conv1d_chunk_kernel(__half* out, const __half* in, const float* conv_w, float* state, int rc,
                                                            int channels) {
@@ -1587,12 +1587,15 @@ int conv1d_chunk(cudaStream_t s, __half* out, const __half* in, const float* con
     const size_t bytes = static_cast<size_t>(batch) * rc * channels * sizeof(__half);
     const char *o = reinterpret_cast<const char*>(out), *i = reinterpret_cast<const char*>(in);
     const bool overlap = o < i + bytes && i < o + bytes;
-    // One channel a thread is the shorter chain, which counts while a launch is no more than that: few rows (10240 channels, us a launch with
-    // four channels a thread and with one: 1 row 2.36 and 2.05, 8 rows 3.25 and 2.63, 33 rows 3.86 and 3.45, 77 rows 5.0 and 5.1, 509 rows 9.7
-    // and 14.0), or every position of a channel one after the other (in place, 509 rows 84 and 65).  More than 65535 blocks of 128 channels
-    // do not fit the grid's third dimension.
+    // One channel a thread is the shorter chain, which counts while a launch is no more than that: as long as its blocks are fewer than
+    // kConvNarrowBlocks an SM (us a launch with four channels a thread and with one, blocks of the latter in brackets: 10240 channels, 1 row 2.46 and
+    // 2.05 (80), 33 rows 3.79 and 3.48 (400), 48 rows 3.66 and 3.97 (480), 100 rows 4.7 and 5.6 (1040), 400 rows 8.1 and 11.4; 20480 channels, 16
+    // rows 3.58 and 3.25 (320), 24 rows 3.58 and 3.99 (480); 4096 channels, 77 rows 3.56 and 3.15 (320), 100 rows 3.67 and 3.77 (416); 512 channels,
+    // 400 rows 3.43 and 2.87 (200)), or with every position of a channel one after the other (in place, 509 x 10240 84 and 65).  More than 65535
+    // blocks of 128 channels do not fit the grid's third dimension.
     const bool vec_ok = channels % 4 == 0 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in)) & 7) == 0;
-    const bool vec = vec_ok && (channels > 65535 * 128 || (!overlap && static_cast<long long>(batch) * rc > kConvNarrowRows));
+    const long long narrow_blocks = (channels + 127ll) / 128 * batch * ((rc + kAhead - 1) / kAhead);
+    const bool vec = vec_ok && (channels > 65535 * 128 || (!overlap && narrow_blocks >= static_cast<long long>(kConvNarrowBlocks) * sm_count()));
     const int per_block = 128 * (vec ? 4 : 1);
     dim3 grid(overlap ? 1 : (rc + kAhead - 1) / kAhead, batch, (channels + per_block - 1) / per_block);
     launch_pdl(overlap ? (vec ? conv1d_chunk_kernel<4, 0> : conv1d_chunk_kernel<1, 0>) : (vec ? conv1d_chunk_kernel<4, kAhead> : conv1d_chunk_kernel<1, kAhead>),
