@@ -1,5 +1,5 @@
 """Attention over a prompt on either side of the lines where tiles are left whole: the number of keys that one tile, or the largest of several,
-may have; as many tiles as there are groups of CTAs, and one more; batches of chunks by way of the decoder are in its own tests."""
+may have, also where blocks are few for the groups; as many tiles as there are groups of CTAs, and one more; batches of chunks by way of the decoder are in its own tests."""
 import pytest
 
 from test_attn_tiles_gpu import reference
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
     (24, 4, 21, 171), (24, 4, 21, 172),     # one tile, three and four blocks of keys
     (24, 4, 22, 171), (24, 4, 77, 0), (24, 4, 77, 499), (24, 4, 77, 500),  # four tiles, nine and ten blocks
     (24, 4, 777, 0), (24, 4, 778, 0),       # 37 tiles of 21 positions, 38
-    (8, 2, 64, 512), (8, 2, 64, 513), (8, 8, 300, 100), (32, 1, 600, 3), (1, 1, 129, 0), (32, 1, 5, 130)])
+    (8, 2, 64, 384), (8, 2, 64, 385), (8, 2, 64, 512), (8, 2, 64, 513), (1, 1, 512, 0), (8, 8, 300, 100), (32, 1, 600, 3), (1, 1, 129, 0), (32, 1, 5, 130)])
 def test_lines(hq, hkv, T, start):
     torch = pytest.importorskip("torch")
     if not torch.cuda.is_available():

@@ -747,7 +747,11 @@ namespace {
 // as much as kCutBlocks more blocks of the largest item, with one, which few groups share, kOneTileBlocks blocks are as long as two and the merge.
 // 24 heads, us cut and whole: 77 rows behind none 15.4 and 8.4, behind 400 18.7 and 15.6, behind 600 19.1 and 19.7; 128 behind none 17.4 and 8.9;
 // 512 behind none 27.0 and 17.1, behind 256 26.8 and 22.1; 2 rows behind 126 10.5 and 8.3, 1 behind 200 10.2 and 10.4, 4 behind 380 10.5 and 12.6.
-constexpr long long kCutBlocks = 7, kOneTileBlocks = 3;
+// Where groups are many for the blocks, the even share is met without groups that read two parts out, and a cut costs less: kFreeCutBlocks.
+// Twelve head layouts, whole / cut, mean over 16 to 24 calls: less than half a block a group, 7 blocks in the largest item 0.90 to 0.95, 8
+// blocks 1.08 to 1.18 (1 head, 512 rows behind none 15.3 and 12.5 us; 32 / 1 heads, 16 rows behind 496 15.5 and 12.5), 9 blocks 1.02 to 1.09; more
+// blocks a group, 8 blocks 0.87 to 0.96, 9 0.88 to 0.90, 10 0.95 to 1.15.
+constexpr long long kCutBlocks = 7, kFreeCutBlocks = 5, kOneTileBlocks = 3;
 bool whole_items(const AttnTiles& a, const TileDims& d, int groups) {
     if (a.ctx || d.items > groups) return false;  // (only the device knows the number of keys)
     long long most = 0, total = 0;
@@ -757,7 +761,7 @@ bool whole_items(const AttnTiles& a, const TileDims& d, int groups) {
         total += most * a.batch;
     }
     if (d.tiles == 1) return most <= kOneTileBlocks;
-    return most <= (total > 2 * groups ? total / groups : 2) + kCutBlocks;
+    return most <= (total > 2 * groups ? total / groups : 2) + (2 * total < groups ? kFreeCutBlocks : kCutBlocks);
 }
 }  // namespace
 
