@@ -72,7 +72,7 @@ constexpr int gemm_threads(int h, int c) { return kGemmThreads + (gemm_unpack_se
 constexpr int kXSlotsMax = 8, kWSlotsMax = 12, kASlotsMax = 4;
 constexpr int kWSlotBytes = kGemmTileN * 64;                    // 8 KB of packed weights: one group
 constexpr int kGemmMaxProj = 4;
-constexpr long long kOthersWait = 3000;  // clocks
+constexpr long long kOthersWait = 12000;  // clocks
 // Register split of the launch's 512 x 128, or 640 x 96: the fold keeps up to 128, or 96, sums per thread.
 constexpr int kCtrlRegs = 32, kUnpackRegs = 64;
 constexpr int gemm_fold_regs(int h, int c) { return gemm_unpack_sets(h, c) == 2 ? 160 : 208; }
@@ -706,8 +706,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(H, C), 
                 int* counter = p.counters + (c_first * 2 + static_cast<int>(rank)) * (kGemmFoldThreads / 32) + warp;
                 const int n = seg_end - seg_begin;
                 // The pair in whose range a tile starts comes to it last of all it does, after an exchange more than the pairs with one part
-                // only: the others have mostly arrived or are about to.  If they have, its sums stay in registers (writing them, with the
-                // fence behind it, takes 3.5 us at 256 rows: worth a wait of half of that).
+                // only: the others have mostly arrived or are about to, and then its sums stay in registers.  Writing them, with the fence behind
+                // it, takes 3.5 us at 256 rows, and so it does for the others, who may be at it: a wait of less than that is lost where all
+                // parts end together.  5120 x 1024 (five equal parts a tile), us without a wait / 3000 / 12000 clocks: 77 rows 12.6 / 13.5 / 12.6,
+                // 128 rows 14.8 / 16.0 / 14.8, 256 21.3 / 22.5 / 21.3; 17408 x 5120, 128 rows 30.2 / 29.8 / 29.8, 448 67.1 / 66.4 / 66.2.
                 last = false;
                 if (seg_begin == 0) {
                     // (the whole warp asks: a loop of one lane's own costs the epilogue registers)
