@@ -62,9 +62,15 @@ constexpr int kGemmTmemCols = 512, kASlotCols = 64, kDBufsMax = 3;
 constexpr int gemm_halves(int tile_m) { return tile_m > 192 ? 2 : 1; }
 constexpr int gemm_d_bufs(int c) { return c <= 8 ? 3 : 2; }
 constexpr int gemm_a_slots(int c) { return gemm_d_bufs(c) * c * 16 + 4 * kASlotCols <= kGemmTmemCols ? 4 : 2; }  // (at the end of it)
-// Up to 80 rows the two fold threads of a row take the groups in turn, all columns of each, and add their sums up when the tile is
-// done; with more, sums for all columns do not fit the registers and each takes half of the columns of every group.
-constexpr bool gemm_fold_in_turn(int h, int c) { return h == 1 && c <= 5; }
+// Up to 80 rows the two fold threads of a row take the groups in turn (kInTurn), all columns of each, and add their sums up when the tile, or the
+// part of it, is done; with more, sums for all columns do not fit the registers and each takes half of the columns of every group.  So they do
+// on tiles of up to kHalvesGroups groups too, where what they trade at the end is the larger part (us in turn and in halves: 640 x 20000, 64 rows
+// 11.1 and 9.9, 77 rows 11.9 and 10.6; 1024 x 25000, 64 rows 13.4 and 12.4, 77 rows 14.5 and 13.3; 512 x 10000, 48 rows 5.8 in halves; but gate/up
+// 5120 x 17408, 48 rows 37.1 and 38.7, 77 rows 40.8 and 41.8).  Two or three groups in turn, the products of the second thread's first group
+// rounded by themselves, have a tenth larger error against 64 bits than in sequence; with more it is smaller, 0.84 of it at 16 groups and 0.77
+// at 40, which is why tiles of 9 to 24 groups stay in turn although some are faster in halves (2048 x 5632, 64 rows 10.2 and 9.7).
+constexpr bool gemm_may_fold_in_turn(int h, int c) { return h == 1 && c <= 5; }
+constexpr int kHalvesGroups = 8;
 // Sets of unpacking warps, which take the groups in turn.  Up to 128 rows the MMAs of a group take up to 512 clocks, less than a set needs.
 constexpr int gemm_unpack_sets(int h, int c) { return h == 1 && c <= 8 ? 2 : 1; }
 constexpr int gemm_threads(int h, int c) { return kGemmThreads + (gemm_unpack_sets(h, c) - 1) * kGemmUnpackThreads; }
@@ -96,7 +102,7 @@ constexpr int kGemmSmemBytes = 227 * 1024;
 constexpr int kGemmSmemFixed = 1024 + static_cast<int>(sizeof(GemmCtrl));
 constexpr int gemm_x_slots(int h, int c) { return h * c <= 8 ? 8 : 4; }
 constexpr int gemm_x_half_bytes(int h, int c) { return h * c * 8 * 2 * kSwizzleK; }  // 64 k of a CTA's half of the rows
-constexpr int gemm_trade_bytes(int h, int c) { return gemm_fold_in_turn(h, c) ? kGemmFoldThreads * c * 8 * 4 : 0; }
+constexpr int gemm_trade_bytes(int h, int c) { return gemm_may_fold_in_turn(h, c) ? kGemmFoldThreads * c * 8 * 4 : 0; }
 // (the packed weights come from HBM, a microsecond and more away: their ring takes the rest)
 constexpr int gemm_w_slots(int h, int c) {
     const int n = (kGemmSmemBytes - kGemmSmemFixed - gemm_x_slots(h, c) * 2 * gemm_x_half_bytes(h, c) - gemm_trade_bytes(h, c)) / kWSlotBytes & ~1;
@@ -320,9 +326,9 @@ __device__ __forceinline__ void for_steps(F&& f) {
     }
 }
 
-// H accumulator tiles a group of C times 16 columns each.  kSwiglu: a CTA's rows are gate and up of the same
-// 64 features, sixteen and sixteen; y = silu(gate) * up.
-template <int H, int C, typename OutT, bool kSwiglu>
+// H accumulator tiles a group of C times 16 columns each.  kInTurn: see gemm_may_fold_in_turn.  kSwiglu: a CTA's rows are gate and up of the
+// same 64 features, sixteen and sixteen; y = silu(gate) * up.
+template <int H, int C, bool kInTurn, typename OutT, bool kSwiglu>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(H, C), 1) w4a16_gemm_kernel(const __grid_constant__ GemmParams p) {
     extern __shared__ uint8_t gemm_smem_raw[];
     // (the control block first: its addresses are then constants, and the fold, which needs every register, holds none of them)
@@ -350,7 +356,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(H, C), 
             mbar_init(smem_u32(&ctrl->half_done[i]), 1);
         }
         for (int i = 0; i < a_slots; ++i) mbar_init(smem_u32(&ctrl->a_full[i]), 2 * kGemmUnpackThreads / 32);
-        for (int i = 0; i < d_bufs; ++i) mbar_init(smem_u32(&ctrl->d_empty[i]), 2 * kGemmFoldThreads / 32 / (gemm_fold_in_turn(H, C) ? 2 : 1));
+        for (int i = 0; i < d_bufs; ++i) mbar_init(smem_u32(&ctrl->d_empty[i]), 2 * kGemmFoldThreads / 32 / (kInTurn ? 2 : 1));
         ctrl->ws.abort_flag = 0;
         ctrl->ws.dep_ready = 0;
         ctrl->ws.limit = p.wait_limit;
@@ -549,7 +555,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(H, C), 
         // ------------------------------------------------------------------ fold, then write: two threads per weight row
         setmaxnreg_inc<gemm_fold_regs(H, C)>();
         const int r = tid & 127, ch = tid >> 7;  // tile row, and which of the row's two threads
-        constexpr bool kInTurn = gemm_fold_in_turn(H, C);
         const uint32_t d_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + (kInTurn ? 0u : static_cast<uint32_t>(ch * half_cols));
         const uint32_t d_empty0 = mapa_shared_cluster(smem_u32(&ctrl->d_empty[0]), 0);
         const bool up_row = kSwiglu && (r & 16);
@@ -586,6 +591,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(H, C), 
             // One read of tensor memory is in flight while the one before it is added up, and a tile is handed back before its last columns
             // are added: the slowest fold warp of the pair, which shares its scheduler with the MMA warp, is the pace.
             if constexpr (kInTurn) {
+                static_assert(gemm_may_fold_in_turn(H, C), "columns");
                 const int n0 = i + ((i ^ ch) & 1), g0 = group + (n0 - i);  // this thread's first group
                 uint4 q_cur = load_scales(sp, g0 & ~7, p.groups, p.scales_vec), q_next = load_scales(sp, (g0 & ~7) + 8, p.groups, p.scales_vec);
                 const uint32_t pick = g0 & 1 ? 0x4432u : 0x4410u;  // its scales lie in the same half of every word
@@ -882,7 +888,7 @@ bool encode_gemm_x(CUtensorMap* map, const __half* x, long long m, long long k, 
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int H, int C, typename OutT, bool kSwiglu>
+template <int H, int C, bool kInTurn, typename OutT, bool kSwiglu>
 cudaError_t gemm_configure_and_launch(const GemmParams& p, dim3 grid, cudaStream_t stream) {
     static bool configured[64];
     static std::mutex mu;
@@ -895,32 +901,33 @@ cudaError_t gemm_configure_and_launch(const GemmParams& p, dim3 grid, cudaStream
         if (!configured[dev]) {
             // the register re-split draws on what the block was launched with: a request above that would wait forever
             cudaFuncAttributes a;
-            e = cudaFuncGetAttributes(&a, w4a16_gemm_kernel<H, C, OutT, kSwiglu>);
+            e = cudaFuncGetAttributes(&a, w4a16_gemm_kernel<H, C, kInTurn, OutT, kSwiglu>);
             if (e != cudaSuccess) return e;
             if (a.numRegs * gemm_threads(H, C) < gemm_split_regs(H, C)) return cudaErrorLaunchOutOfResources;
-            e = cudaFuncSetAttribute(w4a16_gemm_kernel<H, C, OutT, kSwiglu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemBytes);
+            e = cudaFuncSetAttribute(w4a16_gemm_kernel<H, C, kInTurn, OutT, kSwiglu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemBytes);
             if (e != cudaSuccess) return e;
             configured[dev] = true;
         }
     }
-    return launch_pdl(w4a16_gemm_kernel<H, C, OutT, kSwiglu>, grid, dim3(gemm_threads(H, C)), kGemmSmemBytes, stream, p);
+    return launch_pdl(w4a16_gemm_kernel<H, C, kInTurn, OutT, kSwiglu>, grid, dim3(gemm_threads(H, C)), kGemmSmemBytes, stream, p);
 }
 
 template <typename OutT, bool kSwiglu>
 cudaError_t gemm_configure_and_launch(const GemmParams& p, dim3 grid, cudaStream_t stream) {
+    const bool in_turn = p.groups > kHalvesGroups;
     switch (p.tile_m) {
-        case 48: return gemm_configure_and_launch<1, 3, OutT, kSwiglu>(p, grid, stream);
-        case 64: return gemm_configure_and_launch<1, 4, OutT, kSwiglu>(p, grid, stream);
-        case 80: return gemm_configure_and_launch<1, 5, OutT, kSwiglu>(p, grid, stream);
-        case 96: return gemm_configure_and_launch<1, 6, OutT, kSwiglu>(p, grid, stream);
-        case 112: return gemm_configure_and_launch<1, 7, OutT, kSwiglu>(p, grid, stream);
-        case 128: return gemm_configure_and_launch<1, 8, OutT, kSwiglu>(p, grid, stream);
-        case 144: return gemm_configure_and_launch<1, 9, OutT, kSwiglu>(p, grid, stream);
-        case 160: return gemm_configure_and_launch<1, 10, OutT, kSwiglu>(p, grid, stream);
-        case 176: return gemm_configure_and_launch<1, 11, OutT, kSwiglu>(p, grid, stream);
-        case 192: return gemm_configure_and_launch<1, 12, OutT, kSwiglu>(p, grid, stream);
-        case 224: return gemm_configure_and_launch<2, 7, OutT, kSwiglu>(p, grid, stream);
-        case 256: return gemm_configure_and_launch<2, 8, OutT, kSwiglu>(p, grid, stream);
+        case 48: return in_turn ? gemm_configure_and_launch<1, 3, true, OutT, kSwiglu>(p, grid, stream) : gemm_configure_and_launch<1, 3, false, OutT, kSwiglu>(p, grid, stream);
+        case 64: return in_turn ? gemm_configure_and_launch<1, 4, true, OutT, kSwiglu>(p, grid, stream) : gemm_configure_and_launch<1, 4, false, OutT, kSwiglu>(p, grid, stream);
+        case 80: return in_turn ? gemm_configure_and_launch<1, 5, true, OutT, kSwiglu>(p, grid, stream) : gemm_configure_and_launch<1, 5, false, OutT, kSwiglu>(p, grid, stream);
+        case 96: return gemm_configure_and_launch<1, 6, false, OutT, kSwiglu>(p, grid, stream);
+        case 112: return gemm_configure_and_launch<1, 7, false, OutT, kSwiglu>(p, grid, stream);
+        case 128: return gemm_configure_and_launch<1, 8, false, OutT, kSwiglu>(p, grid, stream);
+        case 144: return gemm_configure_and_launch<1, 9, false, OutT, kSwiglu>(p, grid, stream);
+        case 160: return gemm_configure_and_launch<1, 10, false, OutT, kSwiglu>(p, grid, stream);
+        case 176: return gemm_configure_and_launch<1, 11, false, OutT, kSwiglu>(p, grid, stream);
+        case 192: return gemm_configure_and_launch<1, 12, false, OutT, kSwiglu>(p, grid, stream);
+        case 224: return gemm_configure_and_launch<2, 7, false, OutT, kSwiglu>(p, grid, stream);
+        case 256: return gemm_configure_and_launch<2, 8, false, OutT, kSwiglu>(p, grid, stream);
         default: return cudaErrorInvalidValue;  // (33 rows and more, in the steps of gemm_launch: none)
     }
 }
@@ -996,9 +1003,6 @@ int gemm_launch(cudaStream_t stream, const void* x, const TcProj* proj, int num,
     const int rows = static_cast<int>((m + p.m_tiles - 1) / p.m_tiles), step = 16 * gemm_halves(rows);
     p.tile_m = (rows + step - 1) / step * step;
     p.groups = static_cast<int>(k / 128);
-    // (two or three groups: summed in turn, with the products of the second thread's first group rounded by themselves, the error against 64
-    // bits is a tenth larger than in sequence; from five groups on it is smaller, 0.91 to 0.99 of it)
-    if (p.groups < 5 && gemm_fold_in_turn(1, p.tile_m / 16)) p.tile_m = 96;
     long long tiles = 0;
     if (swiglu) {
         if (!encode_gemm_w(&p.w_map[0], proj[0].w, proj[0].n, k, 64) || !encode_gemm_w(&p.w_map[1], proj[1].w, proj[1].n, k, 64)) return -2;
