@@ -27,9 +27,10 @@ constexpr size_t kSamplingScratchBytes = 4u << 20;  // rows * chunks * 16 B
 // The line was drawn with (33 / 48 / 64 rows, slices and GEMM) gate/up of 5120 x 17408 49 and 55 / 53 and 53 / 55 and 53; 6144 x 5120
 // 19 and 21 / 21 and 21 / 22 and 21; 17408 x 5120 34 and 34 / 36 and 34 / 38 and 34, where the models were good to the 6 % that
 // the slices need as a margin.  From 65 rows on the third slice decides for the GEMM everywhere.
-// Both have gained since, the GEMM more: 47.0 and 38.5 / 48.9 and 38.1 / 51.4 and 38.3; 19.5 and 18.7 / 20.4 and 18.8 / 21.2 and 18.9;
-// 33.7 and 28.0 / 35.7 and 28.2 / 37.7 and 28.3.  So the line lies too far on the side of the slices: with models of today's kernels it
-// would leave them problems of few weights only.  It stays until it is drawn anew together with the routes that the tests pin.
+// Both have gained since, the GEMM more: 46.9 and 37.0 / 49.0 and 37.0 / 51.6 and 38.4; 19.8 and 15.2 / 20.6 and 15.1 / 21.3 and 16.5;
+// 34.1 and 23.9 / 36.4 and 24.1 / 38.1 and 25.7 (40 rows, which these three still send to the slices: 47.2 and 36.9, 20.1 and 15.2, 34.6 and 23.9).
+// So the line lies on the wrong side: with models of today's kernels it would leave the slices problems of few weights only.  It stays
+// until it is drawn anew together with the routes that the tests pin.
 constexpr int64_t kSliceRowsMax = 128, kSliceWeightsMax = 4 << 20, kTwoSlices = 64;
 bool slices_cost_less(const xb::TcProj* proj, int num, bool swiglu, int64_t m, int64_t k, int64_t weights, int num_sms) {
     if (weights <= kSliceWeightsMax) return true;

@@ -111,7 +111,7 @@ constexpr int kNormNarrow = 2048, kNormPairs = 6144;
 // TABLE: some job of the launch reads the embedding table.  VECS: most 8-element vectors of a thread: four of 256 threads (and the path for
 // rows that are not vectors), two of up to 512, or one of up to 1024.  FEW: no row shares its SM.  Bound by latency, then by the rows in flight.
 // One vector a thread is the shorter way through a row, which is what counts as long as every row has an SM to itself, and where 256
-// threads would not all have one: 5120 features with the residual added, 1 row 2.30 -> 1.84 us, 32 rows 2.57 -> 2.13, 148 rows 2.58 -> 2.24;
+// threads would not all have one (a launch of two jobs has two blocks a row, and that is what is counted): 5120 features with the residual added, 1 row 2.30 -> 1.84 us, 32 rows 2.57 -> 2.13, 148 rows 2.58 -> 2.24;
 // 1024 features, 2796 rows 8.9 -> 4.9.  (0.07 to 0.12 us of it since the compiler may use 64 registers, where otherwise it fits two rows of 1024
 // threads on an SM; with many narrow rows those are worth as much: 1024 features, 2796 rows 4.47 against 4.71.)  With more rows the 640
 // threads of a wide row leave an SM three rows at a time: 1024 x 5120 5.93 us with four vectors, 6.83 with one.
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(VECS == 1 ? 1024 : VECS == 2 ? 512 : 256, VECS
         }
         asm volatile("griddepcontrol.wait;" ::: "memory");
         const uint16_t* tr = table ? norm_tokens(job, row, hidden) : nullptr;
-        // one pass: each thread keeps its (up to four) 8-element vectors in registers.  Every load goes out before the first
+        // one pass: each thread keeps its 8-element vectors (VECS at most) in registers.  Every load goes out before the first
         // value is used and before any store (which the compiler must take for a possible alias of the later loads): with
         // the residual stored in between, each further vector was another trip to memory (2.9 us a launch against 2.5).
         uint4 v[VECS], dv[VECS];

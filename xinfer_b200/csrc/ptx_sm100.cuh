@@ -367,7 +367,7 @@ __device__ __forceinline__ uint32_t hfma2_u32(uint32_t a, uint32_t b, uint32_t c
     asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
-// acc0 += d0 * sc, acc1 += d1 * sc: two roundings each as fmaf has, one instruction.  (Volatile: it stays where it stands between the reads.)
+// acc0 += d0 * sc, acc1 += d1 * sc: one rounding each, as fmaf has, in one instruction.  (Volatile: it stays where it stands between the reads.)
 __device__ __forceinline__ void fma_pair(float& acc0, float& acc1, uint32_t d0, uint32_t d1, float sc) {
     asm volatile(
         "{\n\t"

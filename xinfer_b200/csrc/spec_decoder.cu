@@ -1025,8 +1025,8 @@ int xinfer_spec_decoder_step(xinfer_spec_decoder* d, xinfer_stream_t stream) {
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     int rc;
-    // The graph holds the previous pass's row count as a constant (k + 1): right after a prefill whose last chunk was
-    // shorter, one step runs eagerly.
+    // The graph holds the previous pass's row count as a constant (k + 1).  A prefill leaves no rows pending, so the step behind it
+    // runs eagerly.
     if (d->graph_exec && d->prev_rows == d->k + 1) rc = cudaGraphLaunch(d->graph_exec, s) == cudaSuccess ? XINFER_OK : XINFER_ERR_CUDA;
     else rc = enqueue_step(d, s);
     if (rc >= 0) d->ctx_upper += d->k + 1;

@@ -40,8 +40,8 @@ int tc_noalloc_take_status(int device);
 long long tc_wait_limit();  // clocks after which a device-side wait gives up (tc_set_wait_hooks)
 int tc_x_stage_limit();     // test hook of tc_set_wait_hooks: first activation stage that is never requested (-1: off; for the attention, its queries)
 
-// Dense GEMM for more than 32 activation rows (prefill chunks) on tcgen05, both operands from shared memory
-// (w4a16_gemm.cu).  One launch for all projections that share X; gate and up of the fused MLP are one pair.
+// Dense GEMM for more than 32 activation rows (prefill chunks) on tcgen05, the weights unpacked into tensor memory, the activations in
+// shared memory (w4a16_gemm.cu).  One launch for all projections that share X; gate and up of the fused MLP are one pair.
 bool gemm_eligible(const void* x, const TcProj* proj, int num, bool swiglu, long long m, long long k, int group_size);
 // `partials` (gemm_partial_bytes) and `counters` (eight zeroed ints per SM, left zeroed): scratch for tiles whose K range
 // is cut between CTAs (partials null: tiles are not cut).

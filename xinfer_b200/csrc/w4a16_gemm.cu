@@ -973,10 +973,10 @@ GemmDeal gemm_deal(const TcProj* proj, int num, bool swiglu, long long m, long l
 
 }  // namespace
 
-// The kernel as it was when the routes of 33 to 64 rows were drawn (c_api.cu), up to 30 % slower than now: 5.8 us a tile of a pair (fill,
-// read-out and stores) and 0.53 us a group; a cut costs kCutCost groups, or six where it falls on equal parts of every tile.  It was
-// within 6 % of most of 18 shapes at 33 .. 64 rows, and off by more for the narrowest (5120 x 2048 and narrower: within 3 us) and
-// for few tiles in many parts (16384 x 1024: 21 us, modelled 13).
+// The kernel as it was when the routes of 33 to 64 rows were drawn (c_api.cu), not as it is: 5.8 us a tile of a pair (fill, read-out and
+// stores) and 0.53 us a group; a cut costs kCutCost groups, or six where it falls on equal parts of every tile.  Then it was within 6 % of
+// most of 18 shapes at 33 .. 64 rows; now it is 40 to 46 % too long for the larger ones (gate/up 5120 x 17408 at 33 rows 54 modelled, 37
+// measured; 17408 x 5120 34 and 24).
 double gemm_modelled_us(const TcProj* proj, int num, bool swiglu, long long m, long long k, int num_sms) {
     const GemmDeal d = gemm_deal(proj, num, swiglu, m, k, num_sms, true);
     const long long groups = k / 128;
